@@ -1,0 +1,54 @@
+"""The many-row GEMM with a workspace (csrc/qgemm_stream.cu) at the edges of its tiles and of its dispatch: activation tiles of 16 .. 256 rows,
+weight tiles of 128 (up to 64 rows) and 256, one pass (fp16) and three (fp32), tiles split over CTAs or whole, remainders everywhere."""
+import numpy as np
+import pytest
+from tinygrad_b200 import _lib, quant, synth
+from tinygrad_b200.runtime import DeviceBuffer
+from oracle import ggml_quant as gq
+from gpu_util import need_gpu
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _gpu(): need_gpu()
+
+
+@pytest.mark.parametrize("split", [True, False])
+@pytest.mark.parametrize("typ,m,n_out,n_in,dt", [(2, 1, 16, 32, np.float32), (8, 16, 130, 96, np.float32), (2, 17, 1000, 1184, np.float32), (8, 64, 128, 4096, np.float32),
+                                                 (2, 65, 257, 4096, np.float32), (8, 128, 256, 160, np.float32), (2, 129, 300, 992, np.float32), (8, 256, 512, 512, np.float32),
+                                                 (2, 257, 130, 1408, np.float32), (2, 301, 200, 640, np.float16), (8, 64, 300, 1184, np.float16), (8, 600, 72, 96, np.float16)])
+def test_rows_against_the_exact_product(typ, m, n_out, n_in, dt, split):
+  rng = np.random.default_rng(m + n_out)
+  raw = synth.BLOCK_MAKERS[typ](n_out, n_in, rng)
+  w = gq.weight_matrix(raw, n_out, n_in, typ).astype(np.float64)
+  if dt == np.float16: w = w.astype(np.float16).astype(np.float64)          # fp16 activations take the fp16-rounded weight
+  x, bias, res = rng.standard_normal((m, n_in)).astype(dt), rng.standard_normal(n_out).astype(np.float16), rng.standard_normal((m, n_out)).astype(dt)
+  pw = quant.repack(raw, n_out, n_in, typ)
+  dx, db, y = DeviceBuffer.from_numpy(x), DeviceBuffer.from_numpy(bias), DeviceBuffer.from_numpy(res)
+  lib = _lib.load()
+  ws = DeviceBuffer(lib.b200q_qgemm_workspace_bytes_for(m, n_out, n_in) if split else lib.b200q_qgemm_workspace_bytes(m, n_in))
+  code = _lib.F32 if dt == np.float32 else _lib.F16
+  quant.qgemm(pw.buf.ptr, typ, n_out, n_in, dx, y, m, x_dtype=code, y_dtype=code, bias=db, residual=y, workspace=ws)
+  ref = x.astype(np.float64) @ w.T + bias + res
+  # 2^-21: the dropped low x low product and the rounding of the low halves; then one rounding of the running sum (at most the sum of the
+  # magnitudes) per tensor-core instruction, up to three per 16 columns; fp32 (fp16) rounding of the result
+  size = np.abs(x).astype(np.float64) @ np.abs(w).T + np.abs(bias) + np.abs(res)
+  bound = (2.0 ** -21 + 3 * np.ceil(n_in / 16) * 2.0 ** -23) * size + (2.0 ** -11 if dt == np.float16 else 2.0 ** -23) * np.abs(ref) + 1e-7
+  assert (np.abs(y.numpy() - ref) <= bound).all(), f"worst {np.max(np.abs(y.numpy() - ref) / bound):.2f} of the bound"
+
+
+def test_norm_in_front_and_swiglu_behind():
+  m, hidden, dim = 45, 1408, 512
+  rng = np.random.default_rng(4)
+  gate, up = (synth.q4_0_blocks(hidden, dim, rng) for _ in range(2))
+  nw, x = (1 + 0.1 * rng.standard_normal(dim)).astype(np.float16), rng.standard_normal((m, dim)).astype(np.float32)
+  pw = quant.repack(gate, hidden, dim, 2, raw_up=up)
+  y, ws = DeviceBuffer.empty((m, hidden), np.float32), DeviceBuffer(quant.qgemm_workspace_bytes(m, dim))
+  quant.qgemm(pw.buf.ptr, 2, 2 * hidden, dim, DeviceBuffer.from_numpy(x), y, m, epilogue=_lib.EPI_SILU_MUL, workspace=ws, norm_weight=DeviceBuffer.from_numpy(nw), norm_eps=1e-5)
+  xn = x.astype(np.float64) / np.sqrt((x.astype(np.float64) ** 2).mean(-1, keepdims=True) + 1e-5) * nw
+  g, u = (xn @ gq.weight_matrix(b, hidden, dim, 2).astype(np.float64).T for b in (gate, up))
+  ref = g / (1 + np.exp(-g)) * u
+  # each factor is good to 2^-18 of its largest value (the bound above at 512 columns); |d silu| <= 1.1
+  tol = 2.0 ** -18 * (1.1 * np.abs(g).max() * np.abs(u) + np.abs(g) * np.abs(u).max() + 1)
+  assert (np.abs(y.numpy() - ref) <= tol).all()

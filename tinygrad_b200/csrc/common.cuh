@@ -29,6 +29,7 @@ struct PerDeviceFlag {
 int b200q_decode_status_take(int* status);
 int b200q_decode_step_status_take(int* status);   // the same for the whole-step kernel (decode_step.cu)
 int b200q_peer_status_take(int* status);          // the same for the peer-memory collectives (peer.cu)
+int b200q_qgemm_stream_status_take(int* status);  // the same for the many-row GEMM (qgemm_stream.cu)
 int b200q_ep_status_take(int* status);            // the same for the expert-parallel exchange (ep.cu)
 // current device index, or -1 (with the CUDA error recorded) if it cannot be had or is past the tables
 int b200q_current_device();

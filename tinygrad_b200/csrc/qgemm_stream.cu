@@ -1,0 +1,626 @@
+// Linear over many activation rows on packed Q4_0 / Q8_0 weights (prompts, batched rows):  Y[m, n] = X[m, k] W[n, k]^T
+// (+ bias, + residual, or the SwiGLU product of interleaved gate / up rows).  Replaces `Linear.__call__` for T > 1
+// (tinygrad/nn/__init__.py:177; prefill chunks of tinygrad/llm/model.py:464-481).
+//
+// Numerics: fp32 activations are split into fp16 halves x = xh + xl, the dequantised weight into w = wh + wl (wh the fp16 product of
+// quant and scale, wl its exact remainder), and y = wh xh + wh xl + wl xh is accumulated in fp32 on the tensor cores: the fp32
+// activation times the unrounded weight to about 2^-22.  fp16 activations take one pass with the fp16-rounded weight.
+//
+// What bounds it: three fp16 tensor passes for many rows; for few rows the weight stream and the unpacking.  So
+//  * weights are the MMA's A operand (128 rows per instruction) and the activation rows its N: any row count rounded up to 16 fills the
+//    instruction, and up to 128 rows the halves xh | xl sit side by side as ONE operand of 2 N columns (two instructions per K step
+//    instead of three);
+//  * a tile is 256 weight rows (two accumulators, the whole of tensor memory) by up to 256 activation rows: every unpacked weight meets
+//    256 rows and every activation byte 256 weight rows.  With 128 x 128 tiles the activation operand alone took 2.4x the L2 traffic
+//    and every weight was unpacked once per 128 rows.  Up to 64 rows a tile is 128 weight rows (more tiles to share, smaller partial sums);
+//  * roles are separate warps: 16 unpack the weights (global -> registers, several blocks ahead -> fp16 halves in a ring of
+//    shared-memory slots), one thread brings activation tiles in by bulk copies, one issues the MMAs; nothing meets at a block barrier;
+//  * the K x tile space is dealt to one CTA per SM in equal contiguous runs (stream-K): no last wave.  A tile that spans CTAs leaves fp32
+//    partial sums in the workspace; the CTA that arrives last adds them in the order of K (bit-reproducible) and writes the result.
+//    Nobody waits for another CTA.
+// Every mbarrier wait is bounded: on expiry a status word is set, all roles leave, copies and MMAs in flight are drained.
+#include "common.cuh"
+#include "tc_common.cuh"
+#include <cstddef>
+
+namespace {
+
+constexpr int UNPACK_WARPS = 16, UNPACK_THREADS = UNPACK_WARPS * 32;
+constexpr int WARP_COPY = UNPACK_WARPS, WARP_MMA = UNPACK_WARPS + 1;
+constexpr int THREADS = (UNPACK_WARPS + 2) * 32;
+constexpr int KSTEP = 32;                               // one quant block of K per step
+__host__ __device__ constexpr int steps_per_slot(int wt) { return wt == 128 ? 4 : 1; }
+constexpr int RING_BYTES = 224 * 1024, MAX_SLOTS = 6;   // shared memory: slots of unpacked weights + activations
+constexpr int MAX_NT = 256;                             // activation rows per tile
+constexpr size_t COUNTER_BYTES = 4096;                  // one arrival counter per CTA (a split tile is counted at the CTA that holds its head)
+
+struct StreamParams {
+  const uint8_t* w;
+  const unsigned char* xt;       // activation tiles (split_rows)
+  float* part;
+  unsigned* counters;
+  const __half* bias;
+  const void* residual;
+  void* y;
+  long long units;               // tiles x K groups
+  int grain;                     // units are dealt in multiples of this: 1, or a whole tile where the workspace has no room for partial sums
+  int tiles, m, n_out, kgroups, n_row_tiles, nt, tok_tiles, slots, y_f16, silu_mul;
+};
+
+// ---- activations: fp32 (or fp16) rows, optionally RMS-normed, -> fp16 halves as the tensor core reads them ---------------------
+// workspace: per activation tile of nt rows and K step of 32: [4 chunks of 8 columns][nt rows hi | nt rows lo][16 bytes], contiguous, so
+// that a step's operand is one bulk copy.  Element order inside a chunk: [0,2,1,3,4,6,5,7], the order the weight unpack delivers.
+// One CTA: 8 rows (a core matrix) x a stretch of columns; a row's chunk is 32 bytes in, 16 + 16 bytes out, 8 rows make 128 contiguous bytes.
+constexpr int SPLIT_THREADS = 256;
+
+template <typename T>
+__global__ void __launch_bounds__(SPLIT_THREADS) split_rows_kernel(const T* __restrict__ x, const __half* __restrict__ norm_w, float eps, int m, int n_in,
+                                                                   int kgroups, int nt, int chunks_per_cta, unsigned char* __restrict__ xt,
+                                                                   unsigned* __restrict__ counters, int n_counters) {
+  constexpr bool F32 = sizeof(T) == 4;
+  __shared__ float red[SPLIT_THREADS / 32][8];
+  pdl_wait();
+  pdl_launch_dependents();
+  const int tid = threadIdx.x;
+  if (blockIdx.x == 0 && blockIdx.y == 0)
+    for (int i = tid; i < n_counters; i += SPLIT_THREADS) counters[i] = 0;
+  const int r = tid & 7, row = blockIdx.y * 8 + r;                       // row within the padded rows of all tiles
+  const int tile = row / nt, in_tile = row - tile * nt;
+  const bool live = row < m;
+  float sc = 1.f;
+  if (F32 && norm_w) {
+    float ss = 0.f;
+    if (live)
+      for (int k = (tid >> 3) * 4; k < n_in; k += SPLIT_THREADS / 8 * 4) {
+        const float4 a = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(x) + (size_t)row * n_in + k);
+        ss = fmaf(a.x, a.x, fmaf(a.y, a.y, fmaf(a.z, a.z, fmaf(a.w, a.w, ss))));
+      }
+    ss += __shfl_xor_sync(0xffffffffu, ss, 8);
+    ss += __shfl_xor_sync(0xffffffffu, ss, 16);
+    if ((tid & 31) < 8) red[tid >> 5][r] = ss;
+    __syncthreads();
+    float tot = 0.f;
+#pragma unroll
+    for (int i = 0; i < SPLIT_THREADS / 32; i++) tot += red[i][r];
+    sc = 1.0f / sqrtf(tot / (float)n_in + eps);
+  }
+  const int n_chunks = kgroups * 16, c1 = min(n_chunks, (int)(blockIdx.x + 1) * chunks_per_cta);
+  const size_t row_bytes = (F32 ? 2 : 1) * (size_t)nt * 16;               // one chunk of a step
+  unsigned char* base = xt + (size_t)tile * n_chunks * row_bytes + (size_t)in_tile * 16;
+  for (int c = blockIdx.x * chunks_per_cta + (tid >> 3); c < c1; c += SPLIT_THREADS / 8) {
+    const int k = c * 8;
+    float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    unsigned char* dst = base + (size_t)c * row_bytes;
+    if (!F32) {
+      uint4 raw = make_uint4(0, 0, 0, 0);
+      if (live && k < n_in) raw = *reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(x) + (size_t)row * n_in + k);
+      *reinterpret_cast<uint4*>(dst) = make_uint4(prmt(raw.x, raw.y, 0x5410u), prmt(raw.x, raw.y, 0x7632u), prmt(raw.z, raw.w, 0x5410u), prmt(raw.z, raw.w, 0x7632u));
+      continue;
+    }
+    if (live && k < n_in) {
+      const float* src = reinterpret_cast<const float*>(x) + (size_t)row * n_in + k;
+      const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
+      f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+      if (norm_w) {
+        const uint4 nw = *reinterpret_cast<const uint4*>(norm_w + k);
+        const __half2* h = reinterpret_cast<const __half2*>(&nw);
+#pragma unroll
+        for (int q = 0; q < 4; q++) { const float2 t2 = __half22float2(h[q]); f[2 * q] = f[2 * q] * sc * t2.x; f[2 * q + 1] = f[2 * q + 1] * sc * t2.y; }
+      }
+    }
+    uint4 hi, lo;
+    split_chunk(f, hi, lo);
+    *reinterpret_cast<uint4*>(dst) = hi;
+    *reinterpret_cast<uint4*>(dst + (size_t)nt * 16) = lo;
+  }
+}
+
+// ---- the product ---------------------------------------------------------------------------------------------------------------
+struct Shared {                       // barriers and small words (static shared memory)
+  uint64_t full[MAX_SLOTS], empty[MAX_SLOTS], acc_full, acc_empty, stored, counted, drained;
+  uint32_t tmem, last;
+  int abort;
+};
+
+// Barriers are named by their shared-memory address, taken once (`sb` = the address of the Shared block) and kept in a register.
+#define BAR(sb, member) ((sb) + (uint32_t)offsetof(Shared, member))
+__device__ __forceinline__ uint32_t pinned(uint32_t v) { asm volatile("" : "+r"(v)); return v; }
+
+__device__ __forceinline__ void bar_init(uint32_t bar, int n) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(n)); }
+__device__ __forceinline__ void bar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+// Bounded wait: false once another role has given up, or when the time is over (then the others are told).
+__device__ __forceinline__ bool bar_wait(uint32_t sb, uint32_t bar, uint32_t parity) {
+  for (int i = 0; i < (1 << 20); i++) {
+    uint32_t ok, gone;
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\nselp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok) : "r"(bar), "r"(parity), "r"(2000) : "memory");
+    if (ok) return true;
+    asm volatile("ld.volatile.shared::cta.u32 %0, [%1];" : "=r"(gone) : "r"(BAR(sb, abort)) : "memory");
+    if (gone) return false;
+  }
+  asm volatile("st.volatile.shared::cta.u32 [%0], 1;" ::"r"(BAR(sb, abort)) : "memory");
+  atomicExch(&g_tc_status, 1);
+  return false;
+}
+// The copy and MMA threads are elected, not `lane == 0`: under elect.sync the compiler may use uniform registers, which the tcgen05 and
+// barrier instructions take their operands from.  As plain `lane == 0` code the MMA thread needed 80 cycles to issue an instruction and
+// over 300 for a barrier that was ready (8B gate/up, 8 rows: 127 -> 90 us).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(e));
+  return e != 0;
+}
+__device__ __forceinline__ void commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// descriptors as {low word, common high word}: a step's operands differ in the start address alone
+__device__ __forceinline__ void mma(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t acc) {
+  asm volatile("{\n.reg .pred p;\n.reg .b64 a, b;\nmov.b64 a, {%1, %3};\nmov.b64 b, {%2, %3};\nsetp.ne.u32 p, %5, 0;\n"
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n}"
+               ::"r"(d), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(acc) : "memory");
+}
+__device__ __forceinline__ void st_shared(uint32_t a, const uint4& v) {
+  asm volatile("st.shared::cta.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+constexpr int EC = 8;                                   // accumulator columns (activation rows) a thread of the epilogue takes at a time
+__device__ __forceinline__ void ld_tmem(uint32_t a, uint32_t (&v)[EC]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(a));
+}
+
+// unit range of CTA c (in whole grains), and the CTA that holds a unit (grain 1: tiles are split only then)
+__device__ __forceinline__ long long first_unit(long long c, const StreamParams& p, int g) { return c * (p.units / p.grain) / g * p.grain; }
+// Where CTA c leaves its part of a split tile.  Along the units either the CTA or the tile (or both) goes up by one from part to part, so
+// c + tile is a number of its own for each; with more tiles than CTAs, two places per CTA (its first and its last part) take less room.
+__device__ __forceinline__ size_t part_slot(const StreamParams& p, int c, int tile, bool head) {
+  return p.tiles < (int)gridDim.x ? (size_t)(c + tile) : (size_t)(2 * c + (head ? 1 : 0));
+}
+__device__ __forceinline__ int cta_of(long long unit, long long units, int g) { return (int)(((unit + 1) * g - 1) / units); }
+
+// EC consecutive activation rows of one output column (weight row) `feat`
+__device__ __forceinline__ void store_outputs(const StreamParams& p, const float (&v)[EC], int feat, int tok0, int lane) {
+  if (p.silu_mul) {
+    // gate rows sit in lanes with bit 3 clear, the matching up rows 8 lanes on: each of a pair takes every other activation row
+    const bool gate = !(lane & 8);
+    const int col = (feat >> 4) * 8 + (feat & 7), n_y = p.n_out >> 1;
+#pragma unroll
+    for (int j = 0; j < EC; j += 2) {
+      const float other = __shfl_xor_sync(0xffffffffu, gate ? v[j + 1] : v[j], 8);
+      const float g = gate ? v[j] : other, u = gate ? other : v[j + 1], o = (g / (1.f + expf(-g))) * u;
+      const int tok = tok0 + j + (gate ? 0 : 1);
+      if (tok < p.m && col < n_y) {
+        const size_t at = (size_t)tok * n_y + col;
+        if (p.y_f16) reinterpret_cast<__half*>(p.y)[at] = __float2half_rn(o); else reinterpret_cast<float*>(p.y)[at] = o;
+      }
+    }
+    return;
+  }
+  if (feat >= p.n_out) return;
+  const float b = p.bias ? __half2float(p.bias[feat]) : 0.f;
+  float add[EC];
+#pragma unroll
+  for (int j = 0; j < EC; j++) {
+    add[j] = b;
+    if (p.residual && tok0 + j < p.m) {
+      const size_t at = (size_t)(tok0 + j) * p.n_out + feat;
+      add[j] += p.y_f16 ? __half2float(reinterpret_cast<const __half*>(p.residual)[at]) : reinterpret_cast<const float*>(p.residual)[at];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < EC; j++)
+    if (tok0 + j < p.m) {
+      const size_t at = (size_t)(tok0 + j) * p.n_out + feat;
+      if (p.y_f16) reinterpret_cast<__half*>(p.y)[at] = __float2half_rn(v[j] + add[j]); else reinterpret_cast<float*>(p.y)[at] = v[j] + add[j];
+    }
+}
+
+// The 16 unpack warps read the accumulators of segment `seg` (K groups k0 .. k1 of `tile`) back.
+template <int WT, bool F32>
+__device__ __forceinline__ bool finish_segment(const StreamParams& p, Shared& sh, uint32_t sb, int seg, int tile, int k0, int k1) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = warp & 3, q = warp >> 2;
+  const int hf = WT == 256 ? q >> 1 : 0, part0 = WT == 256 ? q & 1 : q, parts = WT == 256 ? 2 : 4;
+  const int tt = tile % p.tok_tiles, row = hf * 128 + sub * 32 + lane, feat = (tile / p.tok_tiles) * WT + row;
+  const bool whole = k0 == 0 && k1 == p.kgroups, stacked = F32 && p.nt <= MAX_NT / 2;
+  const int G = gridDim.x, c = blockIdx.x;
+  int c0 = c, n_seg = 1;
+  if (!whole) {
+    c0 = cta_of((long long)tile * p.kgroups, p.units, G);
+    n_seg = cta_of((long long)(tile + 1) * p.kgroups - 1, p.units, G) - c0 + 1;
+  }
+  const size_t slot = (size_t)WT * p.nt;
+  float* mine = p.part + part_slot(p, c, tile, c == c0) * slot + row * 4;      // [group of 4 columns][row][4]: a warp's store is 512 contiguous bytes
+  if (!bar_wait(sb, BAR(sb, acc_full), seg & 1)) return false;
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t ta = sh.tmem + ((uint32_t)(sub * 32) << 16) + hf * 256;
+  const int groups = p.nt / EC;
+  for (int cg = part0; cg < groups; cg += parts) {
+    uint32_t a[EC], b[EC];
+    ld_tmem(ta + cg * EC, a);
+    if (stacked) ld_tmem(ta + p.nt + cg * EC, b);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    float v[EC];
+#pragma unroll
+    for (int j = 0; j < EC; j++) v[j] = stacked ? __uint_as_float(a[j]) + __uint_as_float(b[j]) : __uint_as_float(a[j]);
+    if (whole) store_outputs(p, v, feat, tt * p.nt + cg * EC, lane);
+    else
+#pragma unroll
+      for (int j = 0; j < EC; j += 4) __stcg(reinterpret_cast<float4*>(mine + (size_t)(cg * EC + j) * WT), make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]));
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  if (!whole) __threadfence();
+  __syncwarp();
+  if (lane == 0) { bar_arrive(BAR(sb, acc_empty)); if (!whole) bar_arrive(BAR(sb, stored)); }
+  if (whole) return true;
+  // a CTA has at most two partial segments: its first and its last; `stored` / `counted` complete once for each
+  const uint32_t par = c == c0 && first_unit(c, p, G) % p.kgroups != 0 ? 1 : 0;
+  if (tid == 0 && bar_wait(sb, BAR(sb, stored), par)) {
+    __threadfence();
+    const unsigned old = atomicAdd(p.counters + c0, 1u);
+    const bool last = old == (unsigned)n_seg - 1;
+    if (last) p.counters[c0] = 0;
+    sh.last = last;
+    __threadfence();
+    bar_arrive(BAR(sb, counted));
+  }
+  if (!bar_wait(sb, BAR(sb, counted), par)) return false;
+  if (!*reinterpret_cast<volatile uint32_t*>(&sh.last)) return true;
+  const float* from = p.part + row * 4;
+  for (int cg = part0; cg < groups; cg += parts) {
+    float v[EC];
+#pragma unroll
+    for (int j = 0; j < EC; j++) v[j] = 0.f;
+#pragma unroll 2
+    for (int s = 0; s < n_seg; s++) {
+      const float* sp = from + part_slot(p, c0 + s, tile, s == 0) * slot + (size_t)cg * EC * WT;
+#pragma unroll
+      for (int j = 0; j < EC; j += 4) {
+        const float4 f = __ldcg(reinterpret_cast<const float4*>(sp + (size_t)j * WT));
+        v[j] += f.x; v[j + 1] += f.y; v[j + 2] += f.z; v[j + 3] += f.w;
+      }
+    }
+    store_outputs(p, v, feat, tt * p.nt + cg * EC, lane);
+  }
+  return true;
+}
+
+// the weights of one 32-wide block of a row as they come from memory
+template <int QT> struct Raw;
+template <> struct Raw<B200Q_Q4_0> { uint4 a; uint32_t d; };
+template <> struct Raw<B200Q_Q8_0> { uint4 a, b; uint32_t d; };
+
+template <int QT, int WT, bool F32>
+__global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamParams p) {
+  constexpr int TB = tile_bytes(QT), GROUPS = UNPACK_THREADS / WT, PER_UNIT = 4 / GROUPS;    // thread groups, each with its own steps of a K group
+  constexpr int W_HALF = WT * KSTEP * 2, W_STEP = 2 * W_HALF;
+  // Steps per ring slot, i.e. per barrier phase.  With few activation rows a step's MMAs take less time than the barrier operations around
+  // them (a ready barrier costs the MMA thread about 100 cycles, an instruction of N <= 128 72), so a slot is a whole K group there.
+  constexpr int SPS = steps_per_slot(WT), W_SLOT = W_STEP * SPS;
+  constexpr int DEPTH = QT == B200Q_Q4_0 ? 4 : 3;                                             // blocks in flight per thread
+  extern __shared__ __align__(128) unsigned char dyn[];
+  __shared__ Shared sh;
+  const uint32_t sb = pinned(s32(&sh)), ring = pinned(s32(dyn));
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int G = gridDim.x, c = blockIdx.x;
+  const long long u0 = first_unit(c, p, G), u1 = first_unit(c + 1, p, G);
+  const int nt = p.nt, slots = p.slots, x_rows = F32 ? 2 * nt : nt;
+  const uint32_t x_step = (uint32_t)x_rows * 64, x_bytes = x_step * SPS, slot_bytes = W_SLOT + x_bytes;      // a step's activations, a slot's; a whole slot
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(&sh.tmem)), "r"(WT == 256 ? 512 : 256) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (tid == 32) {
+    // a slot is full when its unpack warps and the copy thread have arrived and the copy's bytes are there; one commit empties it
+    for (int i = 0; i < MAX_SLOTS; i++) { bar_init(BAR(sb, full) + 8 * i, WT / 32 * SPS + 1); bar_init(BAR(sb, empty) + 8 * i, 1); }
+    bar_init(BAR(sb, acc_full), 1); bar_init(BAR(sb, acc_empty), UNPACK_WARPS);
+    bar_init(BAR(sb, stored), UNPACK_WARPS); bar_init(BAR(sb, counted), 1); bar_init(BAR(sb, drained), 1);
+    sh.abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  pdl_launch_dependents();
+
+  if (warp == WARP_COPY) {
+    if (elect_one()) {
+      pdl_wait();                                        // the activation tiles are the previous kernel's (generic stores, read by bulk copies here)
+      asm volatile("fence.proxy.async.global;" ::: "memory");
+      bool ok = true;
+      int n = 0, slot = 0;                               // steps issued; ring position (counted, not divided: this thread's loop is the copies' pace)
+      uint32_t par = 1;
+      for (long long u = u0; u < u1 && ok;) {
+        const int tile = (int)(u / p.kgroups), k0 = (int)(u - (long long)tile * p.kgroups), k1 = (int)min((long long)p.kgroups, k0 + u1 - u);
+        const unsigned char* src = p.xt + ((size_t)(tile % p.tok_tiles) * p.kgroups + k0) * 4 * x_step;
+        for (int s = 0; s < (k1 - k0) * (4 / SPS); s++, n++, src += x_bytes) {
+          if (!bar_wait(sb, BAR(sb, empty) + 8 * slot, par)) { ok = false; break; }
+          const uint32_t dst = ring + slot * slot_bytes + W_SLOT, bar = BAR(sb, full) + 8 * slot;
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(x_bytes) : "memory");
+          for (uint32_t o = 0; o < x_bytes; o += 8192)   // several copies overlap where one is served slowly
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                         ::"r"(dst + o), "l"(src + o), "r"(min(8192u, x_bytes - o)), "r"(bar) : "memory");
+          if (++slot == slots) { slot = 0; par ^= 1; }
+        }
+        u += k1 - k0;
+      }
+      // Nothing may still be landing in shared memory when the CTA leaves.  After a failed wait a slot's unpack warps may never arrive, so its
+      // barrier cannot tell; the copies are done long before the time that wait took, and one more is spent here.
+      for (int j = max(0, n - slots); j < n; j++)
+        if (!wait_bar(BAR(sb, full) + 8 * (j % slots), (j / slots) & 1)) break;
+    }
+  } else if (warp == WARP_MMA) {
+    if (elect_one()) {
+      bool ok = true;
+      const bool stacked = F32 && nt <= MAX_NT / 2;
+      const uint32_t id1 = make_idesc(128, nt), id2 = make_idesc(128, stacked ? 2 * nt : nt);
+      const uint32_t desc_hi = (uint32_t)(make_desc(0, 0, 128) >> 32);
+      const uint32_t w_base = (ring >> 4) | ((uint32_t)WT << 16), x_base = ((ring + W_SLOT) >> 4) | ((uint32_t)x_rows << 16);
+      int seg = 0, slot = 0;
+      uint32_t par = 0, x_lo = x_base, w_lo = w_base;
+      for (long long u = u0; u < u1 && ok; seg++) {
+        const int k0 = (int)(u % p.kgroups), k1 = (int)min((long long)p.kgroups, k0 + u1 - u);
+        if (!bar_wait(sb, BAR(sb, acc_empty), (seg & 1) ^ 1)) { ok = false; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t tmem = sh.tmem;
+        uint32_t acc = 0;
+        for (int s = (k1 - k0) * (4 / SPS); s > 0; s--) {
+          if (!bar_wait(sb, BAR(sb, full) + 8 * slot, par)) { ok = false; break; }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          // all MMAs of one accumulator back to back: switching the destination costs about 40 cycles of a 128-cycle instruction
+          // (N = 256; nearly 100 at N <= 128, where an instruction takes at least 72 cycles whatever its N)
+#pragma unroll
+          for (int hf = 0; hf < WT / 128; hf++) {
+            const uint32_t d = tmem + hf * 256;
+#pragma unroll
+            for (int kk = 0; kk < SPS * KSTEP / 16; kk++) {
+              const uint32_t xh = x_lo + (kk >> 1) * (x_step >> 4) + (kk & 1) * 2 * x_rows;
+              const uint32_t wh = w_lo + (kk >> 1) * (W_STEP >> 4) + hf * 128 + (kk & 1) * 2 * WT;
+              mma(d, wh, xh, desc_hi, id2, kk ? 1u : acc);          // stacked: wh x [xh | xl] in one instruction
+              if (F32) {
+                if (!stacked) mma(d, wh, xh + nt, desc_hi, id1, 1u);
+                mma(d, wh + (W_HALF >> 4), xh, desc_hi, id1, 1u);
+              }
+            }
+          }
+          acc = 1;
+          commit(BAR(sb, empty) + 8 * slot);
+          x_lo += slot_bytes >> 4; w_lo += slot_bytes >> 4;
+          if (++slot == slots) { slot = 0; par ^= 1; x_lo = x_base; w_lo = w_base; }
+        }
+        if (ok) commit(BAR(sb, acc_full));
+        u += k1 - k0;
+      }
+      commit(BAR(sb, drained));                               // also on the way out after a failed wait: MMAs issued must be done before tensor memory goes back
+      wait_bar(BAR(sb, drained), 0);
+    }
+  } else {
+    // ------------------------------ unpack ------------------------------
+    // Thread group `grp` takes the steps t = grp, grp + GROUPS, .. of every K group; a thread takes one weight row's block of 32.
+    const int grp = tid / WT, r = tid % WT, h8 = (r >> 3) & 1, g = r & 7;
+    // The block being fetched.  A weight row's K groups are contiguous, so within a tile the pointer only moves on.
+    const int in_w = (h8 * (QT == B200Q_Q4_0 ? 32 : 64) + g * 4 + grp) * 16, in_d = TB - 128 + (2 * g * 4 + h8 * 2) * 2;
+    int ft = (int)(u0 / p.kgroups), f_left = (int)min((long long)p.kgroups - (u0 - (long long)ft * p.kgroups), u1 - u0), fs = 0;
+    int f_units = (int)(u1 - u0);                        // units still to fetch
+    const uint8_t* fp = nullptr;
+    auto set_tile = [&](int k0) {
+      const int f_row = ft / p.tok_tiles * (WT / 16) + (r >> 4);
+      fp = f_row < p.n_row_tiles ? p.w + ((size_t)f_row * p.kgroups + k0) * TB : nullptr;
+    };
+    set_tile((int)(u0 - (long long)ft * p.kgroups));
+    auto fetch = [&](Raw<QT>& q) {
+      if (fp && f_units > 0) {
+        const int t = grp + fs * GROUPS;
+        q.d = __ldg(reinterpret_cast<const unsigned short*>(fp + in_d + (t >> 1) * 8 + (t & 1) * 2));
+        q.a = __ldg(reinterpret_cast<const uint4*>(fp + in_w + fs * GROUPS * 16));
+        if constexpr (QT == B200Q_Q8_0) q.b = __ldg(reinterpret_cast<const uint4*>(fp + in_w + fs * GROUPS * 16 + 512));
+        if (PER_UNIT == 1 || fs == PER_UNIT - 1) fp += TB;
+      } else {
+        q.a = make_uint4(0, 0, 0, 0);
+        q.d = 0;
+        if constexpr (QT == B200Q_Q8_0) q.b = make_uint4(0, 0, 0, 0);
+      }
+      if (PER_UNIT == 1 || ++fs == PER_UNIT) {
+        fs = 0; f_units--;
+        if (--f_left == 0) { ft++; f_left = p.kgroups; set_tile(0); }
+      }
+    };
+    Raw<QT> q[DEPTH];
+#pragma unroll
+    for (int d = 0; d < DEPTH; d++) fetch(q[d]);
+    pdl_wait();                                          // the epilogue reads and writes what earlier kernels touched
+    // One block: wait for its slot, unpack, hand over, ask for the block DEPTH further on.
+    int slot = SPS > 1 ? 0 : grp;                        // ring position and its phase; SPS == 1: the thread groups take turns
+    uint32_t par = 1;
+    constexpr int SLOT_STEP = SPS > 1 ? 1 : GROUPS;
+    static_assert(SPS == 1 || (SPS == 4 && GROUPS == 4), "one block per thread and slot");
+    bool ok = true;
+    auto unpack = [&](Raw<QT>& q) {
+      ok = ok && bar_wait(sb, BAR(sb, empty) + 8 * slot, par);
+      const uint32_t dst = ring + slot * slot_bytes + (SPS > 1 ? grp * W_STEP : 0) + r * 16;
+      const uint32_t d2 = q.d | (q.d << 16);
+      uint4 hi[4], lo[4];
+      if constexpr (QT == B200Q_Q4_0) {
+        uint32_t v[4][4];
+        q4_word(q.a.x, v[0]); q4_word(q.a.y, v[1]); q4_word(q.a.z, v[2]); q4_word(q.a.w, v[3]);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const int a = (i & 1) * 2, b = (i >> 1) * 2;      // chunk i: words a, a + 1; low or high nibbles
+          const uint32_t r4[4] = {v[a][b], v[a][b + 1], v[a + 1][b], v[a + 1][b + 1]};
+          hi[i] = hi_lo(r4, d2, lo[i]);
+        }
+      } else {
+        hi[0] = q8_core(q.a.x, q.a.y, d2, lo[0]); hi[1] = q8_core(q.a.z, q.a.w, d2, lo[1]);
+        hi[2] = q8_core(q.b.x, q.b.y, d2, lo[2]); hi[3] = q8_core(q.b.z, q.b.w, d2, lo[3]);
+      }
+      if (ok) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          st_shared(dst + i * (WT * 16), hi[i]);
+          if (F32) st_shared(dst + W_HALF + i * (WT * 16), lo[i]);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      }
+      __syncwarp();
+      if (lane == 0) bar_arrive(BAR(sb, full) + 8 * slot);
+      fetch(q);
+      slot += SLOT_STEP;
+      if (slot >= slots) { slot -= slots; par ^= 1; }
+    };
+    // A segment's accumulators are read back only after the first LEAD blocks of the next one are unpacked: they fill the ring while the
+    // MMAs still in the pipe complete.
+    const int LEAD = SPS > 1 ? slots : slots / GROUPS;
+    int done_tile = -1, done_k0 = 0, done_k1 = 0, seg = 0;
+    long long u = u0;
+    while (ok) {
+      int tile = 0, k0 = 0, k1 = 0, left = 0;
+      if (u < u1) {
+        tile = (int)(u / p.kgroups); k0 = (int)(u - (long long)tile * p.kgroups); k1 = (int)min((long long)p.kgroups, k0 + u1 - u);
+        left = (k1 - k0) * PER_UNIT;
+      }
+      const int lead = done_tile >= 0 ? min(left, LEAD) : left;
+      // one instance of the unpack code, the queue of fetched blocks moving up: unrolled over the queue the loop took 1.6x the cycles per
+      // block (instruction fetch)
+#pragma unroll 1
+      for (int stop = left - lead;; stop = 0) {
+#pragma unroll 1
+        for (; left > stop && ok; left--) {
+          unpack(q[0]);
+          const Raw<QT> head = q[0];
+#pragma unroll
+          for (int d = 0; d + 1 < DEPTH; d++) q[d] = q[d + 1];
+          q[DEPTH - 1] = head;
+        }
+        if (done_tile >= 0 && ok) {
+          ok = finish_segment<WT, F32>(p, sh, sb, seg++, done_tile, done_k0, done_k1);
+          done_tile = -1;
+        } else break;
+      }
+      if (u >= u1) break;
+      done_tile = tile; done_k0 = k0; done_k1 = k1;
+      u += k1 - k0;
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(sh.tmem), "r"(WT == 256 ? 512 : 256) : "memory");
+}
+
+// ---- launch --------------------------------------------------------------------------------------------------------------------
+struct Plan { int nt, tok_tiles, wt; };
+Plan make_plan(int m) {
+  Plan pl;
+  pl.tok_tiles = ceil_div(m, MAX_NT);
+  pl.nt = ceil_div(ceil_div(m, pl.tok_tiles), 16) * 16;      // equal tiles: 301 rows are 2 x 160, not 256 + 45
+  pl.wt = pl.nt <= 64 ? 128 : 256;
+  return pl;
+}
+size_t tiles_bytes(const Plan& pl, int kgroups, bool f32) { return (size_t)pl.tok_tiles * pl.nt * kgroups * GROUP_ELEMS * (f32 ? 4 : 2); }
+int slot_bytes(const Plan& pl, bool f32) { return steps_per_slot(pl.wt) * (pl.wt * KSTEP * 4 + pl.nt * (f32 ? 128 : 64)); }
+size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
+
+template <int QT, int WT, bool F32>
+int launch_stream(const StreamParams& p, int grid, cudaStream_t st) {
+  auto kern = qgemm_stream_kernel<QT, WT, F32>;
+  static PerDeviceFlag attr;
+  const int dev = b200q_current_device();
+  if (dev < 0) return B200Q_ERR_CUDA;
+  if (!attr.test(dev)) {
+    B200Q_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, RING_BYTES));
+    attr.set(dev);
+  }
+  B200Q_CHECK_CUDA(launch_k(kern, dim3(grid), dim3(THREADS), (size_t)p.slots * slot_bytes({p.nt, p.tok_tiles, WT}, F32), st, true, p));
+  return B200Q_OK;
+}
+
+}  // namespace
+
+int b200q_qgemm_stream_status_take(int* status) {
+  int zero = 0;
+  B200Q_CHECK_CUDA(cudaMemcpyFromSymbol(status, g_tc_status, sizeof(int)));
+  B200Q_CHECK_CUDA(cudaMemcpyToSymbol(g_tc_status, &zero, sizeof(int)));
+  return B200Q_OK;
+}
+
+// CTAs of a launch: one per SM, but at least two K groups each (below that filling and draining the pipeline is all that a CTA does)
+static int stream_grid(long long units, int n_sm) {
+  const long long g = (units + 1) / 2, most = n_sm < (int)(COUNTER_BYTES / sizeof(unsigned)) ? n_sm : (int)(COUNTER_BYTES / sizeof(unsigned));
+  return (int)(g < most ? g : most);
+}
+
+// counters and partial sums behind the activation tiles; n_out = 0: enough for any
+static size_t split_workspace(const Plan& pl, int n_out, int kgroups, int n_sm) {
+  long long parts = 2LL * n_sm;
+  if (n_out > 0) {
+    const long long tiles = (long long)ceil_div(n_out, pl.wt) * pl.tok_tiles;
+    const int grid = stream_grid(tiles * kgroups, n_sm);
+    parts = tiles < grid ? grid + tiles : 2 * grid;
+  }
+  return COUNTER_BYTES + (size_t)parts * pl.wt * pl.nt * sizeof(float);
+}
+
+// room for the activations in tiles of 128 rows (the kernel's own tiles never take more): enough to run, tiles then going whole to the CTAs
+extern "C" size_t b200q_qgemm_workspace_bytes(int m, int n_in) {
+  if (m <= 0 || n_in <= 0) return 0;
+  return (size_t)ceil_div(m, 128) * 128 * ceil_div(n_in, GROUP_ELEMS) * GROUP_ELEMS * 4;
+}
+extern "C" size_t b200q_qgemm_workspace_bytes_for(int m, int n_out, int n_in) {
+  if (m <= 0 || n_in <= 0 || n_out < 0) return 0;
+  const int n_sm = b200q_sm_count();
+  return align256(b200q_qgemm_workspace_bytes(m, n_in)) + split_workspace(make_plan(m), n_out, ceil_div(n_in, GROUP_ELEMS), n_sm > 0 ? n_sm : 148);
+}
+
+// norm_weight (fp16 [n_in], fp32 activations only): the RMSNorm in front of the Linear, applied while the rows are split.
+extern "C" int b200q_qgemm_ws_norm(int qtype, const void* w_packed, const void* x, int x_dtype, const void* norm_weight, float norm_eps,
+                                   const void* bias_f16, const void* residual, int epilogue, void* y, int y_dtype, int m, int n_out, int n_in,
+                                   void* workspace, size_t workspace_bytes, void* stream) {
+  if (!w_packed || !x || !y || !workspace || m <= 0 || n_out <= 0 || n_in <= 0) return B200Q_ERR_BAD_ARG;
+  if (epilogue != B200Q_EPI_LINEAR && epilogue != B200Q_EPI_SILU_MUL) return B200Q_ERR_BAD_ARG;
+  if (epilogue == B200Q_EPI_SILU_MUL && (bias_f16 || residual || n_out % 16)) return B200Q_ERR_BAD_ARG;
+  if (qtype == B200Q_Q6_K) return B200Q_ERR_UNSUPPORTED;
+  if (qtype != B200Q_Q4_0 && qtype != B200Q_Q8_0) return B200Q_ERR_BAD_ARG;
+  if ((x_dtype != B200Q_F32 && x_dtype != B200Q_F16) || (y_dtype != B200Q_F32 && y_dtype != B200Q_F16)) return B200Q_ERR_BAD_ARG;
+  if (norm_weight && x_dtype != B200Q_F32) return B200Q_ERR_BAD_ARG;
+  if (n_in % 32) return B200Q_ERR_BAD_SHAPE;
+  if (((uintptr_t)w_packed | (uintptr_t)x | (uintptr_t)workspace | (uintptr_t)norm_weight) & 15) return B200Q_ERR_MISALIGNED;
+  cudaStream_t st = (cudaStream_t)stream;
+  const Plan pl = make_plan(m);
+  const bool f32 = x_dtype == B200Q_F32;
+  const int kgroups = ceil_div(n_in, GROUP_ELEMS);
+  const size_t xt_bytes = align256(tiles_bytes(pl, kgroups, f32));
+  if (workspace_bytes < tiles_bytes(pl, kgroups, f32)) return B200Q_ERR_TOO_LARGE;
+  const int n_sm = b200q_sm_count();
+  if (n_sm <= 0) return B200Q_ERR_CUDA;
+  StreamParams p;
+  p.w = (const uint8_t*)w_packed;
+  p.xt = (const unsigned char*)workspace;
+  p.counters = (unsigned*)((unsigned char*)workspace + xt_bytes);
+  p.part = (float*)((unsigned char*)workspace + xt_bytes + COUNTER_BYTES);
+  p.bias = (const __half*)bias_f16; p.residual = residual; p.y = y;
+  p.m = m; p.n_out = n_out; p.kgroups = kgroups; p.n_row_tiles = ceil_div(n_out, TILE_ROWS);
+  p.nt = pl.nt; p.tok_tiles = pl.tok_tiles;
+  p.slots = RING_BYTES / slot_bytes(pl, f32);                  // 2 (64 rows) to 3 K groups, or 3 (256 rows) to 5 steps
+  if (p.slots > MAX_SLOTS) p.slots = MAX_SLOTS;
+  p.y_f16 = y_dtype == B200Q_F16; p.silu_mul = epilogue == B200Q_EPI_SILU_MUL;
+  p.tiles = ceil_div(n_out, pl.wt) * pl.tok_tiles;
+  p.units = (long long)p.tiles * kgroups;
+  const bool split = workspace_bytes >= xt_bytes + split_workspace(pl, n_out, kgroups, n_sm);
+  p.grain = split ? 1 : kgroups;
+  const int grid = split ? stream_grid(p.units, n_sm) : (p.tiles < n_sm ? p.tiles : n_sm);
+  // one CTA of the splitting kernel: 8 rows x the whole width, or a part of it where there are few rows
+  const int row_groups = pl.tok_tiles * pl.nt / 8, n_chunks = kgroups * 16;
+  const int parts = row_groups >= n_sm ? 1 : (row_groups * 4 >= n_sm || n_chunks < 256 ? 4 : 8), per = ceil_div(n_chunks, parts);
+  const dim3 sgrid(ceil_div(n_chunks, per), row_groups);
+  if (f32) B200Q_CHECK_CUDA(launch_k(split_rows_kernel<float>, sgrid, dim3(SPLIT_THREADS), 0, st, true, (const float*)x, (const __half*)norm_weight, norm_eps, m,
+                                     n_in, kgroups, pl.nt, per, (unsigned char*)p.xt, p.counters, split ? grid : 0));
+  else B200Q_CHECK_CUDA(launch_k(split_rows_kernel<__half>, sgrid, dim3(SPLIT_THREADS), 0, st, true, (const __half*)x, (const __half*)nullptr, 0.f, m, n_in,
+                                 kgroups, pl.nt, per, (unsigned char*)p.xt, p.counters, split ? grid : 0));
+#define STREAM_CASE(QT) (pl.wt == 256 ? (f32 ? launch_stream<QT, 256, true>(p, grid, st) : launch_stream<QT, 256, false>(p, grid, st)) \
+                                      : (f32 ? launch_stream<QT, 128, true>(p, grid, st) : launch_stream<QT, 128, false>(p, grid, st)))
+  return qtype == B200Q_Q4_0 ? STREAM_CASE(B200Q_Q4_0) : STREAM_CASE(B200Q_Q8_0);
+#undef STREAM_CASE
+}
+
+extern "C" int b200q_qgemm_ws(int qtype, const void* w_packed, const void* x, int x_dtype, const void* bias_f16, const void* residual, int epilogue,
+                              void* y, int y_dtype, int m, int n_out, int n_in, void* workspace, size_t workspace_bytes, void* stream) {
+  return b200q_qgemm_ws_norm(qtype, w_packed, x, x_dtype, nullptr, 0.f, bias_f16, residual, epilogue, y, y_dtype, m, n_out, n_in, workspace,
+                             workspace_bytes, stream);
+}

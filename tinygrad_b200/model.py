@@ -346,7 +346,7 @@ class Transformer:
                       qkv=DeviceBuffer.empty((T, self.q_dim + 2 * self.kv_dim), np.float32), q16=DeviceBuffer.empty((T, self.q_dim), np.float32),
                       att=DeviceBuffer.empty((T, self.q_dim), np.float32),
                       act=DeviceBuffer.empty((T, max(c.hidden_dim, c.shared_expert_dim, 1)), np.float32),
-                      # activation tiles of the pipelined GEMM (split once per GEMM, read by every column tile's CTA)
+                      # activation tiles and partial sums of the GEMMs
                       ws=DeviceBuffer(quant.qgemm_workspace_bytes(T, max(c.dim, self.q_dim, c.hidden_dim, c.shared_expert_dim, 1))) if self.pipelined_gemm else None)
       if self.is_moe:
         self._pf.update(xb=DeviceBuffer.empty((T, c.dim), np.uint16), logits=DeviceBuffer.empty((T, c.num_experts), np.float32))
@@ -365,15 +365,19 @@ class Transformer:
       T = min(self.prefill_chunk, start_pos + n - p0)
       check(lib.b200q_embed_rows(self.token_embd.ptr, self.tokens.ptr + 4 * (seq * (c.max_context + 1) + p0), 1, None, T, c.dim,
                                  self.full_config.vocab_size, f["x"].ptr, s))
+      def normed(norm):       # the GEMM with a workspace applies the RMSNorm while it splits its activations
+        if f["ws"] is not None and quant.PIPELINED_GEMM: return f["x"], {"norm_weight": norm, "norm_eps": c.norm_eps}
+        check(lib.b200q_rmsnorm_rows(f["x"].ptr, norm.ptr, c.norm_eps, T, c.dim, f["xn"].ptr, F32, s))
+        return f["xn"], {}
       for b in self.blk:
-        check(lib.b200q_rmsnorm_rows(f["x"].ptr, b.attn_norm.ptr, c.norm_eps, T, c.dim, f["xn"].ptr, F32, s))
-        quant.qgemm(b.qkv.ptr, self.qtype, qkv_rows, c.dim, f["xn"], f["qkv"], T, x_dtype=F32, y_dtype=F32, bias=b.qkv_bias, stream=s, workspace=f["ws"])
+        xin, kw = normed(b.attn_norm)
+        quant.qgemm(b.qkv.ptr, self.qtype, qkv_rows, c.dim, xin, f["qkv"], T, x_dtype=F32, y_dtype=F32, bias=b.qkv_bias, stream=s, workspace=f["ws"], **kw)
         check(lib.b200q_attn_prefill(f["qkv"].ptr, b.k_cache.ptr + seq * self.seq_cache_bytes, b.v_cache.ptr + seq * self.seq_cache_bytes, kvdt,
                                      self.rope.ptr, p0, T, c.n_heads, c.n_kv_heads, c.head_dim,
                                      c.rope_dim, c.max_context, f["q16"].ptr, f["att"].ptr, F32, s))
         quant.qgemm(b.attn_output.buf.ptr, self.qtype, c.dim, self.q_dim, f["att"], f["x"], T, x_dtype=F32, y_dtype=F32, residual=f["x"], stream=s, workspace=f["ws"])
-        check(lib.b200q_rmsnorm_rows(f["x"].ptr, b.ffn_norm.ptr, c.norm_eps, T, c.dim, f["xn"].ptr, F32, s))
         if b.moe is not None:
+          check(lib.b200q_rmsnorm_rows(f["x"].ptr, b.ffn_norm.ptr, c.norm_eps, T, c.dim, f["xn"].ptr, F32, s))
           # router on the fp32 normed rows, experts on their bf16 rounding (the activation dtype of the MXFP8 path); bf16 result + residual
           quant.gemv_dense(b.router.buf, b.router.dtype, c.num_experts, c.dim, f["xn"], f["logits"], m=T, stream=s)
           check(lib.b200q_rmsnorm_rows(f["x"].ptr, b.ffn_norm.ptr, c.norm_eps, T, c.dim, f["xb"].ptr, _lib.BF16, s))
@@ -386,8 +390,9 @@ class Transformer:
             check(lib.b200q_add_rows_gated(f["x"].ptr, f["sh"].ptr, f["shg"].ptr if b.sh_inp is not None else None, T, c.dim, s))
           check(lib.b200q_add_rows_bf16(f["x"].ptr, y.ptr, T * c.dim, s))
           continue
-        quant.qgemm(b.gate_up.buf.ptr, self.qtype, 2 * c.hidden_dim, c.dim, f["xn"], f["act"], T, x_dtype=F32, y_dtype=F32, epilogue=EPI_SILU_MUL,
-                    stream=s, workspace=f["ws"])
+        xin, kw = normed(b.ffn_norm)
+        quant.qgemm(b.gate_up.buf.ptr, self.qtype, 2 * c.hidden_dim, c.dim, xin, f["act"], T, x_dtype=F32, y_dtype=F32, epilogue=EPI_SILU_MUL,
+                    stream=s, workspace=f["ws"], **kw)
         quant.qgemm(b.ffn_down.buf.ptr, self.qtype, c.dim, c.hidden_dim, f["act"], f["x"], T, x_dtype=F32, y_dtype=F32, residual=f["x"], stream=s, workspace=f["ws"])
     if sync:
       self.stream.synchronize()

@@ -88,22 +88,24 @@ def gemv(w_ptr: int, qtype: int, n_out: int, n_in: int, x, y, m: int = 1, x_dtyp
 
 
 import os
-PIPELINED_GEMM = os.environ.get("B200Q_PIPELINED_GEMM", "1") == "1"   # qgemm uses the pipelined kernel when it is handed a workspace
+PIPELINED_GEMM = os.environ.get("B200Q_PIPELINED_GEMM", "1") == "1"   # qgemm uses the streaming kernel when it is handed a workspace
 
 
-def qgemm_workspace_bytes(m: int, n_in: int) -> int:
-  return int(_lib.load().b200q_qgemm_workspace_bytes(m, n_in))
+def qgemm_workspace_bytes(m: int, n_in: int, n_out: int = 0) -> int:
+  """Scratch of the GEMM for m rows of n_in columns and any n_out, or (less) for the one given."""
+  return int(_lib.load().b200q_qgemm_workspace_bytes_for(m, n_out, n_in))
 
 
 def qgemm(w_ptr: int, qtype: int, n_out: int, n_in: int, x, y, m: int, x_dtype=F32, y_dtype=F32, bias=None, residual=None,
-          epilogue: int = EPI_LINEAR, stream=None, workspace: DeviceBuffer = None) -> None:
-  """Batched / prefill linear on the tcgen05 tensor cores: the weights are streamed once per 128 activation rows.  With a `workspace`
-  (qgemm_workspace_bytes(m, n_in) bytes) the pipelined kernel runs: activations pre-split once, bulk-copied operands, MMAs under the unpacking."""
+          epilogue: int = EPI_LINEAR, stream=None, workspace: DeviceBuffer = None, norm_weight=None, norm_eps: float = 0.0) -> None:
+  """Batched / prefill linear on the tcgen05 tensor cores.  With a `workspace` (qgemm_workspace_bytes(m, n_in) bytes) the streaming kernel
+  runs: activations split once (with the RMSNorm in front, if its weight is given), roles on separate warps, even deal over the SMs."""
   lib = _lib.load()
   if workspace is not None and PIPELINED_GEMM:
-    check(lib.b200q_qgemm_ws(qtype, w_ptr, ptr_of(x), x_dtype, ptr_of(bias), ptr_of(residual), epilogue, ptr_of(y), y_dtype, m, n_out, n_in,
-                             workspace.ptr, workspace.nbytes, stream_ptr(stream)))
+    check(lib.b200q_qgemm_ws_norm(qtype, w_ptr, ptr_of(x), x_dtype, ptr_of(norm_weight), norm_eps, ptr_of(bias), ptr_of(residual), epilogue, ptr_of(y), y_dtype,
+                                  m, n_out, n_in, workspace.ptr, workspace.nbytes, stream_ptr(stream)))
     return
+  assert norm_weight is None, "the RMSNorm in front is part of the kernel with a workspace"
   check(lib.b200q_qgemm(qtype, w_ptr, ptr_of(x), x_dtype, ptr_of(bias), ptr_of(residual), epilogue, ptr_of(y), y_dtype, m, n_out, n_in,
                         stream_ptr(stream)))
 
@@ -194,7 +196,7 @@ class QuantLinear:
     self.fused = ggml_type in (Q4_0, Q8_0) or (ggml_type == Q6_K and in_features % 256 == 0)
     self.weight = repack(raw, out_features, in_features, ggml_type) if self.fused else DenseWeight(raw, out_features, in_features, ggml_type)
     self.bias = None if bias is None else DeviceBuffer.from_numpy(np.asarray(bias, dtype=np.float16))
-    self._ws = None      # activation tiles of the pipelined GEMM, grown on demand
+    self._ws = None      # activation tiles and partial sums of the GEMM, grown on demand
 
   def __call__(self, x: DeviceBuffer, stream=None) -> DeviceBuffer:
     if x.dtype not in _DT: raise TypeError(f"activations must be float16 or float32, got {x.dtype}")
@@ -206,7 +208,7 @@ class QuantLinear:
       if m: gemv_dense(self.weight.buf, self.weight.dtype, self.out_features, self.in_features, x, y, m=m, x_dtype=dt, y_dtype=dt, bias=self.bias,
                        stream=stream)
     elif m >= GEMM_MIN_ROWS and self.ggml_type != Q6_K:
-      need = qgemm_workspace_bytes(m, self.in_features)
+      need = qgemm_workspace_bytes(m, self.in_features, self.out_features)
       if self._ws is None or self._ws.nbytes < need: self._ws = DeviceBuffer(need)
       qgemm(self.weight.buf.ptr, self.ggml_type, self.out_features, self.in_features, x, y, m, x_dtype=dt, y_dtype=dt, bias=self.bias, stream=stream,
             workspace=self._ws)
