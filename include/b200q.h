@@ -64,12 +64,6 @@ int b200q_set_device(int device);
 int b200q_device_props(int device, int* sm_count, int* cc_major, int* cc_minor, size_t* total_mem);
 int b200q_malloc(void** device_ptr, size_t bytes);
 int b200q_free(void* device_ptr);
-/* Device blocks for results that are allocated on every call: a freed block is handed out again once the device has been idle since it was
- * freed, so (as with b200q_free) work queued before the free may still use it, on any stream.  At most 256 MiB are kept per device;
- * b200q_pool_trim gives everything unused back. */
-int b200q_pool_alloc(void** device_ptr, size_t bytes);
-int b200q_pool_free(void* device_ptr);
-int b200q_pool_trim(void);
 int b200q_host_alloc(void** host_ptr, size_t bytes);              /* pinned host memory */
 int b200q_host_free(void* host_ptr);
 int b200q_memcpy_h2d(void* device_dst, const void* host_src, size_t bytes, void* stream);
@@ -286,10 +280,6 @@ int b200q_attn_decode_static(const b200q_attn_args* args, void* stream);
 size_t b200q_argmax_scratch_bytes(void);
 int b200q_argmax_advance(const float* device_logits, int n, int32_t* device_tokens, int32_t* device_pos, int max_context, void* scratch,
                          int flags, void* stream);
-/* The same for n_seqs sequences in one launch: logits [n_seqs, n], tokens rows token_stride apart, pos [n_seqs], scratch n_seqs x
- * b200q_argmax_scratch_bytes, zeroed once. */
-int b200q_argmax_advance_seqs(const float* logits, int n, int32_t* tokens, int token_stride, int32_t* pos, int max_context, void* scratch, int n_seqs,
-                              int flags, void* stream);
 /* *pos += 1 (a prompt token whose logits are not needed); stops at max_context like b200q_argmax_advance */
 int b200q_advance(int32_t* device_pos, int max_context, int flags, void* stream);
 
@@ -379,18 +369,6 @@ int b200q_qgemm_ws(int qtype, const void* w_packed, const void* x, int x_dtype, 
 int b200q_qgemm_ws_norm(int qtype, const void* w_packed, const void* x, int x_dtype, const void* norm_weight, float norm_eps, const void* bias_f16,
                         const void* residual, int epilogue, void* y, int y_dtype, int m, int n_out, int n_in, void* workspace, size_t workspace_bytes,
                         void* stream);
-/* `Linear.__call__` on a held weight in one call: *y = a new b200q_pool_alloc block [m, n_out] of x's type (dtype, B200Q_F32 | B200Q_F16) with
- * x [m, n_in] W^T (+ bias).  From gemm_min_rows rows on a Q4_0 / Q8_0 weight runs the GEMM in `workspace`, else the GEMV; dense weights the
- * dense GEMV. */
-typedef struct b200q_linear_desc {
-  int dense;                /* 0: w is packed (b200q_repack), w_type its GGML type; 1: row-major values, w_type B200Q_F32 | F16 | BF16 */
-  int w_type, n_out, n_in, gemm_min_rows;
-  const void* w;
-  const void* bias;         /* fp16 [n_out] or NULL */
-  void* workspace;          /* for the GEMM: b200q_qgemm_workspace_bytes_for(m, n_out, n_in) bytes */
-  size_t workspace_bytes;
-} b200q_linear_desc;
-int b200q_linear(const b200q_linear_desc* l, const void* x, int dtype, int m, void** y, void* stream);
 /* The same Linear for a few activation rows (m <= 32: batched decode), the weight-streaming shape: the operands swap roles on the
  * tensor core (weight rows = M, activation rows = N = 32), K is split over CTAs so that every layer fills the GPU, partial sums go
  * through `workspace` (b200q_qgemm_skinny_workspace_bytes) and are added in a fixed order by a second kernel that also applies
@@ -431,30 +409,6 @@ int b200q_add_rows_bf16(float* x, const void* y_bf16, int64_t n, void* stream);
 int b200q_add_rows_gated(float* x, const float* y, const float* gate_logit, int n_rows, int dim, void* stream);
 int b200q_attn_prefill(const float* qkv, void* k_cache, void* v_cache, int kv_dtype, const float* rope, int start_pos, int n_rows, int n_heads,
                        int n_kv_heads, int head_dim, int rope_dim, int max_context, void* q_scratch, void* out, int out_dtype, void* stream);
-/* The same for n_seqs sequences (caches and rows one after another), n_rows new tokens of each from start_pos on. */
-int b200q_attn_prefill_seqs(const float* qkv, void* k_cache, void* v_cache, int kv_dtype, const float* rope, int start_pos, int n_rows, int n_seqs,
-                            int n_heads, int n_kv_heads, int head_dim, int rope_dim, int max_context, void* q_scratch, void* out, int out_dtype,
-                            void* stream);
-/* n_rows tokens of each of n_seqs sequences, from position start_pos on, through the embedding and every block of a dense Q4_0 / Q8_0 model:
- * fills the KV caches, leaves the last block's rows in x (no head).  The token table is [sequences][max_context + 1]; a cache holds the
- * sequences one after another.  n_seqs * n_rows <= rows_max rows of scratch; workspace for b200q_qgemm_ws on rows_max rows of the widest
- * input. */
-typedef struct b200q_rows_args {
-  const b200q_decode_layer* layers;   /* host array [n_layers] */
-  int n_layers, qtype, dim, hidden_dim, n_heads, n_kv_heads, head_dim, rope_dim, max_context, vocab, kv_dtype, rows_max;
-  float norm_eps;
-  const void* token_embd;   /* fp16 [vocab, dim] */
-  const float* rope;        /* [max_context][rope_dim] cos || sin */
-  const int32_t* tokens;
-  float* x;                 /* [rows_max, dim] */
-  float* qkv;               /* [rows_max, q_dim + 2 kv_dim] */
-  float* q;                 /* [rows_max, q_dim] */
-  float* att;               /* [rows_max, q_dim] */
-  float* act;               /* [rows_max, hidden_dim] */
-  void* workspace;
-  size_t workspace_bytes;
-} b200q_rows_args;
-int b200q_prompt_rows(const b200q_rows_args* args, int first_seq, int n_seqs, int start_pos, int n_rows, void* stream);
 /* Batched decode (the reference's forward on tokens [B, 1], tinygrad/llm/model.py:358-364 with B > 1): row b of qkv is sequence b's
  * new token, every sequence at position pos (or *pos_dev when that device pointer is given: graph replay); caches
  * [n_seqs, n_kv_heads, max_context, head_dim]; otherwise as b200q_attn_prefill. */
@@ -532,23 +486,6 @@ int b200q_fp8_absmax(const void* x, int x_dtype, int64_t n, float* amax, void* s
 int b200q_fp8_quantize(const void* x, int x_dtype, int64_t n, const float* amax, void* q, float* factor, void* stream);
 int b200q_fp8_scale_bias(const float* acc, int64_t rows, int n, const float* factor_w, const float* factor_x, const float* bias, void* y, int y_dtype,
                          void* stream);
-/* The whole `FP8Linear.__call__` (m >= 1 rows of x, dtype B200Q_F32 | B200Q_F16; *y = a new b200q_pool_alloc block [m, n_out] of that type):
- * w_q / w_e8 / w_factor the quantised weight (unit block scales), bias fp32 [n_out] or NULL; scratch of the caller: x_q [rows_max, n_in] and
- * x_e8 [rows_max, n_in / 32] (all 127), rows_max a multiple of 256 and at least m; off int32 {0, rows_max}; parts float [592]; factor float. */
-typedef struct b200q_fp8_linear_desc {
-  int n_out, n_in, rows_max;
-  const void* w_q;
-  const void* w_e8;
-  const float* w_factor;
-  const float* bias;
-  void* x_q;
-  const void* x_e8;
-  const int32_t* off;
-  float* parts;
-  float* factor;
-} b200q_fp8_linear_desc;
-int b200q_fp8_linear(const b200q_fp8_linear_desc* l, const void* x, int dtype, int m, void** y, void* stream);
-
 
 /* ---- expert-parallel exchange over peer memory (NVLink), planned on the device ------------------------------------------
  * `dispatch` / `combine` (extra/gemm/moe_routing.py:124-131) ACROSS ranks: experts split contiguously over the ranks (rank r owns

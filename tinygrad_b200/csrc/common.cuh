@@ -26,11 +26,6 @@ struct PerDeviceFlag {
   void set(int dev) { v[dev].store(1, std::memory_order_release); }
 };
 // reads and clears the status word of the decode-step kernels (decode.cu); folded into b200q_status_read_clear
-// gives the result pool's unused blocks of a device back (pool.cu); false: there were none
-bool b200q_pool_release(int dev);
-// fp8 product with factors, bias and output type in the epilogue (mxfp8_gemm.cu)
-int b200q_mx_gemm_scaled(const void* a_q, const void* a_e8, const void* b_q, const void* b_e8, const int32_t* off, int m_total, int n, int k, void* y, int y_dtype,
-                         int rows, const float* fw, const float* fx, const float* bias, cudaStream_t st);
 int b200q_decode_status_take(int* status);
 int b200q_decode_step_status_take(int* status);   // the same for the whole-step kernel (decode_step.cu)
 int b200q_peer_status_take(int* status);          // the same for the peer-memory collectives (peer.cu)
@@ -80,15 +75,6 @@ __device__ __forceinline__ uint32_t mailbox_load(const uint32_t* p) {
   uint32_t v;
   asm volatile("ld.relaxed.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
-}
-
-// One thread of a converged warp.  A producer or MMA thread is elected, not taken as `lane == 0`: under elect.sync the compiler may use
-// uniform registers, which the tcgen05, bulk-copy and barrier instructions take their operands from.  As plain `lane == 0` code an MMA thread
-// needed 80 cycles to issue an instruction and over 300 for a barrier that was ready (many-row GEMM, 8B gate/up, 8 rows: 127 -> 90 us).
-__device__ __forceinline__ bool elect_one() {
-  uint32_t e;
-  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(e));
-  return e != 0;
 }
 
 __device__ __forceinline__ float warp_sum(float v) {
