@@ -77,6 +77,15 @@ __device__ __forceinline__ uint32_t mailbox_load(const uint32_t* p) {
   return v;
 }
 
+// One thread of a converged warp.  A producer or MMA thread is elected, not taken as `lane == 0`: under elect.sync the compiler may use
+// uniform registers, which the tcgen05, bulk-copy and barrier instructions take their operands from.  As plain `lane == 0` code an MMA thread
+// needed 80 cycles to issue an instruction and over 300 for a barrier that was ready (many-row GEMM, 8B gate/up, 8 rows: 127 -> 90 us).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(e));
+  return e != 0;
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

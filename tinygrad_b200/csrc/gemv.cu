@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
 
   if (warp == CONS_WARPS) {
     // ------------------------------ producer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       int it = 0;
       bool ok = true, x_issued = false;
       // The first NS fills need no consumer.  After them the consumers must be running, and they start only when the

@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(R_THREADS, 1) qgemv_rows_kernel(const RowsPara
   pdl_launch_dependents();
   if (warp == R_WARPS) {
     // ------------------------------ producer: weights do not depend on the previous kernel, the record does
-    if (lane == 0) {
+    if (elect_one()) {
       int it = 0;
       bool ok = true, rec_issued = false;
 #ifdef B200Q_ROWS_PROF

@@ -194,7 +194,8 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
         const uint8_t* pa = ap + kt * BK;
         const uint8_t* pb = bp + kt * BK;
 #if B200Q_MX_TMA
-        if (lt == 0) {
+        __syncwarp();
+        if (warp == EPI_WARPS && elect_one()) {
           // the 128-byte-swizzle tiled copy writes exactly the layout above (chunk c of row r at c ^ (r & 7)); no multicast
           const uint32_t fb = s32(&bar_full[slot]);
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb), "r"(A_BYTES + B_BYTES) : "memory");
@@ -231,7 +232,7 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
 #endif
   } else if (warp == EPI_WARPS + LOAD_WARPS) {
     // ---------------------------------------------------------------- MMA issue (one thread)
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t g = 0, tile_i = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, tile_i++) {

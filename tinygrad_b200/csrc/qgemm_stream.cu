@@ -142,14 +142,6 @@ __device__ __forceinline__ bool bar_wait(uint32_t sb, uint32_t bar, uint32_t par
   atomicExch(&g_tc_status, 1);
   return false;
 }
-// The copy and MMA threads are elected, not `lane == 0`: under elect.sync the compiler may use uniform registers, which the tcgen05 and
-// barrier instructions take their operands from.  As plain `lane == 0` code the MMA thread needed 80 cycles to issue an instruction and
-// over 300 for a barrier that was ready (8B gate/up, 8 rows: 127 -> 90 us).
-__device__ __forceinline__ bool elect_one() {
-  uint32_t e;
-  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(e));
-  return e != 0;
-}
 __device__ __forceinline__ void commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
