@@ -64,6 +64,12 @@ int b200q_set_device(int device);
 int b200q_device_props(int device, int* sm_count, int* cc_major, int* cc_minor, size_t* total_mem);
 int b200q_malloc(void** device_ptr, size_t bytes);
 int b200q_free(void* device_ptr);
+/* Device blocks for results that are allocated on every call: a freed block is handed out again once the device has been idle since it was
+ * freed, so (as with b200q_free) work queued before the free may still use it, on any stream.  At most 256 MiB are kept per device;
+ * b200q_pool_trim gives everything unused back. */
+int b200q_pool_alloc(void** device_ptr, size_t bytes);
+int b200q_pool_free(void* device_ptr);
+int b200q_pool_trim(void);
 int b200q_host_alloc(void** host_ptr, size_t bytes);              /* pinned host memory */
 int b200q_host_free(void* host_ptr);
 int b200q_memcpy_h2d(void* device_dst, const void* host_src, size_t bytes, void* stream);
@@ -369,6 +375,18 @@ int b200q_qgemm_ws(int qtype, const void* w_packed, const void* x, int x_dtype, 
 int b200q_qgemm_ws_norm(int qtype, const void* w_packed, const void* x, int x_dtype, const void* norm_weight, float norm_eps, const void* bias_f16,
                         const void* residual, int epilogue, void* y, int y_dtype, int m, int n_out, int n_in, void* workspace, size_t workspace_bytes,
                         void* stream);
+/* `Linear.__call__` on a held weight in one call: *y = a new b200q_pool_alloc block [m, n_out] of x's type (dtype, B200Q_F32 | B200Q_F16) with
+ * x [m, n_in] W^T (+ bias).  From gemm_min_rows rows on a Q4_0 / Q8_0 weight runs the GEMM in `workspace`, else the GEMV; dense weights the
+ * dense GEMV. */
+typedef struct b200q_linear_desc {
+  int dense;                /* 0: w is packed (b200q_repack), w_type its GGML type; 1: row-major values, w_type B200Q_F32 | F16 | BF16 */
+  int w_type, n_out, n_in, gemm_min_rows;
+  const void* w;
+  const void* bias;         /* fp16 [n_out] or NULL */
+  void* workspace;          /* for the GEMM: b200q_qgemm_workspace_bytes_for(m, n_out, n_in) bytes */
+  size_t workspace_bytes;
+} b200q_linear_desc;
+int b200q_linear(const b200q_linear_desc* l, const void* x, int dtype, int m, void** y, void* stream);
 /* The same Linear for a few activation rows (m <= 32: batched decode), the weight-streaming shape: the operands swap roles on the
  * tensor core (weight rows = M, activation rows = N = 32), K is split over CTAs so that every layer fills the GPU, partial sums go
  * through `workspace` (b200q_qgemm_skinny_workspace_bytes) and are added in a fixed order by a second kernel that also applies
@@ -486,6 +504,23 @@ int b200q_fp8_absmax(const void* x, int x_dtype, int64_t n, float* amax, void* s
 int b200q_fp8_quantize(const void* x, int x_dtype, int64_t n, const float* amax, void* q, float* factor, void* stream);
 int b200q_fp8_scale_bias(const float* acc, int64_t rows, int n, const float* factor_w, const float* factor_x, const float* bias, void* y, int y_dtype,
                          void* stream);
+/* The whole `FP8Linear.__call__` (m >= 1 rows of x, dtype B200Q_F32 | B200Q_F16; *y = a new b200q_pool_alloc block [m, n_out] of that type):
+ * w_q / w_e8 / w_factor the quantised weight (unit block scales), bias fp32 [n_out] or NULL; scratch of the caller: x_q [rows_max, n_in] and
+ * x_e8 [rows_max, n_in / 32] (all 127), rows_max a multiple of 256 and at least m; off int32 {0, rows_max}; parts float [592]; factor float. */
+typedef struct b200q_fp8_linear_desc {
+  int n_out, n_in, rows_max;
+  const void* w_q;
+  const void* w_e8;
+  const float* w_factor;
+  const float* bias;
+  void* x_q;
+  const void* x_e8;
+  const int32_t* off;
+  float* parts;
+  float* factor;
+} b200q_fp8_linear_desc;
+int b200q_fp8_linear(const b200q_fp8_linear_desc* l, const void* x, int dtype, int m, void** y, void* stream);
+
 
 /* ---- expert-parallel exchange over peer memory (NVLink), planned on the device ------------------------------------------
  * `dispatch` / `combine` (extra/gemm/moe_routing.py:124-131) ACROSS ranks: experts split contiguously over the ranks (rank r owns

@@ -48,6 +48,16 @@ class EpArgs(Structure):
               ("send_base", c_void_p), ("off_local", c_void_p), ("remote_row", c_void_p), ("scratch", c_void_p)]
 
 
+class LinearDesc(Structure):
+  _fields_ = [("dense", c_int), ("w_type", c_int), ("n_out", c_int), ("n_in", c_int), ("gemm_min_rows", c_int), ("w", c_void_p), ("bias", c_void_p),
+              ("workspace", c_void_p), ("workspace_bytes", c_size_t)]
+
+
+class Fp8LinearDesc(Structure):
+  _fields_ = [("n_out", c_int), ("n_in", c_int), ("rows_max", c_int), ("w_q", c_void_p), ("w_e8", c_void_p), ("w_factor", c_void_p), ("bias", c_void_p),
+              ("x_q", c_void_p), ("x_e8", c_void_p), ("off", c_void_p), ("parts", c_void_p), ("factor", c_void_p)]
+
+
 # name -> (restype, argtypes); every symbol include/b200q.h declares
 SIGNATURES = {
   "b200q_strerror": (c_char_p, [c_int]),
@@ -59,6 +69,11 @@ SIGNATURES = {
   "b200q_device_props": (c_int, [c_int, POINTER(c_int), POINTER(c_int), POINTER(c_int), POINTER(c_size_t)]),
   "b200q_malloc": (c_int, [POINTER(c_void_p), c_size_t]),
   "b200q_free": (c_int, [c_void_p]),
+  "b200q_pool_alloc": (c_int, [POINTER(c_void_p), c_size_t]),
+  "b200q_pool_free": (c_int, [c_void_p]),
+  "b200q_pool_trim": (c_int, []),
+  "b200q_linear": (c_int, [POINTER(LinearDesc), c_void_p, c_int, c_int, POINTER(c_void_p), c_void_p]),
+  "b200q_fp8_linear": (c_int, [POINTER(Fp8LinearDesc), c_void_p, c_int, c_int, POINTER(c_void_p), c_void_p]),
   "b200q_host_alloc": (c_int, [POINTER(c_void_p), c_size_t]),
   "b200q_host_free": (c_int, [c_void_p]),
   "b200q_memcpy_h2d": (c_int, [c_void_p, c_void_p, c_size_t, c_void_p]),

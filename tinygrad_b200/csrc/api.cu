@@ -57,7 +57,17 @@ extern "C" int b200q_device_props(int device, int* sm_count, int* cc_major, int*
   if (total_mem) *total_mem = p.totalGlobalMem;
   return B200Q_OK;
 }
-extern "C" int b200q_malloc(void** ptr, size_t bytes) { if (!ptr) return B200Q_ERR_BAD_ARG; B200Q_CHECK_CUDA(cudaMalloc(ptr, bytes ? bytes : 1)); return B200Q_OK; }
+extern "C" int b200q_malloc(void** ptr, size_t bytes) {
+  if (!ptr) return B200Q_ERR_BAD_ARG;
+  cudaError_t e = cudaMalloc(ptr, bytes ? bytes : 1);
+  if (e == cudaErrorMemoryAllocation) {          // the result pool may be holding what is missing
+    cudaGetLastError();
+    const int dev = b200q_current_device();
+    if (dev >= 0 && b200q_pool_release(dev)) e = cudaMalloc(ptr, bytes ? bytes : 1);
+  }
+  B200Q_CHECK_CUDA(e);
+  return B200Q_OK;
+}
 extern "C" int b200q_free(void* ptr) { B200Q_CHECK_CUDA(cudaFree(ptr)); return B200Q_OK; }
 extern "C" int b200q_host_alloc(void** ptr, size_t bytes) { if (!ptr) return B200Q_ERR_BAD_ARG; B200Q_CHECK_CUDA(cudaMallocHost(ptr, bytes ? bytes : 1)); return B200Q_OK; }
 extern "C" int b200q_host_free(void* ptr) { B200Q_CHECK_CUDA(cudaFreeHost(ptr)); return B200Q_OK; }

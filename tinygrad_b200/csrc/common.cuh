@@ -26,6 +26,11 @@ struct PerDeviceFlag {
   void set(int dev) { v[dev].store(1, std::memory_order_release); }
 };
 // reads and clears the status word of the decode-step kernels (decode.cu); folded into b200q_status_read_clear
+// gives the result pool's unused blocks of a device back (pool.cu); false: there were none
+bool b200q_pool_release(int dev);
+// fp8 product with factors, bias and output type in the epilogue (mxfp8_gemm.cu)
+int b200q_mx_gemm_scaled(const void* a_q, const void* a_e8, const void* b_q, const void* b_e8, const int32_t* off, int m_total, int n, int k, void* y, int y_dtype,
+                         int rows, const float* fw, const float* fx, const float* bias, cudaStream_t st);
 int b200q_decode_status_take(int* status);
 int b200q_decode_step_status_take(int* status);   // the same for the whole-step kernel (decode_step.cu)
 int b200q_peer_status_take(int* status);          // the same for the peer-memory collectives (peer.cu)

@@ -22,6 +22,7 @@
 #include "mxq.cuh"
 #include <cuda.h>
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #ifndef B200Q_MX_TMA
 #define B200Q_MX_TMA 1      // 1: the A / B tiles of a K step arrive by two tensor-map (TMA) copies; 0: by 16-byte cp.async of 128 threads
@@ -126,13 +127,16 @@ __device__ __forceinline__ void swiglu_quant_store(const uint32_t (&vg)[32], con
   act_e8[row * (f >> 5) + (col >> 5)] = e;
 }
 
+// fp32 results with the per-tensor FP8 linear's last steps: y = acc * *fw * *fx + bias in y's type, for the first `rows` rows (fw NULL: plain sums)
+struct ScaledOut { const float *fw, *fx, *bias; int rows, y_f16; };
+
 __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint8_t* __restrict__ a_q, const uint8_t* __restrict__ a_e8,
                                                                       const uint8_t* __restrict__ b_q, const uint8_t* __restrict__ b_e8,
                                                                       const int32_t* __restrict__ off, int n_experts, int m_total, int n, int k,
                                                                       __nv_bfloat16* __restrict__ c, uint8_t* __restrict__ act_q,
                                                                       uint8_t* __restrict__ act_e8, const __grid_constant__ CUtensorMap tm_a,
                                                                       const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_c,
-                                                                      int c_f32) {
+                                                                      int c_f32, const ScaledOut so) {
   extern __shared__ unsigned char sm_raw[];
   __shared__ __align__(8) uint64_t bar_full[STAGES], bar_empty[STAGES], bar_acc_full, bar_acc_empty, bar_drain;
   __shared__ uint32_t tmem_base;
@@ -150,14 +154,16 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     s_abort = 0;
   }
-  for (int i = tid; i <= n_experts; i += THREADS) s_off[i] = off[i];
   if (warp == EPI_WARPS + LOAD_WARPS) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(&tmem_base)), "r"(TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  pdl_wait();                                       // everything above runs under the previous kernel's tail
+  for (int i = tid; i <= n_experts; i += THREADS) s_off[i] = off[i];
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  pdl_launch_dependents();
   const uint32_t taddr = tmem_base;
   volatile int* abort_flag = &s_abort;
   const int kb_total = k >> 5, ktiles = k / BK;
@@ -301,6 +307,30 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       arrive(s32(&bar_acc_empty));
+      if (so.fw) {
+        const float w = *so.fw, xf = *so.fx;
+        const int col = n0 + cq * 64;
+        if (row < (size_t)so.rows) {
+          float b[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int j = 0; j < 64; j += 4) {
+            const uint32_t* v = j < 32 ? v0 + j : v1 + (j - 32);
+            if (so.bias) { const float4 b4 = __ldg(reinterpret_cast<const float4*>(so.bias + col + j)); b[0] = b4.x; b[1] = b4.y; b[2] = b4.z; b[3] = b4.w; }
+            float o[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+              o[q] = __fmul_rn(__fmul_rn(__uint_as_float(v[q]), w), xf);      // y * w_scale * x_scale, in that order
+              if (so.bias) o[q] = __fadd_rn(o[q], b[q]);
+            }
+            const size_t at = row * n + col + j;
+            if (so.y_f16) {
+              const __half2 h[2] = {__floats2half2_rn(o[0], o[1]), __floats2half2_rn(o[2], o[3])};
+              *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(c) + at) = *reinterpret_cast<const uint2*>(h);
+            } else *reinterpret_cast<float4*>(reinterpret_cast<float*>(c) + at) = make_float4(o[0], o[1], o[2], o[3]);
+          }
+        }
+        continue;
+      }
       if (c_f32) {      // unrounded sums (the per-tensor FP8 linear scales them afterwards): each thread stores its own row
         float4* o4 = reinterpret_cast<float4*>(reinterpret_cast<float*>(c) + row * n + n0 + cq * 64);
 #pragma unroll
@@ -407,7 +437,7 @@ static int make_map(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t k
 }
 
 static int grouped_launch(const void* a_q, const void* a_e8, const void* b_q, const void* b_e8, const int32_t* off, int n_experts, int m_total, int n, int k,
-                          void* c_bf16, void* act_q, void* act_e8, void* stream, bool c_f32 = false) {
+                          void* c_bf16, void* act_q, void* act_e8, void* stream, bool c_f32 = false, ScaledOut so = ScaledOut{}, bool pdl = false) {
   if (!a_q || !a_e8 || !b_q || !b_e8 || !off || (!c_bf16 && !act_q) || n_experts <= 0 || m_total <= 0 || n <= 0 || k <= 0) return B200Q_ERR_BAD_ARG;
   if (act_q && (!act_e8 || (((uintptr_t)act_q) & 15))) return B200Q_ERR_BAD_ARG;
   if (m_total % 256 || n % BN || k % BK) return B200Q_ERR_BAD_SHAPE;       // the reference asks M % 256 == N % 256 == K % 128 == 0 (moe_gemm.py:120)
@@ -432,10 +462,15 @@ static int grouped_launch(const void* a_q, const void* a_e8, const void* b_q, co
   if (rc == B200Q_OK) rc = make_map(&tm_b, b_q, (uint64_t)n_experts * n, (uint64_t)k, BN);
   if (rc != B200Q_OK) return rc;
 #endif
-  grouped_mxfp8_tc_kernel<<<grid, THREADS, SMEM_BYTES, (cudaStream_t)stream>>>((const uint8_t*)a_q, (const uint8_t*)a_e8, (const uint8_t*)b_q, (const uint8_t*)b_e8, off,
-                                                            n_experts, m_total, n, k, (__nv_bfloat16*)c_bf16, (uint8_t*)act_q, (uint8_t*)act_e8, tm_a, tm_b, tm_c, c_f32 ? 1 : 0);
-  B200Q_CHECK_CUDA(cudaGetLastError());
+  B200Q_CHECK_CUDA(launch_k(grouped_mxfp8_tc_kernel, dim3(grid), dim3(THREADS), (size_t)SMEM_BYTES, (cudaStream_t)stream, pdl, (const uint8_t*)a_q, (const uint8_t*)a_e8,
+                            (const uint8_t*)b_q, (const uint8_t*)b_e8, off, n_experts, m_total, n, k, (__nv_bfloat16*)c_bf16, (uint8_t*)act_q, (uint8_t*)act_e8,
+                            tm_a, tm_b, tm_c, c_f32 ? 1 : 0, so));
   return B200Q_OK;
+}
+
+int b200q_mx_gemm_scaled(const void* a_q, const void* a_e8, const void* b_q, const void* b_e8, const int32_t* off, int m_total, int n, int k, void* y, int y_dtype,
+                         int rows, const float* fw, const float* fx, const float* bias, cudaStream_t st) {
+  return grouped_launch(a_q, a_e8, b_q, b_e8, off, 1, m_total, n, k, y, nullptr, nullptr, st, true, ScaledOut{fw, fx, bias, rows, y_dtype == B200Q_F16}, true);
 }
 
 extern "C" int b200q_grouped_mxfp8_gemm(const void* a_q, const void* a_e8, const void* b_q, const void* b_e8, const int32_t* off, int n_experts,

@@ -1,6 +1,7 @@
 """`FP8Linear` of extra/fp8/fp8_linear.py:43-63 on the B200 path: per-tensor E4M3 quantisation of weight and activations, the product on
 the tcgen05 tensor cores with fp32 accumulation, the two scale factors and the bias applied afterwards.  Inference only: the weight is
 quantised once (the reference re-quantises it on every call because it trains it); call `requantize()` after changing `weight`."""
+import ctypes, math
 import numpy as np
 from . import _lib
 from ._lib import check, F32, F16, BF16
@@ -35,26 +36,27 @@ class FP8Linear:
     self.w_q, self.w_factor = quantize_to_fp8(self.weight, self.out_features * self.in_features, F32)
 
   def _workspace(self, m: int):
+    mp = -(-m // 256) * 256
     w = self._ws.get(m)
     if w is None:
-      lib, mp = _lib.load(), -(-m // 256) * 256
-      w = dict(mp=mp, x_q=DeviceBuffer.empty((mp, self.in_features), np.uint8, zero=True), x_e8=DeviceBuffer(mp * self.in_features // 32),
-               amax=DeviceBuffer.empty((1,), np.float32), factor=DeviceBuffer.empty((1,), np.float32), off=DeviceBuffer.from_numpy(np.array([0, mp], np.int32)),
-               acc=DeviceBuffer.empty((mp, self.out_features), np.float32))
+      lib = _lib.load()
+      w = dict(x_q=DeviceBuffer.empty((mp, self.in_features), np.uint8, zero=True), x_e8=DeviceBuffer(mp * self.in_features // 32),
+               off=DeviceBuffer.from_numpy(np.array([0, mp], np.int32)), parts=DeviceBuffer.empty((592,), np.float32), factor=DeviceBuffer.empty((1,), np.float32))
       check(lib.b200q_memset(w["x_e8"].ptr, 127, w["x_e8"].nbytes, None))
+      check(lib.b200q_device_synchronize())
+      w["desc"] = _lib.Fp8LinearDesc(self.out_features, self.in_features, mp, None, self._w_e8.ptr, None, self.bias.ptr if self.bias else None, w["x_q"].ptr,
+                                     w["x_e8"].ptr, w["off"].ptr, w["parts"].ptr, w["factor"].ptr)
       self._ws[m] = w
-    return w
+    return w["desc"]
 
   def __call__(self, x: DeviceBuffer, stream=None) -> DeviceBuffer:
-    if x.dtype not in _DT: raise TypeError(f"activations must be float16 or float32, got {x.dtype}")
-    if x.shape[-1] != self.in_features: raise ValueError(f"Input Tensor shapes {x.shape} cannot be multiplied with in_features={self.in_features}")
-    m = int(np.prod(x.shape[:-1], dtype=np.int64))
-    y = DeviceBuffer.empty((*x.shape[:-1], self.out_features), x.dtype)
-    if m == 0: return y
-    lib, s, dt, w = _lib.load(), stream_ptr(stream), _DT[x.dtype], self._workspace(m)
-    check(lib.b200q_fp8_absmax(x.ptr, dt, m * self.in_features, w["amax"].ptr, s))
-    check(lib.b200q_fp8_quantize(x.ptr, dt, m * self.in_features, w["amax"].ptr, w["x_q"].ptr, w["factor"].ptr, s))      # rows past m stay zero
-    check(lib.b200q_grouped_mxfp8_gemm_f32(w["x_q"].ptr, w["x_e8"].ptr, self.w_q.ptr, self._w_e8.ptr, w["off"].ptr, 1, w["mp"], self.out_features,
-                                           self.in_features, w["acc"].ptr, s))
-    check(lib.b200q_fp8_scale_bias(w["acc"].ptr, m, self.out_features, self.w_factor.ptr, w["factor"].ptr, self.bias.ptr if self.bias else None, y.ptr, dt, s))
-    return y
+    dt = _DT.get(x.dtype)
+    if dt is None: raise TypeError(f"activations must be float16 or float32, got {x.dtype}")
+    *lead, k = x.shape
+    if k != self.in_features: raise ValueError(f"Input Tensor shapes {x.shape} cannot be multiplied with in_features={self.in_features}")
+    m, shape = math.prod(lead), (*lead, self.out_features)
+    if m == 0: return DeviceBuffer.empty(shape, x.dtype)
+    d, y = self._workspace(m), ctypes.c_void_p()
+    d.w_q, d.w_factor = self.w_q.ptr, self.w_factor.ptr
+    check(_lib.load().b200q_fp8_linear(ctypes.byref(d), x.ptr, dt, m, ctypes.byref(y), stream_ptr(stream)))
+    return DeviceBuffer.adopt(y.value, m * self.out_features * x.dtype.itemsize, shape, x.dtype)

@@ -6,7 +6,7 @@ Host-side mirror of the reference's interface for this path: `dequantize` is
 argument meaning, same output dtype rule (the activation's dtype), errors raised
 as exceptions.  All compute happens in libb200q.so.
 """
-import ctypes
+import ctypes, math, threading
 import numpy as np
 from . import _lib
 from ._lib import check, Q4_0, Q8_0, Q6_K, F32, F16, EPI_LINEAR, EPI_SILU_MUL, FLAG_PDL
@@ -25,7 +25,7 @@ def dequantize(raw, n: int, ggml_type: int, dtype=np.float32, stream=None) -> De
   """Raw GGUF block bytes -> n values (fp32 bit-exact with the reference; fp16 = its RNE cast)."""
   if ggml_type not in GGML_QUANT: raise ValueError(f"GGML type '{ggml_type}' is not supported!")   # gguf.py:119
   raw = _as_device(raw)
-  out = DeviceBuffer.empty((n,), dtype)
+  out = DeviceBuffer.result((n,), dtype)
   check(_lib.load().b200q_dequant_raw(ggml_type, raw.ptr, out.ptr, n, _DT[np.dtype(dtype)], stream_ptr(stream)))
   return out
 
@@ -197,21 +197,23 @@ class QuantLinear:
     self.weight = repack(raw, out_features, in_features, ggml_type) if self.fused else DenseWeight(raw, out_features, in_features, ggml_type)
     self.bias = None if bias is None else DeviceBuffer.from_numpy(np.asarray(bias, dtype=np.float16))
     self._ws = None      # activation tiles and partial sums of the GEMM, grown on demand
+    w = self.weight.buf
+    self._desc = _lib.LinearDesc(not self.fused, ggml_type if self.fused else self.weight.dtype, out_features, in_features, 0, w.ptr,
+                                 self.bias.ptr if self.bias else None, None, 0)
+    self._desc_ref, self._lock = ctypes.byref(self._desc), threading.Lock()
 
   def __call__(self, x: DeviceBuffer, stream=None) -> DeviceBuffer:
-    if x.dtype not in _DT: raise TypeError(f"activations must be float16 or float32, got {x.dtype}")
-    if x.shape[-1] != self.in_features: raise ValueError(f"Input Tensor shapes {x.shape} cannot be multiplied with in_features={self.in_features}")
-    m = int(np.prod(x.shape[:-1], dtype=np.int64))
-    y = DeviceBuffer.empty((*x.shape[:-1], self.out_features), x.dtype)
-    dt = _DT[x.dtype]
-    if not self.fused:
-      if m: gemv_dense(self.weight.buf, self.weight.dtype, self.out_features, self.in_features, x, y, m=m, x_dtype=dt, y_dtype=dt, bias=self.bias,
-                       stream=stream)
-    elif m >= GEMM_MIN_ROWS and self.ggml_type != Q6_K:
-      need = qgemm_workspace_bytes(m, self.in_features, self.out_features)
-      if self._ws is None or self._ws.nbytes < need: self._ws = DeviceBuffer(need)
-      qgemm(self.weight.buf.ptr, self.ggml_type, self.out_features, self.in_features, x, y, m, x_dtype=dt, y_dtype=dt, bias=self.bias, stream=stream,
-            workspace=self._ws)
-    elif m:
-      gemv(self.weight.buf.ptr, self.ggml_type, self.out_features, self.in_features, x, y, m=m, x_dtype=dt, y_dtype=dt, bias=self.bias, stream=stream)
-    return y
+    dt = _DT.get(x.dtype)
+    if dt is None: raise TypeError(f"activations must be float16 or float32, got {x.dtype}")
+    *lead, k = x.shape
+    if k != self.in_features: raise ValueError(f"Input Tensor shapes {x.shape} cannot be multiplied with in_features={self.in_features}")
+    m, d, y = math.prod(lead), self._desc, ctypes.c_void_p()
+    with self._lock:       # the workspace and the descriptor are this object's
+      d.gemm_min_rows = GEMM_MIN_ROWS
+      if self.fused and m >= GEMM_MIN_ROWS and self.ggml_type != Q6_K:
+        need = qgemm_workspace_bytes(m, self.in_features, self.out_features)
+        if self._ws is None or self._ws.nbytes < need:
+          self._ws = DeviceBuffer(need)
+          d.workspace, d.workspace_bytes = self._ws.ptr, need
+      check(_lib.load().b200q_linear(self._desc_ref, ptr_of(x), dt, m, ctypes.byref(y), stream_ptr(stream)))
+    return DeviceBuffer.adopt(y.value, m * self.out_features * x.dtype.itemsize, (*lead, self.out_features), x.dtype)

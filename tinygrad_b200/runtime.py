@@ -5,7 +5,7 @@ the Python host code and libb200q.so.  A caller that already owns device memory
 (a tinygrad Tensor's `Buffer._buf`, any object with `data_ptr()`) can pass raw
 addresses to the ops instead; see `ptr_of`.
 """
-import ctypes
+import ctypes, math
 import numpy as np
 from . import _lib
 from ._lib import check
@@ -24,6 +24,8 @@ def ptr_of(obj) -> int:
 
 class DeviceBuffer:
   """Owning device allocation with an optional (shape, dtype) view for copies to numpy."""
+  pooled = False       # True: a block of the result pool (b200q_pool_alloc), which `free` hands back to it
+
   def __init__(self, nbytes: int, shape=None, dtype=None, zero: bool = False):
     p = ctypes.c_void_p()
     check(_lib.load().b200q_malloc(ctypes.byref(p), nbytes))
@@ -34,6 +36,21 @@ class DeviceBuffer:
   def empty(shape, dtype, zero: bool = False) -> "DeviceBuffer":
     shape = (shape,) if isinstance(shape, int) else tuple(shape)
     return DeviceBuffer(int(np.prod(shape, dtype=np.int64)) * np.dtype(dtype).itemsize, shape, dtype, zero)
+
+  @staticmethod
+  def adopt(ptr: int, nbytes: int, shape: tuple, dtype: np.dtype) -> "DeviceBuffer":
+    """A result-pool block that the library has allocated."""
+    b = DeviceBuffer.__new__(DeviceBuffer)
+    b.ptr, b.nbytes, b.shape, b.dtype, b.pooled = ptr, nbytes, shape, dtype, True
+    return b
+
+  @staticmethod
+  def result(shape: tuple, dtype) -> "DeviceBuffer":
+    """Uninitialised memory for a result, from the result pool: for outputs that are made anew on every call."""
+    dtype = np.dtype(dtype)
+    nbytes, p = math.prod(shape) * dtype.itemsize, ctypes.c_void_p()
+    check(_lib.load().b200q_pool_alloc(ctypes.byref(p), nbytes))
+    return DeviceBuffer.adopt(p.value, nbytes, shape, dtype)
 
   @staticmethod
   def from_numpy(a: np.ndarray) -> "DeviceBuffer":
@@ -63,7 +80,7 @@ class DeviceBuffer:
 
   def free(self) -> None:
     if self.ptr:
-      _lib.load().b200q_free(self.ptr)
+      (_lib.load().b200q_pool_free if self.pooled else _lib.load().b200q_free)(self.ptr)
       self.ptr = 0
 
   def __del__(self):
