@@ -7,7 +7,7 @@
 // cudaFree's own guarantee is kept: a block is handed out again only after the device has been seen idle (one cudaDeviceSynchronize) at some
 // time after it was freed.  Freed blocks wait in a list; when the list holds PENDING_BLOCKS blocks or PENDING_BYTES, the next allocation
 // waits for the device once and turns the whole list into free blocks.  So a loop of calls waits once per 64 results (or 64 MiB) instead of
-// once per result.  Bounded: at most POOL_BYTES are kept per device (past that a block goes back with cudaFree), larger blocks than
+// once per result.  Bounded: at most POOL_BYTES are kept per device (past that everything unused goes back with cudaFree), larger blocks than
 // BLOCK_MAX never enter, and everything goes back when an allocation fails or b200q_pool_trim is called.  One lock; any thread may call.
 #include "common.cuh"
 #include <mutex>
@@ -16,7 +16,7 @@
 
 namespace {
 
-constexpr size_t BLOCK_MAX = (size_t)64 << 20, POOL_BYTES = (size_t)256 << 20, PENDING_BYTES = (size_t)64 << 20;
+constexpr size_t BLOCK_MAX = (size_t)32 << 20, POOL_BYTES = (size_t)256 << 20, PENDING_BYTES = (size_t)64 << 20;
 constexpr size_t PENDING_BLOCKS = 64;
 
 struct Block { void* p; size_t size; };
@@ -104,7 +104,8 @@ extern "C" int b200q_pool_free(void* device_ptr) {
   const size_t size = it->second.second;
   g_out.erase(it);
   DevicePool& d = g_pool[dev];
-  if (size && d.kept + size <= POOL_BYTES) {
+  if (size) {
+    if (d.kept + size > POOL_BYTES) give_back(d);              // full of blocks that nobody has asked for lately
     d.pending.push_back({device_ptr, size});
     d.pending_bytes += size;
     d.kept += size;
