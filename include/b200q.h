@@ -286,6 +286,10 @@ int b200q_attn_decode_static(const b200q_attn_args* args, void* stream);
 size_t b200q_argmax_scratch_bytes(void);
 int b200q_argmax_advance(const float* device_logits, int n, int32_t* device_tokens, int32_t* device_pos, int max_context, void* scratch,
                          int flags, void* stream);
+/* The same for n_seqs sequences in one launch: logits [n_seqs, n], tokens rows token_stride apart, pos [n_seqs], scratch n_seqs x
+ * b200q_argmax_scratch_bytes, zeroed once. */
+int b200q_argmax_advance_seqs(const float* logits, int n, int32_t* tokens, int token_stride, int32_t* pos, int max_context, void* scratch, int n_seqs,
+                              int flags, void* stream);
 /* *pos += 1 (a prompt token whose logits are not needed); stops at max_context like b200q_argmax_advance */
 int b200q_advance(int32_t* device_pos, int max_context, int flags, void* stream);
 
@@ -367,14 +371,15 @@ int b200q_qgemm(int qtype, const void* w_packed, const void* x, int x_dtype, con
  * b200q_qgemm_workspace_bytes_for(m, n_out, n_in) (n_out = 0: for any) tiles may also be split along K, which deals the work evenly over the
  * SMs; their partial sums are added in the order of K, so the result does not depend on timing.  Same arguments, same numerics (the order
  * of the fp32 additions aside), same epilogues.  Two launches.  b200q_qgemm_ws_norm (fp32 x): norm_weight fp16 [n_in], the RMSNorm in
- * front of the Linear, applied while x is split (NULL: none). */
+ * front of the Linear, applied while x is split (NULL: none); unsplit != 0: tiles are never split, every output is one running sum with the bits of
+ * b200q_qgemm. */
 size_t b200q_qgemm_workspace_bytes(int m, int n_in);
 size_t b200q_qgemm_workspace_bytes_for(int m, int n_out, int n_in);
 int b200q_qgemm_ws(int qtype, const void* w_packed, const void* x, int x_dtype, const void* bias_f16, const void* residual, int epilogue, void* y,
                    int y_dtype, int m, int n_out, int n_in, void* workspace, size_t workspace_bytes, void* stream);
 int b200q_qgemm_ws_norm(int qtype, const void* w_packed, const void* x, int x_dtype, const void* norm_weight, float norm_eps, const void* bias_f16,
                         const void* residual, int epilogue, void* y, int y_dtype, int m, int n_out, int n_in, void* workspace, size_t workspace_bytes,
-                        void* stream);
+                        int unsplit, void* stream);
 /* `Linear.__call__` on a held weight in one call: *y = a new b200q_pool_alloc block [m, n_out] of x's type (dtype, B200Q_F32 | B200Q_F16) with
  * x [m, n_in] W^T (+ bias).  From gemm_min_rows rows on a Q4_0 / Q8_0 weight runs the GEMM in `workspace`, else the GEMV; dense weights the
  * dense GEMV. */
@@ -427,6 +432,30 @@ int b200q_add_rows_bf16(float* x, const void* y_bf16, int64_t n, void* stream);
 int b200q_add_rows_gated(float* x, const float* y, const float* gate_logit, int n_rows, int dim, void* stream);
 int b200q_attn_prefill(const float* qkv, void* k_cache, void* v_cache, int kv_dtype, const float* rope, int start_pos, int n_rows, int n_heads,
                        int n_kv_heads, int head_dim, int rope_dim, int max_context, void* q_scratch, void* out, int out_dtype, void* stream);
+/* The same for n_seqs sequences (caches and rows one after another), n_rows new tokens of each from start_pos on. */
+int b200q_attn_prefill_seqs(const float* qkv, void* k_cache, void* v_cache, int kv_dtype, const float* rope, int start_pos, int n_rows, int n_seqs,
+                            int n_heads, int n_kv_heads, int head_dim, int rope_dim, int max_context, void* q_scratch, void* out, int out_dtype,
+                            void* stream);
+/* n_rows tokens of each of n_seqs sequences, from position start_pos on, through the embedding and every block of a dense Q4_0 / Q8_0 model:
+ * fills the KV caches, leaves the last block's rows in x (no head).  The token table is [sequences][max_context + 1]; a cache holds the
+ * sequences one after another.  n_seqs * n_rows <= rows_max rows of scratch; workspace for b200q_qgemm_ws on rows_max rows of the widest
+ * input. */
+typedef struct b200q_rows_args {
+  const b200q_decode_layer* layers;   /* host array [n_layers] */
+  int n_layers, qtype, dim, hidden_dim, n_heads, n_kv_heads, head_dim, rope_dim, max_context, vocab, kv_dtype, rows_max;
+  float norm_eps;
+  const void* token_embd;   /* fp16 [vocab, dim] */
+  const float* rope;        /* [max_context][rope_dim] cos || sin */
+  const int32_t* tokens;
+  float* x;                 /* [rows_max, dim] */
+  float* qkv;               /* [rows_max, q_dim + 2 kv_dim] */
+  float* q;                 /* [rows_max, q_dim] */
+  float* att;               /* [rows_max, q_dim] */
+  float* act;               /* [rows_max, hidden_dim] */
+  void* workspace;
+  size_t workspace_bytes;
+} b200q_rows_args;
+int b200q_prompt_rows(const b200q_rows_args* args, int first_seq, int n_seqs, int start_pos, int n_rows, void* stream);
 /* Batched decode (the reference's forward on tokens [B, 1], tinygrad/llm/model.py:358-364 with B > 1): row b of qkv is sequence b's
  * new token, every sequence at position pos (or *pos_dev when that device pointer is given: graph replay); caches
  * [n_seqs, n_kv_heads, max_context, head_dim]; otherwise as b200q_attn_prefill. */

@@ -38,6 +38,16 @@ def test_rows_against_the_exact_product(typ, m, n_out, n_in, dt, split):
   assert (np.abs(y.numpy() - ref) <= bound).all(), f"worst {np.max(np.abs(y.numpy() - ref) / bound):.2f} of the bound"
 
 
+@pytest.mark.parametrize("typ,m,n_out,n_in", [(2, 1, 64, 32), (8, 1, 1536, 1024), (8, 52, 130, 128), (2, 200, 512, 992)])
+def test_unsplit_sums_have_the_bits_of_the_kernel_without_a_workspace(typ, m, n_out, n_in):
+  rng = np.random.default_rng(m)
+  pw, x = quant.repack(synth.BLOCK_MAKERS[typ](n_out, n_in, rng), n_out, n_in, typ), DeviceBuffer.from_numpy(rng.standard_normal((m, n_in)).astype(np.float32))
+  a, b, ws = DeviceBuffer.empty((m, n_out), np.float32), DeviceBuffer.empty((m, n_out), np.float32), DeviceBuffer(quant.qgemm_workspace_bytes(m, n_in))
+  quant.qgemm(pw.buf.ptr, typ, n_out, n_in, x, a, m)
+  quant.qgemm(pw.buf.ptr, typ, n_out, n_in, x, b, m, workspace=ws, unsplit=True)
+  np.testing.assert_array_equal(a.numpy(), b.numpy())
+
+
 def test_norm_in_front_and_swiglu_behind():
   m, hidden, dim = 45, 1408, 512
   rng = np.random.default_rng(4)

@@ -48,6 +48,13 @@ class EpArgs(Structure):
               ("send_base", c_void_p), ("off_local", c_void_p), ("remote_row", c_void_p), ("scratch", c_void_p)]
 
 
+class RowsArgs(Structure):
+  _fields_ = [("layers", POINTER(DecodeLayer)), ("n_layers", c_int), ("qtype", c_int), ("dim", c_int), ("hidden_dim", c_int), ("n_heads", c_int),
+              ("n_kv_heads", c_int), ("head_dim", c_int), ("rope_dim", c_int), ("max_context", c_int), ("vocab", c_int), ("kv_dtype", c_int), ("rows_max", c_int),
+              ("norm_eps", c_float), ("token_embd", c_void_p), ("rope", c_void_p), ("tokens", c_void_p), ("x", c_void_p), ("qkv", c_void_p), ("q", c_void_p),
+              ("att", c_void_p), ("act", c_void_p), ("workspace", c_void_p), ("workspace_bytes", c_size_t)]
+
+
 class LinearDesc(Structure):
   _fields_ = [("dense", c_int), ("w_type", c_int), ("n_out", c_int), ("n_in", c_int), ("gemm_min_rows", c_int), ("w", c_void_p), ("bias", c_void_p),
               ("workspace", c_void_p), ("workspace_bytes", c_size_t)]
@@ -124,13 +131,17 @@ SIGNATURES = {
   "b200q_decode_step": (c_int, [POINTER(DecodeStepArgs), c_void_p]),
   "b200q_argmax_scratch_bytes": (c_size_t, []),
   "b200q_argmax_advance": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p]),
+  "b200q_argmax_advance_seqs": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p]),
+  "b200q_prompt_rows": (c_int, [POINTER(RowsArgs), c_int, c_int, c_int, c_int, c_void_p]),
+  "b200q_attn_prefill_seqs": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
+                                      c_int, c_void_p]),
   "b200q_advance": (c_int, [c_void_p, c_int, c_int, c_void_p]),
   "b200q_gemm_f16": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
   "b200q_qgemm": (c_int, [c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
   "b200q_qgemm_workspace_bytes": (c_size_t, [c_int, c_int]),
   "b200q_qgemm_workspace_bytes_for": (c_size_t, [c_int, c_int, c_int]),
   "b200q_qgemm_ws_norm": (c_int, [c_int, c_void_p, c_void_p, c_int, c_void_p, c_float, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p,
-                                 c_size_t, c_void_p]),
+                                 c_size_t, c_int, c_void_p]),
   "b200q_qgemm_ws": (c_int, [c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),
   "b200q_qgemv_rows_workspace_bytes": (c_size_t, [c_int, c_int, c_int]),
   "b200q_qgemv_rows": (c_int, [c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_size_t,

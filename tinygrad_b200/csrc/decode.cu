@@ -374,16 +374,22 @@ namespace {
 // scratch: float val[ARGMAX_CTAS], int idx[ARGMAX_CTAS], uint counter.
 constexpr int ARGMAX_CTAS = 128;
 constexpr int ARGMAX_THREADS = 256;
+constexpr size_t ARGMAX_SCRATCH = ARGMAX_CTAS * (sizeof(float) + sizeof(int)) + sizeof(unsigned);
 
 __device__ __forceinline__ void argmax_combine(float& v, int& i, float ov, int oi) {
   if (ov > v || (ov == v && oi < i)) { v = ov; i = oi; }
 }
 
 __global__ void __launch_bounds__(ARGMAX_THREADS) argmax_kernel(const float* __restrict__ logits, int n, int32_t* tokens, int32_t* pos,
-                                                                int max_context, float* sval, int* sidx, unsigned* counter) {
+                                                                int max_context, int token_stride, unsigned char* scratch) {
   __shared__ float wv[ARGMAX_THREADS / 32];
   __shared__ int wi[ARGMAX_THREADS / 32];
   __shared__ int s_last;
+  // blockIdx.y: the sequence
+  logits += (size_t)blockIdx.y * n; tokens += (size_t)blockIdx.y * token_stride; pos += blockIdx.y;
+  float* sval = reinterpret_cast<float*>(scratch + (size_t)blockIdx.y * ARGMAX_SCRATCH);
+  int* sidx = reinterpret_cast<int*>(sval + ARGMAX_CTAS);
+  unsigned* counter = reinterpret_cast<unsigned*>(sidx + ARGMAX_CTAS);
   pdl_launch_dependents();
   pdl_wait();
   float v = -INFINITY; int idx = 0x7fffffff;
@@ -520,15 +526,18 @@ extern "C" int b200q_attn_decode_seqs(const b200q_attn_args* a, int n_seqs, void
   return attn_decode_launch(a, n_seqs, stream);
 }
 
-extern "C" size_t b200q_argmax_scratch_bytes(void) { return ARGMAX_CTAS * (sizeof(float) + sizeof(int)) + sizeof(unsigned); }
+extern "C" size_t b200q_argmax_scratch_bytes(void) { return ARGMAX_SCRATCH; }
 
-extern "C" int b200q_argmax_advance(const float* logits, int n, int32_t* tokens, int32_t* pos, int max_context, void* scratch, int flags, void* stream) {
-  if (!logits || !tokens || !pos || !scratch || n <= 0 || max_context <= 0) return B200Q_ERR_BAD_ARG;
-  float* sval = (float*)scratch; int* sidx = (int*)(sval + ARGMAX_CTAS); unsigned* counter = (unsigned*)(sidx + ARGMAX_CTAS);
+extern "C" int b200q_argmax_advance_seqs(const float* logits, int n, int32_t* tokens, int token_stride, int32_t* pos, int max_context, void* scratch, int n_seqs,
+                                         int flags, void* stream) {
+  if (!logits || !tokens || !pos || !scratch || n <= 0 || max_context <= 0 || n_seqs <= 0 || n_seqs > 65535 || token_stride < 0) return B200Q_ERR_BAD_ARG;
   int grid = ceil_div(n, ARGMAX_THREADS); if (grid > ARGMAX_CTAS) grid = ARGMAX_CTAS;
-  B200Q_CHECK_CUDA(launch_k(argmax_kernel, dim3(grid), dim3(ARGMAX_THREADS), 0, (cudaStream_t)stream, (flags & B200Q_FLAG_PDL) != 0,
-                            logits, n, tokens, pos, max_context, sval, sidx, counter));
+  B200Q_CHECK_CUDA(launch_k(argmax_kernel, dim3(grid, n_seqs), dim3(ARGMAX_THREADS), 0, (cudaStream_t)stream, (flags & B200Q_FLAG_PDL) != 0,
+                            logits, n, tokens, pos, max_context, token_stride, (unsigned char*)scratch));
   return B200Q_OK;
+}
+extern "C" int b200q_argmax_advance(const float* logits, int n, int32_t* tokens, int32_t* pos, int max_context, void* scratch, int flags, void* stream) {
+  return b200q_argmax_advance_seqs(logits, n, tokens, 0, pos, max_context, scratch, 1, flags, stream);
 }
 
 // ---------------------------------------------------------------------------

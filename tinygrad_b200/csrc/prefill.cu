@@ -13,9 +13,11 @@
 namespace {
 
 __global__ void embed_rows_kernel(const __half* __restrict__ table, const int32_t* __restrict__ tokens, int token_stride, const int32_t* __restrict__ pos_dev,
-                                  int n_rows, int dim, int vocab, float* __restrict__ x) {
-  const int t = blockIdx.x;
-  int tok = tokens[(size_t)t * token_stride + (pos_dev ? *pos_dev : 0)];
+                                  int per_seq, int dim, int vocab, float* __restrict__ x) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int t = blockIdx.x, seq = t / per_seq;           // row t: token t % per_seq of sequence t / per_seq
+  int tok = tokens[(size_t)seq * token_stride + (t - seq * per_seq) + (pos_dev ? *pos_dev : 0)];
   tok = min(max(tok, 0), vocab - 1);
   const __half2* src = reinterpret_cast<const __half2*>(table + (size_t)tok * dim);
   float2* dst = reinterpret_cast<float2*>(x + (size_t)t * dim);
@@ -61,12 +63,14 @@ template <> __device__ __forceinline__ float kv_cast<float>(float v) { return v;
 // qkv [T][(n_heads + 2 n_kv) * hd] fp32 -> q_out [T][n_heads * hd] fp32 (rotated), cache rows start_pos + t
 template <typename KV>
 __global__ void rope_kv_rows_kernel(const float* __restrict__ qkv, const float* __restrict__ rope, int start_pos, int n_heads, int n_kv, int hd,
-                                    int rope_dim, int max_context, KV* __restrict__ k_cache, KV* __restrict__ v_cache, float* __restrict__ q_out, int batch,
+                                    int rope_dim, int max_context, KV* __restrict__ k_cache, KV* __restrict__ v_cache, float* __restrict__ q_out, int per_seq,
                                     const int32_t* __restrict__ pos_dev) {
+  pdl_wait();
+  pdl_launch_dependents();
   if (pos_dev) start_pos = min(max(*pos_dev, 0), max_context - 1);      // position kept on the device (graph replay)
-  // batch = 0: row t is the token at position start_pos + t of one sequence; batch = 1: row t is sequence t's token at start_pos
-  const int t = blockIdx.x, pos = start_pos + (batch ? 0 : t), half_r = rope_dim >> 1;
-  if (batch) { k_cache += (size_t)t * n_kv * max_context * hd; v_cache += (size_t)t * n_kv * max_context * hd; }
+  // row t is the token at position start_pos + t % per_seq of sequence t / per_seq
+  const int t = blockIdx.x, seq = t / per_seq, pos = start_pos + t - seq * per_seq, half_r = rope_dim >> 1;
+  k_cache += (size_t)seq * n_kv * max_context * hd; v_cache += (size_t)seq * n_kv * max_context * hd;
   const int row = (n_heads + 2 * n_kv) * hd;
   const float* src = qkv + (size_t)t * row;
   const float* rp = rope + (size_t)pos * rope_dim;
@@ -105,23 +109,28 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
 template <int HD, typename KV, typename O>
 __global__ void __launch_bounds__(PF_THREADS) attn_prefill_kernel(const float* __restrict__ q, const KV* __restrict__ k_cache, const KV* __restrict__ v_cache,
                                                                   int start_pos, int n_rows, int n_heads, int n_kv, int max_context,
-                                                                  O* __restrict__ out, int batch, const int32_t* __restrict__ pos_dev) {
+                                                                  O* __restrict__ out, const int32_t* __restrict__ pos_dev) {
+  pdl_wait();
+  pdl_launch_dependents();
   if (pos_dev) start_pos = min(max(*pos_dev, 0), max_context - 1);
   constexpr int STRIDE = HD + 8;                         // halves per shared row: 32-bit fragment loads hit distinct banks
   extern __shared__ __align__(16) unsigned char psm[];
   __half* s_q = reinterpret_cast<__half*>(psm);          // [2][PQ][STRIDE]: fp16 high and low halves of the fp32 queries
   __half* s_k = s_q + 2 * PQ * STRIDE;                   // [PK][STRIDE]
   __half* s_v = s_k + PK * STRIDE;                       // [PK][STRIDE]
-  // batch = 1 (one new token per sequence, all at start_pos): the CTA serves row blockIdx.y alone, on that sequence's cache
-  const int head = blockIdx.x, q0 = batch ? blockIdx.y : blockIdx.y * PQ, kvh = head / (n_heads / n_kv);
+  // n_rows new tokens of each of gridDim.z sequences, all from start_pos on; one row per sequence (decode): warp 0 works, the others stage
+  const int head = blockIdx.x, q0 = blockIdx.y * PQ, seq = blockIdx.z, kvh = head / (n_heads / n_kv);
+  const bool single = n_rows == 1;
+  q += (size_t)seq * n_rows * n_heads * HD;
+  out += (size_t)seq * n_rows * n_heads * HD;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
-  const int rows_end = batch ? q0 + 1 : n_rows;                       // rows of this tile are q0 .. min(q0 + PQ, rows_end) - 1
-  const int pos0 = start_pos + (batch ? 0 : q0);                     // position of the tile's first row
-  const size_t seq_off = batch ? (size_t)q0 * n_kv * max_context * HD : 0;
+  const int rows_end = n_rows;                                        // rows of this tile are q0 .. min(q0 + PQ, rows_end) - 1
+  const int pos0 = start_pos + q0;                                    // position of the tile's first row
+  const size_t seq_off = (size_t)seq * n_kv * max_context * HD;
   const KV* kc = k_cache + seq_off + (size_t)kvh * max_context * HD;
   const KV* vc = v_cache + seq_off + (size_t)kvh * max_context * HD;
   // queries of this tile (rows past n_rows read as zero)
-  const int q_rows = batch ? 16 : PQ;                    // batch: only warp 0's 16 rows are read (one of them live)
+  const int q_rows = single ? 16 : PQ;                   // single: only warp 0's 16 rows are read (one of them live)
   for (int i = tid; i < q_rows * (HD / 8); i += PF_THREADS) {
     const int r = i / (HD / 8), c = (i - r * (HD / 8)) * 8;
     uint4 hi4 = make_uint4(0, 0, 0, 0), lo4 = make_uint4(0, 0, 0, 0);
@@ -146,7 +155,7 @@ __global__ void __launch_bounds__(PF_THREADS) attn_prefill_kernel(const float* _
   // q = hi + lo (both fp16): the scores keep the fp32 query's precision, as the one-token kernel's fp32 dot products do
   uint32_t qa[HD / 16][4], ql[HD / 16][4];
   {
-    const __half* qr = s_q + ((batch ? 0 : warp * 16) + g) * STRIDE + tq * 2;
+    const __half* qr = s_q + ((single ? 0 : warp * 16) + g) * STRIDE + tq * 2;
     const __half* qs = qr + PQ * STRIDE;
 #pragma unroll
     for (int kk = 0; kk < HD / 16; kk++) {
@@ -189,7 +198,7 @@ __global__ void __launch_bounds__(PF_THREADS) attn_prefill_kernel(const float* _
     }
     __syncthreads();
     if (k0 > pos0 + warp * 16 + 15) continue;  // every key of the chunk is after this warp's last query
-    if (batch && warp > 0) continue;           // one query row per CTA: warps 1..3 only help to stage the keys and values
+    if (single && warp > 0) continue;          // one query row per CTA: warps 1..3 only help to stage the keys and values
     // S = Q K^T for 16 rows x 64 keys
     float s[PK / 8][4];
 #pragma unroll
@@ -272,19 +281,24 @@ __global__ void __launch_bounds__(PF_THREADS) attn_prefill_kernel(const float* _
 
 template <int HD, typename KV, typename O>
 cudaError_t launch_prefill_attn2(const void* q, const void* kc, const void* vc, int start_pos, int n_rows, int n_heads, int n_kv, int max_context, void* out,
-                                 int batch, const int32_t* pos_dev, cudaStream_t st) {
+                                 int n_seqs, const int32_t* pos_dev, cudaStream_t st) {
   const size_t smem = (size_t)(2 * PQ + 2 * PK) * (HD + 8) * sizeof(__half);
-  cudaError_t e = cudaFuncSetAttribute(attn_prefill_kernel<HD, KV, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  attn_prefill_kernel<HD, KV, O><<<dim3(n_heads, batch ? n_rows : ceil_div(n_rows, PQ)), PF_THREADS, smem, st>>>(
-      (const float*)q, (const KV*)kc, (const KV*)vc, start_pos, n_rows, n_heads, n_kv, max_context, (O*)out, batch, pos_dev);
-  return cudaGetLastError();
+  static PerDeviceFlag attr;
+  const int dev = b200q_current_device();
+  if (dev < 0) return cudaErrorInvalidDevice;
+  if (!attr.test(dev)) {
+    const cudaError_t e = cudaFuncSetAttribute(attn_prefill_kernel<HD, KV, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    attr.set(dev);
+  }
+  return launch_k(attn_prefill_kernel<HD, KV, O>, dim3(n_heads, ceil_div(n_rows, PQ), n_seqs), dim3(PF_THREADS), smem, st, true, (const float*)q, (const KV*)kc,
+                  (const KV*)vc, start_pos, n_rows, n_heads, n_kv, max_context, (O*)out, pos_dev);
 }
 template <int HD, typename KV>
 cudaError_t launch_prefill_attn(const void* q, const void* kc, const void* vc, int start_pos, int n_rows, int n_heads, int n_kv, int max_context, void* out,
-                                bool out_f16, int batch, const int32_t* pos_dev, cudaStream_t st) {
-  return out_f16 ? launch_prefill_attn2<HD, KV, __half>(q, kc, vc, start_pos, n_rows, n_heads, n_kv, max_context, out, batch, pos_dev, st)
-                 : launch_prefill_attn2<HD, KV, float>(q, kc, vc, start_pos, n_rows, n_heads, n_kv, max_context, out, batch, pos_dev, st);
+                                bool out_f16, int n_seqs, const int32_t* pos_dev, cudaStream_t st) {
+  return out_f16 ? launch_prefill_attn2<HD, KV, __half>(q, kc, vc, start_pos, n_rows, n_heads, n_kv, max_context, out, n_seqs, pos_dev, st)
+                 : launch_prefill_attn2<HD, KV, float>(q, kc, vc, start_pos, n_rows, n_heads, n_kv, max_context, out, n_seqs, pos_dev, st);
 }
 
 }  // namespace
@@ -293,8 +307,16 @@ extern "C" int b200q_embed_rows(const void* table_f16, const int32_t* tokens, in
                                 float* x, void* stream) {
   if (!table_f16 || !tokens || !x || n_rows <= 0 || dim <= 0 || vocab <= 0 || token_stride < 0) return B200Q_ERR_BAD_ARG;
   if (dim % 2) return B200Q_ERR_BAD_SHAPE;
-  embed_rows_kernel<<<n_rows, 256, 0, (cudaStream_t)stream>>>((const __half*)table_f16, tokens, token_stride, pos_dev, n_rows, dim, vocab, x);
-  B200Q_CHECK_CUDA(cudaGetLastError());
+  B200Q_CHECK_CUDA(launch_k(embed_rows_kernel, dim3(n_rows), dim3(256), 0, (cudaStream_t)stream, false, (const __half*)table_f16, tokens, token_stride, pos_dev, 1, dim,
+                            vocab, x));
+  return B200Q_OK;
+}
+
+// per_seq consecutive tokens of each sequence, token_stride entries apart
+int b200q_embed_rows_seqs(const void* table_f16, const int32_t* tokens, int token_stride, int per_seq, int n_rows, int dim, int vocab, float* x, cudaStream_t st) {
+  if (dim % 2) return B200Q_ERR_BAD_SHAPE;
+  B200Q_CHECK_CUDA(launch_k(embed_rows_kernel, dim3(n_rows), dim3(256), 0, st, false, (const __half*)table_f16, tokens, token_stride, (const int32_t*)nullptr, per_seq, dim,
+                            vocab, x));
   return B200Q_OK;
 }
 
@@ -334,28 +356,27 @@ extern "C" int b200q_add_rows_bf16(float* x, const void* y_bf16, int64_t n, void
 }
 
 static int attn_rows(const float* qkv, void* k_cache, void* v_cache, int kv_dtype, const float* rope, int start_pos, int n_rows, int n_heads,
-                     int n_kv_heads, int head_dim, int rope_dim, int max_context, void* q_scratch, void* out, int out_dtype, int batch,
-                     const int32_t* pos_dev, void* stream) {
+                     int n_kv_heads, int head_dim, int rope_dim, int max_context, void* q_scratch, void* out, int out_dtype, int n_seqs,
+                     const int32_t* pos_dev, void* stream, bool pdl = false) {      // n_rows: per sequence
   if (!qkv || !k_cache || !v_cache || !rope || !q_scratch || !out || (out_dtype != B200Q_F16 && out_dtype != B200Q_F32)) return B200Q_ERR_BAD_ARG;
   const bool of16 = out_dtype == B200Q_F16;
-  if (n_rows <= 0 || start_pos < 0 || n_heads <= 0 || n_kv_heads <= 0 || n_heads % n_kv_heads) return B200Q_ERR_BAD_ARG;
+  if (n_rows <= 0 || n_seqs <= 0 || n_seqs > 65535 || start_pos < 0 || n_heads <= 0 || n_kv_heads <= 0 || n_heads % n_kv_heads) return B200Q_ERR_BAD_ARG;
   if (kv_dtype != B200Q_F16 && kv_dtype != B200Q_F32) return B200Q_ERR_BAD_ARG;
-  if (start_pos + (batch ? 1 : n_rows) > max_context) return B200Q_ERR_TOO_LARGE;
+  if (start_pos + n_rows > max_context) return B200Q_ERR_TOO_LARGE;
   if (rope_dim < 0 || rope_dim > head_dim || rope_dim % 2) return B200Q_ERR_BAD_SHAPE;
   if (head_dim != 16 && head_dim != 32 && head_dim != 64 && head_dim != 128) return B200Q_ERR_UNSUPPORTED;
   cudaStream_t st = (cudaStream_t)stream;
   const bool h = kv_dtype == B200Q_F16;
-  const int row_ctas = n_rows >= 64 ? 1 : ceil_div((n_heads + n_kv_heads) * head_dim, 256);
-  const dim3 rgrid(n_rows, row_ctas);
-  if (h) rope_kv_rows_kernel<__half><<<rgrid, 256, 0, st>>>(qkv, rope, start_pos, n_heads, n_kv_heads, head_dim, rope_dim, max_context, (__half*)k_cache,
-                                                           (__half*)v_cache, (float*)q_scratch, batch, pos_dev);
-  else rope_kv_rows_kernel<float><<<rgrid, 256, 0, st>>>(qkv, rope, start_pos, n_heads, n_kv_heads, head_dim, rope_dim, max_context, (float*)k_cache,
-                                                        (float*)v_cache, (float*)q_scratch, batch, pos_dev);
-  B200Q_CHECK_CUDA(cudaGetLastError());
+  const int row_ctas = n_rows * n_seqs >= 256 ? 1 : ceil_div((n_heads + n_kv_heads) * head_dim, n_rows * n_seqs >= 32 ? 1024 : 256);
+  const dim3 rgrid(n_rows * n_seqs, row_ctas);
+  if (h) B200Q_CHECK_CUDA(launch_k(rope_kv_rows_kernel<__half>, rgrid, dim3(256), 0, st, pdl, qkv, rope, start_pos, n_heads, n_kv_heads, head_dim, rope_dim, max_context,
+                                   (__half*)k_cache, (__half*)v_cache, (float*)q_scratch, n_rows, pos_dev));
+  else B200Q_CHECK_CUDA(launch_k(rope_kv_rows_kernel<float>, rgrid, dim3(256), 0, st, pdl, qkv, rope, start_pos, n_heads, n_kv_heads, head_dim, rope_dim, max_context,
+                                 (float*)k_cache, (float*)v_cache, (float*)q_scratch, n_rows, pos_dev));
   cudaError_t e;
 #define PF_CASE(HD)                                                                                                                     \
-  case HD: e = h ? launch_prefill_attn<HD, __half>(q_scratch, k_cache, v_cache, start_pos, n_rows, n_heads, n_kv_heads, max_context, out, of16, batch, pos_dev, st)  \
-                 : launch_prefill_attn<HD, float>(q_scratch, k_cache, v_cache, start_pos, n_rows, n_heads, n_kv_heads, max_context, out, of16, batch, pos_dev, st); break;
+  case HD: e = h ? launch_prefill_attn<HD, __half>(q_scratch, k_cache, v_cache, start_pos, n_rows, n_heads, n_kv_heads, max_context, out, of16, n_seqs, pos_dev, st)  \
+                 : launch_prefill_attn<HD, float>(q_scratch, k_cache, v_cache, start_pos, n_rows, n_heads, n_kv_heads, max_context, out, of16, n_seqs, pos_dev, st); break;
   switch (head_dim) { PF_CASE(16) PF_CASE(32) PF_CASE(64) default: PF_CASE(128) }
 #undef PF_CASE
   B200Q_CHECK_CUDA(e);
@@ -365,13 +386,26 @@ static int attn_rows(const float* qkv, void* k_cache, void* v_cache, int kv_dtyp
 extern "C" int b200q_attn_prefill(const float* qkv, void* k_cache, void* v_cache, int kv_dtype, const float* rope, int start_pos, int n_rows,
                                   int n_heads, int n_kv_heads, int head_dim, int rope_dim, int max_context, void* q_scratch, void* out,
                                   int out_dtype, void* stream) {
-  return attn_rows(qkv, k_cache, v_cache, kv_dtype, rope, start_pos, n_rows, n_heads, n_kv_heads, head_dim, rope_dim, max_context, q_scratch, out, out_dtype, 0,
+  return attn_rows(qkv, k_cache, v_cache, kv_dtype, rope, start_pos, n_rows, n_heads, n_kv_heads, head_dim, rope_dim, max_context, q_scratch, out, out_dtype, 1,
                    nullptr, stream);
+}
+
+int b200q_attn_rows_chain(const float* qkv, void* k_cache, void* v_cache, int kv_dtype, const float* rope, int start_pos, int n_rows, int n_seqs, int n_heads,
+                          int n_kv_heads, int head_dim, int rope_dim, int max_context, void* q_scratch, void* out, int out_dtype, cudaStream_t st, bool pdl) {
+  return attn_rows(qkv, k_cache, v_cache, kv_dtype, rope, start_pos, n_rows, n_heads, n_kv_heads, head_dim, rope_dim, max_context, q_scratch, out, out_dtype,
+                   n_seqs, nullptr, st, pdl);
+}
+
+extern "C" int b200q_attn_prefill_seqs(const float* qkv, void* k_cache, void* v_cache, int kv_dtype, const float* rope, int start_pos, int n_rows, int n_seqs,
+                                       int n_heads, int n_kv_heads, int head_dim, int rope_dim, int max_context, void* q_scratch, void* out,
+                                       int out_dtype, void* stream) {
+  return attn_rows(qkv, k_cache, v_cache, kv_dtype, rope, start_pos, n_rows, n_heads, n_kv_heads, head_dim, rope_dim, max_context, q_scratch, out, out_dtype,
+                   n_seqs, nullptr, stream);
 }
 
 extern "C" int b200q_attn_decode_batch(const float* qkv, void* k_cache, void* v_cache, int kv_dtype, const float* rope, int pos, const int32_t* pos_dev,
                                        int n_seqs, int n_heads, int n_kv_heads, int head_dim, int rope_dim, int max_context, void* q_scratch, void* out,
                                        int out_dtype, void* stream) {
-  return attn_rows(qkv, k_cache, v_cache, kv_dtype, rope, pos_dev ? 0 : pos, n_seqs, n_heads, n_kv_heads, head_dim, rope_dim, max_context, q_scratch, out,
-                   out_dtype, 1, pos_dev, stream);
+  return attn_rows(qkv, k_cache, v_cache, kv_dtype, rope, pos_dev ? 0 : pos, 1, n_heads, n_kv_heads, head_dim, rope_dim, max_context, q_scratch, out, out_dtype,
+                   n_seqs, pos_dev, stream);
 }

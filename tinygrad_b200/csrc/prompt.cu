@@ -1,0 +1,37 @@
+// A stretch of prompt rows through every block of a dense model, launched from native code: Transformer.forward for T > 1 tokens
+// (tinygrad/llm/model.py:358-362) over one or several sequences of equal length.
+// Per block: split (+ RMSNorm) and QKV GEMM, RoPE + cache append, causal attention, split and O GEMM (+ residual), split (+ RMSNorm) and
+// gate/up GEMM (SwiGLU), split and down GEMM (+ residual); every launch programmatic, so the next kernel's prologue runs under the tail of
+// the one before.  As one ctypes call per Linear the host took 35 us per block, as much as the device for a short prompt.
+#include "common.cuh"
+
+int b200q_embed_rows_seqs(const void* table_f16, const int32_t* tokens, int token_stride, int per_seq, int n_rows, int dim, int vocab, float* x, cudaStream_t st);
+
+extern "C" int b200q_prompt_rows(const b200q_rows_args* a, int first_seq, int n_seqs, int start_pos, int n_rows, void* stream) {
+  if (!a || !a->layers || !a->token_embd || !a->rope || !a->tokens || !a->x || !a->qkv || !a->q || !a->att || !a->act || !a->workspace) return B200Q_ERR_BAD_ARG;
+  if (first_seq < 0 || n_seqs <= 0 || start_pos < 0 || n_rows <= 0 || a->n_layers < 0 || (long long)n_seqs * n_rows > a->rows_max) return B200Q_ERR_BAD_ARG;
+  if (start_pos + n_rows > a->max_context) return B200Q_ERR_TOO_LARGE;
+  cudaStream_t st = (cudaStream_t)stream;
+  const int T = n_seqs * n_rows, q_dim = a->n_heads * a->head_dim, qkv_rows = q_dim + 2 * a->n_kv_heads * a->head_dim;
+  const size_t seq_bytes = (size_t)a->n_kv_heads * a->max_context * a->head_dim * (a->kv_dtype == B200Q_F16 ? 2 : 4);
+  const int stride = a->max_context + 1;
+  int rc = b200q_embed_rows_seqs(a->token_embd, a->tokens + (size_t)first_seq * stride + start_pos, stride, n_rows, T, a->dim, a->vocab, a->x, st);
+  for (int i = 0; i < a->n_layers && rc == B200Q_OK; i++) {
+    const b200q_decode_layer& l = a->layers[i];
+    rc = b200q_qgemm_chain(a->qtype, l.qkv, a->x, B200Q_F32, l.attn_norm, a->norm_eps, l.qkv_bias, nullptr, B200Q_EPI_LINEAR, a->qkv, B200Q_F32, T, qkv_rows,
+                             a->dim, a->workspace, a->workspace_bytes, st, true);
+    if (rc == B200Q_OK)
+      rc = b200q_attn_rows_chain(a->qkv, (char*)l.k_cache + first_seq * seq_bytes, (char*)l.v_cache + first_seq * seq_bytes, a->kv_dtype, a->rope, start_pos, n_rows,
+                                   n_seqs, a->n_heads, a->n_kv_heads, a->head_dim, a->rope_dim, a->max_context, a->q, a->att, B200Q_F32, st, true);
+    if (rc == B200Q_OK)
+      rc = b200q_qgemm_chain(a->qtype, l.attn_output, a->att, B200Q_F32, nullptr, 0.f, nullptr, a->x, B200Q_EPI_LINEAR, a->x, B200Q_F32, T, a->dim, q_dim, a->workspace,
+                          a->workspace_bytes, st, true);
+    if (rc == B200Q_OK)
+      rc = b200q_qgemm_chain(a->qtype, l.gate_up, a->x, B200Q_F32, l.ffn_norm, a->norm_eps, nullptr, nullptr, B200Q_EPI_SILU_MUL, a->act, B200Q_F32, T,
+                               2 * a->hidden_dim, a->dim, a->workspace, a->workspace_bytes, st, true);
+    if (rc == B200Q_OK)
+      rc = b200q_qgemm_chain(a->qtype, l.ffn_down, a->act, B200Q_F32, nullptr, 0.f, nullptr, a->x, B200Q_EPI_LINEAR, a->x, B200Q_F32, T, a->dim, a->hidden_dim, a->workspace,
+                          a->workspace_bytes, st, true);
+  }
+  return rc;
+}

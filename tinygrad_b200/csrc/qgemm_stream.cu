@@ -43,7 +43,9 @@ struct StreamParams {
   const void* residual;
   void* y;
   long long units;               // tiles x K groups
-  int grain;                     // units are dealt in multiples of this: 1, or a whole tile where the workspace has no room for partial sums
+  // Units are dealt in multiples of this: 1, or a whole tile where the caller wants it so (`unsplit`) or the workspace has no room for partial
+  // sums.  With whole tiles every output is one running sum (halves not side by side either) in the order of b200q_qgemm: the same bits.
+  int grain, unsplit;
   int tiles, m, n_out, kgroups, n_row_tiles, nt, tok_tiles, slots, y_f16, silu_mul;
 };
 
@@ -212,7 +214,7 @@ __device__ __forceinline__ bool finish_segment(const StreamParams& p, Shared& sh
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = warp & 3, q = warp >> 2;
   const int hf = WT == 256 ? q >> 1 : 0, part0 = WT == 256 ? q & 1 : q, parts = WT == 256 ? 2 : 4;
   const int tt = tile % p.tok_tiles, row = hf * 128 + sub * 32 + lane, feat = (tile / p.tok_tiles) * WT + row;
-  const bool whole = k0 == 0 && k1 == p.kgroups, stacked = F32 && p.nt <= MAX_NT / 2;
+  const bool whole = k0 == 0 && k1 == p.kgroups, stacked = F32 && p.nt <= MAX_NT / 2 && !p.unsplit;
   const int G = gridDim.x, c = blockIdx.x;
   int c0 = c, n_seg = 1;
   if (!whole) {
@@ -342,7 +344,7 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
   } else if (warp == WARP_MMA) {
     if (elect_one()) {
       bool ok = true;
-      const bool stacked = F32 && nt <= MAX_NT / 2;
+      const bool stacked = F32 && nt <= MAX_NT / 2 && !p.unsplit;
       const uint32_t id1 = make_idesc(128, nt), id2 = make_idesc(128, stacked ? 2 * nt : nt);
       const uint32_t desc_hi = (uint32_t)(make_desc(0, 0, 128) >> 32);
       const uint32_t w_base = (ring >> 4) | ((uint32_t)WT << 16), x_base = ((ring + W_SLOT) >> 4) | ((uint32_t)x_rows << 16);
@@ -549,7 +551,7 @@ static size_t split_workspace(const Plan& pl, int n_out, int kgroups, int n_sm) 
   return COUNTER_BYTES + (size_t)parts * pl.wt * pl.nt * sizeof(float);
 }
 
-// room for the activations in tiles of 128 rows (the kernel's own tiles never take more): enough to run, tiles then going whole to the CTAs
+// Room for the activations in tiles of 128 rows (the kernel's own tiles never take more): enough to run, tiles then going whole to the CTAs
 extern "C" size_t b200q_qgemm_workspace_bytes(int m, int n_in) {
   if (m <= 0 || n_in <= 0) return 0;
   return (size_t)ceil_div(m, 128) * 128 * ceil_div(n_in, GROUP_ELEMS) * GROUP_ELEMS * 4;
@@ -561,9 +563,8 @@ extern "C" size_t b200q_qgemm_workspace_bytes_for(int m, int n_out, int n_in) {
 }
 
 // norm_weight (fp16 [n_in], fp32 activations only): the RMSNorm in front of the Linear, applied while the rows are split.
-extern "C" int b200q_qgemm_ws_norm(int qtype, const void* w_packed, const void* x, int x_dtype, const void* norm_weight, float norm_eps,
-                                   const void* bias_f16, const void* residual, int epilogue, void* y, int y_dtype, int m, int n_out, int n_in,
-                                   void* workspace, size_t workspace_bytes, void* stream) {
+int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtype, const void* norm_weight, float norm_eps, const void* bias_f16, const void* residual,
+                      int epilogue, void* y, int y_dtype, int m, int n_out, int n_in, void* workspace, size_t workspace_bytes, cudaStream_t st, bool pdl, bool unsplit) {
   if (!w_packed || !x || !y || !workspace || m <= 0 || n_out <= 0 || n_in <= 0) return B200Q_ERR_BAD_ARG;
   if (epilogue != B200Q_EPI_LINEAR && epilogue != B200Q_EPI_SILU_MUL) return B200Q_ERR_BAD_ARG;
   if (epilogue == B200Q_EPI_SILU_MUL && (bias_f16 || residual || n_out % 16)) return B200Q_ERR_BAD_ARG;
@@ -573,7 +574,6 @@ extern "C" int b200q_qgemm_ws_norm(int qtype, const void* w_packed, const void* 
   if (norm_weight && x_dtype != B200Q_F32) return B200Q_ERR_BAD_ARG;
   if (n_in % 32) return B200Q_ERR_BAD_SHAPE;
   if (((uintptr_t)w_packed | (uintptr_t)x | (uintptr_t)workspace | (uintptr_t)norm_weight) & 15) return B200Q_ERR_MISALIGNED;
-  cudaStream_t st = (cudaStream_t)stream;
   const Plan pl = make_plan(m);
   const bool f32 = x_dtype == B200Q_F32;
   const int kgroups = ceil_div(n_in, GROUP_ELEMS);
@@ -594,16 +594,16 @@ extern "C" int b200q_qgemm_ws_norm(int qtype, const void* w_packed, const void* 
   p.y_f16 = y_dtype == B200Q_F16; p.silu_mul = epilogue == B200Q_EPI_SILU_MUL;
   p.tiles = ceil_div(n_out, pl.wt) * pl.tok_tiles;
   p.units = (long long)p.tiles * kgroups;
-  const bool split = workspace_bytes >= xt_bytes + split_workspace(pl, n_out, kgroups, n_sm);
-  p.grain = split ? 1 : kgroups;
+  const bool split = !unsplit && workspace_bytes >= xt_bytes + split_workspace(pl, n_out, kgroups, n_sm);
+  p.grain = split ? 1 : kgroups; p.unsplit = !split;
   const int grid = split ? stream_grid(p.units, n_sm) : (p.tiles < n_sm ? p.tiles : n_sm);
   // one CTA of the splitting kernel: 8 rows x the whole width, or a part of it where there are few rows
   const int row_groups = pl.tok_tiles * pl.nt / 8, n_chunks = kgroups * 16;
   const int parts = row_groups >= n_sm ? 1 : (row_groups * 4 >= n_sm || n_chunks < 256 ? 4 : 8), per = ceil_div(n_chunks, parts);
   const dim3 sgrid(ceil_div(n_chunks, per), row_groups);
-  if (f32) B200Q_CHECK_CUDA(launch_k(split_rows_kernel<float>, sgrid, dim3(SPLIT_THREADS), 0, st, true, (const float*)x, (const __half*)norm_weight, norm_eps, m,
+  if (f32) B200Q_CHECK_CUDA(launch_k(split_rows_kernel<float>, sgrid, dim3(SPLIT_THREADS), 0, st, pdl, (const float*)x, (const __half*)norm_weight, norm_eps, m,
                                      n_in, kgroups, pl.nt, per, (unsigned char*)p.xt, p.counters, split ? grid : 0));
-  else B200Q_CHECK_CUDA(launch_k(split_rows_kernel<__half>, sgrid, dim3(SPLIT_THREADS), 0, st, true, (const __half*)x, (const __half*)nullptr, 0.f, m, n_in,
+  else B200Q_CHECK_CUDA(launch_k(split_rows_kernel<__half>, sgrid, dim3(SPLIT_THREADS), 0, st, pdl, (const __half*)x, (const __half*)nullptr, 0.f, m, n_in,
                                  kgroups, pl.nt, per, (unsigned char*)p.xt, p.counters, split ? grid : 0));
 #define STREAM_CASE(QT) (pl.wt == 256 ? (f32 ? launch_stream<QT, 256, true>(p, grid, st) : launch_stream<QT, 256, false>(p, grid, st)) \
                                       : (f32 ? launch_stream<QT, 128, true>(p, grid, st) : launch_stream<QT, 128, false>(p, grid, st)))
@@ -611,8 +611,14 @@ extern "C" int b200q_qgemm_ws_norm(int qtype, const void* w_packed, const void* 
 #undef STREAM_CASE
 }
 
+extern "C" int b200q_qgemm_ws_norm(int qtype, const void* w_packed, const void* x, int x_dtype, const void* norm_weight, float norm_eps,
+                                   const void* bias_f16, const void* residual, int epilogue, void* y, int y_dtype, int m, int n_out, int n_in,
+                                   void* workspace, size_t workspace_bytes, int unsplit, void* stream) {
+  return b200q_qgemm_chain(qtype, w_packed, x, x_dtype, norm_weight, norm_eps, bias_f16, residual, epilogue, y, y_dtype, m, n_out, n_in, workspace,
+                           workspace_bytes, (cudaStream_t)stream, false, unsplit != 0);
+}
 extern "C" int b200q_qgemm_ws(int qtype, const void* w_packed, const void* x, int x_dtype, const void* bias_f16, const void* residual, int epilogue,
                               void* y, int y_dtype, int m, int n_out, int n_in, void* workspace, size_t workspace_bytes, void* stream) {
   return b200q_qgemm_ws_norm(qtype, w_packed, x, x_dtype, nullptr, 0.f, bias_f16, residual, epilogue, y, y_dtype, m, n_out, n_in, workspace,
-                             workspace_bytes, stream);
+                             workspace_bytes, 0, stream);
 }

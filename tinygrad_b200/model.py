@@ -20,6 +20,11 @@ import ctypes, os
 SEQ_ATTENTION = os.environ.get("B200Q_SEQ_ATTENTION", "0") == "1"
 
 
+# prompts of at least this many uncached tokens take the GEMM path (unless it is off) even below prefill_rows: one pass over the weights for all of them
+# costs about as much as this many one-token steps
+SHORT_PROMPT_ROWS = 6
+
+
 @dataclass(frozen=True)
 class TransformerConfig:           # field names of tinygrad/llm/model.py:52-83 (dense GQA subset)
   num_blocks: int
@@ -70,8 +75,8 @@ class Transformer:
     GGUF block bytes (uint8), embeddings / norms / biases as fp16.
     tp: a tensor_parallel.TPGroup; `config` is then the FULL model and `state_dict` this rank's shard (shard_state_dict).
     output_type: GGML type of `output.weight` when it differs from the block Linears' (F16 / BF16 / F32 heads run the dense GEMV).
-    prefill_rows: prompts with at least this many uncached tokens go through the tensor-core GEMM path, `prefill_chunk` rows at a
-    time (0: always one token per step, whose fp32-activation numerics are the reference's own); shorter ones take decode steps.
+    prefill_rows: prompts with at least this many uncached tokens, or SHORT_PROMPT_ROWS, go through the tensor-core GEMM path, `prefill_chunk`
+    rows at a time (0: always one token per step); shorter ones take decode steps.
     engine: how a one-token step runs.  "step": one persistent kernel for the whole step (b200q_decode_step); "chain": five launches per
     block chained with programmatic dependent launch and replayed as a CUDA graph (the default: at batch 1 it measured faster, the
     grid-wide waits inside one kernel costing more than kernel boundaries do).
@@ -199,7 +204,7 @@ class Transformer:
     self.pos = DeviceBuffer.empty((batch,), np.int32, zero=True)
     self.seq_cache_bytes = c.n_kv_heads * c.max_context * c.head_dim * np.dtype(kvdt).itemsize
     self.attn_scratch = DeviceBuffer(_lib.load().b200q_attn_scratch_bytes(c.n_heads, c.n_kv_heads, c.head_dim, self.n_split), zero=True)
-    self.argmax_scratch = DeviceBuffer(_lib.load().b200q_argmax_scratch_bytes(), zero=True)
+    self.argmax_scratch = DeviceBuffer(batch * _lib.load().b200q_argmax_scratch_bytes(), zero=True)
     # Quantised activation hand-over between consecutive kernels (needs whole 128-wide groups everywhere).  Each edge of
     # the chain can be switched on its own: attn_o (attention -> output projection), o_gateup, gateup_down, down_qkv.
     can = c.head_dim == 128 and c.dim % 128 == 0 and c.hidden_dim % 128 == 0 and self.q_dim % 128 == 0 and not self.dense_blocks
@@ -225,9 +230,10 @@ class Transformer:
     self._graphs = {}
     self._cached_tokens: list = []
     self.prefill_rows = prefill_rows if (tp is None and not self.dense_blocks and c.hidden_dim % 8 == 0 and c.head_dim in (16, 32, 64, 128)) else 0
-    self.prefill_chunk, self._pf, self._batch_logits, self._skinny_ws, self._batch_graph = max(1, prefill_chunk), None, None, None, None
+    self.prefill_chunk, self._pf, self._batch_logits, self._rows_ws, self._batch_graph = max(1, prefill_chunk), None, None, None, None
+    self._rows_args = None
     self._seq_attn_scratch = None
-    self.is_moe, self._host_pos = c.num_experts > 0, 0
+    self.is_moe, self._host_pos, self._rows_warm = c.num_experts > 0, 0, False
     if self.is_moe:
       assert tp is None and c.head_dim in (16, 32, 64, 128), "the mixture-of-experts model runs on the row path of one GPU"
       self.prefill_rows = 1
@@ -339,6 +345,11 @@ class Transformer:
       check(lib.b200q_advance(self.pos.ptr, c.max_context, 0 if (tp is not None and not peer) else fl, s))
 
   # ---- several prompt tokens at once: tcgen05 dequant GEMMs + batched causal attention ----
+  def _rows_workspace_bytes(self, T: int) -> int:
+    c, qkv_rows = self.config, self.q_dim + 2 * self.kv_dim
+    if self.is_moe: return quant.qgemm_unsplit_workspace_bytes(T, max(c.dim, self.q_dim, c.shared_expert_dim))
+    return max(quant.qgemm_workspace_bytes(T, i, o) for o, i in ((qkv_rows, c.dim), (c.dim, self.q_dim), (2 * c.hidden_dim, c.dim), (c.dim, c.hidden_dim)))
+
   def _prefill_buffers(self):
     if self._pf is None:
       c, T = self.config, self.prefill_chunk
@@ -346,8 +357,10 @@ class Transformer:
                       qkv=DeviceBuffer.empty((T, self.q_dim + 2 * self.kv_dim), np.float32), q16=DeviceBuffer.empty((T, self.q_dim), np.float32),
                       att=DeviceBuffer.empty((T, self.q_dim), np.float32),
                       act=DeviceBuffer.empty((T, max(c.hidden_dim, c.shared_expert_dim, 1)), np.float32),
-                      # activation tiles and partial sums of the GEMMs
-                      ws=DeviceBuffer(quant.qgemm_workspace_bytes(T, max(c.dim, self.q_dim, c.hidden_dim, c.shared_expert_dim, 1))) if self.pipelined_gemm else None)
+                      # Activation tiles and partial sums of the GEMMs.  Mixture-of-experts models take sums that are not split: their expert
+                      # choice and E4M3 codes turn a last-bit difference into a visible one, and a token's result must not depend on how
+                      # many rows it was computed with.
+                      ws=DeviceBuffer(self._rows_workspace_bytes(T)) if self.pipelined_gemm else None)
       if self.is_moe:
         self._pf.update(xb=DeviceBuffer.empty((T, c.dim), np.uint16), logits=DeviceBuffer.empty((T, c.num_experts), np.float32))
         if c.shared_expert_dim: self._pf.update(sh=DeviceBuffer.empty((T, c.dim), np.float32), shg=DeviceBuffer.empty((T,), np.float32))
@@ -359,45 +372,69 @@ class Transformer:
     causal attention -> O GEMM (+residual) -> rmsnorm -> gate/up GEMM with SwiGLU epilogue -> down GEMM (+residual).
     Activations stay fp32 between the kernels; the GEMMs split them into fp16 hi + lo halves for the tensor core."""
     c, lib, s, f = self.config, _lib.load(), self.stream.ptr, self._prefill_buffers()
-    kvdt = F16 if c.kv_dtype == "float16" else F32
-    qkv_rows = self.q_dim + 2 * self.kv_dim
-    for p0 in range(start_pos, start_pos + n, self.prefill_chunk):
+    native = self._native_rows()
+    for p0 in range(start_pos, start_pos + n, self.prefill_chunk) if native else ():
+      check(lib.b200q_prompt_rows(native, seq, 1, p0, min(self.prefill_chunk, start_pos + n - p0), s))
+    for p0 in () if native else range(start_pos, start_pos + n, self.prefill_chunk):
       T = min(self.prefill_chunk, start_pos + n - p0)
       check(lib.b200q_embed_rows(self.token_embd.ptr, self.tokens.ptr + 4 * (seq * (c.max_context + 1) + p0), 1, None, T, c.dim,
                                  self.full_config.vocab_size, f["x"].ptr, s))
-      def normed(norm):       # the GEMM with a workspace applies the RMSNorm while it splits its activations
-        if f["ws"] is not None and quant.PIPELINED_GEMM: return f["x"], {"norm_weight": norm, "norm_eps": c.norm_eps}
-        check(lib.b200q_rmsnorm_rows(f["x"].ptr, norm.ptr, c.norm_eps, T, c.dim, f["xn"].ptr, F32, s))
-        return f["xn"], {}
-      for b in self.blk:
-        xin, kw = normed(b.attn_norm)
-        quant.qgemm(b.qkv.ptr, self.qtype, qkv_rows, c.dim, xin, f["qkv"], T, x_dtype=F32, y_dtype=F32, bias=b.qkv_bias, stream=s, workspace=f["ws"], **kw)
-        check(lib.b200q_attn_prefill(f["qkv"].ptr, b.k_cache.ptr + seq * self.seq_cache_bytes, b.v_cache.ptr + seq * self.seq_cache_bytes, kvdt,
-                                     self.rope.ptr, p0, T, c.n_heads, c.n_kv_heads, c.head_dim,
-                                     c.rope_dim, c.max_context, f["q16"].ptr, f["att"].ptr, F32, s))
-        quant.qgemm(b.attn_output.buf.ptr, self.qtype, c.dim, self.q_dim, f["att"], f["x"], T, x_dtype=F32, y_dtype=F32, residual=f["x"], stream=s, workspace=f["ws"])
-        if b.moe is not None:
-          check(lib.b200q_rmsnorm_rows(f["x"].ptr, b.ffn_norm.ptr, c.norm_eps, T, c.dim, f["xn"].ptr, F32, s))
-          # router on the fp32 normed rows, experts on their bf16 rounding (the activation dtype of the MXFP8 path); bf16 result + residual
-          quant.gemv_dense(b.router.buf, b.router.dtype, c.num_experts, c.dim, f["xn"], f["logits"], m=T, stream=s)
-          check(lib.b200q_rmsnorm_rows(f["x"].ptr, b.ffn_norm.ptr, c.norm_eps, T, c.dim, f["xb"].ptr, _lib.BF16, s))
-          y = b.moe(f["xb"], f["logits"], T, stream=s)
-          if b.sh_gate_up is not None:      # shared expert on the fp32 normed rows (model.py:131-134), added before x moves
-            quant.qgemm(b.sh_gate_up.buf.ptr, self.qtype, 2 * c.shared_expert_dim, c.dim, f["xn"], f["act"], T, x_dtype=F32, y_dtype=F32,
-                        epilogue=EPI_SILU_MUL, stream=s, workspace=f["ws"])
-            quant.qgemm(b.sh_down.buf.ptr, self.qtype, c.dim, c.shared_expert_dim, f["act"], f["sh"], T, x_dtype=F32, y_dtype=F32, stream=s, workspace=f["ws"])
-            if b.sh_inp is not None: quant.gemv_dense(b.sh_inp.buf, b.sh_inp.dtype, 1, c.dim, f["xn"], f["shg"], m=T, stream=s)
-            check(lib.b200q_add_rows_gated(f["x"].ptr, f["sh"].ptr, f["shg"].ptr if b.sh_inp is not None else None, T, c.dim, s))
-          check(lib.b200q_add_rows_bf16(f["x"].ptr, y.ptr, T * c.dim, s))
-          continue
-        xin, kw = normed(b.ffn_norm)
-        quant.qgemm(b.gate_up.buf.ptr, self.qtype, 2 * c.hidden_dim, c.dim, xin, f["act"], T, x_dtype=F32, y_dtype=F32, epilogue=EPI_SILU_MUL,
-                    stream=s, workspace=f["ws"], **kw)
-        quant.qgemm(b.ffn_down.buf.ptr, self.qtype, c.dim, c.hidden_dim, f["act"], f["x"], T, x_dtype=F32, y_dtype=F32, residual=f["x"], stream=s, workspace=f["ws"])
+      for b in self.blk: self._enqueue_rows_block(b, T, f, p0, seq)
     if sync:
       self.stream.synchronize()
       self.pos.copy_from(np.array([start_pos + n], dtype=np.int32), offset=4 * seq)
       self._host_pos = start_pos + n
+
+  def _enqueue_rows_block(self, b, T: int, f: dict, p0, seq: int) -> None:
+    """One block for T rows in f["x"]: positions p0 .. of sequence `seq`, or (p0 None) one row at the position kept on the device."""
+    c, lib, s = self.config, _lib.load(), self.stream.ptr
+    kvdt = F16 if c.kv_dtype == "float16" else F32
+    qkv_rows = self.q_dim + 2 * self.kv_dim
+    def normed(norm):       # the GEMM with a workspace applies the RMSNorm while it splits its activations
+      if f["ws"] is not None and quant.PIPELINED_GEMM and not self.is_moe: return f["x"], {"norm_weight": norm, "norm_eps": c.norm_eps}
+      check(lib.b200q_rmsnorm_rows(f["x"].ptr, norm.ptr, c.norm_eps, T, c.dim, f["xn"].ptr, F32, s))
+      return f["xn"], {}
+    xin, kw = normed(b.attn_norm)
+    quant.qgemm(b.qkv.ptr, self.qtype, qkv_rows, c.dim, xin, f["qkv"], T, x_dtype=F32, y_dtype=F32, bias=b.qkv_bias, stream=s, workspace=f["ws"], unsplit=self.is_moe, **kw)
+    if p0 is None:       # position on the device
+      check(lib.b200q_attn_decode_batch(f["qkv"].ptr, b.k_cache.ptr, b.v_cache.ptr, kvdt, self.rope.ptr, 0, self.pos.ptr, T, c.n_heads, c.n_kv_heads, c.head_dim,
+                                        c.rope_dim, c.max_context, f["q16"].ptr, f["att"].ptr, F32, s))
+    else:
+      check(lib.b200q_attn_prefill(f["qkv"].ptr, b.k_cache.ptr + seq * self.seq_cache_bytes, b.v_cache.ptr + seq * self.seq_cache_bytes, kvdt,
+                                   self.rope.ptr, p0, T, c.n_heads, c.n_kv_heads, c.head_dim,
+                                   c.rope_dim, c.max_context, f["q16"].ptr, f["att"].ptr, F32, s))
+    quant.qgemm(b.attn_output.buf.ptr, self.qtype, c.dim, self.q_dim, f["att"], f["x"], T, x_dtype=F32, y_dtype=F32, residual=f["x"], stream=s, workspace=f["ws"], unsplit=self.is_moe)
+    if b.moe is not None:
+      check(lib.b200q_rmsnorm_rows(f["x"].ptr, b.ffn_norm.ptr, c.norm_eps, T, c.dim, f["xn"].ptr, F32, s))
+      # router on the fp32 normed rows, experts on their bf16 rounding (the activation dtype of the MXFP8 path); bf16 result + residual
+      quant.gemv_dense(b.router.buf, b.router.dtype, c.num_experts, c.dim, f["xn"], f["logits"], m=T, stream=s)
+      check(lib.b200q_rmsnorm_rows(f["x"].ptr, b.ffn_norm.ptr, c.norm_eps, T, c.dim, f["xb"].ptr, _lib.BF16, s))
+      y = b.moe(f["xb"], f["logits"], T, stream=s)
+      if b.sh_gate_up is not None:      # shared expert on the fp32 normed rows (model.py:131-134), added before x moves
+        quant.qgemm(b.sh_gate_up.buf.ptr, self.qtype, 2 * c.shared_expert_dim, c.dim, f["xn"], f["act"], T, x_dtype=F32, y_dtype=F32,
+                    epilogue=EPI_SILU_MUL, stream=s, workspace=f["ws"], unsplit=self.is_moe)
+        quant.qgemm(b.sh_down.buf.ptr, self.qtype, c.dim, c.shared_expert_dim, f["act"], f["sh"], T, x_dtype=F32, y_dtype=F32, stream=s, workspace=f["ws"], unsplit=self.is_moe)
+        if b.sh_inp is not None: quant.gemv_dense(b.sh_inp.buf, b.sh_inp.dtype, 1, c.dim, f["xn"], f["shg"], m=T, stream=s)
+        check(lib.b200q_add_rows_gated(f["x"].ptr, f["sh"].ptr, f["shg"].ptr if b.sh_inp is not None else None, T, c.dim, s))
+      check(lib.b200q_add_rows_bf16(f["x"].ptr, y.ptr, T * c.dim, s))
+      return
+    xin, kw = normed(b.ffn_norm)
+    quant.qgemm(b.gate_up.buf.ptr, self.qtype, 2 * c.hidden_dim, c.dim, xin, f["act"], T, x_dtype=F32, y_dtype=F32, epilogue=EPI_SILU_MUL,
+                stream=s, workspace=f["ws"], unsplit=self.is_moe, **kw)
+    quant.qgemm(b.ffn_down.buf.ptr, self.qtype, c.dim, c.hidden_dim, f["act"], f["x"], T, x_dtype=F32, y_dtype=F32, residual=f["x"], stream=s, workspace=f["ws"], unsplit=self.is_moe)
+
+  def _native_rows(self):
+    """The argument block of b200q_prompt_rows (every launch of a chunk from one call), or None where the model does not run on it."""
+    if self.is_moe or self.dense_blocks or self.tp is not None or not self.pipelined_gemm or not quant.PIPELINED_GEMM: return None
+    if self._rows_args is None:
+      c, f = self.config, self._prefill_buffers()
+      self._layer_host = (_lib.DecodeLayer * c.num_blocks)(*[_lib.DecodeLayer(b.qkv.ptr, b.qkv_bias.ptr if b.qkv_bias else None, b.attn_output.buf.ptr, b.gate_up.buf.ptr,
+                                                                             b.ffn_down.buf.ptr, b.attn_norm.ptr, b.ffn_norm.ptr, b.k_cache.ptr, b.v_cache.ptr) for b in self.blk])
+      a = _lib.RowsArgs(self._layer_host, c.num_blocks, self.qtype, c.dim, c.hidden_dim, c.n_heads, c.n_kv_heads, c.head_dim, c.rope_dim, c.max_context,
+                        self.full_config.vocab_size, F16 if c.kv_dtype == "float16" else F32, self.prefill_chunk, c.norm_eps, self.token_embd.ptr, self.rope.ptr,
+                        self.tokens.ptr, f["x"].ptr, f["qkv"].ptr, f["q16"].ptr, f["att"].ptr, f["act"].ptr, f["ws"].ptr, f["ws"].nbytes)
+      self._rows_args = (a, ctypes.byref(a))
+    return self._rows_args[1]
 
   # ---- several sequences in lock-step ----
   def decode_batch_step(self) -> None:
@@ -420,21 +457,18 @@ class Transformer:
     kvdt = F16 if c.kv_dtype == "float16" else F32
     qkv_rows = self.q_dim + 2 * self.kv_dim
     head_q = not isinstance(self.output, quant.DenseWeight)
-    if B <= quant.FEW_ROW_MAX and quant.FEW_ROW_FUSED:       # 8 rows per pass on the int8 tensor cores at the one-row GEMV's arithmetic (weights streamed once per pass)
-      if self._skinny_ws is None:
-        shapes = [(qkv_rows, c.dim), (c.dim, self.q_dim), (2 * c.hidden_dim, c.dim), (c.dim, c.hidden_dim)] + ([(c.vocab_size, c.dim)] if head_q else [])
-        self._skinny_ws = DeviceBuffer(max(quant.qgemv_rows_workspace_bytes(B, o, i) for o, i in shapes))
-      def gemm(w, qt, n_out, n_in, x, y, **kw): quant.qgemv_rows(w, qt, n_out, n_in, x, y, B, self._skinny_ws, x_dtype=F32, y_dtype=F32, stream=s, **kw)
-    elif B <= 32:    # the weight-streaming GEMM shape (swapped operands, split K); its partial sums go through one workspace
-      if self._skinny_ws is None:
-        shapes = [(qkv_rows, c.dim), (c.dim, self.q_dim), (2 * c.hidden_dim, c.dim), (c.dim, c.hidden_dim)] + ([(c.vocab_size, c.dim)] if head_q else [])
-        self._skinny_ws = DeviceBuffer(max(quant.qgemm_skinny_workspace_bytes(B, o, i) for o, i in shapes))
-      def gemm(w, qt, n_out, n_in, x, y, **kw): quant.qgemm_skinny(w, qt, n_out, n_in, x, y, B, self._skinny_ws, x_dtype=F32, y_dtype=F32, stream=s, **kw)
+    few = B <= quant.FEW_ROW_MAX and quant.FEW_ROW_FUSED     # 8 rows per pass on the int8 tensor cores at the one-row GEMV's arithmetic; else one pass of the GEMM
+    if self._rows_ws is None:
+      shapes = [(qkv_rows, c.dim), (c.dim, self.q_dim), (2 * c.hidden_dim, c.dim), (c.dim, c.hidden_dim)] + ([(c.vocab_size, c.dim)] if head_q else [])
+      need = quant.qgemv_rows_workspace_bytes if few else (lambda m, o, i: quant.qgemm_workspace_bytes(m, i, o))
+      self._rows_ws = DeviceBuffer(max(need(B, o, i) for o, i in shapes))
+    if few:
+      def gemm(w, qt, n_out, n_in, x, y, **kw): quant.qgemv_rows(w, qt, n_out, n_in, x, y, B, self._rows_ws, x_dtype=F32, y_dtype=F32, stream=s, **kw)
     else:
-      def gemm(w, qt, n_out, n_in, x, y, **kw): quant.qgemm(w, qt, n_out, n_in, x, y, B, x_dtype=F32, y_dtype=F32, stream=s, **kw)
+      def gemm(w, qt, n_out, n_in, x, y, **kw): quant.qgemm(w, qt, n_out, n_in, x, y, B, x_dtype=F32, y_dtype=F32, stream=s, workspace=self._rows_ws, **kw)
     # the position comes from the device (sequence 0's counter; all sequences move together), so the launch sequence can be replayed as a graph
     check(lib.b200q_embed_rows(self.token_embd.ptr, self.tokens.ptr, c.max_context + 1, self.pos.ptr, B, c.dim, c.vocab_size, f["x"].ptr, s))
-    fold = B <= quant.FEW_ROW_MAX and quant.FEW_ROW_FUSED     # the few-row kernel's pre-pass applies the RMSNorm itself: no norm launches
+    fold = few or quant.PIPELINED_GEMM     # both apply the RMSNorm in their pre-pass: no norm launches
     seq_attn = SEQ_ATTENTION and c.n_heads // c.n_kv_heads <= 8 and c.head_dim % 8 == 0 and c.head_dim <= 128
     if seq_attn and self._seq_attn_scratch is None:
       stride = lib.b200q_attn_seq_scratch_stride(c.n_heads, c.n_kv_heads, c.head_dim, self.n_split)
@@ -464,10 +498,19 @@ class Transformer:
       check(lib.b200q_rmsnorm_rows(f["x"].ptr, self.output_norm.ptr, c.norm_eps, B, c.dim, f["xn"].ptr, F32, s))
       if head_q: gemm(self.output.buf.ptr, self.output_type, c.vocab_size, c.dim, f["xn"], self._batch_logits)
       else: quant.gemv_dense(self.output.buf, self.output.dtype, c.vocab_size, c.dim, f["xn"], self._batch_logits, m=B, stream=s)
-    for i in range(B):
-      check(lib.b200q_argmax_advance(self._batch_logits.ptr + 4 * i * c.vocab_size, c.vocab_size, self.tokens.ptr + 4 * i * (c.max_context + 1),
-                                     self.pos.ptr + 4 * i, c.max_context, self.argmax_scratch.ptr, 0, s))
+    check(lib.b200q_argmax_advance_seqs(self._batch_logits.ptr, c.vocab_size, self.tokens.ptr, c.max_context + 1, self.pos.ptr, c.max_context,
+                                        self.argmax_scratch.ptr, B, FLAG_PDL, s))
     if count: self._host_pos += 1
+
+  def _prefill_batch(self, n: int) -> None:
+    """tokens[:n] of every sequence: as many whole sequences per pass as fit prefill_chunk rows (the weights are streamed once per pass)."""
+    native, per = self._native_rows(), self.prefill_chunk // n
+    if native is None or per < 2:
+      for i in range(self.batch): self.prefill(0, n, seq=i)
+      return
+    for i in range(0, self.batch, per):
+      check(_lib.load().b200q_prompt_rows(native, i, min(per, self.batch - i), 0, n, self.stream.ptr))
+    self.stream.synchronize()
 
   def generate_batch(self, prompts: list):
     """Greedy generation for `batch` prompts of equal length; yields the list of the sequences' next tokens per step."""
@@ -478,8 +521,7 @@ class Transformer:
     tok = np.zeros((B, c.max_context + 1), np.int32)
     for i, p in enumerate(prompts): tok[i, :L] = p
     self.tokens.copy_from(tok)
-    for i in range(B):
-      if L > 1: self.prefill(0, L - 1, seq=i)
+    if L > 1: self._prefill_batch(L - 1)
     self.pos.copy_from(np.full((B,), L - 1, dtype=np.int32))
     self._host_pos, n = L - 1, L
     while n < c.max_context:
@@ -489,9 +531,25 @@ class Transformer:
       n += 1
 
   def _step_rows(self, with_head: bool) -> None:
-    """One token through the row path (mixture-of-experts models: their FFN is not part of the fused one-token chain)."""
-    c, lib, s = self.config, _lib.load(), self.stream.ptr
-    self.prefill(self._host_pos, 1, sync=False)
+    """One token through the row path (mixture-of-experts models: their FFN is not part of the fused one-token chain).  Positions come
+    from the device, so the launches are captured once (behind a first step that allocates) and replayed as a CUDA graph."""
+    if not self.use_graph: self._enqueue_step_rows(with_head)
+    elif with_head not in self._graphs and not self._rows_warm:
+      self._enqueue_step_rows(with_head)
+      self._rows_warm = True
+    else:
+      g = self._graphs.get(with_head)
+      if g is None:
+        g = Graph(self.stream)
+        with g: self._enqueue_step_rows(with_head)
+        self._graphs[with_head] = g
+      g.launch()
+    self._host_pos += 1
+
+  def _enqueue_step_rows(self, with_head: bool) -> None:
+    c, lib, s, f = self.config, _lib.load(), self.stream.ptr, self._prefill_buffers()
+    check(lib.b200q_embed_rows(self.token_embd.ptr, self.tokens.ptr, 1, self.pos.ptr, 1, c.dim, self.full_config.vocab_size, f["x"].ptr, s))
+    for b in self.blk: self._enqueue_rows_block(b, 1, f, None, 0)
     if with_head:
       x_last = self._pf["x"]
       if isinstance(self.output, quant.DenseWeight):
@@ -503,7 +561,6 @@ class Transformer:
       check(lib.b200q_argmax_advance(self.logits.ptr, c.vocab_size, self.tokens.ptr, self.pos.ptr, c.max_context, self.argmax_scratch.ptr, 0, s))
     else:
       check(lib.b200q_advance(self.pos.ptr, c.max_context, 0, s))
-    self._host_pos += 1
 
   def _check_room(self) -> None:
     if self._host_pos >= self.max_context:
@@ -568,7 +625,7 @@ class Transformer:
     start_pos = self.get_start_pos(tokens)
     self.set_state(tokens, start_pos)
     n_pre = len(tokens) - 1 - start_pos
-    if self.prefill_rows and n_pre >= self.prefill_rows: self.prefill(start_pos, n_pre)
+    if self.prefill_rows and n_pre >= min(self.prefill_rows, SHORT_PROMPT_ROWS): self.prefill(start_pos, n_pre)
     else:
       for _ in range(n_pre): self.step(with_head=False)
     while len(tokens) < self.max_context:

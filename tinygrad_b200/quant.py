@@ -96,14 +96,20 @@ def qgemm_workspace_bytes(m: int, n_in: int, n_out: int = 0) -> int:
   return int(_lib.load().b200q_qgemm_workspace_bytes_for(m, n_out, n_in))
 
 
+def qgemm_unsplit_workspace_bytes(m: int, n_in: int) -> int:
+  """The least scratch the GEMM runs in: no tile is split, every output is one running sum (the same bits as without a workspace)."""
+  return int(_lib.load().b200q_qgemm_workspace_bytes(m, n_in))
+
+
 def qgemm(w_ptr: int, qtype: int, n_out: int, n_in: int, x, y, m: int, x_dtype=F32, y_dtype=F32, bias=None, residual=None,
-          epilogue: int = EPI_LINEAR, stream=None, workspace: DeviceBuffer = None, norm_weight=None, norm_eps: float = 0.0) -> None:
+          epilogue: int = EPI_LINEAR, stream=None, workspace: DeviceBuffer = None, norm_weight=None, norm_eps: float = 0.0, unsplit: bool = False) -> None:
   """Batched / prefill linear on the tcgen05 tensor cores.  With a `workspace` (qgemm_workspace_bytes(m, n_in) bytes) the streaming kernel
-  runs: activations split once (with the RMSNorm in front, if its weight is given), roles on separate warps, even deal over the SMs."""
+  runs: activations split once (with the RMSNorm in front, if its weight is given), roles on separate warps, even deal over the SMs.
+  unsplit: no tile's K is split over SMs, every output is one running sum with the bits of the form without a workspace."""
   lib = _lib.load()
   if workspace is not None and PIPELINED_GEMM:
     check(lib.b200q_qgemm_ws_norm(qtype, w_ptr, ptr_of(x), x_dtype, ptr_of(norm_weight), norm_eps, ptr_of(bias), ptr_of(residual), epilogue, ptr_of(y), y_dtype,
-                                  m, n_out, n_in, workspace.ptr, workspace.nbytes, stream_ptr(stream)))
+                                  m, n_out, n_in, workspace.ptr, workspace.nbytes, int(unsplit), stream_ptr(stream)))
     return
   assert norm_weight is None, "the RMSNorm in front is part of the kernel with a workspace"
   check(lib.b200q_qgemm(qtype, w_ptr, ptr_of(x), x_dtype, ptr_of(bias), ptr_of(residual), epilogue, ptr_of(y), y_dtype, m, n_out, n_in,
@@ -111,9 +117,8 @@ def qgemm(w_ptr: int, qtype: int, n_out: int, n_in: int, x, y, m: int, x_dtype=F
 
 
 FEW_ROW_FUSED = os.environ.get("B200Q_FEW_ROW_FUSED", "1") == "1"      # batched decode with few rows: the int8-MMA few-row kernel
-# ... up to this many rows, 8 per pass over the weights (measured at 16 / 32 sequences of the 7B Q8_0 shape: 5.1 / 10.2 ms per step
-# against 10.5 / 11.9 on the tcgen05 few-row GEMM, whose unpacking to fp16 halves costs more than streaming the weights again)
-FEW_ROW_MAX = int(os.environ.get("B200Q_FEW_ROW_MAX", "32"))
+# ... up to this many rows, 8 per pass over the weights (7B Q8_0 gate/up: 34.5 us per pass against 88 for up to 64 rows on the GEMM; down 24 against 73)
+FEW_ROW_MAX = int(os.environ.get("B200Q_FEW_ROW_MAX", "16"))
 
 
 def qgemv_rows_workspace_bytes(m: int, n_out: int, n_in: int) -> int:
