@@ -99,6 +99,9 @@ __device__ __forceinline__ bool elect_one() {
   return e != 0;
 }
 
+// Ask for a line that will be read behind pdl_wait (weights, tables): in a model whose weights exceed L2 it is a DRAM miss by then.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

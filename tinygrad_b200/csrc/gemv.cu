@@ -335,6 +335,7 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
   }
 
   // -------------------------------- consumers --------------------------------
+  if (p.norm_w && blockIdx.x < 8 && (blockIdx.x * 64 + tid) * 64 < p.n_in && tid < 64) prefetch_l2(p.norm_w + (blockIdx.x * 64 + tid) * 64);
   pdl_wait();
   PSTAMP(1);
   const int g = lane >> 2, t = lane & 3;
@@ -344,39 +345,54 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
     // the row arrives quantised (the producer thread copies the record); only the RMSNorm scalar is computed here
     if (p.norm_w) for (int i = tid; i < p.ss_count; i += CONS_THREADS) ss += p.ss_in[i];
   } else {
-    // quantise the activation row here: 8 threads per block of 32, 4 elements each.  The loads of PF blocks are issued
+    // Quantise the activation row here: 4 threads per block of 32, 8 elements each.  The loads of PF blocks are issued
     // before any is used, so a batch costs one L2 round trip instead of one per block.
 #ifndef B200Q_XPF
-#define B200Q_XPF 4
+#define B200Q_XPF 2
 #endif
-    constexpr int PF = B200Q_XPF, BSTEP = CONS_THREADS / 8;
-    const int nblk_pad = p.kgroups * 4, q = tid & 7;
+    constexpr int PF = B200Q_XPF, BSTEP = CONS_THREADS / 4;
+    const int nblk_pad = p.kgroups * 4, q = tid & 3;
     const XqDst dst(record, p.kgroups);
-    for (int b0 = tid >> 3; b0 < nblk_pad; b0 += PF * BSTEP) {
-      float4 v[PF];
-      uint2 nw[PF];
+    for (int w0 = warp * 8; w0 < nblk_pad; w0 += PF * BSTEP) {          // 8 blocks per warp and round
+      const int b0 = w0 + (lane >> 2);
+      float4 v[PF][2];
+      uint4 nw[PF];
 #pragma unroll
       for (int u = 0; u < PF; u++) {
-        const int k = (b0 + u * BSTEP) * 32 + 4 * q;
-        v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-        nw[u] = make_uint2(0x3C003C00u, 0x3C003C00u);      // fp16 ones
+        const int k = (b0 + u * BSTEP) * 32 + 8 * q;
+        v[u][0] = v[u][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        nw[u] = make_uint4(0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u);      // fp16 ones
         if (b0 + u * BSTEP < nblk_pad && k < p.n_in) {
           if (p.x_f16) {
-            const uint2 r = *reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(p.x) + (size_t)m * p.n_in + k);
-            const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&r.x)), c = __half22float2(*reinterpret_cast<const __half2*>(&r.y));
-            v[u] = make_float4(a.x, a.y, c.x, c.y);
+            const uint2 r0 = *reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(p.x) + (size_t)m * p.n_in + k);
+            const uint2 r1 = *reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(p.x) + (size_t)m * p.n_in + k + 4);
+            const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&r0.x)), c = __half22float2(*reinterpret_cast<const __half2*>(&r0.y));
+            const float2 e = __half22float2(*reinterpret_cast<const __half2*>(&r1.x)), f = __half22float2(*reinterpret_cast<const __half2*>(&r1.y));
+            v[u][0] = make_float4(a.x, a.y, c.x, c.y); v[u][1] = make_float4(e.x, e.y, f.x, f.y);
           } else {
-            v[u] = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.x) + (size_t)m * p.n_in + k);
+            const float* src = reinterpret_cast<const float*>(p.x) + (size_t)m * p.n_in + k;
+            v[u][0] = *reinterpret_cast<const float4*>(src); v[u][1] = *reinterpret_cast<const float4*>(src + 4);
           }
-          if (p.norm_w) nw[u] = *reinterpret_cast<const uint2*>(p.norm_w + k);
+          if (p.norm_w) {
+            const uint2 n0 = *reinterpret_cast<const uint2*>(p.norm_w + k), n1 = *reinterpret_cast<const uint2*>(p.norm_w + k + 4);
+            nw[u] = make_uint4(n0.x, n0.y, n1.x, n1.y);
+          }
         }
       }
 #pragma unroll
       for (int u = 0; u < PF; u++) {
-        if (b0 + u * BSTEP < nblk_pad) {      // uniform over the 8 lanes of a block (and over the warp: 4 consecutive blocks)
-          ss = fmaf(v[u].x, v[u].x, fmaf(v[u].y, v[u].y, fmaf(v[u].z, v[u].z, fmaf(v[u].w, v[u].w, ss))));
-          const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&nw[u].x)), c = __half22float2(*reinterpret_cast<const __half2*>(&nw[u].y));
-          quant_block_8x4(make_float4(v[u].x * a.x, v[u].y * a.y, v[u].z * c.x, v[u].w * c.y), q, b0 + u * BSTEP, dst, XSUB ? sub16 : nullptr);
+        if (w0 + u * BSTEP < nblk_pad) {      // uniform over the warp
+          float f[8] = {v[u][0].x, v[u][0].y, v[u][0].z, v[u][0].w, v[u][1].x, v[u][1].y, v[u][1].z, v[u][1].w};
+          if (p.norm_w) {
+            const __half2* h = reinterpret_cast<const __half2*>(&nw[u]);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+              const float2 w = __half22float2(h[i]);
+              ss = fmaf(f[2 * i], f[2 * i], fmaf(f[2 * i + 1], f[2 * i + 1], ss));
+              f[2 * i] *= w.x; f[2 * i + 1] *= w.y;
+            }
+          }
+          quant_block_4x8(f, q, b0 + u * BSTEP, b0 + u * BSTEP < nblk_pad, dst, XSUB ? sub16 : nullptr);
         }
       }
     }
