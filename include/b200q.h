@@ -287,9 +287,13 @@ size_t b200q_argmax_scratch_bytes(void);
 int b200q_argmax_advance(const float* device_logits, int n, int32_t* device_tokens, int32_t* device_pos, int max_context, void* scratch,
                          int flags, void* stream);
 /* The same for n_seqs sequences in one launch: logits [n_seqs, n], tokens rows token_stride apart, pos [n_seqs], scratch n_seqs x
- * b200q_argmax_scratch_bytes, zeroed once. */
+ * b200q_argmax_scratch_bytes, zeroed once.  mirror: NULL, or page-locked host memory (b200q_host_alloc) [n_seqs] that also gets the tokens.
+ * b200q_wait_words: waits until none of n such words is `empty` any more (the host fills them with it before the launch): it polls the
+ * words, which sees a token several microseconds before a stream synchronisation returns, and falls back to one after 20 ms; an error
+ * if the words are still empty then. */
 int b200q_argmax_advance_seqs(const float* logits, int n, int32_t* tokens, int token_stride, int32_t* pos, int max_context, void* scratch, int n_seqs,
-                              int flags, void* stream);
+                              int32_t* mirror, int flags, void* stream);
+int b200q_wait_words(const int32_t* words, int n, int32_t empty, void* stream);
 /* *pos += 1 (a prompt token whose logits are not needed); stops at max_context like b200q_argmax_advance */
 int b200q_advance(int32_t* device_pos, int max_context, int flags, void* stream);
 

@@ -2,6 +2,7 @@
 #include "common.cuh"
 #include <string.h>
 #include <stdio.h>
+#include <chrono>
 
 static thread_local char g_cuda_err[256] = "";
 
@@ -121,6 +122,22 @@ extern "C" int b200q_graph_end(void* stream, void** graph_exec) {
 extern "C" int b200q_graph_launch(void* graph_exec, void* stream) {
   if (!graph_exec) return B200Q_ERR_BAD_ARG;
   B200Q_CHECK_CUDA(cudaGraphLaunch((cudaGraphExec_t)graph_exec, (cudaStream_t)stream));
+  return B200Q_OK;
+}
+extern "C" int b200q_wait_words(const int32_t* words, int n, int32_t empty, void* stream) {
+  if (!words || n <= 0) return B200Q_ERR_BAD_ARG;
+  const volatile int32_t* w = words;
+  auto all = [&]() { for (int i = 0; i < n; i++) if (w[i] == empty) return false; return true; };
+  const auto t0 = std::chrono::steady_clock::now();
+  for (unsigned k = 0; !all(); k++) {
+#if defined(__x86_64__)
+    __builtin_ia32_pause();
+#endif
+    if ((k & 255) == 255 && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(20)) {
+      B200Q_CHECK_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+      return all() ? B200Q_OK : B200Q_ERR_BAD_ARG;
+    }
+  }
   return B200Q_OK;
 }
 extern "C" int b200q_graph_destroy(void* graph_exec) { B200Q_CHECK_CUDA(cudaGraphExecDestroy((cudaGraphExec_t)graph_exec)); return B200Q_OK; }

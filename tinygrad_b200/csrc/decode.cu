@@ -622,7 +622,7 @@ __device__ __forceinline__ void argmax_combine(float& v, int& i, float ov, int o
 }
 
 __global__ void __launch_bounds__(ARGMAX_THREADS) argmax_kernel(const float* __restrict__ logits, int n, int32_t* tokens, int32_t* pos,
-                                                                int max_context, int token_stride, unsigned char* scratch) {
+                                                                int max_context, int token_stride, unsigned char* scratch, int32_t* mirror) {
   __shared__ float wv[ARGMAX_THREADS / 32];
   __shared__ int wi[ARGMAX_THREADS / 32];
   __shared__ int s_last;
@@ -671,7 +671,11 @@ __global__ void __launch_bounds__(ARGMAX_THREADS) argmax_kernel(const float* __r
   if (threadIdx.x == 0) {
     const int p = *pos;
     if (p < 0 || p >= max_context) atomicExch(&g_decode_status, 2);      // tokens[max_context] is the last entry
-    else { tokens[p + 1] = idx == 0x7fffffff ? 0 : idx; *pos = p + 1; }
+    else {
+      const int tok = idx == 0x7fffffff ? 0 : idx;
+      tokens[p + 1] = tok; *pos = p + 1;
+      if (mirror) { __threadfence_system(); *reinterpret_cast<volatile int32_t*>(mirror + blockIdx.y) = tok; }      // the host is waiting for it
+    }
   }
 }
 
@@ -818,15 +822,15 @@ extern "C" int b200q_attn_decode_seqs(const b200q_attn_args* a, int n_seqs, void
 extern "C" size_t b200q_argmax_scratch_bytes(void) { return ARGMAX_SCRATCH; }
 
 extern "C" int b200q_argmax_advance_seqs(const float* logits, int n, int32_t* tokens, int token_stride, int32_t* pos, int max_context, void* scratch, int n_seqs,
-                                         int flags, void* stream) {
+                                         int32_t* mirror, int flags, void* stream) {
   if (!logits || !tokens || !pos || !scratch || n <= 0 || max_context <= 0 || n_seqs <= 0 || n_seqs > 65535 || token_stride < 0) return B200Q_ERR_BAD_ARG;
   int grid = ceil_div(n, ARGMAX_THREADS); if (grid > ARGMAX_CTAS) grid = ARGMAX_CTAS;
   B200Q_CHECK_CUDA(launch_k(argmax_kernel, dim3(grid, n_seqs), dim3(ARGMAX_THREADS), 0, (cudaStream_t)stream, (flags & B200Q_FLAG_PDL) != 0,
-                            logits, n, tokens, pos, max_context, token_stride, (unsigned char*)scratch));
+                            logits, n, tokens, pos, max_context, token_stride, (unsigned char*)scratch, mirror));
   return B200Q_OK;
 }
 extern "C" int b200q_argmax_advance(const float* logits, int n, int32_t* tokens, int32_t* pos, int max_context, void* scratch, int flags, void* stream) {
-  return b200q_argmax_advance_seqs(logits, n, tokens, 0, pos, max_context, scratch, 1, flags, stream);
+  return b200q_argmax_advance_seqs(logits, n, tokens, 0, pos, max_context, scratch, 1, nullptr, flags, stream);
 }
 
 // ---------------------------------------------------------------------------

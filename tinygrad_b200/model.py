@@ -12,7 +12,7 @@ from dataclasses import dataclass
 import numpy as np
 from . import _lib, quant
 from ._lib import check, F32, F16, EPI_LINEAR, EPI_SILU_MUL, FLAG_PDL
-from .runtime import DeviceBuffer, Stream, Graph, Event, synchronize as runtime_sync
+from .runtime import DeviceBuffer, PinnedBuffer, Stream, Graph, Event, synchronize as runtime_sync
 import ctypes, os
 
 # batched decode: attention of all sequences in one launch of the one-token kernel instead of the prompt-pass kernels with one query row
@@ -204,6 +204,7 @@ class Transformer:
     self.pos = DeviceBuffer.empty((batch,), np.int32, zero=True)
     self.seq_cache_bytes = c.n_kv_heads * c.max_context * c.head_dim * np.dtype(kvdt).itemsize
     self.attn_scratch = DeviceBuffer(_lib.load().b200q_attn_scratch_bytes(c.n_heads, c.n_kv_heads, c.head_dim, self.n_split), zero=True)
+    self._mirror = PinnedBuffer((batch,), np.int32)      # the sampled tokens as the arg-max kernel leaves them for the host
     self.argmax_scratch = DeviceBuffer(batch * _lib.load().b200q_argmax_scratch_bytes(), zero=True)
     # Quantised activation hand-over between consecutive kernels (needs whole 128-wide groups everywhere).  Each edge of
     # the chain can be switched on its own: attn_o (attention -> output projection), o_gateup, gateup_down, down_qkv.
@@ -339,8 +340,8 @@ class Transformer:
                    **(dict(peers=self.mb_logits.targets, peer_rank=tp.rank) if peer else {}))
       if peer: self.mb_logits.reduce(self.logits, flags=fl, stream=s)          # every rank's vocabulary slice, handed over
       elif tp is not None: tp.all_gather(self.logits, self.logits_part)
-      if tail: check(lib.b200q_argmax_advance(self.logits.ptr, vocab_full, self.tokens.ptr, self.pos.ptr, c.max_context, self.argmax_scratch.ptr,
-                                              0 if (tp is not None and not peer) else fl, s))
+      if tail: check(lib.b200q_argmax_advance_seqs(self.logits.ptr, vocab_full, self.tokens.ptr, 0, self.pos.ptr, c.max_context, self.argmax_scratch.ptr, 1,
+                                                   self._mirror.ptr, 0 if (tp is not None and not peer) else fl, s))
     elif tail:
       check(lib.b200q_advance(self.pos.ptr, c.max_context, 0 if (tp is not None and not peer) else fl, s))
 
@@ -499,7 +500,7 @@ class Transformer:
       if head_q: gemm(self.output.buf.ptr, self.output_type, c.vocab_size, c.dim, f["xn"], self._batch_logits)
       else: quant.gemv_dense(self.output.buf, self.output.dtype, c.vocab_size, c.dim, f["xn"], self._batch_logits, m=B, stream=s)
     check(lib.b200q_argmax_advance_seqs(self._batch_logits.ptr, c.vocab_size, self.tokens.ptr, c.max_context + 1, self.pos.ptr, c.max_context,
-                                        self.argmax_scratch.ptr, B, FLAG_PDL, s))
+                                        self.argmax_scratch.ptr, B, self._mirror.ptr, FLAG_PDL, s))
     if count: self._host_pos += 1
 
   def _prefill_batch(self, n: int) -> None:
@@ -525,9 +526,7 @@ class Transformer:
     self.pos.copy_from(np.full((B,), L - 1, dtype=np.int32))
     self._host_pos, n = L - 1, L
     while n < c.max_context:
-      self.decode_batch_step()
-      self.stream.synchronize()
-      yield [int(t) for t in self.tokens.numpy((B, c.max_context + 1), np.int32)[:, n]]
+      yield self._sampled(self.decode_batch_step)
       n += 1
 
   def _step_rows(self, with_head: bool) -> None:
@@ -558,7 +557,8 @@ class Transformer:
       else:
         quant.gemv(self.output.buf.ptr, self.output_type, c.vocab_size, c.dim, x_last, self.logits, norm_weight=self.output_norm, norm_eps=c.norm_eps,
                    stream=s)
-      check(lib.b200q_argmax_advance(self.logits.ptr, c.vocab_size, self.tokens.ptr, self.pos.ptr, c.max_context, self.argmax_scratch.ptr, 0, s))
+      check(lib.b200q_argmax_advance_seqs(self.logits.ptr, c.vocab_size, self.tokens.ptr, 0, self.pos.ptr, c.max_context, self.argmax_scratch.ptr, 1,
+                                          self._mirror.ptr, 0, s))
     else:
       check(lib.b200q_advance(self.pos.ptr, c.max_context, 0, s))
 
@@ -601,9 +601,23 @@ class Transformer:
     self.pos.copy_from(np.array([pos], dtype=np.int32))
     self._host_pos = pos
 
+  def _put_tokens(self, tokens: list, pos: int) -> None:
+    """set_state for a prompt whose first `pos` tokens are in the cache: only the others are copied, in stream order (no waiting)."""
+    self.tokens.copy_from(np.asarray(tokens[pos:], dtype=np.int32), stream=self.stream, offset=4 * pos)
+    self.pos.copy_from(np.array([pos], dtype=np.int32), stream=self.stream)
+    self._host_pos = pos
+
   def read_token(self, index: int) -> int:
     self.stream.synchronize()
     return int(self.tokens.numpy((1,), np.int32, offset=4 * index)[0])
+
+  def _sampled(self, step) -> list:
+    """Run `step` and wait for the tokens it samples: the arg-max kernel also writes them to page-locked memory, which is polled."""
+    m = self._mirror.array
+    m[:] = -1
+    step()
+    check(_lib.load().b200q_wait_words(self._mirror.ptr, len(m), -1, self.stream.ptr))
+    return m.tolist()
 
   def read_logits(self) -> np.ndarray:
     self.stream.synchronize()
@@ -611,11 +625,14 @@ class Transformer:
 
   def get_start_pos(self, tokens: list) -> int:
     """How much of the KV cache the new prompt can reuse (model.py:456-462)."""
-    n = 0
-    for a, b in zip(tokens[:-1], self._cached_tokens):
-      if a != b: break
-      n += 1
-    return n
+    n, old = min(len(tokens) - 1, len(self._cached_tokens)), self._cached_tokens
+    if tokens[:n] == old[:n]: return n
+    lo = 0                                    # tokens[:lo] agree, tokens[:n] do not
+    while n - lo > 1:
+      mid = (lo + n) // 2
+      if tokens[lo:mid] == old[lo:mid]: lo = mid
+      else: n = mid
+    return lo
 
   def generate(self, tokens: list, temperature: float = 0.0):
     """Greedy generation (model.py:464-484 at temperature 0).  Yields one token id at a time;
@@ -623,14 +640,16 @@ class Transformer:
     if temperature != 0.0: raise NotImplementedError("only greedy decoding (temperature 0) is implemented")
     tokens = list(tokens)
     start_pos = self.get_start_pos(tokens)
-    self.set_state(tokens, start_pos)
+    self._put_tokens(tokens, start_pos)
     n_pre = len(tokens) - 1 - start_pos
     if self.prefill_rows and n_pre >= min(self.prefill_rows, SHORT_PROMPT_ROWS): self.prefill(start_pos, n_pre)
     else:
       for _ in range(n_pre): self.step(with_head=False)
     while len(tokens) < self.max_context:
-      self.step(with_head=True)
-      tok = self.read_token(len(tokens))
+      if self._step_args:
+        self.step(with_head=True)
+        tok = self.read_token(len(tokens))
+      else: tok = self._sampled(self.step)[0]
       tokens.append(tok)
       self._cached_tokens = tokens[:-1]
       yield tok

@@ -104,6 +104,10 @@ class PinnedBuffer:
       _lib.load().b200q_host_free(self.ptr)
       self.ptr = 0
 
+  def __del__(self):
+    try: self.free()
+    except Exception: pass
+
 
 def stream_ptr(stream) -> int:
   return 0 if stream is None else (stream.ptr if isinstance(stream, Stream) else int(stream))
