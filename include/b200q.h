@@ -39,6 +39,9 @@ extern "C" {
 #define B200Q_Q4_K 12
 #define B200Q_Q5_K 13
 #define B200Q_Q6_K 14
+#define B200Q_WIDE 64        /* added to Q4_K / Q6_K for a packed weight that meets full-precision activations (b200q_packed_bytes, b200q_repack, b200q_gemv) */
+#define B200Q_Q4_K_WIDE (B200Q_WIDE + B200Q_Q4_K)
+#define B200Q_Q6_K_WIDE (B200Q_WIDE + B200Q_Q6_K)
 /* element types of activations / outputs */
 #define B200Q_F32 0
 #define B200Q_F16 1
@@ -119,6 +122,8 @@ int b200q_dequant_raw(int qtype, const void* device_raw, void* device_out, int64
  *                       [lane l: 8 bytes of high bit pairs: byte k of word 0 holds elements k, 4+k, 8+k, 12+k at bits 0, 2, 4, 6;
  *                        word 1 the same for elements 16..31] x32, the same for rows +8,
  *                       int8 sub-block scales [16 rows][8], fp16 super-block scales [16 rows]  (106 bytes per row against 105 in the file).
+ *   Q4_K_WIDE tile = 1216 B (n_in a multiple of 256): the quants as in Q4_0, uint8 {scale, minimum} of the 4 blocks [16 rows][4][2],
+ *                       fp16 {d, dmin} [16 rows]  (76 bytes per row against 72 in the file).  Q6_K_WIDE tile = Q6_K tile.
  * The bytes per weight element are exactly the GGUF format's for Q4_0 / Q8_0 (18 or 34 bytes per 32).
  * n_out is padded up to a multiple of 16 and n_in to a multiple of 128 with zero-scale blocks.
  * With raw1 != NULL two matrices of equal shape are interleaved 8 rows at a
@@ -139,8 +144,11 @@ int b200q_dequant_packed(int qtype, const void* device_packed, void* device_out,
  * activation row.  Activations are quantised on the fly to 15-bit integers with one fp32 scale per 32
  * (error ~3e-5 relative, far inside the 1e-2 tolerance of this path); products and sums inside a block
  * are exact integers, accumulation across blocks is fp32. */
+#define B200Q_WIDE_MAX_IN 27648
 typedef struct b200q_gemv_args {
-  int qtype;                /* B200Q_Q4_0 | B200Q_Q8_0 | B200Q_Q6_K (plain linears: EPI_LINEAR, no xq_in; n_in a multiple of 256) */
+  int qtype;                /* B200Q_Q4_0 | B200Q_Q8_0 | B200Q_Q6_K (plain linears: EPI_LINEAR, no xq_in; n_in a multiple of 256) |
+                               B200Q_Q4_K_WIDE | B200Q_Q6_K_WIDE (activations as two fp16 numbers, within 2^-23 of the fp32 value; no hand-over
+                               records; n_in a multiple of 256, at most B200Q_WIDE_MAX_IN) */
   int n_out;                /* logical output features (for EPI_SILU_MUL: features of gate == up) */
   int n_in;                 /* input features, multiple of 32 */
   int m;                    /* activation rows (1 at decode) */

@@ -7,6 +7,7 @@ import os
 LIB_PATH = pathlib.Path(os.environ.get("B200Q_LIB") or pathlib.Path(__file__).resolve().parent / "libb200q.so")   # B200Q_LIB: another build of the library
 
 Q4_0, Q8_0, Q6_K = 2, 8, 14
+Q4_K_WIDE, Q6_K_WIDE, WIDE_MAX_IN = 64 + 12, 64 + 14, 27648      # packed K-quant weights that meet full-precision activations (b200q.h)
 F32, F16, BF16 = 0, 1, 2
 EPI_LINEAR, EPI_SILU_MUL = 0, 1
 FLAG_PDL = 1

@@ -54,7 +54,7 @@ constexpr int TILE_ROWS = 16;       // output rows per tile (one mma.m16n8k16 A 
 constexpr int GROUP_ELEMS = 128;    // K elements per tile: 4 quant blocks of 32 (Q4_0/Q8_0), half a super-block (Q6_K)
 
 __host__ __device__ constexpr int tile_bytes(int qtype) {
-  return qtype == B200Q_Q4_0 ? 1152 : qtype == B200Q_Q8_0 ? 2176 : qtype == B200Q_Q6_K ? 1696 : 0;
+  return qtype == B200Q_Q4_0 ? 1152 : qtype == B200Q_Q8_0 ? 2176 : qtype == B200Q_Q6_K || qtype == B200Q_Q6_K_WIDE ? 1696 : qtype == B200Q_Q4_K_WIDE ? 1216 : 0;
 }
 
 static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }

@@ -24,6 +24,7 @@
 #include "common.cuh"
 #include "actquant.cuh"
 #include "qgemv_core.cuh"
+#include "kquant_wide.cuh"
 
 namespace {
 
@@ -80,6 +81,11 @@ template <int QT> struct Cfg;      // NS: ring depth, SG: weight tiles per stage
 template <> struct Cfg<B200Q_Q4_0> { static constexpr int NS = B200Q_NS_Q4, SG = STAGE_GROUPS, XSUB = 0; };   // stage = SG x 1152 B
 template <> struct Cfg<B200Q_Q8_0> { static constexpr int NS = 2, SG = STAGE_GROUPS, XSUB = 0; };             // stage = SG x 2176 B
 template <> struct Cfg<B200Q_Q6_K> { static constexpr int NS = 3, SG = CONS_WARPS, XSUB = 32; };              // stage = SG x 1696 B
+// K-quants against full-precision activations: the record takes 512 bytes per 128 columns.  Two CTAs fit on an SM up to 8192 columns, above that one.
+// Two Q4_K tiles per warp and stage: 4 % over one (14336 x 4096 gate / up); Q6_K tiles are too large for that with two CTAs.
+template <> struct Cfg<B200Q_Q4_K_WIDE> { static constexpr int NS = 2, SG = STAGE_GROUPS, XSUB = 0; };        // stage = SG x 1216 B
+template <> struct Cfg<B200Q_Q6_K_WIDE> { static constexpr int NS = 3, SG = CONS_WARPS, XSUB = 0; };          // stage = SG x 1696 B
+template <int QT> constexpr int X_BYTES = is_wide(QT) ? 512 : XQ_GROUP_BYTES;  // staged bytes per 128 columns
 
 #ifdef B200Q_GEMV_PROF
 // experiment build only: per-launch time stamps of CTA 0 (entry, dependency resolved, row staged, first stage landed, tiles done, exit)
@@ -152,14 +158,16 @@ __device__ __noinline__ void settle_handover(const GemvParams& p, float* ubuf, i
 template <int QT, bool XQ_IN, bool XQ_OUT>
 __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(const GemvParams p) {
   constexpr int NS = Cfg<QT>::NS, SG = Cfg<QT>::SG, XSUB = Cfg<QT>::XSUB, TB = tile_bytes(QT), STAGE_BYTES = SG * TB;
-  static_assert(!(XQ_IN && XSUB), "a ready-made record carries no per-sub-block sums");
+  constexpr bool WIDE = is_wide(QT);
+  constexpr int XB = X_BYTES<QT>;
+  static_assert(!(XQ_IN && (XSUB || WIDE)), "ready-made records are the plain int8 form");
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned char* ring = smem;
   unsigned char* record = smem + NS * STAGE_BYTES;
   const uint4* xq = reinterpret_cast<const uint4*>(record);
   const float4* xsc = reinterpret_cast<const float4*>(record + (size_t)p.kgroups * 256);
-  float* sub16 = reinterpret_cast<float*>(record + (size_t)p.kgroups * XQ_GROUP_BYTES);        // [kgroups][4 blocks][2 halves], Q6_K only
-  uint4* zero = reinterpret_cast<uint4*>(record + (size_t)p.kgroups * (XQ_GROUP_BYTES + XSUB));
+  float* sub16 = reinterpret_cast<float*>(record + (size_t)p.kgroups * XB);        // [kgroups][4 blocks][2 halves], Q6_K only
+  uint4* zero = reinterpret_cast<uint4*>(record + (size_t)p.kgroups * (XB + XSUB));
   float* red = reinterpret_cast<float*>(zero + 1);
   float* ssq = red + 2 * CONS_WARPS * 16;
   float* ubuf = ssq + CONS_WARPS;
@@ -341,6 +349,7 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
   const int g = lane >> 2, t = lane & 3;
   if (tid == 0) *zero = make_uint4(0, 0, 0, 0);
   float ss = 0.f;
+  [[maybe_unused]] float amax = 0.f, x_up = 0.f, x_down = 0.f;       // full precision: largest magnitude of the row, its power of two and the inverse
   if (XQ_IN) {
     // the row arrives quantised (the producer thread copies the record); only the RMSNorm scalar is computed here
     if (p.norm_w) for (int i = tid; i < p.ss_count; i += CONS_THREADS) ss += p.ss_in[i];
@@ -353,6 +362,18 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
     constexpr int PF = B200Q_XPF, BSTEP = CONS_THREADS / 4;
     const int nblk_pad = p.kgroups * 4, q = tid & 3;
     const XqDst dst(record, p.kgroups);
+#pragma unroll 1
+    for (int pass = 0; pass < (WIDE ? 2 : 1); pass++) {                 // full precision: first the row's largest value, then the values (from L1)
+    if constexpr (WIDE) {
+      if (pass == 1) {
+        amax = warp_max(amax);
+        if (lane == 0) red[warp] = amax;
+        cons_bar_sync();
+#pragma unroll
+        for (int w = 0; w < CONS_WARPS; w++) amax = fmaxf(amax, red[w]);
+        wide_row_scale(amax, x_up, x_down);
+      }
+    }
     for (int w0 = warp * 8; w0 < nblk_pad; w0 += PF * BSTEP) {          // 8 blocks per warp and round
       const int b0 = w0 + (lane >> 2);
       float4 v[PF][2];
@@ -388,13 +409,19 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
 #pragma unroll
             for (int i = 0; i < 4; i++) {
               const float2 w = __half22float2(h[i]);
-              ss = fmaf(f[2 * i], f[2 * i], fmaf(f[2 * i + 1], f[2 * i + 1], ss));
+              if (pass == 0) ss = fmaf(f[2 * i], f[2 * i], fmaf(f[2 * i + 1], f[2 * i + 1], ss));
               f[2 * i] *= w.x; f[2 * i + 1] *= w.y;
             }
           }
-          quant_block_4x8(f, q, b0 + u * BSTEP, b0 + u * BSTEP < nblk_pad, dst, XSUB ? sub16 : nullptr);
+          if constexpr (WIDE) {
+            if (pass == 0) {
+#pragma unroll
+              for (int i = 0; i < 8; i++) amax = fmaxf(amax, fabsf(f[i]));
+            } else if (b0 + u * BSTEP < nblk_pad) wide_store_8(f, q, b0 + u * BSTEP, x_up, record);
+          } else quant_block_4x8(f, q, b0 + u * BSTEP, b0 + u * BSTEP < nblk_pad, dst, XSUB ? sub16 : nullptr);
         }
       }
+    }
     }
   }
   if (p.norm_w) {
@@ -413,6 +440,7 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
       const int rt = unit * run + ti;
       if (rt >= p.n_row_tiles) break;
       float acc0 = 0.f, acc1 = 0.f;
+      [[maybe_unused]] float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
       for (int s = 0; s < stages_per_tile; s++, it++) {
         const int slot = it % NS, groups = min(SG, p.kgroups - s * SG);
         if (!mbar_wait(full0 + 8 * slot, (it / NS) & 1)) { *s_abort = 1; break; }
@@ -423,18 +451,24 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
           const int gi = warp + u * CONS_WARPS;
           if (gi < groups) {
             const int j = s * SG + gi;
-            // the address is selected, not the loaded value: `diag ? xq[..] : *zero` compiled to a divergent branch around the loads
-            // (5 % of the decode step)
-            const uint4* q0 = diag ? xq + (j * 2 + 0) * 8 + g : zero;
-            const uint4* q1 = diag ? xq + (j * 2 + 1) * 8 + g : zero;
-            const uint4 bq0 = *q0, bq1 = *q1;
-            const float4 st = xsc[(j * 2 + (t >> 1)) * 2 + (t & 1)];
-            if constexpr (QT == B200Q_Q6_K) {
-              // the offsets belong to the high digits only (their columns sit on the lanes t < 2)
-              const float4 sub = *(t < 2 ? reinterpret_cast<const float4*>(sub16 + j * 8 + t * 4) : reinterpret_cast<const float4*>(zero));
-              tile_mac_q6k(stage + gi * TB, lane, bq0, bq1, st, sub, acc0, acc1);
+            if constexpr (WIDE) {
+              const uint4* xb = xq + j * 32 + (g & 1) * 4 + t;
+              if constexpr (QT == B200Q_Q4_K_WIDE) tile_mac_q4k(stage + gi * TB, lane, xb, c0, c1);
+              else tile_mac_q6k_wide(stage + gi * TB, lane, xb, c0, c1);
             } else {
-              tile_mac<QT>(stage + gi * TB, lane, bq0, bq1, st, acc0, acc1);
+              const float4 st = xsc[(j * 2 + (t >> 1)) * 2 + (t & 1)];
+              // the address is selected, not the loaded value: `diag ? xq[..] : *zero` compiled to a divergent branch around the loads
+              // (5 % of the decode step)
+              const uint4* q0 = diag ? xq + (j * 2 + 0) * 8 + g : zero;
+              const uint4* q1 = diag ? xq + (j * 2 + 1) * 8 + g : zero;
+              const uint4 bq0 = *q0, bq1 = *q1;
+              if constexpr (QT == B200Q_Q6_K) {
+                // the offsets belong to the high digits only (their columns sit on the lanes t < 2)
+                const float4 sub = *(t < 2 ? reinterpret_cast<const float4*>(sub16 + j * 8 + t * 4) : reinterpret_cast<const float4*>(zero));
+                tile_mac_q6k(stage + gi * TB, lane, bq0, bq1, st, sub, acc0, acc1);
+              } else {
+                tile_mac<QT>(stage + gi * TB, lane, bq0, bq1, st, acc0, acc1);
+              }
             }
           }
         }
@@ -442,9 +476,14 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
         if (lane == 0) mbar_arrive(empty0 + 8 * slot);
       }
       PSTAMP(4);
-      // quad lanes hold the columns {blocks 0,1 hi}, {2,3 hi}, {0,1 lo}, {2,3 lo}: add them
-      acc0 += __shfl_xor_sync(0xffffffffu, acc0, 1); acc0 += __shfl_xor_sync(0xffffffffu, acc0, 2);
-      acc1 += __shfl_xor_sync(0xffffffffu, acc1, 1); acc1 += __shfl_xor_sync(0xffffffffu, acc1, 2);
+      if constexpr (WIDE) {      // even columns: high parts, odd: remainders x 2^11
+        acc0 = fmaf(c0[1] + c1[1], 1.f / 2048.f, c0[0] + c1[0]) * x_down;
+        acc1 = fmaf(c0[3] + c1[3], 1.f / 2048.f, c0[2] + c1[2]) * x_down;
+      } else {
+        // quad lanes hold the columns {blocks 0,1 hi}, {2,3 hi}, {0,1 lo}, {2,3 lo}: add them
+        acc0 += __shfl_xor_sync(0xffffffffu, acc0, 1); acc0 += __shfl_xor_sync(0xffffffffu, acc0, 2);
+        acc1 += __shfl_xor_sync(0xffffffffu, acc1, 1); acc1 += __shfl_xor_sync(0xffffffffu, acc1, 2);
+      }
       // hand the partial sums to the finisher: buffer n & 1, free again once the finisher has read tile n - 2
       const int par = n & 1;
       if (n >= 2 && !mbar_wait(rempty0 + 8 * par, ((n >> 1) - 1) & 1)) *s_abort = 1;
@@ -478,7 +517,7 @@ namespace {
 template <int QT, bool XQ_IN, bool XQ_OUT>
 int launch_gemv(const b200q_gemv_args* a, const GemvParams& p, cudaStream_t stream) {
   constexpr int NS = Cfg<QT>::NS;
-  const size_t smem = (size_t)NS * Cfg<QT>::SG * tile_bytes(QT) + (size_t)p.kgroups * (XQ_GROUP_BYTES + Cfg<QT>::XSUB) + 16 +
+  const size_t smem = (size_t)NS * Cfg<QT>::SG * tile_bytes(QT) + (size_t)p.kgroups * (X_BYTES<QT> + Cfg<QT>::XSUB) + 16 +
                       (2 * CONS_WARPS * 16 + CONS_WARPS + 32) * sizeof(float) + (2 * NS + 5) * sizeof(uint64_t) + 16;
   if (smem > 220 * 1024) return B200Q_ERR_TOO_LARGE;
   auto kern = qgemv_kernel<QT, XQ_IN, XQ_OUT>;
@@ -541,9 +580,12 @@ extern "C" size_t b200q_xq_bytes(int n) { return n > 0 ? xq_record_bytes(n) : 0;
 
 extern "C" int b200q_gemv(const b200q_gemv_args* a, void* stream) {
   if (!a || !a->w_packed || (!a->x && !a->xq_in) || (!a->y && !a->xq_out && !a->n_peers)) return B200Q_ERR_BAD_ARG;
-  if (a->qtype != B200Q_Q4_0 && a->qtype != B200Q_Q8_0 && a->qtype != B200Q_Q6_K) return B200Q_ERR_BAD_ARG;
+  const bool wide = is_wide(a->qtype), kquant = wide || a->qtype == B200Q_Q6_K;
+  if (a->qtype != B200Q_Q4_0 && a->qtype != B200Q_Q8_0 && !kquant) return B200Q_ERR_BAD_ARG;
   if (a->n_out <= 0 || a->n_in <= 0 || a->m <= 0 || a->m > 65535) return B200Q_ERR_BAD_ARG;
-  if (a->n_in % (a->qtype == B200Q_Q6_K ? 256 : 32)) return B200Q_ERR_BAD_SHAPE;
+  if (a->n_in % (kquant ? 256 : 32)) return B200Q_ERR_BAD_SHAPE;
+  if (wide && a->n_in > B200Q_WIDE_MAX_IN) return B200Q_ERR_TOO_LARGE;
+  if (wide && (a->xq_in || a->xq_out)) return B200Q_ERR_UNSUPPORTED;
   // Q6_K: plain linears only, and the kernel quantises the activations itself (it needs sums per 16-element sub-block)
   if (a->qtype == B200Q_Q6_K && (a->epilogue != B200Q_EPI_LINEAR || a->xq_in)) return B200Q_ERR_UNSUPPORTED;
   if ((a->x_dtype != B200Q_F32 && a->x_dtype != B200Q_F16) || (a->y_dtype != B200Q_F32 && a->y_dtype != B200Q_F16)) return B200Q_ERR_BAD_ARG;
@@ -581,6 +623,8 @@ extern "C" int b200q_gemv(const b200q_gemv_args* a, void* stream) {
   p.unit = (a->xq_out && !a->xq_out_stage) ? (a->epilogue == B200Q_EPI_SILU_MUL ? 4 : 2) : 1;
   p.n_units = ceil_div(p.n_row_tiles, p.unit);
   const bool xi = a->xq_in != nullptr, xo = a->xq_out != nullptr;
+  if (a->qtype == B200Q_Q4_K_WIDE) return launch_gemv<B200Q_Q4_K_WIDE, false, false>(a, p, (cudaStream_t)stream);
+  if (a->qtype == B200Q_Q6_K_WIDE) return launch_gemv<B200Q_Q6_K_WIDE, false, false>(a, p, (cudaStream_t)stream);
   if (a->qtype == B200Q_Q4_0) {
     if (xi) return xo ? launch_gemv<B200Q_Q4_0, true, true>(a, p, (cudaStream_t)stream) : launch_gemv<B200Q_Q4_0, true, false>(a, p, (cudaStream_t)stream);
     return xo ? launch_gemv<B200Q_Q4_0, false, true>(a, p, (cudaStream_t)stream) : launch_gemv<B200Q_Q4_0, false, false>(a, p, (cudaStream_t)stream);

@@ -114,14 +114,15 @@ __device__ __forceinline__ int q6k_quant(const uint8_t* b, int e) {
   const int xl = (b[hh * 64 + (m & 63)] >> ((m >> 6) * 4)) & 0xF, xh = (b[128 + hh * 32 + (m & 31)] >> ((m >> 5) * 2)) & 3;
   return xl | (xh << 4);
 }
-__global__ void repack_q6k_kernel(const uint8_t* __restrict__ raw, uint8_t* __restrict__ packed, int n_out, int nsb, int n_row_tiles, int kgroups) {
+__global__ void repack_q6k_kernel(const uint8_t* __restrict__ raw0, const uint8_t* __restrict__ raw1, uint8_t* __restrict__ packed, int n_out, int nsb, int n_row_tiles, int kgroups) {
   int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t total = (int64_t)n_row_tiles * kgroups * 64;
   if (idx >= total) return;
   const int l = (int)(idx & 31), h = (int)((idx >> 5) & 1);
   const int64_t tile = idx >> 6;
   const int j = (int)(tile % kgroups), rt = (int)(tile / kgroups);
-  const int g = l >> 2, t = l & 3, row = rt * 16 + h * 8 + g, sb = j >> 1, e0 = (j & 1) * 128 + t * 32;
+  const int g = l >> 2, t = l & 3, row = raw1 ? rt * 8 + g : rt * 16 + h * 8 + g, sb = j >> 1, e0 = (j & 1) * 128 + t * 32;
+  const uint8_t* raw = raw1 && h ? raw1 : raw0;
   uint8_t* tp = packed + tile * 1696;
   uint32_t lw[4] = {0u, 0u, 0u, 0u}, hw[2] = {0u, 0u};
   int sc0 = 0, sc1 = 0;
@@ -142,6 +143,37 @@ __global__ void repack_q6k_kernel(const uint8_t* __restrict__ raw, uint8_t* __re
   tp[1536 + (h * 8 + g) * 8 + t * 2] = (uint8_t)sc0;
   tp[1536 + (h * 8 + g) * 8 + t * 2 + 1] = (uint8_t)sc1;
   if (t == 0) reinterpret_cast<unsigned short*>(tp + 1664)[h * 8 + g] = d;
+}
+
+// Q4_K re-tiling (tile layout: tile_mac_q4k, kquant_wide.cuh).  Element e of a super-block: nibble (e >> 5) & 1 of byte 16 + (e >> 6) * 32 + (e & 31);
+// the 6-bit scales and minima of the eight blocks of 32 share 12 bytes (tinygrad/llm/gguf.py:57-67).
+__global__ void repack_q4k_kernel(const uint8_t* __restrict__ raw0, const uint8_t* __restrict__ raw1, uint8_t* __restrict__ packed, int n_out, int nsb,
+                                  int n_row_tiles, int kgroups) {
+  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, total = (int64_t)n_row_tiles * kgroups * 64;
+  if (idx >= total) return;
+  const int l = (int)(idx & 31), h = (int)((idx >> 5) & 1);
+  const int64_t tile = idx >> 6;
+  const int j = (int)(tile % kgroups), rt = (int)(tile / kgroups);
+  const int g = l >> 2, t = l & 3, row = raw1 ? rt * 8 + g : rt * 16 + h * 8 + g, sb = j >> 1, grp = (j & 1) * 4 + t;
+  const uint8_t* raw = raw1 && h ? raw1 : raw0;
+  uint8_t* tp = packed + tile * 1216;
+  uint32_t lw[4] = {0u, 0u, 0u, 0u};
+  int sc = 0, mn = 0;
+  uint32_t dd = 0;               // a padded row contributes nothing
+  if (row < n_out && sb < nsb) {
+    const uint8_t* b = raw + ((int64_t)row * nsb + sb) * 144;
+    const uint8_t* s = b + 4;
+    const uint8_t* q = b + 16 + (grp >> 1) * 32;
+    for (int i = 0; i < 16; i++)
+      lw[i >> 2] |= (uint32_t)(((q[i] >> ((grp & 1) * 4)) & 15) | (((q[i + 16] >> ((grp & 1) * 4)) & 15) << 4)) << ((i & 3) * 8);
+    if (grp < 4) { sc = s[grp] & 63; mn = s[4 + grp] & 63; }
+    else { sc = (s[4 + grp] & 0xF) | ((s[grp - 4] >> 6) << 4); mn = (s[4 + grp] >> 4) | ((s[grp] >> 6) << 4); }
+    dd = b[0] | (b[1] << 8) | (b[2] << 16) | ((uint32_t)b[3] << 24);
+  }
+  reinterpret_cast<uint4*>(tp)[h * 32 + l] = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+  tp[1024 + (h * 8 + g) * 8 + t * 2] = (uint8_t)sc;
+  tp[1024 + (h * 8 + g) * 8 + t * 2 + 1] = (uint8_t)mn;
+  if (t == 0) reinterpret_cast<uint32_t*>(tp + 1152)[h * 8 + g] = dd;
 }
 
 template <typename OutT>
@@ -223,22 +255,25 @@ extern "C" int b200q_dequant_raw(int qtype, const void* raw, void* out, int64_t 
   return B200Q_OK;
 }
 
+static bool is_kquant(int q) { return q == B200Q_Q6_K || q == B200Q_Q4_K_WIDE || q == B200Q_Q6_K_WIDE; }
+
 extern "C" size_t b200q_packed_bytes(int qtype, int n_out, int n_in) {
-  if ((qtype != B200Q_Q4_0 && qtype != B200Q_Q8_0 && qtype != B200Q_Q6_K) || n_out <= 0 || n_in <= 0) return 0;
-  if (qtype == B200Q_Q6_K && n_in % 256) return 0;
+  if (n_out <= 0 || n_in <= 0 || tile_bytes(qtype) == 0) return 0;
+  if (is_kquant(qtype) && n_in % 256) return 0;
   return (size_t)ceil_div(n_out, TILE_ROWS) * ceil_div(n_in, GROUP_ELEMS) * tile_bytes(qtype);
 }
 
 extern "C" int b200q_repack(int qtype, const void* raw0, const void* raw1, void* packed, int n_out, int n_in, void* stream) {
-  if (qtype != B200Q_Q4_0 && qtype != B200Q_Q8_0 && qtype != B200Q_Q6_K) return B200Q_ERR_BAD_ARG;
+  if (tile_bytes(qtype) == 0) return B200Q_ERR_BAD_ARG;
   if (!raw0 || !packed || n_out <= 0 || n_in <= 0) return B200Q_ERR_BAD_ARG;
-  if (n_in % (qtype == B200Q_Q6_K ? 256 : 32)) return B200Q_ERR_BAD_SHAPE;
+  if (n_in % (is_kquant(qtype) ? 256 : 32)) return B200Q_ERR_BAD_SHAPE;
   if ((uintptr_t)packed & 15) return B200Q_ERR_MISALIGNED;
-  if (qtype == B200Q_Q6_K) {
-    if (raw1) return B200Q_ERR_UNSUPPORTED;       // no interleaved gate / up tiles for this format
-    const int nrt = ceil_div(n_out, TILE_ROWS), kg = n_in / GROUP_ELEMS;
-    const int64_t tot = (int64_t)nrt * kg * 64;
-    repack_q6k_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, (cudaStream_t)stream>>>((const uint8_t*)raw0, (uint8_t*)packed, n_out, n_in / 256, nrt, kg);
+  if (is_kquant(qtype)) {
+    if (raw1 && qtype == B200Q_Q6_K) return B200Q_ERR_UNSUPPORTED;       // its GEMV has no SwiGLU epilogue
+    const int nrt = raw1 ? ceil_div(n_out, 8) : ceil_div(n_out, TILE_ROWS), kg = n_in / GROUP_ELEMS;
+    const unsigned blocks = (unsigned)(((int64_t)nrt * kg * 64 + 255) / 256);
+    auto kernel = qtype == B200Q_Q4_K_WIDE ? repack_q4k_kernel : repack_q6k_kernel;
+    kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>((const uint8_t*)raw0, (const uint8_t*)raw1, (uint8_t*)packed, n_out, n_in / 256, nrt, kg);
     B200Q_CHECK_CUDA(cudaGetLastError());
     return B200Q_OK;
   }

@@ -13,7 +13,7 @@ import numpy as np
 from . import _lib, quant
 from ._lib import check, F32, F16, EPI_LINEAR, EPI_SILU_MUL, FLAG_PDL
 from .runtime import DeviceBuffer, PinnedBuffer, Stream, Graph, Event, synchronize as runtime_sync
-import ctypes, os
+import ctypes, itertools, os
 
 # batched decode with an fp32 cache or another head_dim: attention of all sequences in one launch of the one-lane-per-position decode kernel
 # instead of the prompt-pass kernels with one query row per CTA (measured 1.4 % slower at 8 sequences x 130 positions: off unless asked for)
@@ -62,6 +62,26 @@ class _Block:
   pass
 
 
+class _BlockLinear:
+  """A Linear of a block that keeps full-precision activations: a packed K-quant matrix, or an fp16 one (qtype None).  `row0`: where its rows
+  start in the vector it writes."""
+  def __init__(self, qtype, n_out: int, n_in: int, buf: DeviceBuffer, row0: int, swiglu: bool = False):
+    self.qtype, self.n_out, self.n_in, self.buf, self.row0, self.swiglu = qtype, n_out, n_in, buf, row0, swiglu
+
+  @property
+  def algorithmic_bytes(self) -> int:
+    if self.qtype is None: return 2 * self.n_out * self.n_in
+    return quant.PackedWeight(self.qtype, self.n_out, self.n_in, self.buf, self.swiglu).algorithmic_bytes
+
+  def run(self, x, y, bias=None, residual=None, flags=0, **kw) -> None:
+    at = lambda buf, size: None if buf is None else buf.ptr + size * self.row0
+    if self.qtype is None:
+      quant.gemv_dense(self.buf, F16, self.n_out, self.n_in, x, at(y, 4), bias=at(bias, 2), residual=at(residual, 4), flags=flags, **kw)
+    else:
+      quant.gemv(self.buf.ptr, self.qtype, self.n_out, self.n_in, x, at(y, 4), bias=at(bias, 2), residual=at(residual, 4), flags=flags,
+                 epilogue=EPI_SILU_MUL if self.swiglu else quant.EPI_LINEAR, **kw)
+
+
 # hand-over edges used when the caller does not choose (see Transformer.__init__): the ones that measured faster
 DEFAULT_HANDOVER = tuple(e for e in os.environ.get("B200Q_HANDOVER", "attn_o").split(",") if e)
 STAGED_HANDOVER = os.environ.get("B200Q_STAGED_HANDOVER", "1") == "1"
@@ -81,8 +101,9 @@ class Transformer:
     block chained with programmatic dependent launch and replayed as a CUDA graph (the default: at batch 1 it measured faster, the
     grid-wide waits inside one kernel costing more than kernel boundaries do).
     linear_types: state-dict name -> GGML type of block Linear weights whose type is not `ggml_type` (files that mix block formats, e.g.
-    Q4_K with Q6_K).  Unless every block Linear is of one fused type (Q4_0 / Q8_0) the blocks run on the dense-weight GEMV: every
-    weight is dequantised once to fp16 on the device -- the cast the reference applies to every loaded tensor (model.py:376).
+    Q4_K with Q6_K).  Unless every block Linear is of one fused type (Q4_0 / Q8_0) the blocks keep their activations in full
+    precision: Q4_K and Q6_K weights stay in their file form and run the K-quant GEMV, the others are dequantised once to fp16 on the device (the
+    cast the reference applies to every loaded tensor, model.py:376) and run the dense-weight GEMV.
     batch: sequences decoded in lock-step (`generate_batch`): one KV cache per sequence, every Linear a tensor-core GEMM over the
     batch rows (the reference's forward on tokens [B, T], model.py:358-364; its cache is sized by the first call's batch, model.py:200-203)."""
     self.tp, self.full_config = tp, config
@@ -115,18 +136,37 @@ class Transformer:
         raw, typ = sd[name], lt.get(name, ggml_type)
         if typ in quant.GGML_QUANT: return quant.dequantize(np.ascontiguousarray(raw).view(np.uint8).reshape(-1), n_out * n_in, typ, np.float16)
         return DeviceBuffer.from_numpy(np.asarray(raw).astype(np.float16).reshape(n_out, n_in))
+      def wide(name, n_in):                 # the packed type of a Linear the K-quant GEMV takes, else None
+        return quant.WIDE_QUANT.get(lt.get(name, ggml_type)) if n_in % 256 == 0 and n_in <= _lib.WIDE_MAX_IN else None
+      def stacked(names, rows, n_in):       # Linears that read the same vector: neighbours of one type become one matrix
+        out, at = [], 0
+        for typ, run in itertools.groupby(zip(names, rows), key=lambda nr: wide(nr[0], n_in)):
+          run = list(run)
+          n_out = sum(r for _, r in run)
+          buf, off = DeviceBuffer(quant.packed_bytes(typ, n_out, n_in) if typ else 2 * n_out * n_in), 0
+          for name, r in run:
+            if typ:
+              quant.repack(sd[name], r, n_in, typ, out=buf, out_offset=off)
+              off += quant.packed_bytes(typ, r, n_in)
+            else:
+              part = dense16(name, r, n_in)
+              check(_lib.load().b200q_memcpy_d2d(buf.ptr + off, part.ptr, part.nbytes, None)); off += part.nbytes
+              runtime_sync()
+          out.append(_BlockLinear(typ, n_out, n_in, buf, at))
+          at += n_out
+        return out
     for i in range(c.num_blocks if self.dense_blocks else 0):
       b = _Block()
-      parts = [dense16(f"blk.{i}.attn_{n}.weight", rows, c.dim) for n, rows in (("q", self.q_dim), ("k", self.kv_dim), ("v", self.kv_dim))]
-      b.qkv = DeviceBuffer(2 * qkv_rows * c.dim)
-      off = 0
-      for part in parts:
-        check(_lib.load().b200q_memcpy_d2d(b.qkv.ptr + off, part.ptr, part.nbytes, None)); off += part.nbytes
-      runtime_sync()
+      blk = lambda *names: [f"blk.{i}.{n}.weight" for n in names]
+      b.qkv = stacked(blk("attn_q", "attn_k", "attn_v"), (self.q_dim, self.kv_dim, self.kv_dim), c.dim)
       b.qkv_bias = DeviceBuffer.from_numpy(np.concatenate([np.asarray(sd[f"blk.{i}.attn_{n}.bias"], dtype=np.float16) for n in "qkv"])) if c.qkv_bias else None
-      b.o_w = dense16(f"blk.{i}.attn_output.weight", c.dim, self.q_dim)
-      b.gate_w, b.up_w = dense16(f"blk.{i}.ffn_gate.weight", c.hidden_dim, c.dim), dense16(f"blk.{i}.ffn_up.weight", c.hidden_dim, c.dim)
-      b.down_w = dense16(f"blk.{i}.ffn_down.weight", c.dim, c.hidden_dim)
+      b.o_w, = stacked(blk("attn_output"), (c.dim,), self.q_dim)
+      gate, up = blk("ffn_gate", "ffn_up")
+      if wide(gate, c.dim) and wide(gate, c.dim) == wide(up, c.dim):          # interleaved: the SwiGLU product comes out of one launch
+        pw = quant.repack(sd[gate], c.hidden_dim, c.dim, wide(gate, c.dim), raw_up=sd[up])
+        b.gate_up = [_BlockLinear(pw.qtype, c.hidden_dim, c.dim, pw.buf, 0, swiglu=True)]
+      else: b.gate_up = [stacked([n], (c.hidden_dim,), c.dim)[0] for n in (gate, up)]
+      b.down_w, = stacked(blk("ffn_down"), (c.dim,), c.hidden_dim)
       b.moe = b.router = None
       b.attn_norm = DeviceBuffer.from_numpy(np.asarray(sd[f"blk.{i}.attn_norm.weight"], dtype=np.float16))
       b.ffn_norm = DeviceBuffer.from_numpy(np.asarray(sd[f"blk.{i}.ffn_norm.weight"], dtype=np.float16))
@@ -134,7 +174,7 @@ class Transformer:
       b.k_cache = DeviceBuffer.empty((batch, c.n_kv_heads, c.max_context, c.head_dim), kvdt, zero=True)
       b.v_cache = DeviceBuffer.empty((batch, c.n_kv_heads, c.max_context, c.head_dim), kvdt, zero=True)
       self.blk.append(b)
-      self.weight_bytes += 2 * (qkv_rows * c.dim + c.dim * self.q_dim + 3 * c.hidden_dim * c.dim)
+      self.weight_bytes += sum(w.algorithmic_bytes for w in b.qkv + [b.o_w] + b.gate_up + [b.down_w])
     for i in range(0 if self.dense_blocks else c.num_blocks):
       b = _Block()
       b.qkv = DeviceBuffer(quant.packed_bytes(ggml_type, qkv_rows, c.dim))
@@ -238,7 +278,7 @@ class Transformer:
     if self.is_moe:
       assert tp is None and c.head_dim in (16, 32, 64, 128), "the mixture-of-experts model runs on the row path of one GPU"
       self.prefill_rows = 1
-    self.launches_per_step = (7 if self.dense_blocks else 5) * c.num_blocks + 3
+    self.launches_per_step = 3 + (sum(3 + len(b.qkv) + len(b.gate_up) + (not b.gate_up[0].swiglu) for b in self.blk) if self.dense_blocks else 5 * c.num_blocks)
     # ---- the whole-step kernel: a device table of the blocks' pointers, its workspace, and the two argument blocks (with / without head)
     self._step_args = None
     if engine not in (None, "step", "chain"): raise ValueError(f"unknown engine {engine!r}")
@@ -296,16 +336,15 @@ class Transformer:
       check(lib.b200q_embed(self.token_embd.ptr, self.tokens.ptr, self.pos.ptr, self.x.ptr, c.dim, vocab_full, c.max_context,
                             self.xq_a.ptr if ho else None, self.blk[0].attn_norm.ptr if ho else None, self.ss_a.ptr if ho else None, fl, s))
     for i, b in enumerate(self.blk if self.dense_blocks else ()):
-      # dense-weight blocks: the same step on fp16 matrices, one launch per Linear (norm / bias / residual fused as in the quantised GEMV)
-      quant.gemv_dense(b.qkv, F16, qkv_rows, c.dim, self.x, self.qkv, norm_weight=b.attn_norm, norm_eps=c.norm_eps, bias=b.qkv_bias, flags=fl, stream=s)
+      # K-quant and fp16 blocks: the same step with the row between the launches in fp32 (norm / bias / residual / SwiGLU fused)
+      for w in b.qkv: w.run(self.x, self.qkv, norm_weight=b.attn_norm, norm_eps=c.norm_eps, bias=b.qkv_bias, flags=fl, stream=s)
       a = _lib.AttnArgs(self.qkv.ptr, b.k_cache.ptr, b.v_cache.ptr, kvdt, self.rope.ptr, self.pos.ptr, self.attn.ptr, self.attn_scratch.ptr,
                         c.n_heads, c.n_kv_heads, c.head_dim, c.rope_dim, c.max_context, self.n_split, fl, None)
       check(lib.b200q_attn_decode(ctypes.byref(a), s))
-      quant.gemv_dense(b.o_w, F16, c.dim, self.q_dim, self.attn, self.x, residual=self.x, flags=fl, stream=s)
-      quant.gemv_dense(b.gate_w, F16, c.hidden_dim, c.dim, self.x, self.act, norm_weight=b.ffn_norm, norm_eps=c.norm_eps, flags=fl, stream=s)
-      quant.gemv_dense(b.up_w, F16, c.hidden_dim, c.dim, self.x, self.up_buf, norm_weight=b.ffn_norm, norm_eps=c.norm_eps, flags=fl, stream=s)
-      check(lib.b200q_silu_mul(self.act.ptr, self.up_buf.ptr, self.act.ptr, c.hidden_dim, fl, s))
-      quant.gemv_dense(b.down_w, F16, c.dim, c.hidden_dim, self.act, self.x, residual=self.x, flags=fl, stream=s)
+      b.o_w.run(self.attn, self.x, residual=self.x, flags=fl, stream=s)
+      for w, y in zip(b.gate_up, (self.act, self.up_buf)): w.run(self.x, y, norm_weight=b.ffn_norm, norm_eps=c.norm_eps, flags=fl, stream=s)
+      if not b.gate_up[0].swiglu: check(lib.b200q_silu_mul(self.act.ptr, self.up_buf.ptr, self.act.ptr, c.hidden_dim, fl, s))
+      b.down_w.run(self.act, self.x, residual=self.x, flags=fl, stream=s)
     for i, b in enumerate(() if self.dense_blocks else self.blk):
       nxt_norm = self.blk[i + 1].attn_norm if i + 1 < len(self.blk) else self.output_norm
       st = (lambda n: dict(xq_out_stage=self.ho_stage[n])) if self.ho_stage is not None else (lambda n: {})

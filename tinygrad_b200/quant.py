@@ -9,11 +9,13 @@ as exceptions.  All compute happens in libb200q.so.
 import ctypes, math, threading
 import numpy as np
 from . import _lib
-from ._lib import check, Q4_0, Q8_0, Q6_K, F32, F16, EPI_LINEAR, EPI_SILU_MUL, FLAG_PDL
+from ._lib import check, Q4_0, Q8_0, Q6_K, Q4_K_WIDE, Q6_K_WIDE, F32, F16, EPI_LINEAR, EPI_SILU_MUL, FLAG_PDL
 from .runtime import DeviceBuffer, ptr_of, stream_ptr
 
 # (elements, bytes) per block of the formats the dequantiser covers (tinygrad/llm/gguf.py:20-21); Q4_0 and Q8_0 also have fused kernels
 GGML_QUANT = {Q4_0: (32, 18), 3: (32, 20), 6: (32, 22), 7: (32, 24), Q8_0: (32, 34), 12: (256, 144), 13: (256, 176), Q6_K: (256, 210)}
+WIDE_QUANT = {12: Q4_K_WIDE, Q6_K: Q6_K_WIDE}        # K-quants with a fused GEMV at full activation precision
+_BLOCKS = GGML_QUANT | {wide: GGML_QUANT[t] for t, wide in WIDE_QUANT.items()}
 _DT = {np.dtype(np.float32): F32, np.dtype(np.float16): F16}
 
 
@@ -40,7 +42,7 @@ class PackedWeight:
 
   @property
   def algorithmic_bytes(self) -> int:
-    nel, nby = GGML_QUANT[self.qtype]
+    nel, nby = _BLOCKS[self.qtype]
     return self.rows * self.n_in // nel * nby
 
   def dequantize(self, dtype=np.float32) -> DeviceBuffer:
@@ -61,7 +63,7 @@ def repack(raw, n_out: int, n_in: int, qtype: int, raw_up=None, out: DeviceBuffe
   """Re-tile raw GGUF blocks of a [n_out, n_in] weight.  With `raw_up` the two
   matrices (gate, up) are interleaved for the fused SwiGLU epilogue.  `out` /
   `out_offset` place the tiles inside a larger buffer (e.g. q|k|v back to back)."""
-  if n_in % GGML_QUANT[qtype][0]: raise ValueError(f"n_in={n_in} is not a multiple of the block size")
+  if n_in % _BLOCKS[qtype][0]: raise ValueError(f"n_in={n_in} is not a multiple of the block size")
   raw, raw_up = _as_device(raw), _as_device(raw_up)
   rows = 2 * (-(-n_out // 8) * 8) if raw_up is not None else n_out
   nbytes = packed_bytes(qtype, rows, n_in)
