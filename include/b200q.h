@@ -518,6 +518,35 @@ int b200q_moe_route_tables(const int32_t* topi, int n_tokens, int n_experts, int
 int b200q_permute_rows(const void* src, const int32_t* idx, int64_t n_rows, int row_bytes, void* dst, int gather, void* stream);
 /* `combine` (extra/gemm/moe_routing.py:128-131): out[t] = sum_j weights[t,j] * y[dest_row[t*k+j]], fp32 sum, bf16 in/out. */
 int b200q_moe_combine(const void* y_bf16, const int32_t* dest_row, const float* weights, int n_tokens, int k, int d, void* out_bf16, void* stream);
+/* The expert layer in one call: b200q_moe_route_pad (gating 0) or _gating, pad 256 -> b200q_quantize_mxfp8 into the groups -> b200q_grouped_mxfp8_gemm_swiglu
+ * -> b200q_grouped_mxfp8_gemm -> b200q_moe_combine, the same values as those calls.  f a multiple of 128, d of 256.  x [n_tokens, d] bf16, logits
+ * [n_tokens, n_experts] fp32; out [n_tokens, d] bf16; add_to: NULL, or fp32 [n_tokens, d] to which out is added.  Tables as in b200q_moe_route_pad
+ * (ends [n_experts]: the row behind each expert's last), a_q / a_e8 / act_q / act_e8 / y for b200q_moe_rows_max rows, a_q and a_e8 zeroed once. */
+typedef struct b200q_moe_args {
+  int n_experts, k, d, f;
+  int mode, gating, normalize;
+  float scale;
+  const float* sel_bias;
+  const void *gu_q, *gu_e8, *dn_q, *dn_e8;
+  int32_t* topi;
+  float* weights;
+  int32_t *dest_row, *off, *ends;
+  void *scratch, *a_q, *a_e8, *act_q, *act_e8, *y, *out;
+} b200q_moe_args;
+int b200q_moe_layer(const b200q_moe_args* m, const void* x_bf16, const float* logits, int n_tokens, float* add_to, void* stream);
+/* b200q_prompt_rows for a mixture-of-experts model, one sequence: rows start_pos .. (or one row at *pos_dev) through every block.  The layers' gate_up /
+ * ffn_down and the argument block's act / hidden_dim are not used; `blocks` is a host array of the FFNs, with scratch xn (fp32 [n_rows, dim]), xb (bf16),
+ * logits ([n_rows, n_experts]) and, if shared_dim > 0, sh_act ([n_rows, shared_dim]), sh ([n_rows, dim]), shg ([n_rows]; sh_inp NULL: no gate).  The
+ * expert layers' tables must be sized for n_rows tokens. */
+typedef struct b200q_moe_block {
+  const b200q_moe_args* moe;
+  const void *router, *sh_gate_up, *sh_down, *sh_inp;
+  int router_dtype, sh_inp_dtype, shared_dim;
+  float* xn;
+  void* xb;
+  float *logits, *sh_act, *sh, *shg;
+} b200q_moe_block;
+int b200q_moe_rows(const b200q_rows_args* args, const b200q_moe_block* blocks, int seq, int start_pos, const int32_t* pos_dev, int n_rows, void* stream);
 /* `grouped_mx_gemm` (extra/gemm/moe_gemm.py:112-134; kernel contract extra/thunder/amd/grouped_mxfp8_gemm.cpp:32-158):
  * C[m_total, n] bf16 = A_q[m_total, k] x B_q[e][n, k]^T with both operands' E8M0 scales, fp32 accumulation; rows
  * off[e]..off[e+1] use expert e; rows past off[n_experts] are left untouched.  m_total % 256 == n % 256 == k % 128 == 0

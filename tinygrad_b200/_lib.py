@@ -56,6 +56,18 @@ class RowsArgs(Structure):
               ("att", c_void_p), ("act", c_void_p), ("workspace", c_void_p), ("workspace_bytes", c_size_t)]
 
 
+class MoeArgs(Structure):
+  _fields_ = [("n_experts", c_int), ("k", c_int), ("d", c_int), ("f", c_int), ("mode", c_int), ("gating", c_int), ("normalize", c_int), ("scale", c_float)] + \
+             [(n, c_void_p) for n in ("sel_bias", "gu_q", "gu_e8", "dn_q", "dn_e8", "topi", "weights", "dest_row", "off", "ends", "scratch", "a_q", "a_e8", "act_q",
+                                      "act_e8", "y", "out")]
+
+
+class MoeBlock(Structure):
+  _fields_ = [("moe", POINTER(MoeArgs)), ("router", c_void_p), ("sh_gate_up", c_void_p), ("sh_down", c_void_p), ("sh_inp", c_void_p), ("router_dtype", c_int),
+              ("sh_inp_dtype", c_int), ("shared_dim", c_int), ("xn", c_void_p), ("xb", c_void_p), ("logits", c_void_p), ("sh_act", c_void_p), ("sh", c_void_p),
+              ("shg", c_void_p)]
+
+
 class LinearDesc(Structure):
   _fields_ = [("dense", c_int), ("w_type", c_int), ("n_out", c_int), ("n_in", c_int), ("gemm_min_rows", c_int), ("w", c_void_p), ("bias", c_void_p),
               ("workspace", c_void_p), ("workspace_bytes", c_size_t)]
@@ -176,6 +188,8 @@ SIGNATURES = {
   "b200q_permute_rows": (c_int, [c_void_p, c_void_p, c_int64, c_int, c_void_p, c_int, c_void_p]),
   "b200q_moe_combine": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]),
   "b200q_mx_status_read_clear": (c_int, [POINTER(c_int)]),
+  "b200q_moe_layer": (c_int, [POINTER(MoeArgs), c_void_p, c_void_p, c_int, c_void_p, c_void_p]),
+  "b200q_moe_rows": (c_int, [POINTER(RowsArgs), POINTER(MoeBlock), c_int, c_int, c_void_p, c_int, c_void_p]),
   "b200q_grouped_mxfp8_gemm": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
   "b200q_grouped_mxfp8_gemm_f32": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
   "b200q_fp8_absmax": (c_int, [c_void_p, c_int, c_int64, c_void_p, c_void_p]),

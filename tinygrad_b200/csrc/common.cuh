@@ -39,6 +39,14 @@ bool b200q_pool_release(int dev);
 // fp8 product with factors, bias and output type in the epilogue (mxfp8_gemm.cu)
 int b200q_mx_gemm_scaled(const void* a_q, const void* a_e8, const void* b_q, const void* b_e8, const int32_t* off, int m_total, int n, int k, void* y, int y_dtype,
                          int rows, const float* fw, const float* fx, const float* bias, cudaStream_t st);
+int b200q_mx_gemm_chain(const void* a_q, const void* a_e8, const void* b_q, const void* b_e8, const int32_t* off, const int32_t* ends, int n_experts, int m_total, int n,
+                        int k, void* c_bf16, void* act_q, void* act_e8, cudaStream_t st);
+int b200q_moe_layer_chain(const b200q_moe_args* m, const void* x_bf16, const float* logits, int n_tokens, float* add_to, cudaStream_t st, bool pdl);
+// out (fp32) and out_bf16 (either may be NULL): RMSNorm(x) * weight (prefill.cu)
+int b200q_rmsnorm_rows_chain(const float* x, const void* weight_f16, float eps, int n_rows, int dim, float* out, void* out_bf16, cudaStream_t st);
+int b200q_add_rows_gated_chain(float* x, const float* y, const float* gate_logit, int n_rows, int dim, cudaStream_t st);
+int b200q_attn_rows_pos_chain(const float* qkv, void* k_cache, void* v_cache, int kv_dtype, const float* rope, const int32_t* pos_dev, int n_heads, int n_kv_heads, int head_dim,
+                              int rope_dim, int max_context, void* q_scratch, void* out, int out_dtype, cudaStream_t st);
 int b200q_decode_status_take(int* status);
 int b200q_decode_step_status_take(int* status);   // the same for the whole-step kernel (decode_step.cu)
 int b200q_peer_status_take(int* status);          // the same for the peer-memory collectives (peer.cu)

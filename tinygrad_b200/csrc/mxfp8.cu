@@ -42,6 +42,8 @@ __device__ __forceinline__ float amax8_quad(const float (&v)[8]) {      // |max|
 template <typename T>
 __global__ void quantize_mxfp8_kernel(const T* __restrict__ x, int64_t rows, int k, const int32_t* __restrict__ dest, int fan,
                                       uint8_t* __restrict__ q, uint8_t* __restrict__ e8) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int kb = k >> 5, chunks = (kb + 7) >> 3;
@@ -65,6 +67,8 @@ __global__ void quantize_mxfp8_kernel(const T* __restrict__ x, int64_t rows, int
 // rounded to bf16 as a tensor would be stored, then quantised like any activation.  Same work split as the quantiser.
 __global__ void swiglu_quant_kernel(const __nv_bfloat16* __restrict__ h, int64_t rows, const int32_t* __restrict__ rows_used, int f,
                                     uint8_t* __restrict__ q, uint8_t* __restrict__ e8) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int kb = f >> 5, chunks = (kb + 7) >> 3;
@@ -95,11 +99,10 @@ __global__ void swiglu_quant_kernel(const __nv_bfloat16* __restrict__ h, int64_t
 // Ties: the lower expert index ranks higher (model.py:35-41).
 constexpr int MAX_E_PER_LANE = 8;   // up to 256 experts
 
-__global__ void route_topk_kernel(const float* __restrict__ logits, int n_tokens, int n_experts, int k, int mode, int32_t* __restrict__ topi,
-                                  float* __restrict__ weights) {
+// One token by one warp; s_topi (optional): shared memory that gets the choices too.
+__device__ __forceinline__ void route_topk_token(const float* __restrict__ logits, int tok, int n_experts, int k, int mode, int32_t* __restrict__ topi,
+                                                 float* __restrict__ weights, int* s_topi) {
   const int lane = threadIdx.x & 31;
-  const int tok = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (tok >= n_tokens) return;
   float v[MAX_E_PER_LANE];
   float mx = -INFINITY;
 #pragma unroll
@@ -132,7 +135,7 @@ __global__ void route_topk_kernel(const float* __restrict__ logits, int n_tokens
     float w;
     if (mode == 1) w = expf(bv - mx) / denom;
     else { w = expf(bv - top1); ksum += w; }
-    if (lane == 0) { topi[(size_t)tok * k + slot] = bi; weights[(size_t)tok * k + slot] = w; }
+    if (lane == 0) { topi[(size_t)tok * k + slot] = bi; weights[(size_t)tok * k + slot] = w; if (s_topi) s_topi[tok * k + slot] = bi; }
   }
   if (mode == 0) {
     __syncwarp();
@@ -149,11 +152,9 @@ __global__ void route_topk_kernel(const float* __restrict__ logits, int n_tokens
 // The reference's own shortcut is applied by the caller: SOFTMAX with normalize and no bias is run as SOFTMAX_WEIGHT (model.py:116-117).
 enum { GATE_SOFTMAX = 1, GATE_SIGMOID = 2, GATE_SOFTMAX_WEIGHT = 3, GATE_SQRT_SOFTPLUS = 4 };     // ExpertGating, model.py:9-13
 
-__global__ void route_gating_kernel(const float* __restrict__ logits, const float* __restrict__ sel_bias, int n_tokens, int n_experts, int k, int gating,
-                                    int normalize, float scale, int32_t* __restrict__ topi, float* __restrict__ weights) {
+__device__ __forceinline__ void route_gating_token(const float* __restrict__ logits, const float* __restrict__ sel_bias, int tok, int n_experts, int k, int gating,
+                                                   int normalize, float scale, int32_t* __restrict__ topi, float* __restrict__ weights, int* s_topi) {
   const int lane = threadIdx.x & 31;
-  const int tok = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (tok >= n_tokens) return;
   float sc[MAX_E_PER_LANE], key[MAX_E_PER_LANE];
   float mx = -INFINITY;
 #pragma unroll
@@ -196,7 +197,7 @@ __global__ void route_gating_kernel(const float* __restrict__ logits, const floa
     for (int i = 0; i < MAX_E_PER_LANE; i++) if (i * 32 + lane == bi) key[i] = -INFINITY;    // taken
     const int slot = k - 1 - j;          // ascending order of rank
     if (lane == slot) pv = bs;
-    if (lane == 0) topi[(size_t)tok * k + slot] = bi;
+    if (lane == 0) { topi[(size_t)tok * k + slot] = bi; if (s_topi) s_topi[tok * k + slot] = bi; }
   }
   const bool mine = lane < k;
   if (gating == GATE_SOFTMAX_WEIGHT) {
@@ -208,12 +209,83 @@ __global__ void route_gating_kernel(const float* __restrict__ logits, const floa
   if (mine) weights[(size_t)tok * k + lane] = pv * scale;
 }
 
+// How a call chooses: gating 0 = `mode` of route_topk_token, else an ExpertGating.
+struct RouteRule { int mode, gating, normalize; float scale; const float* sel_bias; };
+
+__device__ __forceinline__ void route_token(const RouteRule& r, const float* logits, int tok, int n_experts, int k, int32_t* topi, float* weights, int* s_topi) {
+  if (r.gating) route_gating_token(logits, r.sel_bias, tok, n_experts, k, r.gating, r.normalize, r.scale, topi, weights, s_topi);
+  else route_topk_token(logits, tok, n_experts, k, r.mode, topi, weights, s_topi);
+}
+__global__ void route_choose_kernel(const RouteRule r, const float* __restrict__ logits, int n_tokens, int n_experts, int k, int32_t* __restrict__ topi,
+                                    float* __restrict__ weights) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int tok = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (tok < n_tokens) route_token(r, logits, tok, n_experts, k, topi, weights, nullptr);
+}
+
 // routing, steps 2-4: stable counting sort of the T*k (token, slot) pairs by expert.
 // dest_row[i] = off[e_i] + (number of pairs before i with the same expert); off = cumulative group sizes padded to 256.
 constexpr int ROUTE_CHUNK = 1024;
+// ends (optional) [n_experts]: off + size, the row behind each expert's last.
+
+// Padded offsets from the group sizes `tot` (shared memory), by one warp.
+__device__ __forceinline__ void route_offsets(const int* tot, int n_experts, int pad, int32_t* __restrict__ off, int32_t* __restrict__ counts, int32_t* __restrict__ ends,
+                                              int* s_off) {
+  const int lane = threadIdx.x & 31;
+  int carry = 0;
+  for (int e0 = 0; e0 < n_experts; e0 += 32) {
+    const int e = e0 + lane, n = e < n_experts ? tot[e] : 0, padded = (n + pad - 1) / pad * pad;
+    int incl = padded;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += v; }
+    const int at = carry + incl - padded;
+    if (e < n_experts) {
+      off[e + 1] = at + padded;
+      if (counts) counts[e] = n;
+      if (ends) ends[e] = at + n;
+      if (s_off) s_off[e] = at;
+    }
+    carry += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  if (lane == 0) off[0] = 0;
+}
+
+// The whole routing of at most ROUTE_CHUNK pairs and ROUTE_ONE_TOKENS tokens in one CTA: a warp per token, then the counting sort in shared memory.
+// As four launches it took 18.5 us whatever the size, nearly all of it launches.  logits == nullptr: the choices are there already (topi).
+constexpr int ROUTE_ONE_TOKENS = 256;
+__global__ void __launch_bounds__(ROUTE_CHUNK) route_one_kernel(const RouteRule r, const float* __restrict__ logits, int n_tokens, int n_experts, int k, int pad,
+                                                                int32_t* __restrict__ topi, float* __restrict__ weights, int32_t* __restrict__ dest_row,
+                                                                int32_t* __restrict__ off, int32_t* __restrict__ counts, int32_t* __restrict__ ends) {
+  extern __shared__ int s_route[];                // [ROUTE_CHUNK choices][n_experts sizes][n_experts offsets][warps][n_experts]
+  int *s_topi = s_route, *s_tot = s_topi + ROUTE_CHUNK, *s_off = s_tot + n_experts, *s_wcnt = s_off + n_experts;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = n_tokens * k, n_warps = (n + 31) >> 5;
+  for (int i = threadIdx.x; i < n_warps * n_experts; i += ROUTE_CHUNK) s_wcnt[i] = 0;
+  pdl_launch_dependents();
+  pdl_wait();
+  if (logits) for (int tok = warp; tok < n_tokens; tok += ROUTE_CHUNK / 32) route_token(r, logits, tok, n_experts, k, topi, weights, s_topi);
+  else for (int i = threadIdx.x; i < n; i += ROUTE_CHUNK) s_topi[i] = topi[i];
+  __syncthreads();
+  const int i = threadIdx.x, e = i < n ? s_topi[i] : -1;
+  const unsigned same = __match_any_sync(0xffffffffu, e);
+  const int before_in_warp = __popc(same & ((1u << lane) - 1));
+  if (e >= 0 && before_in_warp == 0) s_wcnt[warp * n_experts + e] = __popc(same);
+  __syncthreads();
+  for (int x = threadIdx.x; x < n_experts; x += ROUTE_CHUNK) {
+    int run = 0;
+    for (int w = 0; w < n_warps; w++) { const int v = s_wcnt[w * n_experts + x]; s_wcnt[w * n_experts + x] = run; run += v; }
+    s_tot[x] = run;
+  }
+  __syncthreads();
+  if (warp == 0) route_offsets(s_tot, n_experts, pad, off, counts, ends, s_off);
+  __syncthreads();
+  if (e >= 0) dest_row[i] = s_off[e] + s_wcnt[warp * n_experts + e] + before_in_warp;
+}
 
 __global__ void __launch_bounds__(ROUTE_CHUNK) route_count_kernel(const int32_t* __restrict__ topi, int n, int n_experts, int32_t* __restrict__ counts) {
   extern __shared__ int s_cnt[];
+  pdl_launch_dependents();
+  pdl_wait();
   for (int e = threadIdx.x; e < n_experts; e += blockDim.x) s_cnt[e] = 0;
   __syncthreads();
   const int i = blockIdx.x * ROUTE_CHUNK + threadIdx.x;
@@ -222,22 +294,27 @@ __global__ void __launch_bounds__(ROUTE_CHUNK) route_count_kernel(const int32_t*
   for (int e = threadIdx.x; e < n_experts; e += blockDim.x) counts[(size_t)blockIdx.x * n_experts + e] = s_cnt[e];
 }
 
-// one thread per expert: exclusive scan of its chunk counts (in place), then thread 0 builds the padded offsets
-__global__ void route_scan_kernel(int32_t* __restrict__ counts, int n_chunks, int n_experts, int32_t* __restrict__ off, int pad,
-                                  int32_t* __restrict__ counts_out) {
+// one warp per expert: exclusive scan of its chunk counts (in place, 32 chunks at a time); then one warp builds the padded offsets
+__global__ void __launch_bounds__(ROUTE_CHUNK) route_scan_kernel(int32_t* __restrict__ counts, int n_chunks, int n_experts, int32_t* __restrict__ off, int pad,
+                                                                 int32_t* __restrict__ counts_out, int32_t* __restrict__ ends) {
   extern __shared__ int s_tot[];
-  for (int e = threadIdx.x; e < n_experts; e += blockDim.x) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  pdl_launch_dependents();
+  pdl_wait();
+  for (int e = warp; e < n_experts; e += ROUTE_CHUNK / 32) {
     int run = 0;
-    for (int c = 0; c < n_chunks; c++) { const int v = counts[(size_t)c * n_experts + e]; counts[(size_t)c * n_experts + e] = run; run += v; }
-    s_tot[e] = run;
-    if (counts_out) counts_out[e] = run;
+    for (int c0 = 0; c0 < n_chunks; c0 += 32) {
+      const int c = c0 + lane, v = c < n_chunks ? counts[(size_t)c * n_experts + e] : 0;
+      int incl = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += u; }
+      if (c < n_chunks) counts[(size_t)c * n_experts + e] = run + incl - v;
+      run += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) s_tot[e] = run;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int run = 0;
-    off[0] = 0;
-    for (int e = 0; e < n_experts; e++) { run += (s_tot[e] + pad - 1) / pad * pad; off[e + 1] = run; }
-  }
+  if (warp == 0) route_offsets(s_tot, n_experts, pad, off, counts_out, ends, nullptr);
 }
 
 // rows of `row_bytes` bytes moved by an index table: scatter dst[idx[i]] = src[i] or gather dst[i] = src[idx[i]]; idx < 0 skips
@@ -258,6 +335,8 @@ __global__ void __launch_bounds__(ROUTE_CHUNK) route_place_kernel(const int32_t*
   extern __shared__ int s_wcnt[];                 // [32 warps][n_experts] pairs of each expert seen by each warp
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int j = threadIdx.x; j < 32 * n_experts; j += blockDim.x) s_wcnt[j] = 0;
+  pdl_launch_dependents();
+  pdl_wait();
   __syncthreads();
   const int i = blockIdx.x * ROUTE_CHUNK + threadIdx.x;
   const int e = i < n ? topi[i] : -1;
@@ -272,40 +351,68 @@ __global__ void __launch_bounds__(ROUTE_CHUNK) route_place_kernel(const int32_t*
   }
 }
 
-// combine (extra/gemm/moe_routing.py:128-131): out[t] = sum_j weights[t, j] * y[dest_row[t*k + j]], fp32 sum in slot order, bf16 out
+// combine (extra/gemm/moe_routing.py:128-131): out[t] = sum_j weights[t, j] * y[dest_row[t*k + j]], fp32 sum in slot order, bf16 out; add_to
+// (optional, fp32 [n_tokens, d]): the rounded sum is added to it as well (the residual behind the expert layer)
 __global__ void combine_kernel(const __nv_bfloat16* __restrict__ y, const int32_t* __restrict__ dest_row, const float* __restrict__ weights,
-                               int n_tokens, int k, int d, __nv_bfloat16* __restrict__ out) {
+                               int n_tokens, int k, int d, __nv_bfloat16* __restrict__ out, float* __restrict__ add_to) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int t = blockIdx.x;
   for (int c = threadIdx.x; c < d; c += blockDim.x) {
     float acc = 0.f;
     for (int j = 0; j < k; j++) acc += weights[(size_t)t * k + j] * __bfloat162float(y[(size_t)dest_row[(size_t)t * k + j] * d + c]);
-    out[(size_t)t * d + c] = __float2bfloat16_rn(acc);
+    const __nv_bfloat16 r = __float2bfloat16_rn(acc);
+    out[(size_t)t * d + c] = r;
+    if (add_to) add_to[(size_t)t * d + c] += __bfloat162float(r);
   }
 }
-// d % 8 == 0: a thread sums 8 neighbouring columns over the k rows (16-byte loads), same order of additions
-__global__ void combine8_kernel(const __nv_bfloat16* __restrict__ y, const int32_t* __restrict__ dest_row, const float* __restrict__ weights,
-                                int n_tokens, int k, int d, __nv_bfloat16* __restrict__ out) {
+// d % 8 == 0: a thread sums 8 neighbouring columns over the k rows (16-byte loads), same order of additions.  A CTA stages its token's rows and
+// weights, so that four rows are in flight at once (4096 tokens x 8 rows of 2048: 34.9 us with the row numbers loaded one by one).
+constexpr int COMBINE_MAX_K = 32;
+__global__ void __launch_bounds__(256) combine8_kernel(const __nv_bfloat16* __restrict__ y, const int32_t* __restrict__ dest_row, const float* __restrict__ weights,
+                                                       int n_tokens, int k, int d, __nv_bfloat16* __restrict__ out, float* __restrict__ add_to) {
+  __shared__ int s_row[COMBINE_MAX_K];
+  __shared__ float s_w[COMBINE_MAX_K];
   const int t = blockIdx.x;
+  pdl_launch_dependents();
+  pdl_wait();
+  if (threadIdx.x < k) { s_row[threadIdx.x] = dest_row[(size_t)t * k + threadIdx.x]; s_w[threadIdx.x] = weights[(size_t)t * k + threadIdx.x]; }
+  __syncthreads();
   for (int c = threadIdx.x * 8; c < d; c += blockDim.x * 8) {
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int j = 0; j < k; j++) {
-      const float w = weights[(size_t)t * k + j];
-      float v[8];
-      load8<__nv_bfloat16>(y + (size_t)dest_row[(size_t)t * k + j] * d + c, v);
+    for (int j0 = 0; j0 < k; j0 += 4) {
+      uint4 u[4];
 #pragma unroll
-      for (int i = 0; i < 8; i++) acc[i] += w * v[i];
+      for (int j = 0; j < 4; j++) if (j0 + j < k) u[j] = *reinterpret_cast<const uint4*>(y + (size_t)s_row[j0 + j] * d + c);
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        if (j0 + j < k) {
+          const float w = s_w[j0 + j];
+          float v[8];
+          bf16x8_to_f32(u[j], v);
+#pragma unroll
+          for (int i = 0; i < 8; i++) acc[i] += w * v[i];
+        }
+      }
     }
     uint4 pk;
     __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&pk);
 #pragma unroll
     for (int i = 0; i < 4; i++) hp[i] = __floats2bfloat162_rn(acc[2 * i], acc[2 * i + 1]);
     *reinterpret_cast<uint4*>(out + (size_t)t * d + c) = pk;
+    if (add_to) {
+      float v[8];
+      bf16x8_to_f32(pk, v);
+      float4* x = reinterpret_cast<float4*>(add_to + (size_t)t * d + c);
+      float4 a = x[0], b = x[1];
+      a.x += v[0]; a.y += v[1]; a.z += v[2]; a.w += v[3]; b.x += v[4]; b.y += v[5]; b.z += v[6]; b.w += v[7];
+      x[0] = a; x[1] = b;
+    }
   }
 }
 
-}  // namespace
-
-extern "C" int b200q_quantize_mxfp8(const void* x, int x_dtype, int64_t rows, int k, const int32_t* dest_row, int fan, void* q, void* e8, void* stream) {
+// ---- launches; pdl: programmatic, behind a kernel of this library on the same stream ----
+int quantize_launch(const void* x, int x_dtype, int64_t rows, int k, const int32_t* dest_row, int fan, void* q, void* e8, cudaStream_t st, bool pdl) {
   if (rows < 0 || k <= 0 || (rows && (!x || !q || !e8))) return B200Q_ERR_BAD_ARG;
   if (x_dtype != B200Q_F32 && x_dtype != B200Q_BF16) return B200Q_ERR_BAD_ARG;
   if (k % 32) return B200Q_ERR_BAD_SHAPE;
@@ -313,11 +420,47 @@ extern "C" int b200q_quantize_mxfp8(const void* x, int x_dtype, int64_t rows, in
   if (rows == 0) return B200Q_OK;
   if (((uintptr_t)x | (uintptr_t)q) & 15) return B200Q_ERR_MISALIGNED;
   const int64_t warps = rows * ((k / 32 + 7) / 8);
-  const unsigned blocks = (unsigned)((warps + 7) / 8);
-  if (x_dtype == B200Q_F32) quantize_mxfp8_kernel<float><<<blocks, 256, 0, (cudaStream_t)stream>>>((const float*)x, rows, k, dest_row, fan, (uint8_t*)q, (uint8_t*)e8);
-  else quantize_mxfp8_kernel<__nv_bfloat16><<<blocks, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)x, rows, k, dest_row, fan, (uint8_t*)q, (uint8_t*)e8);
-  B200Q_CHECK_CUDA(cudaGetLastError());
+  const dim3 grid((unsigned)((warps + 7) / 8));
+  if (x_dtype == B200Q_F32)
+    B200Q_CHECK_CUDA(launch_k(quantize_mxfp8_kernel<float>, grid, dim3(256), 0, st, pdl, (const float*)x, rows, k, dest_row, fan, (uint8_t*)q, (uint8_t*)e8));
+  else
+    B200Q_CHECK_CUDA(launch_k(quantize_mxfp8_kernel<__nv_bfloat16>, grid, dim3(256), 0, st, pdl, (const __nv_bfloat16*)x, rows, k, dest_row, fan, (uint8_t*)q, (uint8_t*)e8));
   return B200Q_OK;
+}
+
+int combine_launch(const void* y_bf16, const int32_t* dest_row, const float* weights, int n_tokens, int k, int d, void* out_bf16, float* add_to, cudaStream_t st,
+                   bool pdl) {
+  if (!y_bf16 || !dest_row || !weights || !out_bf16 || n_tokens <= 0 || k <= 0 || d <= 0) return B200Q_ERR_BAD_ARG;
+  const bool wide = d % 8 == 0 && k <= COMBINE_MAX_K && !(((uintptr_t)y_bf16 | (uintptr_t)out_bf16 | (uintptr_t)add_to) & 15);
+  B200Q_CHECK_CUDA(launch_k(wide ? combine8_kernel : combine_kernel, dim3(n_tokens), dim3(256), 0, st, pdl, (const __nv_bfloat16*)y_bf16, dest_row, weights, n_tokens, k, d,
+                            (__nv_bfloat16*)out_bf16, add_to));
+  return B200Q_OK;
+}
+
+// logits == nullptr: the choices are in topi already.
+int route_launch(const RouteRule& r, const float* logits, int n_tokens, int n_experts, int k, int pad, int32_t* topi, float* weights, int32_t* dest_row, int32_t* off,
+                 int32_t* counts, int32_t* ends, void* scratch, cudaStream_t st, bool pdl) {
+  const int n = n_tokens * k, n_chunks = ceil_div(n, ROUTE_CHUNK);
+  if (n <= ROUTE_CHUNK && n_tokens <= ROUTE_ONE_TOKENS) {
+    const size_t smem = (ROUTE_CHUNK + (2 + (size_t)ceil_div(n, 32)) * n_experts) * sizeof(int);      // at most 38 KB
+    B200Q_CHECK_CUDA(launch_k(route_one_kernel, dim3(1), dim3(ROUTE_CHUNK), smem, st, pdl, r, logits, n_tokens, n_experts, k, pad, topi, weights, dest_row, off, counts, ends));
+    return B200Q_OK;
+  }
+  int32_t* cnt = (int32_t*)scratch;
+  if (logits) {
+    B200Q_CHECK_CUDA(launch_k(route_choose_kernel, dim3(ceil_div(n_tokens, 8)), dim3(256), 0, st, pdl, r, logits, n_tokens, n_experts, k, topi, weights));
+    pdl = true;
+  }
+  B200Q_CHECK_CUDA(launch_k(route_count_kernel, dim3(n_chunks), dim3(ROUTE_CHUNK), n_experts * sizeof(int), st, pdl, topi, n, n_experts, cnt));
+  B200Q_CHECK_CUDA(launch_k(route_scan_kernel, dim3(1), dim3(ROUTE_CHUNK), n_experts * sizeof(int), st, true, cnt, n_chunks, n_experts, off, pad, counts, ends));
+  B200Q_CHECK_CUDA(launch_k(route_place_kernel, dim3(n_chunks), dim3(ROUTE_CHUNK), 32 * n_experts * sizeof(int), st, true, topi, n, n_experts, cnt, off, dest_row));
+  return B200Q_OK;
+}
+
+}  // namespace
+
+extern "C" int b200q_quantize_mxfp8(const void* x, int x_dtype, int64_t rows, int k, const int32_t* dest_row, int fan, void* q, void* e8, void* stream) {
+  return quantize_launch(x, x_dtype, rows, k, dest_row, fan, q, e8, (cudaStream_t)stream, false);
 }
 
 extern "C" int b200q_swiglu_quantize_mxfp8(const void* h_bf16, int64_t rows, const int32_t* rows_used, int f, void* q, void* e8, void* stream) {
@@ -363,27 +506,14 @@ extern "C" int b200q_moe_route_pad(const float* logits, int n_tokens, int n_expe
   if (!logits || !topi || !weights || !dest_row || !off || !scratch || pad <= 0) return B200Q_ERR_BAD_ARG;
   if (n_tokens <= 0 || n_experts <= 0 || k <= 0 || k > n_experts || (mode != 0 && mode != 1)) return B200Q_ERR_BAD_ARG;
   if (n_experts > 32 * MAX_E_PER_LANE || k > 32) return B200Q_ERR_BAD_SHAPE;
-  cudaStream_t st = (cudaStream_t)stream;
-  const int n = n_tokens * k, n_chunks = ceil_div(n, ROUTE_CHUNK);
-  route_topk_kernel<<<ceil_div(n_tokens, 8), 256, 0, st>>>(logits, n_tokens, n_experts, k, mode, topi, weights);
-  route_count_kernel<<<n_chunks, ROUTE_CHUNK, n_experts * sizeof(int), st>>>(topi, n, n_experts, (int32_t*)scratch);
-  route_scan_kernel<<<1, 256, n_experts * sizeof(int), st>>>((int32_t*)scratch, n_chunks, n_experts, off, pad, counts);
-  route_place_kernel<<<n_chunks, ROUTE_CHUNK, 32 * n_experts * sizeof(int), st>>>(topi, n, n_experts, (const int32_t*)scratch, off, dest_row);
-  B200Q_CHECK_CUDA(cudaGetLastError());
-  return B200Q_OK;
+  return route_launch(RouteRule{mode, 0, 0, 1.f, nullptr}, logits, n_tokens, n_experts, k, pad, topi, weights, dest_row, off, counts, nullptr, scratch, (cudaStream_t)stream, false);
 }
 
 extern "C" int b200q_moe_route_tables(const int32_t* topi, int n_tokens, int n_experts, int k, int pad, int32_t* dest_row, int32_t* off, int32_t* counts,
                                       void* scratch, void* stream) {
   if (!topi || !dest_row || !off || !scratch || pad <= 0 || n_tokens <= 0 || n_experts <= 0 || k <= 0) return B200Q_ERR_BAD_ARG;
   if (n_experts > 32 * MAX_E_PER_LANE) return B200Q_ERR_BAD_SHAPE;
-  cudaStream_t st = (cudaStream_t)stream;
-  const int n = n_tokens * k, n_chunks = ceil_div(n, ROUTE_CHUNK);
-  route_count_kernel<<<n_chunks, ROUTE_CHUNK, n_experts * sizeof(int), st>>>(topi, n, n_experts, (int32_t*)scratch);
-  route_scan_kernel<<<1, 256, n_experts * sizeof(int), st>>>((int32_t*)scratch, n_chunks, n_experts, off, pad, counts);
-  route_place_kernel<<<n_chunks, ROUTE_CHUNK, 32 * n_experts * sizeof(int), st>>>(topi, n, n_experts, (const int32_t*)scratch, off, dest_row);
-  B200Q_CHECK_CUDA(cudaGetLastError());
-  return B200Q_OK;
+  return route_launch(RouteRule{}, nullptr, n_tokens, n_experts, k, pad, const_cast<int32_t*>(topi), nullptr, dest_row, off, counts, nullptr, scratch, (cudaStream_t)stream, false);
 }
 
 extern "C" int b200q_moe_route_gating(const float* logits, const float* sel_bias, int n_tokens, int n_experts, int k, int gating, int normalize, float scale,
@@ -391,23 +521,32 @@ extern "C" int b200q_moe_route_gating(const float* logits, const float* sel_bias
   if (!logits || !topi || !weights || !dest_row || !off || !scratch || pad <= 0) return B200Q_ERR_BAD_ARG;
   if (n_tokens <= 0 || n_experts <= 0 || k <= 0 || k > n_experts || gating < GATE_SOFTMAX || gating > GATE_SQRT_SOFTPLUS) return B200Q_ERR_BAD_ARG;
   if (n_experts > 32 * MAX_E_PER_LANE || k > 32) return B200Q_ERR_BAD_SHAPE;
-  cudaStream_t st = (cudaStream_t)stream;
-  const int n = n_tokens * k, n_chunks = ceil_div(n, ROUTE_CHUNK);
-  route_gating_kernel<<<ceil_div(n_tokens, 8), 256, 0, st>>>(logits, sel_bias, n_tokens, n_experts, k, gating, normalize, scale, topi, weights);
-  route_count_kernel<<<n_chunks, ROUTE_CHUNK, n_experts * sizeof(int), st>>>(topi, n, n_experts, (int32_t*)scratch);
-  route_scan_kernel<<<1, 256, n_experts * sizeof(int), st>>>((int32_t*)scratch, n_chunks, n_experts, off, pad, counts);
-  route_place_kernel<<<n_chunks, ROUTE_CHUNK, 32 * n_experts * sizeof(int), st>>>(topi, n, n_experts, (const int32_t*)scratch, off, dest_row);
-  B200Q_CHECK_CUDA(cudaGetLastError());
-  return B200Q_OK;
+  return route_launch(RouteRule{0, gating, normalize, scale, sel_bias}, logits, n_tokens, n_experts, k, pad, topi, weights, dest_row, off, counts, nullptr, scratch,
+                      (cudaStream_t)stream, false);
 }
 
 extern "C" int b200q_moe_combine(const void* y_bf16, const int32_t* dest_row, const float* weights, int n_tokens, int k, int d, void* out_bf16,
                                  void* stream) {
-  if (!y_bf16 || !dest_row || !weights || !out_bf16 || n_tokens <= 0 || k <= 0 || d <= 0) return B200Q_ERR_BAD_ARG;
-  if (d % 8 == 0 && !(((uintptr_t)y_bf16 | (uintptr_t)out_bf16) & 15))
-    combine8_kernel<<<n_tokens, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)y_bf16, dest_row, weights, n_tokens, k, d, (__nv_bfloat16*)out_bf16);
-  else
-    combine_kernel<<<n_tokens, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)y_bf16, dest_row, weights, n_tokens, k, d, (__nv_bfloat16*)out_bf16);
-  B200Q_CHECK_CUDA(cudaGetLastError());
-  return B200Q_OK;
+  return combine_launch(y_bf16, dest_row, weights, n_tokens, k, d, out_bf16, nullptr, (cudaStream_t)stream, false);
+}
+
+// The expert layer in one call, its launches programmatic behind one another: route, dispatch + quantise, gate/up GEMM with SwiGLU + requantise, down GEMM,
+// combine.  The GEMMs take the rows each expert has, not those its group is padded to.
+int b200q_moe_layer_chain(const b200q_moe_args* m, const void* x_bf16, const float* logits, int n_tokens, float* add_to, cudaStream_t st, bool pdl) {
+  if (!m || !x_bf16 || !logits || n_tokens <= 0 || !m->topi || !m->weights || !m->dest_row || !m->off || !m->ends || !m->scratch) return B200Q_ERR_BAD_ARG;
+  if (m->n_experts <= 0 || m->k <= 0 || m->k > m->n_experts || (m->gating == 0 && m->mode != 0 && m->mode != 1)) return B200Q_ERR_BAD_ARG;
+  if (m->gating && (m->gating < GATE_SOFTMAX || m->gating > GATE_SQRT_SOFTPLUS)) return B200Q_ERR_BAD_ARG;
+  if (m->n_experts > 32 * MAX_E_PER_LANE || m->k > 32 || m->f % 128) return B200Q_ERR_BAD_SHAPE;
+  const int rows = b200q_moe_rows_max(n_tokens, m->n_experts, m->k);
+  int rc = route_launch(RouteRule{m->mode, m->gating, m->normalize, m->scale, m->sel_bias}, logits, n_tokens, m->n_experts, m->k, BLOCK_ROW, m->topi, m->weights, m->dest_row,
+                        m->off, nullptr, m->ends, m->scratch, st, pdl);
+  if (rc == B200Q_OK) rc = quantize_launch(x_bf16, B200Q_BF16, n_tokens, m->d, m->dest_row, m->k, m->a_q, m->a_e8, st, true);
+  if (rc == B200Q_OK)
+    rc = b200q_mx_gemm_chain(m->a_q, m->a_e8, m->gu_q, m->gu_e8, m->off, m->ends, m->n_experts, rows, 2 * m->f, m->d, nullptr, m->act_q, m->act_e8, st);
+  if (rc == B200Q_OK)
+    rc = b200q_mx_gemm_chain(m->act_q, m->act_e8, m->dn_q, m->dn_e8, m->off, m->ends, m->n_experts, rows, m->d, m->f, m->y, nullptr, nullptr, st);
+  return rc == B200Q_OK ? combine_launch(m->y, m->dest_row, m->weights, n_tokens, m->k, m->d, m->out, add_to, st, true) : rc;
+}
+extern "C" int b200q_moe_layer(const b200q_moe_args* m, const void* x_bf16, const float* logits, int n_tokens, float* add_to, void* stream) {
+  return b200q_moe_layer_chain(m, x_bf16, logits, n_tokens, add_to, (cudaStream_t)stream, false);
 }

@@ -136,12 +136,12 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
                                                                       __nv_bfloat16* __restrict__ c, uint8_t* __restrict__ act_q,
                                                                       uint8_t* __restrict__ act_e8, const __grid_constant__ CUtensorMap tm_a,
                                                                       const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_c,
-                                                                      int c_f32, const ScaledOut so) {
+                                                                      int c_f32, const ScaledOut so, const int32_t* __restrict__ ends) {
   extern __shared__ unsigned char sm_raw[];
   __shared__ __align__(8) uint64_t bar_full[STAGES], bar_empty[STAGES], bar_acc_full, bar_acc_empty, bar_drain;
   __shared__ uint32_t tmem_base;
   __shared__ int s_abort;
-  __shared__ int s_off[MAX_EXPERTS + 1];
+  __shared__ int s_off[MAX_EXPERTS], s_tile[MAX_EXPERTS + 1];       // first row of each group, row tiles before it
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     for (int s = 0; s < STAGES; s++) {
@@ -159,7 +159,26 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   pdl_wait();                                       // everything above runs under the previous kernel's tail
-  for (int i = tid; i <= n_experts; i += THREADS) s_off[i] = off[i];
+  // row tiles of the rows each group has (`ends`: without its padding); everything else of the padded layout is left alone
+  if (warp == 0) {
+    int carry = 0;
+    for (int e0 = 0; e0 < n_experts; e0 += 32) {
+      const int e = e0 + lane;
+      int lo = 0, tiles = 0;
+      if (e < n_experts) {
+        lo = min(max(off[e], 0), m_total);
+        int hi = min(max(ends ? ends[e] : off[e + 1], lo), m_total);
+        if (so.fw) hi = min(hi, max(so.rows, lo));
+        tiles = min((hi - lo + BM - 1) / BM, (m_total - lo) / BM);
+      }
+      int incl = tiles;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += v; }
+      if (e < n_experts) { s_off[e] = lo; s_tile[e] = carry + incl - tiles; }
+      carry += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) s_tile[n_experts] = carry;
+  }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -167,8 +186,12 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
   const uint32_t taddr = tmem_base;
   volatile int* abort_flag = &s_abort;
   const int kb_total = k >> 5, ktiles = k / BK;
-  const int m_used = min(max(s_off[n_experts], 0), m_total);
-  const int tiles_n = n / BN, n_tiles = (m_used / BM) * tiles_n;
+  const int tiles_n = n / BN, n_tiles = s_tile[n_experts] * tiles_n;
+  auto group_of = [&](int mt) {                     // the group whose row tile `mt` is
+    int lo = 0, hi = n_experts - 1;
+    while (lo < hi) { const int mid = (lo + hi) >> 1; if (s_tile[mid + 1] <= mt) lo = mid + 1; else hi = mid; }
+    return lo;
+  };
   const uint32_t ring = (s32(sm_raw) + 1023u) & ~1023u;
 
   if (warp >= EPI_WARPS && warp < EPI_WARPS + LOAD_WARPS) {
@@ -177,16 +200,14 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
     const int r0 = lt >> 3, ch = lt & 7;            // this thread copies chunk ch of rows r0 + 16 j
     const uint32_t t_off = (uint32_t)(r0 * 128 + ((ch ^ (r0 & 7)) << 4));
     const uint32_t sf_off = (uint32_t)((lt & 31) * 16 + (lt >> 5) * 4);      // scale word of row lt (A), rows lt and lt + 128 (B)
-    int b_row0 = 0;       // first row of the tile's B operand inside [n_experts * n, k]
+    int b_row0 = 0, a_row0 = 0;      // first rows of the tile's operands: B inside [n_experts * n, k], A inside [m_total, k]
     auto tile_ptrs = [&](int t, const uint8_t*& ap, const uint8_t*& bp, const uint8_t*& ae, const uint8_t*& be) {
-      const int m0 = (t / tiles_n) * BM, n0 = (t % tiles_n) * BN;
-      int lo = 0, hi = n_experts - 1;
-      while (lo < hi) { const int mid = (lo + hi) >> 1; if (s_off[mid + 1] <= m0) lo = mid + 1; else hi = mid; }
+      const int mt = t / tiles_n, n0 = (t % tiles_n) * BN, lo = group_of(mt), m0 = s_off[lo] + (mt - s_tile[lo]) * BM;
       ap = a_q + (size_t)(m0 + r0) * k + ch * 16;
       bp = b_q + ((size_t)lo * n + n0 + r0) * k + ch * 16;
       ae = a_e8 + (size_t)(m0 + lt) * kb_total;
       be = b_e8 + ((size_t)lo * n + n0 + lt) * kb_total;
-      b_row0 = lo * n + n0;
+      b_row0 = lo * n + n0; a_row0 = m0;
     };
     uint32_t g = 0;
     bool ok = true;
@@ -206,7 +227,7 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
           const uint32_t fb = s32(&bar_full[slot]);
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb), "r"(A_BYTES + B_BYTES) : "memory");
           asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                       ::"r"(sA), "l"(&tm_a), "r"(kt * BK), "r"((t / tiles_n) * BM), "r"(fb) : "memory");
+                       ::"r"(sA), "l"(&tm_a), "r"(kt * BK), "r"(a_row0), "r"(fb) : "memory");
           asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                        ::"r"(sB), "l"(&tm_b), "r"(kt * BK), "r"(b_row0), "r"(fb) : "memory");
         }
@@ -287,7 +308,7 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
     for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, tile_i++) {
       if (!wait_bar(s32(&bar_acc_full), tile_i & 1, abort_flag)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int m0 = (t / tiles_n) * BM, n0 = (t % tiles_n) * BN;
+      const int mt = t / tiles_n, n0 = (t % tiles_n) * BN, grp = group_of(mt), m0 = s_off[grp] + (mt - s_tile[grp]) * BM;
       const uint32_t ta = taddr + ((uint32_t)(sub * 32) << 16);
       const size_t row = (size_t)(m0 + sub * 32 + lane);
       uint32_t v0[32], v1[32];
@@ -437,7 +458,7 @@ static int make_map(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t k
 }
 
 static int grouped_launch(const void* a_q, const void* a_e8, const void* b_q, const void* b_e8, const int32_t* off, int n_experts, int m_total, int n, int k,
-                          void* c_bf16, void* act_q, void* act_e8, void* stream, bool c_f32 = false, ScaledOut so = ScaledOut{}, bool pdl = false) {
+                          void* c_bf16, void* act_q, void* act_e8, void* stream, bool c_f32 = false, ScaledOut so = ScaledOut{}, bool pdl = false, const int32_t* ends = nullptr) {
   if (!a_q || !a_e8 || !b_q || !b_e8 || !off || (!c_bf16 && !act_q) || n_experts <= 0 || m_total <= 0 || n <= 0 || k <= 0) return B200Q_ERR_BAD_ARG;
   if (act_q && (!act_e8 || (((uintptr_t)act_q) & 15))) return B200Q_ERR_BAD_ARG;
   if (m_total % 256 || n % BN || k % BK) return B200Q_ERR_BAD_SHAPE;       // the reference asks M % 256 == N % 256 == K % 128 == 0 (moe_gemm.py:120)
@@ -464,13 +485,19 @@ static int grouped_launch(const void* a_q, const void* a_e8, const void* b_q, co
 #endif
   B200Q_CHECK_CUDA(launch_k(grouped_mxfp8_tc_kernel, dim3(grid), dim3(THREADS), (size_t)SMEM_BYTES, (cudaStream_t)stream, pdl, (const uint8_t*)a_q, (const uint8_t*)a_e8,
                             (const uint8_t*)b_q, (const uint8_t*)b_e8, off, n_experts, m_total, n, k, (__nv_bfloat16*)c_bf16, (uint8_t*)act_q, (uint8_t*)act_e8,
-                            tm_a, tm_b, tm_c, c_f32 ? 1 : 0, so));
+                            tm_a, tm_b, tm_c, c_f32 ? 1 : 0, so, ends));
   return B200Q_OK;
 }
 
 int b200q_mx_gemm_scaled(const void* a_q, const void* a_e8, const void* b_q, const void* b_e8, const int32_t* off, int m_total, int n, int k, void* y, int y_dtype,
                          int rows, const float* fw, const float* fx, const float* bias, cudaStream_t st) {
   return grouped_launch(a_q, a_e8, b_q, b_e8, off, 1, m_total, n, k, y, nullptr, nullptr, st, true, ScaledOut{fw, fx, bias, rows, y_dtype == B200Q_F16}, true);
+}
+
+// the expert layer's GEMMs (c_bf16: plain rows, else SwiGLU + requantise into act_q / act_e8), programmatic behind this library's kernels
+int b200q_mx_gemm_chain(const void* a_q, const void* a_e8, const void* b_q, const void* b_e8, const int32_t* off, const int32_t* ends, int n_experts, int m_total, int n,
+                        int k, void* c_bf16, void* act_q, void* act_e8, cudaStream_t st) {
+  return grouped_launch(a_q, a_e8, b_q, b_e8, off, n_experts, m_total, n, k, c_bf16, act_q, act_e8, st, false, ScaledOut{}, true, ends);
 }
 
 extern "C" int b200q_grouped_mxfp8_gemm(const void* a_q, const void* a_e8, const void* b_q, const void* b_e8, const int32_t* off, int n_experts,

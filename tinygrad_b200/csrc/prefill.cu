@@ -40,9 +40,12 @@ __global__ void add_rows_bf16_kernel(float* __restrict__ x, const __nv_bfloat16*
   } else if (i < n) x[i] += __bfloat162float(y[i]);
 }
 
+// out_bf16 (optional): the same rows rounded to bf16
 template <typename O>
-__global__ void rmsnorm_rows_kernel(const float* __restrict__ x, const __half* __restrict__ w, float eps, int dim, O* __restrict__ out) {
+__global__ void rmsnorm_rows_kernel(const float* __restrict__ x, const __half* __restrict__ w, float eps, int dim, O* __restrict__ out, __nv_bfloat16* __restrict__ out_bf16) {
   __shared__ float red[32];
+  pdl_launch_dependents();
+  pdl_wait();
   const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const float* xr = x + (size_t)t * dim;
   float ss = 0.f;
@@ -53,7 +56,11 @@ __global__ void rmsnorm_rows_kernel(const float* __restrict__ x, const __half* _
   float tot = 0.f;
   for (int i = 0; i < nw; i++) tot += red[i];
   const float sc = 1.0f / sqrtf(tot / (float)dim + eps);
-  for (int i = threadIdx.x; i < dim; i += blockDim.x) out[(size_t)t * dim + i] = out_cast<O>(xr[i] * sc * __half2float(w[i]));
+  for (int i = threadIdx.x; i < dim; i += blockDim.x) {
+    const float v = xr[i] * sc * __half2float(w[i]);
+    if (out) out[(size_t)t * dim + i] = out_cast<O>(v);
+    if (out_bf16) out_bf16[(size_t)t * dim + i] = out_cast<__nv_bfloat16>(v);
+  }
 }
 
 template <typename KV> __device__ __forceinline__ KV kv_cast(float v);
@@ -323,16 +330,22 @@ int b200q_embed_rows_seqs(const void* table_f16, const int32_t* tokens, int toke
 extern "C" int b200q_rmsnorm_rows(const float* x, const void* weight_f16, float eps, int n_rows, int dim, void* out, int out_dtype, void* stream) {
   if (!x || !weight_f16 || !out || n_rows <= 0 || dim <= 0) return B200Q_ERR_BAD_ARG;
   if (out_dtype != B200Q_F16 && out_dtype != B200Q_F32 && out_dtype != B200Q_BF16) return B200Q_ERR_BAD_ARG;
-  if (out_dtype == B200Q_BF16) rmsnorm_rows_kernel<__nv_bfloat16><<<n_rows, 256, 0, (cudaStream_t)stream>>>(x, (const __half*)weight_f16, eps, dim,
-                                                                                                           (__nv_bfloat16*)out);
-  else if (out_dtype == B200Q_F16) rmsnorm_rows_kernel<__half><<<n_rows, 256, 0, (cudaStream_t)stream>>>(x, (const __half*)weight_f16, eps, dim, (__half*)out);
-  else rmsnorm_rows_kernel<float><<<n_rows, 256, 0, (cudaStream_t)stream>>>(x, (const __half*)weight_f16, eps, dim, (float*)out);
+  const __half* w = (const __half*)weight_f16;
+  if (out_dtype == B200Q_F16) rmsnorm_rows_kernel<__half><<<n_rows, 256, 0, (cudaStream_t)stream>>>(x, w, eps, dim, (__half*)out, nullptr);
+  else rmsnorm_rows_kernel<float><<<n_rows, 256, 0, (cudaStream_t)stream>>>(x, w, eps, dim, out_dtype == B200Q_F32 ? (float*)out : nullptr,
+                                                                            out_dtype == B200Q_BF16 ? (__nv_bfloat16*)out : nullptr);
   B200Q_CHECK_CUDA(cudaGetLastError());
+  return B200Q_OK;
+}
+int b200q_rmsnorm_rows_chain(const float* x, const void* weight_f16, float eps, int n_rows, int dim, float* out, void* out_bf16, cudaStream_t st) {
+  B200Q_CHECK_CUDA(launch_k(rmsnorm_rows_kernel<float>, dim3(n_rows), dim3(256), 0, st, true, x, (const __half*)weight_f16, eps, dim, out, (__nv_bfloat16*)out_bf16));
   return B200Q_OK;
 }
 
 // x[r][c] += y[r][c] * (gate ? sigmoid(gate[r]) : 1): the shared expert's output joining the residual stream (tinygrad/llm/model.py:131-134)
 __global__ void add_rows_gated_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ gate, int n_rows, int dim) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int r = blockIdx.x;
   const float g = gate ? 1.f / (1.f + expf(-gate[r])) : 1.f;
   for (int c = threadIdx.x; c < dim; c += blockDim.x) x[(size_t)r * dim + c] += y[(size_t)r * dim + c] * g;
@@ -343,6 +356,11 @@ extern "C" int b200q_add_rows_gated(float* x, const float* y, const float* gate_
   if (n_rows == 0) return B200Q_OK;
   add_rows_gated_kernel<<<n_rows, 256, 0, (cudaStream_t)stream>>>(x, y, gate_logit, n_rows, dim);
   B200Q_CHECK_CUDA(cudaGetLastError());
+  return B200Q_OK;
+}
+
+int b200q_add_rows_gated_chain(float* x, const float* y, const float* gate_logit, int n_rows, int dim, cudaStream_t st) {
+  B200Q_CHECK_CUDA(launch_k(add_rows_gated_kernel, dim3(n_rows), dim3(256), 0, st, true, x, y, gate_logit, n_rows, dim));
   return B200Q_OK;
 }
 
@@ -394,6 +412,11 @@ int b200q_attn_rows_chain(const float* qkv, void* k_cache, void* v_cache, int kv
                           int n_kv_heads, int head_dim, int rope_dim, int max_context, void* q_scratch, void* out, int out_dtype, cudaStream_t st, bool pdl) {
   return attn_rows(qkv, k_cache, v_cache, kv_dtype, rope, start_pos, n_rows, n_heads, n_kv_heads, head_dim, rope_dim, max_context, q_scratch, out, out_dtype,
                    n_seqs, nullptr, st, pdl);
+}
+
+int b200q_attn_rows_pos_chain(const float* qkv, void* k_cache, void* v_cache, int kv_dtype, const float* rope, const int32_t* pos_dev, int n_heads, int n_kv_heads, int head_dim,
+                              int rope_dim, int max_context, void* q_scratch, void* out, int out_dtype, cudaStream_t st) {
+  return attn_rows(qkv, k_cache, v_cache, kv_dtype, rope, 0, 1, n_heads, n_kv_heads, head_dim, rope_dim, max_context, q_scratch, out, out_dtype, 1, pos_dev, st, true);
 }
 
 extern "C" int b200q_attn_prefill_seqs(const float* qkv, void* k_cache, void* v_cache, int kv_dtype, const float* rope, int start_pos, int n_rows, int n_seqs,

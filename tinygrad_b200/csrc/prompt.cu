@@ -35,3 +35,47 @@ extern "C" int b200q_prompt_rows(const b200q_rows_args* a, int first_seq, int n_
   }
   return rc;
 }
+
+// The same for a mixture-of-experts model: the FFN of a block is the router, the expert layer and, where the model has one, the shared expert
+// (tinygrad/llm/model.py:110-134).  The GEMMs' sums are not split (see b200q_qgemm_ws_norm), so a token's expert choice does not depend on the rows it
+// came with.  pos_dev: one row of sequence 0 at the position kept on the device (graph replay).  As single calls, each fully ordered behind the one
+// before, a one-token block took 19 launches and 95 us (1024-wide, 32 experts); here 14, programmatic.
+extern "C" int b200q_moe_rows(const b200q_rows_args* a, const b200q_moe_block* blocks, int seq, int start_pos, const int32_t* pos_dev, int n_rows, void* stream) {
+  if (!a || !blocks || !a->layers || !a->token_embd || !a->rope || !a->tokens || !a->x || !a->qkv || !a->q || !a->att || !a->workspace) return B200Q_ERR_BAD_ARG;
+  if (seq < 0 || start_pos < 0 || n_rows <= 0 || a->n_layers < 0 || n_rows > a->rows_max || (pos_dev && (n_rows != 1 || seq != 0))) return B200Q_ERR_BAD_ARG;
+  if (!pos_dev && start_pos + n_rows > a->max_context) return B200Q_ERR_TOO_LARGE;
+  cudaStream_t st = (cudaStream_t)stream;
+  const int T = n_rows, q_dim = a->n_heads * a->head_dim, qkv_rows = q_dim + 2 * a->n_kv_heads * a->head_dim;
+  const size_t seq_bytes = (size_t)a->n_kv_heads * a->max_context * a->head_dim * (a->kv_dtype == B200Q_F16 ? 2 : 4);
+  auto gemm = [&](const void* w, const float* x, const void* bias, const float* residual, int epilogue, float* y, int n_out, int n_in) {
+    return b200q_qgemm_chain(a->qtype, w, x, B200Q_F32, nullptr, 0.f, bias, residual, epilogue, y, B200Q_F32, T, n_out, n_in, a->workspace, a->workspace_bytes, st, true, true);
+  };
+  int rc = pos_dev ? b200q_embed_rows(a->token_embd, a->tokens, 1, pos_dev, 1, a->dim, a->vocab, a->x, stream)
+                   : b200q_embed_rows_seqs(a->token_embd, a->tokens + (size_t)seq * (a->max_context + 1) + start_pos, a->max_context + 1, T, T, a->dim, a->vocab, a->x, st);
+  for (int i = 0; i < a->n_layers && rc == B200Q_OK; i++) {
+    const b200q_decode_layer& l = a->layers[i];
+    const b200q_moe_block& b = blocks[i];
+    if (!b.moe || !b.router || !b.xn || !b.xb || !b.logits) return B200Q_ERR_BAD_ARG;
+    rc = b200q_rmsnorm_rows_chain(a->x, l.attn_norm, a->norm_eps, T, a->dim, b.xn, nullptr, st);
+    if (rc == B200Q_OK) rc = gemm(l.qkv, b.xn, l.qkv_bias, nullptr, B200Q_EPI_LINEAR, a->qkv, qkv_rows, a->dim);
+    if (rc == B200Q_OK)
+      rc = pos_dev ? b200q_attn_rows_pos_chain(a->qkv, l.k_cache, l.v_cache, a->kv_dtype, a->rope, pos_dev, a->n_heads, a->n_kv_heads, a->head_dim, a->rope_dim, a->max_context,
+                                               a->q, a->att, B200Q_F32, st)
+                   : b200q_attn_rows_chain(a->qkv, (char*)l.k_cache + seq * seq_bytes, (char*)l.v_cache + seq * seq_bytes, a->kv_dtype, a->rope, start_pos, T, 1, a->n_heads,
+                                           a->n_kv_heads, a->head_dim, a->rope_dim, a->max_context, a->q, a->att, B200Q_F32, st, true);
+    if (rc == B200Q_OK) rc = gemm(l.attn_output, a->att, nullptr, a->x, B200Q_EPI_LINEAR, a->x, a->dim, q_dim);
+    // router on the fp32 normed rows, experts on their bf16 rounding (the activation type of the MXFP8 path)
+    if (rc == B200Q_OK) rc = b200q_rmsnorm_rows_chain(a->x, l.ffn_norm, a->norm_eps, T, a->dim, b.xn, b.xb, st);
+    if (rc == B200Q_OK)
+      rc = b200q_gemv_dense(b.router, b.router_dtype, b.moe->n_experts, a->dim, T, b.xn, B200Q_F32, nullptr, 0.f, nullptr, nullptr, b.logits, B200Q_F32, B200Q_FLAG_PDL, stream);
+    if (rc == B200Q_OK && b.shared_dim) {
+      rc = gemm(b.sh_gate_up, b.xn, nullptr, nullptr, B200Q_EPI_SILU_MUL, b.sh_act, 2 * b.shared_dim, a->dim);
+      if (rc == B200Q_OK) rc = gemm(b.sh_down, b.sh_act, nullptr, nullptr, B200Q_EPI_LINEAR, b.sh, a->dim, b.shared_dim);
+      if (rc == B200Q_OK && b.sh_inp)
+        rc = b200q_gemv_dense(b.sh_inp, b.sh_inp_dtype, 1, a->dim, T, b.xn, B200Q_F32, nullptr, 0.f, nullptr, nullptr, b.shg, B200Q_F32, B200Q_FLAG_PDL, stream);
+      if (rc == B200Q_OK) rc = b200q_add_rows_gated_chain(a->x, b.sh, b.sh_inp ? b.shg : nullptr, T, a->dim, st);
+    }
+    if (rc == B200Q_OK) rc = b200q_moe_layer_chain(b.moe, b.xb, b.logits, T, a->x, st, true);
+  }
+  return rc;
+}

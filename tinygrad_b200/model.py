@@ -272,7 +272,7 @@ class Transformer:
     self._cached_tokens: list = []
     self.prefill_rows = prefill_rows if (tp is None and not self.dense_blocks and c.hidden_dim % 8 == 0 and c.head_dim in (16, 32, 64, 128)) else 0
     self.prefill_chunk, self._pf, self._batch_logits, self._rows_ws, self._batch_graph = max(1, prefill_chunk), None, None, None, None
-    self._rows_args = None
+    self._rows_args, self._moe_blocks = None, {}
     self._seq_attn_scratch = None
     self.is_moe, self._host_pos, self._rows_warm = c.num_experts > 0, 0, False
     if self.is_moe:
@@ -417,6 +417,9 @@ class Transformer:
       check(lib.b200q_prompt_rows(native, seq, 1, p0, min(self.prefill_chunk, start_pos + n - p0), s))
     for p0 in () if native else range(start_pos, start_pos + n, self.prefill_chunk):
       T = min(self.prefill_chunk, start_pos + n - p0)
+      if (blocks := self._native_moe(T)) is not None:
+        check(lib.b200q_moe_rows(self._rows_args[1], blocks, seq, p0, None, T, s))
+        continue
       check(lib.b200q_embed_rows(self.token_embd.ptr, self.tokens.ptr + 4 * (seq * (c.max_context + 1) + p0), 1, None, T, c.dim,
                                  self.full_config.vocab_size, f["x"].ptr, s))
       for b in self.blk: self._enqueue_rows_block(b, T, f, p0, seq)
@@ -466,10 +469,30 @@ class Transformer:
   def _native_rows(self):
     """The argument block of b200q_prompt_rows (every launch of a chunk from one call), or None where the model does not run on it."""
     if self.is_moe or self.dense_blocks or self.tp is not None or not self.pipelined_gemm or not quant.PIPELINED_GEMM: return None
+    return self._row_arguments()
+
+  def _native_moe(self, T: int):
+    """The expert FFNs' argument blocks of b200q_moe_rows for T rows (self._rows_args is its first argument then), or None where it does not run."""
+    if not self.is_moe or not self.pipelined_gemm or not quant.PIPELINED_GEMM: return None
+    if T not in self._moe_blocks:
+      c, f = self.config, self._prefill_buffers()
+      self._row_arguments()
+      args = [b.moe.native_args(T) for b in self.blk]
+      ptr = lambda o: o.ptr if o is not None else None
+      def block(b, a):
+        sh = b.sh_gate_up is not None
+        return _lib.MoeBlock(ctypes.pointer(a), b.router.buf.ptr, b.sh_gate_up.buf.ptr if sh else None, b.sh_down.buf.ptr if sh else None,
+                             b.sh_inp.buf.ptr if sh and b.sh_inp is not None else None, b.router.dtype, b.sh_inp.dtype if sh and b.sh_inp is not None else 0,
+                             c.shared_expert_dim if sh else 0, f["xn"].ptr, f["xb"].ptr, f["logits"].ptr, f["act"].ptr, ptr(f.get("sh")), ptr(f.get("shg")))
+      self._moe_blocks[T] = None if any(a is None for a in args) else (_lib.MoeBlock * len(args))(*[block(b, a) for b, a in zip(self.blk, args)])
+    return self._moe_blocks[T]
+
+  def _row_arguments(self):
     if self._rows_args is None:
       c, f = self.config, self._prefill_buffers()
-      self._layer_host = (_lib.DecodeLayer * c.num_blocks)(*[_lib.DecodeLayer(b.qkv.ptr, b.qkv_bias.ptr if b.qkv_bias else None, b.attn_output.buf.ptr, b.gate_up.buf.ptr,
-                                                                             b.ffn_down.buf.ptr, b.attn_norm.ptr, b.ffn_norm.ptr, b.k_cache.ptr, b.v_cache.ptr) for b in self.blk])
+      self._layer_host = (_lib.DecodeLayer * c.num_blocks)(*[_lib.DecodeLayer(b.qkv.ptr, b.qkv_bias.ptr if b.qkv_bias else None, b.attn_output.buf.ptr,
+                                                                             *((None, None) if self.is_moe else (b.gate_up.buf.ptr, b.ffn_down.buf.ptr)),
+                                                                             b.attn_norm.ptr, b.ffn_norm.ptr, b.k_cache.ptr, b.v_cache.ptr) for b in self.blk])
       a = _lib.RowsArgs(self._layer_host, c.num_blocks, self.qtype, c.dim, c.hidden_dim, c.n_heads, c.n_kv_heads, c.head_dim, c.rope_dim, c.max_context,
                         self.full_config.vocab_size, F16 if c.kv_dtype == "float16" else F32, self.prefill_chunk, c.norm_eps, self.token_embd.ptr, self.rope.ptr,
                         self.tokens.ptr, f["x"].ptr, f["qkv"].ptr, f["q16"].ptr, f["att"].ptr, f["act"].ptr, f["ws"].ptr, f["ws"].nbytes)
@@ -587,18 +610,23 @@ class Transformer:
 
   def _enqueue_step_rows(self, with_head: bool) -> None:
     c, lib, s, f = self.config, _lib.load(), self.stream.ptr, self._prefill_buffers()
-    check(lib.b200q_embed_rows(self.token_embd.ptr, self.tokens.ptr, 1, self.pos.ptr, 1, c.dim, self.full_config.vocab_size, f["x"].ptr, s))
-    for b in self.blk: self._enqueue_rows_block(b, 1, f, None, 0)
+    fl = 0
+    if (blocks := self._native_moe(1)) is not None:
+      check(lib.b200q_moe_rows(self._rows_args[1], blocks, 0, 0, self.pos.ptr, 1, s))
+      fl = self.flags
+    else:
+      check(lib.b200q_embed_rows(self.token_embd.ptr, self.tokens.ptr, 1, self.pos.ptr, 1, c.dim, self.full_config.vocab_size, f["x"].ptr, s))
+      for b in self.blk: self._enqueue_rows_block(b, 1, f, None, 0)
     if with_head:
       x_last = self._pf["x"]
       if isinstance(self.output, quant.DenseWeight):
         quant.gemv_dense(self.output.buf, self.output.dtype, c.vocab_size, c.dim, x_last, self.logits, norm_weight=self.output_norm, norm_eps=c.norm_eps,
-                         stream=s)
+                         flags=fl, stream=s)
       else:
         quant.gemv(self.output.buf.ptr, self.output_type, c.vocab_size, c.dim, x_last, self.logits, norm_weight=self.output_norm, norm_eps=c.norm_eps,
-                   stream=s)
+                   flags=fl, stream=s)
       check(lib.b200q_argmax_advance_seqs(self.logits.ptr, c.vocab_size, self.tokens.ptr, 0, self.pos.ptr, c.max_context, self.argmax_scratch.ptr, 1,
-                                          self._mirror.ptr, 0, s))
+                                          self._mirror.ptr, fl, s))
     else:
       check(lib.b200q_advance(self.pos.ptr, c.max_context, 0, s))
 

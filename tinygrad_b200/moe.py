@@ -5,6 +5,7 @@
 activation -> grouped_mx_gemm -> combine), with the SwiGLU of tinygrad/llm/model.py:129.  bf16 tensors travel as
 uint16 arrays on the host (numpy has no bfloat16).  All compute is in libb200q.so.
 """
+import ctypes
 from dataclasses import dataclass
 import numpy as np
 from . import _lib
@@ -107,12 +108,31 @@ class MxMoE:
                       out=DeviceBuffer.empty((n_tokens, self.D), np.uint16))
     return self._ws
 
+  def native_args(self, n_tokens: int):
+    """The argument block of b200q_moe_layer for n_tokens tokens, or None where the layer does not run on it."""
+    if not self.fused or self.D % 256: return None
+    w = self._workspace(n_tokens)
+    if "args" not in w:
+      r = w["r"]
+      gating, norm, scale = (*self.mode.resolved(), float(self.mode.routed_scaling_factor)) if isinstance(self.mode, Gating) else (0, 0, 1.0)
+      w["ends"] = DeviceBuffer.empty((self.E,), np.int32)
+      w["args"] = _lib.MoeArgs(self.E, self.k, self.D, self.F, 0 if gating else self.mode, gating, int(norm), scale, r._bias.ptr if r._bias else None, self.gu_q.ptr,
+                               self.gu_e8.ptr, self.dn_q.ptr, self.dn_e8.ptr, r.topi.ptr, r.weights.ptr, r.dest_row.ptr, r.off.ptr, w["ends"].ptr, r._scratch.ptr,
+                               w["a_q"].ptr, w["a_e8"].ptr, w["act_q"].ptr, w["act_e8"].ptr, w["y"].ptr, w["out"].ptr)
+      w["args_ref"] = ctypes.byref(w["args"])
+    return w["args"]
+
   def __call__(self, x_bf16: DeviceBuffer, logits: DeviceBuffer, n_tokens: int, stream=None) -> DeviceBuffer:
     """x (T, D) bf16, router logits (T, E) fp32 -> (T, D) bf16."""
-    lib, s, w = _lib.load(), stream_ptr(stream), self._workspace(n_tokens)
+    lib, s = _lib.load(), stream_ptr(stream)
+    if self.native_args(n_tokens) is not None:
+      check(lib.b200q_moe_layer(self._ws["args_ref"], x_bf16.ptr, logits.ptr, n_tokens, None, s))
+      self.last_routing = self._ws["r"]
+      return self._ws["out"]
+    w = self._workspace(n_tokens)
     r = w["r"].run(logits, stream)
     check(lib.b200q_quantize_mxfp8(x_bf16.ptr, BF16, n_tokens, self.D, r.dest_row.ptr, self.k, w["a_q"].ptr, w["a_e8"].ptr, s))
-    if self.fused:
+    if self.fused:      # D not a multiple of 256: refused by the GEMM, like the layer always did
       check(lib.b200q_grouped_mxfp8_gemm_swiglu(w["a_q"].ptr, w["a_e8"].ptr, self.gu_q.ptr, self.gu_e8.ptr, r.off.ptr, self.E, r.m_l, 2 * self.F, self.D,
                                                 w["act_q"].ptr, w["act_e8"].ptr, s))
     else:
