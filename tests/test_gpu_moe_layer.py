@@ -44,3 +44,28 @@ def test_layer_is_its_parts(sizes):
   np.testing.assert_array_equal(acc.numpy(), res + moe.from_bf16_bits(got))
   for f in layer.phases(x, lg, T).values(): f()
   np.testing.assert_array_equal(got, layer._workspace(T)["out"].numpy())
+
+
+# a row tile of CTA pairs per group / half-empty last tiles / one K step, and more K steps than the ring has stages / several column tiles
+@pytest.mark.parametrize("E,rows,n,k", [(1, 256, 256, 128), (2, 512, 512, 640), (3, 768, 256, 2048)])
+def test_pair_gemm(E, rows, n, k):
+  """Groups of 256 rows and more go to pairs of CTAs: every row against the oracle (fp32 sums of at most k products, then one rounding to bf16)."""
+  need_gpu()
+  from tinygrad_b200 import _lib, moe
+  from tinygrad_b200.runtime import DeviceBuffer
+  rng = np.random.default_rng(n + k)
+  m = E * rows + (256 * E if E > 1 else 0)                        # room for padding, as the routing sizes it
+  off = (np.arange(E + 1) * rows).astype(np.int32)
+  aq, ae = mx.quantize_mxfp8(rng.standard_normal((m, k)).astype(np.float32))
+  bq, be = mx.quantize_mxfp8((rng.standard_normal((E * n, k)) * np.exp(rng.uniform(-3, 3, (E * n, 1)))).astype(np.float32))
+  c = DeviceBuffer.empty((m, n), np.uint16, zero=True)
+  bufs = [DeviceBuffer.from_numpy(v) for v in (aq, ae, bq, be, off)]
+  _lib.check(_lib.load().b200q_grouped_mxfp8_gemm(*(b.ptr for b in bufs), E, m, n, k, c.ptr, None))
+  got = moe.from_bf16_bits(c.numpy())
+  a, b = mx.dequantize_mxfp8(aq, ae).astype(np.float64), mx.dequantize_mxfp8(bq, be).astype(np.float64).reshape(E, n, k)
+  for e in range(E):
+    x = a[off[e]:off[e + 1]]
+    want, mag = x @ b[e].T, np.abs(x) @ np.abs(b[e]).T
+    err = np.abs(got[off[e]:off[e + 1]] - want)
+    assert (err <= 2.0 ** -8 * np.abs(want) + 2.0 ** -23 * (k / 32 + 32) * mag).all(), (e, err.max())
+  assert not got[off[E]:].any()

@@ -24,10 +24,6 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
-#ifndef B200Q_MX_TMA
-#define B200Q_MX_TMA 1      // 1: the A / B tiles of a K step arrive by two tensor-map (TMA) copies; 0: by 16-byte cp.async of 128 threads
-#endif
-
 namespace {
 
 #ifndef B200Q_MX_STAGES
@@ -38,10 +34,7 @@ constexpr int EPI_WARPS = 4, LOAD_WARPS = 4, EPI_Q = 4;      // epilogue: warps 
 constexpr int THREADS = (EPI_Q * EPI_WARPS + LOAD_WARPS + 1) * 32;
 constexpr int A_BYTES = BM * BK, B_BYTES = BN * BK, SF_BYTES = 2048;                    // scale chunks: A 512 B, B 2 x 512 B
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES + SF_BYTES;                               // 50 KB, a multiple of 1024
-#ifndef B200Q_MX_STAGED_EPI
-#define B200Q_MX_STAGED_EPI 2     // bf16 epilogue: 0 = each thread stores its own row (16-byte pieces of 32 different rows per instruction); 1 = through
-#endif                            // 4 KB of shared memory per warp, stores of whole 128-byte row segments; 2 = the same, stored by one tensor-map copy
-constexpr int EPI_STAGE_BYTES = B200Q_MX_STAGED_EPI ? 16 * 4096 : 0;
+constexpr int EPI_STAGE_BYTES = 16 * 4096;                                              // bf16 epilogue: 4 KB per warp, stored by one tensor-map copy
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + EPI_STAGE_BYTES;               // + room to align the ring to 1024 B
 constexpr int TMEM_COLS = 512;            // 256 accumulator columns + scale columns, rounded up to a power of two
 constexpr int SFA_COL = 256, SFB_COL = 256 + 4 * STAGES;   // per stage 4 columns (A: 128 rows) and 8 columns (B: 256 rows)
@@ -51,7 +44,6 @@ constexpr int SPIN = 1 << 22;
 __device__ int g_mx_status = 0;
 
 __device__ __forceinline__ uint32_t s32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void cp16(uint32_t s, const void* g) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(g) : "memory"); }
 __device__ __forceinline__ void cp4(uint32_t s, const void* g) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(s), "l"(g) : "memory"); }
 __device__ __forceinline__ uint64_t desc_plain(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
   uint64_t d = 0;
@@ -92,16 +84,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t ta, uint32_t (&v)[32]) {
                  "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]),
                  "=r"(v[31])
                : "r"(ta));
-}
-__device__ __forceinline__ void bf16_store32(const uint32_t (&v)[32], __nv_bfloat16* dst) {
-#pragma unroll
-  for (int j = 0; j < 32; j += 8) {
-    uint4 pk;
-    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&pk);
-#pragma unroll
-    for (int q = 0; q < 4; q++) h[q] = __floats2bfloat162_rn(__uint_as_float(v[j + 2 * q]), __uint_as_float(v[j + 2 * q + 1]));
-    *reinterpret_cast<uint4*>(dst + j) = pk;
-  }
 }
 // one MX block of the activation: gate / up accumulators of 32 columns -> silu(gate) * up -> E4M3 codes + block exponent at [row, col..col+31]
 __device__ __forceinline__ void swiglu_quant_store(const uint32_t (&vg)[32], const uint32_t (&vu)[32], uint8_t* act_q, uint8_t* act_e8, size_t row, int f,
@@ -145,11 +127,11 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     for (int s = 0; s < STAGES; s++) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(s32(&bar_full[s])), "r"(LOAD_WARPS * 32 + B200Q_MX_TMA));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(s32(&bar_full[s])), "r"(LOAD_WARPS * 32 + 1));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(s32(&bar_empty[s])));
     }
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(s32(&bar_acc_full)));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(s32(&bar_acc_empty)), "r"(EPI_Q * EPI_WARPS * 32));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(s32(&bar_acc_empty)), "r"(EPI_Q * EPI_WARPS));
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(s32(&bar_drain)));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     s_abort = 0;
@@ -197,14 +179,10 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
   if (warp >= EPI_WARPS && warp < EPI_WARPS + LOAD_WARPS) {
     // ---------------------------------------------------------------- loaders
     const int lt = tid - EPI_WARPS * 32;            // 0..127
-    const int r0 = lt >> 3, ch = lt & 7;            // this thread copies chunk ch of rows r0 + 16 j
-    const uint32_t t_off = (uint32_t)(r0 * 128 + ((ch ^ (r0 & 7)) << 4));
     const uint32_t sf_off = (uint32_t)((lt & 31) * 16 + (lt >> 5) * 4);      // scale word of row lt (A), rows lt and lt + 128 (B)
     int b_row0 = 0, a_row0 = 0;      // first rows of the tile's operands: B inside [n_experts * n, k], A inside [m_total, k]
-    auto tile_ptrs = [&](int t, const uint8_t*& ap, const uint8_t*& bp, const uint8_t*& ae, const uint8_t*& be) {
+    auto tile_ptrs = [&](int t, const uint8_t*& ae, const uint8_t*& be) {
       const int mt = t / tiles_n, n0 = (t % tiles_n) * BN, lo = group_of(mt), m0 = s_off[lo] + (mt - s_tile[lo]) * BM;
-      ap = a_q + (size_t)(m0 + r0) * k + ch * 16;
-      bp = b_q + ((size_t)lo * n + n0 + r0) * k + ch * 16;
       ae = a_e8 + (size_t)(m0 + lt) * kb_total;
       be = b_e8 + ((size_t)lo * n + n0 + lt) * kb_total;
       b_row0 = lo * n + n0; a_row0 = m0;
@@ -212,15 +190,12 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
     uint32_t g = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
-      const uint8_t *ap, *bp, *ae, *be;
-      tile_ptrs(t, ap, bp, ae, be);
+      const uint8_t *ae, *be;
+      tile_ptrs(t, ae, be);
       for (int kt = 0; kt < ktiles; kt++, g++) {
         const uint32_t slot = g % STAGES;
         if (g >= STAGES && !wait_bar(s32(&bar_empty[slot]), ((g / STAGES) - 1) & 1, abort_flag)) { ok = false; break; }
         const uint32_t sA = ring + slot * STAGE_BYTES, sB = sA + A_BYTES, sF = sB + B_BYTES;
-        const uint8_t* pa = ap + kt * BK;
-        const uint8_t* pb = bp + kt * BK;
-#if B200Q_MX_TMA
         __syncwarp();
         if (warp == EPI_WARPS && elect_one()) {
           // the 128-byte-swizzle tiled copy writes exactly the layout above (chunk c of row r at c ^ (r & 7)); no multicast
@@ -231,13 +206,6 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
           asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                        ::"r"(sB), "l"(&tm_b), "r"(kt * BK), "r"(b_row0), "r"(fb) : "memory");
         }
-        (void)pa; (void)pb; (void)t_off;
-#else
-#pragma unroll
-        for (int j = 0; j < BM / 16; j++) cp16(sA + t_off + j * 2048, pa + (size_t)(16 * j) * k);
-#pragma unroll
-        for (int j = 0; j < BN / 16; j++) cp16(sB + t_off + j * 2048, pb + (size_t)(16 * j) * k);
-#endif
         cp4(sF + sf_off, ae + kt * 4);
         cp4(sF + 512 + sf_off, be + kt * 4);
         cp4(sF + 1024 + sf_off, be + (size_t)128 * kb_total + kt * 4);
@@ -245,7 +213,6 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
       }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-#if B200Q_MX_TMA
     // nothing of this thread's tensor-map copies may still be landing when the CTA leaves (they are all consumed unless a wait ran out)
     if (lt == 0)
       for (uint32_t j = g > STAGES ? g - STAGES : 0; j < g; j++) {
@@ -256,7 +223,6 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
           if (done) break;
         }
       }
-#endif
   } else if (warp == EPI_WARPS + LOAD_WARPS) {
     // ---------------------------------------------------------------- MMA issue (one thread)
     if (elect_one()) {
@@ -305,6 +271,12 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
     // and stores: the next tile's MMAs wait for one tensor-memory round trip, not for the epilogue.
     const int sub = warp & 3, cq = warp < EPI_WARPS ? 0 : 1 + (warp - (EPI_WARPS + LOAD_WARPS + 1)) / 4;      // column quarter 0..3
     uint32_t tile_i = 0;
+    // the accumulator has been read: one arrival per warp
+    auto release = [&]() {
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) arrive(s32(&bar_acc_empty));
+    };
     for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, tile_i++) {
       if (!wait_bar(s32(&bar_acc_full), tile_i & 1, abort_flag)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -319,15 +291,13 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
         // bf16-round, block exponent from the amax, E4M3 codes -- the arithmetic of swiglu_quant_kernel, with no trip through HBM.
         tmem_ld32(ta + cq * 32, v0); tmem_ld32(ta + BN / 2 + cq * 32, v1);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        arrive(s32(&bar_acc_empty));
+        release();
         swiglu_quant_store(v0, v1, act_q, act_e8, row, n >> 1, (n0 >> 1) + cq * 32);
         continue;
       }
       tmem_ld32(ta + cq * 64, v0); tmem_ld32(ta + cq * 64 + 32, v1);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      arrive(s32(&bar_acc_empty));
+      release();
       if (so.fw) {
         const float w = *so.fw, xf = *so.fx;
         const int col = n0 + cq * 64;
@@ -361,8 +331,6 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
         }
         continue;
       }
-      __nv_bfloat16* out_row = c + row * n + n0 + cq * 64;
-#if B200Q_MX_STAGED_EPI
       {
         // row `lane`, 64 columns = eight 16-byte packets -> this warp's staging rows (packet p of row r at p ^ (r & 7): conflict-free
         // both ways) -> read back four rows x 128 contiguous bytes per instruction and store those
@@ -379,7 +347,6 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
           }
           *reinterpret_cast<uint4*>(stg + lane * 128 + ((p8 ^ (lane & 7)) << 4)) = pk;
         }
-#if B200Q_MX_STAGED_EPI == 2
         // the staging rows are in the 128-byte-swizzle layout a tiled tensor-map store reads: one copy per warp and tile
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
@@ -390,28 +357,9 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
           asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // the rows may be overwritten for the next tile
         }
         __syncwarp();
-#else
-        __syncwarp();
-        __nv_bfloat16* out_tile = c + (size_t)(m0 + sub * 32) * n + n0 + cq * 64;
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const int r = 4 * i + (lane >> 3), p8 = lane & 7;
-          const uint4 pk = *reinterpret_cast<const uint4*>(stg + r * 128 + ((p8 ^ (r & 7)) << 4));
-          *reinterpret_cast<uint4*>(out_tile + (size_t)r * n + p8 * 8) = pk;
-        }
-        __syncwarp();
-#endif
-        (void)out_row;
       }
-#elif !defined(B200Q_MX_EXP_NOSTORE)
-      bf16_store32(v0, out_row); bf16_store32(v1, out_row + 32);
-#else
-      if (v0[0] == 0x12345678u && v1[5] == 0x9abcdef0u) bf16_store32(v0, out_row);
-#endif
     }
-#if B200Q_MX_STAGED_EPI == 2
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");      // this warp's stores have left before the CTA does
-#endif
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -475,14 +423,10 @@ static int grouped_launch(const void* a_q, const void* a_e8, const void* b_q, co
   const int grid = (int)(tiles < n_sm ? tiles : n_sm);
   alignas(64) CUtensorMap tm_a, tm_b, tm_c;
   memset(&tm_a, 0, sizeof(tm_a)); memset(&tm_b, 0, sizeof(tm_b)); memset(&tm_c, 0, sizeof(tm_c));
-#if B200Q_MX_STAGED_EPI == 2
   if (c_bf16 && !c_f32) { const int rcc = make_map(&tm_c, c_bf16, (uint64_t)m_total, (uint64_t)n, 32, true); if (rcc != B200Q_OK) return rcc; }
-#endif
-#if B200Q_MX_TMA
   int rc = make_map(&tm_a, a_q, (uint64_t)m_total, (uint64_t)k, BM);
   if (rc == B200Q_OK) rc = make_map(&tm_b, b_q, (uint64_t)n_experts * n, (uint64_t)k, BN);
   if (rc != B200Q_OK) return rc;
-#endif
   B200Q_CHECK_CUDA(launch_k(grouped_mxfp8_tc_kernel, dim3(grid), dim3(THREADS), (size_t)SMEM_BYTES, (cudaStream_t)stream, pdl, (const uint8_t*)a_q, (const uint8_t*)a_e8,
                             (const uint8_t*)b_q, (const uint8_t*)b_e8, off, n_experts, m_total, n, k, (__nv_bfloat16*)c_bf16, (uint8_t*)act_q, (uint8_t*)act_e8,
                             tm_a, tm_b, tm_c, c_f32 ? 1 : 0, so, ends));
