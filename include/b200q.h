@@ -192,6 +192,10 @@ typedef struct b200q_gemv_args {
    * out one by one, every tile leaves its outputs in this row as self-validating words and counts into its block's counter, and
    * the CTA that counts last collects and quantises the block.  Same record either way. */
   void* xq_out_stage;
+  /* Two matrices that read the same row in one launch (NULL: one): output rows from n_first (a multiple of 16) on are those of w_packed2, whose type
+   * is B200Q_Q6_K_WIDE; qtype must be B200Q_Q4_K_WIDE and the epilogue linear. */
+  const void* w_packed2;
+  int n_first;
 } b200q_gemv_args;
 int b200q_gemv(const b200q_gemv_args* args, void* stream);
 size_t b200q_xq_bytes(int n);

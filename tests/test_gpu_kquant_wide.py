@@ -58,6 +58,21 @@ def test_kquant_wide(typ, n_out, n_in, m):
   assert (err <= bound).all(), (err / bound).max()
 
 
+def test_kquant_two_matrices():
+  """Q4_K rows with Q6_K rows behind them in one launch: the same bits as two launches."""
+  need_gpu()
+  rng = np.random.default_rng(7)
+  n_in, rows = 1280, (48, 21)
+  x, bias = DeviceBuffer.from_numpy(rng.standard_normal(n_in).astype(np.float32)), DeviceBuffer.from_numpy(rng.standard_normal(sum(rows)).astype(np.float16))
+  p4, p6 = (quant.repack(synth.random_blocks(t, r, n_in, rng), r, n_in, TYPES[t]) for t, r in zip((12, 14), rows))
+  y, z = DeviceBuffer.empty((sum(rows),), np.float32), DeviceBuffer.empty((sum(rows),), np.float32)
+  quant.gemv(p4.buf.ptr, _lib.Q4_K_WIDE, sum(rows), n_in, x, y, bias=bias, w2_ptr=p6.buf.ptr, n_first=rows[0])
+  quant.gemv(p4.buf.ptr, _lib.Q4_K_WIDE, rows[0], n_in, x, z, bias=bias)
+  quant.gemv(p6.buf.ptr, _lib.Q6_K_WIDE, rows[1], n_in, x, z.ptr + 4 * rows[0], bias=bias.ptr + 2 * rows[0])
+  np.testing.assert_array_equal(y.numpy(), z.numpy())
+  with pytest.raises(_lib.B200QError): quant.gemv(p4.buf.ptr, _lib.Q4_K_WIDE, sum(rows), n_in, x, y, w2_ptr=p6.buf.ptr, n_first=40)      # not a whole row tile
+
+
 def test_kquant_wide_refuses():
   need_gpu()
   raw = synth.random_blocks(12, 16, 512, np.random.default_rng(0))

@@ -19,7 +19,7 @@ class GemvArgs(Structure):
               ("bias", c_void_p), ("residual", c_void_p), ("y", c_void_p), ("flags", c_int), ("max_ctas", c_int),
               ("xq_in", c_void_p), ("ss_in", c_void_p), ("ss_count", c_int), ("xq_out", c_void_p), ("xq_out_norm_weight", c_void_p),
               ("ss_out", c_void_p), ("residual_scale", c_float), ("peer_mailboxes", POINTER(c_void_p)), ("n_peers", c_int), ("peer_rank", c_int),
-              ("xq_out_stage", c_void_p)]
+              ("xq_out_stage", c_void_p), ("w_packed2", c_void_p), ("n_first", c_int)]
 
 
 class AttnArgs(Structure):

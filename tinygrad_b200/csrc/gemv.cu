@@ -29,7 +29,8 @@
 namespace {
 
 struct GemvParams {
-  const uint8_t* w;
+  const uint8_t *w, *w2;    // w2: the rows from tile `tiles_first` on (Q4_K with Q6_K behind it)
+  int tiles_first;
   const void* x;
   const __half* norm_w;
   const __half* bias;
@@ -85,6 +86,8 @@ template <> struct Cfg<B200Q_Q6_K> { static constexpr int NS = 3, SG = CONS_WARP
 // Two Q4_K tiles per warp and stage: 4 % over one (14336 x 4096 gate / up); Q6_K tiles are too large for that with two CTAs.
 template <> struct Cfg<B200Q_Q4_K_WIDE> { static constexpr int NS = 2, SG = STAGE_GROUPS, XSUB = 0; };        // stage = SG x 1216 B
 template <> struct Cfg<B200Q_Q6_K_WIDE> { static constexpr int NS = 3, SG = CONS_WARPS, XSUB = 0; };          // stage = SG x 1696 B
+constexpr int K_MIX = B200Q_Q4_K_WIDE + B200Q_Q6_K_WIDE;      // row tiles of both: query and key rows with value rows behind them
+template <> struct Cfg<K_MIX> : Cfg<B200Q_Q6_K_WIDE> {};
 template <int QT> constexpr int X_BYTES = is_wide(QT) ? 512 : XQ_GROUP_BYTES;  // staged bytes per 128 columns
 
 #ifdef B200Q_GEMV_PROF
@@ -157,7 +160,7 @@ __device__ __noinline__ void settle_handover(const GemvParams& p, float* ubuf, i
 // XQ_IN / XQ_OUT: compiled-in use of a ready-made input record / production of an output record.
 template <int QT, bool XQ_IN, bool XQ_OUT>
 __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(const GemvParams p) {
-  constexpr int NS = Cfg<QT>::NS, SG = Cfg<QT>::SG, XSUB = Cfg<QT>::XSUB, TB = tile_bytes(QT), STAGE_BYTES = SG * TB;
+  constexpr int NS = Cfg<QT>::NS, SG = Cfg<QT>::SG, XSUB = Cfg<QT>::XSUB, STAGE_BYTES = SG * tile_bytes(QT == K_MIX ? B200Q_Q6_K_WIDE : QT);
   constexpr bool WIDE = is_wide(QT);
   constexpr int XB = X_BYTES<QT>;
   static_assert(!(XQ_IN && (XSUB || WIDE)), "ready-made records are the plain int8 form");
@@ -225,7 +228,9 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
         for (int ti = 0; ti < run && ok; ti++) {
           const int rt = unit * run + ti;
           if (rt >= p.n_row_tiles) break;
-          const uint8_t* src = p.w + (size_t)rt * p.kgroups * TB;
+          const bool second = QT == K_MIX && rt >= p.tiles_first;
+          const int TB = QT == K_MIX ? tile_bytes(second ? B200Q_Q6_K_WIDE : B200Q_Q4_K_WIDE) : tile_bytes(QT);
+          const uint8_t* src = second ? p.w2 + (size_t)(rt - p.tiles_first) * p.kgroups * TB : p.w + (size_t)rt * p.kgroups * TB;
           for (int s = 0; s < stages_per_tile; s++, it++) {
             const int slot = it % NS, groups = min(SG, p.kgroups - s * SG);
             if (it == NS && !x_issued) after_prefetch();
@@ -234,7 +239,7 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
             // one stage = several bulk copies on the same barrier: a single copy is served slowly, several overlap
             for (int g0 = 0; g0 < groups; g0 += COPY_GROUPS) {
               const int gn = min(COPY_GROUPS, groups - g0);
-              bulk_g2s(smem_u32(ring + slot * STAGE_BYTES + g0 * TB), src + (size_t)s * STAGE_BYTES + (size_t)g0 * TB, gn * TB, full0 + 8 * slot);
+              bulk_g2s(smem_u32(ring + slot * STAGE_BYTES + g0 * TB), src + (size_t)(s * SG + g0) * TB, gn * TB, full0 + 8 * slot);
             }
           }
         }
@@ -439,6 +444,8 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
     for (int ti = 0; ti < run; ti++, n++) {
       const int rt = unit * run + ti;
       if (rt >= p.n_row_tiles) break;
+      const bool second = QT == K_MIX && rt >= p.tiles_first;
+      const int TB = QT == K_MIX ? tile_bytes(second ? B200Q_Q6_K_WIDE : B200Q_Q4_K_WIDE) : tile_bytes(QT);
       float acc0 = 0.f, acc1 = 0.f;
       [[maybe_unused]] float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
       for (int s = 0; s < stages_per_tile; s++, it++) {
@@ -453,7 +460,7 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
             const int j = s * SG + gi;
             if constexpr (WIDE) {
               const uint4* xb = xq + j * 32 + (g & 1) * 4 + t;
-              if constexpr (QT == B200Q_Q4_K_WIDE) tile_mac_q4k(stage + gi * TB, lane, xb, c0, c1);
+              if (QT == B200Q_Q4_K_WIDE || (QT == K_MIX && !second)) tile_mac_q4k(stage + gi * TB, lane, xb, c0, c1);
               else tile_mac_q6k_wide(stage + gi * TB, lane, xb, c0, c1);
             } else {
               const float4 st = xsc[(j * 2 + (t >> 1)) * 2 + (t & 1)];
@@ -517,7 +524,7 @@ namespace {
 template <int QT, bool XQ_IN, bool XQ_OUT>
 int launch_gemv(const b200q_gemv_args* a, const GemvParams& p, cudaStream_t stream) {
   constexpr int NS = Cfg<QT>::NS;
-  const size_t smem = (size_t)NS * Cfg<QT>::SG * tile_bytes(QT) + (size_t)p.kgroups * (X_BYTES<QT> + Cfg<QT>::XSUB) + 16 +
+  const size_t smem = (size_t)NS * Cfg<QT>::SG * tile_bytes(QT == K_MIX ? B200Q_Q6_K_WIDE : QT) + (size_t)p.kgroups * (X_BYTES<QT> + Cfg<QT>::XSUB) + 16 +
                       (2 * CONS_WARPS * 16 + CONS_WARPS + 32) * sizeof(float) + (2 * NS + 5) * sizeof(uint64_t) + 16;
   if (smem > 220 * 1024) return B200Q_ERR_TOO_LARGE;
   auto kern = qgemv_kernel<QT, XQ_IN, XQ_OUT>;
@@ -602,6 +609,12 @@ extern "C" int b200q_gemv(const b200q_gemv_args* a, void* stream) {
   if (a->xq_out && a->n_out % GROUP_ELEMS) return B200Q_ERR_BAD_SHAPE;
   if (a->xq_out_stage && (!a->xq_out || ((uintptr_t)a->xq_out_stage & 3))) return B200Q_ERR_BAD_ARG;
   GemvParams p;
+  p.w2 = (const uint8_t*)a->w_packed2; p.tiles_first = a->n_first / TILE_ROWS;
+  if (p.w2) {
+    if (a->qtype != B200Q_Q4_K_WIDE || a->epilogue != B200Q_EPI_LINEAR) return B200Q_ERR_UNSUPPORTED;
+    if (a->n_first <= 0 || a->n_first >= a->n_out || a->n_first % TILE_ROWS) return B200Q_ERR_BAD_SHAPE;
+    if ((uintptr_t)p.w2 & 15) return B200Q_ERR_MISALIGNED;
+  }
   p.w = (const uint8_t*)a->w_packed; p.x = a->x; p.norm_w = (const __half*)a->norm_weight; p.bias = (const __half*)a->bias;
   p.residual = (const float*)a->residual; p.residual_scale = a->residual_scale == 0.f ? 1.f : a->residual_scale; p.y = a->y;
   p.n_out = a->n_out; p.n_in = a->n_in; p.kgroups = ceil_div(a->n_in, GROUP_ELEMS);
@@ -623,6 +636,7 @@ extern "C" int b200q_gemv(const b200q_gemv_args* a, void* stream) {
   p.unit = (a->xq_out && !a->xq_out_stage) ? (a->epilogue == B200Q_EPI_SILU_MUL ? 4 : 2) : 1;
   p.n_units = ceil_div(p.n_row_tiles, p.unit);
   const bool xi = a->xq_in != nullptr, xo = a->xq_out != nullptr;
+  if (p.w2) return launch_gemv<K_MIX, false, false>(a, p, (cudaStream_t)stream);
   if (a->qtype == B200Q_Q4_K_WIDE) return launch_gemv<B200Q_Q4_K_WIDE, false, false>(a, p, (cudaStream_t)stream);
   if (a->qtype == B200Q_Q6_K_WIDE) return launch_gemv<B200Q_Q6_K_WIDE, false, false>(a, p, (cudaStream_t)stream);
   if (a->qtype == B200Q_Q4_0) {

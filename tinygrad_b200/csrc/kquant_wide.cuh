@@ -20,7 +20,7 @@
 
 namespace {
 
-__host__ __device__ constexpr bool is_wide(int qt) { return qt == B200Q_Q4_K_WIDE || qt == B200Q_Q6_K_WIDE; }
+__host__ __device__ constexpr bool is_wide(int qt) { return qt == B200Q_Q4_K_WIDE || qt == B200Q_Q6_K_WIDE || qt == B200Q_Q4_K_WIDE + B200Q_Q6_K_WIDE; }      // the last: both in one launch
 
 __device__ __forceinline__ uint32_t half2_bits(float a, float b) {
   const __half2 h = __floats2half2_rn(a, b);

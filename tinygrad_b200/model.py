@@ -67,19 +67,22 @@ class _BlockLinear:
   start in the vector it writes."""
   def __init__(self, qtype, n_out: int, n_in: int, buf: DeviceBuffer, row0: int, swiglu: bool = False):
     self.qtype, self.n_out, self.n_in, self.buf, self.row0, self.swiglu = qtype, n_out, n_in, buf, row0, swiglu
+    self.behind = None       # (Q6_K matrix, rows) of the rows behind a Q4_K one
 
   @property
   def algorithmic_bytes(self) -> int:
     if self.qtype is None: return 2 * self.n_out * self.n_in
-    return quant.PackedWeight(self.qtype, self.n_out, self.n_in, self.buf, self.swiglu).algorithmic_bytes
+    more = quant.PackedWeight(_lib.Q6_K_WIDE, self.behind[1], self.n_in, self.behind[0], False).algorithmic_bytes if self.behind else 0
+    return quant.PackedWeight(self.qtype, self.n_out, self.n_in, self.buf, self.swiglu).algorithmic_bytes + more
 
   def run(self, x, y, bias=None, residual=None, flags=0, **kw) -> None:
     at = lambda buf, size: None if buf is None else buf.ptr + size * self.row0
     if self.qtype is None:
       quant.gemv_dense(self.buf, F16, self.n_out, self.n_in, x, at(y, 4), bias=at(bias, 2), residual=at(residual, 4), flags=flags, **kw)
     else:
-      quant.gemv(self.buf.ptr, self.qtype, self.n_out, self.n_in, x, at(y, 4), bias=at(bias, 2), residual=at(residual, 4), flags=flags,
-                 epilogue=EPI_SILU_MUL if self.swiglu else quant.EPI_LINEAR, **kw)
+      w2, rows2 = self.behind or (None, 0)
+      quant.gemv(self.buf.ptr, self.qtype, self.n_out + rows2, self.n_in, x, at(y, 4), bias=at(bias, 2), residual=at(residual, 4), flags=flags,
+                 epilogue=EPI_SILU_MUL if self.swiglu else quant.EPI_LINEAR, w2_ptr=w2.ptr if w2 else None, n_first=self.n_out if w2 else 0, **kw)
 
 
 # hand-over edges used when the caller does not choose (see Transformer.__init__): the ones that measured faster
@@ -152,7 +155,8 @@ class Transformer:
               part = dense16(name, r, n_in)
               check(_lib.load().b200q_memcpy_d2d(buf.ptr + off, part.ptr, part.nbytes, None)); off += part.nbytes
               runtime_sync()
-          out.append(_BlockLinear(typ, n_out, n_in, buf, at))
+          if out and out[-1].qtype == _lib.Q4_K_WIDE and typ == _lib.Q6_K_WIDE: out[-1].behind = buf, n_out      # one launch for both
+          else: out.append(_BlockLinear(typ, n_out, n_in, buf, at))
           at += n_out
         return out
     for i in range(c.num_blocks if self.dense_blocks else 0):
