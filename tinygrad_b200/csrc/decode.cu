@@ -371,7 +371,7 @@ namespace {
 #endif
 
 // ---------------------------------------------------------------------------
-// The same attention for fp16 caches and head_dim 64 / 128: one thread-block cluster of 8 or 16 CTAs per KV head.
+// The same attention for head_dim 64 / 128: one thread-block cluster of 8 or 16 CTAs per KV head.
 //
 // What bounds it: at a few hundred positions nothing but latency.  In the kernel above (8B shape, position 520: 8.4 us from the row's arrival
 // to the last store; 10.4 us of a block with its launch, 6.5 now) 3.4 us went into dot products of one lane per position and head, which read every cached row once per query head, and
@@ -382,16 +382,29 @@ namespace {
 //  * the positions are split over the cluster's CTAs in whole chunks of 64; the CTAs' partial results meet in distributed shared memory: one
 //    cluster barrier and one round of remote loads.  The split follows the position, so contexts of any length are spread over all CTAs;
 //  * two chunks are in flight, the first two already before the wait for the previous kernel.
+// fp32 caches: the same with m16n8k8 tf32 products.  Queries, probabilities and cached values are all split in two tf32 numbers (2^-22 of the value
+// together, with the range of fp32), a cached value on its way from shared memory to the operand.
 constexpr int AC_THREADS = 256, AC_POS = 64;
-template <int HD> struct AcSmem {           // bytes; rows padded by 16 so that fragment loads hit distinct banks
-  static constexpr int KROW = (HD + 8) * 2, CHUNK = AC_POS * KROW, PROW = (AC_POS + 8) * 2;
-  static constexpr int KV = 0, Q = KV + 4 * CHUNK, P = Q + 16 * KROW, S = P + 16 * PROW, O = S + 8 * (AC_POS + 4) * 4, ST = O + 8 * HD * 4, NEW = ST + 8 * 4 * 4,
-                       TOTAL = NEW + 2 * HD * 2;
+template <int HD, typename KV> struct AcSmem {           // bytes; rows padded so that fragment loads hit distinct banks
+  static constexpr bool F32 = sizeof(KV) == 4;
+  static constexpr int KROW = F32 ? (HD + 4) * 4 : (HD + 8) * 2, VROW = (HD + 8) * (int)sizeof(KV), QROW = KROW, PROW = F32 ? (AC_POS + 4) * 4 : (AC_POS + 8) * 2;
+  static constexpr int VCHUNK = AC_POS * KROW, BUF = AC_POS * (KROW + VROW);      // a buffer: 64 rows of K, 64 rows of V
+  static constexpr int Q = 2 * BUF, P = Q + 16 * QROW, S = P + 16 * PROW, O = S + 8 * (AC_POS + 4) * 4, ST = O + 8 * HD * 4, NEW = ST + 8 * 4 * 4,
+                       TOTAL = NEW + 2 * HD * (int)sizeof(KV);
 };
 
 __device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// tf32 high part and the remainder's tf32 rounding (both are valid fp32 bit patterns)
+__device__ __forceinline__ void split_tf32(float v, uint32_t& hi, uint32_t& lo) {
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(v));
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(v - __uint_as_float(hi)));
 }
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
@@ -415,15 +428,36 @@ __device__ __forceinline__ void split_h(float v, __half& hi, __half& lo) {
   lo = __float2half_rn(fminf(fmaxf(v - __half2float(hi), -65504.f), 65504.f));
 }
 
-template <int HD, int CL>      // CL: CTAs per cluster
+// value d of a row, split in two rows of operand values
+template <typename KV> __device__ __forceinline__ void store_split(float v, unsigned char* hi_row, unsigned char* lo_row, int d) {
+  if constexpr (sizeof(KV) == 4) {
+    split_tf32(v, reinterpret_cast<uint32_t*>(hi_row)[d], reinterpret_cast<uint32_t*>(lo_row)[d]);
+  } else {
+    __half hi, lo;
+    split_h(v, hi, lo);
+    reinterpret_cast<__half*>(hi_row)[d] = hi; reinterpret_cast<__half*>(lo_row)[d] = lo;
+  }
+}
+template <typename KV> __device__ __forceinline__ KV cache_cast(float v);
+template <> __device__ __forceinline__ __half cache_cast<__half>(float v) { return __float2half_rn(v); }
+template <> __device__ __forceinline__ float cache_cast<float>(float v) { return v; }
+// m16n8k8 A fragment: rows g and g + 8 (`down` bytes on), columns t and t + 4
+__device__ __forceinline__ void ld_frag_tf32(uint32_t (&r)[4], const unsigned char* at, int down) {
+  r[0] = *reinterpret_cast<const uint32_t*>(at); r[1] = *reinterpret_cast<const uint32_t*>(at + down);
+  r[2] = *reinterpret_cast<const uint32_t*>(at + 16); r[3] = *reinterpret_cast<const uint32_t*>(at + down + 16);
+}
+
+template <int HD, int CL, typename KV>      // CL: CTAs per cluster
 __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_attn_args a_in, const SeqStride sq) {
-  using M = AcSmem<HD>;
+  using M = AcSmem<HD, KV>;
+  constexpr bool F32 = M::F32;
+  constexpr int VEC = 16 / sizeof(KV), ROW_VECS = HD / VEC;         // cache elements per 16 bytes, 16-byte pieces per row
   extern __shared__ __align__(16) unsigned char asmem[];
   b200q_attn_args a = a_in;
   if (blockIdx.z) {
     const size_t z = blockIdx.z;
     a.qkv += z * sq.qkv; a.out += z * sq.out; a.pos += z * sq.pos;
-    a.k_cache = reinterpret_cast<__half*>(a.k_cache) + z * sq.cache; a.v_cache = reinterpret_cast<__half*>(a.v_cache) + z * sq.cache;
+    a.k_cache = reinterpret_cast<KV*>(a.k_cache) + z * sq.cache; a.v_cache = reinterpret_cast<KV*>(a.v_cache) + z * sq.cache;
   }
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int kvh = blockIdx.x, rank = blockIdx.y, n_rep = a.n_heads / a.n_kv_heads, half_r = a.rope_dim >> 1;
@@ -432,18 +466,18 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
   float* s_o = reinterpret_cast<float*>(asmem + M::O);            // [8][HD] this CTA's unnormalised output
   float* s_m = reinterpret_cast<float*>(asmem + M::ST);           // [8] running max, [8] denominator, [8] rescale factor
   float *s_l = s_m + 8, *s_c = s_m + 16;
-  __half* s_new = reinterpret_cast<__half*>(asmem + M::NEW);      // the new position's K and V rows
-  __half* kc = reinterpret_cast<__half*>(a.k_cache) + (size_t)kvh * a.max_context * HD;
-  __half* vc = reinterpret_cast<__half*>(a.v_cache) + (size_t)kvh * a.max_context * HD;
+  KV* s_new = reinterpret_cast<KV*>(asmem + M::NEW);              // the new position's K and V rows
+  KV* kc = reinterpret_cast<KV*>(a.k_cache) + (size_t)kvh * a.max_context * HD;
+  KV* vc = reinterpret_cast<KV*>(a.v_cache) + (size_t)kvh * a.max_context * HD;
   pdl_launch_dependents();
   // cached rows of chunk `ch` -> buffer `buf` (asynchronously, one commit group)
   auto fetch = [&](int ch, int buf, int pos_now) {
     const int n_old = min(AC_POS, pos_now - ch * AC_POS);
-    for (int i = tid; i < n_old * (HD / 8); i += AC_THREADS) {
-      const int r = i / (HD / 8), c = (i - r * (HD / 8)) * 8;
-      const size_t at = (size_t)(ch * AC_POS + r) * HD + c;
-      cp_async16(asmem + M::KV + (2 * buf) * M::CHUNK + r * M::KROW + c * 2, kc + at);
-      cp_async16(asmem + M::KV + (2 * buf + 1) * M::CHUNK + r * M::KROW + c * 2, vc + at);
+    for (int i = tid; i < n_old * ROW_VECS; i += AC_THREADS) {
+      const int r = i / ROW_VECS, c = i - r * ROW_VECS;
+      const size_t at = (size_t)(ch * AC_POS + r) * HD + c * VEC;
+      cp_async16(asmem + buf * M::BUF + r * M::KROW + c * 16, kc + at);
+      cp_async16(asmem + buf * M::BUF + M::VCHUNK + r * M::VROW + c * 16, vc + at);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -465,7 +499,7 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
   const int pos_early = min(max(__ldcg(a.pos), 0), a.max_context - 1);
   start(pos_early);
   if (tid * 32 < a.rope_dim) prefetch_l2(a.rope + (size_t)pos_early * a.rope_dim + tid * 32);
-  for (int i = tid; i < (16 * M::KROW + 16 * M::PROW) / 16; i += AC_THREADS) reinterpret_cast<uint4*>(asmem + M::Q)[i] = make_uint4(0, 0, 0, 0);   // rows of absent heads
+  for (int i = tid; i < (16 * M::QROW + 16 * M::PROW) / 16; i += AC_THREADS) reinterpret_cast<uint4*>(asmem + M::Q)[i] = make_uint4(0, 0, 0, 0);   // rows of absent heads
   if (tid < 8) { s_m[tid] = -INFINITY; s_l[tid] = 0.f; }
   __syncthreads();
   pdl_wait();
@@ -491,16 +525,13 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
   if (c0 < c1) {
     for (int i = tid; i < n_rep * HD; i += AC_THREADS) {
       const int r = i / HD, d = i - r * HD;
-      __half hi, lo;
-      split_h(roped(a.qkv + (size_t)(kvh * n_rep + r) * HD, d), hi, lo);
-      *reinterpret_cast<__half*>(asmem + M::Q + r * M::KROW + d * 2) = hi;
-      *reinterpret_cast<__half*>(asmem + M::Q + (8 + r) * M::KROW + d * 2) = lo;
+      store_split<KV>(roped(a.qkv + (size_t)(kvh * n_rep + r) * HD, d), asmem + M::Q + r * M::QROW, asmem + M::Q + (8 + r) * M::QROW, d);
     }
     if (owner) {
       for (int i = tid; i < 2 * HD; i += AC_THREADS) {
         const int d = i % HD;
         const bool v = i >= HD;
-        const __half h = __float2half_rn(v ? a.qkv[(size_t)(a.n_heads + a.n_kv_heads + kvh) * HD + d] : roped(a.qkv + (size_t)(a.n_heads + kvh) * HD, d));
+        const KV h = cache_cast<KV>(v ? a.qkv[(size_t)(a.n_heads + a.n_kv_heads + kvh) * HD + d] : roped(a.qkv + (size_t)(a.n_heads + kvh) * HD, d));
         s_new[i] = h;
         (v ? vc : kc)[(size_t)pos * HD + d] = h;
       }
@@ -512,25 +543,39 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
   const float scale = 1.0f / sqrtf((float)HD);
   for (int ch = c0; ch < c1; ch++) {
     const int buf = (ch - c0) & 1, nv = min(AC_POS, pos + 1 - ch * AC_POS);
-    unsigned char* sk = asmem + M::KV + (2 * buf) * M::CHUNK;
+    unsigned char* sk = asmem + buf * M::BUF;
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();                                                 // (also: queries and the new rows are in place)
     if (nv < AC_POS || (owner && ch == c1 - 1)) {                    // the last chunk: append the new row, and no stale values behind it (0 * NaN)
-      for (int i = tid; i < 2 * HD; i += AC_THREADS) *reinterpret_cast<__half*>(sk + (i / HD) * M::CHUNK + (nv - 1) * M::KROW + (i % HD) * 2) = s_new[i];
-      for (int i = tid; i < (AC_POS - nv) * (HD / 8); i += AC_THREADS)
-        *reinterpret_cast<uint4*>(sk + M::CHUNK + (nv + i / (HD / 8)) * M::KROW + (i % (HD / 8)) * 16) = make_uint4(0, 0, 0, 0);
+      for (int i = tid; i < 2 * HD; i += AC_THREADS)
+        *reinterpret_cast<KV*>(sk + (i < HD ? (nv - 1) * M::KROW : M::VCHUNK + (nv - 1) * M::VROW) + (i % HD) * (int)sizeof(KV)) = s_new[i];
+      for (int i = tid; i < (AC_POS - nv) * ROW_VECS; i += AC_THREADS)
+        *reinterpret_cast<uint4*>(sk + M::VCHUNK + (nv + i / ROW_VECS) * M::VROW + (i % ROW_VECS) * 16) = make_uint4(0, 0, 0, 0);
       __syncthreads();
     }
     {   // scores: warp w takes positions 8w .. 8w + 7
       float c[4] = {0.f, 0.f, 0.f, 0.f}, c2[4] = {0.f, 0.f, 0.f, 0.f};
-      const uint32_t qa = base + M::Q + (lane & 15) * M::KROW + (lane >> 4) * 16;
       const unsigned char* kr = sk + (warp * 8 + g) * M::KROW + t * 4;
+      if constexpr (F32) {
+        const unsigned char* qa = asmem + M::Q + g * M::QROW + t * 4;
+#pragma unroll 4
+        for (int kk = 0; kk < HD / 8; kk++) {
+          uint32_t q4[4], h0, l0, h1, l1;
+          ld_frag_tf32(q4, qa + kk * 32, 8 * M::QROW);
+          split_tf32(*reinterpret_cast<const float*>(kr + kk * 32), h0, l0);
+          split_tf32(*reinterpret_cast<const float*>(kr + kk * 32 + 16), h1, l1);
+          mma_tf32(c, q4, h0, h1);
+          mma_tf32(c2, q4, l0, l1);
+        }
+      } else {
+        const uint32_t qa = base + M::Q + (lane & 15) * M::QROW + (lane >> 4) * 16;
 #pragma unroll
-      for (int kk = 0; kk < HD / 16; kk++) {
-        uint32_t q4[4];
-        ldsm4(q4, qa + kk * 32);
-        const uint32_t b0 = *reinterpret_cast<const uint32_t*>(kr + kk * 32), b1 = *reinterpret_cast<const uint32_t*>(kr + kk * 32 + 16);
-        if (kk & 1) mma_f16(c2, q4, b0, b1); else mma_f16(c, q4, b0, b1);
+        for (int kk = 0; kk < HD / 16; kk++) {
+          uint32_t q4[4];
+          ldsm4(q4, qa + kk * 32);
+          const uint32_t b0 = *reinterpret_cast<const uint32_t*>(kr + kk * 32), b1 = *reinterpret_cast<const uint32_t*>(kr + kk * 32 + 16);
+          if (kk & 1) mma_f16(c2, q4, b0, b1); else mma_f16(c, q4, b0, b1);
+        }
       }
       const int p = warp * 8 + 2 * t;
       const float s0 = ((c[0] + c2[0]) + (c[2] + c2[2])) * scale, s1 = ((c[1] + c2[1]) + (c[3] + c2[3])) * scale;
@@ -542,10 +587,15 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
       const float2 s2 = *reinterpret_cast<const float2*>(s_s + warp * (AC_POS + 4) + 2 * lane);
       const float m0 = s_m[warp], m1 = fmaxf(m0, warp_max(fmaxf(s2.x, s2.y)));
       const float p0 = __expf(s2.x - m1), p1 = __expf(s2.y - m1), cr = __expf(m0 - m1), sum = warp_sum(p0 + p1);
-      __half h0, l0, h1, l1;
-      split_h(p0, h0, l0); split_h(p1, h1, l1);
-      *reinterpret_cast<__half2*>(asmem + M::P + warp * M::PROW + lane * 4) = __halves2half2(h0, h1);
-      *reinterpret_cast<__half2*>(asmem + M::P + (8 + warp) * M::PROW + lane * 4) = __halves2half2(l0, l1);
+      if constexpr (F32) {
+        store_split<KV>(p0, asmem + M::P + warp * M::PROW, asmem + M::P + (8 + warp) * M::PROW, 2 * lane);
+        store_split<KV>(p1, asmem + M::P + warp * M::PROW, asmem + M::P + (8 + warp) * M::PROW, 2 * lane + 1);
+      } else {
+        __half h0, l0, h1, l1;
+        split_h(p0, h0, l0); split_h(p1, h1, l1);
+        *reinterpret_cast<__half2*>(asmem + M::P + warp * M::PROW + lane * 4) = __halves2half2(h0, h1);
+        *reinterpret_cast<__half2*>(asmem + M::P + (8 + warp) * M::PROW + lane * 4) = __halves2half2(l0, l1);
+      }
       __syncwarp();
       if (lane == 0) { s_m[warp] = m1; s_l[warp] = s_l[warp] * cr + sum; s_c[warp] = cr; }
     }
@@ -554,9 +604,25 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
       const float cr = g < n_rep ? s_c[g] : 0.f;
 #pragma unroll
       for (int j = 0; j < HD / 64; j++) { acc[j][0] *= cr; acc[j][1] *= cr; acc[j][2] *= cr; acc[j][3] *= cr; }
+      if constexpr (F32) {
+        const unsigned char *pa = asmem + M::P + g * M::PROW + t * 4, *va = sk + M::VCHUNK + t * M::VROW + (warp * (HD / 8) + g) * 4;
+#pragma unroll 4
+        for (int kk = 0; kk < AC_POS / 8; kk++) {
+          uint32_t p4[4];
+          ld_frag_tf32(p4, pa + kk * 32, 8 * M::PROW);
+#pragma unroll
+          for (int j = 0; j < HD / 64; j++) {
+            uint32_t h0, l0, h1, l1;
+            split_tf32(*reinterpret_cast<const float*>(va + kk * 8 * M::VROW + j * 32), h0, l0);
+            split_tf32(*reinterpret_cast<const float*>(va + (kk * 8 + 4) * M::VROW + j * 32), h1, l1);
+            mma_tf32(acc[j], p4, h0, h1);
+            mma_tf32(acc[j], p4, l0, l1);
+          }
+        }
+      } else {
       const uint32_t pa = base + M::P + (lane & 15) * M::PROW + (lane >> 4) * 16;
       // transposing loads: 8x8 blocks of (positions, dims).  128: positions kk*16 + {0..7, 8..15} x dims {0..7, 8..15}; 64: 32 positions x 8 dims
-      const uint32_t va = base + (uint32_t)(sk - asmem) + M::CHUNK + warp * (HD / 8) * 2 +
+      const uint32_t va = base + (uint32_t)(sk - asmem) + M::VCHUNK + warp * (HD / 8) * 2 +
                           (HD == 128 ? (((lane >> 3) & 1) * 8 + (lane & 7)) * M::KROW + (lane >> 4) * 16 : lane * M::KROW);
       if (HD == 128) {
 #pragma unroll
@@ -578,6 +644,7 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
           mma_f16(acc[0], p4, v4[2], v4[3]);
         }
       }
+      }
     }
     if (ch + 2 < c1) {
       __syncthreads();                                               // everybody is done with the buffer
@@ -590,8 +657,7 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
     *reinterpret_cast<float2*>(s_o + g * HD + warp * (HD / 8) + j * 8 + 2 * t) = make_float2(acc[j][0] + acc[j][2], acc[j][1] + acc[j][3]);
   cluster_sync();
   // merge: the (head, 32 dims) units are dealt over the cluster's CTAs, one warp each
-  const int u = warp * CL + rank;
-  if (u < n_rep * (HD / 32)) {
+  for (int u = warp * CL + rank; u < n_rep * (HD / 32); u += AC_THREADS / 32 * CL) {
     const int h = u / (HD / 32), d = (u - h * (HD / 32)) * 32 + lane;
     const uint32_t st = base + M::ST + h * 4, oa = base + M::O + (h * HD + d) * 4;
     float o[CL];
@@ -606,6 +672,7 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
     v /= den;
     a.out[(size_t)(kvh * n_rep + h) * HD + d] = v;
     if (a.xq_out) quant_block_32x1(v, lane, (kvh * n_rep + h) * (HD / 32) + (d >> 5), XqDst(a.xq_out, a.n_heads));      // head_dim 128: one group per head
+    if (CL > 1) break;                                               // one unit per warp at most
   }
   cluster_sync();                                                    // nobody leaves while its partial results are being read
 }
@@ -728,25 +795,25 @@ extern "C" size_t b200q_attn_seq_scratch_stride(int n_heads, int n_kv_heads, int
   return (b200q_attn_scratch_bytes(n_heads, n_kv_heads, head_dim, n_split) + 255) & ~(size_t)255;
 }
 
-template <int HD, int CL>
+template <int HD, int CL, typename KV>
 static int launch_attn_cluster(const b200q_attn_args* a, const SeqStride& sq, int n_seqs, bool pdl, cudaStream_t stream, int* max_clusters = nullptr) {
-  auto kern = attn_cluster_kernel<HD, CL>;
+  auto kern = attn_cluster_kernel<HD, CL, KV>;
   static PerDeviceFlag attr_set;
   const int dev = b200q_current_device();
   if (dev < 0) return B200Q_ERR_CUDA;
   if (!attr_set.test(dev)) {
-    B200Q_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AcSmem<HD>::TOTAL));
+    B200Q_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (AcSmem<HD, KV>::TOTAL)));
     if (CL > 8) B200Q_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     attr_set.set(dev);
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(a->n_kv_heads, CL, n_seqs); cfg.blockDim = dim3(AC_THREADS); cfg.dynamicSmemBytes = AcSmem<HD>::TOTAL; cfg.stream = stream;
+  cfg.gridDim = dim3(a->n_kv_heads, CL, n_seqs); cfg.blockDim = dim3(AC_THREADS); cfg.dynamicSmemBytes = (AcSmem<HD, KV>::TOTAL); cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = CL; attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr; cfg.numAttrs = pdl ? 2 : 1;
+  cfg.attrs = CL > 1 ? attr : attr + 1; cfg.numAttrs = (CL > 1) + pdl;
   if (max_clusters) {                                                // how many clusters run at once (0: not even one)
     cfg.numAttrs = 1;
     B200Q_CHECK_CUDA(cudaOccupancyMaxActiveClusters(max_clusters, kern, &cfg));
@@ -758,19 +825,22 @@ static int launch_attn_cluster(const b200q_attn_args* a, const SeqStride& sq, in
 
 // Clusters of 16 CTAs where the device runs all KV heads' clusters at once (14 of them on B200), of 8 (portable) otherwise: with few KV heads the
 // cached rows stream through twice the SMs (4 heads, position 3507: 17.9 -> 12.6 us per block); at short contexts both take the same time.
-template <int HD>
+template <int HD, typename KV>
 static int attn_cluster(const b200q_attn_args* a, const SeqStride& sq, int n_seqs, bool pdl, cudaStream_t stream) {
+  // one chunk at most: one CTA does it all (a launch with clusters costs a graph replay 1.7 us: 3-block 512-wide model, 54 positions, 950 us for 16 tokens with
+  // clusters of 16, 890 so)
+  if (a->max_context <= AC_POS) return launch_attn_cluster<HD, 1, KV>(a, sq, n_seqs, pdl, stream);
   static std::atomic<int> wide[B200Q_MAX_DEVICES];                   // clusters of 16 that run at once, plus one; 0: not asked yet
   const int dev = b200q_current_device();
   if (dev < 0) return B200Q_ERR_CUDA;
   int w = wide[dev].load(std::memory_order_relaxed);
   if (w == 0) {
     int n = 0;
-    if (launch_attn_cluster<HD, 16>(a, sq, n_seqs, pdl, stream, &n) != B200Q_OK) n = 0;
+    if (launch_attn_cluster<HD, 16, KV>(a, sq, n_seqs, pdl, stream, &n) != B200Q_OK) n = 0;
     w = n + 1;
     wide[dev].store(w, std::memory_order_relaxed);
   }
-  return a->n_kv_heads * n_seqs < w ? launch_attn_cluster<HD, 16>(a, sq, n_seqs, pdl, stream) : launch_attn_cluster<HD, 8>(a, sq, n_seqs, pdl, stream);
+  return a->n_kv_heads * n_seqs < w ? launch_attn_cluster<HD, 16, KV>(a, sq, n_seqs, pdl, stream) : launch_attn_cluster<HD, 8, KV>(a, sq, n_seqs, pdl, stream);
 }
 
 static int attn_decode_launch(const b200q_attn_args* a, int n_seqs, void* stream) {
@@ -788,8 +858,10 @@ static int attn_decode_launch(const b200q_attn_args* a, int n_seqs, void* stream
     sq.scratch_bytes = b200q_attn_seq_scratch_stride(a->n_heads, a->n_kv_heads, a->head_dim, a->n_split);
   }
   bool pdl = (a->flags & B200Q_FLAG_PDL) != 0;
-  if (a->kv_dtype == B200Q_F16 && (a->head_dim == 64 || a->head_dim == 128)) {
-    return a->head_dim == 128 ? attn_cluster<128>(a, sq, n_seqs, pdl, (cudaStream_t)stream) : attn_cluster<64>(a, sq, n_seqs, pdl, (cudaStream_t)stream);
+  if (a->head_dim == 64 || a->head_dim == 128) {
+    cudaStream_t st = (cudaStream_t)stream;
+    if (a->kv_dtype == B200Q_F16) return a->head_dim == 128 ? attn_cluster<128, __half>(a, sq, n_seqs, pdl, st) : attn_cluster<64, __half>(a, sq, n_seqs, pdl, st);
+    return a->head_dim == 128 ? attn_cluster<128, float>(a, sq, n_seqs, pdl, st) : attn_cluster<64, float>(a, sq, n_seqs, pdl, st);
   }
   const int esz = a->kv_dtype == B200Q_F16 ? 2 : 4, vec = 16 / esz;
   size_t smem = (size_t)2 * ATTN_CHUNK * (a->head_dim + vec) * esz + (size_t)n_rep * (a->head_dim + ATTN_CHUNK + a->head_dim + 4) * sizeof(float);

@@ -15,8 +15,8 @@ from ._lib import check, F32, F16, EPI_LINEAR, EPI_SILU_MUL, FLAG_PDL
 from .runtime import DeviceBuffer, PinnedBuffer, Stream, Graph, Event, synchronize as runtime_sync
 import ctypes, itertools, os
 
-# batched decode with an fp32 cache or another head_dim: attention of all sequences in one launch of the one-lane-per-position decode kernel
-# instead of the prompt-pass kernels with one query row per CTA (measured 1.4 % slower at 8 sequences x 130 positions: off unless asked for)
+# batched decode with another head_dim than 64 or 128: attention of all sequences in one launch of the one-lane-per-position decode kernel instead of
+# the prompt-pass kernels with one query row per CTA (measured 1.4 % slower at 8 sequences x 130 positions: off unless asked for)
 SEQ_ATTENTION = os.environ.get("B200Q_SEQ_ATTENTION", "0") == "1"
 
 
@@ -536,8 +536,8 @@ class Transformer:
     # the position comes from the device (sequence 0's counter; all sequences move together), so the launch sequence can be replayed as a graph
     check(lib.b200q_embed_rows(self.token_embd.ptr, self.tokens.ptr, c.max_context + 1, self.pos.ptr, B, c.dim, c.vocab_size, f["x"].ptr, s))
     fold = few or quant.PIPELINED_GEMM     # both apply the RMSNorm in their pre-pass: no norm launches
-    # fp16 caches with head_dim 64 or 128: one launch of the cluster kernel, a cluster per (KV head, sequence)
-    seq_attn = (SEQ_ATTENTION or (kvdt == F16 and c.head_dim in (64, 128))) and c.n_heads // c.n_kv_heads <= 8 and c.head_dim % 8 == 0 and c.head_dim <= 128
+    # head_dim 64 or 128: one launch of the cluster kernel, a cluster per (KV head, sequence)
+    seq_attn = (SEQ_ATTENTION or c.head_dim in (64, 128)) and c.n_heads // c.n_kv_heads <= 8 and c.head_dim % 8 == 0 and c.head_dim <= 128
     if seq_attn and self._seq_attn_scratch is None:
       stride = lib.b200q_attn_seq_scratch_stride(c.n_heads, c.n_kv_heads, c.head_dim, self.n_split)
       self._seq_attn_scratch = DeviceBuffer(B * stride, zero=True)
