@@ -31,6 +31,11 @@ constexpr int THREADS = (UNPACK_WARPS + 2) * 32;
 constexpr int KSTEP = 32;                               // one quant block of K per step
 __host__ __device__ constexpr int steps_per_slot(int wt) { return wt == 128 ? 4 : 1; }
 constexpr int RING_BYTES = 224 * 1024, MAX_SLOTS = 6;   // shared memory: slots of unpacked weights + activations
+// Few activation rows (128 weight rows a tile): packed blocks wait in shared memory, one 16 / 32-byte block and its scale per unpack thread and K
+// group, up to MAX_AHEAD groups ahead.  A queue in registers that moves up by a block waits for the newest load every time: whatever its depth a
+// group took a round trip to HBM (8B gate / up, 45 rows: 83 us, 70 here; 8 rows: 79, 60).
+constexpr int MAX_AHEAD = 4;
+__host__ __device__ constexpr int ahead_bytes(int qt) { return UNPACK_THREADS * (qt == B200Q_Q4_0 ? 20 : 36); }
 constexpr int MAX_NT = 256;                             // activation rows per tile
 constexpr size_t COUNTER_BYTES = 4096;                  // one arrival counter per CTA (a split tile is counted at the CTA that holds its head)
 
@@ -46,7 +51,7 @@ struct StreamParams {
   // Units are dealt in multiples of this: 1, or a whole tile where the caller wants it so (`unsplit`) or the workspace has no room for partial
   // sums.  With whole tiles every output is one running sum (halves not side by side either) in the order of b200q_qgemm: the same bits.
   int grain, unsplit;
-  int tiles, m, n_out, kgroups, n_row_tiles, nt, tok_tiles, slots, y_f16, silu_mul;
+  int tiles, m, n_out, kgroups, n_row_tiles, nt, tok_tiles, slots, ahead, y_f16, silu_mul;
 };
 
 // ---- activations: fp32 (or fp16) rows, optionally RMS-normed, -> fp16 halves as the tensor core reads them ---------------------
@@ -277,6 +282,11 @@ __device__ __forceinline__ bool finish_segment(const StreamParams& p, Shared& sh
   return true;
 }
 
+__device__ __forceinline__ uint4 ld_shared4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
 // the weights of one 32-wide block of a row as they come from memory
 template <int QT> struct Raw;
 template <> struct Raw<B200Q_Q4_0> { uint4 a; uint32_t d; };
@@ -418,8 +428,43 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
       }
     };
     Raw<QT> q[DEPTH];
+    // 128 weight rows: this thread's places in the waiting blocks (never read by another thread, so no barrier)
+    constexpr bool STAGED = WT == 128;
+    constexpr uint32_t AHEAD = ahead_bytes(QT), SCALE_AT = UNPACK_THREADS * (QT == B200Q_Q4_0 ? 16 : 32);
+    const uint32_t wait0 = ring + slots * slot_bytes, wait_end = wait0 + p.ahead * AHEAD;
+    uint32_t wait_at = wait0;                            // the oldest waiting block
+    auto request = [&](uint32_t at) {                    // copies the next block there; zeros past the last row tile or K group
+      const bool in = fp && f_units > 0;
+      const uint8_t* src = in ? fp : p.w;
+      const uint32_t n16 = in ? 16u : 0u, n4 = in ? 4u : 0u;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at + tid * 16), "l"(src + (in ? in_w : 0)), "r"(n16) : "memory");
+      if constexpr (QT == B200Q_Q8_0)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at + UNPACK_THREADS * 16 + tid * 16), "l"(src + (in ? in_w + 512 : 0)), "r"(n16) : "memory");
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(at + SCALE_AT + tid * 4), "l"(src + (in ? in_d + (grp >> 1) * 8 : 0)), "r"(n4) : "memory");
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      if (in) fp += TB;
+      f_units--;
+      if (--f_left == 0) { ft++; f_left = p.kgroups; set_tile(0); }
+    };
+    auto collect = [&](Raw<QT>& q) {
+      switch (p.ahead) {
+        case 1: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
+        case 2: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
+        case 3: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
+        default: asm volatile("cp.async.wait_group 3;" ::: "memory");
+      }
+      q.a = ld_shared4(wait_at + tid * 16);
+      if constexpr (QT == B200Q_Q8_0) q.b = ld_shared4(wait_at + UNPACK_THREADS * 16 + tid * 16);
+      uint32_t d;
+      asm volatile("ld.shared.u32 %0, [%1];" : "=r"(d) : "r"(wait_at + SCALE_AT + tid * 4) : "memory");
+      q.d = grp & 1 ? d >> 16 : d & 0xFFFFu;
+    };
+    if constexpr (STAGED) {
+      for (int d = 0; d < p.ahead; d++) request(wait0 + d * AHEAD);
+    } else {
 #pragma unroll
-    for (int d = 0; d < DEPTH; d++) fetch(q[d]);
+      for (int d = 0; d < DEPTH; d++) fetch(q[d]);
+    }
     pdl_wait();                                          // the epilogue reads and writes what earlier kernels touched
     // One block: wait for its slot, unpack, hand over, ask for the block DEPTH further on.
     int slot = SPS > 1 ? 0 : grp;                        // ring position and its phase; SPS == 1: the thread groups take turns
@@ -429,6 +474,7 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
     bool ok = true;
     auto unpack = [&](Raw<QT>& q) {
       ok = ok && bar_wait(sb, BAR(sb, empty) + 8 * slot, par);
+      if constexpr (STAGED) collect(q);
       const uint32_t dst = ring + slot * slot_bytes + (SPS > 1 ? grp * W_STEP : 0) + r * 16;
       const uint32_t d2 = q.d | (q.d << 16);
       uint4 hi[4], lo[4];
@@ -455,7 +501,10 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
       }
       __syncwarp();
       if (lane == 0) bar_arrive(BAR(sb, full) + 8 * slot);
-      fetch(q);
+      if constexpr (STAGED) {
+        request(wait_at);
+        if ((wait_at += AHEAD) == wait_end) wait_at = wait0;
+      } else fetch(q);
       slot += SLOT_STEP;
       if (slot >= slots) { slot -= slots; par ^= 1; }
     };
@@ -478,10 +527,12 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
 #pragma unroll 1
         for (; left > stop && ok; left--) {
           unpack(q[0]);
-          const Raw<QT> head = q[0];
+          if constexpr (!STAGED) {
+            const Raw<QT> head = q[0];
 #pragma unroll
-          for (int d = 0; d + 1 < DEPTH; d++) q[d] = q[d + 1];
-          q[DEPTH - 1] = head;
+            for (int d = 0; d + 1 < DEPTH; d++) q[d] = q[d + 1];
+            q[DEPTH - 1] = head;
+          }
         }
         if (done_tile >= 0 && ok) {
           ok = finish_segment<WT, F32>(p, sh, sb, seg++, done_tile, done_k0, done_k1);
@@ -492,6 +543,7 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
       done_tile = tile; done_k0 = k0; done_k1 = k1;
       u += k1 - k0;
     }
+    if constexpr (STAGED) asm volatile("cp.async.wait_group 0;" ::: "memory");      // nothing may still be landing when the CTA leaves
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -521,7 +573,7 @@ int launch_stream(const StreamParams& p, int grid, cudaStream_t st) {
     B200Q_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, RING_BYTES));
     attr.set(dev);
   }
-  B200Q_CHECK_CUDA(launch_k(kern, dim3(grid), dim3(THREADS), (size_t)p.slots * slot_bytes({p.nt, p.tok_tiles, WT}, F32), st, true, p));
+  B200Q_CHECK_CUDA(launch_k(kern, dim3(grid), dim3(THREADS), (size_t)p.slots * slot_bytes({p.nt, p.tok_tiles, WT}, F32) + (size_t)p.ahead * ahead_bytes(QT), st, true, p));
   return B200Q_OK;
 }
 
@@ -589,8 +641,11 @@ int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtyp
   p.bias = (const __half*)bias_f16; p.residual = residual; p.y = y;
   p.m = m; p.n_out = n_out; p.kgroups = kgroups; p.n_row_tiles = ceil_div(n_out, TILE_ROWS);
   p.nt = pl.nt; p.tok_tiles = pl.tok_tiles;
-  p.slots = RING_BYTES / slot_bytes(pl, f32);                  // 2 (64 rows) to 3 K groups, or 3 (256 rows) to 5 steps
+  // 2 K groups, or 3 (256 rows) to 5 steps; what two K groups leave, at least one group's blocks, is for the packed blocks ahead
+  p.slots = pl.wt == 128 ? 2 : RING_BYTES / slot_bytes(pl, f32);
   if (p.slots > MAX_SLOTS) p.slots = MAX_SLOTS;
+  p.ahead = pl.wt == 128 ? (RING_BYTES - p.slots * slot_bytes(pl, f32)) / ahead_bytes(qtype) : 0;
+  if (p.ahead > MAX_AHEAD) p.ahead = MAX_AHEAD;
   p.y_f16 = y_dtype == B200Q_F16; p.silu_mul = epilogue == B200Q_EPI_SILU_MUL;
   p.tiles = ceil_div(n_out, pl.wt) * pl.tok_tiles;
   p.units = (long long)p.tiles * kgroups;
