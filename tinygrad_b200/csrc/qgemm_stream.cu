@@ -31,9 +31,9 @@ constexpr int THREADS = (UNPACK_WARPS + 2) * 32;
 constexpr int KSTEP = 32;                               // one quant block of K per step
 __host__ __device__ constexpr int steps_per_slot(int wt) { return wt == 128 ? 4 : 1; }
 constexpr int RING_BYTES = 224 * 1024, MAX_SLOTS = 6;   // shared memory: slots of unpacked weights + activations
-// Few activation rows (128 weight rows a tile): packed blocks wait in shared memory, one 16 / 32-byte block and its scale per unpack thread and K
-// group, up to MAX_AHEAD groups ahead.  A queue in registers that moves up by a block waits for the newest load every time: whatever its depth a
-// group took a round trip to HBM (8B gate / up, 45 rows: 83 us, 70 here; 8 rows: 79, 60).
+// Packed blocks wait in shared memory, one 16 / 32-byte block and its scale per unpack thread and round, up to MAX_AHEAD rounds ahead.  A queue in
+// registers that moves up by a block waits for the newest load every time: whatever its depth, a round took a trip to HBM (8B gate / up, 45 rows: 83 us,
+// 70 here; 8 rows: 79, 60).
 constexpr int MAX_AHEAD = 4;
 __host__ __device__ constexpr int ahead_bytes(int qt) { return UNPACK_THREADS * (qt == B200Q_Q4_0 ? 20 : 36); }
 constexpr int MAX_NT = 256;                             // activation rows per tile
@@ -299,7 +299,6 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
   // Steps per ring slot, i.e. per barrier phase.  With few activation rows a step's MMAs take less time than the barrier operations around
   // them (a ready barrier costs the MMA thread about 100 cycles, an instruction of N <= 128 72), so a slot is a whole K group there.
   constexpr int SPS = steps_per_slot(WT), W_SLOT = W_STEP * SPS;
-  constexpr int DEPTH = QT == B200Q_Q4_0 ? 4 : 3;                                             // blocks in flight per thread
   extern __shared__ __align__(128) unsigned char dyn[];
   __shared__ Shared sh;
   const uint32_t sb = pinned(s32(&sh)), ring = pinned(s32(dyn));
@@ -410,26 +409,7 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
       fp = f_row < p.n_row_tiles ? p.w + ((size_t)f_row * p.kgroups + k0) * TB : nullptr;
     };
     set_tile((int)(u0 - (long long)ft * p.kgroups));
-    auto fetch = [&](Raw<QT>& q) {
-      if (fp && f_units > 0) {
-        const int t = grp + fs * GROUPS;
-        q.d = __ldg(reinterpret_cast<const unsigned short*>(fp + in_d + (t >> 1) * 8 + (t & 1) * 2));
-        q.a = __ldg(reinterpret_cast<const uint4*>(fp + in_w + fs * GROUPS * 16));
-        if constexpr (QT == B200Q_Q8_0) q.b = __ldg(reinterpret_cast<const uint4*>(fp + in_w + fs * GROUPS * 16 + 512));
-        if (PER_UNIT == 1 || fs == PER_UNIT - 1) fp += TB;
-      } else {
-        q.a = make_uint4(0, 0, 0, 0);
-        q.d = 0;
-        if constexpr (QT == B200Q_Q8_0) q.b = make_uint4(0, 0, 0, 0);
-      }
-      if (PER_UNIT == 1 || ++fs == PER_UNIT) {
-        fs = 0; f_units--;
-        if (--f_left == 0) { ft++; f_left = p.kgroups; set_tile(0); }
-      }
-    };
-    Raw<QT> q[DEPTH];
-    // 128 weight rows: this thread's places in the waiting blocks (never read by another thread, so no barrier)
-    constexpr bool STAGED = WT == 128;
+    // this thread's places among the waiting blocks (never read by another thread, so no barrier)
     constexpr uint32_t AHEAD = ahead_bytes(QT), SCALE_AT = UNPACK_THREADS * (QT == B200Q_Q4_0 ? 16 : 32);
     const uint32_t wait0 = ring + slots * slot_bytes, wait_end = wait0 + p.ahead * AHEAD;
     uint32_t wait_at = wait0;                            // the oldest waiting block
@@ -437,14 +417,17 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
       const bool in = fp && f_units > 0;
       const uint8_t* src = in ? fp : p.w;
       const uint32_t n16 = in ? 16u : 0u, n4 = in ? 4u : 0u;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at + tid * 16), "l"(src + (in ? in_w : 0)), "r"(n16) : "memory");
+      const int w_at = in_w + fs * GROUPS * 16;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at + tid * 16), "l"(src + (in ? w_at : 0)), "r"(n16) : "memory");
       if constexpr (QT == B200Q_Q8_0)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at + UNPACK_THREADS * 16 + tid * 16), "l"(src + (in ? in_w + 512 : 0)), "r"(n16) : "memory");
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(at + SCALE_AT + tid * 4), "l"(src + (in ? in_d + (grp >> 1) * 8 : 0)), "r"(n4) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at + UNPACK_THREADS * 16 + tid * 16), "l"(src + (in ? w_at + 512 : 0)), "r"(n16) : "memory");
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(at + SCALE_AT + tid * 4), "l"(src + (in ? in_d + ((grp + fs * GROUPS) >> 1) * 8 : 0)), "r"(n4) : "memory");
       asm volatile("cp.async.commit_group;" ::: "memory");
-      if (in) fp += TB;
-      f_units--;
-      if (--f_left == 0) { ft++; f_left = p.kgroups; set_tile(0); }
+      if (PER_UNIT == 1 || ++fs == PER_UNIT) {
+        fs = 0; f_units--;
+        if (in) fp += TB;
+        if (--f_left == 0) { ft++; f_left = p.kgroups; set_tile(0); }
+      }
     };
     auto collect = [&](Raw<QT>& q) {
       switch (p.ahead) {
@@ -459,12 +442,7 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
       asm volatile("ld.shared.u32 %0, [%1];" : "=r"(d) : "r"(wait_at + SCALE_AT + tid * 4) : "memory");
       q.d = grp & 1 ? d >> 16 : d & 0xFFFFu;
     };
-    if constexpr (STAGED) {
-      for (int d = 0; d < p.ahead; d++) request(wait0 + d * AHEAD);
-    } else {
-#pragma unroll
-      for (int d = 0; d < DEPTH; d++) fetch(q[d]);
-    }
+    for (int d = 0; d < p.ahead; d++) request(wait0 + d * AHEAD);
     pdl_wait();                                          // the epilogue reads and writes what earlier kernels touched
     // One block: wait for its slot, unpack, hand over, ask for the block DEPTH further on.
     int slot = SPS > 1 ? 0 : grp;                        // ring position and its phase; SPS == 1: the thread groups take turns
@@ -472,9 +450,10 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
     constexpr int SLOT_STEP = SPS > 1 ? 1 : GROUPS;
     static_assert(SPS == 1 || (SPS == 4 && GROUPS == 4), "one block per thread and slot");
     bool ok = true;
-    auto unpack = [&](Raw<QT>& q) {
+    auto unpack = [&]() {
       ok = ok && bar_wait(sb, BAR(sb, empty) + 8 * slot, par);
-      if constexpr (STAGED) collect(q);
+      Raw<QT> q;
+      collect(q);
       const uint32_t dst = ring + slot * slot_bytes + (SPS > 1 ? grp * W_STEP : 0) + r * 16;
       const uint32_t d2 = q.d | (q.d << 16);
       uint4 hi[4], lo[4];
@@ -501,10 +480,8 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
       }
       __syncwarp();
       if (lane == 0) bar_arrive(BAR(sb, full) + 8 * slot);
-      if constexpr (STAGED) {
-        request(wait_at);
-        if ((wait_at += AHEAD) == wait_end) wait_at = wait0;
-      } else fetch(q);
+      request(wait_at);
+      if ((wait_at += AHEAD) == wait_end) wait_at = wait0;
       slot += SLOT_STEP;
       if (slot >= slots) { slot -= slots; par ^= 1; }
     };
@@ -520,19 +497,12 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
         left = (k1 - k0) * PER_UNIT;
       }
       const int lead = done_tile >= 0 ? min(left, LEAD) : left;
-      // one instance of the unpack code, the queue of fetched blocks moving up: unrolled over the queue the loop took 1.6x the cycles per
-      // block (instruction fetch)
+      // one instance of the unpack code: unrolled the loop took 1.6x the cycles per block (instruction fetch)
 #pragma unroll 1
       for (int stop = left - lead;; stop = 0) {
 #pragma unroll 1
         for (; left > stop && ok; left--) {
-          unpack(q[0]);
-          if constexpr (!STAGED) {
-            const Raw<QT> head = q[0];
-#pragma unroll
-            for (int d = 0; d + 1 < DEPTH; d++) q[d] = q[d + 1];
-            q[DEPTH - 1] = head;
-          }
+          unpack();
         }
         if (done_tile >= 0 && ok) {
           ok = finish_segment<WT, F32>(p, sh, sb, seg++, done_tile, done_k0, done_k1);
@@ -543,7 +513,7 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
       done_tile = tile; done_k0 = k0; done_k1 = k1;
       u += k1 - k0;
     }
-    if constexpr (STAGED) asm volatile("cp.async.wait_group 0;" ::: "memory");      // nothing may still be landing when the CTA leaves
+    asm volatile("cp.async.wait_group 0;" ::: "memory");      // nothing may still be landing when the CTA leaves
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -641,10 +611,12 @@ int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtyp
   p.bias = (const __half*)bias_f16; p.residual = residual; p.y = y;
   p.m = m; p.n_out = n_out; p.kgroups = kgroups; p.n_row_tiles = ceil_div(n_out, TILE_ROWS);
   p.nt = pl.nt; p.tok_tiles = pl.tok_tiles;
-  // 2 K groups, or 3 (256 rows) to 5 steps; what two K groups leave, at least one group's blocks, is for the packed blocks ahead
-  p.slots = pl.wt == 128 ? 2 : RING_BYTES / slot_bytes(pl, f32);
+  // Slots of unpacked weights and activations, 2 K groups or 3 (256 activation rows) to 5 steps; what they leave is for the packed blocks ahead:
+  // at least two groups of Q4_0 (or one of Q8_0, whose blocks are twice as large) unless even two K groups leave less.
+  const int slot = slot_bytes(pl, f32), one = ahead_bytes(qtype);
+  p.slots = pl.wt == 128 ? 2 : (RING_BYTES - (qtype == B200Q_Q4_0 ? 2 : 1) * one) / slot;
   if (p.slots > MAX_SLOTS) p.slots = MAX_SLOTS;
-  p.ahead = pl.wt == 128 ? (RING_BYTES - p.slots * slot_bytes(pl, f32)) / ahead_bytes(qtype) : 0;
+  p.ahead = (RING_BYTES - p.slots * slot) / one;
   if (p.ahead > MAX_AHEAD) p.ahead = MAX_AHEAD;
   p.y_f16 = y_dtype == B200Q_F16; p.silu_mul = epilogue == B200Q_EPI_SILU_MUL;
   p.tiles = ceil_div(n_out, pl.wt) * pl.tok_tiles;
