@@ -17,7 +17,10 @@ def _gpu(): need_gpu()
 @pytest.mark.parametrize("split", [True, False])
 @pytest.mark.parametrize("typ,m,n_out,n_in,dt", [(2, 1, 16, 32, np.float32), (8, 16, 130, 96, np.float32), (2, 17, 1000, 1184, np.float32), (8, 64, 128, 4096, np.float32),
                                                  (2, 65, 257, 4096, np.float32), (8, 128, 256, 160, np.float32), (2, 129, 300, 992, np.float32), (8, 256, 512, 512, np.float32),
-                                                 (2, 257, 130, 1408, np.float32), (2, 301, 200, 640, np.float16), (8, 64, 300, 1184, np.float16), (8, 600, 72, 96, np.float16)])
+                                                 (2, 257, 130, 1408, np.float32), (2, 301, 200, 640, np.float16), (8, 64, 300, 1184, np.float16), (8, 600, 72, 96, np.float16),
+                                                 # enough row tiles for 256 weight rows each (the others above 64 rows take 128)
+                                                 (2, 65, 19300, 96, np.float32), (8, 130, 30400, 160, np.float32), (2, 257, 15300, 96, np.float32),
+                                                 (8, 300, 15300, 96, np.float16)])
 def test_rows_against_the_exact_product(typ, m, n_out, n_in, dt, split):
   rng = np.random.default_rng(m + n_out)
   raw = synth.BLOCK_MAKERS[typ](n_out, n_in, rng)

@@ -10,10 +10,11 @@
 //  * weights are the MMA's A operand (128 rows per instruction) and the activation rows its N: any row count rounded up to 16 fills the
 //    instruction, and up to 128 rows the halves xh | xl sit side by side as ONE operand of 2 N columns (two instructions per K step
 //    instead of three);
-//  * a tile is 256 weight rows (two accumulators, the whole of tensor memory) by up to 256 activation rows: every unpacked weight meets
+//  * a tile is up to 256 weight rows (two accumulators, the whole of tensor memory) by up to 256 activation rows: every unpacked weight meets
 //    256 rows and every activation byte 256 weight rows.  With 128 x 128 tiles the activation operand alone took 2.4x the L2 traffic
-//    and every weight was unpacked once per 128 rows.  Up to 64 rows a tile is 128 weight rows (more tiles to share, smaller partial sums);
-//  * roles are separate warps: 16 unpack the weights (global -> registers, several blocks ahead -> fp16 halves in a ring of
+//    and every weight was unpacked once per 128 rows.  Up to 64 rows, and where tiles are few, a tile is 128 weight rows
+//    (more tiles to share, smaller partial sums);
+//  * roles are separate warps: 16 unpack the weights (packed blocks by asynchronous copies, several ahead -> fp16 halves in a ring of
 //    shared-memory slots), one thread brings activation tiles in by bulk copies, one issues the MMAs; nothing meets at a block barrier;
 //  * the K x tile space is dealt to one CTA per SM in equal contiguous runs (stream-K): no last wave.  A tile that spans CTAs leaves fp32
 //    partial sums in the workspace; the CTA that arrives last adds them in the order of K (bit-reproducible) and writes the result.
@@ -29,7 +30,7 @@ constexpr int UNPACK_WARPS = 16, UNPACK_THREADS = UNPACK_WARPS * 32;
 constexpr int WARP_COPY = UNPACK_WARPS, WARP_MMA = UNPACK_WARPS + 1;
 constexpr int THREADS = (UNPACK_WARPS + 2) * 32;
 constexpr int KSTEP = 32;                               // one quant block of K per step
-__host__ __device__ constexpr int steps_per_slot(int wt) { return wt == 128 ? 4 : 1; }
+constexpr int steps_per_slot(int wt, int nt) { return wt == 128 && nt <= 64 ? 4 : 1; }
 constexpr int RING_BYTES = 224 * 1024, MAX_SLOTS = 6;   // shared memory: slots of unpacked weights + activations
 // Packed blocks wait in shared memory, one 16 / 32-byte block and its scale per unpack thread and round, up to MAX_AHEAD rounds ahead.  A queue in
 // registers that moves up by a block waits for the newest load every time: whatever its depth, a round took a trip to HBM (8B gate / up, 45 rows: 83 us,
@@ -292,13 +293,13 @@ template <int QT> struct Raw;
 template <> struct Raw<B200Q_Q4_0> { uint4 a; uint32_t d; };
 template <> struct Raw<B200Q_Q8_0> { uint4 a, b; uint32_t d; };
 
-template <int QT, int WT, bool F32>
+template <int QT, int WT, bool F32, int SPS>
 __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamParams p) {
   constexpr int TB = tile_bytes(QT), GROUPS = UNPACK_THREADS / WT, PER_UNIT = 4 / GROUPS;    // thread groups, each with its own steps of a K group
   constexpr int W_HALF = WT * KSTEP * 2, W_STEP = 2 * W_HALF;
   // Steps per ring slot, i.e. per barrier phase.  With few activation rows a step's MMAs take less time than the barrier operations around
   // them (a ready barrier costs the MMA thread about 100 cycles, an instruction of N <= 128 72), so a slot is a whole K group there.
-  constexpr int SPS = steps_per_slot(WT), W_SLOT = W_STEP * SPS;
+  constexpr int W_SLOT = W_STEP * SPS;
   extern __shared__ __align__(128) unsigned char dyn[];
   __shared__ Shared sh;
   const uint32_t sb = pinned(s32(&sh)), ring = pinned(s32(dyn));
@@ -522,20 +523,23 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
 
 // ---- launch --------------------------------------------------------------------------------------------------------------------
 struct Plan { int nt, tok_tiles, wt; };
-Plan make_plan(int m) {
+Plan make_plan(int m, int n_out, int n_sm) {
   Plan pl;
   pl.tok_tiles = ceil_div(m, MAX_NT);
   pl.nt = ceil_div(ceil_div(m, pl.tok_tiles), 16) * 16;      // equal tiles: 301 rows are 2 x 160, not 256 + 45
-  pl.wt = pl.nt <= 64 ? 128 : 256;
+  // 128 weight rows a tile up to 64 activation rows, and where tiles of 256 are too few for the SMs: each is then split over several CTAs, the one
+  // that arrives last adds all parts alone, and halving the tile quarters what it reads.  8B QKV (24 tiles), 256 rows: 75 -> 49 us, down (16)
+  // 117 -> 83; gate/up (112) 154 -> 142, but 79 -> 83 at 80 rows; 7B gate/up (148 tiles, hardly split) 142 -> 146.
+  pl.wt = pl.nt <= 64 || (n_out > 0 && (pl.nt > 96 ? 5LL : 8LL) * ceil_div(n_out, 256) * pl.tok_tiles <= 4LL * n_sm) ? 128 : 256;
   return pl;
 }
 size_t tiles_bytes(const Plan& pl, int kgroups, bool f32) { return (size_t)pl.tok_tiles * pl.nt * kgroups * GROUP_ELEMS * (f32 ? 4 : 2); }
-int slot_bytes(const Plan& pl, bool f32) { return steps_per_slot(pl.wt) * (pl.wt * KSTEP * 4 + pl.nt * (f32 ? 128 : 64)); }
+int slot_bytes(const Plan& pl, bool f32) { return steps_per_slot(pl.wt, pl.nt) * (pl.wt * KSTEP * 4 + pl.nt * (f32 ? 128 : 64)); }
 size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
 
-template <int QT, int WT, bool F32>
+template <int QT, int WT, bool F32, int SPS>
 int launch_stream(const StreamParams& p, int grid, cudaStream_t st) {
-  auto kern = qgemm_stream_kernel<QT, WT, F32>;
+  auto kern = qgemm_stream_kernel<QT, WT, F32, SPS>;
   static PerDeviceFlag attr;
   const int dev = b200q_current_device();
   if (dev < 0) return B200Q_ERR_CUDA;
@@ -581,7 +585,7 @@ extern "C" size_t b200q_qgemm_workspace_bytes(int m, int n_in) {
 extern "C" size_t b200q_qgemm_workspace_bytes_for(int m, int n_out, int n_in) {
   if (m <= 0 || n_in <= 0 || n_out < 0) return 0;
   const int n_sm = b200q_sm_count();
-  return align256(b200q_qgemm_workspace_bytes(m, n_in)) + split_workspace(make_plan(m), n_out, ceil_div(n_in, GROUP_ELEMS), n_sm > 0 ? n_sm : 148);
+  return align256(b200q_qgemm_workspace_bytes(m, n_in)) + split_workspace(make_plan(m, n_out, n_sm > 0 ? n_sm : 148), n_out, ceil_div(n_in, GROUP_ELEMS), n_sm > 0 ? n_sm : 148);
 }
 
 // norm_weight (fp16 [n_in], fp32 activations only): the RMSNorm in front of the Linear, applied while the rows are split.
@@ -596,13 +600,13 @@ int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtyp
   if (norm_weight && x_dtype != B200Q_F32) return B200Q_ERR_BAD_ARG;
   if (n_in % 32) return B200Q_ERR_BAD_SHAPE;
   if (((uintptr_t)w_packed | (uintptr_t)x | (uintptr_t)workspace | (uintptr_t)norm_weight) & 15) return B200Q_ERR_MISALIGNED;
-  const Plan pl = make_plan(m);
+  const int n_sm = b200q_sm_count();
+  if (n_sm <= 0) return B200Q_ERR_CUDA;
+  const Plan pl = make_plan(m, n_out, n_sm);
   const bool f32 = x_dtype == B200Q_F32;
   const int kgroups = ceil_div(n_in, GROUP_ELEMS);
   const size_t xt_bytes = align256(tiles_bytes(pl, kgroups, f32));
   if (workspace_bytes < tiles_bytes(pl, kgroups, f32)) return B200Q_ERR_TOO_LARGE;
-  const int n_sm = b200q_sm_count();
-  if (n_sm <= 0) return B200Q_ERR_CUDA;
   StreamParams p;
   p.w = (const uint8_t*)w_packed;
   p.xt = (const unsigned char*)workspace;
@@ -614,7 +618,7 @@ int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtyp
   // Slots of unpacked weights and activations, 2 K groups or 3 (256 activation rows) to 5 steps; what they leave is for the packed blocks ahead:
   // at least two groups of Q4_0 (or one of Q8_0, whose blocks are twice as large) unless even two K groups leave less.
   const int slot = slot_bytes(pl, f32), one = ahead_bytes(qtype);
-  p.slots = pl.wt == 128 ? 2 : (RING_BYTES - (qtype == B200Q_Q4_0 ? 2 : 1) * one) / slot;
+  p.slots = steps_per_slot(pl.wt, pl.nt) == 4 ? 2 : (RING_BYTES - (qtype == B200Q_Q4_0 ? 2 : 1) * one) / slot;
   if (p.slots > MAX_SLOTS) p.slots = MAX_SLOTS;
   p.ahead = (RING_BYTES - p.slots * slot) / one;
   if (p.ahead > MAX_AHEAD) p.ahead = MAX_AHEAD;
@@ -632,8 +636,9 @@ int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtyp
                                      n_in, kgroups, pl.nt, per, (unsigned char*)p.xt, p.counters, split ? grid : 0));
   else B200Q_CHECK_CUDA(launch_k(split_rows_kernel<__half>, sgrid, dim3(SPLIT_THREADS), 0, st, pdl, (const __half*)x, (const __half*)nullptr, 0.f, m, n_in,
                                  kgroups, pl.nt, per, (unsigned char*)p.xt, p.counters, split ? grid : 0));
-#define STREAM_CASE(QT) (pl.wt == 256 ? (f32 ? launch_stream<QT, 256, true>(p, grid, st) : launch_stream<QT, 256, false>(p, grid, st)) \
-                                      : (f32 ? launch_stream<QT, 128, true>(p, grid, st) : launch_stream<QT, 128, false>(p, grid, st)))
+#define STREAM_CASE(QT) (pl.wt == 256 ? (f32 ? launch_stream<QT, 256, true, 1>(p, grid, st) : launch_stream<QT, 256, false, 1>(p, grid, st)) \
+                         : pl.nt > 64 ? (f32 ? launch_stream<QT, 128, true, 1>(p, grid, st) : launch_stream<QT, 128, false, 1>(p, grid, st)) \
+                                      : (f32 ? launch_stream<QT, 128, true, 4>(p, grid, st) : launch_stream<QT, 128, false, 4>(p, grid, st)))
   return qtype == B200Q_Q4_0 ? STREAM_CASE(B200Q_Q4_0) : STREAM_CASE(B200Q_Q8_0);
 #undef STREAM_CASE
 }
