@@ -600,13 +600,14 @@ int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtyp
   if (norm_weight && x_dtype != B200Q_F32) return B200Q_ERR_BAD_ARG;
   if (n_in % 32) return B200Q_ERR_BAD_SHAPE;
   if (((uintptr_t)w_packed | (uintptr_t)x | (uintptr_t)workspace | (uintptr_t)norm_weight) & 15) return B200Q_ERR_MISALIGNED;
-  const int n_sm = b200q_sm_count();
-  if (n_sm <= 0) return B200Q_ERR_CUDA;
-  const Plan pl = make_plan(m, n_out, n_sm);
+  Plan pl = make_plan(m, 0, 0);                                // the activations' tiling does not depend on the device
   const bool f32 = x_dtype == B200Q_F32;
   const int kgroups = ceil_div(n_in, GROUP_ELEMS);
   const size_t xt_bytes = align256(tiles_bytes(pl, kgroups, f32));
   if (workspace_bytes < tiles_bytes(pl, kgroups, f32)) return B200Q_ERR_TOO_LARGE;
+  const int n_sm = b200q_sm_count();
+  if (n_sm <= 0) return B200Q_ERR_CUDA;
+  pl = make_plan(m, n_out, n_sm);
   StreamParams p;
   p.w = (const uint8_t*)w_packed;
   p.xt = (const unsigned char*)workspace;
