@@ -62,7 +62,7 @@ __device__ __forceinline__ void quant_block_8x4(float4 v, int q, int b, const Xq
   if (q == 0) xq_store_scales(d, b, s, qsum);
 }
 
-// The same for a block held by 4 consecutive lanes, 8 values each (q = lane & 3 gives elements 8q..8q+7): 9 instructions per value against 37 of
+// The same for a block held by 4 consecutive lanes, 8 values each (q = lane & 3 gives elements 8q..8q+7): half the instructions per value of
 // the form above (two divisions, six shuffles and unpacked digit arithmetic per 4 values).  Every GEMV CTA quantises the whole row, so this
 // sits between the arrival of the row and its first tile: 14336 values by 512 threads 4.6 -> 1.9 us with the loads.
 __device__ __forceinline__ uint32_t pack_bytes(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t sel) {      // byte `sel` & 7 of each
@@ -79,8 +79,10 @@ __device__ __forceinline__ void quant_block_4x8(const float (&v)[8], int q, int 
   for (int i = 0; i < 8; i++) amax = fmaxf(amax, fabsf(v[i]));
   amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
   amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-  const bool live = amax > 1e-30f && amax < INFINITY;
-  const float inv = live ? __fdividef(XQ_RANGE, amax) : 0.f, s = live ? amax * (1.f / XQ_RANGE) : 0.f;
+  // The quotients of the forms above and below: with approximate ones some codes come out one off, and none above 2^126 at all.  The one by a constant is the
+  // product with its reciprocal and one fused residual step, correctly rounded wherever it is a normal number (Markstein; every fraction checked).
+  const bool live = amax > 0.f && amax < INFINITY;
+  const float inv = live ? XQ_RANGE / amax : 0.f, s0 = amax * (1.f / XQ_RANGE), s = live ? fmaf(fmaf(-s0, XQ_RANGE, amax), 1.f / XQ_RANGE, s0) : 0.f;
   int i[8], qsum = 0;
 #pragma unroll
   for (int k = 0; k < 8; k++) { i[k] = __float2int_rn(v[k] * inv); qsum += i[k]; }
