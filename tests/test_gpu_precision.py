@@ -1,7 +1,8 @@
 """What the kernels lose against exact arithmetic, held to what 32-bit arithmetic gives."""
+import ctypes
 import numpy as np
 import pytest
-from tinygrad_b200 import quant
+from tinygrad_b200 import _lib, quant
 from tinygrad_b200.runtime import DeviceBuffer
 from gpu_util import need_gpu
 
@@ -29,3 +30,26 @@ def test_activation_codes_are_the_rounded_quotients():
   codes = np.rint(blocks * (np.float32(16256) / amax))
   got = np.rint(y.numpy().reshape(blocks.shape).astype(np.float64) / (amax / np.float32(16256)).astype(np.float64))
   np.testing.assert_array_equal(got, codes)
+
+
+@pytest.mark.parametrize("kv", [np.float16, np.float32])
+@pytest.mark.parametrize("n_heads,n_kv,hd", [(8, 2, 128), (8, 2, 64)])
+def test_decode_attention_rounds_to_nearest(n_heads, n_kv, hd, kv):
+  """Far into a context, where a tensor core that truncates its running sums (always towards zero) is 4.6e-7 (fp16 cache) to 2.4e-6 (fp32 cache) off.  Sums
+  rounded to nearest add up like a random walk: 55 chunks, 8 partial sums a score and 4 or 8 a chunk stay within 6 x 2^-24 of the output's norm."""
+  rng = np.random.default_rng(hd)
+  pos, ctx, lib = 3507, 3520, _lib.load()
+  qkv = rng.standard_normal((n_heads + 2 * n_kv, hd)).astype(np.float32)
+  kc, vc = (rng.standard_normal((n_kv, ctx, hd)).astype(kv) for _ in range(2))
+  rope = np.concatenate([np.ones((ctx, hd // 2)), np.zeros((ctx, hd // 2))], 1).astype(np.float32)
+  q, k, v = (a.astype(np.float64) for a in (qkv[:n_heads], qkv[n_heads:n_heads + n_kv].astype(kv), qkv[n_heads + n_kv:].astype(kv)))
+  rep = lambda c, new: np.repeat(np.concatenate([c[:, :pos].astype(np.float64), new[:, None]], 1), n_heads // n_kv, 0)
+  s = np.einsum("hd,hpd->hp", q, rep(kc, k)) / np.sqrt(hd)
+  p = np.exp(s - s.max(-1, keepdims=True))
+  want = np.einsum("hp,hpd->hd", p / p.sum(-1, keepdims=True), rep(vc, v))
+  d = [DeviceBuffer.from_numpy(a) for a in (qkv, kc, vc, rope, np.array([pos], np.int32))]
+  out, n_split = DeviceBuffer.empty((n_heads, hd), np.float32), lib.b200q_attn_min_split(ctx)
+  scratch = DeviceBuffer(lib.b200q_attn_scratch_bytes(n_heads, n_kv, hd, n_split), zero=True)
+  a = _lib.AttnArgs(d[0].ptr, d[1].ptr, d[2].ptr, _lib.F16 if kv == np.float16 else _lib.F32, d[3].ptr, d[4].ptr, out.ptr, scratch.ptr, n_heads, n_kv, hd, hd, ctx, n_split, 0, None)
+  _lib.check(lib.b200q_attn_decode(ctypes.byref(a), None))
+  assert np.linalg.norm(out.numpy() - want) <= 6 * 2.0 ** -24 * np.linalg.norm(want)
