@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
       const bool second = QT == K_MIX && rt >= p.tiles_first;
       const int TB = QT == K_MIX ? tile_bytes(second ? B200Q_Q6_K_WIDE : B200Q_Q4_K_WIDE) : tile_bytes(QT);
       float acc0 = 0.f, acc1 = 0.f;
-      [[maybe_unused]] float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
+      [[maybe_unused]] float c[4] = {0.f, 0.f, 0.f, 0.f};
       for (int s = 0; s < stages_per_tile; s++, it++) {
         const int slot = it % NS, groups = min(SG, p.kgroups - s * SG);
         if (!mbar_wait(full0 + 8 * slot, (it / NS) & 1)) { *s_abort = 1; break; }
@@ -460,8 +460,8 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
             const int j = s * SG + gi;
             if constexpr (WIDE) {
               const uint4* xb = xq + j * 32 + (g & 1) * 4 + t;
-              if (QT == B200Q_Q4_K_WIDE || (QT == K_MIX && !second)) tile_mac_q4k(stage + gi * TB, lane, xb, c0, c1);
-              else tile_mac_q6k_wide(stage + gi * TB, lane, xb, c0, c1);
+              if (QT == B200Q_Q4_K_WIDE || (QT == K_MIX && !second)) tile_mac_q4k(stage + gi * TB, lane, xb, c);
+              else tile_mac_q6k_wide(stage + gi * TB, lane, xb, c);
             } else {
               const float4 st = xsc[(j * 2 + (t >> 1)) * 2 + (t & 1)];
               // the address is selected, not the loaded value: `diag ? xq[..] : *zero` compiled to a divergent branch around the loads
@@ -484,8 +484,8 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
       }
       PSTAMP(4);
       if constexpr (WIDE) {      // even columns: high parts, odd: remainders x 2^11
-        acc0 = fmaf(c0[1] + c1[1], 1.f / 2048.f, c0[0] + c1[0]) * x_down;
-        acc1 = fmaf(c0[3] + c1[3], 1.f / 2048.f, c0[2] + c1[2]) * x_down;
+        acc0 = fmaf(c[1], 1.f / 2048.f, c[0]) * x_down;
+        acc1 = fmaf(c[3], 1.f / 2048.f, c[2]) * x_down;
       } else {
         // quad lanes hold the columns {blocks 0,1 hi}, {2,3 hi}, {0,1 lo}, {2,3 lo}: add them
         acc0 += __shfl_xor_sync(0xffffffffu, acc0, 1); acc0 += __shfl_xor_sync(0xffffffffu, acc0, 2);

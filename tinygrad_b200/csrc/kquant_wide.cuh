@@ -9,8 +9,12 @@
 // shifts unpack two quants, two conversions and one packed FMA scale them exactly as fp32 would, one conversion rounds the pair to fp16.
 // What bounds it is that dequantisation: 64 conversions and 32 packed FMAs on one pipe, 72 masks, shifts and roundings on another per tile, each
 // good for an instruction every other cycle.  Gate and up of 14336 x 4096 in Q4_K 26.3 us (2.66 TB/s of packed weights; as fp16
-// these are 235 MB, 36 us at HBM rate), down 4096 x 14336 in Q6_K 19.7 us; a step of six 8B-shaped blocks 1005 us on fp16 weights, 505 us here.  Scalar FMAs: 27.0 us.  The mixed-precision FMA on scale * q
+// these are 235 MB, 36 us at HBM rate), down 4096 x 14336 in Q6_K 19.7 us; a step of six 8B-shaped blocks 1005 us on fp16 weights, 510 us here.  Scalar FMAs: 27.0 us.  The mixed-precision FMA on scale * q
 // (exact in fp16), which needs no conversions: 30.1 us.
+//
+// Sums: the tensor core truncates, always towards zero, when it adds to an accumulator, so the high parts' products of two MMAs at a time are added here,
+// rounded to nearest.  Error of 4096 x 14336 outputs against 64 bits 1.5e-7, as in fp32 sums on the dense form; with accumulators that run through the MMAs 5.5e-7
+// (and 486 us a step).  One MMA at a time is no closer and spills (555 us).
 //
 // Record of an activation row (kgroups = n_in / 128): uint4 xh[kgroups][4][8], entry w, column c = block (high parts) or 4 + block (remainders):
 // {x[4w], x[4w+2]} {x[4w+1], x[4w+3]} and the same of elements 16 + 4w ..; the row is scaled by a power of two that puts its largest value into
@@ -77,7 +81,7 @@ constexpr float SUB0 = 16777216.f, SUB4 = 1048576.f;      // 2^24, 2^20: what qu
 // One Q4_K tile, 1216 bytes: uint4 L[2][32] quants (lane (g, t) of half h: row 8h + g, block t; byte i = element i | element i + 16 << 4),
 // uint8 SM[16][4][2] {scale, minimum} of each block, half2 D[16] {d, dmin}.  Weight = d * scale * q - dmin * minimum (tinygrad/llm/gguf.py:57-67).
 // xb: the lane's column and block of the group's xh entries, 8 entries apart.
-__device__ __forceinline__ void tile_mac_q4k(const uint8_t* tile, int lane, const uint4* xb, float (&c0)[4], float (&c1)[4]) {
+__device__ __forceinline__ void tile_mac_q4k(const uint8_t* tile, int lane, const uint4* xb, float (&c)[4]) {
   const uint4* lp = reinterpret_cast<const uint4*>(tile);
   const uint4 r0 = lp[lane], r1 = lp[32 + lane];      // rows g and g + 8
   const int g = lane >> 2;
@@ -92,13 +96,15 @@ __device__ __forceinline__ void tile_mac_q4k(const uint8_t* tile, int lane, cons
   for (int w = 0; w < 4; w++) {
     const uint4 x = xb[w * 8];
     const uint32_t u0 = w0[w] >> 8, u1 = w1[w] >> 8;
-    hmma(c0, lo0(w0[w] & LO), lo1(w1[w] & LO), lo0(u0 & LO), lo1(u1 & LO), x.x, x.y);
-    hmma(c1, hi0(w0[w] & HI), hi1(w1[w] & HI), hi0(u0 & HI), hi1(u1 & HI), x.z, x.w);
+    float p[4] = {0.f, c[1], 0.f, c[3]};
+    hmma(p, lo0(w0[w] & LO), lo1(w1[w] & LO), lo0(u0 & LO), lo1(u1 & LO), x.x, x.y);
+    hmma(p, hi0(w0[w] & HI), hi1(w1[w] & HI), hi0(u0 & HI), hi1(u1 & HI), x.z, x.w);
+    c[0] += p[0]; c[1] = p[1]; c[2] += p[2]; c[3] = p[3];
   }
 }
 
 // One Q6_K tile in the layout of tile_mac_q6k: weight = d * scale * (q - 32).
-__device__ __forceinline__ void tile_mac_q6k_wide(const uint8_t* tile, int lane, const uint4* xb, float (&c0)[4], float (&c1)[4]) {
+__device__ __forceinline__ void tile_mac_q6k_wide(const uint8_t* tile, int lane, const uint4* xb, float (&c)[4]) {
   const uint4* lp = reinterpret_cast<const uint4*>(tile);
   const uint2* hp = reinterpret_cast<const uint2*>(tile + 1024);
   const uint4 r0 = lp[lane], r1 = lp[32 + lane];      // rows g and g + 8
@@ -117,10 +123,12 @@ __device__ __forceinline__ void tile_mac_q6k_wide(const uint8_t* tile, int lane,
   for (int w = 0; w < 4; w++) {
     const uint4 x = xb[w * 8];
     const uint32_t u0 = w0[w] >> 8, u1 = w1[w] >> 8;
-    hmma(c0, lo0((w0[w] & LO) | (sh(h0.x, 4 - 2 * w) & LO2)), lo1((w1[w] & LO) | (sh(h1.x, 4 - 2 * w) & LO2)),
+    float p[4] = {0.f, c[1], 0.f, c[3]};
+    hmma(p, lo0((w0[w] & LO) | (sh(h0.x, 4 - 2 * w) & LO2)), lo1((w1[w] & LO) | (sh(h1.x, 4 - 2 * w) & LO2)),
          lo0((u0 & LO) | (sh(h0.x, -4 - 2 * w) & LO2)), lo1((u1 & LO) | (sh(h1.x, -4 - 2 * w) & LO2)), x.x, x.y);
-    hmma(c1, hi0((w0[w] & HI) | (sh(h0.y, 8 - 2 * w) & HI2)), hi1((w1[w] & HI) | (sh(h1.y, 8 - 2 * w) & HI2)),
+    hmma(p, hi0((w0[w] & HI) | (sh(h0.y, 8 - 2 * w) & HI2)), hi1((w1[w] & HI) | (sh(h1.y, 8 - 2 * w) & HI2)),
          hi0((u0 & HI) | (sh(h0.y, -2 * w) & HI2)), hi1((u1 & HI) | (sh(h1.y, -2 * w) & HI2)), x.z, x.w);
+    c[0] += p[0]; c[1] = p[1]; c[2] += p[2]; c[3] = p[3];
   }
 }
 
