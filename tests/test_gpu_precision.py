@@ -72,3 +72,46 @@ def test_kquant_gemv_is_as_exact_as_the_dense_one(typ):
     quant.gemv_dense(w, _lib.F16, n_out, n_in, dx, z)
     err += [np.linalg.norm(b.numpy() - want) / np.linalg.norm(want) for b in (y, z)]
   assert err[0] <= 1.25 * err[1], err
+
+
+def prompt_attention(q, k, v, kv, hd):
+  """b200q_attn_prefill on rows [T, heads, hd] without rotation, and the exact result."""
+  (T, H, _), K = q.shape, k.shape[1]
+  ctx, lib = -(-T // 64) * 64, _lib.load()
+  rope = np.concatenate([np.ones((ctx, hd // 2)), np.zeros((ctx, hd // 2))], 1).astype(np.float32)
+  d = [DeviceBuffer.from_numpy(a) for a in (np.concatenate([q, k, v], 1).astype(np.float32), rope)]
+  kc, vc = (DeviceBuffer.empty((K, ctx, hd), kv, zero=True) for _ in range(2))
+  qs, out = DeviceBuffer.empty((T, H * hd), np.float32), DeviceBuffer.empty((T, H, hd), np.float32)
+  _lib.check(lib.b200q_attn_prefill(d[0].ptr, kc.ptr, vc.ptr, _lib.F16 if kv == np.float16 else _lib.F32, d[1].ptr, 0, T, H, K, hd, hd, ctx, qs.ptr, out.ptr, _lib.F32, None))
+  q64, k64, v64 = q.astype(np.float64), *(np.repeat(a.astype(kv).astype(np.float64), H // K, 1) for a in (k, v))
+  s = np.einsum("thd,shd->hts", q64, k64) / np.sqrt(hd)
+  s[:, np.triu(np.ones((T, T), bool), 1)] = -np.inf
+  p = np.exp(s - s.max(-1, keepdims=True))
+  return out.numpy(), np.einsum("hts,shd->thd", p / p.sum(-1, keepdims=True), v64)
+
+
+@pytest.mark.parametrize("hd", [16, 32, 64, 128])
+@pytest.mark.parametrize("T", [1, 17, 64, 201])
+def test_prompt_attention_keeps_an_fp32_cache(hd, T):
+  """Keys and values of an fp32 cache are not rounded on the way to the tensor cores (4e-4 when they were, as fp16): the one-token kernel's bound.  Rows of
+  any magnitude, among them values beyond fp16's range and a query that only one row's values reach."""
+  rng = np.random.default_rng(hd + T)
+  q, k, v = (rng.standard_normal((T, n, hd)).astype(np.float32) for n in (4, 2, 2))
+  got, want = prompt_attention(q, k, v, np.float32, hd)
+  assert np.linalg.norm(got - want) <= 6 * 2.0 ** -24 * np.linalg.norm(want)
+  # keys times queries of any magnitude give the same scores; a value row's magnitude shows in the rows that attend to it
+  e = rng.integers(-60, 61, (2, 1, 1, 1)).astype(np.float32)
+  big, size = prompt_attention(q * 2.0 ** e[0], k * 2.0 ** -e[0], v * np.float32(1e6), np.float32, hd), np.float32(1e6)
+  assert np.linalg.norm(big[0] / size - want) <= 8 * 2.0 ** -24 * np.linalg.norm(want)
+  mag = (10.0 ** rng.uniform(-6, 6, (T, 2, 1))).astype(np.float32)
+  got, want = prompt_attention(q, k, v * mag, np.float32, hd)
+  # each output against what its own sum is made of: |p v| summed
+  reach = prompt_attention(q, k, np.abs(v * mag), np.float32, hd)[1]
+  assert (np.abs(got - want) <= 2.0 ** -18 * reach).all()
+
+
+def test_prompt_attention_takes_queries_of_any_magnitude():
+  rng = np.random.default_rng(3)
+  q, k, v = (rng.standard_normal((70, n, 64)).astype(np.float32) for n in (4, 2, 2))
+  got, want = prompt_attention(q * np.float32(2.0 ** 17), k * np.float32(2.0 ** -12), v, np.float16, 64)       # queries past 65504
+  assert np.isfinite(got).all() and np.linalg.norm(got - want) <= 2.0 ** -18 * np.linalg.norm(want)

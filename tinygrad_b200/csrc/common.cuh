@@ -110,6 +110,15 @@ __device__ __forceinline__ bool elect_one() {
 // Ask for a line that will be read behind pdl_wait (weights, tables): in a model whose weights exceed L2 it is a DRAM miss by then.
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
+// The power of two that puts a largest magnitude into [2^13, 2^14), where fp16 holds a value and the remainder's rounding to 2^-22 of it and to 2^-38 of
+// the largest, and its inverse; zeros get the inverse 0, infinities (and NaN) are left as they are.
+__device__ __forceinline__ void pow2_scale(float amax, float& up, float& down) {
+  const int e = max((int)(__float_as_uint(amax) >> 23) - 127, -100);
+  const bool live = amax > 0.f && amax < INFINITY;
+  up = live ? __uint_as_float((uint32_t)(13 - e + 127) << 23) : 1.f;
+  down = live ? __uint_as_float((uint32_t)(e - 13 + 127) << 23) : amax > 0.f ? 1.f : 0.f;
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -101,7 +101,12 @@ __global__ void rope_kv_rows_kernel(const float* __restrict__ qkv, const float* 
 
 // ---------------------------------------------------------------------------
 // causal attention of T queries (positions start_pos .. start_pos+T-1) over cache rows 0 .. start_pos+T-1.
-// grid (n_heads, ceil(T / 64)); 4 warps, 16 query rows each; key chunks of 64 staged in shared memory as fp16.
+// grid (n_heads, ceil(T / 64)); 4 warps, 16 query rows each; key chunks of 64 staged in shared memory as fp16, those of fp32 caches as two halves.
+// Only the cache dtype rounds, as in the one-token kernel: queries and probabilities are two halves as well.  A row of fp32 values is scaled by a power of
+// two that puts its largest into [2^13, 2^14), which is undone in the scores (queries, keys) or in the probabilities (values), so that neither large nor
+// small rows leave fp16's range.  fp32 caches take three products instead of two, and their sums are added outside the tensor core, which
+// truncates: error of the output's norm against 64 bits, 37 / 300 positions, 2.2e-7 / 3.2e-7; with
+// keys and values rounded to one fp16, 4e-4.
 constexpr int PQ = 64, PK = 64, PF_THREADS = 128;
 
 __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -111,6 +116,40 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
 __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
   const __half2 h = __floats2half2_rn(a, b);
   return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// a pair of values as fp16 high parts and what their rounding left
+__device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& lo) {
+  const __half2 h2 = __floats2half2_rn(a, b);
+  const float2 back = __half22float2(h2);
+  hi = *reinterpret_cast<const uint32_t*>(&h2);
+  lo = pack_h2(a - back.x, b - back.y);
+}
+__device__ __forceinline__ void load8f(const float* p, float (&f)[8]) {
+  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+  f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+}
+// Eight values of a row held by HD / 8 consecutive lanes (whole warps take part) -> fp16 halves of the scaled row; returns the power of two that undoes the
+// scaling, 0 for a row of zeros.
+template <int HD>
+__device__ __forceinline__ float stage_row(const float (&f)[8], __half* hi, __half* lo) {
+  float amax = 0.f, up, down;
+#pragma unroll
+  for (int j = 0; j < 8; j++) amax = fmaxf(amax, fabsf(f[j]));
+#pragma unroll
+  for (int o = 1; o < HD / 8; o *= 2) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  pow2_scale(amax, up, down);
+  uint32_t h[4], l[4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) split_pair(f[2 * j] * up, f[2 * j + 1] * up, h[j], l[j]);
+  *reinterpret_cast<uint4*>(hi) = make_uint4(h[0], h[1], h[2], h[3]);
+  *reinterpret_cast<uint4*>(lo) = make_uint4(l[0], l[1], l[2], l[3]);
+  return down;
+}
+// four 8x8 blocks, transposed: rows {0..7, 8..15} x columns {0..7, 8..15}; lane l supplies the row address of block l / 8
+__device__ __forceinline__ void ldsm4_trans(uint32_t (&r)[4], const __half* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)));
 }
 
 template <int HD, typename KV, typename O>
@@ -125,6 +164,10 @@ __global__ void __launch_bounds__(PF_THREADS) attn_prefill_kernel(const float* _
   __half* s_q = reinterpret_cast<__half*>(psm);          // [2][PQ][STRIDE]: fp16 high and low halves of the fp32 queries
   __half* s_k = s_q + 2 * PQ * STRIDE;                   // [PK][STRIDE]
   __half* s_v = s_k + PK * STRIDE;                       // [PK][STRIDE]
+  constexpr bool F32 = sizeof(KV) == 4;
+  [[maybe_unused]] __half* s_kl = s_v + PK * STRIDE;     // fp32 caches: what the rounding to fp16 left, [PK][STRIDE] each
+  [[maybe_unused]] __half* s_vl = s_kl + PK * STRIDE;
+  __shared__ float s_qd[PQ], s_kd[PK], s_vd[PK];         // powers of two that undo the rows' scaling (s_kd, s_vd: fp32 caches)
   // n_rows new tokens of each of gridDim.z sequences, all from start_pos on; one row per sequence (decode): warp 0 works, the others stage
   const int head = blockIdx.x, q0 = blockIdx.y * PQ, seq = blockIdx.z, kvh = head / (n_heads / n_kv);
   const bool single = n_rows == 1;
@@ -140,23 +183,10 @@ __global__ void __launch_bounds__(PF_THREADS) attn_prefill_kernel(const float* _
   const int q_rows = single ? 16 : PQ;                   // single: only warp 0's 16 rows are read (one of them live)
   for (int i = tid; i < q_rows * (HD / 8); i += PF_THREADS) {
     const int r = i / (HD / 8), c = (i - r * (HD / 8)) * 8;
-    uint4 hi4 = make_uint4(0, 0, 0, 0), lo4 = make_uint4(0, 0, 0, 0);
-    if (q0 + r < rows_end) {
-      const float* src = q + ((size_t)(q0 + r) * n_heads + head) * HD + c;
-      const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
-      const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-      uint32_t hw[4], lw[4];
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const __half2 h2 = __floats2half2_rn(f[2 * j], f[2 * j + 1]);
-        const float2 back = __half22float2(h2);
-        hw[j] = *reinterpret_cast<const uint32_t*>(&h2);
-        lw[j] = pack_h2(f[2 * j] - back.x, f[2 * j + 1] - back.y);
-      }
-      hi4 = make_uint4(hw[0], hw[1], hw[2], hw[3]); lo4 = make_uint4(lw[0], lw[1], lw[2], lw[3]);
-    }
-    *reinterpret_cast<uint4*>(s_q + r * STRIDE + c) = hi4;
-    *reinterpret_cast<uint4*>(s_q + (PQ + r) * STRIDE + c) = lo4;
+    float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (q0 + r < rows_end) load8f(q + ((size_t)(q0 + r) * n_heads + head) * HD + c, f);
+    const float down = stage_row<HD>(f, s_q + r * STRIDE + c, s_q + (PQ + r) * STRIDE + c);
+    if (c == 0) s_qd[r] = down;
   }
   __syncthreads();
   // q = hi + lo (both fp16): the scores keep the fp32 query's precision, as the one-token kernel's fp32 dot products do
@@ -183,25 +213,29 @@ __global__ void __launch_bounds__(PF_THREADS) attn_prefill_kernel(const float* _
   const int qpos0 = pos0 + warp * 16 + g, qpos1 = qpos0 + 8;                // positions of this lane's two rows
   const int n_keys = pos0 + min(rows_end - q0, PQ);                          // keys any row of the tile may see
   const float scale = 1.0f / sqrtf((float)HD);
+  const float qd0 = scale * s_qd[(single ? 0 : warp * 16) + g], qd1 = scale * s_qd[(single ? 0 : warp * 16) + g + 8];
 
   for (int k0 = 0; k0 < n_keys; k0 += PK) {
     __syncthreads();                                     // the previous chunk has been consumed
     for (int i = tid; i < PK * (HD / 8); i += PF_THREADS) {
       const int r = i / (HD / 8), c = (i - r * (HD / 8)) * 8;
-      uint4 kk4 = make_uint4(0, 0, 0, 0), vv4 = make_uint4(0, 0, 0, 0);
-      if (k0 + r < n_keys) {
-        if constexpr (sizeof(KV) == 2) {
+      if constexpr (F32) {
+        float fk[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, fv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (k0 + r < n_keys) {
+          load8f(kc + (size_t)(k0 + r) * HD + c, fk);
+          load8f(vc + (size_t)(k0 + r) * HD + c, fv);
+        }
+        const float kd = stage_row<HD>(fk, s_k + r * STRIDE + c, s_kl + r * STRIDE + c), vd = stage_row<HD>(fv, s_v + r * STRIDE + c, s_vl + r * STRIDE + c);
+        if (c == 0) { s_kd[r] = kd; s_vd[r] = vd; }
+      } else {
+        uint4 kk4 = make_uint4(0, 0, 0, 0), vv4 = make_uint4(0, 0, 0, 0);
+        if (k0 + r < n_keys) {
           kk4 = *reinterpret_cast<const uint4*>(kc + (size_t)(k0 + r) * HD + c);
           vv4 = *reinterpret_cast<const uint4*>(vc + (size_t)(k0 + r) * HD + c);
-        } else {
-          const float4 a = *reinterpret_cast<const float4*>(kc + (size_t)(k0 + r) * HD + c), b = *reinterpret_cast<const float4*>(kc + (size_t)(k0 + r) * HD + c + 4);
-          const float4 e = *reinterpret_cast<const float4*>(vc + (size_t)(k0 + r) * HD + c), f = *reinterpret_cast<const float4*>(vc + (size_t)(k0 + r) * HD + c + 4);
-          kk4 = make_uint4(pack_h2(a.x, a.y), pack_h2(a.z, a.w), pack_h2(b.x, b.y), pack_h2(b.z, b.w));
-          vv4 = make_uint4(pack_h2(e.x, e.y), pack_h2(e.z, e.w), pack_h2(f.x, f.y), pack_h2(f.z, f.w));
         }
+        *reinterpret_cast<uint4*>(s_k + r * STRIDE + c) = kk4;
+        *reinterpret_cast<uint4*>(s_v + r * STRIDE + c) = vv4;
       }
-      *reinterpret_cast<uint4*>(s_k + r * STRIDE + c) = kk4;
-      *reinterpret_cast<uint4*>(s_v + r * STRIDE + c) = vv4;
     }
     __syncthreads();
     if (k0 > pos0 + warp * 16 + 15) continue;  // every key of the chunk is after this warp's last query
@@ -215,8 +249,22 @@ __global__ void __launch_bounds__(PF_THREADS) attn_prefill_kernel(const float* _
 #pragma unroll
       for (int kk = 0; kk < HD / 16; kk++) {
         const uint32_t b0 = *reinterpret_cast<const uint32_t*>(kr + kk * 16), b1 = *reinterpret_cast<const uint32_t*>(kr + kk * 16 + 8);
-        mma16816(s[j], qa[kk], b0, b1);
-        mma16816(s[j], ql[kk], b0, b1);
+        if constexpr (F32) {
+          const __half* kl = kr + (s_kl - s_k);
+          float p[4] = {0.f, 0.f, 0.f, 0.f};
+          mma16816(p, ql[kk], b0, b1);
+          mma16816(p, qa[kk], *reinterpret_cast<const uint32_t*>(kl + kk * 16), *reinterpret_cast<const uint32_t*>(kl + kk * 16 + 8));
+          mma16816(p, qa[kk], b0, b1);
+#pragma unroll
+          for (int e = 0; e < 4; e++) s[j][e] += p[e];
+        } else {
+          mma16816(s[j], qa[kk], b0, b1);
+          mma16816(s[j], ql[kk], b0, b1);
+        }
+      }
+      if constexpr (F32) {
+        const float2 kd = *reinterpret_cast<const float2*>(s_kd + j * 8 + tq * 2);
+        s[j][0] *= kd.x; s[j][1] *= kd.y; s[j][2] *= kd.x; s[j][3] *= kd.y;
       }
     }
     // scale, causal mask, online softmax (rows g and g + 8; a row's 64 scores live in the 4 lanes of a quad)
@@ -224,10 +272,10 @@ __global__ void __launch_bounds__(PF_THREADS) attn_prefill_kernel(const float* _
 #pragma unroll
     for (int j = 0; j < PK / 8; j++) {
       const int key = k0 + j * 8 + tq * 2;
-      s[j][0] = key <= qpos0 ? s[j][0] * scale : -INFINITY;
-      s[j][1] = key + 1 <= qpos0 ? s[j][1] * scale : -INFINITY;
-      s[j][2] = key <= qpos1 ? s[j][2] * scale : -INFINITY;
-      s[j][3] = key + 1 <= qpos1 ? s[j][3] * scale : -INFINITY;
+      s[j][0] = key <= qpos0 ? s[j][0] * qd0 : -INFINITY;
+      s[j][1] = key + 1 <= qpos0 ? s[j][1] * qd0 : -INFINITY;
+      s[j][2] = key <= qpos1 ? s[j][2] * qd1 : -INFINITY;
+      s[j][3] = key + 1 <= qpos1 ? s[j][3] * qd1 : -INFINITY;
       mx0 = fmaxf(mx0, fmaxf(s[j][0], s[j][1]));
       mx1 = fmaxf(mx1, fmaxf(s[j][2], s[j][3]));
     }
@@ -247,6 +295,55 @@ __global__ void __launch_bounds__(PF_THREADS) attn_prefill_kernel(const float* _
     sum0 += __shfl_xor_sync(0xffffffffu, sum0, 1); sum0 += __shfl_xor_sync(0xffffffffu, sum0, 2);
     sum1 += __shfl_xor_sync(0xffffffffu, sum1, 1); sum1 += __shfl_xor_sync(0xffffffffu, sum1, 2);
     l0 = l0 * c0 + sum0; l1 = l1 * c1 + sum1; m0 = mn0; m1 = mn1;
+    if constexpr (F32) {
+      // probabilities take the value rows' powers of two along, under one more per query that the chunk's sum gives back
+      float t0 = 0.f, t1 = 0.f, up0, up1, dn0, dn1;
+#pragma unroll
+      for (int j = 0; j < PK / 8; j++) {
+        const float2 vd = *reinterpret_cast<const float2*>(s_vd + j * 8 + tq * 2);
+        s[j][0] *= vd.x; s[j][1] *= vd.y; s[j][2] *= vd.x; s[j][3] *= vd.y;
+        t0 = fmaxf(t0, fmaxf(s[j][0], s[j][1])); t1 = fmaxf(t1, fmaxf(s[j][2], s[j][3]));
+      }
+      t0 = fmaxf(t0, __shfl_xor_sync(0xffffffffu, t0, 1)); t0 = fmaxf(t0, __shfl_xor_sync(0xffffffffu, t0, 2));
+      t1 = fmaxf(t1, __shfl_xor_sync(0xffffffffu, t1, 1)); t1 = fmaxf(t1, __shfl_xor_sync(0xffffffffu, t1, 2));
+      pow2_scale(t0, up0, dn0);
+      pow2_scale(t1, up1, dn1);
+      uint32_t pa[PK / 16][4], pl[PK / 16][4];
+#pragma unroll
+      for (int kk = 0; kk < PK / 16; kk++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const float up = e & 1 ? up1 : up0;
+          split_pair(s[2 * kk + (e >> 1)][(e & 1) * 2] * up, s[2 * kk + (e >> 1)][(e & 1) * 2 + 1] * up, pa[kk][e], pl[kk][e]);
+        }
+#pragma unroll
+      for (int n0 = 0; n0 < HD; n0 += 16) {
+        float t[2][4] = {};
+#pragma unroll
+        for (int kk = 0; kk < PK / 16; kk++) {
+          const __half* vp = s_v + (kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * STRIDE + n0 + (lane >> 4) * 8;
+          uint32_t h[4], l[4];
+          ldsm4_trans(h, vp);
+          ldsm4_trans(l, vp + (s_vl - s_v));
+          float p[2][4] = {};
+#pragma unroll
+          for (int e = 0; e < 2; e++) {
+            mma16816(p[e], pl[kk], h[2 * e], h[2 * e + 1]);
+            mma16816(p[e], pa[kk], l[2 * e], l[2 * e + 1]);
+            mma16816(p[e], pa[kk], h[2 * e], h[2 * e + 1]);
+#pragma unroll
+            for (int i = 0; i < 4; i++) t[e][i] += p[e][i];
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          float (&d)[4] = o[n0 / 8 + e];
+          d[0] = fmaf(t[e][0], dn0, d[0] * c0); d[1] = fmaf(t[e][1], dn0, d[1] * c0);
+          d[2] = fmaf(t[e][2], dn1, d[2] * c1); d[3] = fmaf(t[e][3], dn1, d[3] * c1);
+        }
+      }
+      continue;
+    }
 #pragma unroll
     for (int j = 0; j < HD / 8; j++) { o[j][0] *= c0; o[j][1] *= c0; o[j][2] *= c1; o[j][3] *= c1; }
     // O += P V: P from the score fragments (fp16), V through transposing ldmatrix
@@ -255,24 +352,15 @@ __global__ void __launch_bounds__(PF_THREADS) attn_prefill_kernel(const float* _
       // probabilities as fp16 hi + lo as well (two MMAs per tile): their rounding would otherwise be the largest error left
       uint32_t pa[4], pl[4];
 #pragma unroll
-      for (int e = 0; e < 4; e++) {
-        const float a = s[2 * kk + (e >> 1)][(e & 1) * 2], b = s[2 * kk + (e >> 1)][(e & 1) * 2 + 1];
-        const __half2 h2 = __floats2half2_rn(a, b);
-        const float2 back = __half22float2(h2);
-        pa[e] = *reinterpret_cast<const uint32_t*>(&h2);
-        pl[e] = pack_h2(a - back.x, b - back.y);
-      }
+      for (int e = 0; e < 4; e++) split_pair(s[2 * kk + (e >> 1)][(e & 1) * 2], s[2 * kk + (e >> 1)][(e & 1) * 2 + 1], pa[e], pl[e]);
 #pragma unroll
       for (int n0 = 0; n0 < HD; n0 += 16) {
-        // four 8x8 blocks: keys kk*16 + {0..7, 8..15} x dims n0 + {0..7, 8..15}; lane l supplies the row address of block l / 8
-        const __half* vp = s_v + (kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * STRIDE + n0 + (lane >> 4) * 8;
-        uint32_t r0, r1, r2, r3;
-        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                     : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"((uint32_t)__cvta_generic_to_shared(vp)));
-        mma16816(o[n0 / 8], pa, r0, r1);
-        mma16816(o[n0 / 8], pl, r0, r1);
-        mma16816(o[n0 / 8 + 1], pa, r2, r3);
-        mma16816(o[n0 / 8 + 1], pl, r2, r3);
+        uint32_t r[4];
+        ldsm4_trans(r, s_v + (kk * 16 + ((lane >> 3) & 1) * 8 + (lane & 7)) * STRIDE + n0 + (lane >> 4) * 8);
+        mma16816(o[n0 / 8], pa, r[0], r[1]);
+        mma16816(o[n0 / 8], pl, r[0], r[1]);
+        mma16816(o[n0 / 8 + 1], pa, r[2], r[3]);
+        mma16816(o[n0 / 8 + 1], pl, r[2], r[3]);
       }
     }
   }
@@ -289,7 +377,7 @@ __global__ void __launch_bounds__(PF_THREADS) attn_prefill_kernel(const float* _
 template <int HD, typename KV, typename O>
 cudaError_t launch_prefill_attn2(const void* q, const void* kc, const void* vc, int start_pos, int n_rows, int n_heads, int n_kv, int max_context, void* out,
                                  int n_seqs, const int32_t* pos_dev, cudaStream_t st) {
-  const size_t smem = (size_t)(2 * PQ + 2 * PK) * (HD + 8) * sizeof(__half);
+  const size_t smem = (size_t)(2 * PQ + (sizeof(KV) == 4 ? 4 : 2) * PK) * (HD + 8) * sizeof(__half);      // fp32 caches of head_dim 128: 104 KB, two CTAs an SM
   static PerDeviceFlag attr;
   const int dev = b200q_current_device();
   if (dev < 0) return cudaErrorInvalidDevice;
