@@ -249,6 +249,7 @@ class Transformer:
     self.seq_cache_bytes = c.n_kv_heads * c.max_context * c.head_dim * np.dtype(kvdt).itemsize
     self.attn_scratch = DeviceBuffer(_lib.load().b200q_attn_scratch_bytes(c.n_heads, c.n_kv_heads, c.head_dim, self.n_split), zero=True)
     self._mirror = PinnedBuffer((batch,), np.int32)      # the sampled tokens as the arg-max kernel leaves them for the host
+    self._head_queued = False                            # a step with the head may not have written its token there yet
     self.argmax_scratch = DeviceBuffer(batch * _lib.load().b200q_argmax_scratch_bytes(), zero=True)
     # Quantised activation hand-over between consecutive kernels (needs whole 128-wide groups everywhere).  Each edge of
     # the chain can be switched on its own: attn_o (attention -> output projection), o_gateup, gateup_down, down_qkv.
@@ -509,6 +510,7 @@ class Transformer:
     (weights streamed once per step), attention runs per sequence on its own cache, the arg-max per sequence.  Captured once into a
     CUDA graph (positions and tokens live on the device) and replayed."""
     self._check_room()
+    self._head_queued = True
     if not self.use_graph: return self._enqueue_batch_step()
     if self._batch_graph is None:
       self._enqueue_batch_step()                       # allocates the buffers outside the capture (and is a real step)
@@ -655,6 +657,7 @@ class Transformer:
     """Advance by one token on the device: reads tokens[pos]; with the head, writes tokens[pos+1].
     The host mirrors the device position and refuses a step that has no KV-cache row left (nothing is launched then)."""
     self._check_room()
+    if with_head: self._head_queued = True
     if self.is_moe: return self._step_rows(with_head)
     self._host_pos += 1
     if self._step_args: return check(_lib.load().b200q_decode_step(ctypes.byref(self._step_args[bool(with_head)]), self.stream.ptr))
@@ -684,11 +687,14 @@ class Transformer:
     return int(self.tokens.numpy((1,), np.int32, offset=4 * index)[0])
 
   def _sampled(self, step) -> list:
-    """Run `step` and wait for the tokens it samples: the arg-max kernel also writes them to page-locked memory, which is polled."""
+    """Run `step` and wait for the tokens it samples: the arg-max kernel also writes them to page-locked memory, which is polled.  Steps that a caller has
+    queued must have left theirs first: one that comes after the words are cleared would pass for this step's."""
+    if self._head_queued: self.stream.synchronize()
     m = self._mirror.array
     m[:] = -1
     step()
     check(_lib.load().b200q_wait_words(self._mirror.ptr, len(m), -1, self.stream.ptr))
+    self._head_queued = False
     return m.tolist()
 
   def read_logits(self) -> np.ndarray:
