@@ -41,6 +41,12 @@ def test_rows_against_the_exact_product(typ, m, n_out, n_in, dt, split):
   assert (np.abs(y.numpy() - ref) <= bound).all(), f"worst {np.max(np.abs(y.numpy() - ref) / bound):.2f} of the bound"
 
 
+# more rows than m rounded up to 128: 3 x 224, 10 x 256
+@pytest.mark.parametrize("split", [True, False])
+@pytest.mark.parametrize("typ,m", [(8, 625), (2, 640), (2, 641), (8, 2401)])
+def test_equal_tiles_of_more_rows(typ, m, split): test_rows_against_the_exact_product(typ, m, 300, 416, np.float32, split)
+
+
 @pytest.mark.parametrize("typ,m,n_out,n_in", [(2, 1, 64, 32), (8, 1, 1536, 1024), (8, 52, 130, 128), (2, 200, 512, 992)])
 def test_unsplit_sums_have_the_bits_of_the_kernel_without_a_workspace(typ, m, n_out, n_in):
   rng = np.random.default_rng(m)

@@ -22,6 +22,7 @@
 // Every mbarrier wait is bounded: on expiry a status word is set, all roles leave, copies and MMAs in flight are drained.
 #include "common.cuh"
 #include "tc_common.cuh"
+#include <algorithm>
 #include <cstddef>
 
 namespace {
@@ -577,10 +578,13 @@ static size_t split_workspace(const Plan& pl, int n_out, int kgroups, int n_sm) 
   return COUNTER_BYTES + (size_t)parts * pl.wt * pl.nt * sizeof(float);
 }
 
-// Room for the activations in tiles of 128 rows (the kernel's own tiles never take more): enough to run, tiles then going whole to the CTAs
+// Room for the activation tiles: enough to run, tiles then going whole to the CTAs.  Equal tiles of up to 256 rows may hold more rows than m rounded up to 128
+// (625 rows: 3 x 224), never fewer than a smaller m has.
 extern "C" size_t b200q_qgemm_workspace_bytes(int m, int n_in) {
   if (m <= 0 || n_in <= 0) return 0;
-  return (size_t)ceil_div(m, 128) * 128 * ceil_div(n_in, GROUP_ELEMS) * GROUP_ELEMS * 4;
+  const Plan pl = make_plan(m, 0, 0);
+  const size_t rows = std::max((size_t)ceil_div(m, 128) * 128, (size_t)pl.tok_tiles * pl.nt);
+  return rows * ceil_div(n_in, GROUP_ELEMS) * GROUP_ELEMS * 4;
 }
 extern "C" size_t b200q_qgemm_workspace_bytes_for(int m, int n_out, int n_in) {
   if (m <= 0 || n_in <= 0 || n_out < 0) return 0;
@@ -604,7 +608,7 @@ int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtyp
   const bool f32 = x_dtype == B200Q_F32;
   const int kgroups = ceil_div(n_in, GROUP_ELEMS);
   const size_t xt_bytes = align256(tiles_bytes(pl, kgroups, f32));
-  if (workspace_bytes < tiles_bytes(pl, kgroups, f32)) return B200Q_ERR_TOO_LARGE;
+  if (workspace_bytes < b200q_qgemm_workspace_bytes(m, n_in)) return B200Q_ERR_TOO_LARGE;
   const int n_sm = b200q_sm_count();
   if (n_sm <= 0) return B200Q_ERR_CUDA;
   pl = make_plan(m, n_out, n_sm);

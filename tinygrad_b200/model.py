@@ -391,9 +391,12 @@ class Transformer:
 
   # ---- several prompt tokens at once: tcgen05 dequant GEMMs + batched causal attention ----
   def _rows_workspace_bytes(self, T: int) -> int:
+    """The GEMMs' workspace for chunks of up to T rows (partial sums grow with a tile's rows, and fewer rows may be in larger tiles: 640 are 3 x 224, 512
+    2 x 256)."""
     c, qkv_rows = self.config, self.q_dim + 2 * self.kv_dim
     if self.is_moe: return quant.qgemm_unsplit_workspace_bytes(T, max(c.dim, self.q_dim, c.shared_expert_dim))
-    return max(quant.qgemm_workspace_bytes(T, i, o) for o, i in ((qkv_rows, c.dim), (c.dim, self.q_dim), (2 * c.hidden_dim, c.dim), (c.dim, c.hidden_dim)))
+    shapes = ((qkv_rows, c.dim), (c.dim, self.q_dim), (2 * c.hidden_dim, c.dim), (c.dim, c.hidden_dim))
+    return max(quant.qgemm_workspace_bytes(m, i, o) for o, i in shapes for m in {T, *range(16, T, 16)})      # tiles are whole 16 rows
 
   def _prefill_buffers(self):
     if self._pf is None:
