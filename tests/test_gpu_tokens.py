@@ -23,3 +23,10 @@ def test_queued_steps_do_not_pass_for_the_next_token():
   for _ in range(3):
     for _ in range(300): m.step()                # about 15 ms of work
     assert next(m.generate(prompt)) == first     # all but the last prompt token are in the cache: one step
+
+
+def test_generate_on_a_model_for_batches():
+  """A model built for several sequences also answers one prompt, as one built for it does."""
+  prompt = [int(t) for t in np.random.default_rng(2).integers(0, 2000, 9)]
+  want, got = ([t for t, _ in zip(m.generate(prompt), range(6))] for m in (model(), model(batch=3)))
+  assert got == want

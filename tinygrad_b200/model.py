@@ -598,7 +598,7 @@ class Transformer:
     self.pos.copy_from(np.full((B,), L - 1, dtype=np.int32))
     self._host_pos, n = L - 1, L
     while n < c.max_context:
-      yield self._sampled(self.decode_batch_step)
+      yield self._sampled(self.decode_batch_step, B)
       n += 1
 
   def _step_rows(self, with_head: bool) -> None:
@@ -689,14 +689,14 @@ class Transformer:
     self.stream.synchronize()
     return int(self.tokens.numpy((1,), np.int32, offset=4 * index)[0])
 
-  def _sampled(self, step) -> list:
-    """Run `step` and wait for the tokens it samples: the arg-max kernel also writes them to page-locked memory, which is polled.  Steps that a caller has
+  def _sampled(self, step, n: int = 1) -> list:
+    """Run `step` and wait for the `n` tokens it samples: the arg-max kernel also writes them to page-locked memory, which is polled.  Steps that a caller has
     queued must have left theirs first: one that comes after the words are cleared would pass for this step's."""
     if self._head_queued: self.stream.synchronize()
-    m = self._mirror.array
+    m = self._mirror.array[:n]
     m[:] = -1
     step()
-    check(_lib.load().b200q_wait_words(self._mirror.ptr, len(m), -1, self.stream.ptr))
+    check(_lib.load().b200q_wait_words(self._mirror.ptr, n, -1, self.stream.ptr))
     self._head_queued = False
     return m.tolist()
 
