@@ -706,7 +706,7 @@ class Transformer:
 
   def get_start_pos(self, tokens: list) -> int:
     """How much of the KV cache the new prompt can reuse (model.py:456-462)."""
-    n, old = min(len(tokens) - 1, len(self._cached_tokens)), self._cached_tokens
+    n, old = max(0, min(len(tokens) - 1, len(self._cached_tokens))), self._cached_tokens
     if tokens[:n] == old[:n]: return n
     lo = 0                                    # tokens[:lo] agree, tokens[:n] do not
     while n - lo > 1:
