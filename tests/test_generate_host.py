@@ -1,6 +1,7 @@
 """What `generate` decides on the host, without a device."""
 import random
-from tinygrad_b200.model import Transformer
+import pytest
+from tinygrad_b200.model import PREFILL_ROWS, Transformer
 
 
 def test_reusable_prefix():
@@ -14,3 +15,14 @@ def test_reusable_prefix():
       if a != b: break
       want += 1
     assert m.get_start_pos(prompt) == want, (prompt, m._cached_tokens)
+
+
+@pytest.mark.parametrize("rows,tokens,one_pass", [(64, 21, False), (64, 64, False), (64, 65, True), (20, 21, True), (PREFILL_ROWS, 6, False), (PREFILL_ROWS, 7, True), (1, 2, True), (0, 500, False)])
+def test_prefill_rows_says_which_prompts_go_in_one_pass(monkeypatch, rows, tokens, one_pass):
+  """`prefill_rows` uncached tokens (a prompt but its last) and more take one pass, fewer one step each; 0: always steps."""
+  m, did = Transformer.__new__(Transformer), []
+  m.prefill_rows, m.max_context, m._cached_tokens, m._step_args = rows, 1024, [], None
+  for name, f in dict(_put_tokens=lambda t, p: None, prefill=lambda p, n: did.append(n), step=lambda with_head=True: did.append(1), _sampled=lambda step: [7]).items():
+    monkeypatch.setattr(m, name, f)
+  next(m.generate(list(range(tokens))))
+  assert did == ([tokens - 1] if one_pass else [1] * (tokens - 1))

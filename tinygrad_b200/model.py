@@ -20,9 +20,9 @@ import ctypes, itertools, os
 SEQ_ATTENTION = os.environ.get("B200Q_SEQ_ATTENTION", "0") == "1"
 
 
-# prompts of at least this many uncached tokens take the GEMM path (unless it is off) even below prefill_rows: one pass over the weights for all of them
-# costs about as much as this many one-token steps
-SHORT_PROMPT_ROWS = 6
+# prompts of at least this many uncached tokens take the GEMM path: one pass over the weights for all of them costs about as much as this many
+# one-token steps
+PREFILL_ROWS = 6
 
 
 @dataclass(frozen=True)
@@ -92,14 +92,14 @@ STAGED_HANDOVER = os.environ.get("B200Q_STAGED_HANDOVER", "1") == "1"
 
 class Transformer:
   def __init__(self, config: TransformerConfig, state_dict: dict, ggml_type: int = _lib.Q4_0, n_split: int = 0, use_pdl: bool = True,
-               use_graph: bool = True, gemv_max_ctas: int = 0, handover=None, tp=None, output_type: int = None, prefill_rows: int = 64,
+               use_graph: bool = True, gemv_max_ctas: int = 0, handover=None, tp=None, output_type: int = None, prefill_rows: int = PREFILL_ROWS,
                prefill_chunk: int = 512, batch: int = 1, engine: str = None, linear_types: dict = None, pipelined_gemm: bool = True):
     """state_dict: the reference's tensor names -> numpy arrays; Linear weights as raw
     GGUF block bytes (uint8), embeddings / norms / biases as fp16.
     tp: a tensor_parallel.TPGroup; `config` is then the FULL model and `state_dict` this rank's shard (shard_state_dict).
     output_type: GGML type of `output.weight` when it differs from the block Linears' (F16 / BF16 / F32 heads run the dense GEMV).
-    prefill_rows: prompts with at least this many uncached tokens, or SHORT_PROMPT_ROWS, go through the tensor-core GEMM path, `prefill_chunk`
-    rows at a time (0: always one token per step); shorter ones take decode steps.
+    prefill_rows: prompts with at least this many uncached tokens go through the tensor-core GEMM path, `prefill_chunk` rows at a time (0: always one
+    token per step); shorter ones take decode steps.
     engine: how a one-token step runs.  "step": one persistent kernel for the whole step (b200q_decode_step); "chain": five launches per
     block chained with programmatic dependent launch and replayed as a CUDA graph (the default: at batch 1 it measured faster, the
     grid-wide waits inside one kernel costing more than kernel boundaries do).
@@ -716,14 +716,14 @@ class Transformer:
     return lo
 
   def generate(self, tokens: list, temperature: float = 0.0):
-    """Greedy generation (model.py:464-484 at temperature 0).  Yields one token id at a time;
-    the prompt is consumed one position per step through the same kernels."""
+    """Greedy generation (model.py:464-484 at temperature 0).  Yields one token id at a time; a prompt is consumed in chunks (`prefill_rows`) or one
+    position per step, its last token always in the step that samples the first answer token."""
     if temperature != 0.0: raise NotImplementedError("only greedy decoding (temperature 0) is implemented")
     tokens = list(tokens)
     start_pos = self.get_start_pos(tokens)
     self._put_tokens(tokens, start_pos)
     n_pre = len(tokens) - 1 - start_pos
-    if self.prefill_rows and n_pre >= min(self.prefill_rows, SHORT_PROMPT_ROWS): self.prefill(start_pos, n_pre)
+    if self.prefill_rows and n_pre >= self.prefill_rows: self.prefill(start_pos, n_pre)
     else:
       for _ in range(n_pre): self.step(with_head=False)
     while len(tokens) < self.max_context:
