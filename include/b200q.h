@@ -28,6 +28,7 @@ extern "C" {
 #define B200Q_ERR_UNSUPPORTED (-4)  /* quant type / dtype combination not built */
 #define B200Q_ERR_CUDA (-5)         /* a CUDA call failed: see b200q_last_cuda_error() */
 #define B200Q_ERR_TOO_LARGE (-6)    /* request exceeds a fixed capacity of the library */
+#define B200Q_ERR_NO_RESULT (-7)    /* the stream is done but what was waited for has not been written: see b200q_status_read_clear */
 
 /* ---- enums -------------------------------------------------------------- */
 /* GGML tensor types, numbered as in the GGUF file format (tinygrad/llm/gguf.py:20-21). */
@@ -301,8 +302,8 @@ int b200q_argmax_advance(const float* device_logits, int n, int32_t* device_toke
 /* The same for n_seqs sequences in one launch: logits [n_seqs, n], tokens rows token_stride apart, pos [n_seqs], scratch n_seqs x
  * b200q_argmax_scratch_bytes, zeroed once.  mirror: NULL, or page-locked host memory (b200q_host_alloc) [n_seqs] that also gets the tokens.
  * b200q_wait_words: waits until none of n such words is `empty` any more (the host fills them with it before the launch): it polls the
- * words, which sees a token several microseconds before a stream synchronisation returns, and falls back to one after 20 ms; an error
- * if the words are still empty then. */
+ * words, which sees a token several microseconds before a stream synchronisation returns, and falls back to one after 20 ms;
+ * B200Q_ERR_NO_RESULT if the words are still empty then (a step at a position past the context, for instance). */
 int b200q_argmax_advance_seqs(const float* logits, int n, int32_t* tokens, int token_stride, int32_t* pos, int max_context, void* scratch, int n_seqs,
                               int32_t* mirror, int flags, void* stream);
 int b200q_wait_words(const int32_t* words, int n, int32_t empty, void* stream);

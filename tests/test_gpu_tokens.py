@@ -1,8 +1,9 @@
 """Tokens as `generate` sees them: polled from page-locked memory while the device may still be busy with other steps."""
 import numpy as np
 import pytest
-from tinygrad_b200 import synth
+from tinygrad_b200 import _lib, synth
 from tinygrad_b200.model import Transformer, TransformerConfig
+from tinygrad_b200.runtime import PinnedBuffer, Stream
 from gpu_util import need_gpu
 
 pytestmark = pytest.mark.gpu
@@ -30,3 +31,11 @@ def test_generate_on_a_model_for_batches():
   prompt = [int(t) for t in np.random.default_rng(2).integers(0, 2000, 9)]
   want, got = ([t for t, _ in zip(m.generate(prompt), range(6))] for m in (model(), model(batch=3)))
   assert got == want
+
+
+def test_a_step_without_a_token_is_called_that():
+  """Words that nothing fills: an error of their own once the stream is done, not that of a bad argument."""
+  need_gpu()
+  words, st = PinnedBuffer((2,), np.int32), Stream()
+  words.array[:] = (5, -1)
+  assert _lib.load().b200q_wait_words(words.ptr, 2, -1, st.ptr) == -7 and b"no result" in _lib.load().b200q_strerror(-7)

@@ -43,6 +43,7 @@ extern "C" const char* b200q_strerror(int code) {
     case B200Q_ERR_UNSUPPORTED: return "quant type / dtype / option combination not supported";
     case B200Q_ERR_CUDA: return "CUDA call failed (see b200q_last_cuda_error)";
     case B200Q_ERR_TOO_LARGE: return "request exceeds a fixed capacity of the library";
+    case B200Q_ERR_NO_RESULT: return "the stream is done but left no result (see b200q_status_read_clear)";
     default: return "unknown b200q status";
   }
 }
@@ -135,7 +136,7 @@ extern "C" int b200q_wait_words(const int32_t* words, int n, int32_t empty, void
 #endif
     if ((k & 255) == 255 && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(20)) {
       B200Q_CHECK_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
-      return all() ? B200Q_OK : B200Q_ERR_BAD_ARG;
+      return all() ? B200Q_OK : B200Q_ERR_NO_RESULT;
     }
   }
   return B200Q_OK;
