@@ -88,25 +88,38 @@ class DeviceBuffer:
     except Exception: pass
 
 
-class PinnedBuffer:
-  """Page-locked host memory viewed as a numpy array (source/target of async copies)."""
-  def __init__(self, shape, dtype):
-    shape = (shape,) if isinstance(shape, int) else tuple(shape)
-    self.nbytes = int(np.prod(shape, dtype=np.int64)) * np.dtype(dtype).itemsize
+class _Pages:
+  """Page-locked pages; they go back with the last object that holds this one."""
+  def __init__(self, nbytes: int):
     p = ctypes.c_void_p()
-    check(_lib.load().b200q_host_alloc(ctypes.byref(p), self.nbytes))
+    check(_lib.load().b200q_host_alloc(ctypes.byref(p), nbytes))
     self.ptr = int(p.value)
-    self.array = np.frombuffer((ctypes.c_char * self.nbytes).from_address(self.ptr), dtype=dtype).reshape(shape)
 
   def free(self) -> None:
     if self.ptr:
-      self.array = None
       _lib.load().b200q_host_free(self.ptr)
       self.ptr = 0
 
   def __del__(self):
     try: self.free()
     except Exception: pass
+
+
+class PinnedBuffer:
+  """Page-locked host memory viewed as a numpy array (source/target of async copies).  The memory lives as long as this object or a view of `array`,
+  unless it is given back by `free`."""
+  def __init__(self, shape, dtype):
+    shape = (shape,) if isinstance(shape, int) else tuple(shape)
+    self.nbytes = int(np.prod(shape, dtype=np.int64)) * np.dtype(dtype).itemsize
+    self._pages = _Pages(self.nbytes)
+    self.ptr = self._pages.ptr
+    raw = (ctypes.c_char * self.nbytes).from_address(self.ptr)
+    raw.pages = self._pages                  # every view of the array holds `raw`
+    self.array = np.frombuffer(raw, dtype=dtype).reshape(shape)
+
+  def free(self) -> None:
+    self.array, self.ptr = None, 0
+    self._pages.free()
 
 
 def stream_ptr(stream) -> int:
