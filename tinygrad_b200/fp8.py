@@ -44,7 +44,7 @@ class FP8Linear:
                off=DeviceBuffer.from_numpy(np.array([0, mp], np.int32)), parts=DeviceBuffer.empty((592,), np.float32), factor=DeviceBuffer.empty((1,), np.float32))
       check(lib.b200q_memset(w["x_e8"].ptr, 127, w["x_e8"].nbytes, None))
       check(lib.b200q_device_synchronize())
-      w["desc"] = _lib.Fp8LinearDesc(self.out_features, self.in_features, mp, None, self._w_e8.ptr, None, self.bias.ptr if self.bias else None, w["x_q"].ptr,
+      w["desc"] = _lib.Fp8LinearDesc(self.out_features, self.in_features, mp, None, self._w_e8.ptr, None, None, w["x_q"].ptr,
                                      w["x_e8"].ptr, w["off"].ptr, w["parts"].ptr, w["factor"].ptr)
       self._ws[m] = w
     return w["desc"]
@@ -57,6 +57,6 @@ class FP8Linear:
     m, shape = math.prod(lead), (*lead, self.out_features)
     if m == 0: return DeviceBuffer.empty(shape, x.dtype)
     d, y = self._workspace(m), ctypes.c_void_p()
-    d.w_q, d.w_factor = self.w_q.ptr, self.w_factor.ptr
+    d.w_q, d.w_factor, d.bias = self.w_q.ptr, self.w_factor.ptr, self.bias and self.bias.ptr
     check(_lib.load().b200q_fp8_linear(ctypes.byref(d), x.ptr, dt, m, ctypes.byref(y), stream_ptr(stream)))
     return DeviceBuffer.adopt(y.value, m * self.out_features * x.dtype.itemsize, shape, x.dtype)

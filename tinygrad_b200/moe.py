@@ -116,11 +116,13 @@ class MxMoE:
       r = w["r"]
       gating, norm, scale = (*self.mode.resolved(), float(self.mode.routed_scaling_factor)) if isinstance(self.mode, Gating) else (0, 0, 1.0)
       w["ends"] = DeviceBuffer.empty((self.E,), np.int32)
-      w["args"] = _lib.MoeArgs(self.E, self.k, self.D, self.F, 0 if gating else self.mode, gating, int(norm), scale, r._bias.ptr if r._bias else None, self.gu_q.ptr,
-                               self.gu_e8.ptr, self.dn_q.ptr, self.dn_e8.ptr, r.topi.ptr, r.weights.ptr, r.dest_row.ptr, r.off.ptr, w["ends"].ptr, r._scratch.ptr,
+      w["args"] = _lib.MoeArgs(self.E, self.k, self.D, self.F, 0 if gating else self.mode, gating, int(norm), scale, r._bias.ptr if r._bias else None, None, None, None, None,
+                               r.topi.ptr, r.weights.ptr, r.dest_row.ptr, r.off.ptr, w["ends"].ptr, r._scratch.ptr,
                                w["a_q"].ptr, w["a_e8"].ptr, w["act_q"].ptr, w["act_e8"].ptr, w["y"].ptr, w["out"].ptr)
       w["args_ref"] = ctypes.byref(w["args"])
-    return w["args"]
+    a = w["args"]
+    a.gu_q, a.gu_e8, a.dn_q, a.dn_e8 = self.gu_q.ptr, self.gu_e8.ptr, self.dn_q.ptr, self.dn_e8.ptr      # the weights this layer holds now
+    return a
 
   def __call__(self, x_bf16: DeviceBuffer, logits: DeviceBuffer, n_tokens: int, stream=None) -> DeviceBuffer:
     """x (T, D) bf16, router logits (T, E) fp32 -> (T, D) bf16."""

@@ -205,9 +205,7 @@ class QuantLinear:
     self.weight = repack(raw, out_features, in_features, ggml_type) if self.fused else DenseWeight(raw, out_features, in_features, ggml_type)
     self.bias = None if bias is None else DeviceBuffer.from_numpy(np.asarray(bias, dtype=np.float16))
     self._ws = None      # activation tiles and partial sums of the GEMM, grown on demand
-    w = self.weight.buf
-    self._desc = _lib.LinearDesc(not self.fused, ggml_type if self.fused else self.weight.dtype, out_features, in_features, 0, w.ptr,
-                                 self.bias.ptr if self.bias else None, None, 0)
+    self._desc = _lib.LinearDesc(not self.fused, ggml_type if self.fused else self.weight.dtype, out_features, in_features)
     self._desc_ref, self._lock = ctypes.byref(self._desc), threading.Lock()
 
   def __call__(self, x: DeviceBuffer, stream=None) -> DeviceBuffer:
@@ -217,7 +215,7 @@ class QuantLinear:
     if k != self.in_features: raise ValueError(f"Input Tensor shapes {x.shape} cannot be multiplied with in_features={self.in_features}")
     m, d, y = math.prod(lead), self._desc, ctypes.c_void_p()
     with self._lock:       # the workspace and the descriptor are this object's
-      d.gemm_min_rows = GEMM_MIN_ROWS
+      d.gemm_min_rows, d.w, d.bias = GEMM_MIN_ROWS, self.weight.buf.ptr, self.bias and self.bias.ptr
       if self.fused and m >= GEMM_MIN_ROWS and self.ggml_type != Q6_K:
         need = qgemm_workspace_bytes(m, self.in_features, self.out_features)
         if self._ws is None or self._ws.nbytes < need:
