@@ -8,7 +8,8 @@
 // time after it was freed.  Freed blocks wait in a list; when the list holds PENDING_BLOCKS blocks or PENDING_BYTES, the next allocation
 // waits for the device once and turns the whole list into free blocks.  So a loop of calls waits once per 64 results (or 64 MiB) instead of
 // once per result.  Bounded: at most POOL_BYTES are kept per device (past that everything unused goes back with cudaFree), larger blocks than
-// BLOCK_MAX never enter, and everything goes back when an allocation fails or b200q_pool_trim is called.  One lock; any thread may call.
+// BLOCK_MAX never enter, and everything goes back when an allocation fails or b200q_pool_trim is called.  Any thread may call.  A device's lists have a lock
+// of their own, held during its wait: work on one device may depend on a thread that is allocating on another.
 #include "common.cuh"
 #include <mutex>
 #include <unordered_map>
@@ -24,9 +25,10 @@ struct DevicePool {
   std::unordered_map<size_t, std::vector<void*>> free_;       // by size
   std::vector<Block> pending;
   size_t pending_bytes = 0, kept = 0;                          // kept: free and pending bytes
+  std::mutex lock;
 };
-std::mutex g_lock;
 DevicePool g_pool[B200Q_MAX_DEVICES];
+std::mutex g_out_lock;                                         // never held together with a device's
 std::unordered_map<void*, std::pair<int, size_t>> g_out;      // blocks in use: device, size (0: not a pool size)
 
 // sizes in steps of an eighth of a power of two: at most an eighth is lost, and few sizes occur
@@ -55,12 +57,8 @@ void give_back(DevicePool& d) {                                // cudaFree waits
   d.pending_bytes = d.kept = 0;
 }
 
-int pool_alloc(void** out, size_t bytes) {
-  const int dev = b200q_current_device();
-  if (dev < 0) return B200Q_ERR_CUDA;
-  const size_t size = bytes <= BLOCK_MAX ? round_size(bytes) : bytes;
-  std::lock_guard<std::mutex> g(g_lock);
-  DevicePool& d = g_pool[dev];
+int take_block(DevicePool& d, void** out, size_t size) {
+  std::lock_guard<std::mutex> g(d.lock);
   if (size <= BLOCK_MAX) {
     if (d.pending.size() >= PENDING_BLOCKS || d.pending_bytes >= PENDING_BYTES) B200Q_CHECK_CUDA(recycle(d));
     auto it = d.free_.find(size);
@@ -68,7 +66,6 @@ int pool_alloc(void** out, size_t bytes) {
       *out = it->second.back();
       it->second.pop_back();
       d.kept -= size;
-      g_out[*out] = {dev, size};
       return B200Q_OK;
     }
   }
@@ -79,6 +76,16 @@ int pool_alloc(void** out, size_t bytes) {
     e = cudaMalloc(out, size);
   }
   B200Q_CHECK_CUDA(e);
+  return B200Q_OK;
+}
+
+int pool_alloc(void** out, size_t bytes) {
+  const int dev = b200q_current_device();
+  if (dev < 0) return B200Q_ERR_CUDA;
+  const size_t size = bytes <= BLOCK_MAX ? round_size(bytes) : bytes;
+  const int rc = take_block(g_pool[dev], out, size);
+  if (rc != B200Q_OK) return rc;
+  std::lock_guard<std::mutex> g(g_out_lock);
   g_out[*out] = {dev, size <= BLOCK_MAX ? size : 0};
   return B200Q_OK;
 }
@@ -87,7 +94,7 @@ int pool_alloc(void** out, size_t bytes) {
 
 // called when an ordinary allocation fails: true if there was something to give back
 bool b200q_pool_release(int dev) {
-  std::lock_guard<std::mutex> g(g_lock);
+  std::lock_guard<std::mutex> g(g_pool[dev].lock);
   const bool any = g_pool[dev].kept > 0;
   give_back(g_pool[dev]);
   return any;
@@ -97,21 +104,24 @@ extern "C" int b200q_pool_alloc(void** device_ptr, size_t bytes) { return device
 
 extern "C" int b200q_pool_free(void* device_ptr) {
   if (!device_ptr) return B200Q_OK;
-  std::unique_lock<std::mutex> g(g_lock);
-  auto it = g_out.find(device_ptr);
-  if (it == g_out.end()) return B200Q_ERR_BAD_ARG;
-  const int dev = it->second.first;
-  const size_t size = it->second.second;
-  g_out.erase(it);
-  DevicePool& d = g_pool[dev];
+  int dev;
+  size_t size;
+  {
+    std::lock_guard<std::mutex> g(g_out_lock);
+    auto it = g_out.find(device_ptr);
+    if (it == g_out.end()) return B200Q_ERR_BAD_ARG;
+    dev = it->second.first; size = it->second.second;
+    g_out.erase(it);
+  }
   if (size) {
+    DevicePool& d = g_pool[dev];
+    std::lock_guard<std::mutex> g(d.lock);
     if (d.kept + size > POOL_BYTES) give_back(d);              // full of blocks that nobody has asked for lately
     d.pending.push_back({device_ptr, size});
     d.pending_bytes += size;
     d.kept += size;
     return B200Q_OK;
   }
-  g.unlock();
   B200Q_CHECK_CUDA(cudaFree(device_ptr));
   return B200Q_OK;
 }
