@@ -70,8 +70,9 @@ int b200q_malloc(void** device_ptr, size_t bytes);
 int b200q_free(void* device_ptr);
 /* Device blocks for results that are allocated on every call: a freed block is handed out again once the device has been idle since it was
  * freed, so (as with b200q_free) work queued before the free may still use it, on any stream.  At most 256 MiB are kept per device;
- * b200q_pool_trim gives everything unused back. */
-int b200q_pool_alloc(void** device_ptr, size_t bytes);
+ * b200q_pool_trim gives everything unused back.  stream: the one whose work will write the block first; while it is being captured the block is
+ * an ordinary allocation, subject to the rules of the capture. */
+int b200q_pool_alloc(void** device_ptr, size_t bytes, void* stream);
 int b200q_pool_free(void* device_ptr);
 int b200q_pool_trim(void);
 int b200q_host_alloc(void** host_ptr, size_t bytes);              /* pinned host memory */

@@ -10,10 +10,12 @@
 
 static thread_local int g_device = 0;
 static std::atomic<int> g_syncs[2], g_mallocs, g_frees;
+static cudaStreamCaptureStatus g_capture = cudaStreamCaptureStatusNone;
 static std::atomic<bool> g_hold{false}, g_held{false};       // device 0's synchronisation waits while g_hold is set
 static char g_bytes[1 << 16];
 
 extern "C" {
+cudaError_t cudaStreamIsCapturing(cudaStream_t st, cudaStreamCaptureStatus* s) { *s = st ? g_capture : cudaStreamCaptureStatusNone; return cudaSuccess; }
 cudaError_t cudaMalloc(void** p, size_t) {
   static std::atomic<int> n{0};
   *p = g_bytes + 16 * n++;
@@ -33,9 +35,10 @@ int b200q_qgemm_ws(int, const void*, const void*, int, const void*, const void*,
 }
 void b200q_set_cuda_error(cudaError_t) {}
 int b200q_current_device() { return g_device; }
+extern "C" int b200q_malloc(void** p, size_t n) { return cudaMalloc(p, n) == cudaSuccess ? 0 : B200Q_ERR_CUDA; }
 
 #define CHECK(c) do { if (!(c)) { printf("line %d: %s\n", __LINE__, #c); exit(1); } } while (0)
-static void* get(size_t n) { void* p = nullptr; CHECK(b200q_pool_alloc(&p, n) == 0); return p; }
+static void* get(size_t n, void* st = nullptr) { void* p = nullptr; CHECK(b200q_pool_alloc(&p, n, st) == 0); return p; }
 
 int main() {
   // a freed block comes back only after the device has been waited for since
@@ -57,14 +60,24 @@ int main() {
   CHECK(b200q_pool_free(big) == 0 && g_frees == frees + 1);
   CHECK(b200q_pool_trim() == 0 && g_frees > frees + 1);
   CHECK(b200q_pool_free((char*)a + 8) == B200Q_ERR_BAD_ARG);
+  // what a captured stream is to write comes from no pool and goes back to none
+  CHECK(b200q_pool_free(get(4096)) == 0);
+  for (int i = 0; i < 64; i++) CHECK(b200q_pool_free(get(8192)) == 0);      // the next block of the pool is one that was in use
+  g_capture = cudaStreamCaptureStatusActive;
+  const int syncs = g_syncs[0], mallocs = g_mallocs, freed = g_frees;
+  void* c = get(4096, (void*)1);
+  CHECK(g_syncs[0] == syncs && g_mallocs == mallocs + 1);
+  CHECK(b200q_pool_free(c) == 0 && g_frees == freed + 1);
+  g_capture = cudaStreamCaptureStatusNone;
+  CHECK(b200q_pool_trim() == 0);
   // one device's wait stops nobody on another
   for (int i = 0; i < 64; i++) CHECK(b200q_pool_free(get(512)) == 0);      // no free block, 64 that wait
   g_hold = true;
-  std::thread t([] { void* p = nullptr; b200q_pool_alloc(&p, 512); });
+  std::thread t([] { void* p = nullptr; b200q_pool_alloc(&p, 512, nullptr); });
   for (int i = 0; !g_held && i < 10000; i++) std::this_thread::sleep_for(std::chrono::milliseconds(1));
   CHECK(g_held);
   std::atomic<bool> done{false};
-  std::thread u([&] { g_device = 1; void* p = nullptr; done = b200q_pool_alloc(&p, 512) == 0 && b200q_pool_free(p) == 0; });
+  std::thread u([&] { g_device = 1; void* p = nullptr; done = b200q_pool_alloc(&p, 512, nullptr) == 0 && b200q_pool_free(p) == 0; });
   for (int i = 0; !done && i < 2000; i++) std::this_thread::sleep_for(std::chrono::milliseconds(1));
   const bool other = done;
   g_hold = false;

@@ -49,3 +49,13 @@ def test_fp8_linear_equals_its_parts(m, n_in, n_out, dt, bias):
   _lib.check(lib.b200q_grouped_mxfp8_gemm_f32(xq.ptr, e8.ptr, lin.w_q.ptr, lin._w_e8.ptr, off.ptr, 1, mp, n_out, n_in, acc.ptr, None))
   _lib.check(lib.b200q_fp8_scale_bias(acc.ptr, m, n_out, lin.w_factor.ptr, factor.ptr, lin.bias.ptr if bias else None, y.ptr, code, None))
   np.testing.assert_array_equal(got, y.numpy())
+
+
+def test_results_of_captured_work_are_no_pool_blocks():
+  """A graph writes its results whenever it is replayed: under capture the layers ask for memory of their own, which the capture mode of `Graph` refuses."""
+  lin, x = quant.QuantLinear(512, 300, 2, synth.q4_0_blocks(300, 512, np.random.default_rng(0))), DeviceBuffer.empty((1, 512), np.float32, zero=True)
+  for _ in range(70): lin(x)                  # blocks of that size are waiting in the pool
+  st = runtime.Stream()
+  with pytest.raises(_lib.B200QError):
+    with runtime.Graph(st): lin(x, stream=st)
+  assert not lin(x, stream=st).numpy().any()

@@ -9,7 +9,7 @@ class Device:
   """The C calls a layer makes: memory is a number, the one-call layers leave their argument block in `seen`."""
   def __init__(self): self.next, self.seen = 4096, None
   def __getattr__(self, name): return lambda *a: 4096 if name.endswith(("_bytes", "_bytes_for", "_max")) else 0
-  def _alloc(self, out, nbytes):
+  def _alloc(self, out, nbytes, stream=None):
     self.next += 4096
     out._obj.value = self.next
     return 0

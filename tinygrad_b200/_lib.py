@@ -89,7 +89,7 @@ SIGNATURES = {
   "b200q_device_props": (c_int, [c_int, POINTER(c_int), POINTER(c_int), POINTER(c_int), POINTER(c_size_t)]),
   "b200q_malloc": (c_int, [POINTER(c_void_p), c_size_t]),
   "b200q_free": (c_int, [c_void_p]),
-  "b200q_pool_alloc": (c_int, [POINTER(c_void_p), c_size_t]),
+  "b200q_pool_alloc": (c_int, [POINTER(c_void_p), c_size_t, c_void_p]),
   "b200q_pool_free": (c_int, [c_void_p]),
   "b200q_pool_trim": (c_int, []),
   "b200q_linear": (c_int, [POINTER(LinearDesc), c_void_p, c_int, c_int, POINTER(c_void_p), c_void_p]),

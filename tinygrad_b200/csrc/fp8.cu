@@ -165,7 +165,7 @@ extern "C" int b200q_fp8_linear(const b200q_fp8_linear_desc* l, const void* x, i
   if (!l || !y || m <= 0 || !x || (dtype != B200Q_F32 && dtype != B200Q_F16)) return B200Q_ERR_BAD_ARG;
   if (!l->x_q || !l->x_e8 || !l->off || !l->parts || !l->factor || m > l->rows_max) return B200Q_ERR_BAD_ARG;
   cudaStream_t st = (cudaStream_t)stream;
-  int rc = b200q_pool_alloc(y, (size_t)m * l->n_out * (dtype == B200Q_F32 ? 4 : 2));
+  int rc = b200q_pool_alloc(y, (size_t)m * l->n_out * (dtype == B200Q_F32 ? 4 : 2), stream);
   if (rc != B200Q_OK) return rc;
   const int64_t n = (int64_t)m * l->n_in;
   const int g = quant_grid(n), vec = !((uintptr_t)x & 15);

@@ -59,15 +59,13 @@ void give_back(DevicePool& d) {                                // cudaFree waits
 
 int take_block(DevicePool& d, void** out, size_t size) {
   std::lock_guard<std::mutex> g(d.lock);
-  if (size <= BLOCK_MAX) {
-    if (d.pending.size() >= PENDING_BLOCKS || d.pending_bytes >= PENDING_BYTES) B200Q_CHECK_CUDA(recycle(d));
-    auto it = d.free_.find(size);
-    if (it != d.free_.end() && !it->second.empty()) {
-      *out = it->second.back();
-      it->second.pop_back();
-      d.kept -= size;
-      return B200Q_OK;
-    }
+  if (d.pending.size() >= PENDING_BLOCKS || d.pending_bytes >= PENDING_BYTES) B200Q_CHECK_CUDA(recycle(d));
+  auto it = d.free_.find(size);
+  if (it != d.free_.end() && !it->second.empty()) {
+    *out = it->second.back();
+    it->second.pop_back();
+    d.kept -= size;
+    return B200Q_OK;
   }
   cudaError_t e = cudaMalloc(out, size);
   if (e == cudaErrorMemoryAllocation) {
@@ -79,14 +77,24 @@ int take_block(DevicePool& d, void** out, size_t size) {
   return B200Q_OK;
 }
 
-int pool_alloc(void** out, size_t bytes) {
+// A result of work that is being captured belongs to the graph, which may write it long after it was freed here: it is no block of the pool but an allocation
+// of its own, which most capture modes refuse, as they do for any caller.
+int pool_alloc(void** out, size_t bytes, cudaStream_t st) {
   const int dev = b200q_current_device();
   if (dev < 0) return B200Q_ERR_CUDA;
-  const size_t size = bytes <= BLOCK_MAX ? round_size(bytes) : bytes;
-  const int rc = take_block(g_pool[dev], out, size);
-  if (rc != B200Q_OK) return rc;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) cudaGetLastError();      // the legacy stream beside a capture: not captured itself
+  const bool pooled = bytes <= BLOCK_MAX && capture == cudaStreamCaptureStatusNone;
+  const size_t size = pooled ? round_size(bytes) : bytes ? bytes : 1;
+  if (pooled) {
+    const int rc = take_block(g_pool[dev], out, size);
+    if (rc != B200Q_OK) return rc;
+  } else {
+    const int rc = b200q_malloc(out, size);
+    if (rc != B200Q_OK) return rc;
+  }
   std::lock_guard<std::mutex> g(g_out_lock);
-  g_out[*out] = {dev, size <= BLOCK_MAX ? size : 0};
+  g_out[*out] = {dev, pooled ? size : 0};
   return B200Q_OK;
 }
 
@@ -100,7 +108,9 @@ bool b200q_pool_release(int dev) {
   return any;
 }
 
-extern "C" int b200q_pool_alloc(void** device_ptr, size_t bytes) { return device_ptr ? pool_alloc(device_ptr, bytes) : B200Q_ERR_BAD_ARG; }
+extern "C" int b200q_pool_alloc(void** device_ptr, size_t bytes, void* stream) {
+  return device_ptr ? pool_alloc(device_ptr, bytes, (cudaStream_t)stream) : B200Q_ERR_BAD_ARG;
+}
 
 extern "C" int b200q_pool_free(void* device_ptr) {
   if (!device_ptr) return B200Q_OK;
@@ -137,7 +147,7 @@ extern "C" int b200q_pool_trim(void) {
 extern "C" int b200q_linear(const b200q_linear_desc* l, const void* x, int dtype, int m, void** y, void* stream) {
   if (!l || !y || m < 0 || (dtype != B200Q_F32 && dtype != B200Q_F16) || (m && !x)) return B200Q_ERR_BAD_ARG;
   const size_t row = (size_t)l->n_out * (dtype == B200Q_F32 ? 4 : 2);
-  int rc = pool_alloc(y, (size_t)m * row);
+  int rc = pool_alloc(y, (size_t)m * row, (cudaStream_t)stream);
   if (rc != B200Q_OK || m == 0) return rc;
   if (l->dense) rc = b200q_gemv_dense(l->w, l->w_type, l->n_out, l->n_in, m, x, dtype, nullptr, 0.f, l->bias, nullptr, *y, dtype, 0, stream);
   else if (m >= l->gemm_min_rows && l->w_type != B200Q_Q6_K)

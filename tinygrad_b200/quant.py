@@ -27,7 +27,7 @@ def dequantize(raw, n: int, ggml_type: int, dtype=np.float32, stream=None) -> De
   """Raw GGUF block bytes -> n values (fp32 bit-exact with the reference; fp16 = its RNE cast)."""
   if ggml_type not in GGML_QUANT: raise ValueError(f"GGML type '{ggml_type}' is not supported!")   # gguf.py:119
   raw = _as_device(raw)
-  out = DeviceBuffer.result((n,), dtype)
+  out = DeviceBuffer.result((n,), dtype, stream)
   check(_lib.load().b200q_dequant_raw(ggml_type, raw.ptr, out.ptr, n, _DT[np.dtype(dtype)], stream_ptr(stream)))
   return out
 

@@ -45,11 +45,11 @@ class DeviceBuffer:
     return b
 
   @staticmethod
-  def result(shape: tuple, dtype) -> "DeviceBuffer":
-    """Uninitialised memory for a result, from the result pool: for outputs that are made anew on every call."""
+  def result(shape: tuple, dtype, stream=None) -> "DeviceBuffer":
+    """Uninitialised memory for a result of work on `stream`, from the result pool: for outputs that are made anew on every call."""
     dtype = np.dtype(dtype)
     nbytes, p = math.prod(shape) * dtype.itemsize, ctypes.c_void_p()
-    check(_lib.load().b200q_pool_alloc(ctypes.byref(p), nbytes))
+    check(_lib.load().b200q_pool_alloc(ctypes.byref(p), nbytes, stream_ptr(stream)))
     return DeviceBuffer.adopt(p.value, nbytes, shape, dtype)
 
   @staticmethod
