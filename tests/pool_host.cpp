@@ -4,6 +4,7 @@
 #include <chrono>
 #include <cstdio>
 #include <cstdlib>
+#include <new>
 #include <set>
 #include <thread>
 #include "../include/b200q.h"
@@ -13,6 +14,14 @@ static std::atomic<int> g_syncs[2], g_mallocs, g_frees;
 static cudaStreamCaptureStatus g_capture = cudaStreamCaptureStatusNone;
 static std::atomic<bool> g_hold{false}, g_held{false};       // device 0's synchronisation waits while g_hold is set
 static char g_bytes[1 << 16];
+static bool g_full = false;                                  // host memory has run out
+
+void* operator new(size_t n) {
+  if (g_full) throw std::bad_alloc();
+  return malloc(n);
+}
+void operator delete(void* p) noexcept { free(p); }
+void operator delete(void* p, size_t) noexcept { free(p); }
 
 extern "C" {
 cudaError_t cudaStreamIsCapturing(cudaStream_t st, cudaStreamCaptureStatus* s) { *s = st ? g_capture : cudaStreamCaptureStatusNone; return cudaSuccess; }
@@ -69,6 +78,20 @@ int main() {
   CHECK(g_syncs[0] == syncs && g_mallocs == mallocs + 1);
   CHECK(b200q_pool_free(c) == 0 && g_frees == freed + 1);
   g_capture = cudaStreamCaptureStatusNone;
+  CHECK(b200q_pool_trim() == 0);
+  // no host memory: an error, no exception, and no block lost or handed out twice
+  std::set<void*> out, blocks;
+  for (int i = 0; i < 40; i++) blocks.insert(get(1024));
+  for (void* p : blocks) CHECK(b200q_pool_free(p) == 0);
+  const int given = g_mallocs, returned = g_frees;
+  void* none = nullptr;
+  g_full = true;
+  CHECK(b200q_pool_alloc(&none, 2048, nullptr) == B200Q_ERR_CUDA);
+  g_full = false;
+  CHECK(g_mallocs - given == g_frees - returned);
+  for (int i = 0; i < 60; i++) CHECK(b200q_pool_free(get(512 + 512 * (i & 7))) == 0);
+  for (int i = 0; i < 200; i++) { void* p = get(1024); CHECK(out.insert(p).second); }
+  for (void* p : out) CHECK(b200q_pool_free(p) == 0);
   CHECK(b200q_pool_trim() == 0);
   // one device's wait stops nobody on another
   for (int i = 0; i < 64; i++) CHECK(b200q_pool_free(get(512)) == 0);      // no free block, 64 that wait

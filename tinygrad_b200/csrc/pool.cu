@@ -12,6 +12,7 @@
 // of their own, held during its wait: work on one device may depend on a thread that is allocating on another.
 #include "common.cuh"
 #include <mutex>
+#include <new>
 #include <unordered_map>
 #include <vector>
 
@@ -42,9 +43,12 @@ size_t round_size(size_t n) {
 cudaError_t recycle(DevicePool& d) {                           // after this every pending block is free
   const cudaError_t e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return e;
-  for (const Block& b : d.pending) d.free_[b.size].push_back(b.p);
-  d.pending.clear();
-  d.pending_bytes = 0;
+  while (!d.pending.empty()) {                                 // one by one: a block is in one list at any time, whatever is thrown
+    const Block b = d.pending.back();
+    d.free_[b.size].push_back(b.p);
+    d.pending.pop_back();
+    d.pending_bytes -= b.size;
+  }
   return cudaSuccess;
 }
 
@@ -93,9 +97,22 @@ int pool_alloc(void** out, size_t bytes, cudaStream_t st) {
     const int rc = b200q_malloc(out, size);
     if (rc != B200Q_OK) return rc;
   }
-  std::lock_guard<std::mutex> g(g_out_lock);
-  g_out[*out] = {dev, pooled ? size : 0};
+  try {
+    std::lock_guard<std::mutex> g(g_out_lock);
+    g_out[*out] = {dev, pooled ? size : 0};
+  } catch (...) {
+    cudaFree(*out);
+    *out = nullptr;
+    throw;
+  }
   return B200Q_OK;
+}
+// Nothing is thrown across the C interface: the lists need host memory, and there may be none.
+template <typename F> int guarded(const F& f) {
+  try { return f(); } catch (const std::bad_alloc&) {
+    b200q_set_cuda_error(cudaErrorMemoryAllocation);
+    return B200Q_ERR_CUDA;
+  }
 }
 
 }  // namespace
@@ -109,7 +126,7 @@ bool b200q_pool_release(int dev) {
 }
 
 extern "C" int b200q_pool_alloc(void** device_ptr, size_t bytes, void* stream) {
-  return device_ptr ? pool_alloc(device_ptr, bytes, (cudaStream_t)stream) : B200Q_ERR_BAD_ARG;
+  return device_ptr ? guarded([&] { return pool_alloc(device_ptr, bytes, (cudaStream_t)stream); }) : B200Q_ERR_BAD_ARG;
 }
 
 extern "C" int b200q_pool_free(void* device_ptr) {
@@ -127,10 +144,12 @@ extern "C" int b200q_pool_free(void* device_ptr) {
     DevicePool& d = g_pool[dev];
     std::lock_guard<std::mutex> g(d.lock);
     if (d.kept + size > POOL_BYTES) give_back(d);              // full of blocks that nobody has asked for lately
-    d.pending.push_back({device_ptr, size});
-    d.pending_bytes += size;
-    d.kept += size;
-    return B200Q_OK;
+    const bool kept = guarded([&] { d.pending.push_back({device_ptr, size}); return B200Q_OK; }) == B200Q_OK;
+    if (kept) {
+      d.pending_bytes += size;
+      d.kept += size;
+      return B200Q_OK;
+    }
   }
   B200Q_CHECK_CUDA(cudaFree(device_ptr));
   return B200Q_OK;
@@ -147,7 +166,7 @@ extern "C" int b200q_pool_trim(void) {
 extern "C" int b200q_linear(const b200q_linear_desc* l, const void* x, int dtype, int m, void** y, void* stream) {
   if (!l || !y || m < 0 || (dtype != B200Q_F32 && dtype != B200Q_F16) || (m && !x)) return B200Q_ERR_BAD_ARG;
   const size_t row = (size_t)l->n_out * (dtype == B200Q_F32 ? 4 : 2);
-  int rc = pool_alloc(y, (size_t)m * row, (cudaStream_t)stream);
+  int rc = b200q_pool_alloc(y, (size_t)m * row, stream);
   if (rc != B200Q_OK || m == 0) return rc;
   if (l->dense) rc = b200q_gemv_dense(l->w, l->w_type, l->n_out, l->n_in, m, x, dtype, nullptr, 0.f, l->bias, nullptr, *y, dtype, 0, stream);
   else if (m >= l->gemm_min_rows && l->w_type != B200Q_Q6_K)
