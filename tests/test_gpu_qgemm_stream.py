@@ -47,6 +47,14 @@ def test_rows_against_the_exact_product(typ, m, n_out, n_in, dt, split):
 def test_equal_tiles_of_more_rows(typ, m, split): test_rows_against_the_exact_product(typ, m, 300, 416, np.float32, split)
 
 
+def test_more_rows_than_a_grid_has_along_y():
+  m, n_out, n_in, rng = 8 * 65535 + 9, 16, 32, np.random.default_rng(1)
+  lin = quant.QuantLinear(n_in, n_out, 8, synth.q8_0_blocks(n_out, n_in, rng))
+  x = rng.standard_normal((m, n_in)).astype(np.float32)
+  got, w = lin(DeviceBuffer.from_numpy(x)).numpy(), lin.weight.dequantize().numpy().astype(np.float64)
+  assert (np.abs(got - x @ w.T) <= 2.0 ** -20 * (np.abs(x) @ np.abs(w).T)).all()      # six rounded sums and the rounding of the halves, as above
+
+
 @pytest.mark.parametrize("typ,m,n_out,n_in", [(2, 1, 64, 32), (8, 1, 1536, 1024), (8, 52, 130, 128), (2, 200, 512, 992)])
 def test_unsplit_sums_have_the_bits_of_the_kernel_without_a_workspace(typ, m, n_out, n_in):
   rng = np.random.default_rng(m)

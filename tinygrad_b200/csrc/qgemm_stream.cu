@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_rows_kernel(const T* __re
   const int tid = threadIdx.x;
   if (blockIdx.x == 0 && blockIdx.y == 0)
     for (int i = tid; i < n_counters; i += SPLIT_THREADS) counters[i] = 0;
-  const int r = tid & 7, row = blockIdx.y * 8 + r;                       // row within the padded rows of all tiles
+  const int r = tid & 7, row = blockIdx.x * 8 + r;                       // row within the padded rows of all tiles
   const int tile = row / nt, in_tile = row - tile * nt;
   const bool live = row < m;
   float sc = 1.f;
@@ -93,10 +93,10 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_rows_kernel(const T* __re
     for (int i = 0; i < SPLIT_THREADS / 32; i++) tot += red[i][r];
     sc = 1.0f / sqrtf(tot / (float)n_in + eps);
   }
-  const int n_chunks = kgroups * 16, c1 = min(n_chunks, (int)(blockIdx.x + 1) * chunks_per_cta);
+  const int n_chunks = kgroups * 16, c1 = min(n_chunks, (int)(blockIdx.y + 1) * chunks_per_cta);
   const size_t row_bytes = (F32 ? 2 : 1) * (size_t)nt * 16;               // one chunk of a step
   unsigned char* base = xt + (size_t)tile * n_chunks * row_bytes + (size_t)in_tile * 16;
-  for (int c = blockIdx.x * chunks_per_cta + (tid >> 3); c < c1; c += SPLIT_THREADS / 8) {
+  for (int c = blockIdx.y * chunks_per_cta + (tid >> 3); c < c1; c += SPLIT_THREADS / 8) {
     const int k = c * 8;
     float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     unsigned char* dst = base + (size_t)c * row_bytes;
@@ -636,7 +636,7 @@ int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtyp
   // one CTA of the splitting kernel: 8 rows x the whole width, or a part of it where there are few rows
   const int row_groups = pl.tok_tiles * pl.nt / 8, n_chunks = kgroups * 16;
   const int parts = row_groups >= n_sm ? 1 : (row_groups * 4 >= n_sm || n_chunks < 256 ? 4 : 8), per = ceil_div(n_chunks, parts);
-  const dim3 sgrid(ceil_div(n_chunks, per), row_groups);
+  const dim3 sgrid(row_groups, ceil_div(n_chunks, per));      // rows along x: y ends at 65535
   if (f32) B200Q_CHECK_CUDA(launch_k(split_rows_kernel<float>, sgrid, dim3(SPLIT_THREADS), 0, st, pdl, (const float*)x, (const __half*)norm_weight, norm_eps, m,
                                      n_in, kgroups, pl.nt, per, (unsigned char*)p.xt, p.counters, split ? grid : 0));
   else B200Q_CHECK_CUDA(launch_k(split_rows_kernel<__half>, sgrid, dim3(SPLIT_THREADS), 0, st, pdl, (const __half*)x, (const __half*)nullptr, 0.f, m, n_in,
