@@ -102,6 +102,14 @@ def test_bad_arguments_are_rejected_without_a_device(lib):
   assert lib.b200q_graph_begin(None) == -1
 
 
+def test_fp8_linear_refuses_what_its_vector_loads_cannot_take(lib):
+  d = _lib.Fp8LinearDesc(256, 128, 256, 16, 16, 16, 20, 16, 16, 16, 16, 16)      # the bias is read 16 bytes at a time
+  y = ctypes.c_void_p()
+  assert lib.b200q_fp8_linear(ctypes.byref(d), 16, _lib.F32, 4, ctypes.byref(y), None) == -3 and not y.value
+  d.bias, d.n_out = 32, 200
+  assert lib.b200q_fp8_linear(ctypes.byref(d), 16, _lib.F32, 4, ctypes.byref(y), None) == -2 and not y.value
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
   monkeypatch.setattr(_lib, "_lib", None)
   monkeypatch.setattr(_lib, "LIB_PATH", tmp_path / "nope.so")
