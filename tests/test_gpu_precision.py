@@ -33,15 +33,9 @@ def test_activation_codes_are_the_rounded_quotients():
   np.testing.assert_array_equal(got, codes)
 
 
-@pytest.mark.parametrize("kv", [np.float16, np.float32])
-@pytest.mark.parametrize("n_heads,n_kv,hd", [(8, 2, 128), (8, 2, 64)])
-def test_decode_attention_rounds_to_nearest(n_heads, n_kv, hd, kv):
-  """Far into a context, where a tensor core that truncates its running sums (always towards zero) is 4.6e-7 (fp16 cache) to 2.4e-6 (fp32 cache) off.  Sums
-  rounded to nearest add up like a random walk: 55 chunks, 8 partial sums a score and 4 or 8 a chunk stay within 6 x 2^-24 of the output's norm."""
-  rng = np.random.default_rng(hd)
-  pos, ctx, lib = 3507, 3520, _lib.load()
-  qkv = rng.standard_normal((n_heads + 2 * n_kv, hd)).astype(np.float32)
-  kc, vc = (rng.standard_normal((n_kv, ctx, hd)).astype(kv) for _ in range(2))
+def decode_attention(qkv, kc, vc, n_heads, pos):
+  """b200q_attn_decode at `pos` without rotation, and the exact result."""
+  (n_kv, ctx, hd), kv, lib = kc.shape, kc.dtype, _lib.load()
   rope = np.concatenate([np.ones((ctx, hd // 2)), np.zeros((ctx, hd // 2))], 1).astype(np.float32)
   q, k, v = (a.astype(np.float64) for a in (qkv[:n_heads], qkv[n_heads:n_heads + n_kv].astype(kv), qkv[n_heads + n_kv:].astype(kv)))
   rep = lambda c, new: np.repeat(np.concatenate([c[:, :pos].astype(np.float64), new[:, None]], 1), n_heads // n_kv, 0)
@@ -53,7 +47,34 @@ def test_decode_attention_rounds_to_nearest(n_heads, n_kv, hd, kv):
   scratch = DeviceBuffer(lib.b200q_attn_scratch_bytes(n_heads, n_kv, hd, n_split), zero=True)
   a = _lib.AttnArgs(d[0].ptr, d[1].ptr, d[2].ptr, _lib.F16 if kv == np.float16 else _lib.F32, d[3].ptr, d[4].ptr, out.ptr, scratch.ptr, n_heads, n_kv, hd, hd, ctx, n_split, 0, None)
   _lib.check(lib.b200q_attn_decode(ctypes.byref(a), None))
-  assert np.linalg.norm(out.numpy() - want) <= 6 * 2.0 ** -24 * np.linalg.norm(want)
+  return out.numpy(), want
+
+
+@pytest.mark.parametrize("kv", [np.float16, np.float32])
+@pytest.mark.parametrize("n_heads,n_kv,hd", [(8, 2, 128), (8, 2, 64)])
+def test_decode_attention_rounds_to_nearest(n_heads, n_kv, hd, kv):
+  """Far into a context, where a tensor core that truncates its running sums (always towards zero) is 4.6e-7 (fp16 cache) to 2.4e-6 (fp32 cache) off.  Sums
+  rounded to nearest add up like a random walk: 55 chunks, 8 partial sums a score and 4 or 8 a chunk stay within 6 x 2^-24 of the output's norm."""
+  rng = np.random.default_rng(hd)
+  qkv = rng.standard_normal((n_heads + 2 * n_kv, hd)).astype(np.float32)
+  got, want = decode_attention(qkv, *(rng.standard_normal((n_kv, 3520, hd)).astype(kv) for _ in range(2)), n_heads, 3507)
+  assert np.linalg.norm(got - want) <= 6 * 2.0 ** -24 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("n_heads,n_kv,hd", [(8, 1, 128), (6, 2, 64)])
+def test_decode_attention_takes_queries_of_any_magnitude(n_heads, n_kv, hd):
+  """Heads from far below to far above fp16's range, each against keys that make scores of order one of it; a head that is not a number stays none."""
+  rng, pos = np.random.default_rng(n_heads), 70
+  qkv, kc, vc = rng.standard_normal((n_heads + 2 * n_kv, hd)).astype(np.float32), *(rng.standard_normal((n_kv, 128, hd)).astype(np.float16) for _ in range(2))
+  for up, down in ((2.0 ** 17, 2.0 ** -12), (2.0 ** -18, 2.0 ** 12)):
+    x = qkv.copy()
+    x[:n_heads] *= np.float32(up); x[n_heads:n_heads + n_kv] *= np.float32(down)
+    got, want = decode_attention(x, (kc.astype(np.float32) * np.float32(down)).astype(np.float16), vc, n_heads, pos)
+    # the scores' error is 2^-22 of their size, which is up to 2^5 times that of the test above
+    assert np.isfinite(got).all() and np.linalg.norm(got - want) <= 2.0 ** -17 * np.linalg.norm(want)
+  qkv[1, 3] = np.nan
+  got, _ = decode_attention(qkv, kc, vc, n_heads, pos)
+  assert np.isnan(got[1]).all() and np.isfinite(np.delete(got, 1, 0)).all()
 
 
 @pytest.mark.parametrize("typ", [12, 14])

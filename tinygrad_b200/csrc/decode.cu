@@ -437,10 +437,10 @@ __device__ __forceinline__ float ld_cluster(uint32_t local, uint32_t rank) {    
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// fp16 high part (finite for any input) and the remainder's fp16 rounding
+// fp16 high part and the remainder's fp16 rounding
 __device__ __forceinline__ void split_h(float v, __half& hi, __half& lo) {
-  hi = __float2half_rn(fminf(fmaxf(v, -65504.f), 65504.f));
-  lo = __float2half_rn(fminf(fmaxf(v - __half2float(hi), -65504.f), 65504.f));
+  hi = __float2half_rn(v);
+  lo = __float2half_rn(v - __half2float(hi));
 }
 
 // value d of a row, split in two rows of operand values
@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
   float* s_s = reinterpret_cast<float*>(asmem + M::S);            // [8][64 + 4] scores
   float* s_o = reinterpret_cast<float*>(asmem + M::O);            // [8][HD] this CTA's unnormalised output
   float* s_m = reinterpret_cast<float*>(asmem + M::ST);           // [8] running max, [8] denominator, [8] rescale factor
-  float *s_l = s_m + 8, *s_c = s_m + 16;
+  float *s_l = s_m + 8, *s_c = s_m + 16, *s_q = s_m + 24;        // [8] what a head's scores are multiplied with
   KV* s_new = reinterpret_cast<KV*>(asmem + M::NEW);              // the new position's K and V rows
   KV* kc = reinterpret_cast<KV*>(a.k_cache) + (size_t)kvh * a.max_context * HD;
   KV* vc = reinterpret_cast<KV*>(a.v_cache) + (size_t)kvh * a.max_context * HD;
@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
   start(pos_early);
   if (tid * 32 < a.rope_dim) prefetch_l2(a.rope + (size_t)pos_early * a.rope_dim + tid * 32);
   for (int i = tid; i < (16 * M::QROW + 16 * M::PROW) / 16; i += AC_THREADS) reinterpret_cast<uint4*>(asmem + M::Q)[i] = make_uint4(0, 0, 0, 0);   // rows of absent heads
-  if (tid < 8) { s_m[tid] = -INFINITY; s_l[tid] = 0.f; }
+  if (tid < 8) { s_m[tid] = -INFINITY; s_l[tid] = 0.f; s_q[tid] = 0.f; }
   __syncthreads();
   pdl_wait();
   const int pos = __ldcg(a.pos);
@@ -538,9 +538,20 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
     return v[d];
   };
   if (c0 < c1) {
-    for (int i = tid; i < n_rep * HD; i += AC_THREADS) {
-      const int r = i / HD, d = i - r * HD;
-      store_split<KV>(roped(a.qkv + (size_t)(kvh * n_rep + r) * HD, d), asmem + M::Q + r * M::QROW, asmem + M::Q + (8 + r) * M::QROW, d);
+    if (warp < n_rep) {                                            // a warp takes a query head; fp16: under a power of two of its own
+      const float* src = a.qkv + (size_t)(kvh * n_rep + warp) * HD;
+      float v[HD / 32], up = 1.f, down = 1.f;
+#pragma unroll
+      for (int j = 0; j < HD / 32; j++) v[j] = roped(src, lane + 32 * j);
+      if constexpr (!F32) {
+        float amax = 0.f;
+#pragma unroll
+        for (int j = 0; j < HD / 32; j++) amax = fmaxf(amax, fabsf(v[j]));
+        pow2_scale(warp_max(amax), up, down);
+      }
+#pragma unroll
+      for (int j = 0; j < HD / 32; j++) store_split<KV>(v[j] * up, asmem + M::Q + warp * M::QROW, asmem + M::Q + (8 + warp) * M::QROW, lane + 32 * j);
+      if (lane == 0) s_q[warp] = down * (1.0f / sqrtf((float)HD));
     }
     if (owner) {
       for (int i = tid; i < 2 * HD; i += AC_THREADS) {
@@ -555,7 +566,6 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
   float acc[HD / 64][4];                                             // this warp's HD / 8 output dims: rows g (high parts) and g + 8 (low parts)
 #pragma unroll
   for (int j = 0; j < HD / 64; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-  const float scale = 1.0f / sqrtf((float)HD);
   for (int ch = c0; ch < c1; ch++) {
     const int buf = (ch - c0) & 1, nv = min(AC_POS, pos + 1 - ch * AC_POS);
     unsigned char* sk = asmem + buf * M::BUF;
@@ -592,7 +602,7 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
         }
       }
       const int p = warp * 8 + 2 * t;
-      const float s0 = ((c[0] + c2[0]) + (c[2] + c2[2])) * scale, s1 = ((c[1] + c2[1]) + (c[3] + c2[3])) * scale;
+      const float scale = s_q[g], s0 = ((c[0] + c2[0]) + (c[2] + c2[2])) * scale, s1 = ((c[1] + c2[1]) + (c[3] + c2[3])) * scale;
       s_s[g * (AC_POS + 4) + p] = p < nv ? s0 : -INFINITY;
       s_s[g * (AC_POS + 4) + p + 1] = p + 1 < nv ? s1 : -INFINITY;
     }
