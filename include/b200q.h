@@ -386,12 +386,15 @@ int b200q_qgemm(int qtype, const void* w_packed, const void* x, int x_dtype, con
                 int y_dtype, int m, int n_out, int n_in, void* stream);
 /* The same Linear with a workspace: the activations are first split once into fp16 hi / lo tiles, which the GEMM's CTAs read by bulk
  * copies.  workspace: 16-byte aligned, contents are scratch; b200q_qgemm_workspace_bytes(m, n_in) bytes are enough to run, with
- * b200q_qgemm_workspace_bytes_for(m, n_out, n_in) (n_out = 0: for any) tiles may also be split along K, which deals the work evenly over the
+ * b200q_qgemm_unsplit_workspace_bytes(m, n_in) fp32 rows whose largest value is from 2^15 on (or, with tiles split, below 1) are scaled by a power of two first
+ * (unscaled, values past 65504 overflow, and what a row loses is 2^-25 absolute instead of relative to its largest value), with
+ * b200q_qgemm_workspace_bytes_for(m, n_out, n_in) (n_out = 0: for any) tiles may besides be split along K, which deals the work evenly over the
  * SMs; their partial sums are added in the order of K, so the result does not depend on timing.  Same arguments, same numerics (the order
  * of the fp32 additions aside), same epilogues.  Two launches.  b200q_qgemm_ws_norm (fp32 x): norm_weight fp16 [n_in], the RMSNorm in
- * front of the Linear, applied while x is split (NULL: none); unsplit != 0: tiles are never split, every output is one running sum with the bits of
- * b200q_qgemm. */
+ * front of the Linear, applied while x is split (NULL: none); unsplit != 0: tiles are never split, every output is one running sum, with the bits of
+ * b200q_qgemm where the row is not scaled. */
 size_t b200q_qgemm_workspace_bytes(int m, int n_in);
+size_t b200q_qgemm_unsplit_workspace_bytes(int m, int n_in);
 size_t b200q_qgemm_workspace_bytes_for(int m, int n_out, int n_in);
 int b200q_qgemm_ws(int qtype, const void* w_packed, const void* x, int x_dtype, const void* bias_f16, const void* residual, int epilogue, void* y,
                    int y_dtype, int m, int n_out, int n_in, void* workspace, size_t workspace_bytes, void* stream);

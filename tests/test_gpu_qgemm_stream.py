@@ -79,3 +79,25 @@ def test_norm_in_front_and_swiglu_behind():
   # each factor is good to 2^-18 of its largest value (the bound above at 512 columns); |d silu| <= 1.1
   tol = 2.0 ** -18 * (1.1 * np.abs(g).max() * np.abs(u) + np.abs(g) * np.abs(u).max() + 1)
   assert (np.abs(y.numpy() - ref) <= tol).all()
+
+
+@pytest.mark.parametrize("typ,m,n_out,n_in,split", [(2, 5, 300, 4096, True), (8, 70, 1000, 992, True), (8, 70, 300, 14336, True), (2, 300, 130, 512, False)])
+def test_rows_of_any_magnitude(typ, m, n_out, n_in, split):
+  """Rows far outside fp16's range lose no more than others: the bound of the exact product for each row by itself; and the same behind a norm weight that leads
+  out of it."""
+  rng = np.random.default_rng(m)
+  raw = synth.BLOCK_MAKERS[typ](n_out, n_in, rng)
+  w, pw = gq.weight_matrix(raw, n_out, n_in, typ).astype(np.float64), quant.repack(raw, n_out, n_in, typ)
+  mag = np.concatenate([[0, 1e-30, 3e4, 1e30], 10.0 ** rng.uniform(-20, 20, m - 4)])[:, None]
+  if not split: mag = np.maximum(mag, 1)      # smaller rows keep the bits of the form without a workspace there
+  x = (rng.standard_normal((m, n_in)) * mag).astype(np.float32)
+  y, ws = DeviceBuffer.empty((m, n_out), np.float32), DeviceBuffer(quant.qgemm_workspace_bytes(m, n_in, n_out) if split else quant.qgemm_unsplit_workspace_bytes(m, n_in))
+  quant.qgemm(pw.buf.ptr, typ, n_out, n_in, DeviceBuffer.from_numpy(x), y, m, workspace=ws, unsplit=not split)
+  bound = (2.0 ** -21 + 3 * np.ceil(n_in / 16) * 2.0 ** -23) * (np.abs(x).astype(np.float64) @ np.abs(w).T)
+  assert (np.abs(y.numpy() - x.astype(np.float64) @ w.T) <= bound).all()
+  nw, x = (2e4 * (1 + 0.1 * rng.standard_normal(n_in))).astype(np.float16), rng.standard_normal((m, n_in)).astype(np.float32)
+  quant.qgemm(pw.buf.ptr, typ, n_out, n_in, DeviceBuffer.from_numpy(x), y, m, workspace=ws, unsplit=not split, norm_weight=DeviceBuffer.from_numpy(nw), norm_eps=1e-5)
+  xn = x.astype(np.float64) / np.sqrt((x.astype(np.float64) ** 2).mean(1, keepdims=True) + 1e-5) * nw.astype(np.float64)
+  # ... the norm's own rounding: a few units of 2^-24
+  bound = (2.0 ** -20 + 3 * np.ceil(n_in / 16) * 2.0 ** -23) * (np.abs(xn) @ np.abs(w).T)
+  assert (np.abs(y.numpy() - xn @ w.T) <= bound).all()

@@ -153,6 +153,7 @@ SIGNATURES = {
   "b200q_gemm_f16": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
   "b200q_qgemm": (c_int, [c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
   "b200q_qgemm_workspace_bytes": (c_size_t, [c_int, c_int]),
+  "b200q_qgemm_unsplit_workspace_bytes": (c_size_t, [c_int, c_int]),
   "b200q_qgemm_workspace_bytes_for": (c_size_t, [c_int, c_int, c_int]),
   "b200q_qgemm_ws_norm": (c_int, [c_int, c_void_p, c_void_p, c_int, c_void_p, c_float, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p,
                                  c_size_t, c_int, c_void_p]),

@@ -110,6 +110,18 @@ __device__ __forceinline__ bool elect_one() {
 // Ask for a line that will be read behind pdl_wait (weights, tables): in a model whose weights exceed L2 it is a DRAM miss by then.
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
+// ---- thread-block clusters ----
+__device__ __forceinline__ float ld_cluster(uint32_t local, uint32_t rank) {      // the same shared-memory word of another CTA of the cluster
+  uint32_t a;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // The power of two that puts a largest magnitude into [2^13, 2^14), where fp16 holds a value and the remainder's rounding to 2^-22 of it and to 2^-38 of
 // the largest, and its inverse; zeros get the inverse 0, infinities (and NaN) are left as they are.
 __device__ __forceinline__ void pow2_scale(float amax, float& up, float& down) {

@@ -5,6 +5,9 @@
 // Numerics: fp32 activations are split into fp16 halves x = xh + xl, the dequantised weight into w = wh + wl (wh the fp16 product of
 // quant and scale, wl its exact remainder), and y = wh xh + wh xl + wl xh is accumulated in fp32 on the tensor cores: the fp32
 // activation times the unrounded weight to about 2^-22.  fp16 activations take one pass with the fp16-rounded weight.
+// A row of fp32 activations whose largest value lies outside [1, 2^15) is scaled by a power of two first, which its outputs give back: above that the halves
+// overflow (a value past 65504 made a row of NaN), below it their absolute floor of 2^-25 shows against the row's values.  In between, and with `unsplit` everywhere
+// below 2^15, the halves are those of b200q_qgemm, bit for bit.
 //
 // What bounds it: three fp16 tensor passes for many rows; for few rows the weight stream and the unpacking.  So
 //  * weights are the MMA's A operand (128 rows per instruction) and the activation rows its N: any row count rounded up to 16 fills the
@@ -44,6 +47,7 @@ constexpr size_t COUNTER_BYTES = 4096;                  // one arrival counter p
 struct StreamParams {
   const uint8_t* w;
   const unsigned char* xt;       // activation tiles (split_rows)
+  const float* down;             // per activation row: what undoes its scaling (NULL: rows are not scaled)
   float* part;
   unsigned* counters;
   const __half* bias;
@@ -60,14 +64,17 @@ struct StreamParams {
 // workspace: per activation tile of nt rows and K step of 32: [4 chunks of 8 columns][nt rows hi | nt rows lo][16 bytes], contiguous, so
 // that a step's operand is one bulk copy.  Element order inside a chunk: [0,2,1,3,4,6,5,7], the order the weight unpack delivers.
 // One CTA: 8 rows (a core matrix) x a stretch of columns; a row's chunk is 32 bytes in, 16 + 16 bytes out, 8 rows make 128 contiguous bytes.
+// What is asked of a whole row first (its mean square for the norm, its largest value for the scale) the CTAs of a row's stretches share as a cluster, each
+// reading its own (CLUSTER; rows of 2048 and more); of short rows each reads all.  16 8B-shaped blocks, a prompt of 45: 4560 us with every CTA reading its
+// whole rows for the norm alone, 4211 so with both; 6900 with every CTA reading its whole rows for both.
 constexpr int SPLIT_THREADS = 256;
 
-template <typename T>
+template <typename T, bool CLUSTER>
 __global__ void __launch_bounds__(SPLIT_THREADS) split_rows_kernel(const T* __restrict__ x, const __half* __restrict__ norm_w, float eps, int m, int n_in,
                                                                    int kgroups, int nt, int chunks_per_cta, unsigned char* __restrict__ xt,
-                                                                   unsigned* __restrict__ counters, int n_counters) {
+                                                                   unsigned* __restrict__ counters, int n_counters, float* __restrict__ down, float lowest) {
   constexpr bool F32 = sizeof(T) == 4;
-  __shared__ float red[SPLIT_THREADS / 32][8];
+  __shared__ float red[SPLIT_THREADS / 32][8], red_max[SPLIT_THREADS / 32][8];
   pdl_wait();
   pdl_launch_dependents();
   const int tid = threadIdx.x;
@@ -76,27 +83,58 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_rows_kernel(const T* __re
   const int r = tid & 7, row = blockIdx.x * 8 + r;                       // row within the padded rows of all tiles
   const int tile = row / nt, in_tile = row - tile * nt;
   const bool live = row < m;
-  float sc = 1.f;
-  if (F32 && norm_w) {
-    float ss = 0.f;
-    if (live)
-      for (int k = (tid >> 3) * 4; k < n_in; k += SPLIT_THREADS / 8 * 4) {
-        const float4 a = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(x) + (size_t)row * n_in + k);
-        ss = fmaf(a.x, a.x, fmaf(a.y, a.y, fmaf(a.z, a.z, fmaf(a.w, a.w, ss))));
+  float sc = 1.f, up = 1.f;
+  const int n_chunks = kgroups * 16, c0 = blockIdx.y * chunks_per_cta, c1 = min(n_chunks, c0 + chunks_per_cta);
+  if (F32 && (norm_w || down)) {                                          // the row's mean square and its largest value
+    float ss = 0.f, amax = 0.f;
+    if (live) {
+      const float* src = reinterpret_cast<const float*>(x) + (size_t)row * n_in;
+      const int k1 = CLUSTER ? min(n_in, c1 * 8) : n_in;
+      constexpr int STEP = SPLIT_THREADS / 8 * 4, BATCH = 4;              // loads in flight
+      for (int k0 = (CLUSTER ? c0 * 8 : 0) + (tid >> 3) * 4; k0 < k1; k0 += BATCH * STEP) {
+        float4 a[BATCH];
+        uint2 nw[BATCH];
+#pragma unroll
+        for (int i = 0; i < BATCH; i++) {
+          const int k = k0 + i * STEP;
+          a[i] = k < k1 ? *reinterpret_cast<const float4*>(src + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+          nw[i] = norm_w && k < k1 ? *reinterpret_cast<const uint2*>(norm_w + k) : make_uint2(0x3C003C00u, 0x3C003C00u);      // fp16 ones
+        }
+#pragma unroll
+        for (int i = 0; i < BATCH; i++) {
+          const float2 w0 = __half22float2(*reinterpret_cast<const __half2*>(&nw[i].x)), w1 = __half22float2(*reinterpret_cast<const __half2*>(&nw[i].y));
+          ss = fmaf(a[i].x, a[i].x, fmaf(a[i].y, a[i].y, fmaf(a[i].z, a[i].z, fmaf(a[i].w, a[i].w, ss))));
+          amax = fmaxf(amax, fmaxf(fmaxf(fabsf(a[i].x * w0.x), fabsf(a[i].y * w0.y)), fmaxf(fabsf(a[i].z * w1.x), fabsf(a[i].w * w1.y))));
+        }
       }
+    }
     ss += __shfl_xor_sync(0xffffffffu, ss, 8);
     ss += __shfl_xor_sync(0xffffffffu, ss, 16);
-    if ((tid & 31) < 8) red[tid >> 5][r] = ss;
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 8));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 16));
+    if ((tid & 31) < 8) { red[tid >> 5][r] = ss; red_max[tid >> 5][r] = amax; }
     __syncthreads();
     float tot = 0.f;
 #pragma unroll
-    for (int i = 0; i < SPLIT_THREADS / 32; i++) tot += red[i][r];
-    sc = 1.0f / sqrtf(tot / (float)n_in + eps);
+    for (int i = 0; i < SPLIT_THREADS / 32; i++) { tot += red[i][r]; amax = fmaxf(amax, red_max[i][r]); }
+    if (CLUSTER) {                                                        // with the other stretches of the rows
+      __syncthreads();
+      if (tid < 8) { red[0][r] = tot; red_max[0][r] = amax; }
+      __syncwarp();
+      cluster_sync();
+      tot = 0.f;
+      for (uint32_t c = 0; c < gridDim.y; c++) { tot += ld_cluster(s32(&red[0][r]), c); amax = fmaxf(amax, ld_cluster(s32(&red_max[0][r]), c)); }
+    }
+    if (norm_w) { sc = 1.0f / sqrtf(tot / (float)n_in + eps); amax *= sc; }
+    if (down) {
+      float inv = 1.f;
+      if (!(amax >= lowest && amax < 32768.f)) pow2_scale(amax, up, inv);
+      if (blockIdx.y == 0 && tid < 8) down[row] = inv;
+    }
   }
-  const int n_chunks = kgroups * 16, c1 = min(n_chunks, (int)(blockIdx.y + 1) * chunks_per_cta);
   const size_t row_bytes = (F32 ? 2 : 1) * (size_t)nt * 16;               // one chunk of a step
   unsigned char* base = xt + (size_t)tile * n_chunks * row_bytes + (size_t)in_tile * 16;
-  for (int c = blockIdx.y * chunks_per_cta + (tid >> 3); c < c1; c += SPLIT_THREADS / 8) {
+  for (int c = c0 + (tid >> 3); c < c1; c += SPLIT_THREADS / 8) {
     const int k = c * 8;
     float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     unsigned char* dst = base + (size_t)c * row_bytes;
@@ -116,12 +154,16 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_rows_kernel(const T* __re
 #pragma unroll
         for (int q = 0; q < 4; q++) { const float2 t2 = __half22float2(h[q]); f[2 * q] = f[2 * q] * sc * t2.x; f[2 * q + 1] = f[2 * q + 1] * sc * t2.y; }
       }
+#pragma unroll
+      for (int q = 0; q < 8; q++) f[q] *= up;
     }
     uint4 hi, lo;
     split_chunk(f, hi, lo);
     *reinterpret_cast<uint4*>(dst) = hi;
     *reinterpret_cast<uint4*>(dst + (size_t)nt * 16) = lo;
   }
+  __syncwarp();
+  if (CLUSTER) cluster_sync();                                            // nobody leaves while its sums are being read
 }
 
 // ---- the product ---------------------------------------------------------------------------------------------------------------
@@ -179,7 +221,13 @@ __device__ __forceinline__ size_t part_slot(const StreamParams& p, int c, int ti
 __device__ __forceinline__ int cta_of(long long unit, long long units, int g) { return (int)(((unit + 1) * g - 1) / units); }
 
 // EC consecutive activation rows of one output column (weight row) `feat`
-__device__ __forceinline__ void store_outputs(const StreamParams& p, const float (&v)[EC], int feat, int tok0, int lane) {
+__device__ __forceinline__ void store_outputs(const StreamParams& p, float (&v)[EC], int feat, int tok0, int lane) {
+  if (p.down)
+#pragma unroll
+    for (int j = 0; j < EC; j += 4) {
+      const float4 d = *reinterpret_cast<const float4*>(p.down + tok0 + j);
+      v[j] *= d.x; v[j + 1] *= d.y; v[j + 2] *= d.z; v[j + 3] *= d.w;
+    }
   if (p.silu_mul) {
     // gate rows sit in lanes with bit 3 clear, the matching up rows 8 lanes on: each of a pair takes every other activation row
     const bool gate = !(lane & 8);
@@ -537,6 +585,7 @@ Plan make_plan(int m, int n_out, int n_sm) {
 size_t tiles_bytes(const Plan& pl, int kgroups, bool f32) { return (size_t)pl.tok_tiles * pl.nt * kgroups * GROUP_ELEMS * (f32 ? 4 : 2); }
 int slot_bytes(const Plan& pl, bool f32) { return steps_per_slot(pl.wt, pl.nt) * (pl.wt * KSTEP * 4 + pl.nt * (f32 ? 128 : 64)); }
 size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
+size_t scale_bytes(const Plan& pl) { return align256((size_t)pl.tok_tiles * pl.nt * sizeof(float)); }
 
 template <int QT, int WT, bool F32, int SPS>
 int launch_stream(const StreamParams& p, int grid, cudaStream_t st) {
@@ -567,7 +616,7 @@ static int stream_grid(long long units, int n_sm) {
   return (int)(g < most ? g : most);
 }
 
-// counters and partial sums behind the activation tiles; n_out = 0: enough for any
+// the rows' scales, counters and partial sums behind the activation tiles; n_out = 0: enough for any
 static size_t split_workspace(const Plan& pl, int n_out, int kgroups, int n_sm) {
   long long parts = 2LL * n_sm;
   if (n_out > 0) {
@@ -575,7 +624,7 @@ static size_t split_workspace(const Plan& pl, int n_out, int kgroups, int n_sm) 
     const int grid = stream_grid(tiles * kgroups, n_sm);
     parts = tiles < grid ? grid + tiles : 2 * grid;
   }
-  return COUNTER_BYTES + (size_t)parts * pl.wt * pl.nt * sizeof(float);
+  return scale_bytes(pl) + COUNTER_BYTES + (size_t)parts * pl.wt * pl.nt * sizeof(float);
 }
 
 // Room for the activation tiles: enough to run, tiles then going whole to the CTAs.  Equal tiles of up to 256 rows may hold more rows than m rounded up to 128
@@ -585,6 +634,10 @@ extern "C" size_t b200q_qgemm_workspace_bytes(int m, int n_in) {
   const Plan pl = make_plan(m, 0, 0);
   const size_t rows = std::max((size_t)ceil_div(m, 128) * 128, (size_t)pl.tok_tiles * pl.nt);
   return rows * ceil_div(n_in, GROUP_ELEMS) * GROUP_ELEMS * 4;
+}
+// ... with room for the rows' scales
+extern "C" size_t b200q_qgemm_unsplit_workspace_bytes(int m, int n_in) {
+  return m <= 0 || n_in <= 0 ? 0 : align256(b200q_qgemm_workspace_bytes(m, n_in)) + scale_bytes(make_plan(m, 0, 0));
 }
 extern "C" size_t b200q_qgemm_workspace_bytes_for(int m, int n_out, int n_in) {
   if (m <= 0 || n_in <= 0 || n_out < 0) return 0;
@@ -615,8 +668,9 @@ int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtyp
   StreamParams p;
   p.w = (const uint8_t*)w_packed;
   p.xt = (const unsigned char*)workspace;
-  p.counters = (unsigned*)((unsigned char*)workspace + xt_bytes);
-  p.part = (float*)((unsigned char*)workspace + xt_bytes + COUNTER_BYTES);
+  p.down = f32 && workspace_bytes >= xt_bytes + scale_bytes(pl) ? (const float*)((unsigned char*)workspace + xt_bytes) : nullptr;
+  p.counters = (unsigned*)((unsigned char*)workspace + xt_bytes + scale_bytes(pl));
+  p.part = (float*)((unsigned char*)p.counters + COUNTER_BYTES);
   p.bias = (const __half*)bias_f16; p.residual = residual; p.y = y;
   p.m = m; p.n_out = n_out; p.kgroups = kgroups; p.n_row_tiles = ceil_div(n_out, TILE_ROWS);
   p.nt = pl.nt; p.tok_tiles = pl.tok_tiles;
@@ -637,10 +691,22 @@ int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtyp
   const int row_groups = pl.tok_tiles * pl.nt / 8, n_chunks = kgroups * 16;
   const int parts = row_groups >= n_sm ? 1 : (row_groups * 4 >= n_sm || n_chunks < 256 ? 4 : 8), per = ceil_div(n_chunks, parts);
   const dim3 sgrid(row_groups, ceil_div(n_chunks, per));      // rows along x: y ends at 65535
-  if (f32) B200Q_CHECK_CUDA(launch_k(split_rows_kernel<float>, sgrid, dim3(SPLIT_THREADS), 0, st, pdl, (const float*)x, (const __half*)norm_weight, norm_eps, m,
-                                     n_in, kgroups, pl.nt, per, (unsigned char*)p.xt, p.counters, split ? grid : 0));
-  else B200Q_CHECK_CUDA(launch_k(split_rows_kernel<__half>, sgrid, dim3(SPLIT_THREADS), 0, st, pdl, (const __half*)x, (const __half*)nullptr, 0.f, m, n_in,
-                                 kgroups, pl.nt, per, (unsigned char*)p.xt, p.counters, split ? grid : 0));
+  const bool cluster = f32 && sgrid.y > 1 && n_chunks >= 256;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = sgrid; cfg.blockDim = dim3(SPLIT_THREADS); cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = pdl;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = sgrid.y; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = cluster ? 2 : 1;
+  const int n_counters = split ? grid : 0;
+  if (f32)
+    B200Q_CHECK_CUDA(cudaLaunchKernelEx(&cfg, cluster ? split_rows_kernel<float, true> : split_rows_kernel<float, false>, (const float*)x, (const __half*)norm_weight, norm_eps, m,
+                                        n_in, kgroups, pl.nt, per, (unsigned char*)p.xt, p.counters, n_counters, (float*)p.down, unsplit ? 0.f : 1.f));
+  else
+    B200Q_CHECK_CUDA(cudaLaunchKernelEx(&cfg, split_rows_kernel<__half, false>, (const __half*)x, (const __half*)nullptr, 0.f, m, n_in, kgroups, pl.nt, per,
+                                        (unsigned char*)p.xt, p.counters, n_counters, (float*)nullptr, 0.f));
 #define STREAM_CASE(QT) (pl.wt == 256 ? (f32 ? launch_stream<QT, 256, true, 1>(p, grid, st) : launch_stream<QT, 256, false, 1>(p, grid, st)) \
                          : pl.nt > 64 ? (f32 ? launch_stream<QT, 128, true, 1>(p, grid, st) : launch_stream<QT, 128, false, 1>(p, grid, st)) \
                                       : (f32 ? launch_stream<QT, 128, true, 4>(p, grid, st) : launch_stream<QT, 128, false, 4>(p, grid, st)))

@@ -100,15 +100,15 @@ def qgemm_workspace_bytes(m: int, n_in: int, n_out: int = 0) -> int:
 
 
 def qgemm_unsplit_workspace_bytes(m: int, n_in: int) -> int:
-  """The least scratch the GEMM runs in: no tile is split, every output is one running sum (the same bits as without a workspace)."""
-  return int(_lib.load().b200q_qgemm_workspace_bytes(m, n_in))
+  """Scratch without room for partial sums: no tile is split, every output is one running sum."""
+  return int(_lib.load().b200q_qgemm_unsplit_workspace_bytes(m, n_in))
 
 
 def qgemm(w_ptr: int, qtype: int, n_out: int, n_in: int, x, y, m: int, x_dtype=F32, y_dtype=F32, bias=None, residual=None,
           epilogue: int = EPI_LINEAR, stream=None, workspace: DeviceBuffer = None, norm_weight=None, norm_eps: float = 0.0, unsplit: bool = False) -> None:
   """Batched / prefill linear on the tcgen05 tensor cores.  With a `workspace` (qgemm_workspace_bytes(m, n_in) bytes) the streaming kernel
   runs: activations split once (with the RMSNorm in front, if its weight is given), roles on separate warps, even deal over the SMs.
-  unsplit: no tile's K is split over SMs, every output is one running sum with the bits of the form without a workspace."""
+  unsplit: no tile's K is split over SMs, every output is one running sum."""
   lib = _lib.load()
   if workspace is not None and PIPELINED_GEMM:
     check(lib.b200q_qgemm_ws_norm(qtype, w_ptr, ptr_of(x), x_dtype, ptr_of(norm_weight), norm_eps, ptr_of(bias), ptr_of(residual), epilogue, ptr_of(y), y_dtype,
