@@ -46,16 +46,16 @@ def test_layer_is_its_parts(sizes):
   np.testing.assert_array_equal(got, layer._workspace(T)["out"].numpy())
 
 
-# a row tile of CTA pairs per group / half-empty last tiles / one K step, and more K steps than the ring has stages / several column tiles
-@pytest.mark.parametrize("E,rows,n,k", [(1, 256, 256, 128), (2, 512, 512, 640), (3, 768, 256, 2048)])
-def test_pair_gemm(E, rows, n, k):
-  """Groups of 256 rows and more go to pairs of CTAs: every row against the oracle (fp32 sums of at most k products, then one rounding to bf16)."""
+# one group / empty groups first, between and last / one K step, more K steps than the ring has stages / more tiles than SMs, several tiles of one group on a CTA
+@pytest.mark.parametrize("sizes,n,k", [([256], 256, 128), ([0, 512, 0, 256, 0], 512, 640), ([256, 256, 256], 256, 2048), ([2560, 0, 768], 1536, 256)])
+def test_grouped_gemm(sizes, n, k):
+  """Every row of every group against the oracle (fp32 sums of at most k products, then one rounding to bf16); rows behind the last group are left alone."""
   need_gpu()
   from tinygrad_b200 import _lib, moe
   from tinygrad_b200.runtime import DeviceBuffer
   rng = np.random.default_rng(n + k)
-  m = E * rows + (256 * E if E > 1 else 0)                        # room for padding, as the routing sizes it
-  off = (np.arange(E + 1) * rows).astype(np.int32)
+  E, off = len(sizes), np.cumsum([0, *sizes]).astype(np.int32)
+  m = int(off[-1]) + 256                                          # room behind the groups, as the routing leaves it
   aq, ae = mx.quantize_mxfp8(rng.standard_normal((m, k)).astype(np.float32))
   bq, be = mx.quantize_mxfp8((rng.standard_normal((E * n, k)) * np.exp(rng.uniform(-3, 3, (E * n, 1)))).astype(np.float32))
   c = DeviceBuffer.empty((m, n), np.uint16, zero=True)

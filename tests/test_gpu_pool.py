@@ -15,14 +15,18 @@ def _gpu(): need_gpu()
 
 
 def test_a_result_keeps_its_values_while_later_calls_allocate():
-  """Results are dropped right after a copy of them was queued on another stream: with blocks handed out too early a later result would be copied."""
+  """Results are dropped right after a copy of them was queued on another stream, behind milliseconds of other copies: with blocks handed out too early a later
+  result would be copied."""
   rng = np.random.default_rng(0)
   lin = quant.QuantLinear(512, 300, 2, synth.q4_0_blocks(300, 512, rng))
   xs = [DeviceBuffer.from_numpy(rng.standard_normal((8, 512)).astype(np.float32)) for _ in range(7)]
   want = [lin(x).numpy() for x in xs]
   st, copy = runtime.Stream(), runtime.Stream()
   out, lib = DeviceBuffer.empty((300, 8, 300), np.float32), _lib.load()
+  far = [DeviceBuffer(256 << 20) for _ in range(2)]
   for i in range(300):
+    if i % 30 == 0:
+      for _ in range(40): _lib.check(lib.b200q_memcpy_d2d(far[0].ptr, far[1].ptr, far[0].nbytes, copy.ptr))
     y = lin(xs[i % 7], stream=st)
     st.synchronize()
     _lib.check(lib.b200q_memcpy_d2d(out.ptr + i * y.nbytes, y.ptr, y.nbytes, copy.ptr))
