@@ -130,15 +130,16 @@ __device__ __forceinline__ void load8f(const float* p, float (&f)[8]) {
   f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
 }
 // Eight values of a row held by HD / 8 consecutive lanes (whole warps take part) -> fp16 halves of the scaled row; returns the power of two that undoes the
-// scaling, 0 for a row of zeros.
-template <int HD>
+// scaling, 0 for a row of zeros.  NEAR: a row whose largest value is in [1, 2^15) is left as it is (queries: the halves' floor of 2^-25 is 2^-25 of the row there, and
+// a mixture-of-experts model's expert choice hangs on the last bit of what it has always computed).
+template <int HD, bool NEAR = false>
 __device__ __forceinline__ float stage_row(const float (&f)[8], __half* hi, __half* lo) {
   float amax = 0.f, up, down;
 #pragma unroll
   for (int j = 0; j < 8; j++) amax = fmaxf(amax, fabsf(f[j]));
 #pragma unroll
   for (int o = 1; o < HD / 8; o *= 2) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  pow2_scale(amax, up, down);
+  if (NEAR && amax >= 1.f && amax < 32768.f) up = down = 1.f; else pow2_scale(amax, up, down);
   uint32_t h[4], l[4];
 #pragma unroll
   for (int j = 0; j < 4; j++) split_pair(f[2 * j] * up, f[2 * j + 1] * up, h[j], l[j]);
@@ -185,7 +186,7 @@ __global__ void __launch_bounds__(PF_THREADS) attn_prefill_kernel(const float* _
     const int r = i / (HD / 8), c = (i - r * (HD / 8)) * 8;
     float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (q0 + r < rows_end) load8f(q + ((size_t)(q0 + r) * n_heads + head) * HD + c, f);
-    const float down = stage_row<HD>(f, s_q + r * STRIDE + c, s_q + (PQ + r) * STRIDE + c);
+    const float down = stage_row<HD, true>(f, s_q + r * STRIDE + c, s_q + (PQ + r) * STRIDE + c);
     if (c == 0) s_qd[r] = down;
   }
   __syncthreads();
