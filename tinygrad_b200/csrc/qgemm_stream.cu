@@ -64,17 +64,33 @@ struct StreamParams {
 // workspace: per activation tile of nt rows and K step of 32: [4 chunks of 8 columns][nt rows hi | nt rows lo][16 bytes], contiguous, so
 // that a step's operand is one bulk copy.  Element order inside a chunk: [0,2,1,3,4,6,5,7], the order the weight unpack delivers.
 // One CTA: 8 rows (a core matrix) x a stretch of columns; a row's chunk is 32 bytes in, 16 + 16 bytes out, 8 rows make 128 contiguous bytes.
-// What is asked of a whole row first (its mean square for the norm, its largest value for the scale) the CTAs of a row's stretches share as a cluster, each
-// reading its own (CLUSTER; rows of 2048 and more); of short rows each reads all.  16 8B-shaped blocks, a prompt of 45: 4560 us with every CTA reading its
-// whole rows for the norm alone, 4211 so with both; 6900 with every CTA reading its whole rows for both.
-constexpr int SPLIT_THREADS = 256;
+// What is asked of a whole row (its mean square for the norm, its largest value for the scale) the CTAs of a row's stretches share as a cluster; stretches of up
+// to 2048 columns are read once and kept in registers, so rows that short need no cluster.  A prompt of 45 on 16 8B-shaped blocks: 3734 us; rows read twice, in
+// clusters from 2048 columns on, 4211; every CTA reading its whole rows 6900 (4540 for the mean square alone, without a scale).  Prompts on 384- to
+// 1024-wide models take 2 to 5 % more than without a scale: the reduction in front of the stores, about half a microsecond a launch.
+constexpr int SPLIT_THREADS = 256, SPLIT_HOLD = 8;
+
+__device__ __forceinline__ void load_chunk(const float* row, int k, float (&f)[8]) {
+  const float4 a = *reinterpret_cast<const float4*>(row + k), b = *reinterpret_cast<const float4*>(row + k + 4);
+  f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+}
+__device__ __forceinline__ void weigh_chunk(float (&f)[8], const uint4& nw, float& ss, float& amax) {
+  const __half2* h = reinterpret_cast<const __half2*>(&nw);
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const float2 w = __half22float2(h[q]);
+    ss = fmaf(f[2 * q], f[2 * q], fmaf(f[2 * q + 1], f[2 * q + 1], ss));
+    f[2 * q] *= w.x; f[2 * q + 1] *= w.y;
+    amax = fmaxf(amax, fmaxf(fabsf(f[2 * q]), fabsf(f[2 * q + 1])));
+  }
+}
 
 template <typename T, bool CLUSTER>
 __global__ void __launch_bounds__(SPLIT_THREADS) split_rows_kernel(const T* __restrict__ x, const __half* __restrict__ norm_w, float eps, int m, int n_in,
                                                                    int kgroups, int nt, int chunks_per_cta, unsigned char* __restrict__ xt,
                                                                    unsigned* __restrict__ counters, int n_counters, float* __restrict__ down, float lowest) {
   constexpr bool F32 = sizeof(T) == 4;
-  __shared__ float red[SPLIT_THREADS / 32][8], red_max[SPLIT_THREADS / 32][8];
+  constexpr int STEP = SPLIT_THREADS / 8;                                 // chunks of a row in hand at once
   pdl_wait();
   pdl_launch_dependents();
   const int tid = threadIdx.x;
@@ -82,30 +98,42 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_rows_kernel(const T* __re
     for (int i = tid; i < n_counters; i += SPLIT_THREADS) counters[i] = 0;
   const int r = tid & 7, row = blockIdx.x * 8 + r;                       // row within the padded rows of all tiles
   const int tile = row / nt, in_tile = row - tile * nt;
-  const bool live = row < m;
-  float sc = 1.f, up = 1.f;
-  const int n_chunks = kgroups * 16, c0 = blockIdx.y * chunks_per_cta, c1 = min(n_chunks, c0 + chunks_per_cta);
-  if (F32 && (norm_w || down)) {                                          // the row's mean square and its largest value
-    float ss = 0.f, amax = 0.f;
-    if (live) {
-      const float* src = reinterpret_cast<const float*>(x) + (size_t)row * n_in;
-      const int k1 = CLUSTER ? min(n_in, c1 * 8) : n_in;
-      constexpr int STEP = SPLIT_THREADS / 8 * 4, BATCH = 4;              // loads in flight
-      for (int k0 = (CLUSTER ? c0 * 8 : 0) + (tid >> 3) * 4; k0 < k1; k0 += BATCH * STEP) {
-        float4 a[BATCH];
-        uint2 nw[BATCH];
+  const int n_chunks = kgroups * 16, c0 = blockIdx.y * chunks_per_cta + (tid >> 3), c1 = min(n_chunks, (int)(blockIdx.y + 1) * chunks_per_cta);
+  const int live = row < m ? n_in : 0;                                    // columns the row has
+  const T* src = x + (size_t)row * n_in;
+  const size_t row_bytes = (F32 ? 2 : 1) * (size_t)nt * 16;               // one chunk of a step
+  unsigned char* dst = xt + (size_t)tile * n_chunks * row_bytes + (size_t)in_tile * 16;
+  if constexpr (!F32) {
+    for (int c = c0; c < c1; c += STEP) {
+      uint4 raw = make_uint4(0, 0, 0, 0);
+      if (c * 8 < live) raw = *reinterpret_cast<const uint4*>(src + c * 8);
+      *reinterpret_cast<uint4*>(dst + (size_t)c * row_bytes) =
+          make_uint4(prmt(raw.x, raw.y, 0x5410u), prmt(raw.x, raw.y, 0x7632u), prmt(raw.z, raw.w, 0x5410u), prmt(raw.z, raw.w, 0x7632u));
+    }
+  } else {
+    __shared__ float red[SPLIT_THREADS / 32][8], red_max[SPLIT_THREADS / 32][8];
+    const uint4 ones = make_uint4(0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u);
+    float held[SPLIT_HOLD][8], ss = 0.f, amax = 0.f;
+    // SPLIT_HOLD chunks in flight; a stretch of at most so many per thread stays in registers until its row's factor is known
+    const int first = blockIdx.y * chunks_per_cta;
+    for (int b = first; b < c1; b += SPLIT_HOLD * STEP) {
+      uint4 nw[SPLIT_HOLD];
 #pragma unroll
-        for (int i = 0; i < BATCH; i++) {
-          const int k = k0 + i * STEP;
-          a[i] = k < k1 ? *reinterpret_cast<const float4*>(src + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-          nw[i] = norm_w && k < k1 ? *reinterpret_cast<const uint2*>(norm_w + k) : make_uint2(0x3C003C00u, 0x3C003C00u);      // fp16 ones
-        }
+      for (int i = 0; i < SPLIT_HOLD; i++) {
+        if (b + i * STEP >= c1) break;                                    // (the same for all threads)
+        const int c = b + i * STEP + (tid >> 3);
+        nw[i] = ones;
 #pragma unroll
-        for (int i = 0; i < BATCH; i++) {
-          const float2 w0 = __half22float2(*reinterpret_cast<const __half2*>(&nw[i].x)), w1 = __half22float2(*reinterpret_cast<const __half2*>(&nw[i].y));
-          ss = fmaf(a[i].x, a[i].x, fmaf(a[i].y, a[i].y, fmaf(a[i].z, a[i].z, fmaf(a[i].w, a[i].w, ss))));
-          amax = fmaxf(amax, fmaxf(fmaxf(fabsf(a[i].x * w0.x), fabsf(a[i].y * w0.y)), fmaxf(fabsf(a[i].z * w1.x), fabsf(a[i].w * w1.y))));
+        for (int q = 0; q < 8; q++) held[i][q] = 0.f;
+        if (c < c1 && c * 8 < live) {
+          load_chunk(src, c * 8, held[i]);
+          if (norm_w) nw[i] = *reinterpret_cast<const uint4*>(norm_w + c * 8);
         }
+      }
+#pragma unroll
+      for (int i = 0; i < SPLIT_HOLD; i++) {
+        if (b + i * STEP >= c1) break;
+        weigh_chunk(held[i], nw[i], ss, amax);
       }
     }
     ss += __shfl_xor_sync(0xffffffffu, ss, 8);
@@ -125,45 +153,41 @@ __global__ void __launch_bounds__(SPLIT_THREADS) split_rows_kernel(const T* __re
       tot = 0.f;
       for (uint32_t c = 0; c < gridDim.y; c++) { tot += ld_cluster(s32(&red[0][r]), c); amax = fmaxf(amax, ld_cluster(s32(&red_max[0][r]), c)); }
     }
+    float sc = 1.f;
     if (norm_w) { sc = 1.0f / sqrtf(tot / (float)n_in + eps); amax *= sc; }
     if (down) {
-      float inv = 1.f;
+      float up = 1.f, inv = 1.f;
       if (!(amax >= lowest && amax < 32768.f)) pow2_scale(amax, up, inv);
       if (blockIdx.y == 0 && tid < 8) down[row] = inv;
+      sc *= up;
     }
-  }
-  const size_t row_bytes = (F32 ? 2 : 1) * (size_t)nt * 16;               // one chunk of a step
-  unsigned char* base = xt + (size_t)tile * n_chunks * row_bytes + (size_t)in_tile * 16;
-  for (int c = c0 + (tid >> 3); c < c1; c += SPLIT_THREADS / 8) {
-    const int k = c * 8;
-    float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    unsigned char* dst = base + (size_t)c * row_bytes;
-    if (!F32) {
-      uint4 raw = make_uint4(0, 0, 0, 0);
-      if (live && k < n_in) raw = *reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(x) + (size_t)row * n_in + k);
-      *reinterpret_cast<uint4*>(dst) = make_uint4(prmt(raw.x, raw.y, 0x5410u), prmt(raw.x, raw.y, 0x7632u), prmt(raw.z, raw.w, 0x5410u), prmt(raw.z, raw.w, 0x7632u));
-      continue;
-    }
-    if (live && k < n_in) {
-      const float* src = reinterpret_cast<const float*>(x) + (size_t)row * n_in + k;
-      const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
-      f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
-      if (norm_w) {
-        const uint4 nw = *reinterpret_cast<const uint4*>(norm_w + k);
-        const __half2* h = reinterpret_cast<const __half2*>(&nw);
+    auto store = [&](float (&f)[8], int c) {
+      uint4 hi, lo;
 #pragma unroll
-        for (int q = 0; q < 4; q++) { const float2 t2 = __half22float2(h[q]); f[2 * q] = f[2 * q] * sc * t2.x; f[2 * q + 1] = f[2 * q + 1] * sc * t2.y; }
+      for (int q = 0; q < 8; q++) f[q] *= sc;
+      split_chunk(f, hi, lo);
+      *reinterpret_cast<uint4*>(dst + (size_t)c * row_bytes) = hi;
+      *reinterpret_cast<uint4*>(dst + (size_t)c * row_bytes + (size_t)nt * 16) = lo;
+    };
+    if (chunks_per_cta <= SPLIT_HOLD * STEP) {
+#pragma unroll
+      for (int i = 0; i < SPLIT_HOLD; i++)
+        if (c0 + i * STEP < c1) store(held[i], c0 + i * STEP);
+    } else {
+      for (int c = c0; c < c1; c += STEP) {
+        float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        uint4 nw = ones;
+        if (c * 8 < live) {
+          load_chunk(src, c * 8, f);
+          if (norm_w) nw = *reinterpret_cast<const uint4*>(norm_w + c * 8);
+        }
+        weigh_chunk(f, nw, ss, amax);
+        store(f, c);
       }
-#pragma unroll
-      for (int q = 0; q < 8; q++) f[q] *= up;
     }
-    uint4 hi, lo;
-    split_chunk(f, hi, lo);
-    *reinterpret_cast<uint4*>(dst) = hi;
-    *reinterpret_cast<uint4*>(dst + (size_t)nt * 16) = lo;
+    __syncwarp();
+    if (CLUSTER) cluster_sync();                                          // nobody leaves while its sums are being read
   }
-  __syncwarp();
-  if (CLUSTER) cluster_sync();                                            // nobody leaves while its sums are being read
 }
 
 // ---- the product ---------------------------------------------------------------------------------------------------------------
@@ -687,11 +711,12 @@ int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtyp
   const bool split = !unsplit && workspace_bytes >= xt_bytes + split_workspace(pl, n_out, kgroups, n_sm);
   p.grain = split ? 1 : kgroups; p.unsplit = !split;
   const int grid = split ? stream_grid(p.units, n_sm) : (p.tiles < n_sm ? p.tiles : n_sm);
-  // one CTA of the splitting kernel: 8 rows x the whole width, or a part of it where there are few rows
+  // one CTA of the splitting kernel: 8 rows x the whole width, or a part of it where there are few rows (and, of fp32 rows, more than a CTA keeps in registers)
   const int row_groups = pl.tok_tiles * pl.nt / 8, n_chunks = kgroups * 16;
-  const int parts = row_groups >= n_sm ? 1 : (row_groups * 4 >= n_sm || n_chunks < 256 ? 4 : 8), per = ceil_div(n_chunks, parts);
+  const int parts = row_groups >= n_sm || (f32 && n_chunks <= SPLIT_HOLD * SPLIT_THREADS / 8) ? 1 : (row_groups * 4 >= n_sm || n_chunks < 256 ? 4 : 8);
+  const int per = ceil_div(n_chunks, parts);
   const dim3 sgrid(row_groups, ceil_div(n_chunks, per));      // rows along x: y ends at 65535
-  const bool cluster = f32 && sgrid.y > 1 && n_chunks >= 256;
+  const bool cluster = f32 && sgrid.y > 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = sgrid; cfg.blockDim = dim3(SPLIT_THREADS); cfg.stream = st;
   cudaLaunchAttribute attr[2];
