@@ -413,10 +413,6 @@ typedef struct b200q_linear_desc {
   size_t workspace_bytes;
 } b200q_linear_desc;
 int b200q_linear(const b200q_linear_desc* l, const void* x, int dtype, int m, void** y, void* stream);
-/* The same Linear for a few activation rows (m <= 32: batched decode), the weight-streaming shape: the operands swap roles on the
- * tensor core (weight rows = M, activation rows = N = 32), K is split over CTAs so that every layer fills the GPU, partial sums go
- * through `workspace` (b200q_qgemm_skinny_workspace_bytes) and are added in a fixed order by a second kernel that also applies
- * bias / residual / SwiGLU.  Same operands, numerics and epilogue rules as b200q_qgemm. */
 /* The same Linear for a FEW activation rows on the int8 tensor cores (batched decode): the 8 columns of an m16n8k32 MMA are 8 activation
  * rows, so a pass streams the weights once for 8 rows at the one-row GEMV's arithmetic (15-bit activation integers, exact block sums, fp32
  * across blocks); m > 8 takes ceil(m / 8) passes.  Launches per pass: quantise the rows into the MMA's operand order; the streaming
@@ -431,6 +427,10 @@ int b200q_qgemv_rows(int qtype, const void* w_packed, const void* x, int x_dtype
 int b200q_qgemv_rows_norm(int qtype, const void* w_packed, const void* x, int x_dtype, const void* norm_weight_f16, float norm_eps, const void* bias_f16,
                           const void* residual, int epilogue, void* y, int y_dtype, int m, int n_out, int n_in, void* workspace, size_t workspace_bytes,
                           void* stream);
+/* The same Linear for up to 32 activation rows without a pass over them first, the weight-streaming shape: the operands swap roles on the
+ * tensor core (weight rows = M, activation rows = N = 32), K is split over CTAs so that every layer fills the GPU, partial sums go
+ * through `workspace` (b200q_qgemm_skinny_workspace_bytes) and are added in a fixed order by a second kernel that also applies
+ * bias / residual / SwiGLU.  Same operands, numerics and epilogue rules as b200q_qgemm. */
 size_t b200q_qgemm_skinny_workspace_bytes(int m, int n_out, int n_in);
 int b200q_qgemm_skinny(int qtype, const void* w_packed, const void* x, int x_dtype, const void* bias_f16, const void* residual, int epilogue, void* y,
                        int y_dtype, int m, int n_out, int n_in, void* workspace, size_t workspace_bytes, void* stream);

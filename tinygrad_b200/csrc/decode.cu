@@ -840,8 +840,9 @@ static int launch_attn_cluster(const b200q_attn_args* a, const SeqStride& sq, in
 // cached rows stream through twice the SMs (4 heads, position 3507: 17.9 -> 12.6 us per block); at short contexts both take the same time.
 template <int HD, typename KV>
 static int attn_cluster(const b200q_attn_args* a, const SeqStride& sq, int n_seqs, bool pdl, cudaStream_t stream) {
-  // one chunk at most: one CTA does it all (a launch with clusters costs a graph replay 1.7 us: 3-block 512-wide model, 54 positions, 950 us for 16 tokens with
-  // clusters of 16, 890 so)
+  // A cache of one chunk (a model built for at most 64 positions): one CTA does it all, the others of a cluster would only wait.  16 tokens of a 3-block 512-wide model
+  // 955 us with clusters, 885 so; 8 tokens of a batch of 11 on 14 640-wide blocks 10303 us, 8223 so.  Longer caches always take clusters: the position that would
+  // decide is on the device.
   if (a->max_context <= AC_POS) return launch_attn_cluster<HD, 1, KV>(a, sq, n_seqs, pdl, stream);
   static std::atomic<int> wide[B200Q_MAX_DEVICES];                   // clusters of 16 that run at once, plus one; 0: not asked yet
   const int dev = b200q_current_device();

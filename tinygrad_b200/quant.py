@@ -120,7 +120,8 @@ def qgemm(w_ptr: int, qtype: int, n_out: int, n_in: int, x, y, m: int, x_dtype=F
 
 
 FEW_ROW_FUSED = os.environ.get("B200Q_FEW_ROW_FUSED", "1") == "1"      # batched decode with few rows: the int8-MMA few-row kernel
-# ... up to this many rows, 8 per pass over the weights (7B Q8_0 gate/up: 34.5 us per pass against 88 for up to 64 rows on the GEMM; down 24 against 73)
+# ... up to this many rows, 8 per pass over the weights.  A step of five 7B-shaped Q8_0 blocks and the head: 9 / 16 rows 1.03 / 1.06 ms in two passes against 1.13 / 1.17
+# on the GEMM, 17 rows 1.56 in three against 1.22.
 FEW_ROW_MAX = int(os.environ.get("B200Q_FEW_ROW_MAX", "16"))
 
 
