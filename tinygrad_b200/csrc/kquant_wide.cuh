@@ -8,8 +8,8 @@
 // of a quad end with the same sums).  A nibble or 6 bits at bit 0 of an fp16 are the subnormal q * 2^-24, at bit 4 q * 2^-20: masks and
 // shifts unpack two quants, two conversions and one packed FMA scale them exactly as fp32 would, one conversion rounds the pair to fp16.
 // What bounds it is that dequantisation: 64 conversions and 32 packed FMAs on one pipe, 72 masks, shifts and roundings on another per tile, each
-// good for an instruction every other cycle.  Gate and up of 14336 x 4096 in Q4_K 26.3 us (2.66 TB/s of packed weights; as fp16
-// these are 235 MB, 36 us at HBM rate), down 4096 x 14336 in Q6_K 19.7 us; a step of six 8B-shaped blocks 1005 us on fp16 weights, 510 us here.  Scalar FMAs: 27.0 us.  The mixed-precision FMA on scale * q
+// good for an instruction every other cycle.  Gate and up of 14336 x 4096 in Q4_K 26.3 us with running accumulators (2.66 TB/s of packed
+// weights; as fp16 these are 235 MB, 36 us at HBM rate; a single cold launch with its events 30.8, and 32.8 with the sums below), down 4096 x 14336 in Q6_K 19.7 us; a step of six 8B-shaped blocks 1005 us on fp16 weights, 510 us here.  Scalar FMAs: 27.0 us.  The mixed-precision FMA on scale * q
 // (exact in fp16), which needs no conversions: 30.1 us.
 //
 // Sums: the tensor core truncates, always towards zero, when it adds to an accumulator, so the high parts' products of two MMAs at a time are added here,
