@@ -1,5 +1,5 @@
 """The many-row GEMM with a workspace (csrc/qgemm_stream.cu) at the edges of its tiles and of its dispatch: activation tiles of 16 .. 256 rows,
-weight tiles of 128 (up to 64 rows) and 256, one pass (fp16) and three (fp32), tiles split over CTAs or whole, remainders everywhere."""
+weight tiles of 128 (up to 128 rows) and 256, one pass (fp16) and three (fp32), tiles split over CTAs or whole, remainders everywhere."""
 import numpy as np
 import pytest
 from tinygrad_b200 import _lib, quant, synth
@@ -18,7 +18,7 @@ def _gpu(): need_gpu()
 @pytest.mark.parametrize("typ,m,n_out,n_in,dt", [(2, 1, 16, 32, np.float32), (8, 16, 130, 96, np.float32), (2, 17, 1000, 1184, np.float32), (8, 64, 128, 4096, np.float32),
                                                  (2, 65, 257, 4096, np.float32), (8, 128, 256, 160, np.float32), (2, 129, 300, 992, np.float32), (8, 256, 512, 512, np.float32),
                                                  (2, 257, 130, 1408, np.float32), (2, 301, 200, 640, np.float16), (8, 64, 300, 1184, np.float16), (8, 600, 72, 96, np.float16),
-                                                 # enough row tiles for 256 weight rows each (the others above 64 rows take 128)
+                                                 # enough row tiles for 256 weight rows each above 128 rows (the others take 128)
                                                  (2, 65, 19300, 96, np.float32), (8, 130, 30400, 160, np.float32), (2, 257, 15300, 96, np.float32),
                                                  (8, 300, 15300, 96, np.float16)])
 def test_rows_against_the_exact_product(typ, m, n_out, n_in, dt, split):
@@ -39,6 +39,15 @@ def test_rows_against_the_exact_product(typ, m, n_out, n_in, dt, split):
   size = np.abs(x).astype(np.float64) @ np.abs(w).T + np.abs(bias) + np.abs(res)
   bound = (2.0 ** -21 + 3 * np.ceil(n_in / 16) * 2.0 ** -23) * size + (2.0 ** -11 if dt == np.float16 else 2.0 ** -23) * np.abs(ref) + 1e-7
   assert (np.abs(y.numpy() - ref) <= bound).all(), f"worst {np.max(np.abs(y.numpy() - ref) / bound):.2f} of the bound"
+
+
+# weights through tensor memory: whole tiles between split ones, with and without room for them in shared memory (112 rows of Q4_0, Q8_0), tiles of one K group, one slot
+# of weights per thread group and two, the most rows of either type
+@pytest.mark.parametrize("split", [True, False])
+@pytest.mark.parametrize("typ,m,n_out,n_in,dt", [(2, 45, 51216, 416, np.float32), (8, 112, 38144, 288, np.float32), (2, 112, 40000, 160, np.float32), (8, 3, 57000, 96, np.float32),
+                                                 (2, 128, 1000, 4000, np.float32), (8, 128, 260, 14336, np.float32), (2, 100, 40000, 288, np.float16), (8, 256, 1300, 992, np.float16),
+                                                 (2, 160, 2000, 2080, np.float16), (2, 33, 16, 18944, np.float32)])
+def test_weights_through_tensor_memory(typ, m, n_out, n_in, dt, split): test_rows_against_the_exact_product(typ, m, n_out, n_in, dt, split)
 
 
 # more rows than m rounded up to 128: 3 x 224, 10 x 256

@@ -15,8 +15,8 @@
 //    instead of three);
 //  * a tile is up to 256 weight rows (two accumulators, the whole of tensor memory) by up to 256 activation rows: every unpacked weight meets
 //    256 rows and every activation byte 256 weight rows.  With 128 x 128 tiles the activation operand alone took 2.4x the L2 traffic
-//    and every weight was unpacked once per 128 rows.  Up to 64 rows, and where tiles are few, a tile is 128 weight rows
-//    (more tiles to share, smaller partial sums);
+//    and every weight was unpacked once per 128 rows.  Up to 128 rows, and where tiles are few, a tile is 128 weight rows
+//    (more tiles to share, smaller partial sums); up to 128 rows, and for half-precision rows, its weights go through tensor memory (qgemm_tmem.cuh);
 //  * roles are separate warps: 16 unpack the weights (packed blocks by asynchronous copies, several ahead -> fp16 halves in a ring of
 //    shared-memory slots), one thread brings activation tiles in by bulk copies, one issues the MMAs; nothing meets at a block barrier;
 //  * the K x tile space is dealt to one CTA per SM in equal contiguous runs (stream-K): no last wave.  A tile that spans CTAs leaves fp32
@@ -34,7 +34,6 @@ constexpr int UNPACK_WARPS = 16, UNPACK_THREADS = UNPACK_WARPS * 32;
 constexpr int WARP_COPY = UNPACK_WARPS, WARP_MMA = UNPACK_WARPS + 1;
 constexpr int THREADS = (UNPACK_WARPS + 2) * 32;
 constexpr int KSTEP = 32;                               // one quant block of K per step
-constexpr int steps_per_slot(int wt, int nt) { return wt == 128 && nt <= 64 ? 4 : 1; }
 constexpr int RING_BYTES = 224 * 1024, MAX_SLOTS = 6;   // shared memory: slots of unpacked weights + activations
 // Packed blocks wait in shared memory, one 16 / 32-byte block and its scale per unpack thread and round, up to MAX_AHEAD rounds ahead.  A queue in
 // registers that moves up by a block waits for the newest load every time: whatever its depth, a round took a trip to HBM (8B gate / up, 45 rows: 83 us,
@@ -58,6 +57,7 @@ struct StreamParams {
   // sums.  With whole tiles every output is one running sum (halves not side by side either) in the order of b200q_qgemm: the same bits.
   int grain, unsplit;
   int tiles, m, n_out, kgroups, n_row_tiles, nt, tok_tiles, slots, ahead, y_f16, silu_mul;
+  int dump, d_cols;              // qgemm_tmem.cuh: where whole tiles wait in shared memory (0: nowhere), tensor-memory columns of the accumulators
 };
 
 // ---- activations: fp32 (or fp16) rows, optionally RMS-normed, -> fp16 halves as the tensor core reads them ---------------------
@@ -244,11 +244,11 @@ __device__ __forceinline__ size_t part_slot(const StreamParams& p, int c, int ti
 }
 __device__ __forceinline__ int cta_of(long long unit, long long units, int g) { return (int)(((unit + 1) * g - 1) / units); }
 
-// EC consecutive activation rows of one output column (weight row) `feat`
-__device__ __forceinline__ void store_outputs(const StreamParams& p, float (&v)[EC], int feat, int tok0, int lane) {
+// N consecutive activation rows of one output column (weight row) `feat`
+template <int N> __device__ __forceinline__ void store_outputs(const StreamParams& p, float (&v)[N], int feat, int tok0, int lane) {
   if (p.down)
 #pragma unroll
-    for (int j = 0; j < EC; j += 4) {
+    for (int j = 0; j < N; j += 4) {
       const float4 d = *reinterpret_cast<const float4*>(p.down + tok0 + j);
       v[j] *= d.x; v[j + 1] *= d.y; v[j + 2] *= d.z; v[j + 3] *= d.w;
     }
@@ -257,7 +257,7 @@ __device__ __forceinline__ void store_outputs(const StreamParams& p, float (&v)[
     const bool gate = !(lane & 8);
     const int col = (feat >> 4) * 8 + (feat & 7), n_y = p.n_out >> 1;
 #pragma unroll
-    for (int j = 0; j < EC; j += 2) {
+    for (int j = 0; j < N; j += 2) {
       const float other = __shfl_xor_sync(0xffffffffu, gate ? v[j + 1] : v[j], 8);
       const float g = gate ? v[j] : other, u = gate ? other : v[j + 1], o = (g / (1.f + expf(-g))) * u;
       const int tok = tok0 + j + (gate ? 0 : 1);
@@ -270,9 +270,9 @@ __device__ __forceinline__ void store_outputs(const StreamParams& p, float (&v)[
   }
   if (feat >= p.n_out) return;
   const float b = p.bias ? __half2float(p.bias[feat]) : 0.f;
-  float add[EC];
+  float add[N];
 #pragma unroll
-  for (int j = 0; j < EC; j++) {
+  for (int j = 0; j < N; j++) {
     add[j] = b;
     if (p.residual && tok0 + j < p.m) {
       const size_t at = (size_t)(tok0 + j) * p.n_out + feat;
@@ -280,7 +280,7 @@ __device__ __forceinline__ void store_outputs(const StreamParams& p, float (&v)[
     }
   }
 #pragma unroll
-  for (int j = 0; j < EC; j++)
+  for (int j = 0; j < N; j++)
     if (tok0 + j < p.m) {
       const size_t at = (size_t)(tok0 + j) * p.n_out + feat;
       if (p.y_f16) reinterpret_cast<__half*>(p.y)[at] = __float2half_rn(v[j] + add[j]); else reinterpret_cast<float*>(p.y)[at] = v[j] + add[j];
@@ -293,7 +293,7 @@ __device__ __forceinline__ bool finish_segment(const StreamParams& p, Shared& sh
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = warp & 3, q = warp >> 2;
   const int hf = WT == 256 ? q >> 1 : 0, part0 = WT == 256 ? q & 1 : q, parts = WT == 256 ? 2 : 4;
   const int tt = tile % p.tok_tiles, row = hf * 128 + sub * 32 + lane, feat = (tile / p.tok_tiles) * WT + row;
-  const bool whole = k0 == 0 && k1 == p.kgroups, stacked = F32 && p.nt <= MAX_NT / 2 && !p.unsplit;
+  const bool whole = k0 == 0 && k1 == p.kgroups;
   const int G = gridDim.x, c = blockIdx.x;
   int c0 = c, n_seg = 1;
   if (!whole) {
@@ -307,20 +307,18 @@ __device__ __forceinline__ bool finish_segment(const StreamParams& p, Shared& sh
   const uint32_t ta = sh.tmem + ((uint32_t)(sub * 32) << 16) + hf * 256;
   const int groups = p.nt / EC;
   for (int cg = part0; cg < groups; cg += parts) {
-    uint32_t a[EC], b[EC];
+    uint32_t a[EC];
     ld_tmem(ta + cg * EC, a);
-    if (stacked) ld_tmem(ta + p.nt + cg * EC, b);
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
     float v[EC];
 #pragma unroll
-    for (int j = 0; j < EC; j++) v[j] = stacked ? __uint_as_float(a[j]) + __uint_as_float(b[j]) : __uint_as_float(a[j]);
+    for (int j = 0; j < EC; j++) v[j] = __uint_as_float(a[j]);
     if (whole) store_outputs(p, v, feat, tt * p.nt + cg * EC, lane);
     else
 #pragma unroll
       for (int j = 0; j < EC; j += 4) __stcg(reinterpret_cast<float4*>(mine + (size_t)(cg * EC + j) * WT), make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]));
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  if (!whole) __threadfence();
   __syncwarp();
   if (lane == 0) { bar_arrive(BAR(sb, acc_empty)); if (!whole) bar_arrive(BAR(sb, stored)); }
   if (whole) return true;
@@ -356,23 +354,19 @@ __device__ __forceinline__ bool finish_segment(const StreamParams& p, Shared& sh
   return true;
 }
 
-__device__ __forceinline__ uint4 ld_shared4(uint32_t addr) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
-  return v;
-}
+}  // namespace
+#include "qgemm_tmem.cuh"
+namespace {
+
 // the weights of one 32-wide block of a row as they come from memory
 template <int QT> struct Raw;
 template <> struct Raw<B200Q_Q4_0> { uint4 a; uint32_t d; };
 template <> struct Raw<B200Q_Q8_0> { uint4 a, b; uint32_t d; };
 
-template <int QT, int WT, bool F32, int SPS>
+template <int QT, int WT, bool F32>
 __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamParams p) {
   constexpr int TB = tile_bytes(QT), GROUPS = UNPACK_THREADS / WT, PER_UNIT = 4 / GROUPS;    // thread groups, each with its own steps of a K group
   constexpr int W_HALF = WT * KSTEP * 2, W_STEP = 2 * W_HALF;
-  // Steps per ring slot, i.e. per barrier phase.  With few activation rows a step's MMAs take less time than the barrier operations around
-  // them (a ready barrier costs the MMA thread about 100 cycles, an instruction of N <= 128 72), so a slot is a whole K group there.
-  constexpr int W_SLOT = W_STEP * SPS;
   extern __shared__ __align__(128) unsigned char dyn[];
   __shared__ Shared sh;
   const uint32_t sb = pinned(s32(&sh)), ring = pinned(s32(dyn));
@@ -380,14 +374,14 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
   const int G = gridDim.x, c = blockIdx.x;
   const long long u0 = first_unit(c, p, G), u1 = first_unit(c + 1, p, G);
   const int nt = p.nt, slots = p.slots, x_rows = F32 ? 2 * nt : nt;
-  const uint32_t x_step = (uint32_t)x_rows * 64, x_bytes = x_step * SPS, slot_bytes = W_SLOT + x_bytes;      // a step's activations, a slot's; a whole slot
+  const uint32_t x_step = (uint32_t)x_rows * 64, slot_bytes = W_STEP + x_step;      // a slot: one step's activations and weights
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(&sh.tmem)), "r"(WT == 256 ? 512 : 256) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if (tid == 32) {
     // a slot is full when its unpack warps and the copy thread have arrived and the copy's bytes are there; one commit empties it
-    for (int i = 0; i < MAX_SLOTS; i++) { bar_init(BAR(sb, full) + 8 * i, WT / 32 * SPS + 1); bar_init(BAR(sb, empty) + 8 * i, 1); }
+    for (int i = 0; i < MAX_SLOTS; i++) { bar_init(BAR(sb, full) + 8 * i, WT / 32 + 1); bar_init(BAR(sb, empty) + 8 * i, 1); }
     bar_init(BAR(sb, acc_full), 1); bar_init(BAR(sb, acc_empty), UNPACK_WARPS);
     bar_init(BAR(sb, stored), UNPACK_WARPS); bar_init(BAR(sb, counted), 1); bar_init(BAR(sb, drained), 1);
     sh.abort = 0;
@@ -408,13 +402,13 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
       for (long long u = u0; u < u1 && ok;) {
         const int tile = (int)(u / p.kgroups), k0 = (int)(u - (long long)tile * p.kgroups), k1 = (int)min((long long)p.kgroups, k0 + u1 - u);
         const unsigned char* src = p.xt + ((size_t)(tile % p.tok_tiles) * p.kgroups + k0) * 4 * x_step;
-        for (int s = 0; s < (k1 - k0) * (4 / SPS); s++, n++, src += x_bytes) {
+        for (int s = 0; s < (k1 - k0) * 4; s++, n++, src += x_step) {
           if (!bar_wait(sb, BAR(sb, empty) + 8 * slot, par)) { ok = false; break; }
-          const uint32_t dst = ring + slot * slot_bytes + W_SLOT, bar = BAR(sb, full) + 8 * slot;
-          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(x_bytes) : "memory");
-          for (uint32_t o = 0; o < x_bytes; o += 8192)   // several copies overlap where one is served slowly
+          const uint32_t dst = ring + slot * slot_bytes + W_STEP, bar = BAR(sb, full) + 8 * slot;
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(x_step) : "memory");
+          for (uint32_t o = 0; o < x_step; o += 8192)   // several copies overlap where one is served slowly
             asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                         ::"r"(dst + o), "l"(src + o), "r"(min(8192u, x_bytes - o)), "r"(bar) : "memory");
+                         ::"r"(dst + o), "l"(src + o), "r"(min(8192u, x_step - o)), "r"(bar) : "memory");
           if (++slot == slots) { slot = 0; par ^= 1; }
         }
         u += k1 - k0;
@@ -427,10 +421,9 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
   } else if (warp == WARP_MMA) {
     if (elect_one()) {
       bool ok = true;
-      const bool stacked = F32 && nt <= MAX_NT / 2 && !p.unsplit;
-      const uint32_t id1 = make_idesc(128, nt), id2 = make_idesc(128, stacked ? 2 * nt : nt);
+      const uint32_t idesc = make_idesc(128, nt);
       const uint32_t desc_hi = (uint32_t)(make_desc(0, 0, 128) >> 32);
-      const uint32_t w_base = (ring >> 4) | ((uint32_t)WT << 16), x_base = ((ring + W_SLOT) >> 4) | ((uint32_t)x_rows << 16);
+      const uint32_t w_base = (ring >> 4) | ((uint32_t)WT << 16), x_base = ((ring + W_STEP) >> 4) | ((uint32_t)x_rows << 16);
       int seg = 0, slot = 0;
       uint32_t par = 0, x_lo = x_base, w_lo = w_base;
       for (long long u = u0; u < u1 && ok; seg++) {
@@ -439,7 +432,7 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t tmem = sh.tmem;
         uint32_t acc = 0;
-        for (int s = (k1 - k0) * (4 / SPS); s > 0; s--) {
+        for (int s = (k1 - k0) * 4; s > 0; s--) {
           if (!bar_wait(sb, BAR(sb, full) + 8 * slot, par)) { ok = false; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           // all MMAs of one accumulator back to back: switching the destination costs about 40 cycles of a 128-cycle instruction
@@ -448,13 +441,13 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
           for (int hf = 0; hf < WT / 128; hf++) {
             const uint32_t d = tmem + hf * 256;
 #pragma unroll
-            for (int kk = 0; kk < SPS * KSTEP / 16; kk++) {
+            for (int kk = 0; kk < KSTEP / 16; kk++) {
               const uint32_t xh = x_lo + (kk >> 1) * (x_step >> 4) + (kk & 1) * 2 * x_rows;
               const uint32_t wh = w_lo + (kk >> 1) * (W_STEP >> 4) + hf * 128 + (kk & 1) * 2 * WT;
-              mma(d, wh, xh, desc_hi, id2, kk ? 1u : acc);          // stacked: wh x [xh | xl] in one instruction
+              mma(d, wh, xh, desc_hi, idesc, kk ? 1u : acc);
               if (F32) {
-                if (!stacked) mma(d, wh, xh + nt, desc_hi, id1, 1u);
-                mma(d, wh + (W_HALF >> 4), xh, desc_hi, id1, 1u);
+                mma(d, wh, xh + nt, desc_hi, idesc, 1u);
+                mma(d, wh + (W_HALF >> 4), xh, desc_hi, idesc, 1u);
               }
             }
           }
@@ -519,16 +512,14 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
     for (int d = 0; d < p.ahead; d++) request(wait0 + d * AHEAD);
     pdl_wait();                                          // the epilogue reads and writes what earlier kernels touched
     // One block: wait for its slot, unpack, hand over, ask for the block DEPTH further on.
-    int slot = SPS > 1 ? 0 : grp;                        // ring position and its phase; SPS == 1: the thread groups take turns
+    int slot = grp;                                      // ring position and its phase; the thread groups take turns
     uint32_t par = 1;
-    constexpr int SLOT_STEP = SPS > 1 ? 1 : GROUPS;
-    static_assert(SPS == 1 || (SPS == 4 && GROUPS == 4), "one block per thread and slot");
     bool ok = true;
     auto unpack = [&]() {
       ok = ok && bar_wait(sb, BAR(sb, empty) + 8 * slot, par);
       Raw<QT> q;
       collect(q);
-      const uint32_t dst = ring + slot * slot_bytes + (SPS > 1 ? grp * W_STEP : 0) + r * 16;
+      const uint32_t dst = ring + slot * slot_bytes + r * 16;
       const uint32_t d2 = q.d | (q.d << 16);
       uint4 hi[4], lo[4];
       if constexpr (QT == B200Q_Q4_0) {
@@ -556,12 +547,12 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
       if (lane == 0) bar_arrive(BAR(sb, full) + 8 * slot);
       request(wait_at);
       if ((wait_at += AHEAD) == wait_end) wait_at = wait0;
-      slot += SLOT_STEP;
+      slot += GROUPS;
       if (slot >= slots) { slot -= slots; par ^= 1; }
     };
     // A segment's accumulators are read back only after the first LEAD blocks of the next one are unpacked: they fill the ring while the
     // MMAs still in the pipe complete.
-    const int LEAD = SPS > 1 ? slots : slots / GROUPS;
+    const int LEAD = slots / GROUPS;
     int done_tile = -1, done_k0 = 0, done_k1 = 0, seg = 0;
     long long u = u0;
     while (ok) {
@@ -600,20 +591,20 @@ Plan make_plan(int m, int n_out, int n_sm) {
   Plan pl;
   pl.tok_tiles = ceil_div(m, MAX_NT);
   pl.nt = ceil_div(ceil_div(m, pl.tok_tiles), 16) * 16;      // equal tiles: 301 rows are 2 x 160, not 256 + 45
-  // 128 weight rows a tile up to 64 activation rows, and where tiles of 256 are too few for the SMs: each is then split over several CTAs, the one
-  // that arrives last adds all parts alone, and halving the tile quarters what it reads.  8B QKV (24 tiles), 256 rows: 75 -> 49 us, down (16)
-  // 117 -> 83; gate/up (112) 154 -> 142, but 79 -> 83 at 80 rows; 7B gate/up (148 tiles, hardly split) 142 -> 146.
-  pl.wt = pl.nt <= 64 || (n_out > 0 && (pl.nt > 96 ? 5LL : 8LL) * ceil_div(n_out, 256) * pl.tok_tiles <= 4LL * n_sm) ? 128 : 256;
+  // 128 weight rows a tile up to 128 activation rows (qgemm_tmem.cuh; 28672 x 4096, 128 rows: 256-row tiles through shared memory 87 us, 77), and where tiles of 256
+  // are too few for the SMs: each is then split over several CTAs, the one that arrives last adds all parts alone, and halving the tile quarters what it reads.
+  // 8B QKV (24 tiles), 256 rows: 75 -> 49 us, down (16) 117 -> 83; gate/up (112) 154 -> 142; 7B gate/up (148 tiles, hardly split) 142 -> 146.
+  pl.wt = pl.nt <= 128 || (n_out > 0 && 5LL * ceil_div(n_out, 256) * pl.tok_tiles <= 4LL * n_sm) ? 128 : 256;
   return pl;
 }
 size_t tiles_bytes(const Plan& pl, int kgroups, bool f32) { return (size_t)pl.tok_tiles * pl.nt * kgroups * GROUP_ELEMS * (f32 ? 4 : 2); }
-int slot_bytes(const Plan& pl, bool f32) { return steps_per_slot(pl.wt, pl.nt) * (pl.wt * KSTEP * 4 + pl.nt * (f32 ? 128 : 64)); }
+int slot_bytes(const Plan& pl, bool f32) { return pl.wt * KSTEP * 4 + pl.nt * (f32 ? 128 : 64); }
 size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
 size_t scale_bytes(const Plan& pl) { return align256((size_t)pl.tok_tiles * pl.nt * sizeof(float)); }
 
-template <int QT, int WT, bool F32, int SPS>
+template <int QT, int WT, bool F32>
 int launch_stream(const StreamParams& p, int grid, cudaStream_t st) {
-  auto kern = qgemm_stream_kernel<QT, WT, F32, SPS>;
+  auto kern = qgemm_stream_kernel<QT, WT, F32>;
   static PerDeviceFlag attr;
   const int dev = b200q_current_device();
   if (dev < 0) return B200Q_ERR_CUDA;
@@ -622,6 +613,31 @@ int launch_stream(const StreamParams& p, int grid, cudaStream_t st) {
     attr.set(dev);
   }
   B200Q_CHECK_CUDA(launch_k(kern, dim3(grid), dim3(THREADS), (size_t)p.slots * slot_bytes({p.nt, p.tok_tiles, WT}, F32) + (size_t)p.ahead * ahead_bytes(QT), st, true, p));
+  return B200Q_OK;
+}
+
+// weights through tensor memory: up to 128 rows (of fp32 rows 2 x 128 accumulator columns), half-precision rows wherever a tile has 128 weight rows
+bool takes_tmem(const Plan& pl, bool f32) { return pl.nt <= 128 || (!f32 && pl.wt == 128); }
+template <int QT, bool F32>
+int launch_tmem(StreamParams& p, int grid, cudaStream_t st) {
+  auto kern = qgemm_tmem_kernel<QT, F32>;
+  static PerDeviceFlag attr;
+  const int dev = b200q_current_device();
+  if (dev < 0) return B200Q_ERR_CUDA;
+  if (!attr.test(dev)) {
+    B200Q_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, RING_BYTES));
+    attr.set(dev);
+  }
+  // tensor memory: accumulators, then up to 4 slots of weights; shared memory: a K group of activations per slot, 2 to 6 stages of packed weights, and what is left
+  // of a tile's accumulators once they have been read
+  const int x_bytes = p.nt * (F32 ? 512 : 256), one = w_stage_bytes(QT), dump = p.nt * 512;
+  p.d_cols = ceil_div(F32 && !p.unsplit ? 2 * p.nt : p.nt, 32) * 32;
+  p.slots = std::min({MAX_T_SLOTS, (512 - p.d_cols) / A_COLS<F32>, (RING_BYTES - 2 * one) / x_bytes});
+  p.dump = p.slots * x_bytes + 2 * one + dump <= RING_BYTES ? dump : 0;
+  p.ahead = std::min(MAX_W_STAGES, (RING_BYTES - p.slots * x_bytes - p.dump) / one);
+  const size_t smem = (size_t)p.slots * x_bytes + (size_t)p.ahead * one + p.dump;
+  if (p.dump) p.dump = (int)smem - dump;
+  B200Q_CHECK_CUDA(launch_k(kern, dim3(grid), dim3(T_THREADS), smem, st, true, p));
   return B200Q_OK;
 }
 
@@ -701,7 +717,7 @@ int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtyp
   // Slots of unpacked weights and activations, 2 K groups or 3 (256 activation rows) to 5 steps; what they leave is for the packed blocks ahead:
   // at least two groups of Q4_0 (or one of Q8_0, whose blocks are twice as large) unless even two K groups leave less.
   const int slot = slot_bytes(pl, f32), one = ahead_bytes(qtype);
-  p.slots = steps_per_slot(pl.wt, pl.nt) == 4 ? 2 : (RING_BYTES - (qtype == B200Q_Q4_0 ? 2 : 1) * one) / slot;
+  p.slots = (RING_BYTES - (qtype == B200Q_Q4_0 ? 2 : 1) * one) / slot;
   if (p.slots > MAX_SLOTS) p.slots = MAX_SLOTS;
   p.ahead = (RING_BYTES - p.slots * slot) / one;
   if (p.ahead > MAX_AHEAD) p.ahead = MAX_AHEAD;
@@ -711,6 +727,7 @@ int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtyp
   const bool split = !unsplit && workspace_bytes >= xt_bytes + split_workspace(pl, n_out, kgroups, n_sm);
   p.grain = split ? 1 : kgroups; p.unsplit = !split;
   const int grid = split ? stream_grid(p.units, n_sm) : (p.tiles < n_sm ? p.tiles : n_sm);
+  p.dump = p.d_cols = 0;
   // one CTA of the splitting kernel: 8 rows x the whole width, or a part of it where there are few rows (and, of fp32 rows, more than a CTA keeps in registers)
   const int row_groups = pl.tok_tiles * pl.nt / 8, n_chunks = kgroups * 16;
   const int parts = row_groups >= n_sm || (f32 && n_chunks <= SPLIT_HOLD * SPLIT_THREADS / 8) ? 1 : (row_groups * 4 >= n_sm || n_chunks < 256 ? 4 : 8);
@@ -732,9 +749,9 @@ int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtyp
   else
     B200Q_CHECK_CUDA(cudaLaunchKernelEx(&cfg, split_rows_kernel<__half, false>, (const __half*)x, (const __half*)nullptr, 0.f, m, n_in, kgroups, pl.nt, per,
                                         (unsigned char*)p.xt, p.counters, n_counters, (float*)nullptr, 0.f));
-#define STREAM_CASE(QT) (pl.wt == 256 ? (f32 ? launch_stream<QT, 256, true, 1>(p, grid, st) : launch_stream<QT, 256, false, 1>(p, grid, st)) \
-                         : pl.nt > 64 ? (f32 ? launch_stream<QT, 128, true, 1>(p, grid, st) : launch_stream<QT, 128, false, 1>(p, grid, st)) \
-                                      : (f32 ? launch_stream<QT, 128, true, 4>(p, grid, st) : launch_stream<QT, 128, false, 4>(p, grid, st)))
+#define STREAM_CASE(QT) (takes_tmem(pl, f32) ? (f32 ? launch_tmem<QT, true>(p, grid, st) : launch_tmem<QT, false>(p, grid, st)) \
+                         : pl.wt == 256 ? (f32 ? launch_stream<QT, 256, true>(p, grid, st) : launch_stream<QT, 256, false>(p, grid, st)) \
+                                        : launch_stream<QT, 128, true>(p, grid, st))
   return qtype == B200Q_Q4_0 ? STREAM_CASE(B200Q_Q4_0) : STREAM_CASE(B200Q_Q8_0);
 #undef STREAM_CASE
 }

@@ -87,13 +87,13 @@ __device__ __forceinline__ uint4 q8_core(uint32_t wa, uint32_t wb, uint32_t d2, 
   return hi_lo(r, d2, lo);
 }
 // the 8 nibbles of a word (4 bytes of a block: low nibbles = elements i .. i + 3, high nibbles = elements i + 16 ..) as fp16 pairs of q - 8:
-// a nibble in bits 4..7 under the exponent of 64 reads 64 + q.  One shift for all but one pair, and no multiply for the high nibbles.
+// a nibble in bits 0..3 under the exponent of 1024 reads 1024 + q, in bits 4..7 under that of 64 it reads 64 + q.  One shift, no multiply.
 __device__ __forceinline__ void q4_word(uint32_t w, uint32_t (&v)[4]) {      // v: {e0,e2}, {e1,e3}, {e16,e18}, {e17,e19}
-  const uint32_t M = 0x00F000F0u, E = 0x54005400u, O = 0x54805480u;         // 64, 72
-  v[0] = h2sub(lop3_and_or(w << 4, M, E), O);
-  v[1] = h2sub(lop3_and_or(w >> 4, M, E), O);
-  v[2] = h2sub(lop3_and_or(w, M, E), O);
-  v[3] = h2sub(lop3_and_or(w >> 8, M, E), O);
+  const uint32_t u = w >> 8;
+  v[0] = h2sub(lop3_and_or(w, 0x000F000Fu, 0x64006400u), 0x64086408u);
+  v[1] = h2sub(lop3_and_or(u, 0x000F000Fu, 0x64006400u), 0x64086408u);
+  v[2] = h2sub(lop3_and_or(w, 0x00F000F0u, 0x54005400u), 0x54805480u);
+  v[3] = h2sub(lop3_and_or(u, 0x00F000F0u, 0x54005400u), 0x54805480u);
 }
 
 // 8 fp32 values -> a chunk of 8 fp16 high parts and one of the remainders' fp16 roundings, in the unpack's element order
