@@ -218,25 +218,30 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
           // the record in pieces on one barrier: a single bulk copy is served slowly, several overlap
           const uint32_t bytes = (uint32_t)p.kgroups * XQ_GROUP_BYTES, piece = 8 * XQ_GROUP_BYTES;
           mbar_expect_tx(xbar, bytes);
+#pragma unroll 1
           for (uint32_t o = 0; o < bytes; o += piece)
             bulk_g2s(smem_u32(record) + o, reinterpret_cast<const unsigned char*>(p.xq_in) + o, min(piece, bytes - o), xbar);
         }
         x_issued = true;
       };
       const int run = XQ_OUT ? p.unit : 1;
+#pragma unroll 1
       for (int unit = blockIdx.x; unit < p.n_units && ok; unit += gridDim.x) {
+#pragma unroll 1
         for (int ti = 0; ti < run && ok; ti++) {
           const int rt = unit * run + ti;
           if (rt >= p.n_row_tiles) break;
           const bool second = QT == K_MIX && rt >= p.tiles_first;
           const int TB = QT == K_MIX ? tile_bytes(second ? B200Q_Q6_K_WIDE : B200Q_Q4_K_WIDE) : tile_bytes(QT);
           const uint8_t* src = second ? p.w2 + (size_t)(rt - p.tiles_first) * p.kgroups * TB : p.w + (size_t)rt * p.kgroups * TB;
+#pragma unroll 1
           for (int s = 0; s < stages_per_tile; s++, it++) {
             const int slot = it % NS, groups = min(SG, p.kgroups - s * SG);
             if (it == NS && !x_issued) after_prefetch();
             if (!mbar_wait(empty0 + 8 * slot, ((it / NS) & 1) ^ 1)) { ok = false; break; }
             mbar_expect_tx(full0 + 8 * slot, groups * TB);
             // one stage = several bulk copies on the same barrier: a single copy is served slowly, several overlap
+#pragma unroll 1
             for (int g0 = 0; g0 < groups; g0 += COPY_GROUPS) {
               const int gn = min(COPY_GROUPS, groups - g0);
               bulk_g2s(smem_u32(ring + slot * STAGE_BYTES + g0 * TB), src + (size_t)(s * SG + g0) * TB, gn * TB, full0 + 8 * slot);
@@ -246,6 +251,7 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
       }
       if (!x_issued) after_prefetch();
       // nothing may still be landing in this CTA's shared memory when it exits
+#pragma unroll 1
       for (int j = max(0, it - NS); j < it; j++) mbar_wait(full0 + 8 * (j % NS), (j / NS) & 1);
       if (XQ_IN) mbar_wait(xbar, 0);
     } else {
@@ -271,7 +277,9 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
     unsigned pend_prev = 0;
     bool ok = true;
     const int run = XQ_OUT ? p.unit : 1;
+#pragma unroll 1
     for (int unit = blockIdx.x; unit < p.n_units && ok; unit += gridDim.x) {
+#pragma unroll 1
       for (int ti = 0; ti < run; ti++, n++) {
         const int rt = unit * run + ti;
         if (rt >= p.n_row_tiles) break;
@@ -306,6 +314,7 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
             }
             if (p.n_peers) {
               const uint32_t bits = mailbox_bits(v);
+#pragma unroll 1
               for (int d = 0; d < p.n_peers; d++) mailbox_store(p.peer[d] + (size_t)p.peer_rank * p.n_out + row, bits);
             }
           }
@@ -379,6 +388,7 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
         wide_row_scale(amax, x_up, x_down);
       }
     }
+#pragma unroll 1
     for (int w0 = warp * 8; w0 < nblk_pad; w0 += PF * BSTEP) {          // 8 blocks per warp and round
       const int b0 = w0 + (lane >> 2);
       float4 v[PF][2];
@@ -440,7 +450,9 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
   int it = 0, n = 0;
   bool live = *s_abort == 0;
   const int run = XQ_OUT ? p.unit : 1;
+#pragma unroll 1
   for (int unit = blockIdx.x; unit < p.n_units && live; unit += gridDim.x) {
+#pragma unroll 1
     for (int ti = 0; ti < run; ti++, n++) {
       const int rt = unit * run + ti;
       if (rt >= p.n_row_tiles) break;
@@ -448,6 +460,7 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
       const int TB = QT == K_MIX ? tile_bytes(second ? B200Q_Q6_K_WIDE : B200Q_Q4_K_WIDE) : tile_bytes(QT);
       float acc0 = 0.f, acc1 = 0.f;
       [[maybe_unused]] float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
       for (int s = 0; s < stages_per_tile; s++, it++) {
         const int slot = it % NS, groups = min(SG, p.kgroups - s * SG);
         if (!mbar_wait(full0 + 8 * slot, (it / NS) & 1)) { *s_abort = 1; break; }

@@ -34,8 +34,10 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 #endif
   return ok != 0;
 }
-// Bounded wait: false (and the status word set) if the phase did not complete in time.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+// Bounded wait: false (and the status word set) if the phase did not complete in time.  The first try is inline, the loop is not: unrolled in a dozen places it was
+// a large part of kernels whose time is partly that of fetching their instructions.
+__device__ __noinline__ bool mbar_wait_on(uint32_t bar, uint32_t parity) {
+#pragma unroll 1
   for (int i = 0; i < SPIN_LIMIT; i++) {
     if (mbar_try(bar, parity)) return true;
     if (i > 1024) __nanosleep(128);      // (sleeping after every failed try measured 0.7 % slower)
@@ -43,6 +45,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   atomicExch(&g_status, 1);
   return false;
 }
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) { return mbar_try(bar, parity) || mbar_wait_on(bar, parity); }
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
                : "memory");
