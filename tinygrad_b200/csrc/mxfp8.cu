@@ -97,16 +97,16 @@ __global__ void swiglu_quant_kernel(const __nv_bfloat16* __restrict__ h, int64_t
 // descending order, weights = softmax over the k.  mode 1 (tinygrad/llm/model.py:118,123-124 with the OLMoE defaults):
 // scores = softmax over all experts, top-k listed in ascending order of score, weights = the scores, not renormalised.
 // Ties: the lower expert index ranks higher (model.py:35-41).
-constexpr int MAX_E_PER_LANE = 8;   // up to 256 experts
+constexpr int MAX_E_PER_LANE = 8;   // up to 256 experts; EPL: what a lane has of the number at hand, 1, 2 or 8 (32, 64, 256)
 
 // One token by one warp; s_topi (optional): shared memory that gets the choices too.
-__device__ __forceinline__ void route_topk_token(const float* __restrict__ logits, int tok, int n_experts, int k, int mode, int32_t* __restrict__ topi,
+template <int EPL> __device__ __forceinline__ void route_topk_token(const float* __restrict__ logits, int tok, int n_experts, int k, int mode, int32_t* __restrict__ topi,
                                                  float* __restrict__ weights, int* s_topi) {
   const int lane = threadIdx.x & 31;
-  float v[MAX_E_PER_LANE];
+  float v[EPL];
   float mx = -INFINITY;
 #pragma unroll
-  for (int i = 0; i < MAX_E_PER_LANE; i++) {
+  for (int i = 0; i < EPL; i++) {
     const int e = i * 32 + lane;
     v[i] = e < n_experts ? logits[(size_t)tok * n_experts + e] : -INFINITY;
     mx = fmaxf(mx, v[i]);
@@ -115,21 +115,22 @@ __device__ __forceinline__ void route_topk_token(const float* __restrict__ logit
   float denom = 0.f;
   if (mode == 1) {
 #pragma unroll
-    for (int i = 0; i < MAX_E_PER_LANE; i++) denom += (i * 32 + lane < n_experts) ? expf(v[i] - mx) : 0.f;
+    for (int i = 0; i < EPL; i++) denom += (i * 32 + lane < n_experts) ? expf(v[i] - mx) : 0.f;
     denom = warp_sum(denom);
   }
   float top1 = 0.f, ksum = 0.f;
+#pragma unroll 1
   for (int j = 0; j < k; j++) {
     float bv = -INFINITY; int bi = 0x7fffffff;
 #pragma unroll
-    for (int i = 0; i < MAX_E_PER_LANE; i++) { const int e = i * 32 + lane; if (v[i] > bv) { bv = v[i]; bi = e; } }   // lowest index wins inside a lane
+    for (int i = 0; i < EPL; i++) { const int e = i * 32 + lane; if (v[i] > bv) { bv = v[i]; bi = e; } }   // lowest index wins inside a lane
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const float ov = __shfl_xor_sync(0xffffffffu, bv, o); const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
       if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
     }
 #pragma unroll
-    for (int i = 0; i < MAX_E_PER_LANE; i++) if (i * 32 + lane == bi) v[i] = -INFINITY;    // taken
+    for (int i = 0; i < EPL; i++) if (i * 32 + lane == bi) v[i] = -INFINITY;    // taken
     if (j == 0) top1 = bv;
     const int slot = mode == 1 ? k - 1 - j : j;
     float w;
@@ -152,13 +153,13 @@ __device__ __forceinline__ void route_topk_token(const float* __restrict__ logit
 // The reference's own shortcut is applied by the caller: SOFTMAX with normalize and no bias is run as SOFTMAX_WEIGHT (model.py:116-117).
 enum { GATE_SOFTMAX = 1, GATE_SIGMOID = 2, GATE_SOFTMAX_WEIGHT = 3, GATE_SQRT_SOFTPLUS = 4 };     // ExpertGating, model.py:9-13
 
-__device__ __forceinline__ void route_gating_token(const float* __restrict__ logits, const float* __restrict__ sel_bias, int tok, int n_experts, int k, int gating,
+template <int EPL> __device__ __forceinline__ void route_gating_token(const float* __restrict__ logits, const float* __restrict__ sel_bias, int tok, int n_experts, int k, int gating,
                                                    int normalize, float scale, int32_t* __restrict__ topi, float* __restrict__ weights, int* s_topi) {
   const int lane = threadIdx.x & 31;
-  float sc[MAX_E_PER_LANE], key[MAX_E_PER_LANE];
+  float sc[EPL], key[EPL];
   float mx = -INFINITY;
 #pragma unroll
-  for (int i = 0; i < MAX_E_PER_LANE; i++) {
+  for (int i = 0; i < EPL; i++) {
     const int e = i * 32 + lane;
     sc[i] = e < n_experts ? logits[(size_t)tok * n_experts + e] : -INFINITY;
     mx = fmaxf(mx, sc[i]);
@@ -167,34 +168,35 @@ __device__ __forceinline__ void route_gating_token(const float* __restrict__ log
     mx = warp_max(mx);
     float denom = 0.f;
 #pragma unroll
-    for (int i = 0; i < MAX_E_PER_LANE; i++) { if (i * 32 + lane < n_experts) { sc[i] = expf(sc[i] - mx); denom += sc[i]; } }
+    for (int i = 0; i < EPL; i++) { if (i * 32 + lane < n_experts) { sc[i] = expf(sc[i] - mx); denom += sc[i]; } }
     denom = warp_sum(denom);
 #pragma unroll
-    for (int i = 0; i < MAX_E_PER_LANE; i++) if (i * 32 + lane < n_experts) sc[i] /= denom;
+    for (int i = 0; i < EPL; i++) if (i * 32 + lane < n_experts) sc[i] /= denom;
   } else if (gating == GATE_SIGMOID) {
 #pragma unroll
-    for (int i = 0; i < MAX_E_PER_LANE; i++) if (i * 32 + lane < n_experts) sc[i] = 1.f / (1.f + expf(-sc[i]));
+    for (int i = 0; i < EPL; i++) if (i * 32 + lane < n_experts) sc[i] = 1.f / (1.f + expf(-sc[i]));
   } else if (gating == GATE_SQRT_SOFTPLUS) {
 #pragma unroll
-    for (int i = 0; i < MAX_E_PER_LANE; i++) if (i * 32 + lane < n_experts) sc[i] = sqrtf(sc[i] > 20.f ? sc[i] : log1pf(expf(sc[i])));
+    for (int i = 0; i < EPL; i++) if (i * 32 + lane < n_experts) sc[i] = sqrtf(sc[i] > 20.f ? sc[i] : log1pf(expf(sc[i])));
   }
 #pragma unroll
-  for (int i = 0; i < MAX_E_PER_LANE; i++) {
+  for (int i = 0; i < EPL; i++) {
     const int e = i * 32 + lane;
     key[i] = e < n_experts ? (sel_bias ? sc[i] + sel_bias[e] : sc[i]) : -INFINITY;
   }
   float pv = 0.f;                        // lane j < k keeps the probability of slot j
+#pragma unroll 1
   for (int j = 0; j < k; j++) {
     float bv = -INFINITY, bs = 0.f; int bi = 0x7fffffff;
 #pragma unroll
-    for (int i = 0; i < MAX_E_PER_LANE; i++) { const int e = i * 32 + lane; if (key[i] > bv) { bv = key[i]; bs = sc[i]; bi = e; } }
+    for (int i = 0; i < EPL; i++) { const int e = i * 32 + lane; if (key[i] > bv) { bv = key[i]; bs = sc[i]; bi = e; } }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const float ov = __shfl_xor_sync(0xffffffffu, bv, o), os = __shfl_xor_sync(0xffffffffu, bs, o); const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
       if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bs = os; bi = oi; }
     }
 #pragma unroll
-    for (int i = 0; i < MAX_E_PER_LANE; i++) if (i * 32 + lane == bi) key[i] = -INFINITY;    // taken
+    for (int i = 0; i < EPL; i++) if (i * 32 + lane == bi) key[i] = -INFINITY;    // taken
     const int slot = k - 1 - j;          // ascending order of rank
     if (lane == slot) pv = bs;
     if (lane == 0) { topi[(size_t)tok * k + slot] = bi; if (s_topi) s_topi[tok * k + slot] = bi; }
@@ -212,16 +214,18 @@ __device__ __forceinline__ void route_gating_token(const float* __restrict__ log
 // How a call chooses: gating 0 = `mode` of route_topk_token, else an ExpertGating.
 struct RouteRule { int mode, gating, normalize; float scale; const float* sel_bias; };
 
+template <int EPL>
 __device__ __forceinline__ void route_token(const RouteRule& r, const float* logits, int tok, int n_experts, int k, int32_t* topi, float* weights, int* s_topi) {
-  if (r.gating) route_gating_token(logits, r.sel_bias, tok, n_experts, k, r.gating, r.normalize, r.scale, topi, weights, s_topi);
-  else route_topk_token(logits, tok, n_experts, k, r.mode, topi, weights, s_topi);
+  if (r.gating) route_gating_token<EPL>(logits, r.sel_bias, tok, n_experts, k, r.gating, r.normalize, r.scale, topi, weights, s_topi);
+  else route_topk_token<EPL>(logits, tok, n_experts, k, r.mode, topi, weights, s_topi);
 }
+template <int EPL>
 __global__ void route_choose_kernel(const RouteRule r, const float* __restrict__ logits, int n_tokens, int n_experts, int k, int32_t* __restrict__ topi,
                                     float* __restrict__ weights) {
   pdl_launch_dependents();
   pdl_wait();
   const int tok = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (tok < n_tokens) route_token(r, logits, tok, n_experts, k, topi, weights, nullptr);
+  if (tok < n_tokens) route_token<EPL>(r, logits, tok, n_experts, k, topi, weights, nullptr);
 }
 
 // routing, steps 2-4: stable counting sort of the T*k (token, slot) pairs by expert.
@@ -234,6 +238,7 @@ __device__ __forceinline__ void route_offsets(const int* tot, int n_experts, int
                                               int* s_off) {
   const int lane = threadIdx.x & 31;
   int carry = 0;
+#pragma unroll 1
   for (int e0 = 0; e0 < n_experts; e0 += 32) {
     const int e = e0 + lane, n = e < n_experts ? tot[e] : 0, padded = (n + pad - 1) / pad * pad;
     int incl = padded;
@@ -252,8 +257,10 @@ __device__ __forceinline__ void route_offsets(const int* tot, int n_experts, int
 }
 
 // The whole routing of at most ROUTE_CHUNK pairs and ROUTE_ONE_TOKENS tokens in one CTA: a warp per token, then the counting sort in shared memory.
-// As four launches it took 18.5 us whatever the size, nearly all of it launches.  logits == nullptr: the choices are there already (topi).
-constexpr int ROUTE_ONE_TOKENS = 256;
+// As four launches it took 18.5 us whatever the size, nearly all of it launches.  logits == nullptr: the choices are there already (topi); more tokens than warps are
+// chosen for by a kernel of their own in front: 256 tokens x 4 took 34.5 us as eight tokens a warp here, 5.1 so; 64 x 2 6.9, 3.7.
+constexpr int ROUTE_ONE_TOKENS = 32;
+template <int EPL>
 __global__ void __launch_bounds__(ROUTE_CHUNK) route_one_kernel(const RouteRule r, const float* __restrict__ logits, int n_tokens, int n_experts, int k, int pad,
                                                                 int32_t* __restrict__ topi, float* __restrict__ weights, int32_t* __restrict__ dest_row,
                                                                 int32_t* __restrict__ off, int32_t* __restrict__ counts, int32_t* __restrict__ ends) {
@@ -263,8 +270,10 @@ __global__ void __launch_bounds__(ROUTE_CHUNK) route_one_kernel(const RouteRule 
   for (int i = threadIdx.x; i < n_warps * n_experts; i += ROUTE_CHUNK) s_wcnt[i] = 0;
   pdl_launch_dependents();
   pdl_wait();
-  if (logits) for (int tok = warp; tok < n_tokens; tok += ROUTE_CHUNK / 32) route_token(r, logits, tok, n_experts, k, topi, weights, s_topi);
-  else for (int i = threadIdx.x; i < n; i += ROUTE_CHUNK) s_topi[i] = topi[i];
+  if (logits) {
+#pragma unroll 1
+    for (int tok = warp; tok < n_tokens; tok += ROUTE_CHUNK / 32) route_token<EPL>(r, logits, tok, n_experts, k, topi, weights, s_topi);
+  } else for (int i = threadIdx.x; i < n; i += ROUTE_CHUNK) s_topi[i] = topi[i];
   __syncthreads();
   const int i = threadIdx.x, e = i < n ? s_topi[i] : -1;
   const unsigned same = __match_any_sync(0xffffffffu, e);
@@ -301,8 +310,10 @@ __global__ void __launch_bounds__(ROUTE_CHUNK) route_scan_kernel(int32_t* __rest
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   pdl_launch_dependents();
   pdl_wait();
+#pragma unroll 1
   for (int e = warp; e < n_experts; e += ROUTE_CHUNK / 32) {
     int run = 0;
+#pragma unroll 1
     for (int c0 = 0; c0 < n_chunks; c0 += 32) {
       const int c = c0 + lane, v = c < n_chunks ? counts[(size_t)c * n_experts + e] : 0;
       int incl = v;
@@ -441,16 +452,20 @@ int combine_launch(const void* y_bf16, const int32_t* dest_row, const float* wei
 int route_launch(const RouteRule& r, const float* logits, int n_tokens, int n_experts, int k, int pad, int32_t* topi, float* weights, int32_t* dest_row, int32_t* off,
                  int32_t* counts, int32_t* ends, void* scratch, cudaStream_t st, bool pdl) {
   const int n = n_tokens * k, n_chunks = ceil_div(n, ROUTE_CHUNK);
-  if (n <= ROUTE_CHUNK && n_tokens <= ROUTE_ONE_TOKENS) {
+  const bool one = n <= ROUTE_CHUNK;
+  if (logits && !(one && n_tokens <= ROUTE_ONE_TOKENS)) {
+    auto choose = n_experts <= 32 ? route_choose_kernel<1> : n_experts <= 64 ? route_choose_kernel<2> : route_choose_kernel<MAX_E_PER_LANE>;
+    B200Q_CHECK_CUDA(launch_k(choose, dim3(ceil_div(n_tokens, 8)), dim3(256), 0, st, pdl, r, logits, n_tokens, n_experts, k, topi, weights));
+    pdl = true;
+    logits = nullptr;
+  }
+  if (one) {
     const size_t smem = (ROUTE_CHUNK + (2 + (size_t)ceil_div(n, 32)) * n_experts) * sizeof(int);      // at most 38 KB
-    B200Q_CHECK_CUDA(launch_k(route_one_kernel, dim3(1), dim3(ROUTE_CHUNK), smem, st, pdl, r, logits, n_tokens, n_experts, k, pad, topi, weights, dest_row, off, counts, ends));
+    auto sort = n_experts <= 32 ? route_one_kernel<1> : n_experts <= 64 ? route_one_kernel<2> : route_one_kernel<MAX_E_PER_LANE>;
+    B200Q_CHECK_CUDA(launch_k(sort, dim3(1), dim3(ROUTE_CHUNK), smem, st, pdl, r, logits, n_tokens, n_experts, k, pad, topi, weights, dest_row, off, counts, ends));
     return B200Q_OK;
   }
   int32_t* cnt = (int32_t*)scratch;
-  if (logits) {
-    B200Q_CHECK_CUDA(launch_k(route_choose_kernel, dim3(ceil_div(n_tokens, 8)), dim3(256), 0, st, pdl, r, logits, n_tokens, n_experts, k, topi, weights));
-    pdl = true;
-  }
   B200Q_CHECK_CUDA(launch_k(route_count_kernel, dim3(n_chunks), dim3(ROUTE_CHUNK), n_experts * sizeof(int), st, pdl, topi, n, n_experts, cnt));
   B200Q_CHECK_CUDA(launch_k(route_scan_kernel, dim3(1), dim3(ROUTE_CHUNK), n_experts * sizeof(int), st, true, cnt, n_chunks, n_experts, off, pad, counts, ends));
   B200Q_CHECK_CUDA(launch_k(route_place_kernel, dim3(n_chunks), dim3(ROUTE_CHUNK), 32 * n_experts * sizeof(int), st, true, topi, n, n_experts, cnt, off, dest_row));
