@@ -64,6 +64,7 @@ __device__ __forceinline__ uint64_t desc_sw128(uint32_t saddr) {
   return d;
 }
 __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+#pragma unroll 1
   for (int i = 0; i < SPIN; i++) {
     uint32_t ok;
     asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
@@ -112,13 +113,17 @@ __device__ __forceinline__ void swiglu_quant_store(const uint32_t (&vg)[32], con
 // fp32 results with the per-tensor FP8 linear's last steps: y = acc * *fw * *fx + bias in y's type, for the first `rows` rows (fw NULL: plain sums)
 struct ScaledOut { const float *fw, *fx, *bias; int rows, y_f16; };
 
+// What becomes of the sums: bf16 rows, SwiGLU of gate and up requantised, the FP8 linear's results, fp32 sums.  One kernel each: the registers of one epilogue are not
+// another's, and an expert layer of few rows does not fetch the instructions of all four.
+enum { OUT_BF16, OUT_SWIGLU, OUT_SCALED, OUT_F32 };
+template <int OUT>
 __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint8_t* __restrict__ a_q, const uint8_t* __restrict__ a_e8,
                                                                       const uint8_t* __restrict__ b_q, const uint8_t* __restrict__ b_e8,
                                                                       const int32_t* __restrict__ off, int n_experts, int m_total, int n, int k,
                                                                       __nv_bfloat16* __restrict__ c, uint8_t* __restrict__ act_q,
                                                                       uint8_t* __restrict__ act_e8, const __grid_constant__ CUtensorMap tm_a,
                                                                       const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_c,
-                                                                      int c_f32, const ScaledOut so, const int32_t* __restrict__ ends) {
+                                                                      const ScaledOut so, const int32_t* __restrict__ ends) {
   extern __shared__ unsigned char sm_raw[];
   __shared__ __align__(8) uint64_t bar_full[STAGES], bar_empty[STAGES], bar_acc_full, bar_acc_empty, bar_drain;
   __shared__ uint32_t tmem_base;
@@ -144,13 +149,14 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
   // row tiles of the rows each group has (`ends`: without its padding); everything else of the padded layout is left alone
   if (warp == 0) {
     int carry = 0;
+#pragma unroll 1
     for (int e0 = 0; e0 < n_experts; e0 += 32) {
       const int e = e0 + lane;
       int lo = 0, tiles = 0;
       if (e < n_experts) {
         lo = min(max(off[e], 0), m_total);
         int hi = min(max(ends ? ends[e] : off[e + 1], lo), m_total);
-        if (so.fw) hi = min(hi, max(so.rows, lo));
+        if (OUT == OUT_SCALED) hi = min(hi, max(so.rows, lo));
         tiles = min((hi - lo + BM - 1) / BM, (m_total - lo) / BM);
       }
       int incl = tiles;
@@ -189,9 +195,11 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
     };
     uint32_t g = 0;
     bool ok = true;
+#pragma unroll 1
     for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
       const uint8_t *ae, *be;
       tile_ptrs(t, ae, be);
+#pragma unroll 1
       for (int kt = 0; kt < ktiles; kt++, g++) {
         const uint32_t slot = g % STAGES;
         if (g >= STAGES && !wait_bar(s32(&bar_empty[slot]), ((g / STAGES) - 1) & 1, abort_flag)) { ok = false; break; }
@@ -217,6 +225,7 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
     if (lt == 0)
       for (uint32_t j = g > STAGES ? g - STAGES : 0; j < g; j++) {
         const uint32_t fb = s32(&bar_full[j % STAGES]), par = (j / STAGES) & 1;
+#pragma unroll 1
         for (int i = 0; i < SPIN; i++) {
           uint32_t done;
           asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(done) : "r"(fb), "r"(par) : "memory");
@@ -228,9 +237,11 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
     if (elect_one()) {
       uint32_t g = 0, tile_i = 0;
       bool ok = true;
+#pragma unroll 1
       for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, tile_i++) {
         if (tile_i > 0 && !wait_bar(s32(&bar_acc_empty), (tile_i - 1) & 1, abort_flag)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
         for (int kt = 0; kt < ktiles; kt++, g++) {
           const uint32_t slot = g % STAGES;
           if (!wait_bar(s32(&bar_full[slot]), (g / STAGES) & 1, abort_flag)) { ok = false; break; }
@@ -257,6 +268,7 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
       }
       if (!ok) {     // leave nothing in flight before the tensor memory is given back
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(&bar_drain)) : "memory");
+#pragma unroll 1
         for (int i = 0; i < SPIN; i++) {
           uint32_t done;
           asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(done) : "r"(s32(&bar_drain)) : "memory");
@@ -277,6 +289,7 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
       __syncwarp();
       if (lane == 0) arrive(s32(&bar_acc_empty));
     };
+#pragma unroll 1
     for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, tile_i++) {
       if (!wait_bar(s32(&bar_acc_full), tile_i & 1, abort_flag)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -284,7 +297,7 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
       const uint32_t ta = taddr + ((uint32_t)(sub * 32) << 16);
       const size_t row = (size_t)(m0 + sub * 32 + lane);
       uint32_t v0[32], v1[32];
-      if (act_q) {
+      if constexpr (OUT == OUT_SWIGLU) {
         // Fused activation between the expert GEMMs: the B rows of this tile are 128 gate rows followed by the 128 matching up rows
         // (the caller interleaves them so), so accumulator columns c and 128 + c belong together.  A thread holds 32 consecutive
         // outputs of its row = one MX block: bf16-round gate and up (what the unfused path stores), silu(gate) * up in fp32,
@@ -298,10 +311,26 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
       tmem_ld32(ta + cq * 64, v0); tmem_ld32(ta + cq * 64 + 32, v1);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       release();
-      if (so.fw) {
+      // Results leave through this warp's staging rows (32 rows x 128 bytes, packet p of row r at p ^ (r & 7): conflict-free both ways), which are in the
+      // 128-byte-swizzle layout a tiled tensor-map store reads: one copy of whole 128-byte row segments.  Rows past the tensor's last are not written.
+      unsigned char* const stg = sm_raw + (ring - s32(sm_raw)) + STAGES * STAGE_BYTES + (warp < EPI_WARPS ? warp : warp - (LOAD_WARPS + 1)) * 4096;
+      auto packet = [&](int p) { return stg + lane * 128 + ((p ^ (lane & 7)) << 4); };
+      auto send = [&](int column) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+          asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
+                       ::"l"(&tm_c), "r"(column), "r"(m0 + sub * 32), "r"(s32(stg)) : "memory");
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // the rows may be overwritten
+        }
+        __syncwarp();
+      };
+      if constexpr (OUT == OUT_SCALED) {
+        // (each thread storing its own row, 16 bytes of 32 rows an instruction: 47.7 us for the call of 1000 x 4096 x 4096 with fp32 results, 45.0 so)
         const float w = *so.fw, xf = *so.fx;
         const int col = n0 + cq * 64;
-        if (row < (size_t)so.rows) {
+        if (m0 + sub * 32 < so.rows) {
           float b[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
           for (int j = 0; j < 64; j += 4) {
@@ -313,16 +342,19 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
               o[q] = __fmul_rn(__fmul_rn(__uint_as_float(v[q]), w), xf);      // y * w_scale * x_scale, in that order
               if (so.bias) o[q] = __fadd_rn(o[q], b[q]);
             }
-            const size_t at = row * n + col + j;
             if (so.y_f16) {
               const __half2 h[2] = {__floats2half2_rn(o[0], o[1]), __floats2half2_rn(o[2], o[3])};
-              *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(c) + at) = *reinterpret_cast<const uint2*>(h);
-            } else *reinterpret_cast<float4*>(reinterpret_cast<float*>(c) + at) = make_float4(o[0], o[1], o[2], o[3]);
+              *reinterpret_cast<uint2*>(packet(j >> 3) + (j & 4) * 2) = *reinterpret_cast<const uint2*>(h);
+            } else {
+              *reinterpret_cast<float4*>(packet((j >> 2) & 7)) = make_float4(o[0], o[1], o[2], o[3]);
+              if (j == 28) send(col);
+            }
           }
+          send(so.y_f16 ? col : col + 32);
         }
         continue;
       }
-      if (c_f32) {      // unrounded sums (the per-tensor FP8 linear scales them afterwards): each thread stores its own row
+      if constexpr (OUT == OUT_F32) {      // unrounded sums (the per-tensor FP8 linear scales them afterwards): each thread stores its own row
         float4* o4 = reinterpret_cast<float4*>(reinterpret_cast<float*>(c) + row * n + n0 + cq * 64);
 #pragma unroll
         for (int j = 0; j < 8; j++) {
@@ -332,9 +364,7 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
         continue;
       }
       {
-        // row `lane`, 64 columns = eight 16-byte packets -> this warp's staging rows (packet p of row r at p ^ (r & 7): conflict-free
-        // both ways) -> read back four rows x 128 contiguous bytes per instruction and store those
-        unsigned char* stg = sm_raw + (ring - s32(sm_raw)) + STAGES * STAGE_BYTES + (warp < EPI_WARPS ? warp : warp - (LOAD_WARPS + 1)) * 4096;
+        // row `lane`, 64 columns = eight 16-byte packets
 #pragma unroll
         for (int p8 = 0; p8 < 8; p8++) {
           uint4 pk;
@@ -345,18 +375,9 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
             h[q] = j < 32 ? __floats2bfloat162_rn(__uint_as_float(v0[j]), __uint_as_float(v0[j + 1]))
                           : __floats2bfloat162_rn(__uint_as_float(v1[j - 32]), __uint_as_float(v1[j - 31]));
           }
-          *reinterpret_cast<uint4*>(stg + lane * 128 + ((p8 ^ (lane & 7)) << 4)) = pk;
+          *reinterpret_cast<uint4*>(packet(p8)) = pk;
         }
-        // the staging rows are in the 128-byte-swizzle layout a tiled tensor-map store reads: one copy per warp and tile
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) {
-          asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
-                       ::"l"(&tm_c), "r"(n0 + cq * 64), "r"(m0 + sub * 32), "r"(s32(stg)) : "memory");
-          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // the rows may be overwritten for the next tile
-        }
-        __syncwarp();
+        send(n0 + cq * 64);
       }
     }
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");      // this warp's stores have left before the CTA does
@@ -384,9 +405,9 @@ extern "C" int b200q_mx_status_read_clear(int* status) {
   return B200Q_OK;
 }
 
-// [rows, k] bytes, row-major -> tiled tensor map with boxes of `box_rows` rows x 128 bytes in the 128-byte-swizzle shared-memory layout.
+// [rows, k] elements, row-major -> tiled tensor map with boxes of `box_rows` rows x 128 bytes in the 128-byte-swizzle shared-memory layout.
 // The encoder is a driver entry point; it is looked up through the runtime so that the library links against cudart only.
-static int make_map(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t k, uint32_t box_rows, bool bf16 = false) {
+static int make_map(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t k, uint32_t box_rows, CUtensorMapDataType type = CU_TENSOR_MAP_DATA_TYPE_UINT8, int size = 1) {
   typedef CUresult (*encode_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                 const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
   static encode_fn fn = nullptr;
@@ -397,10 +418,9 @@ static int make_map(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t k
     if (!p || q != cudaDriverEntryPointSuccess) return B200Q_ERR_UNSUPPORTED;
     fn = (encode_fn)p;
   }
-  // bf16: `k` counts elements, a box row is 64 of them (128 bytes); else bytes, a box row is BK = 128 of them
-  const cuuint64_t dims[2] = {k, rows}, strides[1] = {bf16 ? 2 * k : k};
-  const cuuint32_t box[2] = {(cuuint32_t)(bf16 ? 64 : BK), box_rows}, estr[2] = {1, 1};
-  const CUresult r = fn(tm, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
+  const cuuint64_t dims[2] = {k, rows}, strides[1] = {k * size};
+  const cuuint32_t box[2] = {(cuuint32_t)(128 / size), box_rows}, estr[2] = {1, 1};
+  const CUresult r = fn(tm, type, 2, const_cast<void*>(base), dims, strides, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? B200Q_OK : B200Q_ERR_BAD_ARG;
 }
@@ -412,24 +432,30 @@ static int grouped_launch(const void* a_q, const void* a_e8, const void* b_q, co
   if (m_total % 256 || n % BN || k % BK) return B200Q_ERR_BAD_SHAPE;       // the reference asks M % 256 == N % 256 == K % 128 == 0 (moe_gemm.py:120)
   if (n_experts > MAX_EXPERTS) return B200Q_ERR_UNSUPPORTED;
   if (((uintptr_t)a_q | (uintptr_t)b_q | (uintptr_t)c_bf16) & 15 || ((uintptr_t)a_e8 | (uintptr_t)b_e8) & 3) return B200Q_ERR_MISALIGNED;
-  static PerDeviceFlag attr_set;
+  const int out = act_q ? OUT_SWIGLU : so.fw ? OUT_SCALED : c_f32 ? OUT_F32 : OUT_BF16;
+  auto kernel = out == OUT_SWIGLU ? grouped_mxfp8_tc_kernel<OUT_SWIGLU> : out == OUT_SCALED ? grouped_mxfp8_tc_kernel<OUT_SCALED>
+                : out == OUT_F32 ? grouped_mxfp8_tc_kernel<OUT_F32> : grouped_mxfp8_tc_kernel<OUT_BF16>;
+  static PerDeviceFlag attr_set[4];
   const int dev = b200q_current_device(), n_sm = b200q_sm_count();
   if (dev < 0 || n_sm <= 0) return B200Q_ERR_CUDA;
-  if (!attr_set.test(dev)) {
-    B200Q_CHECK_CUDA(cudaFuncSetAttribute(grouped_mxfp8_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-    attr_set.set(dev);
+  if (!attr_set[out].test(dev)) {
+    B200Q_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
+    attr_set[out].set(dev);
   }
   const long long tiles = (long long)(m_total / BM) * (n / BN);
   const int grid = (int)(tiles < n_sm ? tiles : n_sm);
   alignas(64) CUtensorMap tm_a, tm_b, tm_c;
   memset(&tm_a, 0, sizeof(tm_a)); memset(&tm_b, 0, sizeof(tm_b)); memset(&tm_c, 0, sizeof(tm_c));
-  if (c_bf16 && !c_f32) { const int rcc = make_map(&tm_c, c_bf16, (uint64_t)m_total, (uint64_t)n, 32, true); if (rcc != B200Q_OK) return rcc; }
-  int rc = make_map(&tm_a, a_q, (uint64_t)m_total, (uint64_t)k, BM);
+  int rc = B200Q_OK;
+  if (out == OUT_SCALED) rc = so.y_f16 ? make_map(&tm_c, c_bf16, (uint64_t)so.rows, (uint64_t)n, 32, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2)
+                           : make_map(&tm_c, c_bf16, (uint64_t)so.rows, (uint64_t)n, 32, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4);
+  else if (out == OUT_BF16) rc = make_map(&tm_c, c_bf16, (uint64_t)m_total, (uint64_t)n, 32, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2);
+  if (rc == B200Q_OK) rc = make_map(&tm_a, a_q, (uint64_t)m_total, (uint64_t)k, BM);
   if (rc == B200Q_OK) rc = make_map(&tm_b, b_q, (uint64_t)n_experts * n, (uint64_t)k, BN);
   if (rc != B200Q_OK) return rc;
-  B200Q_CHECK_CUDA(launch_k(grouped_mxfp8_tc_kernel, dim3(grid), dim3(THREADS), (size_t)SMEM_BYTES, (cudaStream_t)stream, pdl, (const uint8_t*)a_q, (const uint8_t*)a_e8,
+  B200Q_CHECK_CUDA(launch_k(kernel, dim3(grid), dim3(THREADS), (size_t)SMEM_BYTES, (cudaStream_t)stream, pdl, (const uint8_t*)a_q, (const uint8_t*)a_e8,
                             (const uint8_t*)b_q, (const uint8_t*)b_e8, off, n_experts, m_total, n, k, (__nv_bfloat16*)c_bf16, (uint8_t*)act_q, (uint8_t*)act_e8,
-                            tm_a, tm_b, tm_c, c_f32 ? 1 : 0, so, ends));
+                            tm_a, tm_b, tm_c, so, ends));
   return B200Q_OK;
 }
 
