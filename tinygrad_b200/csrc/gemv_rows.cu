@@ -114,18 +114,18 @@ __global__ void __launch_bounds__(256) rows_record_kernel(const T* __restrict__ 
   }
 }
 
-// 4 x 4 word transpose inside a quad: lane t ends up with word t of lanes 0, 1, 2, 3 (out.x .. out.w).  Two butterfly steps (2 x 2
-// words between lanes t and t ^ 1, then 2 x 2 pairs between t and t ^ 2): four shuffles and twelve selects on two lane-constant bits.
-__device__ __forceinline__ uint4 quad_transpose(const uint4 r, int t) {
-  const bool b0 = (t & 1) != 0, b1 = (t & 2) != 0;
-  uint32_t s0 = b0 ? r.x : r.y, s1 = b0 ? r.z : r.w;             // odd lanes give away words 0, 2; even lanes words 1, 3
-  s0 = __shfl_xor_sync(0xffffffffu, s0, 1); s1 = __shfl_xor_sync(0xffffffffu, s1, 1);
-  const uint32_t x = b0 ? s0 : r.x, y = b0 ? r.y : s0, z = b0 ? s1 : r.z, w = b0 ? r.w : s1;
-  uint32_t u0 = b1 ? x : z, u1 = b1 ? y : w;                     // lanes 2, 3 give away the first pair, lanes 0, 1 the second
-  u0 = __shfl_xor_sync(0xffffffffu, u0, 2); u1 = __shfl_xor_sync(0xffffffffu, u1, 2);
-  uint4 o;
-  o.x = b1 ? u0 : x; o.y = b1 ? u1 : y; o.z = b1 ? z : u0; o.w = b1 ? w : u1;
-  return o;
+// 32 lanes' 16 bytes of a tile (lane 4 g + b: row g, block b) as the MMA wants them: lane (g, t) gets word t of row g of blocks 0 .. 3 (out.x .. out.w), which is what
+// ldmatrix does with a row of 16 bytes.  Rows are 64 bytes apart, eight to a matrix: taken block by block they would meet four to a bank, so matrix m holds block
+// (m + g / 2) % 4 of row g, and the registers are turned back by selects.  As a 16-byte load and two butterfly steps of shuffles and selects (4 + 12) it was nearly
+// half of a Q8_0 tile's instructions: 32 steps of 8 sequences on seven 7B-shaped blocks and their prompts 31.7 ms, 29.0 so (29.4 with two rows to a bank and 4 selects).
+__device__ __forceinline__ uint4 tile_words(const uint8_t* tile, int lane) {
+  const int m = lane >> 3, g = lane & 7;      // this lane's address: row g of matrix m
+  uint32_t r0, r1, r2, r3;
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(smem_u32(tile) + g * 64 + ((m + (g >> 1)) & 3) * 16) : "memory");
+  const bool odd = lane & 8, two = lane & 16; // register i holds block (i + row / 2) % 4, row = lane / 4
+  const uint32_t s0 = odd ? r3 : r0, s1 = odd ? r0 : r1, s2 = odd ? r1 : r2, s3 = odd ? r2 : r3;
+  return make_uint4(two ? s2 : s0, two ? s3 : s1, two ? s0 : s2, two ? s1 : s3);
 }
 
 __device__ __forceinline__ void imma_u8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -141,18 +141,17 @@ __device__ __forceinline__ void imma_s8(int (&c)[4], uint32_t a0, uint32_t a1, u
 // {scale, offset} pairs of the lane's two activation rows (2t, 2t + 1) for the 4 blocks.  acc: rows g / g + 8 x activation rows 2t / 2t + 1.
 template <int QT>
 __device__ __forceinline__ void tile_mac_rows(const uint8_t* tile, int lane, const uint4 (&xw)[4], const float4 (&xs)[4], float (&acc)[4]) {
-  const int g = lane >> 2, t = lane & 3;
-  const uint4* tp = reinterpret_cast<const uint4*>(tile);
+  const int g = lane >> 2;
   const uint32_t M = 0x0F0F0F0Fu;
   uint32_t a[4][4];      // [block][a0..a3]
   if (QT == B200Q_Q4_0) {
-    const uint4 w0 = quad_transpose(tp[lane], t), w1 = quad_transpose(tp[32 + lane], t);      // rows g, g + 8: word t of blocks 0..3
+    const uint4 w0 = tile_words(tile, lane), w1 = tile_words(tile + 512, lane);      // rows g, g + 8: word t of blocks 0..3
     const uint32_t r0[4] = {w0.x, w0.y, w0.z, w0.w}, r1[4] = {w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
     for (int b = 0; b < 4; b++) { a[b][0] = r0[b] & M; a[b][1] = r1[b] & M; a[b][2] = (r0[b] >> 4) & M; a[b][3] = (r1[b] >> 4) & M; }
   } else {
-    const uint4 w0 = quad_transpose(tp[lane], t), w2 = quad_transpose(tp[32 + lane], t);      // row g: elements 0..15, 16..31 of the lane's block
-    const uint4 w1 = quad_transpose(tp[64 + lane], t), w3 = quad_transpose(tp[96 + lane], t); // row g + 8
+    const uint4 w0 = tile_words(tile, lane), w2 = tile_words(tile + 512, lane);      // row g: elements 0..15, 16..31 of the lane's block
+    const uint4 w1 = tile_words(tile + 1024, lane), w3 = tile_words(tile + 1536, lane); // row g + 8
     const uint32_t r0[4] = {w0.x, w0.y, w0.z, w0.w}, r2[4] = {w2.x, w2.y, w2.z, w2.w}, r1[4] = {w1.x, w1.y, w1.z, w1.w}, r3[4] = {w3.x, w3.y, w3.z, w3.w};
 #pragma unroll
     for (int b = 0; b < 4; b++) { a[b][0] = r0[b]; a[b][1] = r1[b]; a[b][2] = r2[b]; a[b][3] = r3[b]; }
