@@ -41,12 +41,14 @@ def test_rows_against_the_exact_product(typ, m, n_out, n_in, dt, split):
   assert (np.abs(y.numpy() - ref) <= bound).all(), f"worst {np.max(np.abs(y.numpy() - ref) / bound):.2f} of the bound"
 
 
-# weights through tensor memory: whole tiles between split ones, with and without room for them in shared memory (112 rows of Q4_0, Q8_0), tiles of one K group, one slot
-# of weights per thread group and two, the most rows of either type
+# Weights through tensor memory: whole tiles between split ones, with and without room for them in shared memory (112 rows of Q4_0, Q8_0), tiles of one K group, the most
+# rows of either type; and either side of the lines where shared memory takes over (32 rows; 4 K groups an SM up to 64, 10 above; 8 CTAs a tile).
 @pytest.mark.parametrize("split", [True, False])
-@pytest.mark.parametrize("typ,m,n_out,n_in,dt", [(2, 45, 51216, 416, np.float32), (8, 112, 38144, 288, np.float32), (2, 112, 40000, 160, np.float32), (8, 3, 57000, 96, np.float32),
-                                                 (2, 128, 1000, 4000, np.float32), (8, 128, 260, 14336, np.float32), (2, 100, 40000, 288, np.float16), (8, 256, 1300, 992, np.float16),
-                                                 (2, 160, 2000, 2080, np.float16), (2, 33, 16, 18944, np.float32)])
+@pytest.mark.parametrize("typ,m,n_out,n_in,dt", [(2, 45, 51216, 416, np.float32), (8, 112, 38144, 640, np.float32), (2, 112, 64000, 416, np.float32), (8, 3, 57000, 96, np.float32),
+                                                 (2, 128, 12800, 2080, np.float32), (2, 100, 40000, 288, np.float16), (8, 256, 1300, 992, np.float16), (2, 160, 2000, 2080, np.float16),
+                                                 (2, 32, 1030, 2048, np.float32), (2, 33, 1030, 2048, np.float32), (8, 64, 18950, 512, np.float32), (8, 64, 18800, 512, np.float32),
+                                                 (8, 65, 18950, 1280, np.float32), (8, 65, 18800, 1280, np.float32), (2, 33, 16, 18944, np.float32), (8, 16, 300, 6144, np.float32),
+                                                 (8, 16, 300, 6400, np.float32), (2, 100, 100, 2048, np.float16), (2, 100, 100, 2176, np.float16)])
 def test_weights_through_tensor_memory(typ, m, n_out, n_in, dt, split): test_rows_against_the_exact_product(typ, m, n_out, n_in, dt, split)
 
 

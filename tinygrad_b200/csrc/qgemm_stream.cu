@@ -293,7 +293,7 @@ __device__ __forceinline__ bool finish_segment(const StreamParams& p, Shared& sh
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = warp & 3, q = warp >> 2;
   const int hf = WT == 256 ? q >> 1 : 0, part0 = WT == 256 ? q & 1 : q, parts = WT == 256 ? 2 : 4;
   const int tt = tile % p.tok_tiles, row = hf * 128 + sub * 32 + lane, feat = (tile / p.tok_tiles) * WT + row;
-  const bool whole = k0 == 0 && k1 == p.kgroups;
+  const bool whole = k0 == 0 && k1 == p.kgroups, stacked = F32 && p.nt <= MAX_NT / 2 && !p.unsplit;
   const int G = gridDim.x, c = blockIdx.x;
   int c0 = c, n_seg = 1;
   if (!whole) {
@@ -307,12 +307,13 @@ __device__ __forceinline__ bool finish_segment(const StreamParams& p, Shared& sh
   const uint32_t ta = sh.tmem + ((uint32_t)(sub * 32) << 16) + hf * 256;
   const int groups = p.nt / EC;
   for (int cg = part0; cg < groups; cg += parts) {
-    uint32_t a[EC];
+    uint32_t a[EC], b[EC];
     ld_tmem(ta + cg * EC, a);
+    if (stacked) ld_tmem(ta + p.nt + cg * EC, b);
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
     float v[EC];
 #pragma unroll
-    for (int j = 0; j < EC; j++) v[j] = __uint_as_float(a[j]);
+    for (int j = 0; j < EC; j++) v[j] = stacked ? __uint_as_float(a[j]) + __uint_as_float(b[j]) : __uint_as_float(a[j]);
     if (whole) store_outputs(p, v, feat, tt * p.nt + cg * EC, lane);
     else
 #pragma unroll
@@ -421,7 +422,8 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
   } else if (warp == WARP_MMA) {
     if (elect_one()) {
       bool ok = true;
-      const uint32_t idesc = make_idesc(128, nt);
+      const bool stacked = F32 && nt <= MAX_NT / 2 && !p.unsplit;
+      const uint32_t id1 = make_idesc(128, nt), id2 = make_idesc(128, stacked ? 2 * nt : nt), lo = stacked ? nt : 0;      // remainders' products beside: see qgemm_tmem.cuh
       const uint32_t desc_hi = (uint32_t)(make_desc(0, 0, 128) >> 32);
       const uint32_t w_base = (ring >> 4) | ((uint32_t)WT << 16), x_base = ((ring + W_STEP) >> 4) | ((uint32_t)x_rows << 16);
       int seg = 0, slot = 0;
@@ -444,10 +446,10 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
             for (int kk = 0; kk < KSTEP / 16; kk++) {
               const uint32_t xh = x_lo + (kk >> 1) * (x_step >> 4) + (kk & 1) * 2 * x_rows;
               const uint32_t wh = w_lo + (kk >> 1) * (W_STEP >> 4) + hf * 128 + (kk & 1) * 2 * WT;
-              mma(d, wh, xh, desc_hi, idesc, kk ? 1u : acc);
+              mma(d, wh, xh, desc_hi, id2, kk ? 1u : acc);          // stacked: wh x [xh | xl] in one instruction
               if (F32) {
-                mma(d, wh, xh + nt, desc_hi, idesc, 1u);
-                mma(d, wh + (W_HALF >> 4), xh, desc_hi, idesc, 1u);
+                if (!stacked) mma(d, wh, xh + nt, desc_hi, id1, 1u);
+                mma(d + lo, wh + (W_HALF >> 4), xh, desc_hi, id1, 1u);
               }
             }
           }
@@ -616,8 +618,16 @@ int launch_stream(const StreamParams& p, int grid, cudaStream_t st) {
   return B200Q_OK;
 }
 
-// weights through tensor memory: up to 128 rows (of fp32 rows 2 x 128 accumulator columns), half-precision rows wherever a tile has 128 weight rows
-bool takes_tmem(const Plan& pl, bool f32) { return pl.nt <= 128 || (!f32 && pl.wt == 128); }
+// Weights through tensor memory, or through shared memory (tiles of 128 weight rows; of fp32 rows at most 128 activation rows, 2 x 128 accumulator columns)?  The first wherever
+// its faster loop runs long enough to pay for its longer way in and out.  Prompts on 1024-wide Q8_0 blocks (their Linears are 64 to 450 K groups, below 4 an SM): 62 tokens 976 us
+// through tensor memory, through shared memory 873; 4096-wide ones from 4 on: 1032, 1179.  Above 64 rows the line is at 10 an SM: 4608 x 3584 (7), 128 rows 35.3 us, 32.0; 3584 x 18944 (28) 70,
+// 74.  Tiles dealt to more than 8 CTAs (400 x 4096, 120 half-precision rows) are mostly the adding of their parts: 32 us, 25.
+bool takes_tmem(const Plan& pl, bool f32, bool unsplit, long long units, long long tiles, int grid, int n_sm) {
+  if (pl.wt != 128 || (f32 && pl.nt > 128)) return false;
+  if (unsplit) return true;
+  if (grid > 8 * tiles) return false;
+  return !f32 || pl.nt <= 32 || units >= (pl.nt <= 64 ? 4LL : 10LL) * n_sm;
+}
 template <int QT, bool F32>
 int launch_tmem(StreamParams& p, int grid, cudaStream_t st) {
   auto kern = qgemm_tmem_kernel<QT, F32>;
@@ -749,9 +759,10 @@ int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtyp
   else
     B200Q_CHECK_CUDA(cudaLaunchKernelEx(&cfg, split_rows_kernel<__half, false>, (const __half*)x, (const __half*)nullptr, 0.f, m, n_in, kgroups, pl.nt, per,
                                         (unsigned char*)p.xt, p.counters, n_counters, (float*)nullptr, 0.f));
-#define STREAM_CASE(QT) (takes_tmem(pl, f32) ? (f32 ? launch_tmem<QT, true>(p, grid, st) : launch_tmem<QT, false>(p, grid, st)) \
+  const bool tmem = takes_tmem(pl, f32, p.unsplit, p.units, p.tiles, grid, n_sm);
+#define STREAM_CASE(QT) (tmem ? (f32 ? launch_tmem<QT, true>(p, grid, st) : launch_tmem<QT, false>(p, grid, st)) \
                          : pl.wt == 256 ? (f32 ? launch_stream<QT, 256, true>(p, grid, st) : launch_stream<QT, 256, false>(p, grid, st)) \
-                                        : launch_stream<QT, 128, true>(p, grid, st))
+                                        : (f32 ? launch_stream<QT, 128, true>(p, grid, st) : launch_stream<QT, 128, false>(p, grid, st)))
   return qtype == B200Q_Q4_0 ? STREAM_CASE(B200Q_Q4_0) : STREAM_CASE(B200Q_Q8_0);
 #undef STREAM_CASE
 }

@@ -68,10 +68,13 @@ __device__ __forceinline__ uint4 ld_shared4(uint32_t addr) {
   return v;
 }
 
-constexpr int NC = 4;                                   // accumulator columns (activation rows) a thread takes at a time at the end of a segment
-__device__ __forceinline__ void ld_tmem4(uint32_t a, uint32_t (&v)[NC]) {
+// Accumulator columns (activation rows) a thread takes at a time at the end of a segment: 8 of half-precision rows (4608 x 3584, 301 rows: 31.9 us with 4, 28.3), but the
+// fp32 kernels have no registers for that (spills in the unpack loop: 4096 x 4096, 45 rows 22.2 us, 24.3 with 8).
+template <bool F32> constexpr int N_COLS = F32 ? 4 : 8;
+__device__ __forceinline__ void ld_columns(uint32_t a, uint32_t (&v)[4]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(a));
 }
+__device__ __forceinline__ void ld_columns(uint32_t a, uint32_t (&v)[8]) { ld_tmem(a, v); }
 
 struct Segment { int seg, tile, k0, k1; bool last; };      // number within the CTA's, K groups k0 .. k1 of tile; `last`: the CTA's last
 // The deal in 32 bits: K groups times CTAs stay below 2^32 for every matrix that fits the GPU (3.2e11 4-bit weights are 2e7 K groups of 128 rows).
@@ -89,7 +92,7 @@ __device__ __forceinline__ int2 tile_ctas(const StreamParams& p, int tile) {
 // six places 4096 x 4096 took 38 us).
 template <bool F32>
 __device__ __forceinline__ bool finish_segment_t(const StreamParams& p, SharedT& sh, uint32_t sb, const Segment& g, int first_tile, bool first_part, int& dumps, uint32_t dump) {
-  constexpr int PARTS = (UNPACK_WARPS + EPI_WARPS) / 4;
+  constexpr int PARTS = (UNPACK_WARPS + EPI_WARPS) / 4, NC = N_COLS<F32>;
   const int tid = threadIdx.x, lane = tid & 31, sub = (tid >> 5) & 3, part = (tid >> 7) - T_UNPACK / 4;
   const int row = sub * 32 + lane;
   int tile = g.tile;
@@ -124,33 +127,42 @@ __device__ __forceinline__ bool finish_segment_t(const StreamParams& p, SharedT&
     const int ft = p.tok_tiles == 1 ? tile : tile / p.tok_tiles, tt = tile - ft * p.tok_tiles, feat = ft * 128 + row;
 #pragma unroll 1
     for (; cg < groups; cg += step) {
-      float v[NC] = {0.f, 0.f, 0.f, 0.f};
+      float v[NC] = {};
       int own = -1, n_add = 0;
       if (pass == 0) {
         uint32_t a[NC], b[NC];
-        ld_tmem4(ta + cg * NC, a);
-        if (second) ld_tmem4(ta + second + cg * NC, b);
+        ld_columns(ta + cg * NC, a);
+        if (second) ld_columns(ta + second + cg * NC, b);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
         for (int j = 0; j < NC; j++) v[j] = second ? __uint_as_float(a[j]) + __uint_as_float(b[j]) : __uint_as_float(a[j]);
         if (dumped || kept) {
-          const uint4 f = make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
-          if (dumped) st_shared(mine_s + cg * 2048, f);
-          else __stcg(reinterpret_cast<uint4*>(mine + (size_t)cg * NC * 128), f);
+#pragma unroll
+          for (int j = 0; j < NC; j += 4) {
+            const uint4 f = make_uint4(__float_as_uint(v[j]), __float_as_uint(v[j + 1]), __float_as_uint(v[j + 2]), __float_as_uint(v[j + 3]));
+            if (dumped) st_shared(mine_s + (cg * NC + j) * 512, f);
+            else __stcg(reinterpret_cast<uint4*>(mine + (size_t)(cg * NC + j) * 128), f);
+          }
           continue;
         }
         if (alone) { own = c - ctas.x; n_add = ctas.y; }
       } else if (from_dump) {
-        const uint4 f = ld_shared4(mine_s + cg * 2048);
-        v[0] = __uint_as_float(f.x); v[1] = __uint_as_float(f.y); v[2] = __uint_as_float(f.z); v[3] = __uint_as_float(f.w);
+#pragma unroll
+        for (int j = 0; j < NC; j += 4) {
+          const uint4 f = ld_shared4(mine_s + (cg * NC + j) * 512);
+          v[j] = __uint_as_float(f.x); v[j + 1] = __uint_as_float(f.y); v[j + 2] = __uint_as_float(f.z); v[j + 3] = __uint_as_float(f.w);
+        }
       } else n_add = ctas.y;
       if (n_add) {                             // the parts in the order of K
-        float w[NC] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
+        float w[NC] = {};
+#pragma unroll(F32 ? 4 : 2)
         for (int s = 0; s < n_add; s++) {
-          float4 f = make_float4(v[0], v[1], v[2], v[3]);
-          if (s != own) f = __ldcg(reinterpret_cast<const float4*>(parts + part_slot(p, ctas.x + s, tile, s == 0) * slot + (size_t)cg * NC * 128));
-          w[0] += f.x; w[1] += f.y; w[2] += f.z; w[3] += f.w;
+#pragma unroll
+          for (int j = 0; j < NC; j += 4) {
+            const float4 f = __ldcg(reinterpret_cast<const float4*>(parts + part_slot(p, ctas.x + s, tile, s == 0) * slot + (size_t)(cg * NC + j) * 128));
+            const bool mine = s == own;        // (loaded all the same: loads under a branch went one by one, 400 x 4096, 120 half-precision rows 41 us)
+            w[j] += mine ? v[j] : f.x; w[j + 1] += mine ? v[j + 1] : f.y; w[j + 2] += mine ? v[j + 2] : f.z; w[j + 3] += mine ? v[j + 3] : f.w;
+          }
         }
 #pragma unroll
         for (int j = 0; j < NC; j++) v[j] = w[j];
