@@ -437,8 +437,7 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
         for (int s = (k1 - k0) * 4; s > 0; s--) {
           if (!bar_wait(sb, BAR(sb, full) + 8 * slot, par)) { ok = false; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          // all MMAs of one accumulator back to back: switching the destination costs about 40 cycles of a 128-cycle instruction
-          // (N = 256; nearly 100 at N <= 128, where an instruction takes at least 72 cycles whatever its N)
+          // all MMAs of one accumulator back to back; with weights in shared memory an instruction of N <= 96 takes 40 to 57 cycles whatever its N, of 256 129
 #pragma unroll
           for (int hf = 0; hf < WT / 128; hf++) {
             const uint32_t d = tmem + hf * 256;
@@ -620,13 +619,14 @@ int launch_stream(const StreamParams& p, int grid, cudaStream_t st) {
 
 // Weights through tensor memory, or through shared memory (tiles of 128 weight rows; of fp32 rows at most 128 activation rows, 2 x 128 accumulator columns)?  The first wherever
 // its faster loop runs long enough to pay for its longer way in and out.  Prompts on 1024-wide Q8_0 blocks (their Linears are 64 to 450 K groups, below 4 an SM): 62 tokens 976 us
-// through tensor memory, through shared memory 873; 4096-wide ones from 4 on: 1032, 1179.  Above 64 rows the line is at 10 an SM: 4608 x 3584 (7), 128 rows 35.3 us, 32.0; 3584 x 18944 (28) 70,
+// through tensor memory, through shared memory 873; 4096-wide (6 an SM and more): 1032, 1179.  45
+// tokens: 1024-wide Q4_0 813, 853, Q8_0 872, 833; 2048-wide Q4_0 1086, 1121.  Above 64 rows the line is at 10 an SM: 4608 x 3584 (7), 128 rows 35.3 us, 32.0; 3584 x 18944 (28) 70,
 // 74.  Tiles dealt to more than 8 CTAs (400 x 4096, 120 half-precision rows) are mostly the adding of their parts: 32 us, 25.
-bool takes_tmem(const Plan& pl, bool f32, bool unsplit, long long units, long long tiles, int grid, int n_sm) {
+bool takes_tmem(int qtype, const Plan& pl, bool f32, bool unsplit, long long units, long long tiles, int grid, int n_sm) {
   if (pl.wt != 128 || (f32 && pl.nt > 128)) return false;
   if (unsplit) return true;
   if (grid > 8 * tiles) return false;
-  return !f32 || pl.nt <= 32 || units >= (pl.nt <= 64 ? 4LL : 10LL) * n_sm;
+  return !f32 || pl.nt <= (qtype == B200Q_Q4_0 ? 48 : 32) || units >= (pl.nt <= 64 ? 4LL : 10LL) * n_sm;
 }
 template <int QT, bool F32>
 int launch_tmem(StreamParams& p, int grid, cudaStream_t st) {
@@ -759,7 +759,7 @@ int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtyp
   else
     B200Q_CHECK_CUDA(cudaLaunchKernelEx(&cfg, split_rows_kernel<__half, false>, (const __half*)x, (const __half*)nullptr, 0.f, m, n_in, kgroups, pl.nt, per,
                                         (unsigned char*)p.xt, p.counters, n_counters, (float*)nullptr, 0.f));
-  const bool tmem = takes_tmem(pl, f32, p.unsplit, p.units, p.tiles, grid, n_sm);
+  const bool tmem = takes_tmem(qtype, pl, f32, p.unsplit, p.units, p.tiles, grid, n_sm);
 #define STREAM_CASE(QT) (tmem ? (f32 ? launch_tmem<QT, true>(p, grid, st) : launch_tmem<QT, false>(p, grid, st)) \
                          : pl.wt == 256 ? (f32 ? launch_stream<QT, 256, true>(p, grid, st) : launch_stream<QT, 256, false>(p, grid, st)) \
                                         : (f32 ? launch_stream<QT, 128, true>(p, grid, st) : launch_stream<QT, 128, false>(p, grid, st)))

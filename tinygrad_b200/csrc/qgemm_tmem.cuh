@@ -18,6 +18,8 @@ namespace {
 
 constexpr int EPI_WARPS = 4;
 constexpr int T_MMA = 0, T_COPY = 1, T_WCOPY = 2, T_SETUP = 3, T_UNPACK = 4, T_EPI = T_UNPACK + UNPACK_WARPS, T_THREADS = (T_EPI + EPI_WARPS) * 32;
+// 8 unpack warps fill a slot, two such groups in turn.  Not more groups than slots: a group that is two uses of a slot ahead would take its barrier's phase for the one
+// before.  Stages of two K groups at most: a group may fill one slot ahead of a segment's end, not two.
 constexpr int MAX_T_SLOTS = 4, MAX_W_STAGES = 6;
 template <bool F32> constexpr int A_COLS = F32 ? 128 : 64;      // tensor-memory columns of a slot's weights: a K group of high halves, then of remainders
 // Packed weights wait in shared memory as they are: stages of 8 row tiles (128 rows) x W_GROUPS K groups, a bulk copy per row tile
