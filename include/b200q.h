@@ -500,6 +500,7 @@ int b200q_swiglu_quantize_mxfp8(const void* h_bf16, int64_t rows, const int32_t*
  * off [n_experts+1] (group starts, every group padded to 256 rows).  mode 0: top-k of the logits in descending order,
  * weights = softmax over the k (moe_routing.py:115-116).  mode 1: softmax over all experts, compare-count top-k in
  * ascending order, weights not renormalised (tinygrad/llm/model.py:35-41,118,123-124, the OLMoE defaults).
+ * Whatever the logits, a token's k choices are different experts: NaN ranks with -infinity, and the weights are what the arithmetic makes of it.
  * Deterministic (stable counting sort).  scratch: b200q_moe_route_scratch_bytes(). */
 size_t b200q_moe_route_scratch_bytes(int n_tokens, int n_experts, int k);
 int b200q_moe_rows_max(int n_tokens, int n_experts, int k);   /* m_max_for, extra/gemm/moe_routing.py:89-90 */
@@ -518,7 +519,8 @@ int b200q_moe_route_pad(const float* logits, int n_tokens, int n_experts, int k,
 int b200q_moe_route_gating(const float* logits, const float* sel_bias, int n_tokens, int n_experts, int k, int gating, int normalize, float scale,
                            int pad, int32_t* topi, float* weights, int32_t* dest_row, int32_t* off, int32_t* counts, void* scratch, void* stream);
 /* The grouping tables alone, for a selection the caller already has (`ExpertWeights.__call__(sel, x)`, tinygrad/llm/model.py:21-27):
- * topi [n_tokens, k] expert ids (entries outside 0..n_experts-1 must not occur) -> dest_row / off / counts as b200q_moe_route_pad. */
+ * topi [n_tokens, k] expert ids -> dest_row / off / counts as b200q_moe_route_pad.  An entry outside 0..n_experts-1 has no row: dest_row -1, which
+ * b200q_quantize_mxfp8, b200q_permute_rows and b200q_moe_combine pass over. */
 int b200q_moe_route_tables(const int32_t* topi, int n_tokens, int n_experts, int k, int pad, int32_t* dest_row, int32_t* off, int32_t* counts,
                            void* scratch, void* stream);
 /* Rows of row_bytes bytes (a multiple of 4) moved through an index table: gather = 0: dst[idx[i]] = src[i]; gather = 1:

@@ -2,7 +2,7 @@
 registers) against the oracle, and the FP8 linear's rows at the edges of its 32-row stores."""
 import numpy as np
 import pytest
-from tinygrad_b200 import moe
+from tinygrad_b200 import _lib, moe
 from tinygrad_b200.fp8 import FP8Linear
 from tinygrad_b200.runtime import DeviceBuffer
 from oracle import fp8_linear as f8, mxfp8 as mx
@@ -25,6 +25,75 @@ def test_route_at_the_edges_of_its_launches(T, E, k):
   np.testing.assert_array_equal(r.dest_row.numpy(), dest)
   np.testing.assert_array_equal(r.off.numpy(), off)
   np.testing.assert_allclose(r.weights.numpy(), w, rtol=2e-6)      # expf and a sum of at most 32 terms: some units of 2^-24
+
+
+MODES = [moe.ROUTE_TOPK_SOFTMAX, moe.ROUTE_SOFTMAX_TOPK, moe.Gating("softmax"), moe.Gating("sigmoid", True), moe.Gating("softmax", True), moe.Gating("sqrt_softplus")]
+
+
+@pytest.mark.parametrize("mode", MODES, ids=lambda m: m if isinstance(m, int) else f"{m.func}-{m.norm_topk_prob}")
+@pytest.mark.parametrize("T,E,k", [(9, 16, 4), (9, 64, 8), (9, 200, 8), (64, 8, 8), (300, 40, 4)])
+def test_route_of_rows_that_are_not_finite(T, E, k, mode):
+  """Each token has k different experts, ranked with NaN as -infinity, whatever its row holds, and their pairs are sorted by them."""
+  rng = np.random.default_rng(E)
+  logits = rng.standard_normal((T, E)).astype(np.float32)
+  logits[0], logits[1] = np.nan, -np.inf
+  logits[2], logits[2, E // 2] = np.nan, 0.5
+  logits[3], logits[3, [E // 3, E - 1]] = -np.inf, (0.25, -0.5)
+  logits[4, rng.permutation(E)[: E // 2]] = np.nan
+  logits[5, rng.permutation(E)[: E - k // 2]] = -np.inf
+  logits[6], logits[6, E - 2] = -np.finfo(np.float32).max, np.nan
+  logits[-1, 1] = np.nan
+  r = moe.Routing(T, E, k, mode).run(DeviceBuffer.from_numpy(logits))
+  topi, w = r.topi.numpy(), r.weights.numpy()
+  best = np.argsort(-np.where(np.isnan(logits), -np.inf, logits), axis=1, kind="stable")[:, :k]
+  if mode != moe.ROUTE_TOPK_SOFTMAX: best = best[:, ::-1]
+  whole = mode == moe.ROUTE_SOFTMAX_TOPK or getattr(mode, "func", "") == "softmax" and not mode.norm_topk_prob      # one NaN makes every score NaN
+  for t in range(T):
+    assert len(set(topi[t])) == k and (0 <= topi[t]).all() and (topi[t] < E).all(), t
+    nan, low = np.isnan(logits[t]).any(), np.isneginf(logits[t])
+    if not (whole and (nan or low.all())): np.testing.assert_array_equal(topi[t], best[t], str(t))
+    if not nan and not low.all(): assert np.isfinite(w[t]).all(), t
+    if whole and nan or np.isnan(logits[t, topi[t]]).any() and mode in MODES[:1] + MODES[4:5]: assert np.isnan(w[t]).all(), t
+  flat = topi.reshape(-1)
+  counts, dest, off = np.bincount(flat, minlength=E), r.dest_row.numpy(), r.off.numpy()
+  np.testing.assert_array_equal(off, np.concatenate([[0], np.cumsum(-(-counts // 256) * 256)]))
+  for e in range(E): np.testing.assert_array_equal(dest[flat == e], off[e] + np.arange(counts[e]))
+
+
+@pytest.mark.parametrize("T,E,k", [(9, 16, 4), (300, 40, 4)])
+def test_choices_that_are_no_experts_have_no_row(T, E, k):
+  lib, rng = _lib.load(), np.random.default_rng(T)
+  topi = rng.integers(0, E, (T, k)).astype(np.int32)
+  topi[0], topi[T // 2, 1], topi[-1, -1] = -1, E, 0x7fffffff
+  dest, off, scratch = DeviceBuffer.empty((T * k,), np.int32), DeviceBuffer.empty((E + 1,), np.int32), DeviceBuffer(lib.b200q_moe_route_scratch_bytes(T, E, k))
+  sel = DeviceBuffer.from_numpy(topi)
+  _lib.check(lib.b200q_moe_route_tables(sel.ptr, T, E, k, 256, dest.ptr, off.ptr, None, scratch.ptr, None))
+  flat, d, o = topi.reshape(-1), dest.numpy(), off.numpy()
+  there = (flat >= 0) & (flat < E)
+  assert (d[~there] == -1).all()
+  for e in range(E): np.testing.assert_array_equal(d[flat == e], o[e] + np.arange((flat == e).sum()))
+  x, y, w = rng.standard_normal((T, 256)).astype(np.float32), rng.standard_normal((int(o[-1]), 64)).astype(np.float32), rng.standard_normal((T, k)).astype(np.float32)
+  q = moe.quantize_mxfp8(DeviceBuffer.from_numpy(x), T, 256, _lib.F32, dest, k, int(o[-1]))[0].numpy()
+  own = mx.quantize_mxfp8(x)[0]
+  for i in np.flatnonzero(there): np.testing.assert_array_equal(q[d[i]], own[i // k])
+  for D in (64, 60):                                # with and without 16-byte loads
+    yb, out = moe.to_bf16_bits(np.ascontiguousarray(y[:, :D])), DeviceBuffer.empty((T, D), np.uint16)
+    dy, dw = DeviceBuffer.from_numpy(yb), DeviceBuffer.from_numpy(w)
+    _lib.check(lib.b200q_moe_combine(dy.ptr, dest.ptr, dw.ptr, T, k, D, out.ptr, None))
+    ref = (np.where(there[:, None], moe.from_bf16_bits(yb)[np.maximum(d, 0)], 0).reshape(T, k, D) * w[..., None].astype(np.float64)).sum(1)
+    assert (np.abs(moe.from_bf16_bits(out.numpy()) - ref) <= 2.0 ** -8 * np.abs(ref) + 1e-5).all()      # bf16; fp32 sums of four terms of size 1
+
+
+def test_a_token_without_finite_logits_leaves_the_others_alone():
+  T, D, F, E, k = 40, 256, 128, 16, 4
+  rng = np.random.default_rng(3)
+  layer = moe.MxMoE(*(rng.standard_normal(s).astype(np.float32) * 0.05 for s in ((E, F, D), (E, F, D), (E, D, F))), k)
+  x, logits = DeviceBuffer.from_numpy(moe.to_bf16_bits(rng.standard_normal((T, D)).astype(np.float32))), rng.standard_normal((T, E)).astype(np.float32)
+  clean = layer(x, DeviceBuffer.from_numpy(logits), T).numpy().reshape(T, D)
+  logits[7], logits[30] = np.nan, -np.inf
+  y, rest = layer(x, DeviceBuffer.from_numpy(logits), T).numpy().reshape(T, D), [t for t in range(T) if t not in (7, 30)]
+  assert np.isnan(moe.from_bf16_bits(y[[7, 30]])).all()
+  np.testing.assert_array_equal(y[rest], clean[rest])
 
 
 @pytest.mark.parametrize("dt", [np.float32, np.float16])

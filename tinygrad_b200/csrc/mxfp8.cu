@@ -58,6 +58,7 @@ __global__ void quantize_mxfp8_kernel(const T* __restrict__ x, int64_t rows, int
   if (!valid) return;
   for (int f = 0; f < fan; f++) {
     const int64_t o = dest ? (int64_t)dest[r * fan + f] : r;
+    if (o < 0) continue;
     *reinterpret_cast<uint2*>(q + o * k + col) = pk;
     if ((lane & 3) == 0) e8[o * kb + b] = e;
   }
@@ -96,8 +97,12 @@ __global__ void swiglu_quant_kernel(const __nv_bfloat16* __restrict__ h, int64_t
 // routing, step 1: one warp per token.  mode 0 (extra/gemm/moe_routing.py:115-116): top-k of the raw logits in
 // descending order, weights = softmax over the k.  mode 1 (tinygrad/llm/model.py:118,123-124 with the OLMoE defaults):
 // scores = softmax over all experts, top-k listed in ascending order of score, weights = the scores, not renormalised.
-// Ties: the lower expert index ranks higher (model.py:35-41).
+// Ties: the lower expert index ranks higher (model.py:35-41).  NaN ranks with -infinity, so that a row of any values has k different choices below n_experts (what
+// sorts the pairs indexes by them); a weight is computed from the value itself, NaN included.  A NaN key marks what is taken or not there: it compares as nothing.
 constexpr int MAX_E_PER_LANE = 8;   // up to 256 experts; EPL: what a lane has of the number at hand, 1, 2 or 8 (32, 64, 256)
+
+#define TAKEN __int_as_float(0x7fffffff)
+__device__ __forceinline__ float select_key(float v, bool there) { return !there ? TAKEN : isnan(v) ? -INFINITY : v; }
 
 // One token by one warp; s_topi (optional): shared memory that gets the choices too.
 template <int EPL> __device__ __forceinline__ void route_topk_token(const float* __restrict__ logits, int tok, int n_experts, int k, int mode, int32_t* __restrict__ topi,
@@ -118,19 +123,22 @@ template <int EPL> __device__ __forceinline__ void route_topk_token(const float*
     for (int i = 0; i < EPL; i++) denom += (i * 32 + lane < n_experts) ? expf(v[i] - mx) : 0.f;
     denom = warp_sum(denom);
   }
+#pragma unroll
+  for (int i = 0; i < EPL; i++) v[i] = select_key(v[i], i * 32 + lane < n_experts);
   float top1 = 0.f, ksum = 0.f;
 #pragma unroll 1
   for (int j = 0; j < k; j++) {
     float bv = -INFINITY; int bi = 0x7fffffff;
 #pragma unroll
-    for (int i = 0; i < EPL; i++) { const int e = i * 32 + lane; if (v[i] > bv) { bv = v[i]; bi = e; } }   // lowest index wins inside a lane
+    for (int i = 0; i < EPL; i++) { const int e = i * 32 + lane; if (v[i] > bv || (v[i] == bv && e < bi)) { bv = v[i]; bi = e; } }   // lowest index wins inside a lane
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const float ov = __shfl_xor_sync(0xffffffffu, bv, o); const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
       if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
     }
 #pragma unroll
-    for (int i = 0; i < EPL; i++) if (i * 32 + lane == bi) v[i] = -INFINITY;    // taken
+    for (int i = 0; i < EPL; i++) if (i * 32 + lane == bi) v[i] = TAKEN;
+    if (bv == -INFINITY) bv = logits[(size_t)tok * n_experts + bi];      // which may be NaN
     if (j == 0) top1 = bv;
     const int slot = mode == 1 ? k - 1 - j : j;
     float w;
@@ -182,21 +190,21 @@ template <int EPL> __device__ __forceinline__ void route_gating_token(const floa
 #pragma unroll
   for (int i = 0; i < EPL; i++) {
     const int e = i * 32 + lane;
-    key[i] = e < n_experts ? (sel_bias ? sc[i] + sel_bias[e] : sc[i]) : -INFINITY;
+    key[i] = select_key(sel_bias && e < n_experts ? sc[i] + sel_bias[e] : sc[i], e < n_experts);
   }
   float pv = 0.f;                        // lane j < k keeps the probability of slot j
 #pragma unroll 1
   for (int j = 0; j < k; j++) {
     float bv = -INFINITY, bs = 0.f; int bi = 0x7fffffff;
 #pragma unroll
-    for (int i = 0; i < EPL; i++) { const int e = i * 32 + lane; if (key[i] > bv) { bv = key[i]; bs = sc[i]; bi = e; } }
+    for (int i = 0; i < EPL; i++) { const int e = i * 32 + lane; if (key[i] > bv || (key[i] == bv && e < bi)) { bv = key[i]; bs = sc[i]; bi = e; } }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const float ov = __shfl_xor_sync(0xffffffffu, bv, o), os = __shfl_xor_sync(0xffffffffu, bs, o); const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
       if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bs = os; bi = oi; }
     }
 #pragma unroll
-    for (int i = 0; i < EPL; i++) if (i * 32 + lane == bi) key[i] = -INFINITY;    // taken
+    for (int i = 0; i < EPL; i++) if (i * 32 + lane == bi) key[i] = TAKEN;
     const int slot = k - 1 - j;          // ascending order of rank
     if (lane == slot) pv = bs;
     if (lane == 0) { topi[(size_t)tok * k + slot] = bi; if (s_topi) s_topi[tok * k + slot] = bi; }
@@ -231,6 +239,8 @@ __global__ void route_choose_kernel(const RouteRule r, const float* __restrict__
 // routing, steps 2-4: stable counting sort of the T*k (token, slot) pairs by expert.
 // dest_row[i] = off[e_i] + (number of pairs before i with the same expert); off = cumulative group sizes padded to 256.
 constexpr int ROUTE_CHUNK = 1024;
+// A choice made by the caller that is no expert has no row: dest_row -1, which the kernels that move rows pass over.
+__device__ __forceinline__ int known_expert(int e, int n_experts) { return e >= 0 && e < n_experts ? e : -1; }
 // ends (optional) [n_experts]: off + size, the row behind each expert's last.
 
 // Padded offsets from the group sizes `tot` (shared memory), by one warp.
@@ -275,7 +285,7 @@ __global__ void __launch_bounds__(ROUTE_CHUNK) route_one_kernel(const RouteRule 
     for (int tok = warp; tok < n_tokens; tok += ROUTE_CHUNK / 32) route_token<EPL>(r, logits, tok, n_experts, k, topi, weights, s_topi);
   } else for (int i = threadIdx.x; i < n; i += ROUTE_CHUNK) s_topi[i] = topi[i];
   __syncthreads();
-  const int i = threadIdx.x, e = i < n ? s_topi[i] : -1;
+  const int i = threadIdx.x, e = i < n ? known_expert(s_topi[i], n_experts) : -1;
   const unsigned same = __match_any_sync(0xffffffffu, e);
   const int before_in_warp = __popc(same & ((1u << lane) - 1));
   if (e >= 0 && before_in_warp == 0) s_wcnt[warp * n_experts + e] = __popc(same);
@@ -288,7 +298,7 @@ __global__ void __launch_bounds__(ROUTE_CHUNK) route_one_kernel(const RouteRule 
   __syncthreads();
   if (warp == 0) route_offsets(s_tot, n_experts, pad, off, counts, ends, s_off);
   __syncthreads();
-  if (e >= 0) dest_row[i] = s_off[e] + s_wcnt[warp * n_experts + e] + before_in_warp;
+  if (i < n) dest_row[i] = e >= 0 ? s_off[e] + s_wcnt[warp * n_experts + e] + before_in_warp : -1;
 }
 
 __global__ void __launch_bounds__(ROUTE_CHUNK) route_count_kernel(const int32_t* __restrict__ topi, int n, int n_experts, int32_t* __restrict__ counts) {
@@ -298,9 +308,10 @@ __global__ void __launch_bounds__(ROUTE_CHUNK) route_count_kernel(const int32_t*
   for (int e = threadIdx.x; e < n_experts; e += blockDim.x) s_cnt[e] = 0;
   __syncthreads();
   const int i = blockIdx.x * ROUTE_CHUNK + threadIdx.x;
-  if (i < n) atomicAdd(&s_cnt[topi[i]], 1);      // integer counts: the order of the adds does not matter
+  const int e = i < n ? known_expert(topi[i], n_experts) : -1;
+  if (e >= 0) atomicAdd(&s_cnt[e], 1);      // integer counts: the order of the adds does not matter
   __syncthreads();
-  for (int e = threadIdx.x; e < n_experts; e += blockDim.x) counts[(size_t)blockIdx.x * n_experts + e] = s_cnt[e];
+  for (int x = threadIdx.x; x < n_experts; x += blockDim.x) counts[(size_t)blockIdx.x * n_experts + x] = s_cnt[x];
 }
 
 // one warp per expert: exclusive scan of its chunk counts (in place, 32 chunks at a time); then one warp builds the padded offsets
@@ -350,7 +361,7 @@ __global__ void __launch_bounds__(ROUTE_CHUNK) route_place_kernel(const int32_t*
   pdl_wait();
   __syncthreads();
   const int i = blockIdx.x * ROUTE_CHUNK + threadIdx.x;
-  const int e = i < n ? topi[i] : -1;
+  const int e = i < n ? known_expert(topi[i], n_experts) : -1;
   const unsigned same = __match_any_sync(0xffffffffu, e);
   const int before_in_warp = __popc(same & ((1u << lane) - 1));
   if (e >= 0 && before_in_warp == 0) s_wcnt[warp * n_experts + e] = __popc(same);
@@ -359,7 +370,7 @@ __global__ void __launch_bounds__(ROUTE_CHUNK) route_place_kernel(const int32_t*
     int before = counts[(size_t)blockIdx.x * n_experts + e] + before_in_warp;
     for (int w = 0; w < warp; w++) before += s_wcnt[w * n_experts + e];
     dest_row[i] = off[e] + before;
-  }
+  } else if (i < n) dest_row[i] = -1;
 }
 
 // combine (extra/gemm/moe_routing.py:128-131): out[t] = sum_j weights[t, j] * y[dest_row[t*k + j]], fp32 sum in slot order, bf16 out; add_to
@@ -371,7 +382,10 @@ __global__ void combine_kernel(const __nv_bfloat16* __restrict__ y, const int32_
   const int t = blockIdx.x;
   for (int c = threadIdx.x; c < d; c += blockDim.x) {
     float acc = 0.f;
-    for (int j = 0; j < k; j++) acc += weights[(size_t)t * k + j] * __bfloat162float(y[(size_t)dest_row[(size_t)t * k + j] * d + c]);
+    for (int j = 0; j < k; j++) {
+      const int row = dest_row[(size_t)t * k + j];
+      if (row >= 0) acc += weights[(size_t)t * k + j] * __bfloat162float(y[(size_t)row * d + c]);
+    }
     const __nv_bfloat16 r = __float2bfloat16_rn(acc);
     out[(size_t)t * d + c] = r;
     if (add_to) add_to[(size_t)t * d + c] += __bfloat162float(r);
@@ -394,10 +408,10 @@ __global__ void __launch_bounds__(256) combine8_kernel(const __nv_bfloat16* __re
     for (int j0 = 0; j0 < k; j0 += 4) {
       uint4 u[4];
 #pragma unroll
-      for (int j = 0; j < 4; j++) if (j0 + j < k) u[j] = *reinterpret_cast<const uint4*>(y + (size_t)s_row[j0 + j] * d + c);
+      for (int j = 0; j < 4; j++) if (j0 + j < k) u[j] = *reinterpret_cast<const uint4*>(y + (size_t)max(s_row[j0 + j], 0) * d + c);
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        if (j0 + j < k) {
+        if (j0 + j < k && s_row[j0 + j] >= 0) {
           const float w = s_w[j0 + j];
           float v[8];
           bf16x8_to_f32(u[j], v);
