@@ -11,8 +11,7 @@
 //
 // What bounds it: three fp16 tensor passes for many rows; for few rows the weight stream and the unpacking.  So
 //  * weights are the MMA's A operand (128 rows per instruction) and the activation rows its N: any row count rounded up to 16 fills the
-//    instruction, and up to 128 rows the halves xh | xl sit side by side as ONE operand of 2 N columns (two instructions per K step
-//    instead of three);
+//    instruction, and up to 128 rows the products with a remainder (wh xl, wl xh) have an accumulator of their own;
 //  * a tile is up to 256 weight rows (two accumulators, the whole of tensor memory) by up to 256 activation rows: every unpacked weight meets
 //    256 rows and every activation byte 256 weight rows.  With 128 x 128 tiles the activation operand alone took 2.4x the L2 traffic
 //    and every weight was unpacked once per 128 rows.  Up to 128 rows, and where tiles are few, a tile is 128 weight rows
@@ -54,7 +53,7 @@ struct StreamParams {
   void* y;
   long long units;               // tiles x K groups
   // Units are dealt in multiples of this: 1, or a whole tile where the caller wants it so (`unsplit`) or the workspace has no room for partial
-  // sums.  With whole tiles every output is one running sum (halves not side by side either) in the order of b200q_qgemm: the same bits.
+  // sums.  With whole tiles every output is one running sum (remainders' products not apart either) in the order of b200q_qgemm: the same bits.
   int grain, unsplit;
   int tiles, m, n_out, kgroups, n_row_tiles, nt, tok_tiles, slots, ahead, y_f16, silu_mul;
   int dump, d_cols;              // qgemm_tmem.cuh: where whole tiles wait in shared memory (0: nowhere), tensor-memory columns of the accumulators
@@ -293,7 +292,7 @@ __device__ __forceinline__ bool finish_segment(const StreamParams& p, Shared& sh
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = warp & 3, q = warp >> 2;
   const int hf = WT == 256 ? q >> 1 : 0, part0 = WT == 256 ? q & 1 : q, parts = WT == 256 ? 2 : 4;
   const int tt = tile % p.tok_tiles, row = hf * 128 + sub * 32 + lane, feat = (tile / p.tok_tiles) * WT + row;
-  const bool whole = k0 == 0 && k1 == p.kgroups, stacked = F32 && p.nt <= MAX_NT / 2 && !p.unsplit;
+  const bool whole = k0 == 0 && k1 == p.kgroups, two_sums = WT == 128 && F32 && p.nt <= MAX_NT / 2 && !p.unsplit;
   const int G = gridDim.x, c = blockIdx.x;
   int c0 = c, n_seg = 1;
   if (!whole) {
@@ -309,11 +308,11 @@ __device__ __forceinline__ bool finish_segment(const StreamParams& p, Shared& sh
   for (int cg = part0; cg < groups; cg += parts) {
     uint32_t a[EC], b[EC];
     ld_tmem(ta + cg * EC, a);
-    if (stacked) ld_tmem(ta + p.nt + cg * EC, b);
+    if (two_sums) ld_tmem(ta + p.nt + cg * EC, b);
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
     float v[EC];
 #pragma unroll
-    for (int j = 0; j < EC; j++) v[j] = stacked ? __uint_as_float(a[j]) + __uint_as_float(b[j]) : __uint_as_float(a[j]);
+    for (int j = 0; j < EC; j++) v[j] = two_sums ? __uint_as_float(a[j]) + __uint_as_float(b[j]) : __uint_as_float(a[j]);
     if (whole) store_outputs(p, v, feat, tt * p.nt + cg * EC, lane);
     else
 #pragma unroll
@@ -422,8 +421,8 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
   } else if (warp == WARP_MMA) {
     if (elect_one()) {
       bool ok = true;
-      const bool stacked = F32 && nt <= MAX_NT / 2 && !p.unsplit;
-      const uint32_t id1 = make_idesc(128, nt), id2 = make_idesc(128, stacked ? 2 * nt : nt), lo = stacked ? nt : 0;      // remainders' products beside: see qgemm_tmem.cuh
+      const bool two_sums = WT == 128 && F32 && nt <= MAX_NT / 2 && !p.unsplit;
+      const uint32_t id = make_idesc(128, nt), lo = two_sums ? nt : 0;      // one shape, the remainders' products beside: see qgemm_tmem.cuh
       const uint32_t desc_hi = (uint32_t)(make_desc(0, 0, 128) >> 32);
       const uint32_t w_base = (ring >> 4) | ((uint32_t)WT << 16), x_base = ((ring + W_STEP) >> 4) | ((uint32_t)x_rows << 16);
       int seg = 0, slot = 0;
@@ -433,7 +432,7 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
         if (!bar_wait(sb, BAR(sb, acc_empty), (seg & 1) ^ 1)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t tmem = sh.tmem;
-        uint32_t acc = 0;
+        uint32_t acc = 0, acc_lo = two_sums ? 0 : 1;
         for (int s = (k1 - k0) * 4; s > 0; s--) {
           if (!bar_wait(sb, BAR(sb, full) + 8 * slot, par)) { ok = false; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -445,14 +444,14 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
             for (int kk = 0; kk < KSTEP / 16; kk++) {
               const uint32_t xh = x_lo + (kk >> 1) * (x_step >> 4) + (kk & 1) * 2 * x_rows;
               const uint32_t wh = w_lo + (kk >> 1) * (W_STEP >> 4) + hf * 128 + (kk & 1) * 2 * WT;
-              mma(d, wh, xh, desc_hi, id2, kk ? 1u : acc);          // stacked: wh x [xh | xl] in one instruction
+              mma(d, wh, xh, desc_hi, id, kk ? 1u : acc);
               if (F32) {
-                if (!stacked) mma(d, wh, xh + nt, desc_hi, id1, 1u);
-                mma(d + lo, wh + (W_HALF >> 4), xh, desc_hi, id1, 1u);
+                mma(d + lo, wh, xh + nt, desc_hi, id, kk ? 1u : acc_lo);
+                mma(d + lo, wh + (W_HALF >> 4), xh, desc_hi, id, 1u);
               }
             }
           }
-          acc = 1;
+          acc = acc_lo = 1;
           commit(BAR(sb, empty) + 8 * slot);
           x_lo += slot_bytes >> 4; w_lo += slot_bytes >> 4;
           if (++slot == slots) { slot = 0; par ^= 1; x_lo = x_base; w_lo = w_base; }

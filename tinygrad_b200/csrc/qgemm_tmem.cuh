@@ -6,7 +6,7 @@
 //
 // What paces it, and what follows from that:
 //  * the thread that issues the MMAs: 4 unpack warps share its scheduler, so each of its instructions takes 7 to 8 cycles and the answer of a barrier that is ready
-//    250.  A slot is a whole K group (16 instructions, one barrier for weights and activations), the next slot's barrier is asked before they are issued, and its loop is
+//    250.  A slot is a whole K group (24 instructions, one barrier for weights and activations), the next slot's barrier is asked before they are issued, and its loop is
 //    kept short.  Slots of half a K group with two barriers: 1000 cycles a slot where the MMAs need 300, no faster than shared memory (8B gate / up, 45 rows: 74 us).
 //  * the unpack warps: packed weights come as bulk copies of a row tile's K groups.  As one cp.async per lane a round's copies took 900 cycles (53 us).  They too ask
 //    for their next barriers before they unpack.
@@ -319,11 +319,13 @@ __global__ void __launch_bounds__(T_THREADS, 1) qgemm_tmem_kernel(const StreamPa
     const uint32_t x0 = __shfl_sync(0xffffffffu, (ring >> 4) | ((uint32_t)x_rows << 16), 0), full0 = __shfl_sync(0xffffffffu, TBAR(sb, full), 0);
     if (elect_one()) {
       bool ok = true;
-      const bool stacked = F32 && !p.unsplit;
-      const uint32_t id1 = make_idesc(128, nt), id2 = make_idesc(128, stacked ? 2 * nt : nt);
-      // Stacked halves: the remainders' products are all added up beside the high parts', where the tensor core's truncating additions to a small sum lose little: one
-      // addition to the large sum per 16 columns instead of two, half the error (28672 x 4096, 45 rows: 7.3e-6 of the result, 4.0e-6 so).
-      const uint32_t d_lo = stacked ? d + nt : d;
+      const bool two_sums = F32 && !p.unsplit;
+      // Every instruction has the one shape 128 x nt, and what two of them add to is the same columns: in that order they are added.  (wh x [xh | xl] as one instruction
+      // of 2 nt columns and wl xh in half of its columns were two shapes in one accumulator, between which no order is promised.)
+      const uint32_t id = make_idesc(128, nt);
+      // Two sums: the remainders' products are all added up beside the high parts', where the tensor core's truncating additions to a small sum lose little: one
+      // addition to the large sum per 16 columns instead of three (28672 x 4096, 45 rows: 7.3e-6 of the result with two, 4.0e-6 so).
+      const uint32_t d_lo = two_sums ? d + nt : d;
       const uint32_t desc_hi = (uint32_t)(make_desc(0, 0, 128) >> 32), x_next = x_bytes >> 4, k32 = x_step >> 4, k16 = 2 * x_rows;
       constexpr uint32_t TO_EMPTY = offsetof(SharedT, empty) - offsetof(SharedT, full);
       int seg = 0, left = p.slots;                            // slots until the ring starts again
@@ -333,7 +335,7 @@ __global__ void __launch_bounds__(T_THREADS, 1) qgemm_tmem_kernel(const StreamPa
         open_segment(u, seg, tile, k0, k1);
         u += k1 - k0;
         if (!t_wait(sb, TBAR(sb, acc_empty), (seg & 1) ^ 1)) { ok = false; break; }
-        uint32_t acc = 0;
+        uint32_t acc = 0, acc_lo = two_sums ? 0 : 1;
 #pragma unroll 1
         for (int s = k1 - k0; s > 0; s--) {
           if (!ready && !t_wait(sb, full, par)) { ok = false; break; }
@@ -345,13 +347,13 @@ __global__ void __launch_bounds__(T_THREADS, 1) qgemm_tmem_kernel(const StreamPa
 #pragma unroll
           for (int kk = 0; kk < 8; kk++) {
             const uint32_t xh = xa + (kk >> 1) * k32 + (kk & 1) * k16;
-            mma_ts(d, wa + kk * 8, xh, desc_hi, id2, kk ? 1u : acc);    // stacked: wh x [xh | xl] in one instruction
+            mma_ts(d, wa + kk * 8, xh, desc_hi, id, kk ? 1u : acc);
             if (F32) {
-              if (!stacked) mma_ts(d, wa + kk * 8, xh + nt, desc_hi, id1, 1u);
-              mma_ts(d_lo, wa + 64 + kk * 8, xh, desc_hi, id1, 1u);
+              mma_ts(d_lo, wa + kk * 8, xh + nt, desc_hi, id, kk ? 1u : acc_lo);
+              mma_ts(d_lo, wa + 64 + kk * 8, xh, desc_hi, id, 1u);
             }
           }
-          acc = 1;
+          acc = acc_lo = 1;
           commit(bar);
         }
         if (ok) commit(TBAR(sb, acc_full));
