@@ -98,11 +98,28 @@ __global__ void swiglu_quant_kernel(const __nv_bfloat16* __restrict__ h, int64_t
 // descending order, weights = softmax over the k.  mode 1 (tinygrad/llm/model.py:118,123-124 with the OLMoE defaults):
 // scores = softmax over all experts, top-k listed in ascending order of score, weights = the scores, not renormalised.
 // Ties: the lower expert index ranks higher (model.py:35-41).  NaN ranks with -infinity, so that a row of any values has k different choices below n_experts (what
-// sorts the pairs indexes by them); a weight is computed from the value itself, NaN included.  A NaN key marks what is taken or not there: it compares as nothing.
+// sorts the pairs indexes by them); a weight is computed from the value itself, NaN included.
 constexpr int MAX_E_PER_LANE = 8;   // up to 256 experts; EPL: what a lane has of the number at hand, 1, 2 or 8 (32, 64, 256)
 
-#define TAKEN __int_as_float(0x7fffffff)
-__device__ __forceinline__ float select_key(float v, bool there) { return !there ? TAKEN : isnan(v) ? -INFINITY : v; }
+// A value as a number that is greater for what ranks higher; 0: not there, or taken.  (-0 + 0 is 0: the two zeros are equal.)
+__device__ __forceinline__ uint32_t rank_key(float v, bool there) {
+  const uint32_t u = __float_as_uint((isnan(v) ? -INFINITY : v) + 0.f);
+  return there ? u ^ (u >> 31 ? 0xffffffffu : 0x80000000u) : 0;
+}
+// The expert of the greatest key of a warp, the lowest among equals, is taken: its number, and of `val` what belongs to it.  (Two integer reductions; as five rounds of shuffled
+// pairs with the same choices a token's routing took 0.7 us more.)
+template <int EPL> __device__ __forceinline__ int take_best(uint32_t (&key)[EPL], const float (&val)[EPL], int lane, float& picked) {
+  uint32_t best = 0; unsigned e = 0xffffffffu;
+  float v = 0.f;
+#pragma unroll
+  for (int i = 0; i < EPL; i++) if (key[i] > best) { best = key[i]; v = val[i]; e = i * 32 + lane; }
+  const uint32_t top = __reduce_max_sync(0xffffffffu, best);
+  e = __reduce_min_sync(0xffffffffu, best == top ? e : 0xffffffffu);
+  picked = __shfl_sync(0xffffffffu, v, e & 31);
+#pragma unroll
+  for (int i = 0; i < EPL; i++) if (i * 32 + lane == (int)e) key[i] = 0;
+  return (int)e;
+}
 
 // One token by one warp; s_topi (optional): shared memory that gets the choices too.
 template <int EPL> __device__ __forceinline__ void route_topk_token(const float* __restrict__ logits, int tok, int n_experts, int k, int mode, int32_t* __restrict__ topi,
@@ -123,22 +140,14 @@ template <int EPL> __device__ __forceinline__ void route_topk_token(const float*
     for (int i = 0; i < EPL; i++) denom += (i * 32 + lane < n_experts) ? expf(v[i] - mx) : 0.f;
     denom = warp_sum(denom);
   }
+  uint32_t key[EPL];
 #pragma unroll
-  for (int i = 0; i < EPL; i++) v[i] = select_key(v[i], i * 32 + lane < n_experts);
+  for (int i = 0; i < EPL; i++) key[i] = rank_key(v[i], i * 32 + lane < n_experts);
   float top1 = 0.f, ksum = 0.f;
 #pragma unroll 1
   for (int j = 0; j < k; j++) {
-    float bv = -INFINITY; int bi = 0x7fffffff;
-#pragma unroll
-    for (int i = 0; i < EPL; i++) { const int e = i * 32 + lane; if (v[i] > bv || (v[i] == bv && e < bi)) { bv = v[i]; bi = e; } }   // lowest index wins inside a lane
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, bv, o); const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-    }
-#pragma unroll
-    for (int i = 0; i < EPL; i++) if (i * 32 + lane == bi) v[i] = TAKEN;
-    if (bv == -INFINITY) bv = logits[(size_t)tok * n_experts + bi];      // which may be NaN
+    float bv;
+    const int bi = take_best(key, v, lane, bv);
     if (j == 0) top1 = bv;
     const int slot = mode == 1 ? k - 1 - j : j;
     float w;
@@ -164,7 +173,8 @@ enum { GATE_SOFTMAX = 1, GATE_SIGMOID = 2, GATE_SOFTMAX_WEIGHT = 3, GATE_SQRT_SO
 template <int EPL> __device__ __forceinline__ void route_gating_token(const float* __restrict__ logits, const float* __restrict__ sel_bias, int tok, int n_experts, int k, int gating,
                                                    int normalize, float scale, int32_t* __restrict__ topi, float* __restrict__ weights, int* s_topi) {
   const int lane = threadIdx.x & 31;
-  float sc[EPL], key[EPL];
+  float sc[EPL];
+  uint32_t key[EPL];
   float mx = -INFINITY;
 #pragma unroll
   for (int i = 0; i < EPL; i++) {
@@ -190,21 +200,13 @@ template <int EPL> __device__ __forceinline__ void route_gating_token(const floa
 #pragma unroll
   for (int i = 0; i < EPL; i++) {
     const int e = i * 32 + lane;
-    key[i] = select_key(sel_bias && e < n_experts ? sc[i] + sel_bias[e] : sc[i], e < n_experts);
+    key[i] = rank_key(sel_bias && e < n_experts ? sc[i] + sel_bias[e] : sc[i], e < n_experts);
   }
   float pv = 0.f;                        // lane j < k keeps the probability of slot j
 #pragma unroll 1
   for (int j = 0; j < k; j++) {
-    float bv = -INFINITY, bs = 0.f; int bi = 0x7fffffff;
-#pragma unroll
-    for (int i = 0; i < EPL; i++) { const int e = i * 32 + lane; if (key[i] > bv || (key[i] == bv && e < bi)) { bv = key[i]; bs = sc[i]; bi = e; } }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, bv, o), os = __shfl_xor_sync(0xffffffffu, bs, o); const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bs = os; bi = oi; }
-    }
-#pragma unroll
-    for (int i = 0; i < EPL; i++) if (i * 32 + lane == bi) key[i] = TAKEN;
+    float bs;
+    const int bi = take_best(key, sc, lane, bs);
     const int slot = k - 1 - j;          // ascending order of rank
     if (lane == slot) pv = bs;
     if (lane == 0) { topi[(size_t)tok * k + slot] = bi; if (s_topi) s_topi[tok * k + slot] = bi; }
@@ -375,11 +377,8 @@ __global__ void __launch_bounds__(ROUTE_CHUNK) route_place_kernel(const int32_t*
 
 // combine (extra/gemm/moe_routing.py:128-131): out[t] = sum_j weights[t, j] * y[dest_row[t*k + j]], fp32 sum in slot order, bf16 out; add_to
 // (optional, fp32 [n_tokens, d]): the rounded sum is added to it as well (the residual behind the expert layer)
-__global__ void combine_kernel(const __nv_bfloat16* __restrict__ y, const int32_t* __restrict__ dest_row, const float* __restrict__ weights,
-                               int n_tokens, int k, int d, __nv_bfloat16* __restrict__ out, float* __restrict__ add_to) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const int t = blockIdx.x;
+__device__ __forceinline__ void combine_token(int t, const __nv_bfloat16* __restrict__ y, const int32_t* __restrict__ dest_row, const float* __restrict__ weights, int k, int d,
+                                              __nv_bfloat16* __restrict__ out, float* __restrict__ add_to) {
   for (int c = threadIdx.x; c < d; c += blockDim.x) {
     float acc = 0.f;
     for (int j = 0; j < k; j++) {
@@ -391,8 +390,15 @@ __global__ void combine_kernel(const __nv_bfloat16* __restrict__ y, const int32_
     if (add_to) add_to[(size_t)t * d + c] += __bfloat162float(r);
   }
 }
+__global__ void combine_kernel(const __nv_bfloat16* __restrict__ y, const int32_t* __restrict__ dest_row, const float* __restrict__ weights,
+                               int n_tokens, int k, int d, __nv_bfloat16* __restrict__ out, float* __restrict__ add_to) {
+  pdl_launch_dependents();
+  pdl_wait();
+  combine_token(blockIdx.x, y, dest_row, weights, k, d, out, add_to);
+}
 // d % 8 == 0: a thread sums 8 neighbouring columns over the k rows (16-byte loads), same order of additions.  A CTA stages its token's rows and
-// weights, so that four rows are in flight at once (4096 tokens x 8 rows of 2048: 34.9 us with the row numbers loaded one by one).
+// weights, so that four rows are in flight at once (4096 tokens x 8 rows of 2048: 34.9 us with the row numbers loaded one by one).  A token with a choice that has no
+// row goes the other way as a whole (asked at every load: 28.9 us, 28.5 so).
 constexpr int COMBINE_MAX_K = 32;
 __global__ void __launch_bounds__(256) combine8_kernel(const __nv_bfloat16* __restrict__ y, const int32_t* __restrict__ dest_row, const float* __restrict__ weights,
                                                        int n_tokens, int k, int d, __nv_bfloat16* __restrict__ out, float* __restrict__ add_to) {
@@ -401,17 +407,18 @@ __global__ void __launch_bounds__(256) combine8_kernel(const __nv_bfloat16* __re
   const int t = blockIdx.x;
   pdl_launch_dependents();
   pdl_wait();
-  if (threadIdx.x < k) { s_row[threadIdx.x] = dest_row[(size_t)t * k + threadIdx.x]; s_w[threadIdx.x] = weights[(size_t)t * k + threadIdx.x]; }
-  __syncthreads();
+  int row = 0;
+  if (threadIdx.x < k) { s_row[threadIdx.x] = row = dest_row[(size_t)t * k + threadIdx.x]; s_w[threadIdx.x] = weights[(size_t)t * k + threadIdx.x]; }
+  if (__syncthreads_or(row < 0)) { combine_token(t, y, dest_row, weights, k, d, out, add_to); return; }
   for (int c = threadIdx.x * 8; c < d; c += blockDim.x * 8) {
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     for (int j0 = 0; j0 < k; j0 += 4) {
       uint4 u[4];
 #pragma unroll
-      for (int j = 0; j < 4; j++) if (j0 + j < k) u[j] = *reinterpret_cast<const uint4*>(y + (size_t)max(s_row[j0 + j], 0) * d + c);
+      for (int j = 0; j < 4; j++) if (j0 + j < k) u[j] = *reinterpret_cast<const uint4*>(y + (size_t)s_row[j0 + j] * d + c);
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        if (j0 + j < k && s_row[j0 + j] >= 0) {
+        if (j0 + j < k) {
           const float w = s_w[j0 + j];
           float v[8];
           bf16x8_to_f32(u[j], v);
