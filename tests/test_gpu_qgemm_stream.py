@@ -66,7 +66,9 @@ def test_more_rows_than_a_grid_has_along_y():
   assert (np.abs(got - x @ w.T) <= 2.0 ** -20 * (np.abs(x) @ np.abs(w).T)).all()      # six rounded sums and the rounding of the halves, as above
 
 
-@pytest.mark.parametrize("typ,m,n_out,n_in", [(2, 1, 64, 32), (8, 1, 1536, 1024), (8, 52, 130, 128), (2, 200, 512, 992)])
+@pytest.mark.parametrize("typ,m,n_out,n_in", [(2, 1, 64, 32), (8, 1, 1536, 1024), (8, 52, 130, 128), (2, 200, 512, 992),
+                                              # 65 to 128 rows: through tensor memory as well
+                                              (8, 65, 300, 416), (2, 112, 1300, 992), (2, 128, 130, 2080), (8, 128, 1536, 1024)])
 def test_unsplit_sums_have_the_bits_of_the_kernel_without_a_workspace(typ, m, n_out, n_in):
   rng = np.random.default_rng(m)
   pw, x = quant.repack(synth.BLOCK_MAKERS[typ](n_out, n_in, rng), n_out, n_in, typ), DeviceBuffer.from_numpy(rng.standard_normal((m, n_in)).astype(np.float32))
@@ -74,6 +76,47 @@ def test_unsplit_sums_have_the_bits_of_the_kernel_without_a_workspace(typ, m, n_
   quant.qgemm(pw.buf.ptr, typ, n_out, n_in, x, a, m)
   quant.qgemm(pw.buf.ptr, typ, n_out, n_in, x, b, m, workspace=ws, unsplit=True)
   np.testing.assert_array_equal(a.numpy(), b.numpy())
+
+
+@pytest.mark.parametrize("typ,m,n_out,n_in", [(2, 45, 6144, 4096), (8, 45, 6144, 4096), (2, 80, 6144, 4096), (8, 80, 6144, 4096), (8, 33, 1024, 4096), (2, 128, 1000, 4096)])
+def test_nothing_of_the_halves_is_lost(typ, m, n_out, n_in):
+  """The whole result's error against 64 bits, which bounds on single values do not see: a lost wl xh or wh xl is some 2^-12.8 of the result (the fp16 rounding of one operand),
+  all three products in one sum 7.3e-6 (a truncating addition to it per product and 16 columns), two sums 4.0e-6 measured; the last two shapes through shared memory."""
+  rng = np.random.default_rng(n_out + m)
+  raw = synth.BLOCK_MAKERS[typ](n_out, n_in, rng)
+  x = rng.standard_normal((m, n_in)).astype(np.float32)
+  pw, y, ws = quant.repack(raw, n_out, n_in, typ), DeviceBuffer.empty((m, n_out), np.float32), DeviceBuffer(quant.qgemm_workspace_bytes(m, n_in, n_out))
+  quant.qgemm(pw.buf.ptr, typ, n_out, n_in, DeviceBuffer.from_numpy(x), y, m, workspace=ws)
+  ref = x.astype(np.float64) @ gq.weight_matrix(raw, n_out, n_in, typ).astype(np.float64).T
+  err = np.linalg.norm(y.numpy() - ref) / np.linalg.norm(ref)
+  assert err < 6e-6, err
+
+
+@pytest.mark.parametrize("epilogue", [_lib.EPI_LINEAR, _lib.EPI_SILU_MUL])
+@pytest.mark.parametrize("typ,m,n_out,n_in,dt", [(2, 45, 4096, 4096, np.float32), (8, 128, 6144, 4096, np.float32), (8, 33, 1024, 2048, np.float32), (8, 301, 4608, 3584, np.float16)])
+def test_split_sums_repeat(typ, m, n_out, n_in, dt, epilogue):
+  """Whichever CTA comes last at a tile, and whether it still has its own part in tensor memory or stored it: the parts are added in the order of K."""
+  rng = np.random.default_rng(m)
+  pw, x = quant.repack(synth.BLOCK_MAKERS[typ](n_out, n_in, rng), n_out, n_in, typ), DeviceBuffer.from_numpy(rng.standard_normal((m, n_in)).astype(dt))
+  code, ws = _lib.F32 if dt == np.float32 else _lib.F16, DeviceBuffer(quant.qgemm_workspace_bytes(m, n_in, n_out))
+  ys = [DeviceBuffer.empty((m, n_out // (2 if epilogue else 1)), dt) for _ in range(40)]
+  for y in ys: quant.qgemm(pw.buf.ptr, typ, n_out, n_in, x, y, m, x_dtype=code, y_dtype=code, epilogue=epilogue, workspace=ws)
+  first = ys[0].numpy().view(np.uint8)
+  for y in ys[1:]: np.testing.assert_array_equal(y.numpy().view(np.uint8), first)
+
+
+@pytest.mark.parametrize("m", [45, 160])
+def test_swiglu_of_half_precision_rows(m):
+  hidden, dim, rng = 1408, 512, np.random.default_rng(m)
+  gate, up = (synth.q8_0_blocks(hidden, dim, rng) for _ in range(2))
+  x, pw = rng.standard_normal((m, dim)).astype(np.float16), quant.repack(gate, hidden, dim, 8, raw_up=up)
+  y, ws = DeviceBuffer.empty((m, hidden), np.float16), DeviceBuffer(quant.qgemm_workspace_bytes(m, dim, 2 * hidden))
+  quant.qgemm(pw.buf.ptr, 8, 2 * hidden, dim, DeviceBuffer.from_numpy(x), y, m, x_dtype=_lib.F16, y_dtype=_lib.F16, epilogue=_lib.EPI_SILU_MUL, workspace=ws)
+  g, u = (x.astype(np.float64) @ gq.weight_matrix(b, hidden, dim, 8).astype(np.float16).astype(np.float64).T for b in (gate, up))
+  ref = g / (1 + np.exp(-g)) * u
+  # as below, sums of one product per 16 columns, and the result's rounding to half precision
+  tol = 2.0 ** -18 * (1.1 * np.abs(g).max() * np.abs(u) + np.abs(g) * np.abs(u).max() + 1) + 2.0 ** -11 * np.abs(ref)
+  assert (np.abs(y.numpy() - ref) <= tol).all()
 
 
 def test_norm_in_front_and_swiglu_behind():
@@ -92,7 +135,9 @@ def test_norm_in_front_and_swiglu_behind():
   assert (np.abs(y.numpy() - ref) <= tol).all()
 
 
-@pytest.mark.parametrize("typ,m,n_out,n_in,split", [(2, 5, 300, 4096, True), (8, 70, 1000, 992, True), (8, 70, 300, 14336, True), (2, 300, 130, 512, False)])
+@pytest.mark.parametrize("typ,m,n_out,n_in,split", [(2, 5, 300, 4096, True), (8, 70, 1000, 992, True), (8, 70, 300, 14336, True), (2, 300, 130, 512, False),
+                                                    # through tensor memory: enough K groups an SM, or no split; with whole tiles that wait in shared memory and without
+                                                    (2, 5, 2400, 4096, True), (8, 17, 19000, 512, True), (2, 45, 51216, 416, True), (8, 70, 19000, 1280, True), (2, 100, 300, 992, False)])
 def test_rows_of_any_magnitude(typ, m, n_out, n_in, split):
   """Rows far outside fp16's range lose no more than others: the bound of the exact product for each row by itself; and the same behind a norm weight that leads
   out of it."""

@@ -99,7 +99,7 @@ def test_a_token_without_finite_logits_leaves_the_others_alone():
 @pytest.mark.parametrize("dt", [np.float32, np.float16])
 @pytest.mark.parametrize("rows", [1, 31, 32, 33, 127, 129, 300])
 def test_fp8_rows(rows, dt):
-  """The rows a call has and no others (its result is a block that other results' neighbours share), against the product of the decoded codes."""
+  """Every row of a call, against the product of the decoded codes."""
   rng = np.random.default_rng(rows)
   n_in, n_out = 256, 512
   lin = FP8Linear(n_in, n_out, rng.standard_normal((n_out, n_in)).astype(np.float32), rng.standard_normal(n_out).astype(np.float32))
@@ -110,3 +110,39 @@ def test_fp8_rows(rows, dt):
   # 15 times the result's size here (256 terms of random sign); half precision: its rounding
   tol = 2.0 ** -10 if dt == np.float16 else 2e-5
   assert y.shape == ref.shape and (np.abs(y - ref) <= tol * (np.abs(ref) + np.sqrt(np.mean(ref.astype(np.float64) ** 2)))).all()
+
+
+def _bytes(ptr, n):
+  out = np.empty(n, np.uint8)
+  _lib.check(_lib.load().b200q_memcpy_d2h(out.ctypes.data, ptr, n, None))
+  return out
+
+
+@pytest.mark.parametrize("with_bias", [True, False])
+@pytest.mark.parametrize("dt", [np.float32, np.float16])
+@pytest.mark.parametrize("rows", [1, 31, 33, 129])
+def test_fp8_rows_and_nothing_behind_them(rows, dt, with_bias):
+  """Results leave as boxes of 32 rows: what lies behind a result's last row, in its own pool block and in its neighbours, keeps its bytes."""
+  lib, rng, n_in, n_out = _lib.load(), np.random.default_rng(rows), 128, 512
+  lin = FP8Linear(n_in, n_out, rng.standard_normal((n_out, n_in)).astype(np.float32), rng.standard_normal(n_out).astype(np.float32) if with_bias else None)
+  x = DeviceBuffer.from_numpy(rng.standard_normal((rows, n_in)).astype(dt))
+  used, step = rows * n_out * np.dtype(dt).itemsize, 64
+  while step * 16 < used: step *= 2
+  block = max(512, -(-used // step) * step)             # what the pool hands out: an eighth of a power of two's steps
+  held = [lin(x) for _ in range(12)]
+  want = held[0].numpy()
+  for y in held: _lib.check(lib.b200q_memset(y.ptr, 0xA5, block, None))
+  _lib.check(lib.b200q_device_synchronize())
+  mine = [y.ptr for y in held[::2]]
+  held = held[1::2]
+  seen = 0
+  for _ in range(300):                                  # until the pool has handed out the blocks between the held ones again
+    y = lin(x)
+    if y.ptr in mine:
+      mine.remove(y.ptr)
+      seen += 1
+      np.testing.assert_array_equal(y.numpy(), want)
+      assert (_bytes(y.ptr + used, block - used) == 0xA5).all()
+    for h in held: assert (_bytes(h.ptr, block) == 0xA5).all()
+    if seen == 3: return
+  pytest.fail("the pool did not hand its blocks out again")
