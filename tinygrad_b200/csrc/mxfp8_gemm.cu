@@ -5,16 +5,16 @@
 // (the reference computation it is tested against: dequantised operands matmul, test/backend/test_asm_gemm.py:289-292,306).
 //
 // Persistent, warp-specialised kernel, one CTA per SM, 128 x 256 output tiles, tiles of the used rows (off[E]) dealt round-robin:
-//   warps 4-7  loaders: cp.async the A (128 x 128 B) and B (256 x 128 B) tiles of a K step into a 4-stage ring (K-major, 128-byte
-//              swizzle: 16-byte chunk c of row r sits at chunk c ^ (r & 7)) together with the step's E8M0 scale words (one 32-bit
-//              word = 4 K blocks per row, stored as 32 x 16 B chunks: row r -> chunk r % 32, word r / 32); each thread's copies
-//              arrive on the stage's "full" mbarrier when they land;
+//   warps 4-7  loaders: one thread brings the A (128 x 128 B) and B (256 x 128 B) tiles of a K step into a 3-stage ring by tensor-map copies (K-major, 128-byte
+//              swizzle: 16-byte chunk c of row r sits at chunk c ^ (r & 7)), all of them the step's E8M0 scale words by cp.async (one 32-bit
+//              word = 4 K blocks per row, stored as 32 x 16 B chunks: row r -> chunk r % 32, word r / 32); the copies' bytes and each thread's
+//              words arrive on the stage's "full" mbarrier when they land;
 //   warp 8     one thread moves the scale chunks to tensor memory with tcgen05.cp 32x128b.warpx4 (row r -> lane r % 32 of every
 //              32-lane sub-partition, column r / 32: the layout the MMA reads), issues tcgen05.mma kind::mxf8f6f4.block_scale
 //              (scale_vec::1X, 128 x 256 x 32 per instruction, the tensor core applies both block scales), four per K step, and
 //              commits each step to the stage's "empty" mbarrier;
 //   warps 0-3, 9-20  epilogue: tcgen05.ld the fp32 accumulator (256 tensor-memory columns; four warps per 32-lane sub-partition,
-//              64 columns each) into registers, release the accumulator, then round to bf16 and store (or SwiGLU + requantise).
+//              64 columns each) into registers, release the accumulator, then one of four endings (OUT_BF16 ..).
 // Loaders run ahead across tile boundaries; the accumulator (one buffer: 2 x 256 columns + the scale columns do not fit the 512 of
 // tensor memory) is handed back after one tensor-memory round trip, the epilogue's arithmetic and stores overlap the next tile's MMAs.
 // Every mbarrier wait is bounded; a wait that runs out raises a status word and makes every role leave.
@@ -34,7 +34,7 @@ constexpr int EPI_WARPS = 4, LOAD_WARPS = 4, EPI_Q = 4;      // epilogue: warps 
 constexpr int THREADS = (EPI_Q * EPI_WARPS + LOAD_WARPS + 1) * 32;
 constexpr int A_BYTES = BM * BK, B_BYTES = BN * BK, SF_BYTES = 2048;                    // scale chunks: A 512 B, B 2 x 512 B
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES + SF_BYTES;                               // 50 KB, a multiple of 1024
-constexpr int EPI_STAGE_BYTES = 16 * 4096;                                              // bf16 epilogue: 4 KB per warp, stored by one tensor-map copy
+constexpr int EPI_STAGE_BYTES = 16 * 4096;                                              // staging rows of the epilogues that store by tensor-map copies (bf16, FP8 linear): 4 KB per warp
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + EPI_STAGE_BYTES;               // + room to align the ring to 1024 B
 constexpr int TMEM_COLS = 512;            // 256 accumulator columns + scale columns, rounded up to a power of two
 constexpr int SFA_COL = 256, SFB_COL = 256 + 4 * STAGES;   // per stage 4 columns (A: 128 rows) and 8 columns (B: 256 rows)
@@ -306,78 +306,74 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         release();
         swiglu_quant_store(v0, v1, act_q, act_e8, row, n >> 1, (n0 >> 1) + cq * 32);
-        continue;
-      }
-      tmem_ld32(ta + cq * 64, v0); tmem_ld32(ta + cq * 64 + 32, v1);
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      release();
-      // Results leave through this warp's staging rows (32 rows x 128 bytes, packet p of row r at p ^ (r & 7): conflict-free both ways), which are in the
-      // 128-byte-swizzle layout a tiled tensor-map store reads: one copy of whole 128-byte row segments.  Rows past the tensor's last are not written.
-      unsigned char* const stg = sm_raw + (ring - s32(sm_raw)) + STAGES * STAGE_BYTES + (warp < EPI_WARPS ? warp : warp - (LOAD_WARPS + 1)) * 4096;
-      auto packet = [&](int p) { return stg + lane * 128 + ((p ^ (lane & 7)) << 4); };
-      auto send = [&](int column) {
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) {
-          asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
-                       ::"l"(&tm_c), "r"(column), "r"(m0 + sub * 32), "r"(s32(stg)) : "memory");
-          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // the rows may be overwritten
-        }
-        __syncwarp();
-      };
-      if constexpr (OUT == OUT_SCALED) {
-        // (each thread storing its own row, 16 bytes of 32 rows an instruction: 47.7 us for the call of 1000 x 4096 x 4096 with fp32 results, 45.0 so)
-        const float w = *so.fw, xf = *so.fx;
-        const int col = n0 + cq * 64;
-        if (m0 + sub * 32 < so.rows) {
-          float b[4] = {0.f, 0.f, 0.f, 0.f};
+      } else {
+        tmem_ld32(ta + cq * 64, v0); tmem_ld32(ta + cq * 64 + 32, v1);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        release();
+        // Results leave through this warp's staging rows (32 rows x 128 bytes, packet p of row r at p ^ (r & 7): conflict-free both ways), which are in the
+        // 128-byte-swizzle layout a tiled tensor-map store reads: one copy of whole 128-byte row segments.  Rows past the tensor's last are not written.
+        unsigned char* const stg = sm_raw + (ring - s32(sm_raw)) + STAGES * STAGE_BYTES + (warp < EPI_WARPS ? warp : warp - (LOAD_WARPS + 1)) * 4096;
+        auto packet = [&](int p) { return stg + lane * 128 + ((p ^ (lane & 7)) << 4); };
+        auto send = [&](int column) {
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) {
+            asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
+                         ::"l"(&tm_c), "r"(column), "r"(m0 + sub * 32), "r"(s32(stg)) : "memory");
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");      // the rows may be overwritten
+          }
+          __syncwarp();
+        };
+        if constexpr (OUT == OUT_SCALED) {
+          // (each thread storing its own row, 16 bytes of 32 rows an instruction: 47.7 us for the call of 1000 x 4096 x 4096 with fp32 results, 45.0 so)
+          const float w = *so.fw, xf = *so.fx;
+          const int col = n0 + cq * 64;
+          if (m0 + sub * 32 < so.rows) {
+            float b[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-          for (int j = 0; j < 64; j += 4) {
-            const uint32_t* v = j < 32 ? v0 + j : v1 + (j - 32);
-            if (so.bias) { const float4 b4 = __ldg(reinterpret_cast<const float4*>(so.bias + col + j)); b[0] = b4.x; b[1] = b4.y; b[2] = b4.z; b[3] = b4.w; }
-            float o[4];
+            for (int j = 0; j < 64; j += 4) {
+              const uint32_t* v = j < 32 ? v0 + j : v1 + (j - 32);
+              if (so.bias) { const float4 b4 = __ldg(reinterpret_cast<const float4*>(so.bias + col + j)); b[0] = b4.x; b[1] = b4.y; b[2] = b4.z; b[3] = b4.w; }
+              float o[4];
+#pragma unroll
+              for (int q = 0; q < 4; q++) {
+                o[q] = __fmul_rn(__fmul_rn(__uint_as_float(v[q]), w), xf);      // y * w_scale * x_scale, in that order
+                if (so.bias) o[q] = __fadd_rn(o[q], b[q]);
+              }
+              if (so.y_f16) {
+                const __half2 h[2] = {__floats2half2_rn(o[0], o[1]), __floats2half2_rn(o[2], o[3])};
+                *reinterpret_cast<uint2*>(packet(j >> 3) + (j & 4) * 2) = *reinterpret_cast<const uint2*>(h);
+              } else {
+                *reinterpret_cast<float4*>(packet((j >> 2) & 7)) = make_float4(o[0], o[1], o[2], o[3]);
+                if (j == 28) send(col);
+              }
+            }
+            send(so.y_f16 ? col : col + 32);
+          }
+        } else if constexpr (OUT == OUT_F32) {      // unrounded sums (the per-tensor FP8 linear scales them afterwards): each thread stores its own row
+          float4* o4 = reinterpret_cast<float4*>(reinterpret_cast<float*>(c) + row * n + n0 + cq * 64);
+#pragma unroll
+          for (int j = 0; j < 8; j++) {
+            o4[j] = make_float4(__uint_as_float(v0[4 * j]), __uint_as_float(v0[4 * j + 1]), __uint_as_float(v0[4 * j + 2]), __uint_as_float(v0[4 * j + 3]));
+            o4[8 + j] = make_float4(__uint_as_float(v1[4 * j]), __uint_as_float(v1[4 * j + 1]), __uint_as_float(v1[4 * j + 2]), __uint_as_float(v1[4 * j + 3]));
+          }
+        } else {
+          // row `lane`, 64 columns = eight 16-byte packets
+#pragma unroll
+          for (int p8 = 0; p8 < 8; p8++) {
+            uint4 pk;
+            __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&pk);
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-              o[q] = __fmul_rn(__fmul_rn(__uint_as_float(v[q]), w), xf);      // y * w_scale * x_scale, in that order
-              if (so.bias) o[q] = __fadd_rn(o[q], b[q]);
+              const int j = p8 * 8 + 2 * q;
+              h[q] = j < 32 ? __floats2bfloat162_rn(__uint_as_float(v0[j]), __uint_as_float(v0[j + 1]))
+                            : __floats2bfloat162_rn(__uint_as_float(v1[j - 32]), __uint_as_float(v1[j - 31]));
             }
-            if (so.y_f16) {
-              const __half2 h[2] = {__floats2half2_rn(o[0], o[1]), __floats2half2_rn(o[2], o[3])};
-              *reinterpret_cast<uint2*>(packet(j >> 3) + (j & 4) * 2) = *reinterpret_cast<const uint2*>(h);
-            } else {
-              *reinterpret_cast<float4*>(packet((j >> 2) & 7)) = make_float4(o[0], o[1], o[2], o[3]);
-              if (j == 28) send(col);
-            }
+            *reinterpret_cast<uint4*>(packet(p8)) = pk;
           }
-          send(so.y_f16 ? col : col + 32);
+          send(n0 + cq * 64);
         }
-        continue;
-      }
-      if constexpr (OUT == OUT_F32) {      // unrounded sums (the per-tensor FP8 linear scales them afterwards): each thread stores its own row
-        float4* o4 = reinterpret_cast<float4*>(reinterpret_cast<float*>(c) + row * n + n0 + cq * 64);
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-          o4[j] = make_float4(__uint_as_float(v0[4 * j]), __uint_as_float(v0[4 * j + 1]), __uint_as_float(v0[4 * j + 2]), __uint_as_float(v0[4 * j + 3]));
-          o4[8 + j] = make_float4(__uint_as_float(v1[4 * j]), __uint_as_float(v1[4 * j + 1]), __uint_as_float(v1[4 * j + 2]), __uint_as_float(v1[4 * j + 3]));
-        }
-        continue;
-      }
-      {
-        // row `lane`, 64 columns = eight 16-byte packets
-#pragma unroll
-        for (int p8 = 0; p8 < 8; p8++) {
-          uint4 pk;
-          __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&pk);
-#pragma unroll
-          for (int q = 0; q < 4; q++) {
-            const int j = p8 * 8 + 2 * q;
-            h[q] = j < 32 ? __floats2bfloat162_rn(__uint_as_float(v0[j]), __uint_as_float(v0[j + 1]))
-                          : __floats2bfloat162_rn(__uint_as_float(v1[j - 32]), __uint_as_float(v1[j - 31]));
-          }
-          *reinterpret_cast<uint4*>(packet(p8)) = pk;
-        }
-        send(n0 + cq * 64);
       }
     }
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");      // this warp's stores have left before the CTA does

@@ -15,7 +15,8 @@
 //  * a tile is up to 256 weight rows (two accumulators, the whole of tensor memory) by up to 256 activation rows: every unpacked weight meets
 //    256 rows and every activation byte 256 weight rows.  With 128 x 128 tiles the activation operand alone took 2.4x the L2 traffic
 //    and every weight was unpacked once per 128 rows.  Up to 128 rows, and where tiles are few, a tile is 128 weight rows
-//    (more tiles to share, smaller partial sums); up to 128 rows, and for half-precision rows, its weights go through tensor memory (qgemm_tmem.cuh);
+//    (more tiles to share, smaller partial sums), and where its loop is long enough the weights of such a tile go through tensor memory (qgemm_tmem.cuh; the rule is
+//    takes_tmem below: of fp32 rows up to 128);
 //  * roles are separate warps: 16 unpack the weights (packed blocks by asynchronous copies, several ahead -> fp16 halves in a ring of
 //    shared-memory slots), one thread brings activation tiles in by bulk copies, one issues the MMAs; nothing meets at a block barrier;
 //  * the K x tile space is dealt to one CTA per SM in equal contiguous runs (stream-K): no last wave.  A tile that spans CTAs leaves fp32
@@ -35,8 +36,8 @@ constexpr int THREADS = (UNPACK_WARPS + 2) * 32;
 constexpr int KSTEP = 32;                               // one quant block of K per step
 constexpr int RING_BYTES = 224 * 1024, MAX_SLOTS = 6;   // shared memory: slots of unpacked weights + activations
 // Packed blocks wait in shared memory, one 16 / 32-byte block and its scale per unpack thread and round, up to MAX_AHEAD rounds ahead.  A queue in
-// registers that moves up by a block waits for the newest load every time: whatever its depth, a round took a trip to HBM (8B gate / up, 45 rows: 83 us,
-// 70 here; 8 rows: 79, 60).
+// registers that moves up by a block waits for the newest load every time: whatever its depth, a round took a trip to HBM (measured when every row count came through
+// here, 8B gate / up: 45 rows 83 us, 70 so; 8 rows 79, 60).
 constexpr int MAX_AHEAD = 4;
 __host__ __device__ constexpr int ahead_bytes(int qt) { return UNPACK_THREADS * (qt == B200Q_Q4_0 ? 20 : 36); }
 constexpr int MAX_NT = 256;                             // activation rows per tile
@@ -64,8 +65,9 @@ struct StreamParams {
 // that a step's operand is one bulk copy.  Element order inside a chunk: [0,2,1,3,4,6,5,7], the order the weight unpack delivers.
 // One CTA: 8 rows (a core matrix) x a stretch of columns; a row's chunk is 32 bytes in, 16 + 16 bytes out, 8 rows make 128 contiguous bytes.
 // What is asked of a whole row (its mean square for the norm, its largest value for the scale) the CTAs of a row's stretches share as a cluster; stretches of up
-// to 2048 columns are read once and kept in registers, so rows that short need no cluster.  A prompt of 45 on 16 8B-shaped blocks: 3734 us; rows read twice, in
-// clusters from 2048 columns on, 4211; every CTA reading its whole rows 6900 (4540 for the mean square alone, without a scale).  Prompts on 384- to
+// to 2048 columns are read once and kept in registers, so rows that short need no cluster.  A prompt of 45 on 16 8B-shaped blocks when that took 3734 us (3080 since its
+// weights go through tensor memory): 477 us more with rows read twice, in clusters from 2048 columns on, 3170 more with every CTA reading its whole rows (806 for the
+// mean square alone, without a scale).  Prompts on 384- to
 // 1024-wide models take 2 to 5 % more than without a scale: the reduction in front of the stores, about half a microsecond a launch.
 constexpr int SPLIT_THREADS = 256, SPLIT_HOLD = 8;
 
@@ -623,6 +625,7 @@ int launch_stream(const StreamParams& p, int grid, cudaStream_t st) {
 // 74.  Tiles dealt to more than 8 CTAs (400 x 4096, 120 half-precision rows) are mostly the adding of their parts: 32 us, 25.
 bool takes_tmem(int qtype, const Plan& pl, bool f32, bool unsplit, long long units, long long tiles, int grid, int n_sm) {
   if (pl.wt != 128 || (f32 && pl.nt > 128)) return false;
+  if ((long long)grid * units >= 1LL << 32) return false;      // what first_group multiplies in 32 bits (no matrix that fits the GPU gets here: see there)
   if (unsplit) return true;
   if (grid > 8 * tiles) return false;
   return !f32 || pl.nt <= (qtype == B200Q_Q4_0 ? 48 : 32) || units >= (pl.nt <= 64 ? 4LL : 10LL) * n_sm;

@@ -79,7 +79,8 @@ __device__ __forceinline__ void ld_columns(uint32_t a, uint32_t (&v)[4]) {
 __device__ __forceinline__ void ld_columns(uint32_t a, uint32_t (&v)[8]) { ld_tmem(a, v); }
 
 struct Segment { int seg, tile, k0, k1; bool last; };      // number within the CTA's, K groups k0 .. k1 of tile; `last`: the CTA's last
-// The deal in 32 bits: K groups times CTAs stay below 2^32 for every matrix that fits the GPU (3.2e11 4-bit weights are 2e7 K groups of 128 rows).
+// The deal in 32 bits: K groups of all tiles times CTAs are below 2^32 (takes_tmem asks).  A matrix that fits the GPU has that: 3.2e11 4-bit weights are 2e7 K groups of
+// 128 rows, and more than one tile of activation rows meets tiles of 128 weight rows only where those are few (make_plan).
 __device__ __forceinline__ uint32_t first_group(uint32_t c, const StreamParams& p, uint32_t g) { return p.grain == 1 ? c * (uint32_t)p.units / g : c * p.tiles / g * p.grain; }
 __device__ __forceinline__ int cta_of_group(uint32_t unit, const StreamParams& p, uint32_t g) { return (int)(((unit + 1) * g - 1) / (uint32_t)p.units); }
 // the first of the CTAs that have a tile, and how many

@@ -120,8 +120,9 @@ def qgemm(w_ptr: int, qtype: int, n_out: int, n_in: int, x, y, m: int, x_dtype=F
 
 
 FEW_ROW_FUSED = os.environ.get("B200Q_FEW_ROW_FUSED", "1") == "1"      # batched decode with few rows: the int8-MMA few-row kernel
-# ... up to this many rows, 8 per pass over the weights.  A step of five 7B-shaped Q8_0 blocks and the head: 9 / 16 rows 1.03 / 1.06 ms in two passes against 1.13 / 1.17
-# on the GEMM, 17 rows 1.56 in three against 1.22.
+# ... up to this many rows, 8 per pass over the weights.  A step of five blocks and the head, 9 / 16 rows in two passes and on the GEMM, 17 in three and on the GEMM (ms):
+# 1024-wide Q8_0 0.25 / 0.26 and 0.31 / 0.31, 0.36 and 0.34; 2048-wide Q8_0 0.38 / 0.38 and 0.43 / 0.44, 0.54 and 0.49; 8B-shaped Q4_0 0.71 / 0.74 and 0.68 / 0.69, 1.06 and
+# 0.76; 7B-shaped Q8_0 0.86 / 0.87 and 0.80 / 0.82, 1.27 and 0.87.  (On the wide ones the GEMM is the faster from 9 rows on since its weights go through tensor memory.)
 FEW_ROW_MAX = int(os.environ.get("B200Q_FEW_ROW_MAX", "16"))
 
 
