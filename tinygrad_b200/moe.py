@@ -170,7 +170,7 @@ class ExpertWeights:
   """`ExpertWeights` of tinygrad/llm/model.py:21-27 on MXFP8 operands: weight (num_experts, out_features, in_features), and
   `__call__(sel, x)` with sel (T, k) int32 and x (T, 1, in) or (T, k, in) bf16 -> (T, k, out) bf16, row (t, j) = x[t, j or 0] @ weight[sel[t, j]].T.
   The rows are grouped by expert (b200q_moe_route_tables), quantised into the groups, multiplied by one grouped GEMM and gathered back
-  into (t, j) order.  out_features must be a multiple of 256 and in_features of 128 (the grouped GEMM's tile sizes)."""
+  into (t, j) order; the row of an entry of sel that is no expert is undefined.  out_features must be a multiple of 256 and in_features of 128 (the grouped GEMM's tile sizes)."""
   def __init__(self, weight: np.ndarray):
     self.num_experts, self.out_features, self.in_features = weight.shape
     if self.out_features % 256 or self.in_features % 128: raise ValueError("out_features % 256 == in_features % 128 == 0 is required")
