@@ -558,6 +558,10 @@ typedef struct b200q_moe_block {
   float *logits, *sh_act, *sh, *shg;
 } b200q_moe_block;
 int b200q_moe_rows(const b200q_rows_args* args, const b200q_moe_block* blocks, int seq, int start_pos, const int32_t* pos_dev, int n_rows, void* stream);
+/* One fp32 row x [n_in] times a packed Q4_0 / Q8_0 matrix in fp32 throughout (no activation codes): y [n_out] fp32 = W . (norm(x)) (+ bias fp16) (+ residual fp32), or
+ * silu(gate) * up of interleaved rows (n_out of them, no bias or residual).  For matrices small enough for a CTA per row tile; n_in a multiple of 32 up to 44032. */
+int b200q_row_gemv(int qtype, const void* w_packed, const float* x, const void* norm_weight, float norm_eps, const void* bias_f16, const float* residual, int epilogue,
+                   float* y, int n_out, int n_in, int flags, void* stream);
 /* `grouped_mx_gemm` (extra/gemm/moe_gemm.py:112-134; kernel contract extra/thunder/amd/grouped_mxfp8_gemm.cpp:32-158):
  * C[m_total, n] bf16 = A_q[m_total, k] x B_q[e][n, k]^T with both operands' E8M0 scales, fp32 accumulation; rows
  * off[e]..off[e+1] use expert e; rows past off[n_experts] are left untouched.  m_total % 256 == n % 256 == k % 128 == 0

@@ -190,6 +190,7 @@ SIGNATURES = {
   "b200q_moe_combine": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]),
   "b200q_mx_status_read_clear": (c_int, [POINTER(c_int)]),
   "b200q_moe_layer": (c_int, [POINTER(MoeArgs), c_void_p, c_void_p, c_int, c_void_p, c_void_p]),
+  "b200q_row_gemv": (c_int, [c_int, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p]),
   "b200q_moe_rows": (c_int, [POINTER(RowsArgs), POINTER(MoeBlock), c_int, c_int, c_void_p, c_int, c_void_p]),
   "b200q_grouped_mxfp8_gemm": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
   "b200q_grouped_mxfp8_gemm_f32": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p]),

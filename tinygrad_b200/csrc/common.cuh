@@ -47,6 +47,9 @@ int b200q_rmsnorm_rows_chain(const float* x, const void* weight_f16, float eps, 
 int b200q_add_rows_gated_chain(float* x, const float* y, const float* gate_logit, int n_rows, int dim, cudaStream_t st);
 int b200q_attn_rows_pos_chain(const float* qkv, void* k_cache, void* v_cache, int kv_dtype, const float* rope, const int32_t* pos_dev, int n_heads, int n_kv_heads, int head_dim,
                               int rope_dim, int max_context, void* q_scratch, void* out, int out_dtype, cudaStream_t st);
+// one row times a packed matrix in fp32 (row_gemv.cu)
+int b200q_row_gemv_chain(int qtype, const void* w_packed, const float* x, const void* norm_weight, float norm_eps, const void* bias_f16, const float* residual, int epilogue,
+                         float* y, int n_out, int n_in, cudaStream_t st, bool pdl);
 int b200q_decode_status_take(int* status);
 int b200q_decode_step_status_take(int* status);   // the same for the whole-step kernel (decode_step.cu)
 int b200q_peer_status_take(int* status);          // the same for the peer-memory collectives (peer.cu)

@@ -596,6 +596,16 @@ extern "C" int b200q_status_read_clear(int* status) {
   return B200Q_OK;
 }
 
+// Plain calls on one fp32 row whose matrix is a launch's latency and no more (row_gemv.cu).  The line, in us a launch in a chain, streaming kernel / that one, Q4_0 (Q8_0):
+// 512 x 512 2.4 / 1.7 (2.3 / 1.7), 2816 x 512 2.6 / 2.3 (3.0 / 2.1), 5632 x 1024 3.7 / 2.9 (3.8 / 2.9), 3072 x 2048 3.3 / 3.2 (3.5 / 3.1); past it 3584 x 3584 4.0 / 4.4
+// (4.4 / 4.5), 11264 x 2048 5.4 / 8.5 (6.7 / 9.6), 1024 x 2816 3.3 / 3.4 (3.0 / 3.2: few tiles, more groups than two a warp).
+static bool takes_row(const b200q_gemv_args* a) {
+  if ((a->qtype != B200Q_Q4_0 && a->qtype != B200Q_Q8_0) || a->m != 1 || a->x_dtype != B200Q_F32 || a->y_dtype != B200Q_F32) return false;
+  if (!a->x || !a->y || a->xq_in || a->xq_out || a->n_peers || a->max_ctas > 0 || (a->residual_scale != 0.f && a->residual_scale != 1.f)) return false;
+  const int groups = ceil_div(a->n_in, GROUP_ELEMS), tiles = ceil_div(a->n_out, a->epilogue == B200Q_EPI_SILU_MUL ? 8 : TILE_ROWS);
+  return groups <= 16 && tiles * (long long)groups <= 4096;
+}
+
 extern "C" size_t b200q_xq_bytes(int n) { return n > 0 ? xq_record_bytes(n) : 0; }
 
 extern "C" int b200q_gemv(const b200q_gemv_args* a, void* stream) {
@@ -645,6 +655,8 @@ extern "C" int b200q_gemv(const b200q_gemv_args* a, void* stream) {
     }
     p.n_peers = a->n_peers; p.peer_rank = a->peer_rank;
   }
+  if (takes_row(a)) return b200q_row_gemv_chain(a->qtype, a->w_packed, (const float*)a->x, a->norm_weight, a->norm_eps, a->bias, (const float*)a->residual, a->epilogue, (float*)a->y,
+                                                a->n_out, a->n_in, (cudaStream_t)stream, (a->flags & B200Q_FLAG_PDL) != 0);
   p.out_stage = (uint32_t*)a->xq_out_stage;
   p.unit = (a->xq_out && !a->xq_out_stage) ? (a->epilogue == B200Q_EPI_SILU_MUL ? 4 : 2) : 1;
   p.n_units = ceil_div(p.n_row_tiles, p.unit);
