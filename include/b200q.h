@@ -477,6 +477,9 @@ typedef struct b200q_rows_args {
   size_t workspace_bytes;
 } b200q_rows_args;
 int b200q_prompt_rows(const b200q_rows_args* args, int first_seq, int n_seqs, int start_pos, int n_rows, void* stream);
+/* The same without what nobody reads when only the last token's logits are wanted: the last block leaves its cache rows (RMSNorm, q | k | v, RoPE, append) and x the
+ * rows that went INTO it.  The caller takes the rows it needs from there through that block and the head. */
+int b200q_prompt_rows_kv(const b200q_rows_args* args, int first_seq, int n_seqs, int start_pos, int n_rows, void* stream);
 /* Batched decode (the reference's forward on tokens [B, 1], tinygrad/llm/model.py:358-364 with B > 1): row b of qkv is sequence b's
  * new token, every sequence at position pos (or *pos_dev when that device pointer is given: graph replay); caches
  * [n_seqs, n_kv_heads, max_context, head_dim]; otherwise as b200q_attn_prefill. */

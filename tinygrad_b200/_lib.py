@@ -147,6 +147,7 @@ SIGNATURES = {
   "b200q_argmax_advance_seqs": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p]),
   "b200q_wait_words": (c_int, [c_void_p, c_int, c_int32, c_void_p]),
   "b200q_prompt_rows": (c_int, [POINTER(RowsArgs), c_int, c_int, c_int, c_int, c_void_p]),
+  "b200q_prompt_rows_kv": (c_int, [POINTER(RowsArgs), c_int, c_int, c_int, c_int, c_void_p]),
   "b200q_attn_prefill_seqs": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                                       c_int, c_void_p]),
   "b200q_advance": (c_int, [c_void_p, c_int, c_int, c_void_p]),

@@ -19,6 +19,7 @@ void b200q_set_cuda_error(cudaError_t e);
 int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtype, const void* norm_weight, float norm_eps, const void* bias_f16, const void* residual,
                       int epilogue, void* y, int y_dtype, int m, int n_out, int n_in, void* workspace, size_t workspace_bytes, cudaStream_t st, bool pdl,
                       bool unsplit = false);
+// out NULL: RoPE and the cache rows only
 int b200q_attn_rows_chain(const float* qkv, void* k_cache, void* v_cache, int kv_dtype, const float* rope, int start_pos, int n_rows, int n_seqs, int n_heads,
                           int n_kv_heads, int head_dim, int rope_dim, int max_context, void* q_scratch, void* out, int out_dtype, cudaStream_t st, bool pdl);
 

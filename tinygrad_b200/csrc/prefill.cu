@@ -464,8 +464,8 @@ extern "C" int b200q_add_rows_bf16(float* x, const void* y_bf16, int64_t n, void
 
 static int attn_rows(const float* qkv, void* k_cache, void* v_cache, int kv_dtype, const float* rope, int start_pos, int n_rows, int n_heads,
                      int n_kv_heads, int head_dim, int rope_dim, int max_context, void* q_scratch, void* out, int out_dtype, int n_seqs,
-                     const int32_t* pos_dev, void* stream, bool pdl = false) {      // n_rows: per sequence
-  if (!qkv || !k_cache || !v_cache || !rope || !q_scratch || !out || (out_dtype != B200Q_F16 && out_dtype != B200Q_F32)) return B200Q_ERR_BAD_ARG;
+                     const int32_t* pos_dev, void* stream, bool pdl = false) {      // n_rows: per sequence; out NULL: the cache rows only
+  if (!qkv || !k_cache || !v_cache || !rope || !q_scratch || (out_dtype != B200Q_F16 && out_dtype != B200Q_F32)) return B200Q_ERR_BAD_ARG;
   const bool of16 = out_dtype == B200Q_F16;
   if (n_rows <= 0 || n_seqs <= 0 || n_seqs > 65535 || start_pos < 0 || n_heads <= 0 || n_kv_heads <= 0 || n_heads % n_kv_heads) return B200Q_ERR_BAD_ARG;
   if (kv_dtype != B200Q_F16 && kv_dtype != B200Q_F32) return B200Q_ERR_BAD_ARG;
@@ -480,6 +480,7 @@ static int attn_rows(const float* qkv, void* k_cache, void* v_cache, int kv_dtyp
                                    (__half*)k_cache, (__half*)v_cache, (float*)q_scratch, n_rows, pos_dev));
   else B200Q_CHECK_CUDA(launch_k(rope_kv_rows_kernel<float>, rgrid, dim3(256), 0, st, pdl, qkv, rope, start_pos, n_heads, n_kv_heads, head_dim, rope_dim, max_context,
                                  (float*)k_cache, (float*)v_cache, (float*)q_scratch, n_rows, pos_dev));
+  if (!out) return B200Q_OK;
   cudaError_t e;
 #define PF_CASE(HD)                                                                                                                     \
   case HD: e = h ? launch_prefill_attn<HD, __half>(q_scratch, k_cache, v_cache, start_pos, n_rows, n_heads, n_kv_heads, max_context, out, of16, n_seqs, pos_dev, st)  \
@@ -493,6 +494,7 @@ static int attn_rows(const float* qkv, void* k_cache, void* v_cache, int kv_dtyp
 extern "C" int b200q_attn_prefill(const float* qkv, void* k_cache, void* v_cache, int kv_dtype, const float* rope, int start_pos, int n_rows,
                                   int n_heads, int n_kv_heads, int head_dim, int rope_dim, int max_context, void* q_scratch, void* out,
                                   int out_dtype, void* stream) {
+  if (!out) return B200Q_ERR_BAD_ARG;
   return attn_rows(qkv, k_cache, v_cache, kv_dtype, rope, start_pos, n_rows, n_heads, n_kv_heads, head_dim, rope_dim, max_context, q_scratch, out, out_dtype, 1,
                    nullptr, stream);
 }
@@ -511,6 +513,7 @@ int b200q_attn_rows_pos_chain(const float* qkv, void* k_cache, void* v_cache, in
 extern "C" int b200q_attn_prefill_seqs(const float* qkv, void* k_cache, void* v_cache, int kv_dtype, const float* rope, int start_pos, int n_rows, int n_seqs,
                                        int n_heads, int n_kv_heads, int head_dim, int rope_dim, int max_context, void* q_scratch, void* out,
                                        int out_dtype, void* stream) {
+  if (!out) return B200Q_ERR_BAD_ARG;
   return attn_rows(qkv, k_cache, v_cache, kv_dtype, rope, start_pos, n_rows, n_heads, n_kv_heads, head_dim, rope_dim, max_context, q_scratch, out, out_dtype,
                    n_seqs, nullptr, stream);
 }
@@ -518,6 +521,7 @@ extern "C" int b200q_attn_prefill_seqs(const float* qkv, void* k_cache, void* v_
 extern "C" int b200q_attn_decode_batch(const float* qkv, void* k_cache, void* v_cache, int kv_dtype, const float* rope, int pos, const int32_t* pos_dev,
                                        int n_seqs, int n_heads, int n_kv_heads, int head_dim, int rope_dim, int max_context, void* q_scratch, void* out,
                                        int out_dtype, void* stream) {
+  if (!out) return B200Q_ERR_BAD_ARG;
   return attn_rows(qkv, k_cache, v_cache, kv_dtype, rope, pos_dev ? 0 : pos, 1, n_heads, n_kv_heads, head_dim, rope_dim, max_context, q_scratch, out, out_dtype,
                    n_seqs, pos_dev, stream);
 }

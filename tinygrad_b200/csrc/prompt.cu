@@ -7,7 +7,10 @@
 
 int b200q_embed_rows_seqs(const void* table_f16, const int32_t* tokens, int token_stride, int per_seq, int n_rows, int dim, int vocab, float* x, cudaStream_t st);
 
-extern "C" int b200q_prompt_rows(const b200q_rows_args* a, int first_seq, int n_seqs, int start_pos, int n_rows, void* stream) {
+// kv_only: the last block only leaves its cache rows; x keeps what goes into it.  What else it would compute nobody reads when the last token's logits are all that is
+// wanted: of a prompt of 1999 tokens on ten 7B-shaped blocks that was 2.3 ms, and the last token as a step of its own 0.7 (29.8 -> 26.8 ms; 45 tokens on 16 8B-shaped blocks
+// 3.08 -> 2.41 ms; eight prompts of 128 and 32 answers on seven blocks 29.1 -> 27.4 ms).
+static int prompt_rows(const b200q_rows_args* a, int first_seq, int n_seqs, int start_pos, int n_rows, bool kv_only, void* stream) {
   if (!a || !a->layers || !a->token_embd || !a->rope || !a->tokens || !a->x || !a->qkv || !a->q || !a->att || !a->act || !a->workspace) return B200Q_ERR_BAD_ARG;
   if (first_seq < 0 || n_seqs <= 0 || start_pos < 0 || n_rows <= 0 || a->n_layers < 0 || (long long)n_seqs * n_rows > a->rows_max) return B200Q_ERR_BAD_ARG;
   if (start_pos + n_rows > a->max_context) return B200Q_ERR_TOO_LARGE;
@@ -18,11 +21,13 @@ extern "C" int b200q_prompt_rows(const b200q_rows_args* a, int first_seq, int n_
   int rc = b200q_embed_rows_seqs(a->token_embd, a->tokens + (size_t)first_seq * stride + start_pos, stride, n_rows, T, a->dim, a->vocab, a->x, st);
   for (int i = 0; i < a->n_layers && rc == B200Q_OK; i++) {
     const b200q_decode_layer& l = a->layers[i];
+    const bool kv = kv_only && i == a->n_layers - 1;
     rc = b200q_qgemm_chain(a->qtype, l.qkv, a->x, B200Q_F32, l.attn_norm, a->norm_eps, l.qkv_bias, nullptr, B200Q_EPI_LINEAR, a->qkv, B200Q_F32, T, qkv_rows,
                              a->dim, a->workspace, a->workspace_bytes, st, true);
     if (rc == B200Q_OK)
       rc = b200q_attn_rows_chain(a->qkv, (char*)l.k_cache + first_seq * seq_bytes, (char*)l.v_cache + first_seq * seq_bytes, a->kv_dtype, a->rope, start_pos, n_rows,
-                                   n_seqs, a->n_heads, a->n_kv_heads, a->head_dim, a->rope_dim, a->max_context, a->q, a->att, B200Q_F32, st, true);
+                                   n_seqs, a->n_heads, a->n_kv_heads, a->head_dim, a->rope_dim, a->max_context, a->q, kv ? nullptr : a->att, B200Q_F32, st, true);
+    if (kv) break;
     if (rc == B200Q_OK)
       rc = b200q_qgemm_chain(a->qtype, l.attn_output, a->att, B200Q_F32, nullptr, 0.f, nullptr, a->x, B200Q_EPI_LINEAR, a->x, B200Q_F32, T, a->dim, q_dim, a->workspace,
                           a->workspace_bytes, st, true);
@@ -34,6 +39,12 @@ extern "C" int b200q_prompt_rows(const b200q_rows_args* a, int first_seq, int n_
                           a->workspace_bytes, st, true);
   }
   return rc;
+}
+extern "C" int b200q_prompt_rows(const b200q_rows_args* a, int first_seq, int n_seqs, int start_pos, int n_rows, void* stream) {
+  return prompt_rows(a, first_seq, n_seqs, start_pos, n_rows, false, stream);
+}
+extern "C" int b200q_prompt_rows_kv(const b200q_rows_args* a, int first_seq, int n_seqs, int start_pos, int n_rows, void* stream) {
+  return prompt_rows(a, first_seq, n_seqs, start_pos, n_rows, true, stream);
 }
 
 // The same for a mixture-of-experts model: the FFN of a block is the router, the expert layer and, where the model has one, the shared expert

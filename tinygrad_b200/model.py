@@ -278,7 +278,7 @@ class Transformer:
     self.prefill_rows = prefill_rows if (tp is None and not self.dense_blocks and c.hidden_dim % 8 == 0 and c.head_dim in (16, 32, 64, 128)) else 0
     self.prefill_chunk, self._pf, self._batch_logits, self._rows_ws, self._batch_graph = max(1, prefill_chunk), None, None, None, None
     self._rows_args, self._moe_blocks = None, {}
-    self._seq_attn_scratch = None
+    self._seq_attn_scratch = self._last_rows = None
     self.is_moe, self._host_pos, self._rows_warm = c.num_experts > 0, 0, False
     if self.is_moe:
       assert tp is None and c.head_dim in (16, 32, 64, 128), "the mixture-of-experts model runs on the row path of one GPU"
@@ -314,7 +314,8 @@ class Transformer:
     self.engine = "step" if self._step_args else "chain"
 
   # ---- one token through the network (launch sequence; captured into a graph) ----
-  def _enqueue_step(self, with_head: bool, attention: bool = True, tail: bool = True) -> None:
+  def _enqueue_step(self, with_head: bool, attention: bool = True, tail: bool = True, last_block: bool = False) -> None:
+    """last_block: the last block and what follows it, on the row in `x` (a prompt's last row, behind the pass over the prompt)."""
     c, lib, s, fl = self.config, _lib.load(), self.stream.ptr, self.flags
     kvdt = F16 if c.kv_dtype == "float16" else F32
     grid = lambda name: self.gemv_max_ctas.get(name, self.gemv_max_ctas.get("*", 0))
@@ -329,14 +330,14 @@ class Transformer:
     rkw_o = dict(peers=self.mb_o.targets, peer_rank=tp.rank) if peer else rkw
     rkw_d = dict(peers=self.mb_down.targets, peer_rank=tp.rank) if peer else rkw
     vocab_full = self.full_config.vocab_size
-    e, nss = self.edges, c.dim // 32
+    e, nss = self.edges - {"down_qkv"} if last_block else self.edges, c.dim // 32
     qkv_rows = self.q_dim + 2 * self.kv_dim
     # the four hand-over edges: kwargs of the consuming (xq_in...) and of the producing (xq_out...) launch
     in_a = dict(xq_in=self.xq_a, ss_in=self.ss_a, ss_count=nss) if "down_qkv" in e else {}
     in_b = dict(xq_in=self.xq_b, ss_in=self.ss_b, ss_count=nss) if "o_gateup" in e else {}
     in_attn = dict(xq_in=self.xq_attn) if "attn_o" in e else {}
     in_act = dict(xq_in=self.xq_act) if "gateup_down" in e else {}
-    if attention or tail:
+    if (attention or tail) and not last_block:
       ho = "down_qkv" in e
       check(lib.b200q_embed(self.token_embd.ptr, self.tokens.ptr, self.pos.ptr, self.x.ptr, c.dim, vocab_full, c.max_context,
                             self.xq_a.ptr if ho else None, self.blk[0].attn_norm.ptr if ho else None, self.ss_a.ptr if ho else None, fl, s))
@@ -350,14 +351,14 @@ class Transformer:
       for w, y in zip(b.gate_up, (self.act, self.up_buf)): w.run(self.x, y, norm_weight=b.ffn_norm, norm_eps=c.norm_eps, flags=fl, stream=s)
       if not b.gate_up[0].swiglu: check(lib.b200q_silu_mul(self.act.ptr, self.up_buf.ptr, self.act.ptr, c.hidden_dim, fl, s))
       b.down_w.run(self.act, self.x, residual=self.x, flags=fl, stream=s)
-    for i, b in enumerate(() if self.dense_blocks else self.blk):
+    for i, b in () if self.dense_blocks else list(enumerate(self.blk))[-1 if last_block else 0:]:
       nxt_norm = self.blk[i + 1].attn_norm if i + 1 < len(self.blk) else self.output_norm
       st = (lambda n: dict(xq_out_stage=self.ho_stage[n])) if self.ho_stage is not None else (lambda n: {})
       out_b = dict(xq_out=self.xq_b, xq_out_norm_weight=b.ffn_norm, ss_out=self.ss_b, **st(c.dim)) if "o_gateup" in e else {}
       out_act = dict(xq_out=self.xq_act, **st(c.hidden_dim)) if "gateup_down" in e else {}
       out_a = dict(xq_out=self.xq_a, xq_out_norm_weight=nxt_norm, ss_out=self.ss_a, **st(c.dim)) if "down_qkv" in e else {}
       quant.gemv(b.qkv.ptr, self.qtype, qkv_rows, c.dim, None if in_a else self.x, self.qkv, norm_weight=b.attn_norm, norm_eps=c.norm_eps,
-                 bias=b.qkv_bias, max_ctas=grid("qkv"), **in_a, **(kw_after_coll if i > 0 else kw))
+                 bias=b.qkv_bias, max_ctas=grid("qkv"), **in_a, **(kw_after_coll if i > 0 else kw))      # (last_block: a graph's first node, or behind a copy: fully ordered)
       if attention:
         a = _lib.AttnArgs(self.qkv.ptr, b.k_cache.ptr, b.v_cache.ptr, kvdt, self.rope.ptr, self.pos.ptr, self.attn.ptr, self.attn_scratch.ptr,
                           c.n_heads, c.n_kv_heads, c.head_dim, c.rope_dim, c.max_context, self.n_split, fl,
@@ -414,13 +415,17 @@ class Transformer:
         if c.shared_expert_dim: self._pf.update(sh=DeviceBuffer.empty((T, c.dim), np.float32), shg=DeviceBuffer.empty((T,), np.float32))
     return self._pf
 
-  def prefill(self, start_pos: int, n: int, sync: bool = True, seq: int = 0) -> None:
+  _take_along = False      # set by `generate` for its call of `prefill`
+
+  def prefill(self, start_pos: int, n: int, sync: bool = True, seq: int = 0):
     """Run tokens[start_pos : start_pos + n] (already on the device) through every block and fill the KV cache; no logits.
     The forward of tinygrad/llm/model.py:358-362 for T = n, in chunks: per block rmsnorm -> QKV GEMM -> RoPE + cache append +
     causal attention -> O GEMM (+residual) -> rmsnorm -> gate/up GEMM with SwiGLU epilogue -> down GEMM (+residual).
-    Activations stay fp32 between the kernels; the GEMMs split them into fp16 hi + lo halves for the tensor core."""
+    Activations stay fp32 between the kernels; the GEMMs split them into fp16 hi + lo halves for the tensor core.
+    Called by `generate`, whose prompt has one more token: that one goes along where it can, and what finishes it is returned."""
     c, lib, s, f = self.config, _lib.load(), self.stream.ptr, self._prefill_buffers()
-    native = self._native_rows()
+    native, along, self._take_along = self._native_rows(), self._take_along, False
+    if along and native and n % self.prefill_chunk: return self._prompt_to_last_block(native, start_pos, n + 1)      # (a last pass of one row would cost what a step does)
     for p0 in range(start_pos, start_pos + n, self.prefill_chunk) if native else ():
       check(lib.b200q_prompt_rows(native, seq, 1, p0, min(self.prefill_chunk, start_pos + n - p0), s))
     for p0 in () if native else range(start_pos, start_pos + n, self.prefill_chunk):
@@ -435,6 +440,37 @@ class Transformer:
       self.stream.synchronize()
       self.pos.copy_from(np.array([start_pos + n], dtype=np.int32), offset=4 * seq)
       self._host_pos = start_pos + n
+
+  def _prompt_rows(self, native, start_pos: int, n: int, seq: int = 0) -> int:
+    """Prompt tokens of one sequence, of which only the cache rows are wanted and what goes into the last block: the rows of the last pass, whose number is returned, are
+    in the row buffer then."""
+    for p0 in range(start_pos, start_pos + n, self.prefill_chunk):
+      rows = min(self.prefill_chunk, start_pos + n - p0)
+      check(_lib.load().b200q_prompt_rows_kv(native, seq, 1, p0, rows, self.stream.ptr))
+    return rows
+
+  def _last_block(self, enqueue) -> None:
+    """Replays the last block, the head and the arg-max on rows that a prompt pass has left (captured on first use)."""
+    self._head_queued = True
+    if not self.use_graph: return enqueue()
+    g = self._graphs.get("last_block")
+    if g is None:
+      g = Graph(self.stream)
+      with g: enqueue()
+      self._graphs["last_block"] = g
+    g.launch()
+
+  def _prompt_to_last_block(self, native, start_pos: int, n: int):
+    """tokens[start_pos : start_pos + n] as rows up to the last block -> what takes the last one of them through that and samples the token behind it."""
+    self.pos.copy_from(np.array([start_pos + n - 1], dtype=np.int32), stream=self.stream)
+    rows, size = self._prompt_rows(native, start_pos, n), 4 * self.config.dim
+    check(_lib.load().b200q_memcpy_d2d(self.x.ptr, self._pf["x"].ptr + (rows - 1) * size, size, self.stream.ptr))
+    self._host_pos = start_pos + n - 1
+    def finish():
+      self._check_room()
+      self._host_pos += 1
+      self._last_block(lambda: self._enqueue_step(True, last_block=True))
+    return finish
 
   def _enqueue_rows_block(self, b, T: int, f: dict, p0, seq: int) -> None:
     """One block for T rows in f["x"]: positions p0 .. of sequence `seq`, or (p0 None) one row at the position kept on the device."""
@@ -523,34 +559,41 @@ class Transformer:
     self._batch_graph.launch()
     self._host_pos += 1
 
-  def _enqueue_batch_step(self, count: bool = True) -> None:
-    c, lib, s, f, B = self.config, _lib.load(), self.stream.ptr, self._prefill_buffers(), self.batch
-    assert B <= self.prefill_chunk and not self.is_moe
-    kvdt = F16 if c.kv_dtype == "float16" else F32
-    qkv_rows = self.q_dim + 2 * self.kv_dim
-    head_q = not isinstance(self.output, quant.DenseWeight)
+  def _batch_buffers(self):
+    """What a step of the batch needs besides the row buffers (allocated on first use) -> (quantised head, few-row kernel, attention in one launch)."""
+    c, lib, B = self.config, _lib.load(), self.batch
+    qkv_rows, head_q = self.q_dim + 2 * self.kv_dim, not isinstance(self.output, quant.DenseWeight)
     few = B <= quant.FEW_ROW_MAX and quant.FEW_ROW_FUSED     # 8 rows per pass on the int8 tensor cores at the one-row GEMV's arithmetic; else one pass of the GEMM
     if self._rows_ws is None:
       shapes = [(qkv_rows, c.dim), (c.dim, self.q_dim), (2 * c.hidden_dim, c.dim), (c.dim, c.hidden_dim)] + ([(c.vocab_size, c.dim)] if head_q else [])
       need = quant.qgemv_rows_workspace_bytes if few else (lambda m, o, i: quant.qgemm_workspace_bytes(m, i, o))
       self._rows_ws = DeviceBuffer(max(need(B, o, i) for o, i in shapes))
-    if few:
-      def gemm(w, qt, n_out, n_in, x, y, **kw): quant.qgemv_rows(w, qt, n_out, n_in, x, y, B, self._rows_ws, x_dtype=F32, y_dtype=F32, stream=s, **kw)
-    else:
-      def gemm(w, qt, n_out, n_in, x, y, **kw): quant.qgemm(w, qt, n_out, n_in, x, y, B, x_dtype=F32, y_dtype=F32, stream=s, workspace=self._rows_ws, **kw)
-    # the position comes from the device (sequence 0's counter; all sequences move together), so the launch sequence can be replayed as a graph
-    check(lib.b200q_embed_rows(self.token_embd.ptr, self.tokens.ptr, c.max_context + 1, self.pos.ptr, B, c.dim, c.vocab_size, f["x"].ptr, s))
-    fold = few or quant.PIPELINED_GEMM     # both apply the RMSNorm in their pre-pass: no norm launches
     # head_dim 64 or 128: one launch of the cluster kernel, a cluster per (KV head, sequence)
     seq_attn = (SEQ_ATTENTION or c.head_dim in (64, 128)) and c.n_heads // c.n_kv_heads <= 8 and c.head_dim % 8 == 0 and c.head_dim <= 128
     if seq_attn and self._seq_attn_scratch is None:
       stride = lib.b200q_attn_seq_scratch_stride(c.n_heads, c.n_kv_heads, c.head_dim, self.n_split)
       self._seq_attn_scratch = DeviceBuffer(B * stride, zero=True)
+    if self._batch_logits is None: self._batch_logits = DeviceBuffer.empty((B, c.vocab_size), np.float32)
+    return head_q, few, seq_attn
+
+  def _enqueue_batch_step(self, count: bool = True, last_block: bool = False) -> None:
+    c, lib, s, f, B = self.config, _lib.load(), self.stream.ptr, self._prefill_buffers(), self.batch
+    assert B <= self.prefill_chunk and not self.is_moe
+    kvdt = F16 if c.kv_dtype == "float16" else F32
+    qkv_rows = self.q_dim + 2 * self.kv_dim
+    head_q, few, seq_attn = self._batch_buffers()
+    if few:
+      def gemm(w, qt, n_out, n_in, x, y, **kw): quant.qgemv_rows(w, qt, n_out, n_in, x, y, B, self._rows_ws, x_dtype=F32, y_dtype=F32, stream=s, **kw)
+    else:
+      def gemm(w, qt, n_out, n_in, x, y, **kw): quant.qgemm(w, qt, n_out, n_in, x, y, B, x_dtype=F32, y_dtype=F32, stream=s, workspace=self._rows_ws, **kw)
+    # the position comes from the device (sequence 0's counter; all sequences move together), so the launch sequence can be replayed as a graph
+    if not last_block: check(lib.b200q_embed_rows(self.token_embd.ptr, self.tokens.ptr, c.max_context + 1, self.pos.ptr, B, c.dim, c.vocab_size, f["x"].ptr, s))
+    fold = few or quant.PIPELINED_GEMM     # both apply the RMSNorm in their pre-pass: no norm launches
     def normed(norm):
       if fold: return f["x"], {"norm_weight": norm, "norm_eps": c.norm_eps}
       check(lib.b200q_rmsnorm_rows(f["x"].ptr, norm.ptr, c.norm_eps, B, c.dim, f["xn"].ptr, F32, s))
       return f["xn"], {}
-    for b in self.blk:
+    for b in self.blk[-1:] if last_block else self.blk:
       xin, kw = normed(b.attn_norm)
       gemm(b.qkv.ptr, self.qtype, qkv_rows, c.dim, xin, f["qkv"], bias=b.qkv_bias, **kw)
       if seq_attn:     # the one-token kernel over (KV head, slice, sequence): RoPE, cache append and attention in one launch
@@ -564,7 +607,6 @@ class Transformer:
       xin, kw = normed(b.ffn_norm)
       gemm(b.gate_up.buf.ptr, self.qtype, 2 * c.hidden_dim, c.dim, xin, f["act"], epilogue=EPI_SILU_MUL, **kw)
       gemm(b.ffn_down.buf.ptr, self.qtype, c.dim, c.hidden_dim, f["act"], f["x"], residual=f["x"])
-    if self._batch_logits is None: self._batch_logits = DeviceBuffer.empty((B, c.vocab_size), np.float32)
     if head_q and fold:
       gemm(self.output.buf.ptr, self.output_type, c.vocab_size, c.dim, f["x"], self._batch_logits, norm_weight=self.output_norm, norm_eps=c.norm_eps)
     else:
@@ -579,11 +621,29 @@ class Transformer:
     """tokens[:n] of every sequence: as many whole sequences per pass as fit prefill_chunk rows (the weights are streamed once per pass)."""
     native, per = self._native_rows(), self.prefill_chunk // n
     if native is None or per < 2:
-      for i in range(self.batch): self.prefill(0, n, seq=i)
-      return
-    for i in range(0, self.batch, per):
-      check(_lib.load().b200q_prompt_rows(native, i, min(per, self.batch - i), 0, n, self.stream.ptr))
+      for i in range(self.batch):
+        if native is None: self.prefill(0, n, seq=i)
+        else: self._prompt_rows(native, 0, n, seq=i)
+    else:
+      for i in range(0, self.batch, per):
+        check(_lib.load().b200q_prompt_rows_kv(native, i, min(per, self.batch - i), 0, n, self.stream.ptr))
     self.stream.synchronize()
+
+  def _prompt_tokens(self, native, per: int, n: int) -> None:
+    """The first n tokens of every sequence, `per` sequences in a pass, and the tokens behind them: the passes' last rows are gathered for the last block."""
+    B, f, lib, s, size = self.batch, self._pf, _lib.load(), self.stream.ptr, 4 * self.config.dim
+    self._batch_buffers()      # (a capture allocates nothing)
+    self.pos.copy_from(np.full((B,), n - 1, dtype=np.int32), stream=self.stream)
+    if self._last_rows is None: self._last_rows = DeviceBuffer.empty((B, self.config.dim), np.float32), DeviceBuffer.empty((B,), np.int32)
+    last, at = self._last_rows
+    at.copy_from(np.arange(n - 1, n * per, n, dtype=np.int32), stream=self.stream)
+    for i in range(0, B, per):
+      seqs = min(per, B - i)
+      check(lib.b200q_prompt_rows_kv(native, i, seqs, 0, n, s))
+      check(lib.b200q_permute_rows(f["x"].ptr, at.ptr, seqs, size, last.ptr + i * size, 1, s))
+    check(lib.b200q_memcpy_d2d(f["x"].ptr, last.ptr, B * size, s))
+    self._host_pos = n
+    self._last_block(lambda: self._enqueue_batch_step(count=False, last_block=True))
 
   def generate_batch(self, prompts: list):
     """Greedy generation for `batch` prompts of equal length; yields the list of the sequences' next tokens per step."""
@@ -594,12 +654,17 @@ class Transformer:
     tok = np.zeros((B, c.max_context + 1), np.int32)
     for i, p in enumerate(prompts): tok[i, :L] = p
     self.tokens.copy_from(tok)
-    if L > 1: self._prefill_batch(L - 1)
-    self.pos.copy_from(np.full((B,), L - 1, dtype=np.int32))
-    self._host_pos, n = L - 1, L
+    step, n = self.decode_batch_step, L
+    native, per = self._native_rows() if 1 < L < c.max_context else None, min(self.prefill_chunk // L, B)
+    # several sequences in a pass, and no more passes than without their last tokens
+    if native is not None and per >= 2 and -(-B // per) == -(-B // min(self.prefill_chunk // (L - 1), B)): step = lambda: self._prompt_tokens(native, per, L)
+    else:
+      if L > 1: self._prefill_batch(L - 1)
+      self.pos.copy_from(np.full((B,), L - 1, dtype=np.int32))
+      self._host_pos = L - 1
     while n < c.max_context:
-      yield self._sampled(self.decode_batch_step, B)
-      n += 1
+      yield self._sampled(step, B)
+      step, n = self.decode_batch_step, n + 1
 
   def _step_rows(self, with_head: bool) -> None:
     """One token through the row path (mixture-of-experts models: their FFN is not part of the fused one-token chain).  Positions come
@@ -716,21 +781,23 @@ class Transformer:
     return lo
 
   def generate(self, tokens: list, temperature: float = 0.0):
-    """Greedy generation (model.py:464-484 at temperature 0).  Yields one token id at a time; a prompt is consumed in chunks (`prefill_rows`) or one
-    position per step, its last token always in the step that samples the first answer token."""
+    """Greedy generation (model.py:464-484 at temperature 0).  Yields one token id at a time; a prompt is consumed in chunks (`prefill_rows`), its last token with them
+    up to the last block, or one position per step."""
     if temperature != 0.0: raise NotImplementedError("only greedy decoding (temperature 0) is implemented")
     tokens = list(tokens)
     start_pos = self.get_start_pos(tokens)
     self._put_tokens(tokens, start_pos)
-    n_pre = len(tokens) - 1 - start_pos
-    if self.prefill_rows and n_pre >= self.prefill_rows: self.prefill(start_pos, n_pre)
+    n_pre, step = len(tokens) - 1 - start_pos, self.step
+    if self.prefill_rows and n_pre >= self.prefill_rows:
+      self._take_along = len(tokens) < self.max_context and not self._step_args
+      step = self.prefill(start_pos, n_pre) or step
     else:
       for _ in range(n_pre): self.step(with_head=False)
     while len(tokens) < self.max_context:
       if self._step_args:
         self.step(with_head=True)
         tok = self.read_token(len(tokens))
-      else: tok = self._sampled(self.step)[0]
+      else: tok, step = self._sampled(step)[0], self.step
       tokens.append(tok)
       self._cached_tokens = tokens[:-1]
       yield tok
