@@ -1,0 +1,36 @@
+"""The grouped FP8 GEMM's tiles of 64, 128 and 256 columns: a row's results are the same bits whatever the number of rows it comes with."""
+import numpy as np
+import pytest
+from gpu_util import need_gpu
+
+pytestmark = pytest.mark.gpu
+
+
+# rows: one, the most of a narrow tile's short copies and one more, one and two row tiles and a row, as many as make tiles of 128 and 256 columns the shorter way
+@pytest.mark.parametrize("n_in,n_out,dt", [(128, 256, np.float32), (640, 4096, np.float16), (1024, 2304, np.float32)])
+def test_fp8_rows_do_not_depend_on_the_tile(n_in, n_out, dt):
+  need_gpu()
+  from tinygrad_b200.fp8 import FP8Linear
+  from tinygrad_b200.runtime import DeviceBuffer
+  rng = np.random.default_rng(n_in)
+  lin = FP8Linear(n_in, n_out, rng.standard_normal((n_out, n_in)).astype(np.float32), rng.standard_normal(n_out).astype(np.float32))
+  x = rng.standard_normal((2100, n_in)).astype(dt)
+  x[0, 0] = 8                                   # the tensor's largest value is in every subset
+  whole = lin(DeviceBuffer.from_numpy(x)).numpy()
+  ref = x.astype(np.float64) @ lin.weight.numpy().astype(np.float64).T + lin.bias.numpy()
+  assert np.linalg.norm(whole - ref) <= 0.06 * np.linalg.norm(ref)      # two E4M3 roundings of at most 2^-4 each, uniform: 2^-4 / sqrt(3) * sqrt(2) and less
+  for m in (1, 31, 32, 33, 128, 129, 300, 500, 900, 1300):
+    np.testing.assert_array_equal(lin(DeviceBuffer.from_numpy(x[:m].copy())).numpy(), whole[:m], err_msg=str(m))
+
+
+@pytest.mark.parametrize("D,F,E,k", [(256, 128, 3, 2), (512, 384, 16, 4), (768, 1024, 40, 8)])
+def test_expert_layer_rows_do_not_depend_on_the_tile(D, F, E, k):
+  need_gpu()
+  from tinygrad_b200 import moe
+  from tinygrad_b200.runtime import DeviceBuffer
+  rng = np.random.default_rng(E)
+  layer = moe.MxMoE(*((rng.standard_normal(s) * 0.05).astype(np.float32) for s in ((E, F, D), (E, F, D), (E, D, F))), k)
+  x, lg = moe.to_bf16_bits(rng.standard_normal((2500, D)).astype(np.float32)), rng.standard_normal((2500, E)).astype(np.float32)
+  run = lambda T: layer(DeviceBuffer.from_numpy(x[:T].copy()), DeviceBuffer.from_numpy(lg[:T].copy()), T).numpy()
+  whole = run(2500)
+  for T in (1, 31, 32, 33, 128, 129, 400, 1200): np.testing.assert_array_equal(run(T), whole[:T], err_msg=str(T))

@@ -578,9 +578,9 @@ int b200q_moe_layer_chain(const b200q_moe_args* m, const void* x_bf16, const flo
                         m->off, nullptr, m->ends, m->scratch, st, pdl);
   if (rc == B200Q_OK) rc = quantize_launch(x_bf16, B200Q_BF16, n_tokens, m->d, m->dest_row, m->k, m->a_q, m->a_e8, st, true);
   if (rc == B200Q_OK)
-    rc = b200q_mx_gemm_chain(m->a_q, m->a_e8, m->gu_q, m->gu_e8, m->off, m->ends, m->n_experts, rows, 2 * m->f, m->d, nullptr, m->act_q, m->act_e8, st);
+    rc = b200q_mx_gemm_chain(m->a_q, m->a_e8, m->gu_q, m->gu_e8, m->off, m->ends, m->n_experts, rows, 2 * m->f, m->d, nullptr, m->act_q, m->act_e8, n_tokens, m->k, st);
   if (rc == B200Q_OK)
-    rc = b200q_mx_gemm_chain(m->act_q, m->act_e8, m->dn_q, m->dn_e8, m->off, m->ends, m->n_experts, rows, m->d, m->f, m->y, nullptr, nullptr, st);
+    rc = b200q_mx_gemm_chain(m->act_q, m->act_e8, m->dn_q, m->dn_e8, m->off, m->ends, m->n_experts, rows, m->d, m->f, m->y, nullptr, nullptr, n_tokens, m->k, st);
   return rc == B200Q_OK ? combine_launch(m->y, m->dest_row, m->weights, n_tokens, m->k, m->d, m->out, add_to, st, true) : rc;
 }
 extern "C" int b200q_moe_layer(const b200q_moe_args* m, const void* x_bf16, const float* logits, int n_tokens, float* add_to, void* stream) {

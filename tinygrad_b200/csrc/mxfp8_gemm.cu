@@ -4,8 +4,9 @@
 // Semantics: extra/gemm/moe_gemm.py:112-134 over the kernel contract of extra/thunder/amd/grouped_mxfp8_gemm.cpp:32-158
 // (the reference computation it is tested against: dequantised operands matmul, test/backend/test_asm_gemm.py:289-292,306).
 //
-// Persistent, warp-specialised kernel, one CTA per SM, 128 x 256 output tiles, tiles of the used rows (off[E]) dealt round-robin:
-//   warps 4-7  loaders: one thread brings the A (128 x 128 B) and B (256 x 128 B) tiles of a K step into a 3-stage ring by tensor-map copies (K-major, 128-byte
+// Persistent, warp-specialised kernel, one CTA per SM, 128 x 256 output tiles (128 x 128 or x 64 where those are too few for the SMs: tile_columns), tiles of the used
+// rows (off[E]) dealt round-robin:
+//   warps 4-7  loaders: one thread brings the A (128 x 128 B) and B (256 x 128 B) tiles of a K step into a ring of 3 stages by tensor-map copies (K-major, 128-byte
 //              swizzle: 16-byte chunk c of row r sits at chunk c ^ (r & 7)), all of them the step's E8M0 scale words by cp.async (one 32-bit
 //              word = 4 K blocks per row, stored as 32 x 16 B chunks: row r -> chunk r % 32, word r / 32); the copies' bytes and each thread's
 //              words arrive on the stage's "full" mbarrier when they land;
@@ -23,21 +24,23 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <algorithm>
 
 namespace {
 
-#ifndef B200Q_MX_STAGES
-#define B200Q_MX_STAGES 3
-#endif
-constexpr int BM = 128, BN = 256, BK = 128, STAGES = B200Q_MX_STAGES;
+constexpr int BM = 128, BN_MAX = 256, BK = 128, FEW_ROWS = 32;
 constexpr int EPI_WARPS = 4, LOAD_WARPS = 4, EPI_Q = 4;      // epilogue: warps 0-3 and 9-20, EPI_Q warps per 32-lane sub-partition (64 columns each)
 constexpr int THREADS = (EPI_Q * EPI_WARPS + LOAD_WARPS + 1) * 32;
-constexpr int A_BYTES = BM * BK, B_BYTES = BN * BK, SF_BYTES = 2048;                    // scale chunks: A 512 B, B 2 x 512 B
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES + SF_BYTES;                               // 50 KB, a multiple of 1024
 constexpr int EPI_STAGE_BYTES = 16 * 4096;                                              // staging rows of the epilogues that store by tensor-map copies (bf16, FP8 linear): 4 KB per warp
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + EPI_STAGE_BYTES;               // + room to align the ring to 1024 B
 constexpr int TMEM_COLS = 512;            // 256 accumulator columns + scale columns, rounded up to a power of two
-constexpr int SFA_COL = 256, SFB_COL = 256 + 4 * STAGES;   // per stage 4 columns (A: 128 rows) and 8 columns (B: 256 rows)
+// The tile's columns: a ring stage holds 128 rows of A, BN of B and the scale chunks (A 512 B, B 2 x 512 B), a multiple of 1024 bytes: 50, 34 or 26 KB
+template <int BN> struct Geo {
+  static constexpr int STAGES = BN == 256 ? 3 : BN == 128 ? 4 : 5;
+  static constexpr int A_BYTES = BM * BK, B_BYTES = BN * BK, SF_BYTES = 2048, STAGE_BYTES = A_BYTES + B_BYTES + SF_BYTES;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + EPI_STAGE_BYTES;        // + room to align the ring to 1024 B
+  static_assert(SMEM_BYTES + 9 * 1024 <= 227 * 1024, "with the tables of groups");
+  static constexpr int SFA_COL = 256, SFB_COL = 256 + 4 * STAGES;   // tensor-memory columns, per stage 4 (A: 128 rows) and 8 (B: 256 rows)
+};
 constexpr int MAX_EXPERTS = 1024;
 constexpr int SPIN = 1 << 22;
 
@@ -110,20 +113,46 @@ __device__ __forceinline__ void swiglu_quant_store(const uint32_t (&vg)[32], con
   act_e8[row * (f >> 5) + (col >> 5)] = e;
 }
 
+// The same for the first `rows` rows of a narrow tile with few: the warp's accumulators (a row per lane, 32 gate and 32 up columns) change places in shared memory, then a
+// row's block is a value per lane.  With a row per lane and everything unrolled, one token's tiles were mostly the time to fetch 3000 instructions.
+__device__ __forceinline__ void swiglu_quant_few(const uint32_t (&vg)[32], const uint32_t (&vu)[32], float* s, uint8_t* act_q, uint8_t* act_e8, size_t row0, int rows, int f, int col) {
+  const int lane = threadIdx.x & 31;
+  constexpr int STRIDE = 65;
+  if (lane < rows) {
+#pragma unroll
+    for (int j = 0; j < 32; j++) { s[lane * STRIDE + j] = __uint_as_float(vg[j]); s[lane * STRIDE + 32 + j] = __uint_as_float(vu[j]); }
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (int r = 0; r < rows; r++) {
+    const float g = __bfloat162float(__float2bfloat16_rn(s[r * STRIDE + lane])), u = __bfloat162float(__float2bfloat16_rn(s[r * STRIDE + 32 + lane]));
+    const float v = __bfloat162float(__float2bfloat16_rn((g / (1.f + expf(-g))) * u));
+    const uint8_t e = mx_scale_exponent(warp_max(fabsf(v)));
+    act_q[(row0 + r) * f + col + lane] = __nv_cvt_float_to_fp8(fminf(fmaxf(v * mx_inv_scale(e), -448.f), 448.f), __NV_SATFINITE, __NV_E4M3);
+    if (lane == 0) act_e8[(row0 + r) * (f >> 5) + (col >> 5)] = e;
+  }
+  __syncwarp();
+}
+
 // fp32 results with the per-tensor FP8 linear's last steps: y = acc * *fw * *fx + bias in y's type, for the first `rows` rows (fw NULL: plain sums)
 struct ScaledOut { const float *fw, *fx, *bias; int rows, y_f16; };
 
 // What becomes of the sums: bf16 rows, SwiGLU of gate and up requantised, the FP8 linear's results, fp32 sums.  One kernel each: the registers of one epilogue are not
 // another's, and an expert layer of few rows does not fetch the instructions of all four.
 enum { OUT_BF16, OUT_SWIGLU, OUT_SCALED, OUT_F32 };
-template <int OUT>
+// UNIT: every block scale is one (the FP8 linear): they are put into tensor memory once, not brought in with every K step.
+// a_rows (BN 64): rows of A that a tile's copies bring, 128 or FEW_ROWS (then every group has at most that many, and the other lanes' results are dropped).
+template <int OUT, int BN>
 __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint8_t* __restrict__ a_q, const uint8_t* __restrict__ a_e8,
                                                                       const uint8_t* __restrict__ b_q, const uint8_t* __restrict__ b_e8,
                                                                       const int32_t* __restrict__ off, int n_experts, int m_total, int n, int k,
                                                                       __nv_bfloat16* __restrict__ c, uint8_t* __restrict__ act_q,
                                                                       uint8_t* __restrict__ act_e8, const __grid_constant__ CUtensorMap tm_a,
                                                                       const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_c,
-                                                                      const ScaledOut so, const int32_t* __restrict__ ends) {
+                                                                      const ScaledOut so, const int32_t* __restrict__ ends, int a_rows) {
+  using G = Geo<BN>;
+  constexpr int STAGES = G::STAGES, A_BYTES = G::A_BYTES, B_BYTES = G::B_BYTES, STAGE_BYTES = G::STAGE_BYTES, SFA_COL = G::SFA_COL, SFB_COL = G::SFB_COL;
+  constexpr bool UNIT = OUT == OUT_SCALED, PAIRED = OUT == OUT_SWIGLU && BN < 256;      // PAIRED: half the tile's rows of B are gate rows, the other half lies 128 rows on
   extern __shared__ unsigned char sm_raw[];
   __shared__ __align__(8) uint64_t bar_full[STAGES], bar_empty[STAGES], bar_acc_full, bar_acc_empty, bar_drain;
   __shared__ uint32_t tmem_base;
@@ -132,7 +161,7 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     for (int s = 0; s < STAGES; s++) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(s32(&bar_full[s])), "r"(LOAD_WARPS * 32 + 1));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(s32(&bar_full[s])), "r"(UNIT ? 1 : LOAD_WARPS * 32 + 1));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(s32(&bar_empty[s])));
     }
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(s32(&bar_acc_full)));
@@ -140,6 +169,10 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(s32(&bar_drain)));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     s_abort = 0;
+  }
+  if (tid == EPI_WARPS * 32) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_a) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&tm_b) : "memory");
   }
   if (warp == EPI_WARPS + LOAD_WARPS) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(&tmem_base)), "r"(TMEM_COLS) : "memory");
@@ -172,6 +205,17 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   pdl_launch_dependents();
   const uint32_t taddr = tmem_base;
+  if constexpr (UNIT) {
+    if (warp < 4) {      // E8M0 127 = 2^0 in all twelve columns, a warp per sub-partition
+      const uint32_t one = 0x7F7F7F7Fu, at = taddr + ((uint32_t)(warp * 32) << 16);
+      asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %1, %1, %1};" ::"r"(at + SFA_COL), "r"(one) : "memory");
+      asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(at + SFB_COL), "r"(one) : "memory");
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    }
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  }
   volatile int* abort_flag = &s_abort;
   const int kb_total = k >> 5, ktiles = k / BK;
   const int tiles_n = n / BN, n_tiles = s_tile[n_experts] * tiles_n;
@@ -189,10 +233,11 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
     int b_row0 = 0, a_row0 = 0;      // first rows of the tile's operands: B inside [n_experts * n, k], A inside [m_total, k]
     auto tile_ptrs = [&](int t, const uint8_t*& ae, const uint8_t*& be) {
       const int mt = t / tiles_n, n0 = (t % tiles_n) * BN, lo = group_of(mt), m0 = s_off[lo] + (mt - s_tile[lo]) * BM;
+      b_row0 = lo * n + (PAIRED ? (n0 >> 8) * 256 + ((n0 >> 1) & 127) : n0); a_row0 = m0;
       ae = a_e8 + (size_t)(m0 + lt) * kb_total;
-      be = b_e8 + ((size_t)lo * n + n0 + lt) * kb_total;
-      b_row0 = lo * n + n0; a_row0 = m0;
+      be = b_e8 + ((size_t)b_row0 + (PAIRED && lt >= BN / 2 ? 128 - BN / 2 : 0) + lt) * kb_total;
     };
+    const uint32_t step_bytes = BN == 64 ? (uint32_t)a_rows * BK + B_BYTES : A_BYTES + B_BYTES;
     uint32_t g = 0;
     bool ok = true;
 #pragma unroll 1
@@ -208,16 +253,21 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
         if (warp == EPI_WARPS && elect_one()) {
           // the 128-byte-swizzle tiled copy writes exactly the layout above (chunk c of row r at c ^ (r & 7)); no multicast
           const uint32_t fb = s32(&bar_full[slot]);
-          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb), "r"(A_BYTES + B_BYTES) : "memory");
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb), "r"(step_bytes) : "memory");
           asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                        ::"r"(sA), "l"(&tm_a), "r"(kt * BK), "r"(a_row0), "r"(fb) : "memory");
           asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                        ::"r"(sB), "l"(&tm_b), "r"(kt * BK), "r"(b_row0), "r"(fb) : "memory");
+          if (PAIRED)
+            asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                         ::"r"(sB + B_BYTES / 2), "l"(&tm_b), "r"(kt * BK), "r"(b_row0 + 128), "r"(fb) : "memory");
         }
-        cp4(sF + sf_off, ae + kt * 4);
-        cp4(sF + 512 + sf_off, be + kt * 4);
-        cp4(sF + 1024 + sf_off, be + (size_t)128 * kb_total + kt * 4);
-        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(s32(&bar_full[slot])) : "memory");
+        if constexpr (!UNIT) {
+          cp4(sF + sf_off, ae + kt * 4);
+          if (BN >= 128 || lt < BN) cp4(sF + 512 + sf_off, be + kt * 4);
+          if (BN == 256) cp4(sF + 1024 + sf_off, be + (size_t)128 * kb_total + kt * 4);
+          asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(s32(&bar_full[slot])) : "memory");
+        }
       }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
@@ -249,9 +299,13 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           const uint32_t sA = ring + slot * STAGE_BYTES, sB = sA + A_BYTES, sF = sB + B_BYTES;
           // scale chunks -> tensor memory (32 lanes x 16 B, replicated into the four sub-partitions); ordered before the MMAs below
-          asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr + SFA_COL + slot * 4), "l"(desc_plain(sF, 128, 128)) : "memory");
-          asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr + SFB_COL + slot * 8), "l"(desc_plain(sF + 512, 128, 128)) : "memory");
-          asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr + SFB_COL + slot * 8 + 4), "l"(desc_plain(sF + 1024, 128, 128)) : "memory");
+          if constexpr (!UNIT) {
+            asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr + SFA_COL + slot * 4), "l"(desc_plain(sF, 128, 128)) : "memory");
+            asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr + SFB_COL + slot * 8), "l"(desc_plain(sF + 512, 128, 128)) : "memory");
+            if (BN == 256)
+              asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr + SFB_COL + slot * 8 + 4), "l"(desc_plain(sF + 1024, 128, 128)) : "memory");
+          }
+          const uint32_t sf_slot = UNIT ? 0 : slot;
 #pragma unroll
           for (int kb = 0; kb < 4; kb++) {
             const uint64_t da = desc_sw128(sA + kb * 32), db = desc_sw128(sB + kb * 32);
@@ -260,7 +314,7 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
             const uint32_t acc = (kt > 0 || kb > 0) ? 1u : 0u;
             asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %6, 0;\n"
                          "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale.scale_vec::1X [%0], %1, %2, %3, [%4], [%5], p;\n}"
-                         ::"r"(taddr), "l"(da), "l"(db), "r"(idesc), "r"(taddr + SFA_COL + slot * 4), "r"(taddr + SFB_COL + slot * 8), "r"(acc) : "memory");
+                         ::"r"(taddr), "l"(da), "l"(db), "r"(idesc), "r"(taddr + SFA_COL + sf_slot * 4), "r"(taddr + SFB_COL + sf_slot * 8), "r"(acc) : "memory");
           }
           asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s32(&bar_empty[slot])) : "memory");
         }
@@ -291,9 +345,15 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
     };
 #pragma unroll 1
     for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, tile_i++) {
+      const int mt = t / tiles_n, n0 = (t % tiles_n) * BN, grp = group_of(mt), m0 = s_off[grp] + (mt - s_tile[grp]) * BM;
+      int few = 0;                      // rows of a tile of FEW_ROWS
+      if constexpr (OUT == OUT_SWIGLU && BN == 64) if (a_rows == FEW_ROWS) few = min(min(ends ? ends[grp] : off[grp + 1], m_total) - m0, FEW_ROWS);
       if (!wait_bar(s32(&bar_acc_full), tile_i & 1, abort_flag)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int mt = t / tiles_n, n0 = (t % tiles_n) * BN, grp = group_of(mt), m0 = s_off[grp] + (mt - s_tile[grp]) * BM;
+      if (BN < 256 && (cq * (OUT == OUT_SWIGLU ? 32 : 64) >= (OUT == OUT_SWIGLU ? BN / 2 : BN) || (BN == 64 && sub * 32 >= a_rows))) {      // no columns or no rows for this warp
+        release();
+        continue;
+      }
       const uint32_t ta = taddr + ((uint32_t)(sub * 32) << 16);
       const size_t row = (size_t)(m0 + sub * 32 + lane);
       uint32_t v0[32], v1[32];
@@ -305,7 +365,8 @@ __global__ void __launch_bounds__(THREADS, 1) grouped_mxfp8_tc_kernel(const uint
         tmem_ld32(ta + cq * 32, v0); tmem_ld32(ta + BN / 2 + cq * 32, v1);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         release();
-        swiglu_quant_store(v0, v1, act_q, act_e8, row, n >> 1, (n0 >> 1) + cq * 32);
+        if (BN == 64 && few) swiglu_quant_few(v0, v1, reinterpret_cast<float*>(sm_raw + (ring - s32(sm_raw)) + STAGES * STAGE_BYTES), act_q, act_e8, (size_t)m0, few, n >> 1, n0 >> 1);
+        else swiglu_quant_store(v0, v1, act_q, act_e8, row, n >> 1, (n0 >> 1) + cq * 32);
       } else {
         tmem_ld32(ta + cq * 64, v0); tmem_ld32(ta + cq * 64 + 32, v1);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -421,49 +482,77 @@ static int make_map(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t k
   return r == CUDA_SUCCESS ? B200Q_OK : B200Q_ERR_BAD_ARG;
 }
 
+// How wide a tile: the one whose waves over the SMs, each as long as the operand bytes of a K step, take the least; the widest among equals.  FP8 Linear 4096 x 4096, us a call
+// with tiles of 256 columns and so: 1 row 33.3 / 20.3, 300 rows 37.5 / 23.1, 2000 rows 74.1 / 56.2 (there the width is the same, and all of the gain, as 2 to 6 us of the
+// others, is the block scales that need not be brought in); 6144 -> 1024, 500 rows 59.4 / 42.1.  Expert layer 2048 x 1024, 64 experts top 8, one token 41.9 / 36.9.
+static int tile_columns(int row_tiles, int n, int n_sm) {
+  int best = 0;
+  long long least = 0;
+  for (int bn : {256, 128, 64}) {
+    const long long tiles = (long long)row_tiles * (n / bn), t = (tiles + n_sm - 1) / n_sm * (BM + bn);
+    if (!best || t < least) { best = bn; least = t; }
+  }
+  return best;
+}
+typedef decltype(&grouped_mxfp8_tc_kernel<OUT_BF16, 256>) GroupedKernel;
+template <int BN> static GroupedKernel pick_out(int out) {
+  return out == OUT_SWIGLU ? grouped_mxfp8_tc_kernel<OUT_SWIGLU, BN> : out == OUT_SCALED ? grouped_mxfp8_tc_kernel<OUT_SCALED, BN>
+         : out == OUT_F32 ? grouped_mxfp8_tc_kernel<OUT_F32, BN> : grouped_mxfp8_tc_kernel<OUT_BF16, BN>;
+}
+static GroupedKernel pick_kernel(int out, int bn) { return bn == 256 ? pick_out<256>(out) : bn == 128 ? pick_out<128>(out) : pick_out<64>(out); }
+
+// row_tiles: about how many tiles of 128 rows there are (0: all of m_total); few_rows: no group has more than FEW_ROWS.
 static int grouped_launch(const void* a_q, const void* a_e8, const void* b_q, const void* b_e8, const int32_t* off, int n_experts, int m_total, int n, int k,
-                          void* c_bf16, void* act_q, void* act_e8, void* stream, bool c_f32 = false, ScaledOut so = ScaledOut{}, bool pdl = false, const int32_t* ends = nullptr) {
+                          void* c_bf16, void* act_q, void* act_e8, void* stream, bool c_f32 = false, ScaledOut so = ScaledOut{}, bool pdl = false, const int32_t* ends = nullptr,
+                          int row_tiles = 0, bool few_rows = false) {
   if (!a_q || !a_e8 || !b_q || !b_e8 || !off || (!c_bf16 && !act_q) || n_experts <= 0 || m_total <= 0 || n <= 0 || k <= 0) return B200Q_ERR_BAD_ARG;
   if (act_q && (!act_e8 || (((uintptr_t)act_q) & 15))) return B200Q_ERR_BAD_ARG;
-  if (m_total % 256 || n % BN || k % BK) return B200Q_ERR_BAD_SHAPE;       // the reference asks M % 256 == N % 256 == K % 128 == 0 (moe_gemm.py:120)
+  if (m_total % 256 || n % BN_MAX || k % BK) return B200Q_ERR_BAD_SHAPE;       // the reference asks M % 256 == N % 256 == K % 128 == 0 (moe_gemm.py:120)
   if (n_experts > MAX_EXPERTS) return B200Q_ERR_UNSUPPORTED;
   if (((uintptr_t)a_q | (uintptr_t)b_q | (uintptr_t)c_bf16) & 15 || ((uintptr_t)a_e8 | (uintptr_t)b_e8) & 3) return B200Q_ERR_MISALIGNED;
   const int out = act_q ? OUT_SWIGLU : so.fw ? OUT_SCALED : c_f32 ? OUT_F32 : OUT_BF16;
-  auto kernel = out == OUT_SWIGLU ? grouped_mxfp8_tc_kernel<OUT_SWIGLU> : out == OUT_SCALED ? grouped_mxfp8_tc_kernel<OUT_SCALED>
-                : out == OUT_F32 ? grouped_mxfp8_tc_kernel<OUT_F32> : grouped_mxfp8_tc_kernel<OUT_BF16>;
-  static PerDeviceFlag attr_set[4];
   const int dev = b200q_current_device(), n_sm = b200q_sm_count();
   if (dev < 0 || n_sm <= 0) return B200Q_ERR_CUDA;
-  if (!attr_set[out].test(dev)) {
-    B200Q_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-    attr_set[out].set(dev);
+  if (row_tiles <= 0 || row_tiles > m_total / BM) row_tiles = m_total / BM;
+  const int bn = tile_columns(row_tiles, n, n_sm);
+  auto kernel = pick_kernel(out, bn);
+  const int smem = bn == 256 ? Geo<256>::SMEM_BYTES : bn == 128 ? Geo<128>::SMEM_BYTES : Geo<64>::SMEM_BYTES;
+  static PerDeviceFlag attr_set[4][3];
+  PerDeviceFlag& flag = attr_set[out][bn == 256 ? 0 : bn == 128 ? 1 : 2];
+  if (!flag.test(dev)) {
+    B200Q_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    flag.set(dev);
   }
-  const long long tiles = (long long)(m_total / BM) * (n / BN);
-  const int grid = (int)(tiles < n_sm ? tiles : n_sm);
+  const long long tiles = (long long)(m_total / BM) * (n / bn);
+  const int grid = (int)(tiles < n_sm ? tiles : n_sm), a_rows = few_rows && bn == 64 ? FEW_ROWS : BM;
   alignas(64) CUtensorMap tm_a, tm_b, tm_c;
   memset(&tm_a, 0, sizeof(tm_a)); memset(&tm_b, 0, sizeof(tm_b)); memset(&tm_c, 0, sizeof(tm_c));
   int rc = B200Q_OK;
   if (out == OUT_SCALED) rc = so.y_f16 ? make_map(&tm_c, c_bf16, (uint64_t)so.rows, (uint64_t)n, 32, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2)
                            : make_map(&tm_c, c_bf16, (uint64_t)so.rows, (uint64_t)n, 32, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4);
   else if (out == OUT_BF16) rc = make_map(&tm_c, c_bf16, (uint64_t)m_total, (uint64_t)n, 32, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2);
-  if (rc == B200Q_OK) rc = make_map(&tm_a, a_q, (uint64_t)m_total, (uint64_t)k, BM);
-  if (rc == B200Q_OK) rc = make_map(&tm_b, b_q, (uint64_t)n_experts * n, (uint64_t)k, BN);
+  if (rc == B200Q_OK) rc = make_map(&tm_a, a_q, (uint64_t)m_total, (uint64_t)k, a_rows);
+  if (rc == B200Q_OK) rc = make_map(&tm_b, b_q, (uint64_t)n_experts * n, (uint64_t)k, out == OUT_SWIGLU && bn < 256 ? bn / 2 : bn);
   if (rc != B200Q_OK) return rc;
-  B200Q_CHECK_CUDA(launch_k(kernel, dim3(grid), dim3(THREADS), (size_t)SMEM_BYTES, (cudaStream_t)stream, pdl, (const uint8_t*)a_q, (const uint8_t*)a_e8,
+  B200Q_CHECK_CUDA(launch_k(kernel, dim3(grid), dim3(THREADS), (size_t)smem, (cudaStream_t)stream, pdl, (const uint8_t*)a_q, (const uint8_t*)a_e8,
                             (const uint8_t*)b_q, (const uint8_t*)b_e8, off, n_experts, m_total, n, k, (__nv_bfloat16*)c_bf16, (uint8_t*)act_q, (uint8_t*)act_e8,
-                            tm_a, tm_b, tm_c, so, ends));
+                            tm_a, tm_b, tm_c, so, ends, a_rows));
   return B200Q_OK;
 }
 
 int b200q_mx_gemm_scaled(const void* a_q, const void* a_e8, const void* b_q, const void* b_e8, const int32_t* off, int m_total, int n, int k, void* y, int y_dtype,
                          int rows, const float* fw, const float* fx, const float* bias, cudaStream_t st) {
-  return grouped_launch(a_q, a_e8, b_q, b_e8, off, 1, m_total, n, k, y, nullptr, nullptr, st, true, ScaledOut{fw, fx, bias, rows, y_dtype == B200Q_F16}, true);
+  return grouped_launch(a_q, a_e8, b_q, b_e8, off, 1, m_total, n, k, y, nullptr, nullptr, st, true, ScaledOut{fw, fx, bias, rows, y_dtype == B200Q_F16}, true, nullptr,
+                        (rows + BM - 1) / BM, rows <= FEW_ROWS);
 }
 
 // the expert layer's GEMMs (c_bf16: plain rows, else SwiGLU + requantise into act_q / act_e8), programmatic behind this library's kernels
+// n_tokens x topk rows: an expert has a token once at most
 int b200q_mx_gemm_chain(const void* a_q, const void* a_e8, const void* b_q, const void* b_e8, const int32_t* off, const int32_t* ends, int n_experts, int m_total, int n,
-                        int k, void* c_bf16, void* act_q, void* act_e8, cudaStream_t st) {
-  return grouped_launch(a_q, a_e8, b_q, b_e8, off, n_experts, m_total, n, k, c_bf16, act_q, act_e8, st, false, ScaledOut{}, true, ends);
+                        int k, void* c_bf16, void* act_q, void* act_e8, int n_tokens, int topk, cudaStream_t st) {
+  const long long pairs = (long long)n_tokens * topk, tiles = n_tokens <= BM ? std::min<long long>(n_experts, pairs) : (pairs + BM - 1) / BM + n_experts / 2;
+  return grouped_launch(a_q, a_e8, b_q, b_e8, off, n_experts, m_total, n, k, c_bf16, act_q, act_e8, st, false, ScaledOut{}, true, ends,
+                        (int)std::min<long long>(tiles, m_total / BM), n_tokens <= FEW_ROWS);
 }
 
 extern "C" int b200q_grouped_mxfp8_gemm(const void* a_q, const void* a_e8, const void* b_q, const void* b_e8, const int32_t* off, int n_experts,
