@@ -16,9 +16,11 @@ void b200q_set_cuda_error(cudaError_t e);
 
 // ---- launch chains.  Exported entry points launch their first kernel fully ordered behind whatever the caller has put on the stream; the `pdl`
 // argument of the internal forms below is for calls whose predecessor on the stream is known to be a kernel of this library.
+// one row of a GEMM that is not split, with what is in front of it: x += the weighted sum of the k rows dest_row of y (bf16; NULL: nothing), RMSNorm (norm_w NULL: none)
+struct b200q_row_input { float* x; const void* y; const int32_t* dest_row; const float* weights; int k; const void* norm_w; float eps; };
 int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtype, const void* norm_weight, float norm_eps, const void* bias_f16, const void* residual,
                       int epilogue, void* y, int y_dtype, int m, int n_out, int n_in, void* workspace, size_t workspace_bytes, cudaStream_t st, bool pdl,
-                      bool unsplit = false);
+                      bool unsplit = false, const b200q_row_input* one = nullptr);
 // out NULL: RoPE and the cache rows only
 int b200q_attn_rows_chain(const float* qkv, void* k_cache, void* v_cache, int kv_dtype, const float* rope, int start_pos, int n_rows, int n_seqs, int n_heads,
                           int n_kv_heads, int head_dim, int rope_dim, int max_context, void* q_scratch, void* out, int out_dtype, cudaStream_t st, bool pdl);
@@ -51,6 +53,12 @@ int b200q_attn_rows_pos_chain(const float* qkv, void* k_cache, void* v_cache, in
 // one row times a packed matrix in fp32 (row_gemv.cu)
 int b200q_row_gemv_chain(int qtype, const void* w_packed, const float* x, const void* norm_weight, float norm_eps, const void* bias_f16, const float* residual, int epilogue,
                          float* y, int n_out, int n_in, cudaStream_t st, bool pdl);
+// behind the expert GEMMs: the weighted sums, added to add_to (mxfp8.cu)
+int b200q_moe_combine_chain(const b200q_moe_args* m, int n_tokens, float* add_to, cudaStream_t st);
+int b200q_moe_gemms_chain(const b200q_moe_args* m, int n_tokens, cudaStream_t st);
+// one token: RMSNorm, router, choice and tables, quantised rows (moe_step.cu); xn (may be NULL): the normed row
+bool b200q_moe_router_one_takes(const b200q_moe_args* m, int router_dtype);
+int b200q_moe_router_one(const b200q_moe_args* m, const void* router, int router_dtype, const float* x, const void* norm_weight, float eps, float* xn, cudaStream_t st);
 int b200q_decode_status_take(int* status);
 int b200q_decode_step_status_take(int* status);   // the same for the whole-step kernel (decode_step.cu)
 int b200q_peer_status_take(int* status);          // the same for the peer-memory collectives (peer.cu)

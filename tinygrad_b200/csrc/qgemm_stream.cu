@@ -25,6 +25,7 @@
 // Every mbarrier wait is bounded: on expiry a status word is set, all roles leave, copies and MMAs in flight are drained.
 #include "common.cuh"
 #include "tc_common.cuh"
+#include <cuda_bf16.h>
 #include <algorithm>
 #include <cstddef>
 
@@ -587,6 +588,93 @@ __global__ void __launch_bounds__(THREADS, 1) qgemm_stream_kernel(const StreamPa
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(sh.tmem), "r"(WT == 256 ? 512 : 256) : "memory");
 }
 
+// ---- one fp32 row -----------------------------------------------------------------------------------------------------------------
+// What stands between two GEMMs of a one-token step of a mixture-of-experts model, in one CTA: the weighted sum of the experts' outputs and its residual add (in.y), the
+// RMSNorm, and the split halves of the row (the other rows of its tile are columns of the product that nobody reads).  Values and their order are those of
+// combine8_kernel, rmsnorm_rows_kernel and split_rows_kernel, bit for bit: an expert's choice and its E4M3 codes turn a last-bit difference into a visible one.
+constexpr int ROW_THREADS = 256;
+__global__ void __launch_bounds__(ROW_THREADS) prepare_row_kernel(const b200q_row_input in, int n_in, int kgroups, int nt, unsigned char* __restrict__ xt, float* __restrict__ down) {
+  extern __shared__ __align__(16) float row_s[];
+  __shared__ float red[ROW_THREADS / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  pdl_launch_dependents();
+  pdl_wait();
+  for (int c = tid * 8; c < n_in; c += ROW_THREADS * 8) {
+    float f[8];
+    load_chunk(in.x, c, f);
+    if (in.y) {
+      const __nv_bfloat16* y = reinterpret_cast<const __nv_bfloat16*>(in.y);
+      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      for (int j0 = 0; j0 < in.k; j0 += 4) {
+        uint4 u[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) if (j0 + j < in.k) u[j] = *reinterpret_cast<const uint4*>(y + (size_t)in.dest_row[j0 + j] * n_in + c);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          if (j0 + j < in.k) {
+            const float w = in.weights[j0 + j];
+            const uint32_t b[4] = {u[j].x, u[j].y, u[j].z, u[j].w};
+#pragma unroll
+            for (int i = 0; i < 4; i++) { acc[2 * i] += w * __uint_as_float(b[i] << 16); acc[2 * i + 1] += w * __uint_as_float(b[i] & 0xFFFF0000u); }
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 8; i++) f[i] += __bfloat162float(__float2bfloat16_rn(acc[i]));
+      *reinterpret_cast<float4*>(in.x + c) = make_float4(f[0], f[1], f[2], f[3]);
+      *reinterpret_cast<float4*>(in.x + c + 4) = make_float4(f[4], f[5], f[6], f[7]);
+    }
+    *reinterpret_cast<float4*>(row_s + c) = make_float4(f[0], f[1], f[2], f[3]);
+    *reinterpret_cast<float4*>(row_s + c + 4) = make_float4(f[4], f[5], f[6], f[7]);
+  }
+  __syncthreads();
+  float sc = 1.f;
+  if (in.norm_w) {
+    float ss = 0.f;
+    for (int i = tid; i < n_in; i += ROW_THREADS) { const float v = row_s[i]; ss += v * v; }
+    ss = warp_sum(ss);
+    if (lane == 0) red[warp] = ss;
+    __syncthreads();
+    float tot = 0.f;
+    for (int i = 0; i < ROW_THREADS / 32; i++) tot += red[i];
+    sc = 1.0f / sqrtf(tot / (float)n_in + in.eps);
+    __syncthreads();
+  }
+  const __half* nw = reinterpret_cast<const __half*>(in.norm_w);
+  auto value = [&](int c, float (&f)[8]) {
+#pragma unroll
+    for (int q = 0; q < 8; q++) f[q] = c + q < n_in ? (nw ? row_s[c + q] * sc * __half2float(nw[c + q]) : row_s[c + q]) : 0.f;
+  };
+  float amax = 0.f;
+  for (int c = tid * 8; c < n_in; c += ROW_THREADS * 8) {
+    float f[8];
+    value(c, f);
+#pragma unroll
+    for (int q = 0; q < 8; q++) amax = fmaxf(amax, fabsf(f[q]));
+  }
+  amax = warp_max(amax);
+  if (lane == 0) red[warp] = amax;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < ROW_THREADS / 32; i++) amax = fmaxf(amax, red[i]);
+  float up = 1.f, inv = 1.f;
+  if (down) {
+    if (!(amax < 32768.f)) pow2_scale(amax, up, inv);
+    if (tid == 0) down[0] = inv;
+  }
+  const size_t row_bytes = (size_t)nt * 32;
+  for (int c = tid; c < kgroups * 16; c += ROW_THREADS) {
+    float f[8];
+    uint4 hi, lo;
+    value(c * 8, f);
+#pragma unroll
+    for (int q = 0; q < 8; q++) f[q] *= up;
+    split_chunk(f, hi, lo);
+    *reinterpret_cast<uint4*>(xt + (size_t)c * row_bytes) = hi;
+    *reinterpret_cast<uint4*>(xt + (size_t)c * row_bytes + (size_t)nt * 16) = lo;
+  }
+}
+
 // ---- launch --------------------------------------------------------------------------------------------------------------------
 struct Plan { int nt, tok_tiles, wt; };
 Plan make_plan(int m, int n_out, int n_sm) {
@@ -699,7 +787,8 @@ extern "C" size_t b200q_qgemm_workspace_bytes_for(int m, int n_out, int n_in) {
 
 // norm_weight (fp16 [n_in], fp32 activations only): the RMSNorm in front of the Linear, applied while the rows are split.
 int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtype, const void* norm_weight, float norm_eps, const void* bias_f16, const void* residual,
-                      int epilogue, void* y, int y_dtype, int m, int n_out, int n_in, void* workspace, size_t workspace_bytes, cudaStream_t st, bool pdl, bool unsplit) {
+                      int epilogue, void* y, int y_dtype, int m, int n_out, int n_in, void* workspace, size_t workspace_bytes, cudaStream_t st, bool pdl, bool unsplit,
+                      const b200q_row_input* row) {
   if (!w_packed || !x || !y || !workspace || m <= 0 || n_out <= 0 || n_in <= 0) return B200Q_ERR_BAD_ARG;
   if (epilogue != B200Q_EPI_LINEAR && epilogue != B200Q_EPI_SILU_MUL) return B200Q_ERR_BAD_ARG;
   if (epilogue == B200Q_EPI_SILU_MUL && (bias_f16 || residual || n_out % 16)) return B200Q_ERR_BAD_ARG;
@@ -755,7 +844,12 @@ int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtyp
   attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = sgrid.y; attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr; cfg.numAttrs = cluster ? 2 : 1;
   const int n_counters = split ? grid : 0;
-  if (f32)
+  if (row) {
+    if (m != 1 || !f32 || split || n_in % 8 || norm_weight) return B200Q_ERR_BAD_ARG;
+    const size_t smem = (size_t)n_in * sizeof(float);
+    if (smem > 48 * 1024) return B200Q_ERR_TOO_LARGE;
+    B200Q_CHECK_CUDA(launch_k(prepare_row_kernel, dim3(1), dim3(ROW_THREADS), smem, st, pdl, *row, n_in, kgroups, pl.nt, (unsigned char*)p.xt, (float*)p.down));
+  } else if (f32)
     B200Q_CHECK_CUDA(cudaLaunchKernelEx(&cfg, cluster ? split_rows_kernel<float, true> : split_rows_kernel<float, false>, (const float*)x, (const __half*)norm_weight, norm_eps, m,
                                         n_in, kgroups, pl.nt, per, (unsigned char*)p.xt, p.counters, n_counters, (float*)p.down, unsplit ? 0.f : 1.f));
   else
