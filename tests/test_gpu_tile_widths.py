@@ -34,3 +34,28 @@ def test_expert_layer_rows_do_not_depend_on_the_tile(D, F, E, k):
   run = lambda T: layer(DeviceBuffer.from_numpy(x[:T].copy()), DeviceBuffer.from_numpy(lg[:T].copy()), T).numpy()
   whole = run(2500)
   for T in (1, 31, 32, 33, 128, 129, 400, 1200): np.testing.assert_array_equal(run(T), whole[:T], err_msg=str(T))
+
+
+# one thread's piece, all of one CTA and a value more, the smallest and largest of one launch, and one past it; what is left of a thread's pieces; both kinds of rows
+@pytest.mark.parametrize("rows,n_in,dt", [(1, 128, np.float32), (8, 1024, np.float16), (65, 128, np.float32), (4096, 256, np.float16), (1025, 1024, np.float32),
+                                         (148 * 32, 1024, np.float32), (148 * 32 + 1, 1024, np.float16)])
+def test_fp8_codes_in_one_launch(rows, n_in, dt):
+  """Codes and factor of a call's activations are those of the separate entry points, the largest magnitude wherever it is."""
+  need_gpu()
+  from tinygrad_b200 import fp8, _lib
+  from tinygrad_b200.runtime import DeviceBuffer
+  rng = np.random.default_rng(rows)
+  lin = fp8.FP8Linear(n_in, 256, rng.standard_normal((256, n_in)).astype(np.float32))
+  for at in (0, rows * n_in // 2, rows * n_in - 1):
+    x = rng.standard_normal((rows, n_in)).astype(dt)
+    x.reshape(-1)[at] = -9.5
+    d = DeviceBuffer.from_numpy(x)
+    lin(d)
+    q, f = fp8.quantize_to_fp8(d, x.size, _lib.F16 if dt == np.float16 else _lib.F32)
+    w = lin._workspace(rows)
+    got = DeviceBuffer.empty((rows, n_in), np.uint8)
+    _lib.check(_lib.load().b200q_memcpy_d2d(got.ptr, w.x_q, rows * n_in, None))
+    np.testing.assert_array_equal(got.numpy().reshape(-1), q.numpy().reshape(-1))
+    factor = DeviceBuffer.empty((1,), np.float32)
+    _lib.check(_lib.load().b200q_memcpy_d2d(factor.ptr, w.factor, 4, None))
+    assert factor.numpy()[0] == f.numpy()[0]
