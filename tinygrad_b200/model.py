@@ -276,7 +276,7 @@ class Transformer:
     self._graphs = {}
     self._cached_tokens: list = []
     self.prefill_rows = prefill_rows if (tp is None and not self.dense_blocks and c.hidden_dim % 8 == 0 and c.head_dim in (16, 32, 64, 128)) else 0
-    self.prefill_chunk, self._pf, self._batch_logits, self._rows_ws, self._batch_graph = max(1, prefill_chunk), None, None, None, None
+    self.prefill_chunk, self._pf, self._batch_logits, self._rows_ws = max(1, prefill_chunk), None, None, None
     self._rows_args, self._moe_blocks = None, {}
     self._seq_attn_scratch = self._last_rows = None
     self.is_moe, self._host_pos, self._rows_warm = c.num_experts > 0, 0, False
@@ -449,16 +449,21 @@ class Transformer:
       check(_lib.load().b200q_prompt_rows_kv(native, seq, 1, p0, rows, self.stream.ptr))
     return rows
 
-  def _last_block(self, enqueue) -> None:
-    """Replays the last block, the head and the arg-max on rows that a prompt pass has left (captured on first use)."""
-    self._head_queued = True
-    if not self.use_graph: return enqueue()
-    g = self._graphs.get("last_block")
+  def _captured(self, key, enqueue) -> Graph:
+    g = self._graphs.get(key)
     if g is None:
       g = Graph(self.stream)
       with g: enqueue()
-      self._graphs["last_block"] = g
-    g.launch()
+      self._graphs[key] = g
+    return g
+
+  def _last_block(self, enqueue, step) -> None:
+    """Replays the last block, the head and the arg-max on rows that a prompt pass has left (captured on first use).  The steps that will follow, `step`, are captured here
+    too: the device still has the prompt to do."""
+    self._head_queued = True
+    if not self.use_graph: return enqueue()
+    self._captured("last_block", enqueue).launch()
+    self._captured(True, step)
 
   def _prompt_to_last_block(self, native, start_pos: int, n: int):
     """tokens[start_pos : start_pos + n] as rows up to the last block -> what takes the last one of them through that and samples the token behind it."""
@@ -469,7 +474,7 @@ class Transformer:
     def finish():
       self._check_room()
       self._host_pos += 1
-      self._last_block(lambda: self._enqueue_step(True, last_block=True))
+      self._last_block(lambda: self._enqueue_step(True, last_block=True), lambda: self._enqueue_step(True))
     return finish
 
   def _enqueue_rows_block(self, b, T: int, f: dict, p0, seq: int) -> None:
@@ -551,12 +556,9 @@ class Transformer:
     self._check_room()
     self._head_queued = True
     if not self.use_graph: return self._enqueue_batch_step()
-    if self._batch_graph is None:
-      self._enqueue_batch_step()                       # allocates the buffers outside the capture (and is a real step)
-      self._batch_graph = Graph(self.stream)
-      with self._batch_graph: self._enqueue_batch_step(count=False)
-      return
-    self._batch_graph.launch()
+    self._prefill_buffers()
+    self._batch_buffers()                              # (a capture allocates nothing)
+    self._captured(True, lambda: self._enqueue_batch_step(count=False)).launch()
     self._host_pos += 1
 
   def _batch_buffers(self):
@@ -643,7 +645,7 @@ class Transformer:
       check(lib.b200q_permute_rows(f["x"].ptr, at.ptr, seqs, size, last.ptr + i * size, 1, s))
     check(lib.b200q_memcpy_d2d(f["x"].ptr, last.ptr, B * size, s))
     self._host_pos = n
-    self._last_block(lambda: self._enqueue_batch_step(count=False, last_block=True))
+    self._last_block(lambda: self._enqueue_batch_step(count=False, last_block=True), lambda: self._enqueue_batch_step(count=False))
 
   def generate_batch(self, prompts: list):
     """Greedy generation for `batch` prompts of equal length; yields the list of the sequences' next tokens per step."""
@@ -730,12 +732,7 @@ class Transformer:
     self._host_pos += 1
     if self._step_args: return check(_lib.load().b200q_decode_step(ctypes.byref(self._step_args[bool(with_head)]), self.stream.ptr))
     if not self.use_graph: return self._enqueue_step(with_head)
-    g = self._graphs.get(with_head)
-    if g is None:
-      g = Graph(self.stream)
-      with g: self._enqueue_step(with_head)
-      self._graphs[with_head] = g
-    g.launch()
+    self._captured(bool(with_head), lambda: self._enqueue_step(with_head)).launch()
 
   # ---- host-visible state ----
   def set_state(self, tokens: list, pos: int) -> None:
