@@ -130,9 +130,9 @@ __device__ __forceinline__ float ld_cluster(uint32_t local, uint32_t rank) {    
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
   return v;
 }
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_sync() { cluster_arrive(); cluster_wait(); }
 
 // The power of two that puts a largest magnitude into [2^13, 2^14), where fp16 holds a value and the remainder's rounding to 2^-22 of it and to 2^-38 of
 // the largest, and its inverse; zeros get the inverse 0, infinities (and NaN) are left as they are.

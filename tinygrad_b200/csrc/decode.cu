@@ -381,16 +381,17 @@ namespace {
 //    same way, so that only the cache dtype rounds (as in the prompt kernel);
 //  * the positions are split over the cluster's CTAs in whole chunks of 64; the CTAs' partial results meet in distributed shared memory: one
 //    cluster barrier and one round of remote loads.  The split follows the position, so contexts of any length are spread over all CTAs;
-//  * two chunks are in flight, the first two already before the wait for the previous kernel.
+//  * two chunks at a time: keys and values of the first two are on their way before the wait for the previous kernel, the next two's keys go out when this round's scores are
+//    there, its values when they are used.  One chunk a round, two in flight: 12.3 us at 3507 positions of 28 / 4 heads (4 chunks a CTA; a launch, in order), 10.3; 14.3, 12.3 with 32 / 8;
+//  * after the wait one round trip through L2: the position comes with the values of q, k and v, cosines and sines are there already (position, then all of these: 8B
+//    Q4_0 10390 us for 8 tokens at 512, 10118); the last cluster barrier is entered at the last remote load, not after the output's store.
 // fp32 caches: the same with m16n8k8 tf32 products.  Queries, probabilities and cached values are all split in two tf32 numbers (2^-22 of the value
 // together, with the range of fp32), a cached value on its way from shared memory to the operand.
-constexpr int AC_THREADS = 256, AC_POS = 64;
+constexpr int AC_THREADS = 256, AC_POS = 64, AC_ROUND = 2 * AC_POS;
 template <int HD, typename KV> struct AcSmem {           // bytes; rows padded so that fragment loads hit distinct banks
   static constexpr bool F32 = sizeof(KV) == 4;
-  static constexpr int KROW = F32 ? (HD + 4) * 4 : (HD + 8) * 2, VROW = (HD + 8) * (int)sizeof(KV), QROW = KROW, PROW = F32 ? (AC_POS + 4) * 4 : (AC_POS + 8) * 2;
-  static constexpr int VCHUNK = AC_POS * KROW, BUF = AC_POS * (KROW + VROW);      // a buffer: 64 rows of K, 64 rows of V
-  static constexpr int Q = 2 * BUF, P = Q + 16 * QROW, S = P + 16 * PROW, O = S + 8 * (AC_POS + 4) * 4, ST = O + 8 * HD * 4, NEW = ST + 8 * 4 * 4,
-                       TOTAL = NEW + 2 * HD * (int)sizeof(KV);
+  static constexpr int KROW = F32 ? (HD + 4) * 4 : (HD + 8) * 2, VROW = (HD + 8) * (int)sizeof(KV), QROW = KROW, PROW = F32 ? (AC_ROUND + 4) * 4 : (AC_ROUND + 8) * 2;
+  static constexpr int V = AC_ROUND * KROW, Q = V + AC_ROUND * VROW, P = Q + 16 * QROW, S = P + 16 * PROW, O = S + 8 * (AC_ROUND + 4) * 4, ST = O + 8 * HD * 4, TOTAL = ST + 8 * 4 * 4;
 };
 
 __device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -443,6 +444,12 @@ template <typename KV> __device__ __forceinline__ void store_split(float v, unsi
     reinterpret_cast<__half*>(hi_row)[d] = hi; reinterpret_cast<__half*>(lo_row)[d] = lo;
   }
 }
+// a load that is issued where it stands
+__device__ __forceinline__ float ld_now(const float* p) {
+  float v;
+  asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
 template <typename KV> __device__ __forceinline__ KV cache_cast(float v);
 template <> __device__ __forceinline__ __half cache_cast<__half>(float v) { return __float2half_rn(v); }
 template <> __device__ __forceinline__ float cache_cast<float>(float v) { return v; }
@@ -467,48 +474,66 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int kvh = blockIdx.x, rank = blockIdx.y, n_rep = a.n_heads / a.n_kv_heads, half_r = a.rope_dim >> 1;
   const uint32_t base = (uint32_t)__cvta_generic_to_shared(asmem);
-  float* s_s = reinterpret_cast<float*>(asmem + M::S);            // [8][64 + 4] scores
+  float* s_s = reinterpret_cast<float*>(asmem + M::S);            // [8][128 + 4] scores
   float* s_o = reinterpret_cast<float*>(asmem + M::O);            // [8][HD] this CTA's unnormalised output
   float* s_m = reinterpret_cast<float*>(asmem + M::ST);           // [8] running max, [8] denominator, [8] rescale factor
   float *s_l = s_m + 8, *s_c = s_m + 16, *s_q = s_m + 24;        // [8] what a head's scores are multiplied with
-  KV* s_new = reinterpret_cast<KV*>(asmem + M::NEW);              // the new position's K and V rows
   KV* kc = reinterpret_cast<KV*>(a.k_cache) + (size_t)kvh * a.max_context * HD;
   KV* vc = reinterpret_cast<KV*>(a.v_cache) + (size_t)kvh * a.max_context * HD;
   pdl_launch_dependents();
-  // cached rows of chunk `ch` -> buffer `buf` (asynchronously, one commit group)
-  auto fetch = [&](int ch, int buf, int pos_now) {
-    const int n_old = min(AC_POS, pos_now - ch * AC_POS);
+  int c0 = 0, c1 = 0;
+  // cached rows of the round that starts with chunk `ch`, of K or of V (asynchronously, one commit group; chunks past c1: an empty one)
+  auto fetch = [&](int ch, const KV* from, int to, int row, int pos_now) {
+    const int n_old = min(AC_ROUND, min(c1 * AC_POS, pos_now) - ch * AC_POS);
     for (int i = tid; i < n_old * ROW_VECS; i += AC_THREADS) {
       const int r = i / ROW_VECS, c = i - r * ROW_VECS;
-      const size_t at = (size_t)(ch * AC_POS + r) * HD + c * VEC;
-      cp_async16(asmem + buf * M::BUF + r * M::KROW + c * 16, kc + at);
-      cp_async16(asmem + buf * M::BUF + M::VCHUNK + r * M::VROW + c * 16, vc + at);
+      cp_async16(asmem + to + r * row + c * 16, from + (size_t)(ch * AC_POS + r) * HD + c * VEC);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  int c0 = 0, c1 = 0;
-  auto split = [&](int pos_now) {                                  // this CTA's chunks for a context of pos_now + 1 positions
+  auto start = [&](int pos_now) {                                  // this CTA's chunks for a context of pos_now + 1 positions, and the first round's copies
     const int n_chunks = pos_now / AC_POS + 1, per = (n_chunks + CL - 1) / CL;
     c0 = min(n_chunks, rank * per); c1 = min(n_chunks, c0 + per);
-  };
-  auto start = [&](int pos_now) {
-    split(pos_now);
-#pragma unroll
-    for (int b = 0; b < 2; b++) {
-      if (c0 + b < c1) fetch(c0 + b, b, pos_now);
-      else asm volatile("cp.async.commit_group;" ::: "memory");
-    }
+    fetch(c0, kc, 0, M::KROW, pos_now);
+    fetch(c0, vc, M::V, M::VROW, pos_now);
   };
   // The rows were written by earlier steps: the copies go out before the wait for the previous kernel.  The position they are sized by is read
   // again after it, and the copies are redone in the (never observed) case that it moved.
   const int pos_early = min(max(__ldcg(a.pos), 0), a.max_context - 1);
   start(pos_early);
-  if (tid * 32 < a.rope_dim) prefetch_l2(a.rope + (size_t)pos_early * a.rope_dim + tid * 32);
   for (int i = tid; i < (16 * M::QROW + 16 * M::PROW) / 16; i += AC_THREADS) reinterpret_cast<uint4*>(asmem + M::Q)[i] = make_uint4(0, 0, 0, 0);   // rows of absent heads
   if (tid < 8) { s_m[tid] = -INFINITY; s_l[tid] = 0.f; s_q[tid] = 0.f; }
+  // RoPE, half-split layout: (x1 cos - x2 sin) || (x2 cos + x1 sin); dims past rope_dim pass through.  The table does not change: cosine and sine of the dims of this thread's
+  // query values and of its value of the new K row are read before the wait, too.
+  constexpr int QV = HD / 32;
+  float2 q_rot[QV], k_rot;
+  auto rotation = [&](int d, int pos_now) {
+    const float* rope = a.rope + (size_t)pos_now * a.rope_dim;
+    return d < half_r ? make_float2(rope[d], rope[d + half_r]) : d < a.rope_dim ? make_float2(rope[d - half_r], rope[d]) : make_float2(1.f, 0.f);
+  };
+  auto rotations = [&](int pos_now) {
+#pragma unroll
+    for (int j = 0; j < QV; j++) q_rot[j] = rotation(lane + 32 * j, pos_now);
+    k_rot = rotation(tid % HD, pos_now);
+  };
+  auto partner = [&](int d) { return d < half_r ? d + half_r : d < a.rope_dim ? d - half_r : d; };
+  auto roped = [&](float v, float other, float2 r, int d) {
+    if (d < half_r) return v * r.x - other * r.y;
+    if (d < a.rope_dim) return v * r.x + other * r.y;
+    return v;
+  };
+  rotations(pos_early);
   __syncthreads();
   pdl_wait();
-  const int pos = __ldcg(a.pos);
+  // one round trip: the position, and the values that do not hang on it (a warp takes a query head; a thread a value of the new K row and one of the new V row)
+  int pos;
+  asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(pos) : "l"(a.pos) : "memory");
+  const float *q_row = a.qkv + (size_t)(kvh * n_rep + warp) * HD, *k_row = a.qkv + (size_t)(a.n_heads + kvh) * HD, *v_row = k_row + (size_t)a.n_kv_heads * HD;
+  float q[QV], q_other[QV], k_new = 0.f, k_other = 0.f, v_new = 0.f;
+  if (warp < n_rep)
+#pragma unroll
+    for (int j = 0; j < QV; j++) { q[j] = ld_now(q_row + lane + 32 * j); q_other[j] = ld_now(q_row + partner(lane + 32 * j)); }
+  if (tid < HD) { k_new = ld_now(k_row + tid); k_other = ld_now(k_row + partner(tid)); v_new = ld_now(v_row + tid); }
   if (pos < 0 || pos >= a.max_context) {                           // no cache row for this position: touch nothing (uniform over the cluster)
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     if (tid == 0 && rank == 0) atomicExch(&g_decode_status, 2);
@@ -518,59 +543,45 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     start(pos);
+    rotations(pos);
   }
   const bool owner = c0 < c1 && pos / AC_POS == c1 - 1;             // the new position is in this CTA's last chunk
-  // RoPE, half-split layout: (x1 cos - x2 sin) || (x2 cos + x1 sin); dims past rope_dim pass through
-  const float* rope = a.rope + (size_t)pos * a.rope_dim;
-  auto roped = [&](const float* v, int d) {
-    if (d < half_r) return v[d] * rope[d] - v[d + half_r] * rope[half_r + d];
-    if (d < a.rope_dim) return v[d] * rope[d - half_r] + v[d - half_r] * rope[d];
-    return v[d];
-  };
-  if (c0 < c1) {
-    if (warp < n_rep) {                                            // a warp takes a query head; fp16: under a power of two of its own
-      const float* src = a.qkv + (size_t)(kvh * n_rep + warp) * HD;
-      float v[HD / 32], up = 1.f, down = 1.f;
+  if (c0 < c1 && warp < n_rep) {                                   // fp16: under a power of two of the head's own
+    float up = 1.f, down = 1.f;
 #pragma unroll
-      for (int j = 0; j < HD / 32; j++) v[j] = roped(src, lane + 32 * j);
-      if constexpr (!F32) {
-        float amax = 0.f;
+    for (int j = 0; j < QV; j++) q[j] = roped(q[j], q_other[j], q_rot[j], lane + 32 * j);
+    if constexpr (!F32) {
+      float amax = 0.f;
 #pragma unroll
-        for (int j = 0; j < HD / 32; j++) amax = fmaxf(amax, fabsf(v[j]));
-        pow2_scale(warp_max(amax), up, down);
-      }
-#pragma unroll
-      for (int j = 0; j < HD / 32; j++) store_split<KV>(v[j] * up, asmem + M::Q + warp * M::QROW, asmem + M::Q + (8 + warp) * M::QROW, lane + 32 * j);
-      if (lane == 0) s_q[warp] = down * (1.0f / sqrtf((float)HD));
+      for (int j = 0; j < QV; j++) amax = fmaxf(amax, fabsf(q[j]));
+      pow2_scale(warp_max(amax), up, down);
     }
-    if (owner) {
-      for (int i = tid; i < 2 * HD; i += AC_THREADS) {
-        const int d = i % HD;
-        const bool v = i >= HD;
-        const KV h = cache_cast<KV>(v ? a.qkv[(size_t)(a.n_heads + a.n_kv_heads + kvh) * HD + d] : roped(a.qkv + (size_t)(a.n_heads + kvh) * HD, d));
-        s_new[i] = h;
-        (v ? vc : kc)[(size_t)pos * HD + d] = h;
-      }
-    }
+#pragma unroll
+    for (int j = 0; j < QV; j++) store_split<KV>(q[j] * up, asmem + M::Q + warp * M::QROW, asmem + M::Q + (8 + warp) * M::QROW, lane + 32 * j);
+    if (lane == 0) s_q[warp] = down * (1.0f / sqrtf((float)HD));
   }
+  const KV k_cast = cache_cast<KV>(roped(k_new, k_other, k_rot, tid)), v_cast = cache_cast<KV>(v_new);
+  if (owner && tid < HD) { kc[(size_t)pos * HD + tid] = k_cast; vc[(size_t)pos * HD + tid] = v_cast; }
   float acc[HD / 64][4];                                             // this warp's HD / 8 output dims: rows g (high parts) and g + 8 (low parts)
 #pragma unroll
   for (int j = 0; j < HD / 64; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-  for (int ch = c0; ch < c1; ch++) {
-    const int buf = (ch - c0) & 1, nv = min(AC_POS, pos + 1 - ch * AC_POS);
-    unsigned char* sk = asmem + buf * M::BUF;
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
-    __syncthreads();                                                 // (also: queries and the new rows are in place)
-    if (nv < AC_POS || (owner && ch == c1 - 1)) {                    // the last chunk: append the new row, and no stale values behind it (0 * NaN)
-      for (int i = tid; i < 2 * HD; i += AC_THREADS)
-        *reinterpret_cast<KV*>(sk + (i < HD ? (nv - 1) * M::KROW : M::VCHUNK + (nv - 1) * M::VROW) + (i % HD) * (int)sizeof(KV)) = s_new[i];
-      for (int i = tid; i < (AC_POS - nv) * ROW_VECS; i += AC_THREADS)
-        *reinterpret_cast<uint4*>(sk + M::VCHUNK + (nv + i / ROW_VECS) * M::VROW + (i % ROW_VECS) * 16) = make_uint4(0, 0, 0, 0);
-      __syncthreads();
+  for (int ch = c0; ch < c1; ch += 2) {
+    const bool two = ch + 1 < c1;
+    const int end = two ? AC_ROUND : AC_POS, nv = min(end, pos + 1 - ch * AC_POS);
+    if (nv < end || (owner && ch + 2 >= c1)) {                       // the last chunk: append the new row, and no stale values behind it (0 * NaN)
+      if (tid < HD) {
+        *reinterpret_cast<KV*>(asmem + (nv - 1) * M::KROW + tid * (int)sizeof(KV)) = k_cast;
+        *reinterpret_cast<KV*>(asmem + M::V + (nv - 1) * M::VROW + tid * (int)sizeof(KV)) = v_cast;
+      }
+      for (int i = tid; i < (end - nv) * ROW_VECS; i += AC_THREADS)
+        *reinterpret_cast<uint4*>(asmem + M::V + (nv + i / ROW_VECS) * M::VROW + (i % ROW_VECS) * 16) = make_uint4(0, 0, 0, 0);
     }
-    {   // scores: warp w takes positions 8w .. 8w + 7
+    asm volatile("cp.async.wait_group 1;" ::: "memory");             // the keys
+    __syncthreads();                                                 // (also: queries and the new rows are in place)
+#pragma unroll 1
+    for (int p0 = 0; p0 < end; p0 += AC_POS) {                       // scores: warp w takes positions 8w .. 8w + 7 of a chunk
       float c[4] = {0.f, 0.f, 0.f, 0.f}, c2[4] = {0.f, 0.f, 0.f, 0.f};
-      const unsigned char* kr = sk + (warp * 8 + g) * M::KROW + t * 4;
+      const unsigned char* kr = asmem + (p0 + warp * 8 + g) * M::KROW + t * 4;
       if constexpr (F32) {
         const unsigned char* qa = asmem + M::Q + g * M::QROW + t * 4;
 #pragma unroll 4
@@ -591,35 +602,44 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
           if (kk & 1) mma_f16_rn(c2, q4, b0, b1); else mma_f16_rn(c, q4, b0, b1);
         }
       }
-      const int p = warp * 8 + 2 * t;
+      const int p = p0 + warp * 8 + 2 * t;
       const float scale = s_q[g], s0 = ((c[0] + c2[0]) + (c[2] + c2[2])) * scale, s1 = ((c[1] + c2[1]) + (c[3] + c2[3])) * scale;
-      s_s[g * (AC_POS + 4) + p] = p < nv ? s0 : -INFINITY;
-      s_s[g * (AC_POS + 4) + p + 1] = p + 1 < nv ? s1 : -INFINITY;
+      s_s[g * (AC_ROUND + 4) + p] = p < nv ? s0 : -INFINITY;
+      s_s[g * (AC_ROUND + 4) + p + 1] = p + 1 < nv ? s1 : -INFINITY;
     }
     __syncthreads();
+    fetch(ch + 2, kc, 0, M::KROW, pos);                              // the next round's keys, while this one's probabilities are made and used
     if (warp < n_rep) {                                              // softmax of head `warp`
-      const float2 s2 = *reinterpret_cast<const float2*>(s_s + warp * (AC_POS + 4) + 2 * lane);
-      const float m0 = s_m[warp], m1 = fmaxf(m0, warp_max(fmaxf(s2.x, s2.y)));
-      const float p0 = __expf(s2.x - m1), p1 = __expf(s2.y - m1), cr = __expf(m0 - m1), sum = warp_sum(p0 + p1);
-      if constexpr (F32) {
-        store_split<KV>(p0, asmem + M::P + warp * M::PROW, asmem + M::P + (8 + warp) * M::PROW, 2 * lane);
-        store_split<KV>(p1, asmem + M::P + warp * M::PROW, asmem + M::P + (8 + warp) * M::PROW, 2 * lane + 1);
-      } else {
-        __half h0, l0, h1, l1;
-        split_h(p0, h0, l0); split_h(p1, h1, l1);
-        *reinterpret_cast<__half2*>(asmem + M::P + warp * M::PROW + lane * 4) = __halves2half2(h0, h1);
-        *reinterpret_cast<__half2*>(asmem + M::P + (8 + warp) * M::PROW + lane * 4) = __halves2half2(l0, l1);
+      const float* sc = s_s + warp * (AC_ROUND + 4) + 2 * lane;
+      const float2 s2 = *reinterpret_cast<const float2*>(sc), s3 = two ? *reinterpret_cast<const float2*>(sc + AC_POS) : make_float2(-INFINITY, -INFINITY);
+      const float m0 = s_m[warp], m1 = fmaxf(m0, warp_max(fmaxf(fmaxf(s2.x, s2.y), fmaxf(s3.x, s3.y))));
+      const float cr = __expf(m0 - m1), p[4] = {__expf(s2.x - m1), __expf(s2.y - m1), __expf(s3.x - m1), __expf(s3.y - m1)}, sum = warp_sum((p[0] + p[1]) + (p[2] + p[3]));
+#pragma unroll
+      for (int j = 0; j < 4; j += 2) {
+        unsigned char* const pr = asmem + M::P + warp * M::PROW;
+        const int at = 2 * lane + j / 2 * AC_POS;
+        if constexpr (F32) {
+          store_split<KV>(p[j], pr, pr + 8 * M::PROW, at);
+          store_split<KV>(p[j + 1], pr, pr + 8 * M::PROW, at + 1);
+        } else {
+          __half h0, l0, h1, l1;
+          split_h(p[j], h0, l0); split_h(p[j + 1], h1, l1);
+          *reinterpret_cast<__half2*>(pr + at * 2) = __halves2half2(h0, h1);
+          *reinterpret_cast<__half2*>(pr + 8 * M::PROW + at * 2) = __halves2half2(l0, l1);
+        }
       }
       __syncwarp();
       if (lane == 0) { s_m[warp] = m1; s_l[warp] = s_l[warp] * cr + sum; s_c[warp] = cr; }
     }
+    asm volatile("cp.async.wait_group 1;" ::: "memory");             // the values
     __syncthreads();
-    {   // O = P V: warp w takes HD / 8 dims
-      const float cr = g < n_rep ? s_c[g] : 0.f;
+    const float cr = g < n_rep ? s_c[g] : 0.f;
 #pragma unroll
-      for (int j = 0; j < HD / 64; j++) { acc[j][0] *= cr; acc[j][1] *= cr; acc[j][2] *= cr; acc[j][3] *= cr; }
+    for (int j = 0; j < HD / 64; j++) { acc[j][0] *= cr; acc[j][1] *= cr; acc[j][2] *= cr; acc[j][3] *= cr; }
+#pragma unroll 1
+    for (int p0 = 0; p0 < end; p0 += AC_POS) {                       // O = P V: warp w takes HD / 8 dims
       if constexpr (F32) {
-        const unsigned char *pa = asmem + M::P + g * M::PROW + t * 4, *va = sk + M::VCHUNK + t * M::VROW + (warp * (HD / 8) + g) * 4;
+        const unsigned char *pa = asmem + M::P + g * M::PROW + (p0 + t) * 4, *va = asmem + M::V + (p0 + t) * M::VROW + (warp * (HD / 8) + g) * 4;
 #pragma unroll 4
         for (int kk = 0; kk < AC_POS / 8; kk++) {
           uint32_t p4[4];
@@ -633,9 +653,9 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
           }
         }
       } else {
-      const uint32_t pa = base + M::P + (lane & 15) * M::PROW + (lane >> 4) * 16;
+      const uint32_t pa = base + M::P + (lane & 15) * M::PROW + (lane >> 4) * 16 + p0 * 2;
       // transposing loads: 8x8 blocks of (positions, dims).  128: positions kk*16 + {0..7, 8..15} x dims {0..7, 8..15}; 64: 32 positions x 8 dims
-      const uint32_t va = base + (uint32_t)(sk - asmem) + M::VCHUNK + warp * (HD / 8) * 2 +
+      const uint32_t va = base + M::V + p0 * M::VROW + warp * (HD / 8) * 2 +
                           (HD == 128 ? (((lane >> 3) & 1) * 8 + (lane & 7)) * M::KROW + (lane >> 4) * 16 : lane * M::KROW);
       if (HD == 128) {
 #pragma unroll
@@ -659,10 +679,8 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
       }
       }
     }
-    if (ch + 2 < c1) {
-      __syncthreads();                                               // everybody is done with the buffer
-      fetch(ch + 2, buf, pos);
-    } else asm volatile("cp.async.commit_group;" ::: "memory");
+    if (ch + 2 < c1) __syncthreads();                                // everybody is done with the values
+    fetch(ch + 2, vc, M::V, M::VROW, pos);
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
@@ -670,6 +688,7 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
     *reinterpret_cast<float2*>(s_o + g * HD + warp * (HD / 8) + j * 8 + 2 * t) = make_float2(acc[j][0] + acc[j][2], acc[j][1] + acc[j][3]);
   cluster_sync();
   // merge: the (head, 32 dims) units are dealt over the cluster's CTAs, one warp each
+  bool arrived = false;
   for (int u = warp * CL + rank; u < n_rep * (HD / 32); u += AC_THREADS / 32 * CL) {
     const int h = u / (HD / 32), d = (u - h * (HD / 32)) * 32 + lane;
     const uint32_t st = base + M::ST + h * 4, oa = base + M::O + (h * HD + d) * 4;
@@ -677,6 +696,7 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
 #pragma unroll
     for (int s = 0; s < CL; s++) o[s] = ld_cluster(oa, s);
     const float m = lane < CL ? ld_cluster(st, lane) : -INFINITY, l = lane < CL ? ld_cluster(st + 32, lane) : 0.f;
+    if (CL > 1) { cluster_arrive(); arrived = true; }                // the last remote load
     const float w = __expf(m - warp_max(m));                         // 0 for CTAs without positions
     const float den = warp_sum(w * l);
     float v = 0.f;
@@ -687,7 +707,10 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
     if (a.xq_out) quant_block_32x1(v, lane, (kvh * n_rep + h) * (HD / 32) + (d >> 5), XqDst(a.xq_out, a.n_heads));      // head_dim 128: one group per head
     if (CL > 1) break;                                               // one unit per warp at most
   }
-  cluster_sync();                                                    // nobody leaves while its partial results are being read
+  if (CL > 1) {                                                      // nobody leaves while its partial results are being read
+    if (!arrived) cluster_arrive();
+    cluster_wait();
+  }
 }
 
 // ---------------------------------------------------------------------------
