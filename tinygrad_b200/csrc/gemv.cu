@@ -157,13 +157,27 @@ __device__ __noinline__ void settle_handover(const GemvParams& p, float* ubuf, i
   __syncwarp();
 }
 
+// A thread that has no part in the copies between CTAs: past the first cluster barrier, and counted for the second (in its own time: not `aligned`)
+__device__ __forceinline__ void cluster_pass() { asm volatile("barrier.cluster.wait.acquire;\nbarrier.cluster.arrive.release;" ::: "memory"); }
+
+// Part of this CTA's shared memory to the same place of another CTA of the cluster, counted on that one's barrier `bar`
+__device__ __forceinline__ void bulk_s2cluster(uint32_t at, uint32_t bytes, uint32_t bar, uint32_t rank) {
+  uint32_t to, to_bar;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(at), "r"(rank));
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to_bar) : "r"(bar), "r"(rank));
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(to), "r"(at), "r"(bytes), "r"(to_bar) : "memory");
+}
+
 // XQ_IN / XQ_OUT: compiled-in use of a ready-made input record / production of an output record.
-template <int QT, bool XQ_IN, bool XQ_OUT>
+// CL: CTAs of a cluster that quantise the row together.  Every CTA needs the whole row's codes, and on a long row making them is what stands between the row's arrival and the first
+// tile (14336 values: 3.4 us, two round trips through L2 and 90 instructions per 8 values, on two CTAs of an SM): each makes an equal part, and a warp's two column
+// groups go to the others as copies between shared memories while the next are made.  The codes and the order of the sums are the same.
+template <int QT, bool XQ_IN, bool XQ_OUT, int CL>
 __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(const GemvParams p) {
   constexpr int NS = Cfg<QT>::NS, SG = Cfg<QT>::SG, XSUB = Cfg<QT>::XSUB, STAGE_BYTES = SG * tile_bytes(QT == K_MIX ? B200Q_Q6_K_WIDE : QT);
   constexpr bool WIDE = is_wide(QT);
   constexpr int XB = X_BYTES<QT>;
-  static_assert(!(XQ_IN && (XSUB || WIDE)), "ready-made records are the plain int8 form");
+  static_assert(!((XQ_IN || CL > 1) && (XSUB || WIDE)), "ready-made and shared records are the plain int8 form");
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned char* ring = smem;
   unsigned char* record = smem + NS * STAGE_BYTES;
@@ -200,6 +214,7 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
+  if (CL > 1) cluster_arrive();
 #ifdef B200Q_GEMV_PROF
   const unsigned prof_slot = s_prof_slot;
 #endif
@@ -213,6 +228,7 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
       // The first NS fills need no consumer.  After them the consumers must be running, and they start only when the
       // previous kernel has finished: wait for it outside the bounded waits, then fetch the activation record it left.
       auto after_prefetch = [&]() {
+        if (CL > 1) cluster_pass();
         pdl_wait();
         if (XQ_IN) {
           // the record in pieces on one barrier: a single bulk copy is served slowly, several overlap
@@ -255,6 +271,7 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
       for (int j = max(0, it - NS); j < it; j++) mbar_wait(full0 + 8 * (j % NS), (j / NS) & 1);
       if (XQ_IN) mbar_wait(xbar, 0);
     } else {
+      if (CL > 1) cluster_pass();
       pdl_wait();   // keep launch order transitive: this grid is not complete before its predecessor
     }
     return;
@@ -265,6 +282,7 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
     // Takes every row tile's cross-warp sum and epilogue off the consumers: they leave their partial sums in `red` (two buffers,
     // a full / empty barrier pair each) and go on with the next tile; nothing in a tile's MMAs waits for the previous tile's
     // stores, residual loads or hand-over bookkeeping.
+    if (CL > 1) cluster_pass();
     pdl_wait();
     float pre_add = 0.f;
     const int first_rt = blockIdx.x * (XQ_OUT ? p.unit : 1);
@@ -358,6 +376,12 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
 
   // -------------------------------- consumers --------------------------------
   if (p.norm_w && blockIdx.x < 8 && (blockIdx.x * 64 + tid) * 64 < p.n_in && tid < 64) prefetch_l2(p.norm_w + (blockIdx.x * 64 + tid) * 64);
+  // this CTA's part of the row, in column groups; the others' parts come as copies, counted on xbar
+  const int rank = CL > 1 ? blockIdx.x % CL : 0, own0 = p.kgroups * rank / CL, own1 = p.kgroups * (rank + 1) / CL;
+  if (CL > 1) {
+    if (tid == 0) mbar_expect_tx(xbar, (uint32_t)(p.kgroups - (own1 - own0)) * XQ_GROUP_BYTES);
+    cluster_wait();                                  // every CTA of the cluster runs, its barriers are there
+  }
   pdl_wait();
   PSTAMP(1);
   const int g = lane >> 2, t = lane & 3;
@@ -374,7 +398,7 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
 #define B200Q_XPF 2
 #endif
     constexpr int PF = B200Q_XPF, BSTEP = CONS_THREADS / 4;
-    const int nblk_pad = p.kgroups * 4, q = tid & 3;
+    const int nblk_pad = own1 * 4, q = tid & 3;
     const XqDst dst(record, p.kgroups);
 #pragma unroll 1
     for (int pass = 0; pass < (WIDE ? 2 : 1); pass++) {                 // full precision: first the row's largest value, then the values (from L1)
@@ -389,7 +413,7 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
       }
     }
 #pragma unroll 1
-    for (int w0 = warp * 8; w0 < nblk_pad; w0 += PF * BSTEP) {          // 8 blocks per warp and round
+    for (int w0 = own0 * 4 + warp * 8; w0 < nblk_pad; w0 += PF * BSTEP) {          // 8 blocks per warp and round
       const int b0 = w0 + (lane >> 2);
       float4 v[PF][2];
       uint4 nw[PF];
@@ -433,7 +457,19 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
 #pragma unroll
               for (int i = 0; i < 8; i++) amax = fmaxf(amax, fabsf(f[i]));
             } else if (b0 + u * BSTEP < nblk_pad) wide_store_8(f, q, b0 + u * BSTEP, x_up, record);
-          } else quant_block_4x8(f, q, b0 + u * BSTEP, b0 + u * BSTEP < nblk_pad, dst, XSUB ? sub16 : nullptr);
+          } else {
+            quant_block_4x8(f, q, b0 + u * BSTEP, b0 + u * BSTEP < nblk_pad, dst, XSUB ? sub16 : nullptr);
+            if (CL > 1) {                                               // the warp's two groups go to the others: a lane per CTA
+              const int j = (w0 + u * BSTEP) >> 2;
+              const uint32_t n = min(2, own1 - j);
+              asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+              __syncwarp();
+              if (lane < CL && lane != rank) {
+                bulk_s2cluster(smem_u32(record) + j * 256, n * 256, xbar, lane);
+                bulk_s2cluster(smem_u32(record) + p.kgroups * 256 + j * 64, n * 64, xbar, lane);
+              }
+            }
+          }
         }
       }
     }
@@ -443,7 +479,8 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
     ss = warp_sum(ss);
     if (lane == 0) ssq[warp] = ss;
   }
-  if (XQ_IN && !mbar_wait(xbar, 0)) *s_abort = 1;
+  if ((XQ_IN || CL > 1) && !mbar_wait(xbar, 0)) *s_abort = 1;
+  if (CL > 1) { __syncwarp(); cluster_arrive(); }    // this CTA has the others' parts
   cons_bar_sync();
   PSTAMP(2);
   const bool diag = (t == (g & 3));
@@ -515,6 +552,7 @@ __global__ void __launch_bounds__(NTHREADS, B200Q_CTAS_PER_SM) qgemv_kernel(cons
       if (lane == 0) mbar_arrive(rfull0 + 8 * par);
     }
   }
+  if (CL > 1) { __syncwarp(); cluster_wait(); }      // the others have this CTA's: it may leave
   PSTAMP(5);
 }
 
@@ -534,13 +572,14 @@ int g_gemv_prof_host_counter = 0;
 namespace {
 #endif
 
-template <int QT, bool XQ_IN, bool XQ_OUT>
+constexpr int NO_ROOM = 1;      // launch_gemv with clusters: they would not all run at once
+template <int QT, bool XQ_IN, bool XQ_OUT, int CL = 1>
 int launch_gemv(const b200q_gemv_args* a, const GemvParams& p, cudaStream_t stream) {
   constexpr int NS = Cfg<QT>::NS;
   const size_t smem = (size_t)NS * Cfg<QT>::SG * tile_bytes(QT == K_MIX ? B200Q_Q6_K_WIDE : QT) + (size_t)p.kgroups * (X_BYTES<QT> + Cfg<QT>::XSUB) + 16 +
                       (2 * CONS_WARPS * 16 + CONS_WARPS + 32) * sizeof(float) + (2 * NS + 5) * sizeof(uint64_t) + 16;
   if (smem > 220 * 1024) return B200Q_ERR_TOO_LARGE;
-  auto kern = qgemv_kernel<QT, XQ_IN, XQ_OUT>;
+  auto kern = qgemv_kernel<QT, XQ_IN, XQ_OUT, CL>;
   // per device (and per instantiation): the shared-memory attribute, and the last occupancy answer packed as (smem << 8) | blocks
   static PerDeviceFlag attr_set;
   static std::atomic<long long> occ_cache[B200Q_MAX_DEVICES];
@@ -570,8 +609,43 @@ int launch_gemv(const b200q_gemv_args* a, const GemvParams& p, cudaStream_t stre
   B200Q_CHECK_CUDA(launch_k(kern, dim3(grid_x, a->m), dim3(NTHREADS), smem, stream, (a->flags & B200Q_FLAG_PDL) != 0, pp));
   return B200Q_OK;
 #endif
+  if (CL > 1) {
+    grid_x = (grid_x + CL - 1) / CL * CL;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid_x, a->m); cfg.blockDim = dim3(NTHREADS); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CL; attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    static std::atomic<long long> room_cache[B200Q_MAX_DEVICES];       // (smem << 16) | clusters that run at once
+    long long room = room_cache[dev].load(std::memory_order_relaxed);
+    if (room == 0 || (room >> 16) != (long long)smem) {
+      int n = 0;
+      B200Q_CHECK_CUDA(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
+      room = ((long long)smem << 16) | n;
+      room_cache[dev].store(room, std::memory_order_relaxed);
+    }
+    if (grid_x > CL * (int)(room & 0xFFFF)) return NO_ROOM;
+    cfg.numAttrs = a->flags & B200Q_FLAG_PDL ? 2 : 1;
+    B200Q_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, p));
+    return B200Q_OK;
+  }
   B200Q_CHECK_CUDA(launch_k(kern, dim3(grid_x, a->m), dim3(NTHREADS), smem, stream, (a->flags & B200Q_FLAG_PDL) != 0, p));
   return B200Q_OK;
+}
+
+// Rows that more than one round of staging loads takes (8192 values) are quantised by clusters: of four CTAs where all of them run at once, else of two.  us a launch in a
+// chain, every CTA the whole row / clusters of 2 / of 4: Q4_0 4096 x 14336 10.6 / 9.8 / 9.5, 4096 x 28672 19.2 / 18.7 / 18.0, 5120 x 18944 (one CTA an SM, 148) 18.3 / 18.0 / 24.2; Q8_0
+// 3584 x 18944 16.7 / 16.5 / 16.1.  On the other side the copies take longer than the round: 4096 x 8192 6.3 / 6.5 / 6.7, 4096 x 4096 4.1 / 4.5 / 4.9.
+template <int QT>
+int launch_long_row(const b200q_gemv_args* a, const GemvParams& p, cudaStream_t stream) {
+  const int rc = launch_gemv<QT, false, false, 4>(a, p, stream);
+  return rc == NO_ROOM ? launch_gemv<QT, false, false, 2>(a, p, stream) : rc;
+}
+static bool takes_long_row(const b200q_gemv_args* a, const GemvParams& p) {
+  return (a->qtype == B200Q_Q4_0 || a->qtype == B200Q_Q8_0) && !a->xq_in && !a->xq_out && !a->norm_weight && a->m == 1 && a->max_ctas <= 0 && p.kgroups * GROUP_ELEMS > 8192;
 }
 
 }  // namespace
@@ -664,6 +738,10 @@ extern "C" int b200q_gemv(const b200q_gemv_args* a, void* stream) {
   if (p.w2) return launch_gemv<K_MIX, false, false>(a, p, (cudaStream_t)stream);
   if (a->qtype == B200Q_Q4_K_WIDE) return launch_gemv<B200Q_Q4_K_WIDE, false, false>(a, p, (cudaStream_t)stream);
   if (a->qtype == B200Q_Q6_K_WIDE) return launch_gemv<B200Q_Q6_K_WIDE, false, false>(a, p, (cudaStream_t)stream);
+  if (takes_long_row(a, p)) {
+    const int rc = a->qtype == B200Q_Q4_0 ? launch_long_row<B200Q_Q4_0>(a, p, (cudaStream_t)stream) : launch_long_row<B200Q_Q8_0>(a, p, (cudaStream_t)stream);
+    if (rc != NO_ROOM) return rc;
+  }
   if (a->qtype == B200Q_Q4_0) {
     if (xi) return xo ? launch_gemv<B200Q_Q4_0, true, true>(a, p, (cudaStream_t)stream) : launch_gemv<B200Q_Q4_0, true, false>(a, p, (cudaStream_t)stream);
     return xo ? launch_gemv<B200Q_Q4_0, false, true>(a, p, (cudaStream_t)stream) : launch_gemv<B200Q_Q4_0, false, false>(a, p, (cudaStream_t)stream);
