@@ -118,6 +118,10 @@ extern "C" int b200q_graph_end(void* stream, void** graph_exec) {
   cudaError_t e = cudaGraphInstantiate((cudaGraphExec_t*)graph_exec, graph, 0);
   cudaGraphDestroy(graph);
   B200Q_CHECK_CUDA(e);
+  // to the device now, behind what the stream has to do, and not with the first launch (a step's graph is captured while the device has the prompt to do)
+  e = cudaGraphUpload((cudaGraphExec_t)*graph_exec, (cudaStream_t)stream);
+  if (e != cudaSuccess) { cudaGraphExecDestroy((cudaGraphExec_t)*graph_exec); *graph_exec = nullptr; }
+  B200Q_CHECK_CUDA(e);
   return B200Q_OK;
 }
 extern "C" int b200q_graph_launch(void* graph_exec, void* stream) {
