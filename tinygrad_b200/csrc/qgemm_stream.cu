@@ -756,28 +756,6 @@ static int stream_grid(long long units, int n_sm) {
   return (int)(g < most ? g : most);
 }
 
-// How a GEMM whose sums may be split is dealt.  A CTA on every SM with an equal share of all units (stream-K) leaves no SM waiting, but the shares end in the middle of tiles: a CTA
-// reads its accumulators back twice, a tile's parts go through L2 and the last of its CTAs adds them.  So where it costs less, the grid is a multiple of the tiles (an equal share
-// is then an equal part of one tile: one accumulator read-back, a part less), or CTAs have whole tiles (no parts at all).  What that costs is the largest share over the mean
-// over all SMs, in K groups of a tile; what it saves, by measurement: whole tiles 7 to 16 us, multiples 2.5 to 7, the more the larger the tile.  450 shapes, 8 to 512 rows, us a call, a
-// CTA on every SM / so: 45 rows of Q4_0 6144 x 4096 (48 tiles x 3) 24.7 / 22.7, 4096 x 4096 (32 x 4) 24.3 / 20.9, 11264 x 2048 (88 whole) 25.4 / 19.6; 13 rows of 4096 x 4096 18.6 / 14.7; 512
-// half-precision rows of Q8_0 5632 x 1024 (88 whole) 38.0 / 20.8, 5120 x 2560 (80 whole) 42.6 / 30.9.  Of tiles of more than 224 rows the parts are so large that many at once cost
-// more than their number saves: 512 rows of 1280 x 3424 (20 x 7) 48.3 / 51.7, 1024 x 2816 (16 x 9) 49.4 / 51.0, in half precision 37.7 / 38.3.
-struct Deal { int grid; bool whole; };
-static Deal deal_units(const Plan& pl, int tiles, int kgroups, bool f32, int n_sm) {
-  const long long units = (long long)tiles * kgroups;
-  const int group_cycles = std::max(950, pl.wt / 128 * (f32 ? 12 : 4) * pl.nt);      // unpacking a K group of 128 rows, or its products
-  const int s = n_sm / tiles, waves = ceil_div(tiles, n_sm), most = pl.nt <= 224 ? 16 : f32 ? 4 : 8;
-  if (s <= 1) {
-    const long long over = ((long long)waves * kgroups * n_sm - units) * group_cycles;      // cycles times the SMs
-    if (over <= (12000LL + 50 * pl.nt) * n_sm) return Deal{ceil_div(tiles, waves), true};
-  } else if (s <= most && kgroups >= 2 * s) {
-    const long long over = ((long long)ceil_div(kgroups, s) * n_sm - units) * group_cycles;
-    if (over <= (4000LL + 30 * pl.nt) * n_sm) return Deal{tiles * s, false};
-  }
-  return Deal{stream_grid(units, n_sm), false};
-}
-
 // the rows' scales, counters and partial sums behind the activation tiles; n_out = 0: enough for any
 static size_t split_workspace(const Plan& pl, int n_out, int kgroups, int n_sm) {
   long long parts = 2LL * n_sm;
@@ -848,9 +826,8 @@ int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtyp
   p.tiles = ceil_div(n_out, pl.wt) * pl.tok_tiles;
   p.units = (long long)p.tiles * kgroups;
   const bool split = !unsplit && workspace_bytes >= xt_bytes + split_workspace(pl, n_out, kgroups, n_sm);
-  const Deal deal = split ? deal_units(pl, p.tiles, kgroups, f32, n_sm) : Deal{p.tiles < n_sm ? p.tiles : n_sm, true};
-  const int grid = deal.grid;
-  p.grain = deal.whole ? kgroups : 1; p.unsplit = !split;
+  p.grain = split ? 1 : kgroups; p.unsplit = !split;
+  const int grid = split ? stream_grid(p.units, n_sm) : (p.tiles < n_sm ? p.tiles : n_sm);
   p.dump = p.d_cols = 0;
   // one CTA of the splitting kernel: 8 rows x the whole width, or a part of it where there are few rows (and, of fp32 rows, more than a CTA keeps in registers)
   const int row_groups = pl.tok_tiles * pl.nt / 8, n_chunks = kgroups * 16;
