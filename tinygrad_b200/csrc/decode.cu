@@ -404,7 +404,7 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], 
 }
 // The same for operands whose rows 8 .. 15 hold what the rounding of rows 0 .. 7 left: the sums of rows 0 .. 7 are added here, to nearest.  The tensor core
 // truncates, always towards zero, when it adds to an accumulator.  Error of the output's norm against 64 bits, 37 .. 3507 positions (root mean square of 64
-// cases): fp16 caches 2.3e-7, with running accumulators 3.1e-7; fp32 caches 2.3e-7, 8.6e-7 (up to 2.4e-6); the one-lane-per-position kernel 2.0e-7.
+// cases): fp16 caches 2.0e-7 (2.3e-7 with probabilities of at most 1), with running accumulators 3.1e-7; fp32 caches 2.3e-7, 8.6e-7 (up to 2.4e-6); the one-lane-per-position kernel 2.0e-7.
 __device__ __forceinline__ void mma_f16_rn(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   float p[4] = {0.f, 0.f, c[2], c[3]};
   mma_f16(p, a, b0, b1);
@@ -610,10 +610,11 @@ __global__ void __launch_bounds__(AC_THREADS) attn_cluster_kernel(const b200q_at
     __syncthreads();
     fetch(ch + 2, kc, 0, M::KROW, pos);                              // the next round's keys, while this one's probabilities are made and used
     if (warp < n_rep) {                                              // softmax of head `warp`
+      constexpr float UP = F32 ? 1.f : 256.f;                        // probabilities (and their sum) 256 times as large: a remainder below 2^-14 loses bits
       const float* sc = s_s + warp * (AC_ROUND + 4) + 2 * lane;
       const float2 s2 = *reinterpret_cast<const float2*>(sc), s3 = two ? *reinterpret_cast<const float2*>(sc + AC_POS) : make_float2(-INFINITY, -INFINITY);
       const float m0 = s_m[warp], m1 = fmaxf(m0, warp_max(fmaxf(fmaxf(s2.x, s2.y), fmaxf(s3.x, s3.y))));
-      const float cr = __expf(m0 - m1), p[4] = {__expf(s2.x - m1), __expf(s2.y - m1), __expf(s3.x - m1), __expf(s3.y - m1)}, sum = warp_sum((p[0] + p[1]) + (p[2] + p[3]));
+      const float cr = __expf(m0 - m1), p[4] = {__expf(s2.x - m1) * UP, __expf(s2.y - m1) * UP, __expf(s3.x - m1) * UP, __expf(s3.y - m1) * UP}, sum = warp_sum((p[0] + p[1]) + (p[2] + p[3]));
 #pragma unroll
       for (int j = 0; j < 4; j += 2) {
         unsigned char* const pr = asmem + M::P + warp * M::PROW;
