@@ -64,3 +64,31 @@ def test_last_tokens_of_a_batch_go_along(batch, tokens, chunk):
   assert [list(t) for t in zip(*got)] == [_first(one, p)[0] for p in prompts]
   again = next(m.generate_batch([p[::-1] for p in prompts]))
   assert again == [_first(one, p[::-1], 1)[0][0] for p in prompts]
+
+
+# prompts that go in one pass, and below `prefill_rows` in steps; a batch of one is the default model
+@pytest.mark.parametrize("batch", [1, 3])
+@pytest.mark.parametrize("use_graph", [True, False])
+@pytest.mark.parametrize("order", ["one batch one batch", "batch one batch one", "short batch one short", "batch short one batch"])
+def test_one_model_answers_prompts_and_batches(order, batch, use_graph):
+  """What one model says to single prompts and to batches in turn, tokens, logits and all: as one that has done nothing else."""
+  need_gpu()
+  kw = dict(batch=batch, prefill_chunk=32, use_graph=use_graph)
+  m = _model(**kw)
+  for i, kind in enumerate(order.split()):
+    rng, fresh = np.random.default_rng(i), _model(**kw)
+    if kind == "batch":
+      prompts = [[i] + [int(t) for t in rng.integers(0, 512, 9 + i)] for _ in range(batch)]
+      got, want = ([t for t, _ in zip(x.generate_batch(prompts), range(4))] for x in (m, fresh))
+      assert got == want
+    else:
+      prompt = [i] + [int(t) for t in rng.integers(0, 512, 20 if kind == "one" else 3)]
+      (got, lg), (want, lw) = _first(m, prompt, 4), _first(fresh, prompt, 4)
+      assert got == want
+      np.testing.assert_array_equal(lg, lw)
+    for a, b in zip(m.blk, fresh.blk):      # the rows that this call has written
+      n = len(prompts[0] if kind == "batch" else prompt) + 3
+      seqs = batch if kind == "batch" else 1
+      for x, y in ((a.k_cache, b.k_cache), (a.v_cache, b.v_cache)):
+        x, y = (t.numpy().reshape(batch, 2, 64, 64)[:seqs, :, :n] for t in (x, y))
+        np.testing.assert_array_equal(x, y)

@@ -449,7 +449,8 @@ class Transformer:
       check(_lib.load().b200q_prompt_rows_kv(native, seq, 1, p0, rows, self.stream.ptr))
     return rows
 
-  def _captured(self, key, enqueue) -> Graph:
+  def _captured(self, key: tuple, enqueue) -> Graph:
+    """The graph of a launch sequence.  key: what `enqueue` enqueues, in full: one model serves single prompts and batches, with sequences of their own."""
     g = self._graphs.get(key)
     if g is None:
       g = Graph(self.stream)
@@ -457,13 +458,13 @@ class Transformer:
       self._graphs[key] = g
     return g
 
-  def _last_block(self, enqueue, step) -> None:
+  def _last_block(self, kind: str, enqueue, step) -> None:
     """Replays the last block, the head and the arg-max on rows that a prompt pass has left (captured on first use).  The steps that will follow, `step`, are captured here
-    too: the device still has the prompt to do."""
+    too: the device still has the prompt to do.  kind: "one" sequence or a "batch"."""
     self._head_queued = True
     if not self.use_graph: return enqueue()
-    self._captured("last_block", enqueue).launch()
-    self._captured(True, step)
+    self._captured((kind, "last block"), enqueue).launch()
+    self._captured((kind, "step", True), step)
 
   def _prompt_to_last_block(self, native, start_pos: int, n: int):
     """tokens[start_pos : start_pos + n] as rows up to the last block -> what takes the last one of them through that and samples the token behind it."""
@@ -474,7 +475,7 @@ class Transformer:
     def finish():
       self._check_room()
       self._host_pos += 1
-      self._last_block(lambda: self._enqueue_step(True, last_block=True), lambda: self._enqueue_step(True))
+      self._last_block("one", lambda: self._enqueue_step(True, last_block=True), lambda: self._enqueue_step(True))
     return finish
 
   def _enqueue_rows_block(self, b, T: int, f: dict, p0, seq: int) -> None:
@@ -558,7 +559,7 @@ class Transformer:
     if not self.use_graph: return self._enqueue_batch_step()
     self._prefill_buffers()
     self._batch_buffers()                              # (a capture allocates nothing)
-    self._captured(True, lambda: self._enqueue_batch_step(count=False)).launch()
+    self._captured(("batch", "step", True), lambda: self._enqueue_batch_step(count=False)).launch()
     self._host_pos += 1
 
   def _batch_buffers(self):
@@ -645,7 +646,7 @@ class Transformer:
       check(lib.b200q_permute_rows(f["x"].ptr, at.ptr, seqs, size, last.ptr + i * size, 1, s))
     check(lib.b200q_memcpy_d2d(f["x"].ptr, last.ptr, B * size, s))
     self._host_pos = n
-    self._last_block(lambda: self._enqueue_batch_step(count=False, last_block=True), lambda: self._enqueue_batch_step(count=False))
+    self._last_block("batch", lambda: self._enqueue_batch_step(count=False, last_block=True), lambda: self._enqueue_batch_step(count=False))
 
   def generate_batch(self, prompts: list):
     """Greedy generation for `batch` prompts of equal length; yields the list of the sequences' next tokens per step."""
@@ -672,16 +673,10 @@ class Transformer:
     """One token through the row path (mixture-of-experts models: their FFN is not part of the fused one-token chain).  Positions come
     from the device, so the launches are captured once (behind a first step that allocates) and replayed as a CUDA graph."""
     if not self.use_graph: self._enqueue_step_rows(with_head)
-    elif with_head not in self._graphs and not self._rows_warm:
+    elif not self._rows_warm:
       self._enqueue_step_rows(with_head)
       self._rows_warm = True
-    else:
-      g = self._graphs.get(with_head)
-      if g is None:
-        g = Graph(self.stream)
-        with g: self._enqueue_step_rows(with_head)
-        self._graphs[with_head] = g
-      g.launch()
+    else: self._captured(("rows", "step", bool(with_head)), lambda: self._enqueue_step_rows(with_head)).launch()
     self._host_pos += 1
 
   def _enqueue_step_rows(self, with_head: bool) -> None:
@@ -732,7 +727,7 @@ class Transformer:
     self._host_pos += 1
     if self._step_args: return check(_lib.load().b200q_decode_step(ctypes.byref(self._step_args[bool(with_head)]), self.stream.ptr))
     if not self.use_graph: return self._enqueue_step(with_head)
-    self._captured(bool(with_head), lambda: self._enqueue_step(with_head)).launch()
+    self._captured(("one", "step", bool(with_head)), lambda: self._enqueue_step(with_head)).launch()
 
   # ---- host-visible state ----
   def set_state(self, tokens: list, pos: int) -> None:
