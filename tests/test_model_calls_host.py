@@ -70,3 +70,11 @@ def test_one_model_for_a_prompt_and_for_a_batch(made, order, batch):
     for _ in range(3): next(answers)
     want = {"one": ONE, "batch": BATCH, "short": [("step", "one")] * 5}[kind]
     assert _steps(log) == want, (kind, i)
+
+
+@pytest.mark.parametrize("batch,tokens", [(40, 8), (17, 7), (17, 1)])
+def test_a_batch_of_more_sequences_than_rows_is_refused_before_its_first_launch(made, batch, tokens):
+  """Their last rows are gathered in the row buffer: nothing may be on its way there when the number of sequences is looked at."""
+  m, log = made(batch)
+  with pytest.raises(AssertionError): next(m.generate_batch([list(range(tokens))] * batch))
+  assert log == [] and m._graphs == {}

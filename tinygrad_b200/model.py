@@ -653,6 +653,7 @@ class Transformer:
     c, B = self.config, self.batch
     assert len(prompts) == B and len({len(p) for p in prompts}) == 1 and len(prompts[0]) >= 1
     L = len(prompts[0])
+    assert L >= c.max_context or B <= self.prefill_chunk and not self.is_moe, "a step takes a row of the row buffers per sequence"
     self.stream.synchronize()
     tok = np.zeros((B, c.max_context + 1), np.int32)
     for i, p in enumerate(prompts): tok[i, :L] = p
