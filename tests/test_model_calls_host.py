@@ -43,7 +43,7 @@ def made(monkeypatch):
     def sampled(step, n=1):
       step()
       return [7] * n
-    for name, f in dict(_native_rows=lambda: "rows", _prefill_buffers=lambda: m._pf, _batch_buffers=lambda: None, _sampled=sampled,
+    for name, f in dict(_native_rows=lambda: m._prefill_buffers() and "rows", _prefill_buffers=lambda: m._pf, _batch_buffers=lambda: None, _sampled=sampled,
                         _enqueue_step=lambda with_head, last_block=False: log.append(("last block" if last_block else "step", "one", with_head)),
                         _enqueue_batch_step=lambda count=True, last_block=False: log.append(("last block" if last_block else "step", "batch", True))).items():
       monkeypatch.setattr(m, name, f)
@@ -78,3 +78,16 @@ def test_a_batch_of_more_sequences_than_rows_is_refused_before_its_first_launch(
   m, log = made(batch)
   with pytest.raises(AssertionError): next(m.generate_batch([list(range(tokens))] * batch))
   assert log == [] and m._graphs == {}
+
+
+def test_prefill_is_the_same_call_after_a_prompt_that_failed(made, monkeypatch):
+  """A prompt for whose buffers there is no memory leaves nothing behind that changes what `prefill` does: n tokens, waited for, the position moved."""
+  m, log = made(1)
+  def no_memory(): raise MemoryError
+  with monkeypatch.context() as mp:
+    mp.setattr(m, "_prefill_buffers", no_memory)
+    with pytest.raises(MemoryError): next(m.generate(list(range(9))))
+  del log[:]
+  assert m.prefill(0, 20) is None
+  assert log == [("b200q_prompt_rows", 0, 1, 0, 16), ("b200q_prompt_rows", 0, 1, 16, 4)]
+  assert m._host_pos == 20

@@ -91,6 +91,8 @@ STAGED_HANDOVER = os.environ.get("B200Q_STAGED_HANDOVER", "1") == "1"
 
 
 class Transformer:
+  engine = None        # "step" or "chain" once the constructor has chosen
+
   def __init__(self, config: TransformerConfig, state_dict: dict, ggml_type: int = _lib.Q4_0, n_split: int = 0, use_pdl: bool = True,
                use_graph: bool = True, gemv_max_ctas: int = 0, handover=None, tp=None, output_type: int = None, prefill_rows: int = PREFILL_ROWS,
                prefill_chunk: int = 512, batch: int = 1, engine: str = None, linear_types: dict = None, pipelined_gemm: bool = True):
@@ -415,17 +417,13 @@ class Transformer:
         if c.shared_expert_dim: self._pf.update(sh=DeviceBuffer.empty((T, c.dim), np.float32), shg=DeviceBuffer.empty((T,), np.float32))
     return self._pf
 
-  _take_along = False      # set by `generate` for its call of `prefill`
-
-  def prefill(self, start_pos: int, n: int, sync: bool = True, seq: int = 0):
+  def prefill(self, start_pos: int, n: int, sync: bool = True, seq: int = 0) -> None:
     """Run tokens[start_pos : start_pos + n] (already on the device) through every block and fill the KV cache; no logits.
     The forward of tinygrad/llm/model.py:358-362 for T = n, in chunks: per block rmsnorm -> QKV GEMM -> RoPE + cache append +
     causal attention -> O GEMM (+residual) -> rmsnorm -> gate/up GEMM with SwiGLU epilogue -> down GEMM (+residual).
-    Activations stay fp32 between the kernels; the GEMMs split them into fp16 hi + lo halves for the tensor core.
-    Called by `generate`, whose prompt has one more token: that one goes along where it can, and what finishes it is returned."""
+    Activations stay fp32 between the kernels; the GEMMs split them into fp16 hi + lo halves for the tensor core."""
     c, lib, s, f = self.config, _lib.load(), self.stream.ptr, self._prefill_buffers()
-    native, along, self._take_along = self._native_rows(), self._take_along, False
-    if along and native and n % self.prefill_chunk: return self._prompt_to_last_block(native, start_pos, n + 1)      # (a last pass of one row would cost what a step does)
+    native = self._native_rows()
     for p0 in range(start_pos, start_pos + n, self.prefill_chunk) if native else ():
       check(lib.b200q_prompt_rows(native, seq, 1, p0, min(self.prefill_chunk, start_pos + n - p0), s))
     for p0 in () if native else range(start_pos, start_pos + n, self.prefill_chunk):
@@ -465,6 +463,10 @@ class Transformer:
     if not self.use_graph: return enqueue()
     self._captured((kind, "last block"), enqueue).launch()
     self._captured((kind, "step", True), step)
+
+  def _last_goes_along(self, n: int) -> bool:
+    """Whether the token behind n prompt tokens goes through the blocks with them (a last pass of one row would cost what a step does)."""
+    return self.engine == "chain" and n % self.prefill_chunk != 0 and self._native_rows() is not None
 
   def _prompt_to_last_block(self, native, start_pos: int, n: int):
     """tokens[start_pos : start_pos + n] as rows up to the last block -> what takes the last one of them through that and samples the token behind it."""
@@ -782,8 +784,8 @@ class Transformer:
     self._put_tokens(tokens, start_pos)
     n_pre, step = len(tokens) - 1 - start_pos, self.step
     if self.prefill_rows and n_pre >= self.prefill_rows:
-      self._take_along = len(tokens) < self.max_context and not self._step_args
-      step = self.prefill(start_pos, n_pre) or step
+      if len(tokens) < self.max_context and self._last_goes_along(n_pre): step = self._prompt_to_last_block(self._native_rows(), start_pos, n_pre + 1)
+      else: self.prefill(start_pos, n_pre)
     else:
       for _ in range(n_pre): self.step(with_head=False)
     while len(tokens) < self.max_context:
