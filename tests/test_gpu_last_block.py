@@ -92,3 +92,16 @@ def test_one_model_answers_prompts_and_batches(order, batch, use_graph):
       for x, y in ((a.k_cache, b.k_cache), (a.v_cache, b.v_cache)):
         x, y = (t.numpy().reshape(batch, 2, 64, 64)[:seqs, :, :n] for t in (x, y))
         np.testing.assert_array_equal(x, y)
+
+
+def test_a_conversation_goes_on_after_a_batch():
+  """The batch has written over sequence 0's cache rows: none of them may be reused."""
+  need_gpu()
+  rng = np.random.default_rng(4)
+  talk = [int(t) for t in rng.integers(0, 512, 20)]
+  m, fresh = _model(batch=2), _model(batch=2)
+  _first(m, talk, 2)
+  next(m.generate_batch([[int(t) for t in rng.integers(0, 512, 15)] for _ in range(2)]))
+  (got, lg), (want, lw) = _first(m, talk + [3, 1], 4), _first(fresh, talk + [3, 1], 4)
+  assert got == want
+  np.testing.assert_array_equal(lg, lw)

@@ -91,3 +91,19 @@ def test_prefill_is_the_same_call_after_a_prompt_that_failed(made, monkeypatch):
   assert m.prefill(0, 20) is None
   assert log == [("b200q_prompt_rows", 0, 1, 0, 16), ("b200q_prompt_rows", 0, 1, 16, 4)]
   assert m._host_pos == 20
+
+
+@pytest.mark.parametrize("between", ["batch", "failed", "full"])
+def test_cache_rows_that_another_call_has_written_are_not_reused(made, monkeypatch, between):
+  """A conversation goes on where its rows are still there.  They are not after a batch, after a prompt that failed on its way, or after one that fills the context (no token
+  follows it): all three have written over them."""
+  m, log = made(2)
+  talk = [5, 6] + list(range(20))
+  next(m.generate(talk))
+  if between == "batch": next(m.generate_batch([[9] * 12] * 2))
+  elif between == "full": assert list(m.generate([5] + [9] * 63)) == []
+  else:
+    with monkeypatch.context() as mp:
+      mp.setattr(m, "_last_block", lambda *a: (_ for _ in ()).throw(MemoryError()))
+      with pytest.raises(MemoryError): next(m.generate([5] + [9] * 19))
+  assert m.get_start_pos(talk + [7, 1]) == {"batch": 0, "failed": 1, "full": 1}[between]

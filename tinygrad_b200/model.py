@@ -656,6 +656,7 @@ class Transformer:
     assert len(prompts) == B and len({len(p) for p in prompts}) == 1 and len(prompts[0]) >= 1
     L = len(prompts[0])
     assert L >= c.max_context or B <= self.prefill_chunk and not self.is_moe, "a step takes a row of the row buffers per sequence"
+    self._cached_tokens = []      # sequence 0's rows are the ones that `generate` reuses
     self.stream.synchronize()
     tok = np.zeros((B, c.max_context + 1), np.int32)
     for i, p in enumerate(prompts): tok[i, :L] = p
@@ -781,6 +782,7 @@ class Transformer:
     if temperature != 0.0: raise NotImplementedError("only greedy decoding (temperature 0) is implemented")
     tokens = list(tokens)
     start_pos = self.get_start_pos(tokens)
+    self._cached_tokens = tokens[:start_pos]      # the rows behind them are about to be written, whether or not a token comes of it
     self._put_tokens(tokens, start_pos)
     n_pre, step = len(tokens) - 1 - start_pos, self.step
     if self.prefill_rows and n_pre >= self.prefill_rows:
