@@ -8,17 +8,18 @@ pytestmark = pytest.mark.gpu
 
 
 # one expert; fewer than a cluster's warps, more than a warp's lanes (fp16 router), more than 64 and the most, more choices than rows loaded ahead; widths below and above
-# a thread's first pieces; every gating but the default's, with a shared expert
+# a thread's first pieces; every gating but the default's, with a shared expert; attention rows of the most values that one CTA takes, and of more (the launches of rows then)
 @pytest.mark.parametrize("dim,f,E,k,router,extra", [
   (256, 128, 1, 1, np.float32, {}), (768, 768, 8, 6, np.float32, {}), (1280, 1152, 40, 3, np.float16, dict(norm_topk_prob=True)),
   (512, 512, 130, 9, np.float32, dict(expert_gating_func="sigmoid", norm_topk_prob=True, routed_scaling_factor=2.0, shared_expert_dim=128)),
-  (2304, 128, 256, 32, np.float32, dict(expert_gating_func="sqrt_softplus", expert_bias=True, shared_expert_dim=96, shared_expert_gate=False))])
+  (2304, 128, 256, 32, np.float32, dict(expert_gating_func="sqrt_softplus", expert_bias=True, shared_expert_dim=96, shared_expert_gate=False)),
+  (256, 128, 8, 2, np.float32, dict(n_heads=96, n_kv_heads=8, head_dim=128, rope_dim=128)), (256, 128, 8, 2, np.float32, dict(n_heads=97, n_kv_heads=1, head_dim=128, rope_dim=128))])
 def test_one_token_block_is_the_row_block(dim, f, E, k, router, extra):
   need_gpu()
   from tinygrad_b200 import _lib
   from tinygrad_b200.model import Transformer, TransformerConfig
   kw = dict(num_blocks=2, dim=dim, hidden_dim=f, n_heads=dim // 64, n_kv_heads=dim // 128, norm_eps=1e-5, vocab_size=64, head_dim=64, rope_theta=10000.0, rope_dim=64,
-            max_context=64, num_experts=E, num_experts_per_tok=k, **extra)
+            max_context=64, num_experts=E, num_experts_per_tok=k) | extra
   cfg, rng = TransformerConfig(**kw), np.random.default_rng(dim + k)
   sd = {n: v for n, v in synth.dense_model_raw(cfg, 8, seed=7, embd_std=0.3, scale_std=0.0015).items() if ".ffn_gate." not in n and ".ffn_up." not in n and ".ffn_down." not in n}
   sh = cfg.shared_expert_dim

@@ -17,6 +17,7 @@ void b200q_set_cuda_error(cudaError_t e);
 // ---- launch chains.  Exported entry points launch their first kernel fully ordered behind whatever the caller has put on the stream; the `pdl`
 // argument of the internal forms below is for calls whose predecessor on the stream is known to be a kernel of this library.
 // one row of a GEMM that is not split, with what is in front of it: x += the weighted sum of the k rows dest_row of y (bf16; NULL: nothing), RMSNorm (norm_w NULL: none)
+constexpr int B200Q_ROW_INPUT_MAX = 12288;      // values of such a row: it stands in shared memory (48 KB)
 struct b200q_row_input { float* x; const void* y; const int32_t* dest_row; const float* weights; int k; const void* norm_w; float eps; };
 int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtype, const void* norm_weight, float norm_eps, const void* bias_f16, const void* residual,
                       int epilogue, void* y, int y_dtype, int m, int n_out, int n_in, void* workspace, size_t workspace_bytes, cudaStream_t st, bool pdl,

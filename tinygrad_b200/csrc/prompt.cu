@@ -103,7 +103,7 @@ extern "C" int b200q_moe_rows(const b200q_rows_args* a, const b200q_moe_block* b
   int rc = pos_dev ? b200q_embed_rows(a->token_embd, a->tokens, 1, pos_dev, 1, a->dim, a->vocab, a->x, stream)
                    : b200q_embed_rows_seqs(a->token_embd, a->tokens + (size_t)seq * (a->max_context + 1) + start_pos, a->max_context + 1, T, T, a->dim, a->vocab, a->x, st);
   for (int i = 0; i < a->n_layers; i++) if (!blocks[i].moe || !blocks[i].router || !blocks[i].xn || !blocks[i].xb || !blocks[i].logits) return B200Q_ERR_BAD_ARG;
-  bool one = pos_dev != nullptr && a->dim <= 12288 && q_dim <= 12288;      // (a row in the 48 KB of shared memory that prepare_row_kernel has)
+  bool one = pos_dev != nullptr && a->dim <= B200Q_ROW_INPUT_MAX && q_dim <= B200Q_ROW_INPUT_MAX;
   for (int i = 0; i < a->n_layers; i++) one = one && b200q_moe_router_one_takes(blocks[i].moe, blocks[i].router_dtype);
   if (one && rc == B200Q_OK) return moe_one_token(a, blocks, pos_dev, st);
   for (int i = 0; i < a->n_layers && rc == B200Q_OK; i++) {

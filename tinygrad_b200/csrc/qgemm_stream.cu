@@ -846,9 +846,16 @@ int b200q_qgemm_chain(int qtype, const void* w_packed, const void* x, int x_dtyp
   const int n_counters = split ? grid : 0;
   if (row) {
     if (m != 1 || !f32 || split || n_in % 8 || norm_weight) return B200Q_ERR_BAD_ARG;
-    const size_t smem = (size_t)n_in * sizeof(float);
-    if (smem > 48 * 1024) return B200Q_ERR_TOO_LARGE;
-    B200Q_CHECK_CUDA(launch_k(prepare_row_kernel, dim3(1), dim3(ROW_THREADS), smem, st, pdl, *row, n_in, kgroups, pl.nt, (unsigned char*)p.xt, (float*)p.down));
+    if (n_in > B200Q_ROW_INPUT_MAX) return B200Q_ERR_TOO_LARGE;
+    static PerDeviceFlag attr_set;
+    const int dev = b200q_current_device();
+    if (dev < 0) return B200Q_ERR_CUDA;
+    if (!attr_set.test(dev)) {      // (without it, 48 KB with the static part)
+      B200Q_CHECK_CUDA(cudaFuncSetAttribute(prepare_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, B200Q_ROW_INPUT_MAX * (int)sizeof(float)));
+      attr_set.set(dev);
+    }
+    B200Q_CHECK_CUDA(launch_k(prepare_row_kernel, dim3(1), dim3(ROW_THREADS), (size_t)n_in * sizeof(float), st, pdl, *row, n_in, kgroups, pl.nt, (unsigned char*)p.xt,
+                              (float*)p.down));
   } else if (f32)
     B200Q_CHECK_CUDA(cudaLaunchKernelEx(&cfg, cluster ? split_rows_kernel<float, true> : split_rows_kernel<float, false>, (const float*)x, (const __half*)norm_weight, norm_eps, m,
                                         n_in, kgroups, pl.nt, per, (unsigned char*)p.xt, p.counters, n_counters, (float*)p.down, unsplit ? 0.f : 1.f));
