@@ -125,3 +125,13 @@ def test_step_past_the_context_end_raises_before_any_launch():
   with pytest.raises(RuntimeError, match="context full"): m.step()
   with pytest.raises(RuntimeError, match="context full"): m.decode_batch_step()
   assert m._host_pos == 64
+
+
+@pytest.mark.parametrize("missing", ["w_q", "w_factor", "x_q", "off", "parts", "factor"])
+def test_fp8_linear_without_one_of_its_pointers(lib, missing):
+  """Refused as a bad argument, before anything is allocated or launched (without the weight's factor the product would take the form that writes whole tiles of rows)."""
+  d = _lib.Fp8LinearDesc(256, 128, 256, *[0x1000] * 3, None, *[0x1000] * 5)
+  setattr(d, missing, None)
+  y = ctypes.c_void_p(0x10)
+  assert lib.b200q_fp8_linear(ctypes.byref(d), 0x1000, _lib.F32, 3, ctypes.byref(y), None) == -1
+  assert y.value == 0x10
