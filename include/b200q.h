@@ -593,8 +593,8 @@ int b200q_fp8_quantize(const void* x, int x_dtype, int64_t n, const float* amax,
 int b200q_fp8_scale_bias(const float* acc, int64_t rows, int n, const float* factor_w, const float* factor_x, const float* bias, void* y, int y_dtype,
                          void* stream);
 /* The whole `FP8Linear.__call__` (m >= 1 rows of x, dtype B200Q_F32 | B200Q_F16; *y = a new b200q_pool_alloc block [m, n_out] of that type):
- * w_q / w_e8 / w_factor the quantised weight (unit block scales), bias fp32 [n_out], 16-byte aligned, or NULL; scratch of the caller: x_q [rows_max, n_in] and
- * x_e8 [rows_max, n_in / 32] (all 127), rows_max a multiple of 256 and at least m; off int32 {0, rows_max}; parts float [592]; factor float. */
+ * w_q / w_factor the quantised weight, bias fp32 [n_out], 16-byte aligned, or NULL; scratch of the caller: x_q [rows_max, n_in], rows_max a multiple of 256 and
+ * at least m; off int32 {0, rows_max}; parts float [592]; factor float.  Per-tensor codes have no block scales: w_e8 and x_e8 are not read and may be NULL. */
 typedef struct b200q_fp8_linear_desc {
   int n_out, n_in, rows_max;
   const void* w_q;

@@ -59,3 +59,20 @@ def test_fp8_codes_in_one_launch(rows, n_in, dt):
     factor = DeviceBuffer.empty((1,), np.float32)
     _lib.check(_lib.load().b200q_memcpy_d2d(factor.ptr, w.factor, 4, None))
     assert factor.numpy()[0] == f.numpy()[0]
+
+
+@pytest.mark.parametrize("m", [1, 40, 300])
+def test_fp8_linear_reads_no_block_scales(m):
+  """The descriptor's block scales may be missing, or anything: per-tensor codes have none."""
+  need_gpu()
+  from tinygrad_b200.fp8 import FP8Linear
+  from tinygrad_b200.runtime import DeviceBuffer
+  rng = np.random.default_rng(m)
+  lin = FP8Linear(256, 512, rng.standard_normal((512, 256)).astype(np.float32))
+  x = DeviceBuffer.from_numpy(rng.standard_normal((m, 256)).astype(np.float32))
+  want, d = lin(x).numpy(), lin._workspace(m)
+  scales = DeviceBuffer.from_numpy(rng.integers(100, 150, (512, 8)).astype(np.uint8))
+  d.w_e8 = d.x_e8 = scales.ptr
+  np.testing.assert_array_equal(lin(x).numpy(), want)
+  d.w_e8 = d.x_e8 = None
+  np.testing.assert_array_equal(lin(x).numpy(), want)

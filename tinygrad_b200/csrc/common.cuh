@@ -41,8 +41,8 @@ struct PerDeviceFlag {
 // gives the result pool's unused blocks of a device back (pool.cu); false: there were none
 bool b200q_pool_release(int dev);
 // fp8 product with factors, bias and output type in the epilogue (mxfp8_gemm.cu)
-int b200q_mx_gemm_scaled(const void* a_q, const void* a_e8, const void* b_q, const void* b_e8, const int32_t* off, int m_total, int n, int k, void* y, int y_dtype,
-                         int rows, const float* fw, const float* fx, const float* bias, cudaStream_t st);
+int b200q_mx_gemm_scaled(const void* a_q, const void* b_q, const int32_t* off, int m_total, int n, int k, void* y, int y_dtype, int rows,
+                         const float* fw, const float* fx, const float* bias, cudaStream_t st);
 int b200q_mx_gemm_chain(const void* a_q, const void* a_e8, const void* b_q, const void* b_e8, const int32_t* off, const int32_t* ends, int n_experts, int m_total, int n,
                         int k, void* c_bf16, void* act_q, void* act_e8, int n_tokens, int topk, cudaStream_t st);
 int b200q_moe_layer_chain(const b200q_moe_args* m, const void* x_bf16, const float* logits, int n_tokens, float* add_to, cudaStream_t st, bool pdl);

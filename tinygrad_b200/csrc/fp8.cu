@@ -224,10 +224,11 @@ extern "C" int b200q_fp8_scale_bias(const float* acc, int64_t rows, int n, const
   return B200Q_OK;
 }
 
-// The whole call in three launches: partial maxima, quantise, product with the factors and the bias in its epilogue; the result in a pool block.
+// The whole call in two launches (maximum and codes, product with the factors and the bias in its epilogue) or, where one cannot have the tensor in registers, three; the
+// result in a pool block.
 extern "C" int b200q_fp8_linear(const b200q_fp8_linear_desc* l, const void* x, int dtype, int m, void** y, void* stream) {
   if (!l || !y || m <= 0 || !x || (dtype != B200Q_F32 && dtype != B200Q_F16)) return B200Q_ERR_BAD_ARG;
-  if (!l->w_q || !l->w_factor || !l->x_q || !l->x_e8 || !l->off || !l->parts || !l->factor || m > l->rows_max) return B200Q_ERR_BAD_ARG;
+  if (!l->w_q || !l->w_factor || !l->x_q || !l->off || !l->parts || !l->factor || m > l->rows_max) return B200Q_ERR_BAD_ARG;
   if (l->n_out <= 0 || l->n_out % 256 || l->n_in <= 0 || l->n_in % 128) return B200Q_ERR_BAD_SHAPE;
   if ((uintptr_t)l->bias & 15) return B200Q_ERR_MISALIGNED;      // read 16 bytes at a time
   cudaStream_t st = (cudaStream_t)stream;
@@ -248,7 +249,7 @@ extern "C" int b200q_fp8_linear(const b200q_fp8_linear_desc* l, const void* x, i
                                         l->factor, vec);
   }
   if (e != cudaSuccess) { b200q_set_cuda_error(e); rc = B200Q_ERR_CUDA; }
-  else rc = b200q_mx_gemm_scaled(l->x_q, l->x_e8, l->w_q, l->w_e8, l->off, l->rows_max, l->n_out, l->n_in, *y, dtype, m, l->w_factor, l->factor, l->bias, st);
+  else rc = b200q_mx_gemm_scaled(l->x_q, l->w_q, l->off, l->rows_max, l->n_out, l->n_in, *y, dtype, m, l->w_factor, l->factor, l->bias, st);
   if (rc != B200Q_OK) { b200q_pool_free(*y); *y = nullptr; }
   return rc;
 }

@@ -505,7 +505,7 @@ static GroupedKernel pick_kernel(int out, int bn) { return bn == 256 ? pick_out<
 static int grouped_launch(const void* a_q, const void* a_e8, const void* b_q, const void* b_e8, const int32_t* off, int n_experts, int m_total, int n, int k,
                           void* c_bf16, void* act_q, void* act_e8, void* stream, bool c_f32 = false, ScaledOut so = ScaledOut{}, bool pdl = false, const int32_t* ends = nullptr,
                           int row_tiles = 0, bool few_rows = false) {
-  if (!a_q || !a_e8 || !b_q || !b_e8 || !off || (!c_bf16 && !act_q) || n_experts <= 0 || m_total <= 0 || n <= 0 || k <= 0) return B200Q_ERR_BAD_ARG;
+  if (!a_q || !b_q || (!so.fw && (!a_e8 || !b_e8)) || !off || (!c_bf16 && !act_q) || n_experts <= 0 || m_total <= 0 || n <= 0 || k <= 0) return B200Q_ERR_BAD_ARG;
   if (act_q && (!act_e8 || (((uintptr_t)act_q) & 15))) return B200Q_ERR_BAD_ARG;
   if (m_total % 256 || n % BN_MAX || k % BK) return B200Q_ERR_BAD_SHAPE;       // the reference asks M % 256 == N % 256 == K % 128 == 0 (moe_gemm.py:120)
   if (n_experts > MAX_EXPERTS) return B200Q_ERR_UNSUPPORTED;
@@ -540,9 +540,10 @@ static int grouped_launch(const void* a_q, const void* a_e8, const void* b_q, co
   return B200Q_OK;
 }
 
-int b200q_mx_gemm_scaled(const void* a_q, const void* a_e8, const void* b_q, const void* b_e8, const int32_t* off, int m_total, int n, int k, void* y, int y_dtype,
-                         int rows, const float* fw, const float* fx, const float* bias, cudaStream_t st) {
-  return grouped_launch(a_q, a_e8, b_q, b_e8, off, 1, m_total, n, k, y, nullptr, nullptr, st, true, ScaledOut{fw, fx, bias, rows, y_dtype == B200Q_F16}, true, nullptr,
+// codes without block scales (the kernel has its own units)
+int b200q_mx_gemm_scaled(const void* a_q, const void* b_q, const int32_t* off, int m_total, int n, int k, void* y, int y_dtype, int rows, const float* fw, const float* fx,
+                         const float* bias, cudaStream_t st) {
+  return grouped_launch(a_q, nullptr, b_q, nullptr, off, 1, m_total, n, k, y, nullptr, nullptr, st, true, ScaledOut{fw, fx, bias, rows, y_dtype == B200Q_F16}, true, nullptr,
                         (rows + BM - 1) / BM, rows <= FEW_ROWS);
 }
 

@@ -28,7 +28,7 @@ class FP8Linear:
     self.weight = DeviceBuffer.from_numpy(np.ascontiguousarray(weight, dtype=np.float32).reshape(out_features, in_features))
     self.bias = None if bias is None else DeviceBuffer.from_numpy(np.asarray(bias, dtype=np.float32).reshape(out_features))
     self._w_e8 = DeviceBuffer(out_features * in_features // 32)
-    check(_lib.load().b200q_memset(self._w_e8.ptr, 127, self._w_e8.nbytes, None))       # E8M0 127 = 2^0: the block scales are all one
+    check(_lib.load().b200q_memset(self._w_e8.ptr, 127, self._w_e8.nbytes, None))       # E8M0 127 = 2^0: the codes as a block-scaled operand (`__call__` needs none)
     self._ws = {}
     self.requantize()
 
@@ -40,12 +40,11 @@ class FP8Linear:
     w = self._ws.get(m)
     if w is None:
       lib = _lib.load()
-      w = dict(x_q=DeviceBuffer.empty((mp, self.in_features), np.uint8, zero=True), x_e8=DeviceBuffer(mp * self.in_features // 32),
+      w = dict(x_q=DeviceBuffer.empty((mp, self.in_features), np.uint8, zero=True),
                off=DeviceBuffer.from_numpy(np.array([0, mp], np.int32)), parts=DeviceBuffer.empty((592,), np.float32), factor=DeviceBuffer.empty((1,), np.float32))
-      check(lib.b200q_memset(w["x_e8"].ptr, 127, w["x_e8"].nbytes, None))
       check(lib.b200q_device_synchronize())
-      w["desc"] = _lib.Fp8LinearDesc(self.out_features, self.in_features, mp, None, self._w_e8.ptr, None, None, w["x_q"].ptr,
-                                     w["x_e8"].ptr, w["off"].ptr, w["parts"].ptr, w["factor"].ptr)
+      w["desc"] = _lib.Fp8LinearDesc(self.out_features, self.in_features, mp, None, None, None, None, w["x_q"].ptr,
+                                     None, w["off"].ptr, w["parts"].ptr, w["factor"].ptr)
       self._ws[m] = w
     return w["desc"]
 
