@@ -49,7 +49,8 @@ def test_row_gemv(typ, n_out, n_in):
 @pytest.mark.parametrize("typ,n_out,n_in,taken", [(2, 4096, 2048, True), (8, 4097, 2048, False), (2, 16, 2080, False), (8, 100, 32, True)])
 @pytest.mark.parametrize("form", ["plain", "norm_bias_residual", "silu"])
 def test_gemv_takes_the_row_kernel(typ, n_out, n_in, taken, form):
-  """A grid limit keeps a call on the streaming kernel: the two differ by its 15-bit activation codes, half a step of a block's largest value per product."""
+  """A grid limit keeps a call on the streaming kernel: the two differ by its 15-bit activation codes, half a step of a block's largest value per product.  Which one a call without
+  a limit took shows on rows whose blocks have one large value beside small ones of less than half a step: codes lose those, fp32 does not."""
   need_gpu()
   from tinygrad_b200 import quant
   from tinygrad_b200.runtime import DeviceBuffer
@@ -57,27 +58,38 @@ def test_gemv_takes_the_row_kernel(typ, n_out, n_in, taken, form):
   if form == "silu": n_out = -(-n_out // 2)
   raw, up = _blocks(typ, n_out, n_in, rng), _blocks(typ, n_out, n_in, rng)
   p = quant.repack(raw, n_out, n_in, typ, raw_up=up if form == "silu" else None)
-  x = rng.standard_normal(n_in).astype(np.float32)
-  dx, nw = DeviceBuffer.from_numpy(x), rng.uniform(0.5, 1.5, n_in).astype(np.float16)
+  w, wu = (gq.weight_matrix(r, n_out, n_in, typ).astype(np.float64) for r in (raw, up))
+  nw, bias, res = rng.uniform(0.5, 1.5, n_in).astype(np.float16), rng.standard_normal(n_out).astype(np.float16), rng.standard_normal(n_out).astype(np.float32)
+  nw[::32] = 1
   kw = {}
   if form != "plain": kw.update(norm_weight=DeviceBuffer.from_numpy(nw), norm_eps=1e-5)
-  if form == "norm_bias_residual":
-    kw.update(bias=DeviceBuffer.from_numpy(rng.standard_normal(n_out).astype(np.float16)), residual=DeviceBuffer.from_numpy(rng.standard_normal(n_out).astype(np.float32)))
+  if form == "norm_bias_residual": kw.update(bias=DeviceBuffer.from_numpy(bias), residual=DeviceBuffer.from_numpy(res))
   if form == "silu": kw.update(epilogue=quant.EPI_SILU_MUL)
-  out = []
-  for limit in (0, 100000):
-    y = DeviceBuffer.empty((n_out,), np.float32, zero=True)
+  def run(x, limit):
+    dx, y = DeviceBuffer.from_numpy(x), DeviceBuffer.empty((n_out,), np.float32, zero=True)
     quant.gemv(p.buf.ptr, typ, n_out, n_in, dx, y, max_ctas=limit, **kw)
-    out.append(y.numpy().astype(np.float64))
-  w, wu = (gq.weight_matrix(r, n_out, n_in, typ).astype(np.float64) for r in (raw, up))
-  xn = x.astype(np.float64)
-  if form != "plain": xn = xn / np.sqrt((xn ** 2).mean() + 1e-5) * nw
-  half = np.repeat(np.abs(xn.reshape(-1, 32)).max(1) / 16256 / 2, 32)
+    return y.numpy().astype(np.float64)
+  def normed(x):
+    return x.astype(np.float64) if form == "plain" else x / np.sqrt((x.astype(np.float64) ** 2).mean() + 1e-5) * nw
+  def exact(xn):
+    if form == "silu": return (w @ xn) / (1 + np.exp(-(w @ xn))) * (wu @ xn)
+    return w @ xn + (bias.astype(np.float64) + res if form == "norm_bias_residual" else 0)
+  def bound(xn, per_value):      # of the result, for an error per_value of each of the row's values (|silu'| <= 1.1)
+    b = np.abs(w) @ per_value
+    if form == "plain": return b
+    if form == "norm_bias_residual": return b + 2.0 ** -22 * (np.abs(bias) + np.abs(res) + np.abs(exact(xn)))
+    ub = np.abs(wu) @ per_value
+    return 1.1 * np.abs(wu @ xn) * b + np.abs(w @ xn) * ub + b * ub + 2.0 ** -22 * np.abs(exact(xn))
   fp = 2.0 ** -24 * (64 + n_in / 64)
-  bound = np.abs(w) @ (half + fp * np.abs(xn)) + fp * 8
-  if form == "silu":
-    g, u = w @ xn, wu @ xn
-    ub = np.abs(wu) @ (half + fp * np.abs(xn))
-    bound = 1.1 * np.abs(u) * bound + np.abs(g) * ub + bound * ub
-  assert (np.abs(out[0] - out[1]) <= bound).all()
-  assert taken == (np.abs(out[0] - out[1]).max() > 1e-6 * np.abs(out[0]).max())      # (the streaming kernel adds bias and residual in another order on another grid)
+  x = rng.standard_normal(n_in).astype(np.float32)
+  xn = normed(x)
+  half = np.repeat(np.abs(xn.reshape(-1, 32)).max(1) / 16256 / 2, 32)
+  assert (np.abs(run(x, 0) - run(x, 100000)) <= bound(xn, half + fp * np.abs(xn)) + fp * 8).all()
+  x = (1.8e-5 * rng.choice([-1.0, 1.0], n_in)).astype(np.float32)      # (norm weights are 1.5 at most: 2.7e-5 of the block's largest; half a step is 3.1e-5)
+  x[::32] = 1
+  xn = normed(x)
+  codes = np.where(np.arange(n_in) % 32 == 0, xn, 0)
+  limit, lost = bound(xn, fp * np.abs(xn)), np.abs(exact(codes) - exact(xn))
+  assert (lost > 2 * limit).any()      # so that a result without the small values, itself off by `limit`, is still off by more than that
+  fp32 = lambda got: (np.abs(got - exact(xn)) <= limit).all()
+  assert fp32(run(x, 0)) == taken and not fp32(run(x, 100000))
