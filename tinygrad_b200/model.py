@@ -782,7 +782,7 @@ class Transformer:
     if temperature != 0.0: raise NotImplementedError("only greedy decoding (temperature 0) is implemented")
     tokens = list(tokens)
     start_pos = self.get_start_pos(tokens)
-    self._cached_tokens = tokens[:start_pos]      # the rows behind them are about to be written, whether or not a token comes of it
+    del self._cached_tokens[start_pos:]      # the rows behind them are about to be written, whether or not a token comes of it
     self._put_tokens(tokens, start_pos)
     n_pre, step = len(tokens) - 1 - start_pos, self.step
     if self.prefill_rows and n_pre >= self.prefill_rows:
