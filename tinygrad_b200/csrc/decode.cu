@@ -404,7 +404,7 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], 
 }
 // The same for operands whose rows 8 .. 15 hold what the rounding of rows 0 .. 7 left: the sums of rows 0 .. 7 are added here, to nearest.  The tensor core
 // truncates, always towards zero, when it adds to an accumulator.  Error of the output's norm against 64 bits, 37 .. 3507 positions (root mean square of 64
-// cases): fp16 caches 2.0e-7 (2.3e-7 with probabilities of at most 1), with running accumulators 3.1e-7; fp32 caches 2.3e-7, 8.6e-7 (up to 2.4e-6); the one-lane-per-position kernel 2.0e-7.
+// cases): fp16 caches 2.0e-7 (2.2e-7 with probabilities of at most 1), with running accumulators 3.1e-7; fp32 caches 2.2e-7, 8.6e-7 (up to 2.4e-6); the one-lane-per-position kernel 2.0e-7.
 __device__ __forceinline__ void mma_f16_rn(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   float p[4] = {0.f, 0.f, c[2], c[3]};
   mma_f16(p, a, b0, b1);

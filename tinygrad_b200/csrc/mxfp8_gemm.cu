@@ -6,18 +6,18 @@
 //
 // Persistent, warp-specialised kernel, one CTA per SM, 128 x 256 output tiles (128 x 128 or x 64 where those are too few for the SMs: tile_columns), tiles of the used
 // rows (off[E]) dealt round-robin:
-//   warps 4-7  loaders: one thread brings the A (128 x 128 B) and B (256 x 128 B) tiles of a K step into a ring of 3 stages by tensor-map copies (K-major, 128-byte
+//   warps 4-7  loaders: one thread brings the A (128 x 128 B) and B (256 x 128 B) tiles of a K step into a ring of 3 to 5 stages by tensor-map copies (K-major, 128-byte
 //              swizzle: 16-byte chunk c of row r sits at chunk c ^ (r & 7)), all of them the step's E8M0 scale words by cp.async (one 32-bit
 //              word = 4 K blocks per row, stored as 32 x 16 B chunks: row r -> chunk r % 32, word r / 32); the copies' bytes and each thread's
-//              words arrive on the stage's "full" mbarrier when they land;
+//              words arrive on the stage's "full" mbarrier when they land (no scale words where all of them are one: UNIT);
 //   warp 8     one thread moves the scale chunks to tensor memory with tcgen05.cp 32x128b.warpx4 (row r -> lane r % 32 of every
 //              32-lane sub-partition, column r / 32: the layout the MMA reads), issues tcgen05.mma kind::mxf8f6f4.block_scale
 //              (scale_vec::1X, 128 x 256 x 32 per instruction, the tensor core applies both block scales), four per K step, and
 //              commits each step to the stage's "empty" mbarrier;
 //   warps 0-3, 9-20  epilogue: tcgen05.ld the fp32 accumulator (256 tensor-memory columns; four warps per 32-lane sub-partition,
 //              64 columns each) into registers, release the accumulator, then one of four endings (OUT_BF16 ..).
-// Loaders run ahead across tile boundaries; the accumulator (one buffer: 2 x 256 columns + the scale columns do not fit the 512 of
-// tensor memory) is handed back after one tensor-memory round trip, the epilogue's arithmetic and stores overlap the next tile's MMAs.
+// Loaders run ahead across tile boundaries; the accumulator (one buffer at every tile width: two of 256 columns and the scale columns do not fit the 512 of
+// tensor memory, and with narrower tiles a CTA has one or few) is handed back after one tensor-memory round trip, the epilogue's arithmetic and stores overlap the next tile's MMAs.
 // Every mbarrier wait is bounded; a wait that runs out raises a status word and makes every role leave.
 #include "common.cuh"
 #include "mxq.cuh"
